@@ -4,20 +4,88 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <mutex>
 #include <new>
 
 #include "../../include/fa_sm120.h"
 #include "fa_fwd_sm100.h"
 
+namespace {
+
+// What all contexts of one GPU share: the stream-ordered pool their scratch is drawn from (freed blocks stay cached in it,
+// so steady-state calls do not reach the driver allocator) and, per stream, scratch kept between calls.  Work on one
+// stream is ordered, so consecutive calls there can use the same buffers and a call costs no allocation.  Kept: small
+// buffers only (a large one is drawn from the pool per call, where the 2 us do not show), for a fixed number of streams.
+// Streams are told apart by their id, which the driver never reuses.  Calls that are being captured into a graph do not
+// use it: a graph may be replayed on any stream.  Created with the first context of the GPU, released with the last.
+struct Kept {
+    unsigned long long stream_id = 0;
+    uint8_t* scratch = nullptr;    // whatever the call writes before it reads it
+    size_t scratch_bytes = 0;
+    uint32_t* flags = nullptr;     // zero when allocated, afterwards values of earlier epochs
+    size_t flag_words = 0;
+    uint32_t epoch = 0;
+    uint32_t* zeros = nullptr;     // words that every call finds zero and leaves zero
+    size_t zero_words = 0;
+    bool used = false;
+};
+constexpr int MAX_DEVICES = 64;
+constexpr int KEPT_STREAMS = 8;
+constexpr size_t KEPT_SCRATCH_MAX = (size_t)64 << 20;
+constexpr size_t KEPT_WORDS_MAX = (size_t)1 << 20;
+struct DeviceScratch {
+    std::mutex lock;               // held from looking a buffer up until the kernels that use it are on the stream
+    int contexts = 0;
+    cudaMemPool_t pool = nullptr;
+    Kept kept[KEPT_STREAMS];
+
+    cudaError_t acquire(int dev) {
+        std::lock_guard<std::mutex> g(lock);
+        if (contexts == 0) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.handleTypes = cudaMemHandleTypeNone;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            const cudaError_t e = cudaMemPoolCreate(&pool, &props);
+            if (e != cudaSuccess) return e;
+            unsigned long long keep = ~0ull;  // keep freed scratch cached in the pool
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        }
+        contexts++;
+        return cudaSuccess;
+    }
+    void release(int dev) {
+        std::lock_guard<std::mutex> g(lock);
+        if (--contexts > 0) return;
+        bool any = false;
+        for (Kept& k : kept) any = any || k.scratch || k.flags || k.zeros;
+        if (any) {   // kernels that still use a kept buffer finish first
+            int cur = -1;
+            cudaGetDevice(&cur);
+            if (cur != dev) cudaSetDevice(dev);
+            cudaDeviceSynchronize();
+            for (Kept& k : kept) {
+                if (k.scratch) cudaFree(k.scratch);
+                if (k.flags) cudaFree(k.flags);
+                if (k.zeros) cudaFree(k.zeros);
+                k = Kept();
+            }
+            if (cur >= 0 && cur != dev) cudaSetDevice(cur);
+        }
+        cudaMemPoolDestroy(pool);  // pending frees complete first (stream-ordered)
+        pool = nullptr;
+    }
+};
+DeviceScratch g_scratch[MAX_DEVICES];
+
+}  // namespace
+
 struct fa_ctx {
     int device;
     int cc_major, cc_minor;
     bool arch_ok;
-    // Stream-ordered pool the per-call scratch (the fp16 copy of V) is drawn from and
-    // returned to; freed blocks stay cached in the pool, so steady-state calls do not
-    // reach the driver allocator.  Owned by the context, destroyed with it.
-    cudaMemPool_t pool;
-    bool has_pool;
+    DeviceScratch* shared;   // nullptr on an unsupported GPU
     char last_err[256];
 };
 
@@ -32,7 +100,7 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 // Checks shared by every forward entry.  `who` prefixes messages.
 fa_status_t validate(fa_ctx_t* c, const char* who, const void* q, const void* k, const void* v, const void* o,
                      int bh, int sl, int hd, int causal, int window, const void* l_out = nullptr) {
-    if (!c->arch_ok || !c->has_pool) { set_err(c, "%s: context was created on an unsupported GPU", who); return FA_ERR_UNSUPPORTED_ARCH; }
+    if (!c->arch_ok || !c->shared) { set_err(c, "%s: context was created on an unsupported GPU", who); return FA_ERR_UNSUPPORTED_ARCH; }
     if (!q || !k || !v || !o) { set_err(c, "%s: null pointer in q/k/v/o", who); return FA_ERR_INVALID_ARG; }
     if (bh <= 0 || sl <= 0) { set_err(c, "%s: bh/sl must be > 0", who); return FA_ERR_INVALID_ARG; }
     if (hd != 64 && hd != 128) { set_err(c, "%s: head_dim must be 64 or 128", who); return FA_ERR_UNSUPPORTED_HD; }
@@ -50,6 +118,92 @@ fa_status_t validate(fa_ctx_t* c, const char* who, const void* q, const void* k,
     return FA_OK;
 }
 
+// One call's scratch: the stream's kept buffers where they serve, else blocks drawn from the pool for this call.
+struct Scratch {
+    void* ptr = nullptr;
+    uint32_t* flags = nullptr;   // nullptr: none kept for this stream (a capture, more streams than slots)
+    uint32_t epoch = 0;
+    uint32_t* zeros = nullptr;
+    void* pooled[2] = {nullptr, nullptr};
+    cudaStream_t stream = nullptr;
+    std::unique_lock<std::mutex> lock;
+
+    // grows one kept buffer of a stream; a block that is replaced is released behind the kernels that use it
+    template <typename T>
+    static cudaError_t grow(cudaMemPool_t pool, T*& buf, size_t& have, size_t want, size_t least, bool zero, cudaStream_t s) {
+        if (have >= want) return cudaSuccess;
+        size_t n = least;
+        while (n < want) n *= 2;
+        if (buf) { cudaFreeAsync(buf, s); buf = nullptr; have = 0; }
+        const size_t bytes = n * sizeof(T);
+        void* p = nullptr;
+        cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, s);
+        if (e != cudaSuccess) return e;
+        if (zero && (e = cudaMemsetAsync(p, 0, bytes, s)) != cudaSuccess) { cudaFreeAsync(p, s); return e; }
+        buf = static_cast<T*>(p);
+        have = n;
+        return cudaSuccess;
+    }
+
+    cudaError_t take(fa_ctx_t* c, cudaStream_t s, size_t bytes, size_t flag_words, size_t zero_words) {
+        stream = s;
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        cudaError_t e = cudaStreamIsCapturing(s, &cap);
+        if (e != cudaSuccess) return e;
+        unsigned long long id = 0;
+        if (cap == cudaStreamCaptureStatusNone && cudaStreamGetId(s, &id) == cudaSuccess) {
+            lock = std::unique_lock<std::mutex>(c->shared->lock);
+            Kept* k = nullptr;
+            for (auto& x : c->shared->kept)
+                if (x.used && x.stream_id == id) { k = &x; break; }
+            if (!k)
+                for (auto& x : c->shared->kept)
+                    if (!x.used) { k = &x; k->used = true; k->stream_id = id; break; }
+            if (k) {
+                if (flag_words && flag_words <= KEPT_WORDS_MAX) {
+                    const uint32_t* before = k->flags;
+                    if ((e = grow(c->shared->pool, k->flags, k->flag_words, flag_words, 4096, true, s)) != cudaSuccess) return e;
+                    if (k->flags != before) k->epoch = 0;
+                    if (++k->epoch == 0) {   // 2^32 calls later the words hold every value again
+                        if ((e = cudaMemsetAsync(k->flags, 0, k->flag_words * 4, s)) != cudaSuccess) return e;
+                        k->epoch = 1;
+                    }
+                    flags = k->flags;
+                    epoch = k->epoch;
+                }
+                if (zero_words && zero_words <= KEPT_WORDS_MAX) {
+                    if ((e = grow(c->shared->pool, k->zeros, k->zero_words, zero_words, 4096, true, s)) != cudaSuccess) return e;
+                    zeros = k->zeros;
+                }
+                if (bytes && bytes <= KEPT_SCRATCH_MAX) {
+                    if ((e = grow(c->shared->pool, k->scratch, k->scratch_bytes, bytes, (size_t)1 << 20, false, s)) != cudaSuccess) return e;
+                    ptr = k->scratch;
+                }
+            }
+        }
+        if (bytes && !ptr) {
+            if ((e = cudaMallocFromPoolAsync(&pooled[0], bytes, c->shared->pool, s)) != cudaSuccess) return e;
+            ptr = pooled[0];
+        }
+        if (zero_words && !zeros) {
+            if ((e = cudaMallocFromPoolAsync(&pooled[1], zero_words * 4, c->shared->pool, s)) != cudaSuccess) { give_back(); return e; }
+            if ((e = cudaMemsetAsync(pooled[1], 0, zero_words * 4, s)) != cudaSuccess) { give_back(); return e; }
+            zeros = static_cast<uint32_t*>(pooled[1]);
+        }
+        return cudaSuccess;
+    }
+    cudaError_t give_back() {
+        cudaError_t r = cudaSuccess;
+        for (void*& p : pooled)
+            if (p) {
+                const cudaError_t e = cudaFreeAsync(p, stream);
+                if (e != cudaSuccess) r = e;
+                p = nullptr;
+            }
+        return r;
+    }
+};
+
 fa_status_t run(fa_ctx_t* c, const char* who, const fa_sm100::LaunchArgs& a) {
     int cur = -1;
     cudaError_t e = cudaGetDevice(&cur);
@@ -60,15 +214,17 @@ fa_status_t run(fa_ctx_t* c, const char* who, const fa_sm100::LaunchArgs& a) {
         return FA_ERR_INVALID_ARG;
     }
     fa_sm100::LaunchArgs b = a;
-    void* ws = nullptr;
-    e = cudaMallocFromPoolAsync(&ws, fa_sm100::workspace_bytes(a.bh, a.sl, a.hd), c->pool, a.stream);
+    Scratch ws;
+    e = ws.take(c, a.stream, fa_sm100::workspace_bytes(a.bh, a.sl, a.hd), fa_sm100::v_flag_count(a.bh, a.sl), 0);
     if (e != cudaSuccess) {
         set_err(c, "%s: workspace allocation: %s", who, cudaGetErrorString(e));
         return e == cudaErrorMemoryAllocation ? FA_ERR_OOM : FA_ERR_CUDA;
     }
-    b.v16_workspace = ws;
+    b.v16_workspace = ws.ptr;
+    b.v_flags = ws.flags;
+    b.v_epoch = ws.epoch;
     e = fa_sm100::launch(b);
-    const cudaError_t fe = cudaFreeAsync(ws, a.stream);  // stream-ordered: released after the kernel
+    const cudaError_t fe = ws.give_back();  // stream-ordered: released after the kernel
     if (e != cudaSuccess) { set_err(c, "%s: launch: %s", who, cudaGetErrorString(e)); return FA_ERR_CUDA; }
     if (fe != cudaSuccess) { set_err(c, "%s: workspace release: %s", who, cudaGetErrorString(fe)); return FA_ERR_CUDA; }
     return FA_OK;
@@ -93,22 +249,15 @@ fa_status_t fa_create(fa_ctx_t** ctx_out) {
         return FA_ERR_CUDA;
     }
     c->arch_ok = (c->cc_major == 10);
-    c->has_pool = false;
+    c->shared = nullptr;
     if (c->arch_ok) {
-        cudaMemPoolProps props = {};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.handleTypes = cudaMemHandleTypeNone;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        cudaError_t pe = cudaMemPoolCreate(&c->pool, &props);
+        const cudaError_t pe = dev < MAX_DEVICES ? g_scratch[dev].acquire(dev) : cudaErrorInvalidDevice;
         if (pe != cudaSuccess) {
             snprintf(c->last_err, sizeof(c->last_err), "fa_create: cudaMemPoolCreate: %s", cudaGetErrorString(pe));
             *ctx_out = c;
             return FA_ERR_CUDA;
         }
-        unsigned long long keep = ~0ull;  // keep freed scratch cached in the pool
-        cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        c->has_pool = true;
+        c->shared = &g_scratch[dev];
     }
     *ctx_out = c;  // returned even on an unsupported GPU so the caller can read the reason
     if (!c->arch_ok) {
@@ -120,7 +269,7 @@ fa_status_t fa_create(fa_ctx_t** ctx_out) {
 }
 
 fa_status_t fa_destroy(fa_ctx_t* ctx) {
-    if (ctx && ctx->has_pool) cudaMemPoolDestroy(ctx->pool);  // pending frees complete first (stream-ordered)
+    if (ctx && ctx->shared) ctx->shared->release(ctx->device);
     delete ctx;
     return FA_OK;
 }
@@ -188,7 +337,7 @@ fa_status_t fa_decode(fa_ctx_t* ctx, const fa_decode_args_t* g) {
     const char* who = "fa_decode";
     if (!ctx) return FA_ERR_INVALID_ARG;
     if (!g) { set_err(ctx, "%s: null argument block", who); return FA_ERR_INVALID_ARG; }
-    if (!ctx->arch_ok || !ctx->has_pool) { set_err(ctx, "%s: context was created on an unsupported GPU", who); return FA_ERR_UNSUPPORTED_ARCH; }
+    if (!ctx->arch_ok || !ctx->shared) { set_err(ctx, "%s: context was created on an unsupported GPU", who); return FA_ERR_UNSUPPORTED_ARCH; }
     if (!g->q || !g->k_cache || !g->v_cache || !g->o) { set_err(ctx, "%s: null pointer in q/k_cache/v_cache/o", who); return FA_ERR_INVALID_ARG; }
     const bool paged = g->block_table != nullptr;
     if (paged && (g->page_size <= 0 || g->page_size % 64 != 0 || g->max_pages_per_seq <= 0 || g->num_pages <= 0 ||
@@ -221,15 +370,12 @@ fa_status_t fa_decode(fa_ctx_t* ctx, const fa_decode_args_t* g) {
     a.scale = g->scale; a.v_descale = (g->v_descale == 0.0f) ? 1.0f : g->v_descale;
     a.scale_q_dev = g->scale_q_dev; a.scale_k_dev = g->scale_k_dev; a.scale_v_dev = g->scale_v_dev;
     a.stream = reinterpret_cast<cudaStream_t>(g->stream);
-    const size_t ws_bytes = fa_sm100::decode_workspace_bytes(a.batch, a.kv_heads, a.hd, fa_sm100::decode_span(a));
-    void* ws = nullptr;
-    if (ws_bytes) {
-        e = cudaMallocFromPoolAsync(&ws, ws_bytes, ctx->pool, a.stream);
-        if (e != cudaSuccess) { set_err(ctx, "%s: workspace allocation: %s", who, cudaGetErrorString(e)); return e == cudaErrorMemoryAllocation ? FA_ERR_OOM : FA_ERR_CUDA; }
-    }
-    a.workspace = ws;
+    Scratch ws;
+    e = ws.take(ctx, a.stream, fa_sm100::decode_workspace_bytes(a.batch, a.kv_heads, a.hd, fa_sm100::decode_span(a)), 0, 0);
+    if (e != cudaSuccess) { set_err(ctx, "%s: workspace allocation: %s", who, cudaGetErrorString(e)); return e == cudaErrorMemoryAllocation ? FA_ERR_OOM : FA_ERR_CUDA; }
+    a.workspace = ws.ptr;
     e = fa_sm100::launch_decode(a);
-    const cudaError_t fe = ws ? cudaFreeAsync(ws, a.stream) : cudaSuccess;  // stream-ordered: released after the kernels
+    const cudaError_t fe = ws.give_back();  // stream-ordered: released after the kernels
     if (e != cudaSuccess) { set_err(ctx, "%s: launch: %s", who, cudaGetErrorString(e)); return FA_ERR_CUDA; }
     if (fe != cudaSuccess) { set_err(ctx, "%s: workspace release: %s", who, cudaGetErrorString(fe)); return FA_ERR_CUDA; }
     return FA_OK;

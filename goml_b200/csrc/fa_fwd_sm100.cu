@@ -39,6 +39,7 @@
 
 #include "../../include/fa_sm120.h"
 #include "fa_fwd_sm100.h"
+#include "pdl.cuh"
 #include "sm100_ptx.cuh"
 #include "tmap.cuh"
 
@@ -99,6 +100,9 @@ struct Params {
     const float* sv;
     __half* o;
     float* lse;
+    const uint32_t* v_flags;   // see LaunchArgs
+    uint32_t v_epoch;
+    int v_chunks;              // chunks per head
 };
 
 __device__ __forceinline__ float ex2(float x) {
@@ -135,20 +139,96 @@ __global__ void __launch_bounds__(32) fa_wait_expiry_selftest_kernel() {
     wait_expiry_selftest_body(&g_fa_status, ST_TIMEOUT_SELFTEST);
 }
 
-// V (e4m3) -> fp16, 16 codes per thread per step; exact.
-__global__ void __launch_bounds__(256) v_to_f16_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, size_t n16) {
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += stride) {
-        const uint4 c = __ldg(in + i);
-        const uint32_t w[4] = {c.x, c.y, c.z, c.w};
-        uint32_t h[8];
+// V (e4m3) -> fp16, exact.  One CTA step = one chunk of V_CHUNK keys of one head, taken in the order the attention tiles
+// ask for them; a finished chunk is published by its flag, so the attention kernel (launched behind this one without
+// waiting for it) starts on the first heads while later ones are still being converted.  HBM-bound (3 bytes moved per
+// element).
+constexpr int V_CHUNK = 128;
+constexpr int V_THREADS = 128;
+constexpr int V_CTAS_PER_SM = 10;   // with 2 the first attention tiles wait for it (S = 2048 causal: 366 us a call), 4 344, 6 340, 10 337
+__device__ __forceinline__ void e4m3x16_to_f16(const uint4 c, uint4& lo, uint4& hi) {
+    const uint32_t w[4] = {c.x, c.y, c.z, c.w};
+    uint32_t h[8];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h[2 * k]) : "h"((uint16_t)(w[k] & 0xffffu)));
-            asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h[2 * k + 1]) : "h"((uint16_t)(w[k] >> 16)));
+    for (int k = 0; k < 4; k++) {
+        asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h[2 * k]) : "h"((uint16_t)(w[k] & 0xffffu)));
+        asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h[2 * k + 1]) : "h"((uint16_t)(w[k] >> 16)));
+    }
+    lo = make_uint4(h[0], h[1], h[2], h[3]);
+    hi = make_uint4(h[4], h[5], h[6], h[7]);
+}
+template <int HD>
+__global__ void __launch_bounds__(V_THREADS, 12) v_to_f16_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, int chunks,
+                                                                int chunks_per_head, int sl, uint32_t* flags, uint32_t epoch) {
+    pdl_wait();      // V may come from the kernel ahead, and the attention of an earlier call may still read `out`
+    pdl_trigger();   // after the wait: the attention kernel reads Q and K without waiting for this kernel
+    constexpr int PER_KEY = HD / 16;                             // 16-byte pieces per key
+    constexpr int STEPS = V_CHUNK * PER_KEY / V_THREADS;         // pieces per thread and chunk: 8 (D = 128) or 4
+    constexpr int BATCH = 4;                                     // loads in flight per thread
+    for (int c = blockIdx.x; c < chunks; c += gridDim.x) {
+        const int head = c / chunks_per_head, k0 = (c - head * chunks_per_head) * V_CHUNK;
+        const int pieces = min(V_CHUNK, sl - k0) * PER_KEY;
+        const size_t base = ((size_t)head * sl + k0) * PER_KEY;
+#pragma unroll 1
+        for (int i0 = 0; i0 < STEPS; i0 += BATCH) {
+            uint4 v[BATCH];
+#pragma unroll
+            for (int i = 0; i < BATCH; i++) {
+                const int at = (i0 + i) * V_THREADS + threadIdx.x;
+                if (at < pieces) v[i] = __ldg(in + base + at);
+            }
+#pragma unroll
+            for (int i = 0; i < BATCH; i++) {
+                const int at = (i0 + i) * V_THREADS + threadIdx.x;
+                uint4 lo, hi;
+                e4m3x16_to_f16(v[i], lo, hi);
+                if (at < pieces) {
+                    out[2 * (base + at)] = lo;
+                    out[2 * (base + at) + 1] = hi;
+                }
+            }
         }
-        out[2 * i] = make_uint4(h[0], h[1], h[2], h[3]);
-        out[2 * i + 1] = make_uint4(h[4], h[5], h[6], h[7]);
+        if (flags) {
+            // the readers copy with TMA (async proxy): order these stores into that proxy before the flag is released
+            asm volatile("fence.proxy.async.global;" ::: "memory");
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                __threadfence();
+                asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flags + c), "r"(epoch) : "memory");
+            }
+        }
+    }
+}
+
+// Producer-side view of the pre-pass: how many leading chunks of this head (from chunk `c` on) are known to be ready.
+// The whole warp asks for 32 flags at a time, so a head of up to 4096 keys costs one load when it is complete.
+// Bounded like every wait of this file.
+__device__ __forceinline__ bool wait_v_chunk(const uint32_t* head_flags, int chunks_per_head, uint32_t epoch, int c, int& ready,
+                                             volatile uint32_t* abort_flag) {
+    if (c < ready) return true;
+    const int lane = threadIdx.x & 31;
+    uint64_t t0 = 0;
+    for (uint32_t polls = 1;; polls++) {
+        uint32_t f = epoch;
+        if (c + lane < chunks_per_head)
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(f) : "l"(head_flags + c + lane) : "memory");
+        const uint32_t missing = __ballot_sync(0xffffffffu, f != epoch);
+        const int n = missing ? __ffs(missing) - 1 : 32;
+        if (n > 0) {
+            ready = c + n;
+            asm volatile("fence.proxy.async.global;" ::: "memory");
+            return true;
+        }
+        if ((polls & 255u) == 0) {
+            uint32_t stop = *abort_flag;
+            const uint64_t now = globaltimer_ns();
+            if (t0 == 0) t0 = now;
+            else if (now - t0 > SM100_WAIT_BUDGET_NS) {
+                if (lane == 0) atomicCAS((uint32_t*)abort_flag, 0u, (uint32_t)ST_TIMEOUT_LOAD);
+                stop = 1;
+            }
+            if (__any_sync(0xffffffffu, stop != 0)) return false;
+        }
     }
 }
 
@@ -244,6 +324,10 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
                 mbar_arrive_expect_tx(bar_q, C::Q_BYTES);
                 tma_load_3d(sbase + C::OFF_Q, &tmap_q, bar_q, 0, q0, head);
             }
+            // Q and K are complete when this kernel starts (the pre-pass triggered it after its own wait); the fp16 copy
+            // of V is waited for chunk by chunk, or as a whole when the launch has no flags
+            int v_ready = 0;
+            const uint32_t* head_flags = p.v_flags ? p.v_flags + (size_t)head * p.v_chunks : nullptr;
             int s = 0;
             uint32_t ph = 1;  // "previous phase complete": the rings start empty
             for (int j = 0; j < nblk; j++) {
@@ -254,6 +338,11 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
                     tma_load_3d(sbase + C::OFF_K + s * C::K_BYTES, &tmap_k, bar_kfull + 8 * s, 0, key0, head);
                 }
                 if (!mbar_wait(bar_pvdone + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD)) break;  // P V three blocks back is done
+                if (!head_flags) {
+                    if (j == 0) pdl_wait();
+                } else if (!wait_v_chunk(head_flags, p.v_chunks, p.v_epoch, key0 / V_CHUNK, v_ready, abort_flag)) {
+                    break;
+                }
                 if (leader) {
                     mbar_arrive_expect_tx(bar_vfull + 8 * s, C::V_BYTES);
 #pragma unroll
@@ -264,6 +353,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
                 __syncwarp();
                 if (++s == STAGES) { s = 0; ph ^= 1; }
             }
+            pdl_wait();   // this kernel completes after the pre-pass
         }
     } else if (warp == MMA_WARP) {
         // -------------------------------------------------------------- MMA issuer
@@ -495,6 +585,9 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     __syncwarp();
     tc_fence_before();
     __syncthreads();
+    // Triggered at the end of a CTA, not at its start: the next call's pre-pass is spread over the SMs that have room when
+    // it is launched, and during this kernel's last wave those are few (S = 2048 causal: 525 us a call against 343).
+    pdl_trigger();
     const uint32_t code = *abort_flag;
     if (code != 0) {
         if (threadIdx.x == 0) atomicCAS(&g_fa_status, 0u, code);
@@ -519,16 +612,9 @@ void init_device(DeviceState* st, int dev);
 template <int HD>
 cudaError_t launch_hd(const LaunchArgs& a, int num_sms) {
     using C = Cfg<HD>;
-    const size_t n = (size_t)a.bh * a.sl * HD;
-    // pre-pass: V codes -> fp16 workspace
-    {
-        const size_t n16 = n / 16;  // HD is a multiple of 16
-        size_t blocks = (n16 + 255) / 256;
-        const size_t cap = (size_t)num_sms * 8;
-        if (blocks > cap) blocks = cap;
-        v_to_f16_kernel<<<(unsigned)blocks, 256, 0, a.stream>>>(reinterpret_cast<const uint4*>(a.v),
-                                                               reinterpret_cast<uint4*>(a.v16_workspace), n16);
-    }
+    const long long grid = (long long)a.bh * ((a.sl + BM - 1) / BM);
+    const int v_chunks = (a.sl + V_CHUNK - 1) / V_CHUNK;
+    if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
     CUtensorMap tq, tk, tv;
     const CUtensorMapSwizzle swz = (HD == 128) ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
     if (!make_tmap_u8_3d(&tq, a.q, a.bh, a.sl, HD, BM, HD, swz) ||
@@ -543,12 +629,16 @@ cudaError_t launch_hd(const LaunchArgs& a, int num_sms) {
     p.sq = a.scale_q_dev; p.sk = a.scale_k_dev; p.sv = a.scale_v_dev;
     p.o = reinterpret_cast<__half*>(a.o);
     p.lse = a.lse;
-    const long long grid = (long long)a.bh * p.n_qtiles;
-    if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
+    p.v_flags = a.v_flags; p.v_epoch = a.v_epoch; p.v_chunks = v_chunks;
+    // pre-pass: V codes -> fp16 workspace
+    const long long chunks = (long long)a.bh * v_chunks, cap = (long long)num_sms * V_CTAS_PER_SM;
+    const cudaError_t e = launch_pdl(v_to_f16_kernel<HD>, (unsigned)(chunks < cap ? chunks : cap), V_THREADS, 0, a.stream,
+                                     reinterpret_cast<const uint4*>(a.v), reinterpret_cast<uint4*>(a.v16_workspace), (int)chunks, v_chunks,
+                                     a.sl, a.v_flags, a.v_epoch);
+    if (e != cudaSuccess) return e;
     const bool masked = a.causal || a.window > 0 || (a.sl % BN) != 0 || !(a.scale > 0.f);
-    if (masked) fa_fwd_kernel<HD, true><<<(unsigned)grid, NUM_THREADS, C::SMEM_BYTES, a.stream>>>(tq, tk, tv, p);
-    else fa_fwd_kernel<HD, false><<<(unsigned)grid, NUM_THREADS, C::SMEM_BYTES, a.stream>>>(tq, tk, tv, p);
-    return cudaGetLastError();
+    return masked ? launch_pdl(fa_fwd_kernel<HD, true>, (unsigned)grid, NUM_THREADS, C::SMEM_BYTES, a.stream, tq, tk, tv, p)
+                  : launch_pdl(fa_fwd_kernel<HD, false>, (unsigned)grid, NUM_THREADS, C::SMEM_BYTES, a.stream, tq, tk, tv, p);
 }
 
 }  // namespace
@@ -565,6 +655,7 @@ void init_device(DeviceState* st, int dev) {
 }  // namespace
 
 size_t workspace_bytes(int bh, int sl, int hd) { return (size_t)bh * sl * hd * 2; }
+size_t v_flag_count(int bh, int sl) { return (size_t)bh * ((sl + V_CHUNK - 1) / V_CHUNK); }
 
 cudaError_t launch(const LaunchArgs& a) {
     int dev = 0;

@@ -21,10 +21,16 @@ struct LaunchArgs {
     const float* scale_k_dev = nullptr;
     const float* scale_v_dev = nullptr;
     cudaStream_t stream;
+    // v_flag_count(bh, sl) words, or nullptr: one flag per 128-key chunk of a head, set to v_epoch when the pre-pass has
+    // written that chunk's fp16 copy.  With flags the attention kernel starts beside the pre-pass and waits per chunk;
+    // without them it waits for the whole pre-pass.  The epoch must differ from every value the words hold.
+    uint32_t* v_flags = nullptr;
+    uint32_t v_epoch = 0;
 };
 
 // Scratch the forward needs (an fp16 copy of V made by a pre-pass on the same stream).
 size_t workspace_bytes(int bh, int sl, int hd);
+size_t v_flag_count(int bh, int sl);
 
 // Launches on the calling thread's current device; asynchronous on a.stream.
 cudaError_t launch(const LaunchArgs& a);

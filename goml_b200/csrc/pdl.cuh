@@ -1,0 +1,39 @@
+// pdl.cuh — programmatic dependent launch: a kernel of this directory is launched before its predecessor on the stream
+// has drained, runs its set-up (barriers, tensor memory, descriptor prefetch, cache hints) and waits on the device for
+// the predecessor's completion before it touches dependent data.
+//
+// Three rules keep the stream's order intact:
+//  * pdl_wait() comes before the first read of anything an earlier kernel may have written and before the first write to
+//    global memory, in every kernel, on every path that touches global memory; a kernel does not complete before every
+//    kernel ahead of it has, because some thread of each of its CTAs waits before the CTA ends;
+//  * a kernel whose successor reads before its own wait (the attention forward, behind its V pre-pass) calls
+//    pdl_trigger() only after pdl_wait(): everything ahead of the pair has then completed;
+//  * what any kernel may do before its wait is to ask for lines of an operand to be brought into L2: a hint moves no
+//    data into the SM, and L2 is where stores of the kernel ahead land, so it cannot be stale.
+// Both instructions do nothing in a launch without the attribute.
+//
+// What it buys: the gap between two dependent kernels of a few microseconds each falls from 1.5-2.5 us to under 1 us.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace sm100 {
+
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+}  // namespace sm100

@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 import threading
 
 from . import loader
@@ -69,9 +70,17 @@ class DecodeArgs(C.Structure):
     ]
 
 
+# The two argument blocks as packed bytes: one struct.pack (native alignment) and a bytes argument cost 1 us of host time
+# a call, filling a ctypes structure field by field and passing a reference to it about 4.
+_PACK_FORWARD = struct.Struct("@5P5i2f4P").pack
+_PACK_DECODE = struct.Struct("@6P6i2f5P3i0P").pack
+assert struct.calcsize("@5P5i2f4P") == C.sizeof(ForwardArgs) and struct.calcsize("@6P6i2f5P3i0P") == C.sizeof(DecodeArgs)
+
 _lock = threading.Lock()
 _lib = None
 _lib_err = None
+_forward_ex = None   # fa_forward_ex / fa_decode taking the packed block, set by FALoad
+_decode = None
 
 
 def _candidates():
@@ -86,7 +95,9 @@ def _candidates():
 
 def FALoad():
     """One-time dlopen of libfa_sm120.so and symbol registration."""
-    global _lib, _lib_err
+    global _lib, _lib_err, _forward_ex, _decode
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is None and _lib_err is None:
             last = None
@@ -128,6 +139,11 @@ def FALoad():
                 lib.fa_noalloc_device_status.argtypes = []
                 lib.fa_selftest_wait_expiry.restype = i
                 lib.fa_selftest_wait_expiry.argtypes = [p, p]
+                forward_ex, decode = lib["fa_forward_ex"], lib["fa_decode"]
+                for fn in (forward_ex, decode):
+                    fn.restype = i
+                    fn.argtypes = [p, C.c_char_p]
+                _forward_ex, _decode = forward_ex, decode
                 _lib = lib
                 break
             if _lib is None:
@@ -190,9 +206,8 @@ class FAContext:
                   scale_q_dev=0, scale_k_dev=0, scale_v_dev=0, stream=0) -> None:
         if not self.ptr:
             raise FAError("FAContext.ForwardEx: nil ctx", FA_ERR_INVALID_ARG)
-        a = ForwardArgs(q, k, v, o, lOut or None, bh, sl, hd, causal, window, scale, v_descale,
-                        scale_q_dev or None, scale_k_dev or None, scale_v_dev or None, stream or None)
-        st = FALoad().fa_forward_ex(self.ptr, C.byref(a))
+        st = _forward_ex(self.ptr, _PACK_FORWARD(q or 0, k or 0, v or 0, o or 0, lOut or 0, bh, sl, hd, causal, window, scale, v_descale,
+                                                 scale_q_dev or 0, scale_k_dev or 0, scale_v_dev or 0, stream or 0))
         if st != FA_OK:
             raise FAError("fa_forward_ex", st, self._msg())
 
@@ -205,10 +220,9 @@ class FAContext:
         hd] and s_max is ignored."""
         if not self.ptr:
             raise FAError("FAContext.Decode: nil ctx", FA_ERR_INVALID_ARG)
-        a = DecodeArgs(q, k_cache, v_cache, o, lOut or None, seq_lens or None, batch, q_heads, kv_heads, hd, s_max, seq_len,
-                       scale, v_descale, scale_q_dev or None, scale_k_dev or None, scale_v_dev or None, stream or None,
-                       block_table or None, page_size, max_pages_per_seq, num_pages)
-        st = FALoad().fa_decode(self.ptr, C.byref(a))
+        st = _decode(self.ptr, _PACK_DECODE(q or 0, k_cache or 0, v_cache or 0, o or 0, lOut or 0, seq_lens or 0, batch, q_heads, kv_heads, hd,
+                                            s_max, seq_len, scale, v_descale, scale_q_dev or 0, scale_k_dev or 0, scale_v_dev or 0, stream or 0,
+                                            block_table or 0, page_size, max_pages_per_seq, num_pages))
         if st != FA_OK:
             raise FAError("fa_decode", st, self._msg())
 
