@@ -371,9 +371,14 @@ fa_status_t fa_decode(fa_ctx_t* ctx, const fa_decode_args_t* g) {
     a.scale_q_dev = g->scale_q_dev; a.scale_k_dev = g->scale_k_dev; a.scale_v_dev = g->scale_v_dev;
     a.stream = reinterpret_cast<cudaStream_t>(g->stream);
     Scratch ws;
-    e = ws.take(ctx, a.stream, fa_sm100::decode_workspace_bytes(a.batch, a.kv_heads, a.hd, fa_sm100::decode_span(a)), 0, 0);
+    const int span = fa_sm100::decode_span(a);
+    e = ws.take(ctx, a.stream, fa_sm100::decode_workspace_bytes(a.batch, a.q_heads, a.kv_heads, a.hd, span),
+                fa_sm100::decode_flag_count(a.batch, a.q_heads, a.kv_heads, span), (size_t)a.batch * a.kv_heads);
     if (e != cudaSuccess) { set_err(ctx, "%s: workspace allocation: %s", who, cudaGetErrorString(e)); return e == cudaErrorMemoryAllocation ? FA_ERR_OOM : FA_ERR_CUDA; }
     a.workspace = ws.ptr;
+    a.arrivals = ws.zeros;
+    a.flags = ws.flags;
+    a.epoch = ws.epoch;
     e = fa_sm100::launch_decode(a);
     const cudaError_t fe = ws.give_back();  // stream-ordered: released after the kernels
     if (e != cudaSuccess) { set_err(ctx, "%s: launch: %s", who, cudaGetErrorString(e)); return FA_ERR_CUDA; }

@@ -7,56 +7,69 @@
 //   o        [B, Hq, D]          fp16,  lse [B, Hq] fp32 (natural log, optional)
 //   seq_lens [B] int32 on the device (keys [0, seq_lens[b]) of sequence b are visible), or one length for all
 //
-// The step reads every cached key and value once and does 4*Hq*D FLOP per key: HBM-bound, so this is a
-// streaming kernel, not a tcgen05 one.  One CTA (4 warps) per (sequence, kv head, split of the key range); the
-// G = Hq/Hkv (<= 16) query heads that share a kv head form the 16 rows of the warp-level MMAs:
-//   S = Q K^T   mma.sync m16n8k32 e4m3 x e4m3 -> fp32, K fragments straight from a padded shared-memory copy
-//   P V         mma.sync m16n8k16 fp16 x fp16 -> fp32, P kept in fp16 (an e4m3 P costs 2.5e-2 relative error),
-//               V converted to fp16 on its way into shared memory and read with ldmatrix.trans
-// Each warp owns 16 of the 64 keys of a chunk and carries its own online-softmax state (m, l, O) over all chunks,
-// loading and converting its own keys, so the loop needs only warp-level synchronisation; the four states are merged
-// once at the end.  K and V chunks arrive through a 2-stage cp.async ring (one chunk = 16 KB in flight per CTA,
-// four CTAs = 16 warps per SM: the loop is bound by instruction issue and dependency stalls, which more warps hide
-// better than a deeper ring).  With more than one
-// split the partial states go to a workspace and a second kernel merges them.
+// The step reads every cached key and value once and does 4*Hq*D FLOP per key: HBM-bound, so this is a streaming
+// kernel on the warp-level tensor path, built to need as few instructions per cached byte as possible:
+//
+//  * K and V go from global memory straight into MMA fragments, with no shared memory in between.  Contraction and row
+//    indices of an MMA may be permuted as long as both operands agree, so every lane's share of a key row is contiguous
+//    (D/4 bytes of K, D/8 bytes of V) and a warp's loads cover whole rows.
+//  * S^T = K Q^T (m16n8k32, e4m3): 16 keys are the rows, up to 8 query heads of the kv head the columns (two column tiles
+//    for groups of 9 to 16); O^T += V^T P^T (m16n8k16, fp16): V bytes of two keys are paired with a byte permute and
+//    converted in registers, P (kept in fp16: an e4m3 P costs 2.5e-2 relative error) is transposed by movmatrix.
+//  * Each warp carries its own online-softmax state over the 16-key tiles it takes.  Whether a running maximum moves is
+//    one vote per tile; row sums stay in the lanes until the end: the loop has no shuffles.
+//  * A warp's next K block is on its way while it works on this block's softmax and V, and the next V block during the
+//    next block's scores (Little's law asks for about 45 KB in flight per SM).
+//
+// How the keys are divided (Plan below): a pair (sequence, kv head) may be cut between chunks; the pieces leave partial
+// states in a workspace and the CTA that finishes last merges them in a fixed order, so results do not depend on timing
+// and there is no second kernel.
+//
+// STREAMS: the rounding of P to fp16 depends on the running maximum it is taken against, so which keys share a warp and
+// where a pair is cut show in the last bits of O.  A block that re-quantises its activations turns last bits into e4m3
+// steps further on.  For one query head per kv head (what the decoder block runs) warp w therefore always takes keys
+// 16w .. 16w + 15 of every 64-key chunk, and the plans keep each such stream's maximum what an uncut walk over the pair
+// (or over a fixed split of it) gives.  Grouped heads are free of that: the maximum may lag by 2^LAG, a warp takes 32
+// (D = 64: 64) contiguous keys, pairs are cut anywhere.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
 
 #include "fa_fwd_sm100.h"
+#include "pdl.cuh"
 
 namespace fa_sm100 {
 
 namespace {
 
-constexpr int CHUNK = 64;     // keys per step of a CTA
-constexpr int THREADS = 128;  // 4 warps x 16 keys
-constexpr int ROWS = 16;      // MMA rows = query heads of one kv head (padded)
-#ifndef FA_DECODE_STAGES
-#define FA_DECODE_STAGES 2
-#endif
-#ifndef FA_DECODE_CTAS
-#define FA_DECODE_CTAS 4
-#endif
-constexpr int STAGES = FA_DECODE_STAGES;     // cp.async ring depth (chunks)
-constexpr int CTAS_PER_SM = FA_DECODE_CTAS;  // resident CTAs the register budget is set for
+using namespace sm100;
 
-// D = A B with a zero accumulator input (no registers to clear first)
-__device__ __forceinline__ void mma_e4m3_m16n8k32_zero(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
+constexpr int CHUNK = 64;        // keys per unit of work (page sizes are multiples of it)
+constexpr int THREADS = 128;
+constexpr int WARPS = THREADS / 32;
+constexpr float LAG = 6.0f;      // log2 units
+// A wide warp step takes twice the keys of a narrow one (8 against 4 KB in flight per warp) and leaves registers for 12
+// warps per SM instead of 16 (8 with two column tiles).  It streams faster (0.8 GB of cache: 137 us against 146); the
+// narrow one lets more CTAs be resident.
+constexpr int ctas_per_sm(int nq, bool wide) { return nq == 2 ? 2 : wide ? 3 : 4; }
+
+// D = A B with a zero accumulator input
+__device__ __forceinline__ void mma_e4m3_m16n8k32_zero(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k32.row.col.f32.e4m3.e4m3.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 __device__ __forceinline__ void mma_f16_m16n8k16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, uint32_t saddr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(saddr));
+__device__ __forceinline__ uint32_t transpose_8x8_b16(uint32_t x) {
+    uint32_t y;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+    return y;
 }
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ float ex2f(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -66,6 +79,30 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
     const __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&h);
 }
+// two e4m3 pairs (the halves of w) -> two fp16 pairs
+__device__ __forceinline__ void e4m3x4_to_h2x2(uint32_t w, uint32_t& lo, uint32_t& hi) {
+    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, l;\n\tcvt.rn.f16x2.e4m3x2 %1, h;\n\t}" : "=r"(lo), "=r"(hi) : "r"(w));
+}
+// read once: not kept in L1 (with the default policy the D = 128 kernel is 9 % slower; one 256-bit load in place of two of
+// these costs 3 %)
+__device__ __forceinline__ void ldg128(uint32_t* r, const uint8_t* p) {
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "l"(p));
+}
+__device__ __forceinline__ void ldg64(uint32_t* r, const uint8_t* p) {
+    asm volatile("ld.global.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "l"(p));
+}
+
+// Plans.
+//  SPLITS: CTA i is split i % splits of pair i / splits; a split is chunks_per_split chunks.  Few pairs: one resident CTA
+//          per split.
+//  LINE:   the chunks of all pairs form one line that is cut into equal pieces, one per resident CTA, so sequences of very
+//          different lengths load all SMs alike.
+//  LINE_HANDED: the same with pieces at least as long as the longest pair, so that a pair is cut at most once.  A CTA
+//          takes the pair that its piece ends in first, publishes the running maxima it ended with, and takes the pair its
+//          piece begins in last, starting from the maxima of the CTA before it.  Those were published about a piece ago;
+//          the wait for them is bounded and gives up to a start from scratch, which changes only roundings.
+enum Plan : int { SPLITS, LINE, LINE_HANDED };
+
 struct DecodeParams {
     const uint8_t* q;
     const uint8_t* k;
@@ -78,367 +115,618 @@ struct DecodeParams {
     const float* sq;
     const float* sk;
     const float* sv;
-    int splits, chunks_per_split;
-    // paged cache: k, v are [num_pages, Hkv, page_size, D]; logical chunk c of sequence b lives in page
-    // block_table[b * max_pages + c / chunks_per_page]
+    int plan, splits, chunks_per_split;
+    // paged cache: k, v are [num_pages, Hkv, page_size, D]; the chunk at key k0 of sequence b lives in page
+    // block_table[b * max_pages + k0 / page_size]
     const int* block_table;
-    int page_size, max_pages, num_pages, chunks_per_page;
-    float* ws_o;   // [B*Hkv, splits, ROWS, D] un-normalised partial outputs
-    float* ws_ml;  // [B*Hkv, splits, ROWS, 2] (m in log2 units, l)
+    int page_size, max_pages, num_pages;
+    uint32_t page_mul, page_shr;   // key / page_size as multiply-high and shift
+    // partial states, two slots per CTA: [slot][rows][D] un-normalised outputs, then [slot][rows][2] (m in log2 units, l)
+    float* ws_o;
+    float* ws_ml;
+    float* ws_handed;     // [CTA][WARPS][rows] running maxima
+    uint32_t* arrivals;   // [B*Hkv], zero before and after every launch
+    uint32_t* handed;     // [CTA], set to epoch when the CTA's maxima are published; nullptr: nothing is handed on
+    uint32_t epoch;
 };
 
+template <int D, int NQ, bool WIDE>
+struct Cfg {
+    static constexpr int TILES = (D == 128 ? 1 : 2) * (WIDE ? 2 : 1);   // 16-key tiles per warp step = chunks per CTA step
+    static constexpr int KSTEPS = D / 32;
+    static constexpr int KW = D / 16;                    // 32-bit words of a lane's share of one K row
+    static constexpr int MT = D / 16;                    // 16-row tiles of O^T
+    static constexpr int VW = D / 32;                    // 32-bit words of a lane's share of one V row
+    static constexpr int ROWS = 8 * NQ;                  // query columns
+    static constexpr int PITCH = D + 4;                  // floats per row of the merge buffer
+};
+
+__device__ __forceinline__ int seq_len_of(const DecodeParams& p, int b) { return p.seq_lens ? min(max(__ldcg(p.seq_lens + b), 0), p.s_max) : p.seq_len; }
+__device__ __forceinline__ int chunks_of(int len) { return (len + CHUNK - 1) / CHUNK; }
+
+// [begin, end) of piece i of equal pieces of a line (the first `remainder` pieces are one unit longer), and back
+struct Cut {
+    int q, r;
+    __device__ __forceinline__ Cut(int quotient, int remainder) : q(quotient), r(remainder) {}
+    __device__ __forceinline__ int begin(int i) const { return i * q + min(i, r); }
+    __device__ __forceinline__ int piece_of(int u) const { return u < r * (q + 1) ? u / (q + 1) : r + (u - r * (q + 1)) / q; }
+};
+
+__device__ __forceinline__ void fold(float& L, float4& O, float l, const float4& o, float f) {
+    L += l * f;
+    O.x += o.x * f; O.y += o.y * f; O.z += o.z * f; O.w += o.w * f;
+}
 template <int D>
-struct Smem {
-    static constexpr int K_STRIDE = D + 16;          // bytes per key row of the e4m3 K copy (16 spreads rows over banks)
-    static constexpr int V_STRIDE = 2 * D + 16;      // bytes per key row of the fp16 V copy
-    static constexpr int K_BYTES = CHUNK * K_STRIDE;      // one ring stage of K
-    static constexpr int VRAW_BYTES = CHUNK * D;          // one ring stage of V codes (dense)
-    static constexpr int V_BYTES = CHUNK * V_STRIDE;      // the fp16 copy of the chunk being computed
-    static constexpr int OFF_VRAW = STAGES * K_BYTES;
-    static constexpr int OFF_V = OFF_VRAW + STAGES * VRAW_BYTES;
-    static constexpr int MERGE_BYTES = 4 * ROWS * (D + 2) * 4;   // four warps' (O, m, l) for the final merge
-    static constexpr int BYTES = (OFF_V + V_BYTES) > MERGE_BYTES ? (OFF_V + V_BYTES) : MERGE_BYTES;
+__device__ __forceinline__ void store_out(const DecodeParams& p, size_t row, int col, float M, float L, const float4& O, float vds) {
+    const float inv = L > 0.f ? vds / L : 0.f;
+    if ((reinterpret_cast<uintptr_t>(p.o) & 7) == 0) {   // o need only be 2-byte aligned
+        *reinterpret_cast<uint2*>(p.o + row * D + col) = make_uint2(pack_h2(O.x * inv, O.y * inv), pack_h2(O.z * inv, O.w * inv));
+    } else {
+        __half* h = p.o + row * D + col;
+        h[0] = __float2half_rn(O.x * inv); h[1] = __float2half_rn(O.y * inv);
+        h[2] = __float2half_rn(O.z * inv); h[3] = __float2half_rn(O.w * inv);
+    }
+    if (col == 0 && p.lse) p.lse[row] = (L > 0.f) ? (M + log2f(L)) * 0.6931471805599453f : -INFINITY;
+}
+
+struct Segment {
+    int b, kvh, len;                // sequence, kv head, keys of the sequence
+    int n_chunks, c_begin, c_end;   // chunks of the pair, and those of them this CTA takes
+    int pair_u0;                    // unit of the line where the pair starts
 };
 
-template <int D, bool PAGED>
-__global__ void __launch_bounds__(THREADS, CTAS_PER_SM) fa_decode_kernel(const DecodeParams p) {
-    using S = Smem<D>;
-    extern __shared__ __align__(16) uint8_t smem[];
-    uint8_t* Vs = smem + S::OFF_V;
+template <int D, int NQ, bool WIDE, bool STREAMS, bool PAGED>
+__global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kernel(const DecodeParams p) {
+    using C = Cfg<D, NQ, WIDE>;
+    __shared__ float s_o[WARPS][C::ROWS][C::PITCH];
+    __shared__ float s_m[WARPS][C::ROWS], s_l[WARPS][C::ROWS];
+    __shared__ Segment s_next[WARPS];
+    __shared__ uint32_t s_last;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;              // MMA fragment coordinates
-    const int bh = blockIdx.x;                          // sequence * Hkv + kv head
-    const int b = bh / p.hkv, kvh = bh % p.hkv;
-    const int split = blockIdx.y;
-    const int seq_len = p.seq_lens ? min(max(p.seq_lens[b], 0), p.s_max) : p.seq_len;
-    const int n_chunks = (seq_len + CHUNK - 1) / CHUNK;
-    const int c_begin = split * p.chunks_per_split;
-    const int c_end = min(n_chunks, c_begin + p.chunks_per_split);
+    pdl_wait();
+    pdl_trigger();
 
     float scale_log2 = p.scale_log2;
     if (p.sq) scale_log2 *= __ldg(p.sq);
     if (p.sk) scale_log2 *= __ldg(p.sk);
 
-    // Q fragments (A operand, 16 x D): rows g and g + 8 are query heads kvh*group + row of sequence b.
-    // The contraction order over d is free, so the MMA's k index is fed a permutation of d that makes every lane's
-    // share of a key row contiguous: lane t supplies d = (D/4)*t + 8*ks + {0..3} as k = 4t + {0..3} and
-    // d = (D/4)*t + 8*ks + 4 + {0..3} as k = 16 + 4t + {0..3} of k-step ks, for Q (here) and K (below) alike; its K
-    // fragments of all k-steps are then D/4 contiguous bytes (two 128-bit shared loads for D = 128).
-    constexpr int KSTEPS = D / 32;
-    uint32_t qa[KSTEPS][4];
-    {
-        const uint8_t* qb = p.q + ((size_t)b * p.hq + (size_t)kvh * p.group) * D;
+    // a sequence with no visible key is on nobody's piece: O = 0, LSE = -inf
+    auto empty_sequence = [&](int b) {
+        for (int i = 0; i < p.hq * D; i++) p.o[(size_t)b * p.hq * D + i] = __float2half_rn(0.f);
+        if (p.lse)
+            for (int i = 0; i < p.hq; i++) p.lse[(size_t)b * p.hq + i] = -INFINITY;
+    };
+
+    // ---- this CTA's piece of the line.  Every warp adds the lengths up for itself (no barrier); lane i keeps those of
+    // sequences i, i + 32, .. of the first 32 * LENS, larger batches read theirs again where they need them.
+    constexpr int LENS = 4;
+    int lens[LENS];
 #pragma unroll
-        for (int ks = 0; ks < KSTEPS; ks++) {
+    for (int i = 0; i < LENS; i++) lens[i] = p.plan != SPLITS && 32 * i + lane < p.batch ? seq_len_of(p, 32 * i + lane) : 0;
+    auto lane_len = [&](int b0) -> int {   // length of sequence b0 + lane, b0 a multiple of 32
+        if (b0 < 32 * LENS) {
+            int x = lens[0];
+#pragma unroll
+            for (int i = 1; i < LENS; i++)
+                if (b0 == 32 * i) x = lens[i];
+            return x;
+        }
+        return b0 + lane < p.batch ? seq_len_of(p, b0 + lane) : 0;
+    };
+    auto len_of = [&](int b) -> int { return b < 32 * LENS ? __shfl_sync(0xffffffffu, lane_len(b & ~31), b & 31) : seq_len_of(p, b); };
+    // the part of one pair that starts at unit u and ends at unit end or with the pair
+    auto segment_at = [&](int u, int end) {
+        Segment x;
+        int seq_u0 = 0;
+        x.b = 0;
+        for (int b0 = 0, before = 0; b0 < p.batch; b0 += 32) {
+            const int n = chunks_of(lane_len(b0)) * p.hkv;
+            int incl = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            const uint32_t past = __ballot_sync(0xffffffffu, before + incl > u);   // first lane whose sequence ends past u
+            if (past) {
+                const int at = __ffs(past) - 1;
+                x.b = b0 + at;
+                seq_u0 = before + __shfl_sync(0xffffffffu, incl - n, at);
+                break;
+            }
+            before += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        x.len = len_of(x.b);
+        x.n_chunks = chunks_of(x.len);
+        x.kvh = (u - seq_u0) / x.n_chunks;
+        x.pair_u0 = seq_u0 + x.kvh * x.n_chunks;
+        x.c_begin = u - x.pair_u0;
+        x.c_end = min(x.n_chunks, x.c_begin + (end - u));
+        return x;
+    };
+
+    Segment seg;
+    int u_begin = 0, u_end = 0, cut_q = 0, cut_r = 0;
+    int mid = 0, mid_end = 0;    // units of the segments still to come in line order
+    bool head_last = false;      // the cut pair this piece begins in is still to come, behind them
+    if (p.plan == SPLITS) {
+        const int pair = blockIdx.x / p.splits, split = blockIdx.x - pair * p.splits;
+        seg.b = pair / p.hkv;
+        seg.kvh = pair - seg.b * p.hkv;
+        seg.len = seq_len_of(p, seg.b);
+        seg.n_chunks = chunks_of(seg.len);
+        seg.pair_u0 = 0;
+        seg.c_begin = split * p.chunks_per_split;
+        seg.c_end = min(seg.n_chunks, seg.c_begin + p.chunks_per_split);
+        if (seg.n_chunks == 0 && seg.kvh == 0 && split == 0 && threadIdx.x == 0) empty_sequence(seg.b);
+        if (seg.c_begin >= seg.c_end) return;
+    } else {
+        int total = 0, longest = 1;
+        for (int b0 = 0; b0 < p.batch; b0 += 32) {
+            const int b = b0 + lane, n = chunks_of(lane_len(b0));
+            if (n == 0 && b < p.batch && warp == 0 && b % gridDim.x == blockIdx.x) empty_sequence(b);
+            total += __reduce_add_sync(0xffffffffu, n);
+            longest = max(longest, __reduce_max_sync(0xffffffffu, n));
+        }
+        total *= p.hkv;
+        int pieces = gridDim.x;
+        if (p.plan == LINE_HANDED) pieces = max(1, min(pieces, total / longest));
+        if ((int)blockIdx.x >= pieces) return;
+        cut_q = total / pieces;
+        cut_r = total - cut_q * pieces;
+        const Cut cut(cut_q, cut_r);
+        u_begin = cut.begin(blockIdx.x);
+        u_end = cut.begin(blockIdx.x + 1);
+        if (u_begin >= u_end) return;
+        mid = u_begin;
+        mid_end = u_end;
+        if (p.plan == LINE_HANDED) {
+            const Segment head = segment_at(u_begin, u_end), tail = segment_at(u_end - 1, u_end);
+            if (head.c_begin > 0) {
+                head_last = true;
+                mid = min(u_end, head.pair_u0 + head.n_chunks);
+            }
+            if (tail.c_end < tail.n_chunks && tail.pair_u0 >= u_begin) mid_end = tail.pair_u0;
+            if (mid_end < u_end) seg = segment_at(mid_end, u_end);
+            else if (mid < mid_end) { seg = segment_at(mid, mid_end); mid += seg.c_end - seg.c_begin; }
+            else { seg = head; head_last = false; }
+        } else {
+            seg = segment_at(mid, mid_end);
+            mid += seg.c_end - seg.c_begin;
+        }
+    }
+    const Cut cut(cut_q, cut_r);
+
+    // A CTA step is TILES chunks.  Tile i of warp w: keys 16w.. of chunk i (STREAMS), or 16i.. of the warp's own contiguous
+    // run of TILES * 16 keys.
+    auto tile_chunk = [&](int i) { return STREAMS ? i : (warp * C::TILES * 16) / CHUNK; };
+    auto tile_key = [&](int i) { return STREAMS ? 16 * warp : (warp * C::TILES * 16) % CHUNK + 16 * i; };
+    constexpr int OFFS = STREAMS ? C::TILES : 1;        // chunks a warp touches per step
+    // lane-constant byte offsets inside a tile: K rows g and g + 8, V rows 2t, 2t + 1, 2t + 8, 2t + 9
+    const uint32_t k_lane = g * D + (D / 4) * t, v_lane = 2 * t * D + (D / 8) * g;
+    uint32_t kr[C::TILES][2][C::KW];    // [tile][row g / g + 8][words]
+    uint32_t vr[C::TILES][4][C::VW];
+    auto page_of = [&](int key) -> int { return (int)(__umulhi((uint32_t)key, p.page_mul) >> (p.page_shr - 1)); };
+    auto entry = [&](const Segment& x, int c) -> int {   // table entry of chunk c
+        return PAGED && c < x.c_end ? __ldg(p.block_table + (size_t)x.b * p.max_pages + page_of(c * CHUNK)) : 0;
+    };
+    // byte offset of chunk c (the same in K and V), or -1 where the table names no page of the pool: nothing is read
+    // there, the keys count as zeros
+    auto offset = [&](const Segment& x, int c, int page) -> long long {
+        if (!PAGED) return (((long long)x.b * p.hkv + x.kvh) * p.s_max + (long long)c * CHUNK) * D;
+        if (page < 0 || page >= p.num_pages) return -1;
+        const int key = c * CHUNK;
+        return (((long long)page * p.hkv + x.kvh) * p.page_size + (key - page_of(key) * p.page_size)) * D;
+    };
+    // left: keys from the chunk's first one to the end of the sequence.  Keys past it are not read but taken as zeros: they
+    // may hold anything (0 x NaN would poison O)
+    auto load_k = [&](int i, int left, long long off) {
+        const uint8_t* base = p.k + off + (k_lane + tile_key(i) * D);
+        if (left >= CHUNK) {
+#pragma unroll
+            for (int r = 0; r < 2; r++)
+#pragma unroll
+                for (int h = 0; h < D / 64; h++) ldg128(kr[i][r] + 4 * h, base + 8 * r * D + 16 * h);
+        } else {
 #pragma unroll
             for (int r = 0; r < 2; r++) {
-                const int row = g + 8 * r;
-                const bool live = row < p.group;
-                qa[ks][r] = live ? *reinterpret_cast<const uint32_t*>(qb + (size_t)row * D + (D / 4) * t + 8 * ks) : 0u;
-                qa[ks][2 + r] = live ? *reinterpret_cast<const uint32_t*>(qb + (size_t)row * D + (D / 4) * t + 8 * ks + 4) : 0u;
-            }
-        }
-    }
-
-    // online-softmax state of this warp for rows g and g + 8
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
-    float oacc[D / 8][4];
 #pragma unroll
-    for (int n = 0; n < D / 8; n++) oacc[n][0] = oacc[n][1] = oacc[n][2] = oacc[n][3] = 0.f;
-
-    // Each warp loads, converts and consumes its own 16 keys of every chunk (16 * D contiguous bytes of K and of V:
-    // PER_THREAD 16-byte pieces per lane), so the loop needs only warp-level synchronisation and the four warps of a
-    // CTA drift apart freely: their load latencies and MMA dependency stalls overlap instead of adding up.
-    // The loop is issue-bound, so everything lane-constant is hoisted: 32-bit shared addresses, byte offsets of the
-    // lane's pieces and fragments; only the last chunk of a sequence is masked.
-    constexpr int PER_THREAD = 16 * D / 16 / 32;   // 4 (D = 128) or 2 (D = 64)
-    constexpr int PARTS = D / 16;                   // 16-byte pieces per key row
-    const uint32_t sm = smem_addr(smem);
-    // piece i of this lane: key (16w + (32i + lane) / PARTS), part ((32i + lane) % PARTS); consecutive i are 32 pieces apart
-    const int key_l = 16 * warp + lane / PARTS, part_l = lane % PARTS;
-    const uint32_t k_dst = sm + key_l * S::K_STRIDE + part_l * 16;                      // + st * K_BYTES + i * (32 / PARTS) * K_STRIDE
-    const uint32_t vraw = sm + S::OFF_VRAW + (key_l * PARTS + part_l) * 16;              // + st * VRAW_BYTES + i * 512
-    const uint32_t k_frag = sm + (16 * warp + g) * S::K_STRIDE + (D / 4) * t;            // + st * K_BYTES + nt * 8 * K_STRIDE: D/4 bytes = all k-steps
-    // ldmatrix.x4: lanes 0-15 address the 16 key rows at d-tile n, lanes 16-31 the same rows at d-tile n + 1
-    const uint32_t v_frag = sm + S::OFF_V + (16 * warp + (lane & 15)) * S::V_STRIDE + (lane >> 4) * 16;   // + n * 16
-    const size_t lane_goff = (size_t)(key_l * PARTS + part_l) * 16;                      // byte offset of piece 0 inside a chunk
-    const uint8_t* kg = p.k + (PAGED ? 0 : (size_t)bh * p.s_max * D) + lane_goff;
-    const uint8_t* vg = p.v + (PAGED ? 0 : (size_t)bh * p.s_max * D) + lane_goff;
-    // paged: chunks are issued in order, so the position inside the block table advances incrementally (no division
-    // per chunk), and the entry of the next page is fetched when the last chunk of the current page is issued: its
-    // latency is hidden behind one loop iteration
-    const int* table = nullptr;      // entry of the page the next chunk to be issued lives in
-    int page_next = 0, within = 0;   // that entry's value; index of that chunk inside its page
-    size_t head_off = 0, page_stride = 0;
-    if (PAGED) {
-        const int pg = c_begin / p.chunks_per_page;
-        within = c_begin - pg * p.chunks_per_page;
-        table = p.block_table + (size_t)b * p.max_pages + pg;
-        if (c_begin < c_end) page_next = __ldg(table);
-        page_stride = (size_t)p.hkv * p.page_size * D;
-        head_off = (size_t)kvh * p.page_size * D;
-    }
-    auto issue_chunk = [&](int c) {   // global -> ring stage (c - c_begin) % STAGES, one commit group per chunk
-        const int st = (c - c_begin) % STAGES;
-        size_t off = (size_t)c * CHUNK * D;
-        // keys at or past seq_len are not read but zero-filled: past s_max they would belong to the next head, and
-        // below it they hold whatever the cache held before (possibly NaN codes; P = 0 there, but 0 x NaN would
-        // still poison O).  Only a sequence's last chunk has such keys.
-        const bool whole = (c + 1) * CHUNK <= seq_len;
-        bool none = false;
-        if (PAGED) {
-            const int page = page_next;
-            none = page < 0 || page >= p.num_pages;   // a table entry outside the pool: nothing is read, the keys count as zeros
-            // a chunk never crosses a page (page_size is a multiple of CHUNK)
-            off = none ? 0 : (size_t)page * page_stride + head_off + (size_t)within * (CHUNK * D);
-            if (++within == p.chunks_per_page) {
-                within = 0;
-                ++table;
-                if (c + 1 < c_end) page_next = __ldg(table);
-            }
-        }
+                for (int w = 0; w < C::KW; w++) kr[i][r][w] = 0u;
+                if (tile_key(i) + 8 * r + g < left) {
 #pragma unroll
-        for (int i = 0; i < PER_THREAD; i++) {
-            const uint32_t nbytes = (!none && (whole || c * CHUNK + key_l + i * (32 / PARTS) < seq_len)) ? 16u : 0u;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(k_dst + st * S::K_BYTES + i * (32 / PARTS) * S::K_STRIDE),
-                         "l"(kg + off + i * 512), "r"(nbytes)
-                         : "memory");
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(vraw + st * S::VRAW_BYTES + i * 512), "l"(vg + off + i * 512), "r"(nbytes)
-                         : "memory");
-        }
-    };
-    auto commit = [&]() { asm volatile("cp.async.commit_group;" ::: "memory"); };
-    // V codes of the landed stage -> fp16 copy the P V fragments are read from
-    auto convert_v = [&](int st) {
-        // lane j of the 8 (4) lanes of a key row converts codes [8j, 8j+8) and [D/2 + 8j, D/2 + 8j + 8): each of its two
-        // 16-byte stores then lands next to its neighbours' (bank-conflict free), unlike a 32-byte run per lane
-#pragma unroll
-        for (int i = 0; i < PER_THREAD; i++) {
-            const uint32_t src = sm + S::OFF_VRAW + st * S::VRAW_BYTES + (key_l + i * (32 / PARTS)) * D + part_l * 8;
-            const uint32_t dst = sm + S::OFF_V + (key_l + i * (32 / PARTS)) * S::V_STRIDE + part_l * 16;
-#pragma unroll
-            for (int hlf = 0; hlf < 2; hlf++) {
-                uint32_t w[2], h[4];
-                asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "r"(src + hlf * (D / 2)));
-#pragma unroll
-                for (int k = 0; k < 2; k++)
-                    asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, lo;\n\tcvt.rn.f16x2.e4m3x2 %1, hi;\n\t}"
-                        : "=r"(h[2 * k]), "=r"(h[2 * k + 1])
-                        : "r"(w[k]));
-                asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst + hlf * D), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]) : "memory");
+                    for (int h = 0; h < D / 64; h++) ldg128(kr[i][r] + 4 * h, base + 8 * r * D + 16 * h);
+                }
             }
         }
     };
-
-    // prologue: STAGES - 1 chunks in flight (empty groups keep the group count uniform)
+    auto load_v_row = [&](int i, int r, const uint8_t* row) {
+        if (D == 128) ldg128(vr[i][r], row);
+        else ldg64(vr[i][r], row);
+    };
+    auto load_v = [&](int i, int left, long long off) {
+        const uint8_t* base = p.v + off + (v_lane + tile_key(i) * D);
+        if (left >= CHUNK) {
 #pragma unroll
-    for (int i = 0; i < STAGES - 1; i++) {
-        if (c_begin + i < c_end) issue_chunk(c_begin + i);
-        commit();
-    }
-    for (int c = c_begin; c < c_end; c++) {
-        const int st = (c - c_begin) % STAGES;
-        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");   // chunk c has landed (this lane's pieces)
-        __syncwarp();             // ... the whole warp's pieces; and every lane is done with the previous chunk's fragments
-        convert_v(st);
-        if (c + STAGES - 1 < c_end) issue_chunk(c + STAGES - 1);   // into the stage computed one iteration ago
-        commit();
-        __syncwarp();
+            for (int r = 0; r < 4; r++) load_v_row(i, r, base + ((r & 1) + 8 * (r >> 1)) * D);
+        } else {
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const int key = (r & 1) + 8 * (r >> 1);   // + 2t
+#pragma unroll
+                for (int w = 0; w < C::VW; w++) vr[i][r][w] = 0u;
+                if (tile_key(i) + key + 2 * t < left) load_v_row(i, r, base + key * D);
+            }
+        }
+    };
+    // keys left of chunk c of a segment for load_k / load_v: none past the segment's end or where there is no page
+    auto left_of = [&](const Segment& x, int c, long long off) { return c < x.c_end && off >= 0 ? x.len - c * CHUNK : 0; };
+    auto chunk_at = [&](int j) { return STREAMS ? j : tile_chunk(0); };   // j-th chunk a warp touches in a step
 
-        // ---- S = Q K^T for this warp's 16 keys: two n-tiles of 8 keys.
-        // one accumulator per (n-tile, k-step): eight independent MMAs instead of two chains of four (the legacy
-        // mma.sync path has a 63-clock dependent-issue latency here), summed afterwards
-        float s[2][4];
+    bool loaded = false;   // the segment's first chunks are already on their way
+    for (;;) {             // one segment per trip
+        int page_next[OFFS];
+        if (!loaded) {
+#pragma unroll
+            for (int j = 0; j < OFFS; j++) {
+                const int c = seg.c_begin + chunk_at(j);
+                const long long off = offset(seg, c, entry(seg, c));
+                const int left = left_of(seg, c, off);
+#pragma unroll
+                for (int i = j; i < (STREAMS ? j + 1 : C::TILES); i++) {
+                    load_k(i, left, off);
+                    load_v(i, left, off);
+                }
+            }
+        }
+        loaded = false;
+#pragma unroll
+        for (int j = 0; j < OFFS; j++) page_next[j] = entry(seg, seg.c_begin + C::TILES + chunk_at(j));
+
+        // the segment behind this one waits in shared memory (a copy per warp: no barrier)
+        bool more = true;
+        int next_entry[OFFS];
         {
-            float part[2][KSTEPS][4];
-            const uint32_t kf = k_frag + st * S::K_BYTES;
-#pragma unroll
-            for (int nt = 0; nt < 2; nt++) {
-                // B fragments of every k-step: key = column g of the n-tile, this lane's D/4 contiguous bytes of its row
-                uint32_t kw[D / 16];
-#pragma unroll
-                for (int v = 0; v < D / 64; v++)
-                    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];"
-                                 : "=r"(kw[4 * v]), "=r"(kw[4 * v + 1]), "=r"(kw[4 * v + 2]), "=r"(kw[4 * v + 3])
-                                 : "r"(kf + nt * 8 * S::K_STRIDE + 16 * v));
-#pragma unroll
-                for (int ks = 0; ks < KSTEPS; ks++) mma_e4m3_m16n8k32_zero(part[nt][ks], qa[ks], kw[2 * ks], kw[2 * ks + 1]);
+            Segment next;
+            if (mid < mid_end) {
+                next = segment_at(mid, mid_end);
+                mid += next.c_end - next.c_begin;
+            } else if (head_last) {
+                next = segment_at(u_begin, u_end);
+                head_last = false;
+            } else {
+                more = false;
             }
+            if (more) {
 #pragma unroll
-            for (int nt = 0; nt < 2; nt++)
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    float acc = part[nt][0][e];
-#pragma unroll
-                    for (int ks = 1; ks < KSTEPS; ks++) acc += part[nt][ks][e];
-                    s[nt][e] = acc * scale_log2;
-                }
-        }
-        // scores: s[nt][0..1] = row g, keys 8nt + 2t, +1 ; s[nt][2..3] = row g + 8
-        if ((c + 1) * CHUNK > seq_len) {   // only the last chunk of a sequence has keys past its end
-            const int key0 = c * CHUNK + 16 * warp;
-#pragma unroll
-            for (int nt = 0; nt < 2; nt++)
-#pragma unroll
-                for (int e = 0; e < 4; e++)
-                    if (key0 + 8 * nt + 2 * t + (e & 1) >= seq_len) s[nt][e] = -INFINITY;
-        }
-        float mx[2];
-        mx[0] = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]));
-        mx[1] = fmaxf(fmaxf(s[0][2], s[0][3]), fmaxf(s[1][2], s[1][3]));
-        float corr[2];
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
-            mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
-            const float m_new = fmaxf(m[r], mx[r]);
-            corr[r] = (m[r] == -INFINITY) ? 0.f : ex2f(m[r] - m_new);   // m_new = -inf only if m is too
-            m[r] = m_new;
-        }
-        uint32_t pa[4];
-        float psum[2] = {0.f, 0.f};
-#pragma unroll
-        for (int nt = 0; nt < 2; nt++) {
-            float pv[4];
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                pv[e] = (m[e >> 1] == -INFINITY) ? 0.f : ex2f(s[nt][e] - m[e >> 1]);
-                psum[e >> 1] += pv[e];
+                for (int j = 0; j < OFFS; j++) next_entry[j] = entry(next, next.c_begin + chunk_at(j));
+                if (lane == 0) s_next[warp] = next;
             }
-            // A fragment of the 16 x 16 P tile: a0 = (row g, keys 2t..), a1 = (row g+8, ...), a2/a3 = keys + 8
-            pa[2 * nt] = pack_h2(pv[0], pv[1]);
-            pa[2 * nt + 1] = pack_h2(pv[2], pv[3]);
+            __syncwarp();
         }
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            psum[r] += __shfl_xor_sync(0xffffffffu, psum[r], 1);
-            psum[r] += __shfl_xor_sync(0xffffffffu, psum[r], 2);
-            l[r] = l[r] * corr[r] + psum[r];
-        }
-        // ---- O = O * corr + P V over this warp's 16 keys (the running maxima rarely move once a few chunks are in)
-        const bool rescale = !__all_sync(0xffffffffu, corr[0] == 1.0f && corr[1] == 1.0f);
-#pragma unroll
-        for (int n = 0; n < D / 8; n += 2) {
-            uint32_t b0, b1, b2, b3;
-            ldmatrix_x4_trans(b0, b1, b2, b3, v_frag + n * 16);
-            if (rescale) {
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    oacc[n + h][0] *= corr[0];
-                    oacc[n + h][1] *= corr[0];
-                    oacc[n + h][2] *= corr[1];
-                    oacc[n + h][3] *= corr[1];
-                }
-            }
-            mma_f16_m16n8k16(oacc[n], pa, b0, b1);
-            mma_f16_m16n8k16(oacc[n + 1], pa, b2, b3);
-        }
-    }
 
-    // ---- merge the four warps' states (shared memory reused)
-    __syncthreads();
-    float* mo = reinterpret_cast<float*>(smem);            // [4][ROWS][D]
-    float* mml = mo + 4 * ROWS * D;                        // [4][ROWS][2]
+        const int b = seg.b, kvh = seg.kvh;
+        // Q fragments (B operand): column g of tile n is query head kvh * group + 8n + g, words as in the K rows
+        uint32_t qf[NQ][C::KW];
 #pragma unroll
-    for (int n = 0; n < D / 8; n++) {
-        float* base = mo + ((size_t)warp * ROWS) * D + n * 8 + 2 * t;
-        base[(size_t)g * D] = oacc[n][0];
-        base[(size_t)g * D + 1] = oacc[n][1];
-        base[(size_t)(g + 8) * D] = oacc[n][2];
-        base[(size_t)(g + 8) * D + 1] = oacc[n][3];
-    }
-    if (t == 0) {
+        for (int n = 0; n < NQ; n++) {
+            const bool live = 8 * n + g < p.group;
+            const uint8_t* qb = p.q + ((size_t)b * p.hq + (size_t)kvh * p.group + 8 * n + g) * D + (D / 4) * t;
 #pragma unroll
-        for (int r = 0; r < 2; r++) {
-            mml[(warp * ROWS + g + 8 * r) * 2] = m[r];
-            mml[(warp * ROWS + g + 8 * r) * 2 + 1] = l[r];
+            for (int w = 0; w < C::KW; w++) qf[n][w] = live ? *reinterpret_cast<const uint32_t*>(qb + 4 * w) : 0u;
         }
-    }
-    __syncthreads();
-    const float vds = p.sv ? p.v_descale * __ldg(p.sv) : p.v_descale;
-    for (int idx = threadIdx.x; idx < ROWS * D; idx += THREADS) {
-        const int row = idx / D, col = idx % D;
-        float M = -INFINITY;
-#pragma unroll
-        for (int w = 0; w < 4; w++) M = fmaxf(M, mml[(w * ROWS + row) * 2]);
-        float L = 0.f, O = 0.f;
-#pragma unroll
-        for (int w = 0; w < 4; w++) {
-            const float mw = mml[(w * ROWS + row) * 2];
-            const float f = (mw == -INFINITY) ? 0.f : ex2f(mw - M);
-            L += mml[(w * ROWS + row) * 2 + 1] * f;
-            O += mo[((size_t)w * ROWS + row) * D + col] * f;
-        }
-        if (p.splits > 1) {
-            const size_t slot = ((size_t)bh * p.splits + split) * ROWS + row;
-            p.ws_o[slot * D + col] = O;
-            if (col == 0) {
-                p.ws_ml[slot * 2] = M;
-                p.ws_ml[slot * 2 + 1] = L;
-            }
-        } else if (row < p.group) {
-            const size_t orow = (size_t)b * p.hq + (size_t)kvh * p.group + row;
-            p.o[orow * D + col] = __float2half_rn(L > 0.f ? O * (vds / L) : 0.f);
-            if (col == 0 && p.lse) p.lse[orow] = (L > 0.f) ? (M + log2f(L)) * 0.6931471805599453f : -INFINITY;
-        }
-    }
-}
 
-// merges the splits of one (sequence, kv head): grid = B*Hkv, threads over ROWS x D
-template <int D>
-__global__ void __launch_bounds__(THREADS) fa_decode_combine_kernel(const DecodeParams p) {
-    const int bh = blockIdx.x;
-    const int b = bh / p.hkv, kvh = bh % p.hkv;
-    const float vds = p.sv ? p.v_descale * __ldg(p.sv) : p.v_descale;
-    for (int idx = threadIdx.x; idx < p.group * D; idx += THREADS) {
-        const int row = idx / D, col = idx % D;
-        float M = -INFINITY;
-        for (int s = 0; s < p.splits; s++) M = fmaxf(M, p.ws_ml[(((size_t)bh * p.splits + s) * ROWS + row) * 2]);
-        float L = 0.f, O = 0.f;
-        for (int s = 0; s < p.splits; s++) {
-            const size_t slot = ((size_t)bh * p.splits + s) * ROWS + row;
-            const float ms = p.ws_ml[slot * 2];
-            const float f = (ms == -INFINITY) ? 0.f : ex2f(ms - M);
-            L += p.ws_ml[slot * 2 + 1] * f;
-            O += p.ws_o[slot * D + col] * f;
+        // online-softmax state for query columns 2t and 2t + 1 of every column tile: running maximum (the same in all lanes
+        // g) and this lane's part of the sum
+        float m[NQ][2], l[NQ][2];
+        float acc[NQ][C::MT][4];
+#pragma unroll
+        for (int n = 0; n < NQ; n++) {
+#pragma unroll
+            for (int e = 0; e < 2; e++) { m[n][e] = -INFINITY; l[n][e] = 0.f; }
+#pragma unroll
+            for (int i = 0; i < C::MT; i++) acc[n][i][0] = acc[n][i][1] = acc[n][i][2] = acc[n][i][3] = 0.f;
         }
-        const size_t orow = (size_t)b * p.hq + (size_t)kvh * p.group + row;
-        p.o[orow * D + col] = __float2half_rn(L > 0.f ? O * (vds / L) : 0.f);
-        if (col == 0 && p.lse) p.lse[orow] = (L > 0.f) ? (M + log2f(L)) * 0.6931471805599453f : -INFINITY;
+        if (STREAMS && p.plan == LINE_HANDED && seg.c_begin > 0 && p.handed) {
+            uint32_t f = ~p.epoch;
+            for (int polls = 0; polls < 20000 && f != p.epoch; polls++)
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(f) : "l"(p.handed + blockIdx.x - 1) : "memory");
+            if (__all_sync(0xffffffffu, f == p.epoch)) {
+#pragma unroll
+                for (int n = 0; n < NQ; n++)
+#pragma unroll
+                    for (int e = 0; e < 2; e++)
+                        m[n][e] = __ldcg(p.ws_handed + ((size_t)(blockIdx.x - 1) * WARPS + warp) * C::ROWS + 8 * n + 2 * t + e);
+            }
+        }
+
+        for (int c = seg.c_begin; c < seg.c_end; c += C::TILES) {
+            // ---- S^T = K Q^T, one accumulator per k-step: independent MMAs instead of a chain
+            float s[NQ][C::TILES][4];
+#pragma unroll
+            for (int n = 0; n < NQ; n++)
+#pragma unroll
+                for (int i = 0; i < C::TILES; i++) {
+                    float part[C::KSTEPS][4];
+#pragma unroll
+                    for (int ks = 0; ks < C::KSTEPS; ks++)
+                        mma_e4m3_m16n8k32_zero(part[ks], kr[i][0][2 * ks], kr[i][1][2 * ks], kr[i][0][2 * ks + 1], kr[i][1][2 * ks + 1],
+                                               qf[n][2 * ks], qf[n][2 * ks + 1]);
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        float x = part[0][e];
+#pragma unroll
+                        for (int ks = 1; ks < C::KSTEPS; ks++) x += part[ks][e];
+                        s[n][i][e] = x * scale_log2;
+                    }
+                }
+            // ---- the next chunks' keys, of this segment or, behind its last ones, of the next: the merge below then hides
+            // their latency
+            const bool roll = c + C::TILES >= seg.c_end;
+            const bool fetch = !roll || more;
+            int left_n[OFFS];
+            long long off_n[OFFS];
+            if (!roll) {
+#pragma unroll
+                for (int j = 0; j < OFFS; j++) {
+                    const int cn = c + C::TILES + chunk_at(j);
+                    off_n[j] = offset(seg, cn, page_next[j]);
+                    left_n[j] = left_of(seg, cn, off_n[j]);
+                    page_next[j] = entry(seg, cn + C::TILES);
+                }
+            } else if (more) {
+                const Segment next = s_next[warp];
+#pragma unroll
+                for (int j = 0; j < OFFS; j++) {
+                    const int cn = next.c_begin + chunk_at(j);
+                    off_n[j] = offset(next, cn, next_entry[j]);
+                    left_n[j] = left_of(next, cn, off_n[j]);
+                }
+                loaded = true;
+            }
+            if (fetch) {
+#pragma unroll
+                for (int i = 0; i < C::TILES; i++) load_k(i, left_n[STREAMS ? i : 0], off_n[STREAMS ? i : 0]);
+            }
+            // ---- softmax and O^T += V^T P^T, 16 keys at a time.  s[n][i][e] = key g (e < 2) or g + 8 of tile i,
+            // query 8n + 2t + (e & 1)
+#pragma unroll
+            for (int i = 0; i < C::TILES; i++) {
+                const int ci = c + tile_chunk(i);
+                const int key0 = ci * CHUNK + tile_key(i), key_end = ci < seg.c_end ? seg.len : 0;
+                if (key0 + 16 > key_end) {   // only the last chunk of a sequence has keys past its end
+#pragma unroll
+                    for (int n = 0; n < NQ; n++)
+#pragma unroll
+                        for (int e = 0; e < 4; e++)
+                            if (key0 + g + 8 * (e >> 1) >= key_end) s[n][i][e] = -INFINITY;
+                }
+                float mx[NQ][2];
+                bool bump = false;
+#pragma unroll
+                for (int n = 0; n < NQ; n++)
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        mx[n][e] = fmaxf(s[n][i][e], s[n][i][e + 2]);
+                        bump = bump || mx[n][e] > (STREAMS ? m[n][e] : m[n][e] + LAG);
+                    }
+                if (__any_sync(0xffffffffu, bump)) {   // rare once a few chunks are in
+#pragma unroll
+                    for (int n = 0; n < NQ; n++)
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+#pragma unroll
+                            for (int o = 4; o < 32; o <<= 1) mx[n][e] = fmaxf(mx[n][e], __shfl_xor_sync(0xffffffffu, mx[n][e], o));
+                            const float m_new = fmaxf(m[n][e], mx[n][e]);
+                            const float f = m[n][e] == -INFINITY ? 0.f : ex2f(m[n][e] - m_new);
+                            m[n][e] = m_new;
+                            l[n][e] *= f;
+#pragma unroll
+                            for (int j = 0; j < C::MT; j++) {
+                                acc[n][j][e] *= f;
+                                acc[n][j][e + 2] *= f;
+                            }
+                        }
+                }
+                // P^T as B fragments: rows (keys) 2t, 2t + 1 and 2t + 8, 2t + 9 of column g
+                uint32_t pf[NQ][2];
+#pragma unroll
+                for (int n = 0; n < NQ; n++) {
+                    float pv[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        pv[e] = m[n][e & 1] == -INFINITY ? 0.f : ex2f(s[n][i][e] - m[n][e & 1]);
+                        l[n][e & 1] += pv[e];
+                    }
+                    pf[n][0] = transpose_8x8_b16(pack_h2(pv[0], pv[1]));
+                    pf[n][1] = transpose_8x8_b16(pack_h2(pv[2], pv[3]));
+                }
+                // rows g and g + 8 of tile j of O^T are d = (D/8) g + 2j and + 1
+#pragma unroll
+                for (int w = 0; w < C::VW; w++)
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const uint32_t sel = h ? 0x7362 : 0x5140;   // bytes (2h, 2h + 1) of two keys, interleaved
+                        uint32_t a[4];
+                        e4m3x4_to_h2x2(__byte_perm(vr[i][0][w], vr[i][1][w], sel), a[0], a[1]);
+                        e4m3x4_to_h2x2(__byte_perm(vr[i][2][w], vr[i][3][w], sel), a[2], a[3]);
+#pragma unroll
+                        for (int n = 0; n < NQ; n++) mma_f16_m16n8k16(acc[n][2 * w + h], a, pf[n][0], pf[n][1]);
+                    }
+            }
+            if (fetch) {
+#pragma unroll
+                for (int i = 0; i < C::TILES; i++) load_v(i, left_n[STREAMS ? i : 0], off_n[STREAMS ? i : 0]);
+            }
+        }
+
+        // ---- merge the four warps' states
+        const bool whole = seg.c_begin == 0 && seg.c_end == seg.n_chunks;
+        const bool hand_on = STREAMS && p.plan == LINE_HANDED && p.handed && seg.c_end < seg.n_chunks;
+#pragma unroll
+        for (int n = 0; n < NQ; n++)
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) l[n][e] += __shfl_xor_sync(0xffffffffu, l[n][e], o);
+                const int row = 8 * n + 2 * t + e;
+                if (g == 0) {
+                    s_m[warp][row] = m[n][e];
+                    s_l[warp][row] = l[n][e];
+                    if (hand_on) __stcg(p.ws_handed + ((size_t)blockIdx.x * WARPS + warp) * C::ROWS + row, m[n][e]);
+                }
+                if (row < p.group) {
+#pragma unroll
+                    for (int j = 0; j < C::MT; j++)
+                        *reinterpret_cast<float2*>(&s_o[warp][row][(D / 8) * g + 2 * j]) = make_float2(acc[n][j][e], acc[n][j][e + 2]);
+                }
+            }
+        if (hand_on) __threadfence();
+        __syncthreads();
+        if (hand_on && threadIdx.x == 0)
+            asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p.handed + blockIdx.x), "r"(p.epoch) : "memory");
+        // slots of a cut pair: its splits in order, or on the line the odd slot of the CTA that has its first piece and the
+        // even slots of the CTAs after that
+        const int slot = p.plan == SPLITS ? blockIdx.x : 2 * blockIdx.x + (seg.c_begin == 0 ? 1 : 0);
+        const float vds = p.sv ? p.v_descale * __ldg(p.sv) : p.v_descale;
+        for (int idx = threadIdx.x; idx < p.group * (D / 4); idx += THREADS) {   // four columns per thread and step
+            const int row = idx / (D / 4), col = idx % (D / 4) * 4;
+            float M = -INFINITY;
+#pragma unroll
+            for (int w = 0; w < WARPS; w++) M = fmaxf(M, s_m[w][row]);
+            float L = 0.f;
+            float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int w = 0; w < WARPS; w++) {
+                const float mw = s_m[w][row];
+                fold(L, O, s_l[w][row], *reinterpret_cast<const float4*>(&s_o[w][row][col]), mw == -INFINITY ? 0.f : ex2f(mw - M));
+            }
+            if (whole) {
+                store_out<D>(p, ((size_t)b * p.hq + (size_t)kvh * p.group + row), col, M, L, O, vds);
+            } else {
+                const size_t at = (size_t)slot * C::ROWS + row;
+                __stcg(reinterpret_cast<float4*>(p.ws_o + at * D + col), O);
+                if (col == 0) __stcg(reinterpret_cast<float2*>(p.ws_ml + at * 2), make_float2(M, L));
+            }
+        }
+        if (!whole) {
+            int parts, slot0, slot_step;   // the pair's pieces: slot0, then slot0 + 1 + i * slot_step
+            if (p.plan == SPLITS) {
+                parts = (seg.n_chunks + p.chunks_per_split - 1) / p.chunks_per_split;
+                slot0 = (blockIdx.x / p.splits) * p.splits;
+                slot_step = 1;
+            } else {
+                const int first = cut.piece_of(seg.pair_u0);
+                parts = cut.piece_of(seg.pair_u0 + seg.n_chunks - 1) - first + 1;
+                slot0 = 2 * first + 1;
+                slot_step = 2;
+            }
+            const int bh = b * p.hkv + kvh;
+            __threadfence();
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                s_last = atomicAdd(p.arrivals + bh, 1u) == (uint32_t)(parts - 1);
+                if (s_last) p.arrivals[bh] = 0;   // for the next launch
+            }
+            __syncthreads();
+            if (s_last) {
+                __threadfence();
+                for (int idx = threadIdx.x; idx < p.group * (D / 4); idx += THREADS) {
+                    const int row = idx / (D / 4), col = idx % (D / 4) * 4;
+                    float M = -INFINITY, L = 0.f;
+                    float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int i0 = 0; i0 < parts; i0 += 8) {   // eight pieces' loads in flight
+                        float2 ml[8];
+                        float4 oi[8];
+#pragma unroll
+                        for (int k = 0; k < 8; k++) {
+                            const int i = i0 + k;
+                            ml[k] = make_float2(-INFINITY, 0.f);
+                            oi[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                            if (i >= parts) continue;
+                            const size_t at = (size_t)(i == 0 ? slot0 : slot0 + 1 + (i - 1) * slot_step) * C::ROWS + row;
+                            ml[k] = __ldcg(reinterpret_cast<const float2*>(p.ws_ml + at * 2));
+                            oi[k] = __ldcg(reinterpret_cast<const float4*>(p.ws_o + at * D + col));
+                        }
+                        float M2 = M;
+#pragma unroll
+                        for (int k = 0; k < 8; k++) M2 = fmaxf(M2, ml[k].x);
+                        if (M2 == -INFINITY) continue;
+                        const float f = ex2f(M - M2);
+                        L *= f;
+                        O.x *= f; O.y *= f; O.z *= f; O.w *= f;
+#pragma unroll
+                        for (int k = 0; k < 8; k++) fold(L, O, ml[k].y, oi[k], ex2f(ml[k].x - M2));
+                        M = M2;
+                    }
+                    store_out<D>(p, ((size_t)b * p.hq + (size_t)kvh * p.group + row), col, M, L, O, vds);
+                }
+            }
+        } else {
+            __syncthreads();   // the merge buffer is free again
+        }
+        if (!more) break;
+        seg = s_next[warp];
+        __syncwarp();
     }
 }
 
 int num_sms_of_current_device() {
+    static int cached[64];   // 0 = not asked yet; every thread would store the same value
     int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaGetDevice(&dev) != cudaSuccess) return sms;
+    if (dev >= 0 && dev < 64 && cached[dev]) return cached[dev];
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (dev >= 0 && dev < 64) cached[dev] = sms;
     return sms;
 }
 
-}  // namespace
-
-namespace {
-int decode_splits(int batch, int kv_heads, int span) {
-    // Enough CTAs to fill the GPU once (CTAS_PER_SM fit an SM) and no more: all of them resident at the same time, equal
-    // key ranges, so none waits for a second wave; with batch * kv_heads CTAs or more there is nothing to split.
-    const int chunks = (span + CHUNK - 1) / CHUNK;
-    const long long ctas = (long long)batch * kv_heads;
-    const long long slots = (long long)CTAS_PER_SM * num_sms_of_current_device();
-    long long splits = slots / ctas;
+struct Layout {
+    int plan, splits, grid, rows;
+};
+// One query head per kv head keeps the streams: fixed splits while the pairs leave room for them, else the line with
+// hand-over.  Groups take the freely cut line, which balances best (24 sequences of 3000 to 6000 keys, 8 kv heads: 45 us
+// against 70 with fixed splits and a merging kernel).
+Layout layout_of(int batch, int q_heads, int kv_heads, int span) {
+    Layout x;
+    const int group = q_heads / kv_heads;
+    x.rows = group <= 8 ? 8 : 16;
+    const long long pairs = (long long)batch * kv_heads, chunks = (span + CHUNK - 1) / CHUNK;
+    const long long narrow = (long long)ctas_per_sm(1, false) * num_sms_of_current_device();
+    long long splits = narrow / pairs;
     if (splits > chunks) splits = chunks;
     if (splits > 64) splits = 64;
     if (splits < 1) splits = 1;
-    return (int)splits;
+    x.splits = (int)splits;
+    if (group == 1 && pairs * splits <= narrow) {
+        x.plan = SPLITS;
+        x.grid = (int)(pairs * splits);
+    } else {
+        x.plan = group == 1 ? LINE_HANDED : LINE;
+        const long long slots = (long long)ctas_per_sm(x.rows / 8, true) * num_sms_of_current_device();
+        const long long units = pairs * chunks;
+        x.grid = (int)(units < slots ? (units > 0 ? units : 1) : slots);
+    }
+    return x;
 }
+
 }  // namespace
 
-size_t decode_workspace_bytes(int batch, int kv_heads, int head_dim, int span) {
-    const int splits = decode_splits(batch, kv_heads, span);
-    if (splits <= 1) return 0;
-    return (size_t)batch * kv_heads * splits * ROWS * (head_dim + 2) * sizeof(float);
+size_t decode_workspace_bytes(int batch, int q_heads, int kv_heads, int head_dim, int span) {
+    const Layout x = layout_of(batch, q_heads, kv_heads, span);
+    return (size_t)x.grid * x.rows * (2 * (head_dim + 2) + WARPS) * sizeof(float);
+}
+size_t decode_flag_count(int batch, int q_heads, int kv_heads, int span) {
+    const Layout x = layout_of(batch, q_heads, kv_heads, span);
+    return x.plan == LINE_HANDED ? (size_t)x.grid : 0;
 }
 
 cudaError_t launch_decode(const DecodeArgs& a) {
+    const int span = decode_span(a);
+    if ((long long)a.batch * a.kv_heads * ((span + CHUNK - 1) / CHUNK) > 0x7fffffffLL) return cudaErrorInvalidValue;
+    if (!a.workspace || !a.arrivals) return cudaErrorInvalidValue;
+    const Layout x = layout_of(a.batch, a.q_heads, a.kv_heads, span);
     DecodeParams p;
     p.q = static_cast<const uint8_t*>(a.q);
     p.k = static_cast<const uint8_t*>(a.k_cache);
@@ -451,33 +739,31 @@ cudaError_t launch_decode(const DecodeArgs& a) {
     p.scale_log2 = a.scale * 1.4426950408889634f;
     p.v_descale = a.v_descale;
     p.sq = a.scale_q_dev; p.sk = a.scale_k_dev; p.sv = a.scale_v_dev;
-    const int span = decode_span(a);
-    p.splits = decode_splits(a.batch, a.kv_heads, span);
-    const int chunks = (span + CHUNK - 1) / CHUNK;
-    p.chunks_per_split = (chunks + p.splits - 1) / p.splits;
-    p.ws_o = static_cast<float*>(a.workspace);
-    p.ws_ml = p.ws_o ? p.ws_o + (size_t)a.batch * a.kv_heads * p.splits * ROWS * a.hd : nullptr;
-    if (p.splits > 1 && !a.workspace) return cudaErrorInvalidValue;
+    p.plan = x.plan; p.splits = x.splits;
+    p.chunks_per_split = ((span + CHUNK - 1) / CHUNK + x.splits - 1) / x.splits;
     p.block_table = a.block_table;
+    p.page_mul = p.page_shr = 0;
+    if (a.block_table) {   // page_size >= 64; exact for numerators below 2^31, and the multiplier fits 32 bits
+        uint32_t lg = 0;
+        while ((1ull << lg) < (unsigned)a.page_size) lg++;
+        p.page_mul = (uint32_t)(((1ull << (31 + lg)) + a.page_size - 1) / a.page_size);
+        p.page_shr = lg;   // umulhi is >> 32: >> (31 + lg) is >> (lg - 1) more
+    }
     p.page_size = a.page_size; p.max_pages = a.max_pages; p.num_pages = a.num_pages;
-    p.chunks_per_page = a.block_table ? a.page_size / CHUNK : 1;
-    const dim3 grid((unsigned)(a.batch * a.kv_heads), (unsigned)p.splits);
-    auto run = [&](auto kernel, auto combine, int smem_bytes) -> cudaError_t {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-        if (e != cudaSuccess) return e;
-        kernel<<<grid, THREADS, smem_bytes, a.stream>>>(p);
-        if (p.splits > 1) combine<<<grid.x, THREADS, 0, a.stream>>>(p);
-        return cudaSuccess;
-    };
-    cudaError_t e;
-    if (a.hd == 128)
-        e = a.block_table ? run(fa_decode_kernel<128, true>, fa_decode_combine_kernel<128>, Smem<128>::BYTES)
-                          : run(fa_decode_kernel<128, false>, fa_decode_combine_kernel<128>, Smem<128>::BYTES);
-    else
-        e = a.block_table ? run(fa_decode_kernel<64, true>, fa_decode_combine_kernel<64>, Smem<64>::BYTES)
-                          : run(fa_decode_kernel<64, false>, fa_decode_combine_kernel<64>, Smem<64>::BYTES);
-    if (e != cudaSuccess) return e;
-    return cudaGetLastError();
+    p.ws_o = static_cast<float*>(a.workspace);
+    p.ws_ml = p.ws_o + (size_t)x.grid * 2 * x.rows * a.hd;
+    p.ws_handed = p.ws_ml + (size_t)x.grid * 2 * x.rows * 2;
+    p.arrivals = a.arrivals;
+    p.handed = a.flags; p.epoch = a.epoch;
+    auto run = [&](auto contiguous, auto paged) { return launch_pdl(a.block_table ? paged : contiguous, x.grid, THREADS, 0, a.stream, p); };
+#define KERNEL(D, NQ, WIDE, STREAMS) run(fa_decode_kernel<D, NQ, WIDE, STREAMS, false>, fa_decode_kernel<D, NQ, WIDE, STREAMS, true>)
+#define KERNELS(D)                                                    \
+    (x.plan == SPLITS        ? KERNEL(D, 1, false, true)              \
+     : x.plan == LINE_HANDED ? KERNEL(D, 1, true, true)               \
+     : x.rows == 8           ? KERNEL(D, 1, true, false) : KERNEL(D, 2, true, false))
+    return a.hd == 128 ? KERNELS(128) : KERNELS(64);
+#undef KERNELS
+#undef KERNEL
 }
 
 }  // namespace fa_sm100

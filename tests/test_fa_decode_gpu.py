@@ -175,3 +175,30 @@ def test_paged_rejects_bad_page_size(cuda, built_libs, fa_ctx):
         with pytest.raises(F.FAError) as e:
             fa_ctx.Decode(p, p, p, p, 0, 0, 1, 8, 2, 128, 0, 64, 1.0, block_table=p, **kw)
         assert e.value.status == F.FA_ERR_INVALID_ARG
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,Smax,D,lens", [
+    (150, 2, 1, 70, 128, "ramp"),        # more sequences than a warp keeps lengths for, empty ones among them
+    (40, 9, 1, 130, 64, "ramp"),         # nine query heads per kv head: two column tiles, the second nearly empty
+    (1, 3, 1, 20000, 128, "full"),       # one pair cut into hundreds of pieces (several batches of the merge)
+    (1, 16, 1, 9000, 64, "full"),
+    (2, 8, 8, 65, 128, "full"),          # fewer chunks than CTAs: every chunk is a piece, a one-key second chunk
+    (7, 4, 2, 1500, 128, "one long"),    # one long sequence among very short ones
+    (25, 32, 32, 200, 128, "ramp"),      # one query head per kv head, more pairs than CTAs: each pair cut at most once
+    (23, 30, 30, 1100, 64, "one long"),
+])
+def test_decode_work_split(cuda, built_libs, fa_ctx, B, Hq, Hkv, Smax, D, lens):
+    # the key range is cut at chunk borders wherever the pieces of the work line end, whatever the lengths are
+    name = f"decode-split{B}_{Hq}_{Hkv}_{Smax}_{D}"
+    q, k, v, sq, sk, sv = make_case(name, B, Hq, Hkv, Smax, D)
+    seq_lens = {"ramp": np.arange(B) * Smax // B, "full": np.full(B, Smax), "one long": np.where(np.arange(B) == 3, Smax, 1 + np.arange(B))}[lens]
+    scale = sq * sk / math.sqrt(D)
+    got, lse = run_decode(fa_ctx, q, k, v, seq_lens, scale, sv)
+    again, lse2 = run_decode(fa_ctx, q, k, v, seq_lens, scale, sv)
+    ref, rl = glue.decode_attention_f64(q, k, v, seq_lens, scale, sv)
+    assert np.array_equal(got, again) and np.array_equal(lse, lse2)      # merged in a fixed order
+    some = seq_lens > 0
+    assert np.all(got[~some] == 0) and np.all(np.isneginf(lse[~some]))
+    maxabs, meanrel = O.error_stats(got[some], ref[some])
+    assert maxabs <= 2e-2 and meanrel <= 1e-2, (maxabs, meanrel)
+    assert np.abs(lse[some] - rl[some]).max() <= 5e-3
