@@ -1,0 +1,444 @@
+// fp8_gemm_skinny.cuh — the GEMM for few rows of A (M up to 192: the tokens of a decode step or of a short prompt).
+// Included by fp8_gemm_sm100.cu, which owns the argument checks, the status word and the call of plan().
+//
+// Such a product reads the weight B[N,K] once and does next to no arithmetic: its floor is N*K bytes of HBM traffic.  What
+// it needs is many bytes in flight from the first microsecond to the last, which the square kernel does not give it (it
+// puts the tokens on the 128 MMA rows, fills half of shared memory with zero rows for them, covers N with as few as 64
+// CTAs and streams a weight panel twice once M passes 128).  Here
+//  * the weight rows are the MMA's M dimension and the tokens its N dimension (any multiple of 16), so a stage of the ring
+//    holds 16 KB of weights and only 128 bytes per token, and every weight byte is read once;
+//  * the K range of a 128-row tile is cut over a thread-block cluster of 1 to 8 CTAs; the fp32 partial sums meet in
+//    distributed shared memory and are added in rank order (no atomics: the result does not depend on timing);
+//  * all CTAs are resident at once, up to two to an SM, so the kernel is one wave of equal streams (an SM takes in about
+//    57 bytes a nanosecond, so weights have to be spread over nearly all of them to reach the 6.5 TB/s of HBM);
+//  * the kernel starts before its predecessor on the stream has drained and asks for its first weight tiles to be
+//    brought into L2 while the small kernel ahead (a quantiser, usually) still runs.
+// What is left is 3 us of start, fill and finish beside the stream: M = 16, 8192 x 8192 16.7 -> 13.7 us (floor 10.3),
+// 11008 x 4096 12.8 -> 10.3 (6.9), 4096 x 11008 12.9 -> 10.8 (6.9), 4096 x 4096 7.8 -> 6.1 (2.6).
+#pragma once
+
+namespace skinny {
+
+constexpr int W_ROWS = 128;                 // weight rows per tile = TMEM lanes
+constexpr int W_BYTES = W_ROWS * BK;        // of one k-block
+constexpr int MAX_TOKENS = 192;
+constexpr int MAX_STAGES = 16;
+constexpr int MAX_SPLIT = 8;                // portable cluster size
+constexpr int PREFETCH_BLOCKS = 16;         // k-blocks per CTA asked for ahead of the wait
+constexpr int THREADS = 192;                // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2-5: read the accumulators back
+constexpr int TAIL_BYTES = 1024 /*align*/ + 512 /*barriers*/;
+constexpr int SMEM_ONE = 227 * 1024;        // of one CTA when it has the SM to itself
+constexpr int SMEM_TWO = 112 * 1024;        // of one of two CTAs on an SM
+
+struct Params {
+    GemmParams g;
+    int tn;            // tokens rounded up to 16: MMA N
+    int tmem_cols;
+    uint32_t idesc;
+    int stages;
+    int vec;           // four neighbouring outputs of a token may be stored at once
+};
+
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_dsmem(uint32_t addr, uint32_t rank) {
+    float4 v;
+    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\t"
+                 "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(rank) : "memory");
+    return v;
+}
+__device__ __forceinline__ void prefetch_l2_2d(const CUtensorMap* m, int x, int y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];"
+                 ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y) : "memory");
+}
+// a scalar that a kernel ahead on the stream may have written: a plain load behind the wait, never a read-only one
+__device__ __forceinline__ float ld_scalar(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+// the cluster's partial results for weight rows [row, row + 4) and token j: loads, and their sum in rank order
+template <int SPLIT>
+__device__ __forceinline__ void gather(float4* v, uint32_t part, int j, int row) {
+    const uint32_t a = part + j * (W_ROWS * 4) + row * 4;
+    if (SPLIT == 1) {
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[0].z), "=f"(v[0].w) : "r"(a) : "memory");
+    } else {
+#pragma unroll
+        for (int s = 0; s < SPLIT; s++) v[s] = ld_dsmem(a, s);
+    }
+}
+template <int SPLIT>
+__device__ __forceinline__ void add_up(const float4* v, float* r) {
+    r[0] = v[0].x; r[1] = v[0].y; r[2] = v[0].z; r[3] = v[0].w;
+#pragma unroll
+    for (int s = 1; s < SPLIT; s++) { r[0] += v[s].x; r[1] += v[s].y; r[2] += v[s].z; r[3] += v[s].w; }
+}
+
+template <int SPLIT>
+__global__ void __launch_bounds__(THREADS, 2)
+fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_t, const Params p) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;   // swizzle atoms are 1024 bytes
+    uint8_t* ring_gen = smem_raw + (ring - smem_u32(smem_raw));
+    const int stage_bytes = W_BYTES + p.tn * BK;                   // a multiple of 2048
+    const uint32_t bar_full = ring + p.stages * stage_bytes;
+    const uint32_t bar_empty = bar_full + 8 * MAX_STAGES;
+    const uint32_t bar_done = bar_empty + 8 * MAX_STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ring_gen + p.stages * stage_bytes + 16 * MAX_STAGES + 8);
+    volatile uint32_t* abort_flag = tmem_slot + 1;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = (int)blockIdx.x % SPLIT;
+    const int n0 = ((int)blockIdx.x / SPLIT) * W_ROWS;
+    const int kb0 = (int)((long long)rank * p.g.k_blocks / SPLIT), kb1 = (int)((long long)(rank + 1) * p.g.k_blocks / SPLIT);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < p.stages; s++) {
+            mbar_init(bar_full + 8 * s, 1);
+            mbar_init(bar_empty + 8 * s, 1);
+        }
+        mbar_init(bar_done, 1);
+        *abort_flag = 0;
+        fence_mbar_init();
+    }
+    __syncwarp();
+    if (warp == 0) {
+        const int pf1 = min(kb1, kb0 + PREFETCH_BLOCKS);
+        for (int kb = kb0 + lane; kb < pf1; kb += 32) prefetch_l2_2d(&tmap_w, kb * BK, n0);
+        __syncwarp();
+    } else if (warp == 1) {
+        tmem_alloc(smem_u32(tmem_slot), p.tmem_cols);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    pdl_wait();
+    pdl_trigger();
+
+    if (warp == 0) {
+        const bool leader = elect_one();
+        int stage = 0;
+        uint32_t phase = 1;
+        for (int kb = kb0; kb < kb1; kb++) {
+            if (!mbar_wait(bar_empty + 8 * stage, phase, abort_flag, ST_TIMEOUT_PRODUCER)) break;
+            if (leader) {
+                const uint32_t fb = bar_full + 8 * stage, sw = ring + stage * stage_bytes;
+                mbar_arrive_expect_tx(fb, stage_bytes);   // parts of a box outside the matrix are zero-filled and counted
+                tma_load_2d(sw, &tmap_w, fb, kb * BK, n0);
+                tma_load_2d(sw + W_BYTES, &tmap_t, fb, kb * BK, 0);
+            }
+            __syncwarp();
+            if (++stage == p.stages) { stage = 0; phase ^= 1; }
+        }
+    } else if (warp == 1) {
+        const bool leader = elect_one();
+        int stage = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int kb = kb0; kb < kb1; kb++) {
+            if (!mbar_wait(bar_full + 8 * stage, phase, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t sw = ring + stage * stage_bytes;
+            const uint64_t wdesc = kmajor_desc_sw128(sw), tdesc = kmajor_desc_sw128(sw + W_BYTES);
+#pragma unroll
+            for (int k = 0; k < BK / 32; k++)
+                if (leader) mma_f8f6f4_ss(tmem, wdesc + 2 * k, tdesc + 2 * k, p.idesc, ((kb - kb0) | k) != 0);
+            if (leader) mma_commit(bar_empty + 8 * stage);
+            __syncwarp();
+            if (++stage == p.stages) { stage = 0; phase ^= 1; }
+        }
+        if (ok && leader) mma_commit(bar_done);
+        __syncwarp();
+    } else {
+        // accumulators -> shared memory, token-major ([token][128 weight rows] fp32): lanes write neighbouring words.  The
+        // ring is free by then: every load that was issued has been consumed by an MMA that has retired.
+        const int quad = warp & 3;
+        if (mbar_wait(bar_done, 0, abort_flag, ST_TIMEOUT_EPILOGUE)) {
+            tc_fence_after();
+            for (int j0 = 0; j0 < p.tn; j0 += 16) {
+                uint32_t acc[16];
+                tmem_ld_32x32b_x16(tmem + j0 + (uint32_t(quad * 32) << 16), acc);
+                tmem_ld_wait();
+                const uint32_t dst = ring + j0 * (W_ROWS * 4) + (quad * 32 + lane) * 4;
+#pragma unroll
+                for (int i = 0; i < 16; i++)
+                    asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + i * (W_ROWS * 4)), "r"(acc[i]) : "memory");
+            }
+        }
+        tc_fence_before();
+    }
+    __syncwarp();
+    cluster_sync_all();
+
+    {
+        // The CTAs of the cluster finish the tile's outputs together, blocks of THREADS groups of four outputs in turn.  A
+        // thread takes several groups at a time, all their loads (partial sums, and the residual stream in the accumulate
+        // mode) issued before the first use: one group at a time was bound by their latency (0.35 us a round, 16 rounds for 64
+        // tokens).
+        const GemmParams& g = p.g;
+        constexpr int STEP = SPLIT * THREADS;
+        float alpha = g.alpha;
+        if (g.scale_a) alpha *= ld_scalar(g.scale_a);
+        if (g.scale_b) alpha *= ld_scalar(g.scale_b);
+        const float scale_d = (g.D8 && g.scale_d) ? ld_scalar(g.scale_d) : 1.0f;
+        float tmax = 0.f;
+        if (g.H) {
+            // gate rows [64c, 64c + 32), up rows [64c + 32, 64c + 64) of the tile
+            constexpr int QUADS = W_ROWS / 8;   // groups of four activation columns
+            constexpr int U = SPLIT == 1 ? 4 : SPLIT == 2 ? 2 : 1;
+            const int items = g.M * QUADS;
+            for (int it0 = rank * THREADS + threadIdx.x; it0 < items; it0 += U * STEP) {
+                float4 gt[U][SPLIT], up[U][SPLIT];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int it = min(it0 + u * STEP, items - 1), j = it / QUADS, q = it % QUADS;
+                    const int row = (q >> 3) * 64 + (q & 7) * 4;
+                    gather<SPLIT>(gt[u], ring, j, row);
+                    gather<SPLIT>(up[u], ring, j, row + 32);
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int it = it0 + u * STEP, j = it / QUADS, q = it % QUADS;
+                    if (it >= items) break;
+                    const int col = (n0 >> 1) + q * 4;
+                    float gv[4], uv[4], h[4];
+                    add_up<SPLIT>(gt[u], gv);
+                    add_up<SPLIT>(up[u], uv);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const float a = gv[i] * alpha;
+                        float r;
+                        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + __expf(-a)));
+                        h[i] = a * r * (uv[i] * alpha);
+                    }
+                    const uint32_t w[2] = {pack_out(h[0], h[1], 1), pack_out(h[2], h[3], 1)};
+                    if (col >= g.F) continue;
+#pragma unroll
+                    for (int i = 0; i < 2; i++)   // max of the rounded values; columns past F are zero
+                        tmax = fmaxf(tmax, fmaxf(fabsf(__uint_as_float(w[i] << 16)), fabsf(__uint_as_float(w[i] & 0xffff0000u))));
+                    uint16_t* dst = reinterpret_cast<uint16_t*>(g.H) + (size_t)j * g.F + col;
+                    if (p.vec && col + 4 <= g.F) {
+                        *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 4; i++)
+                            if (col + i < g.F) dst[i] = (uint16_t)(w[i >> 1] >> (16 * (i & 1)));
+                    }
+                }
+            }
+        } else {
+            constexpr int QUADS = W_ROWS / 4;
+            constexpr int U = SPLIT <= 2 ? 4 : SPLIT <= 4 ? 2 : 1;
+            const int items = g.M * QUADS;
+            for (int it0 = rank * THREADS + threadIdx.x; it0 < items; it0 += U * STEP) {
+                float4 part[U][SPLIT];
+                float x[U][4];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int it = min(it0 + u * STEP, items - 1), j = it / QUADS, row = (it % QUADS) * 4, col = n0 + row;
+                    if (g.X) {
+                        const float* src = g.X + (size_t)j * g.N + col;
+                        if (p.vec && col + 4 <= g.N) {
+                            const float4 t = *reinterpret_cast<const float4*>(src);
+                            x[u][0] = t.x; x[u][1] = t.y; x[u][2] = t.z; x[u][3] = t.w;
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; i++) x[u][i] = col + i < g.N ? src[i] : 0.f;
+                        }
+                    }
+                    gather<SPLIT>(part[u], ring, j, row);
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int it = it0 + u * STEP, j = it / QUADS, row = (it % QUADS) * 4, col = n0 + row;
+                    if (it >= items) break;
+                    if (col >= g.N) continue;
+                    float v[4];
+                    add_up<SPLIT>(part[u], v);
+                    const size_t off = (size_t)j * g.N + col;
+                    const bool whole = p.vec && col + 4 <= g.N;
+                    if (g.X) {
+#pragma unroll
+                        for (int i = 0; i < 4; i++) v[i] = fmaf(v[i], alpha, x[u][i]);
+                        if (whole) {
+                            *reinterpret_cast<float4*>(g.X + off) = make_float4(v[0], v[1], v[2], v[3]);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; i++)
+                                if (col + i < g.N) g.X[off + i] = v[i];
+                        }
+                        continue;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; i++) v[i] *= alpha;
+                    if (g.D8) {
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            tmax = fmaxf(tmax, fabsf(v[i]));   // columns past N are zero
+                            v[i] *= scale_d;
+                        }
+                        const uint32_t w = pack_e4m3x4(v[0], v[1], v[2], v[3]);
+                        if (whole) {
+                            *reinterpret_cast<uint32_t*>(g.D8 + off) = w;
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; i++)
+                                if (col + i < g.N) g.D8[off + i] = (uint8_t)(w >> (8 * i));
+                        }
+                    } else {
+                        const uint32_t w[2] = {pack_out(v[0], v[1], g.out_bf16), pack_out(v[2], v[3], g.out_bf16)};
+                        uint16_t* dst = reinterpret_cast<uint16_t*>(g.C) + off;
+                        if (whole) {
+                            *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; i++)
+                                if (col + i < g.N) dst[i] = (uint16_t)(w[i >> 1] >> (16 * (i & 1)));
+                        }
+                    }
+                }
+            }
+        }
+        if (g.amax) {
+            __syncwarp();
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
+            if (lane == 0) atomicMax(reinterpret_cast<unsigned int*>(g.amax), __float_as_uint(tmax));
+        }
+    }
+    // ------------------------------------------------------------- teardown
+    __syncwarp();
+    cluster_sync_all();   // peers have read this CTA's partial sums
+    const uint32_t code = *abort_flag;
+    if (code != 0) {
+        if (threadIdx.x == 0) atomicCAS(&g_gemm_status, 0u, code);
+        for (int i = 0; i < 200; i++) __nanosleep(1000);   // copies in flight land before shared memory is released
+        __syncthreads();
+    }
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem, p.tmem_cols);
+    }
+}
+
+using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const Params);
+inline Kernel kernel_for(int split) {
+    static const Kernel table[MAX_SPLIT] = {fp8_gemm_skinny_kernel<1>, fp8_gemm_skinny_kernel<2>, fp8_gemm_skinny_kernel<3>, fp8_gemm_skinny_kernel<4>,
+                                            fp8_gemm_skinny_kernel<5>, fp8_gemm_skinny_kernel<6>, fp8_gemm_skinny_kernel<7>, fp8_gemm_skinny_kernel<8>};
+    return table[split - 1];
+}
+
+// clusters of each size that are resident at once with one CTA to an SM (a cluster stays inside one group of SMs, so this
+// is less than SMs / size); with two CTAs to an SM it is at least twice as many
+struct Fit {
+    int one[MAX_SPLIT + 1] = {};
+};
+
+inline void configure(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int tiles, int split, size_t smem, cudaStream_t stream) {
+    cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles * split));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)split;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+}
+
+inline cudaError_t init(Fit* fit) {
+    for (int split = 1; split <= MAX_SPLIT; split++) {
+        cudaError_t e = cudaFuncSetAttribute(kernel_for(split), cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_ONE);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel_for(split), cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr[2];
+        configure(cfg, attr, 1, split, SMEM_ONE, nullptr);
+        cfg.numAttrs = 1;
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fit->one[split], kernel_for(split), &cfg);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+// How a problem is cut, or split = 0 where the square kernel is the faster one.
+struct Plan {
+    int split = 0;
+    bool two = false;   // two CTAs to an SM, each with half of its shared memory
+};
+inline Plan plan(int M, int N, int K, int num_sms, const Fit& fit) {
+    Plan r;
+    if (M > MAX_TOKENS) return r;
+    const long long weights = (long long)N * K;
+    const long long tiles = ((long long)N + W_ROWS - 1) / W_ROWS;
+    const int k_blocks = (K + BK - 1) / BK, tn = (M + 15) / 16 * 16;
+    // Past 80 tokens the tokens' own traffic and the longer finish (2 us more at 128) weigh against a square kernel that
+    // needs one row of tiles: 4096 x 4096, 112 tokens 8.4 / 8.0 us, but 8192 x 8192 16.2 / 17.1.  Past 128 that one reads
+    // the weight twice: 144 tokens, 4096 x 4096 8.7 / 10.1 us, 2048 x 2048 6.3 / 6.2.
+    if (M > 80 && weights < (M > 128 ? 1ll << 24 : 1ll << 25)) return r;
+    // the K range is cut as long as all slices are resident, one to an SM, and two k-blocks are left to each (16 tokens, 1 / 2 /
+    // 3 / 4 slices: 8192 x 8192 17.4 / 13.9 / 14.8 / 13.7 us, of which 2 fit; 4096 x 4096 9.9 / 7.0 / 6.3 / 6.2);
+    // past four slices the finish grows faster than the stream shrinks, unless less than three fifths of the SMs are in use and
+    // the slices are long (4 / more: 2048 x 2048 3.9 / 4.5, 3000 x 8000 8.0 / 8.4, but 2048 x 8192 6.7 / 5.9)
+    int split = tiles <= fit.one[1] ? 1 : 0;
+    for (int s = 2; s <= MAX_SPLIT; s++)
+        if (split > 0 && tiles <= fit.one[s] && (s <= 4 ? k_blocks >= 2 * s : k_blocks >= 10 * s && 20 * tiles < 3 * num_sms)) split = s;
+    if (split > 0 && 4 * tiles * split >= 3 * num_sms) { r.split = split; return r; }
+    // Too few CTAs that way (or more tiles than SMs): two to an SM.  Four stages and the partial sums have to fit in half of
+    // its shared memory (80 tokens), and with fewer than one and a half CTAs per SM the imbalance costs what the spread
+    // gains (16 tokens: 11008 x 4096 3 slices 10.3 us / 1 slice 12.2, 12288 x 4096 2 slices 12.1 / 12.4).
+    const bool half_fits = 4 * (W_BYTES + tn * BK) <= SMEM_TWO - TAIL_BYTES && tn * W_ROWS * 4 <= SMEM_TWO - TAIL_BYTES;
+    if (half_fits && split > 0 && k_blocks >= 24)
+        for (int s = 4; s > split; s--)
+            if (tiles <= 2 * fit.one[s] && 2 * tiles * s >= 3 * num_sms) { r.split = s; r.two = true; return r; }
+    if (split > 0) {
+        // a third of the SMs idle: still ahead of the square kernel up to 48 tokens (12288 x 4096, 40 / 64 / 96 tokens: 12.8 / 13.4 /
+        // 13.8 us against 13.2 / 13.2 / 13.4), or where that one reads the weight twice
+        if (M <= 48 || M > 128 || 4 * tiles < num_sms) r.split = split;
+        return r;
+    }
+    // More tiles than SMs: in one wave of two to an SM, unless only a few SMs would get a second one (16 tokens: 172 tiles
+    // of K = 4096 22.8 us against 25.4, 256 tiles 22.9 against 25.2; 157 tiles 20.0 against 19.7, 512 tiles 44.9 against 45.7)
+    if (half_fits && M <= 64 && tiles <= 2 * fit.one[1] && 8 * tiles >= 9 * num_sms) { r.split = 1; r.two = true; }
+    return r;
+}
+
+// A: tokens [M, K], B: weights [N, K]; g is complete but for k_blocks
+inline int launch(GemmParams g, const Plan& plan, const void* A, const void* B, cudaStream_t stream) {
+    Params p;
+    g.k_blocks = (g.K + BK - 1) / BK;
+    p.tn = (g.M + 15) / 16 * 16;
+    p.tmem_cols = 32;
+    while (p.tmem_cols < p.tn) p.tmem_cols *= 2;
+    p.idesc = make_idesc_e4m3_f32(W_ROWS, p.tn, 0, 0);
+    const int tiles = (g.N + W_ROWS - 1) / W_ROWS;
+    const int stage_bytes = W_BYTES + p.tn * BK, part_bytes = p.tn * W_ROWS * 4;
+    const int slice = (g.k_blocks + plan.split - 1) / plan.split;
+    p.stages = ((plan.two ? SMEM_TWO : SMEM_ONE) - TAIL_BYTES) / stage_bytes;
+    if (p.stages > slice) p.stages = slice;
+    if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
+    int ring_bytes = p.stages * stage_bytes;
+    while (ring_bytes < part_bytes) { p.stages++; ring_bytes += stage_bytes; }   // the partial sums take the ring's place
+    p.vec = g.H ? (g.F % 4 == 0 && (reinterpret_cast<uintptr_t>(g.H) & 7) == 0)
+          : g.X ? (g.N % 4 == 0 && (reinterpret_cast<uintptr_t>(g.X) & 15) == 0)
+          : g.D8 ? (g.N % 4 == 0 && (reinterpret_cast<uintptr_t>(g.D8) & 3) == 0)
+                 : (g.N % 4 == 0 && (reinterpret_cast<uintptr_t>(g.C) & 7) == 0);
+    p.g = g;
+    CUtensorMap tw, tt;
+    if (!make_tmap_u8_2d(&tw, B, (uint64_t)g.N, (uint64_t)g.K, W_ROWS, BK, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !make_tmap_u8_2d(&tt, A, (uint64_t)g.M, (uint64_t)g.K, (uint32_t)p.tn, BK, CU_TENSOR_MAP_SWIZZLE_128B))
+        return (int)cudaErrorInvalidValue;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[2];
+    configure(cfg, attr, tiles, plan.split, (size_t)ring_bytes + TAIL_BYTES, stream);
+    return (int)cudaLaunchKernelEx(&cfg, kernel_for(plan.split), tw, tt, p);
+}
+
+}  // namespace skinny

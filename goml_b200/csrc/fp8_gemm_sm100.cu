@@ -24,6 +24,7 @@
 #include <mutex>
 
 #include "../../include/fp8_gemm.h"
+#include "pdl.cuh"
 #include "sm100_ptx.cuh"
 #include "tmap.cuh"
 
@@ -594,6 +595,8 @@ fp8_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     }
 }
 
+#include "fp8_gemm_skinny.cuh"
+
 __global__ void __launch_bounds__(32) gemm_wait_expiry_selftest_kernel() {
     wait_expiry_selftest_body(&g_gemm_status, ST_TIMEOUT_SELFTEST);
 }
@@ -606,6 +609,7 @@ struct DeviceState {
     std::once_flag once;      // first call on this device, from whichever host thread gets there first
     cudaError_t init_error = cudaSuccess;
     int num_sms = 0;
+    skinny::Fit skinny_fit;   // read-only after init
 };
 constexpr int MAX_DEVICES = 64;
 DeviceState g_dev[MAX_DEVICES];
@@ -637,6 +641,7 @@ void init_device(DeviceState* st, int dev) {
                                   Tile<128>::SMEM_BYTES)) != cudaSuccess) { st->init_error = e; return; }
     if ((e = cudaFuncSetAttribute(fp8_gemm_tcgen05_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   Tile<64>::SMEM_BYTES)) != cudaSuccess) { st->init_error = e; return; }
+    if ((e = skinny::init(&st->skinny_fit)) != cudaSuccess) { st->init_error = e; return; }
     st->num_sms = sms;
 }
 
@@ -659,6 +664,16 @@ int launch(int M, int N, int K, const void* A, const void* B, void* C, float alp
     DeviceState& st = g_dev[dev];
     std::call_once(st.once, init_device, &st, dev);
     if (st.init_error != cudaSuccess) return (int)st.init_error;
+
+    GemmParams p{};
+    p.M = M; p.N = N; p.K = K; p.C = C;
+    p.alpha = alpha; p.scale_a = sa; p.scale_b = sb; p.out_bf16 = out_bf16;
+    p.X = X;
+    p.H = H; p.F = F; p.amax = amax;
+    p.D8 = D8; p.scale_d = scale_d;
+    // few rows of A: a kernel of its own, without tile pairs or their policy
+    const skinny::Plan few = skinny::plan(M, N, K, st.num_sms, st.skinny_fit);
+    if (few.split > 0) return skinny::launch(p, few, A, B, stream);
 
     // Tile width: 256 unless a narrower tile cuts (waves x per-k-block MMA time) by more than a quarter —
     // i.e. only when the 128x256 tiling leaves most SMs idle (small or skinny problems).  Per-k-block MMA
@@ -695,12 +710,6 @@ int launch(int M, int N, int K, const void* A, const void* B, void* C, float alp
         const long long pair_cost = ((pairs + st.num_sms - 1) / st.num_sms) * 2 * 92;
         if (pair_cost > single_cost) pair = false;
     }
-    GemmParams p;
-    p.M = M; p.N = N; p.K = K; p.C = C;
-    p.alpha = alpha; p.scale_a = sa; p.scale_b = sb; p.out_bf16 = out_bf16;
-    p.X = X;
-    p.H = H; p.F = F; p.amax = amax;
-    p.D8 = D8; p.scale_d = scale_d;
     p.x_tma = (X && (N % 4) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0) ? 1 : 0;
     p.c_tma = (C && !X && !H && !D8 && (N % 8) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) ? 1 : 0;
     p.h_tma = (H && bn >= 128 && (F % 8) == 0 && (reinterpret_cast<uintptr_t>(H) & 15) == 0) ? 1 : 0;

@@ -351,3 +351,44 @@ def test_skinny_shapes_in_full(cuda, built_libs, M):
     rms = float(np.sqrt(np.mean(ref ** 2)))
     err = np.abs(x.double().cpu().numpy() - (x0.double().cpu().numpy() + ref)).max()
     assert err <= 1e-5 * max(rms, 1.0) * np.sqrt(K), err
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 16), (1, 1003, 144), (15, 4096, 512), (16, 5000, 1040), (17, 2048, 10256), (33, 11008, 3088),
+                                   (64, 21440, 256), (65, 512, 4112), (80, 130, 2064), (96, 8192, 4096), (128, 8192, 4096), (129, 4099, 4096),
+                                   (173, 12288, 2048), (192, 8200, 2064), (193, 4096, 4096)])
+def test_few_rows_exact_on_integer_data(cuda, built_libs, M, N, K):
+    # every way the few-row kernel cuts a problem (1 to 7 slices of K, one or two CTAs to an SM, ragged M, N and K, the rows
+    # just past its range).  Codes of small integers: products and sums are exact in fp32 whatever their order, so the
+    # accumulate mode has to match to the bit and the 16-bit output to its one rounding; stores stay inside the matrix.
+    from goml_b200 import fp8_gemm as G
+    rng = np.random.default_rng(M + N + K)
+    vals = np.array([0x00, 0x38, 0xB8, 0x40, 0xC0, 0x44], np.uint8)       # 0, 1, -1, 2, -2, 3
+    a, b = vals[rng.integers(0, 6, (M, K))], vals[rng.integers(0, 6, (N, K))]
+    ad, bd = dev_u8(a), dev_u8(b)
+    f = lambda t: t.view(torch.float8_e4m3fn).double()
+    ref = f(ad) @ f(bd).t()
+    for shift in (0, 1):     # an output that starts one element off takes the element-wise stores
+        c = torch.full((M * N + 16,), 7.0, dtype=torch.bfloat16, device="cuda")
+        x = torch.full((M * N + 16,), 3.0, dtype=torch.float32, device="cuda")
+        G.FP8GEMMScaled(M, N, K, ad.data_ptr(), bd.data_ptr(), c.data_ptr() + 2 * (8 + shift), 0.5, 0, 0, G.OutBF16, 0)
+        G.FP8GEMMAccumulateF32(M, N, K, ad.data_ptr(), bd.data_ptr(), x.data_ptr() + 4 * (4 + shift), 0.5, 0, 0)
+        torch.cuda.synchronize()
+        assert G.device_status() == 0
+        lo, n = 8 + shift, M * N
+        assert torch.equal(c[lo:lo + n].view(M, N), (ref * 0.5).to(torch.bfloat16))
+        assert torch.all(c[:lo] == 7.0) and torch.all(c[lo + n:] == 7.0)
+        lo = 4 + shift
+        assert torch.equal(x[lo:lo + n].view(M, N), (ref * 0.5 + 3.0).float())
+        assert torch.all(x[:lo] == 3.0) and torch.all(x[lo + n:] == 3.0)
+    if N % 64 == 0:
+        F = N // 2 - 3       # the last group of 32 activation columns is a ragged one
+        h = torch.full((M, F), 7.0, dtype=torch.bfloat16, device="cuda")
+        amax = torch.full((1,), 99.0, device="cuda")
+        G.FP8GEMMSwiGLU(M, F, K, ad.data_ptr(), bd.data_ptr(), h.data_ptr(), 2.0 ** -6, 0, 0, amax.data_ptr(), 0)
+        torch.cuda.synchronize()
+        gu = (ref * 2.0 ** -6).view(M, N // 64, 2, 32)
+        g, u = gu[:, :, 0].reshape(M, -1)[:, :F], gu[:, :, 1].reshape(M, -1)[:, :F]
+        want = g / (1 + torch.exp(-g)) * u
+        # one bf16 rounding of a value whose exponential and reciprocal are good to a few fp32 ulp
+        assert torch.all((h.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6)
+        assert amax.item() == h.float().abs().max().item()
