@@ -45,7 +45,9 @@ def _init():
             for name, args in {
                 "fp8_rope_table": [p, p, i, i, f, p],
                 "fp8_rmsnorm_quantize": [p, p, p, p, p, p, p, p, i, i, f, p],
+                "fp8_rmsnorm_quantize_into": [p, p, p, p, p, p, p, p, i, i, f, p],
                 "fp8_rope_quantize_qkv": [p, p, p, p, p, p, p, p, i, i, i, i, p],
+                "fp8_rope_quantize_qkv_cache": [p, p, p, p, p, p, p, p, p, p, p, p, i, i, i, i, i, p],
                 "fp8_permute_quantize_heads": [p, p, p, p, i, i, i, i, p],
                 "fp8_swiglu_quantize": [p, p, p, p, i, i, p],
                 "fp8_quantize_bf16": [p, p, p, p, z, p],
@@ -74,10 +76,26 @@ def RMSNormQuantize(x: int, residual_bf16: int, h_out: int, gamma: int, q: int, 
                                                                 rows, hidden, eps, stream or None))
 
 
+def RMSNormQuantizeInto(x: int, h_out: int, gamma: int, q: int, scale: int, amax: int, rstd_ws: int, zero_word: int,
+                        rows: int, hidden: int, eps: float, stream: int = 0) -> None:
+    """RMSNormQuantize without a residual; h_out (0: none) receives a copy of x, *zero_word (0: none) is set to 0."""
+    _check("fp8_rmsnorm_quantize_into", _init().fp8_rmsnorm_quantize_into(x, h_out or None, gamma, q, scale, amax, rstd_ws, zero_word or None,
+                                                                          rows, hidden, eps, stream or None))
+
+
 def RopeQuantizeQKV(qkv_bf16: int, cos: int, sin: int, q: int, k: int, v: int, scales: int, amaxes: int,
                     batch: int, seq_len: int, heads: int, head_dim: int, stream: int = 0) -> None:
     _check("fp8_rope_quantize_qkv", _init().fp8_rope_quantize_qkv(qkv_bf16, cos, sin, q, k, v, scales, amaxes, batch, seq_len, heads,
                                                                   head_dim, stream or None))
+
+
+def RopeQuantizeQKVCache(qkv_bf16: int, cos: int, sin: int, q: int, k: int, v: int, scales: int, amaxes: int, k_cache: int, v_cache: int,
+                         cache_scales: int, cache_lens: int, batch: int, seq_len: int, s_max: int, heads: int, head_dim: int,
+                         stream: int = 0) -> None:
+    """RopeQuantizeQKV that also stores the K and V codes, their scales and the lengths into a KV cache."""
+    _check("fp8_rope_quantize_qkv_cache", _init().fp8_rope_quantize_qkv_cache(qkv_bf16, cos, sin, q, k, v, scales, amaxes, k_cache, v_cache,
+                                                                              cache_scales, cache_lens, batch, seq_len, s_max, heads,
+                                                                              head_dim, stream or None))
 
 
 def PermuteQuantizeHeads(o_fp16: int, q: int, scale: int, amax: int, batch: int, seq_len: int, heads: int, head_dim: int,

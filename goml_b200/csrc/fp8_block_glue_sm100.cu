@@ -2,7 +2,8 @@
 // residual add of a Llama-style decoder block, each fused with the per-tensor e4m3 quantiser that
 // feeds the FP8 GEMM / FP8 attention libraries.
 //
-// All of it is HBM-bound row-local work.  Every op runs as two kernels on the caller's stream: pass 1
+// All of it is row-local work.  A small tensor is done by one cluster in one kernel (one_cluster.cuh).  For a larger one
+// the op is HBM-bound and runs as two kernels on the caller's stream: pass 1
 // reduces the per-tensor amax of the op's fp32 result (one atomicMax per CTA), pass 2 recomputes the
 // result and writes codes.  Nothing intermediate is stored, so the traffic per op is
 // 2 x (input bytes) + 1 byte per output element.  Pass 2 walks the tensor backwards, so it starts on the part
@@ -13,8 +14,11 @@
 #include <stdint.h>
 
 #include "../../include/fp8_block.h"
+#include "one_cluster.cuh"
 
 namespace {
+
+using namespace sm100;
 
 constexpr int THREADS = 256;
 
@@ -39,18 +43,11 @@ struct FastDiv {
         r = n - q * d;
     }
 };
-// 256-bit global loads (sm_100): one instruction per 16 bf16 / 8 fp32 values, 32-byte aligned addresses
+// 256-bit global loads (sm_100): one instruction per 16 bf16 / 8 fp32 values, 32-byte aligned addresses.  Coherent ones:
+// see one_cluster.cuh, and the residual stream is updated in place
 struct U8 {
     uint32_t v[8];
 };
-__device__ __forceinline__ U8 ldg256(const void* p) {
-    U8 r;
-    asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7])
-                 : "l"(p));
-    return r;
-}
-// same through the coherent path: for buffers the kernel also writes (the residual stream updated in place)
 __device__ __forceinline__ U8 ld256(const void* p) {
     U8 r;
     asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -116,17 +113,6 @@ __device__ __forceinline__ float block_max(float m, float* sh) {
     for (int w = 1; w < THREADS / 32; w++) m = fmaxf(m, sh[w]);
     return m;
 }
-__device__ __forceinline__ float block_sum(float s, float* sh) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-    __syncthreads();
-    s = sh[0];
-#pragma unroll
-    for (int w = 1; w < THREADS / 32; w++) s += sh[w];  // fixed order: the same in every CTA
-    return s;
-}
 // non-negative floats order like their bit patterns
 __device__ __forceinline__ void atomic_amax(float* amax, float m) { atomicMax(reinterpret_cast<unsigned int*>(amax), __float_as_uint(m)); }
 
@@ -141,6 +127,24 @@ int grid_for(size_t items) {
 }
 bool misaligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; }
 bool misaligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31) != 0; }  // operands of 256-bit loads
+
+// Input bytes up to which one cluster does an op.  Rows of 4096 values (32 heads of 128), one cluster, or two kernels behind
+// a clearing one as overlapped launches (behind a memset and in turn, as it was: 8.3 / 8.5 / 7.0 us at every size here):
+// RMSNorm 1 / 16 / 40 rows 3.9 / 4.1 / 5.7 us, two kernels 4.1 from 42 rows on; RoPE of Q, K and V 1 / 16 rows 4.3 / 5.2 us, two
+// kernels 5.4 at 20; head permute 1 / 40 / 128 rows 2.2 / 3.2 / 4.7 us, two kernels 3.5 at 130.  One launch also costs the host a
+// third of three.
+constexpr size_t OC_BYTES_RMS = 320 << 10;
+constexpr size_t OC_BYTES_QKV = 448 << 10;
+constexpr size_t OC_BYTES_DEC = 448 << 10;
+constexpr size_t OC_BYTES_O = 512 << 10;
+
+// sets the maxima of an op to zero ahead of its pass 1 (a kernel and not a memset: it takes part in the overlapped launches)
+__global__ void clear_words_kernel(float* w, int n) {
+    pdl_wait();
+    pdl_trigger();
+    if ((int)threadIdx.x < n) w[threadIdx.x] = 0.f;
+}
+cudaError_t clear_words(float* w, int n, cudaStream_t s) { return launch_pdl(clear_words_kernel, dim3(1), dim3(32), 0, s, w, n); }
 
 // ---------------------------------------------------------------------------------- RoPE table
 __global__ void rope_table_kernel(float* cos_out, float* sin_out, int seq_len, int half, double theta, double hd) {
@@ -158,7 +162,7 @@ __global__ void rope_table_kernel(float* cos_out, float* sin_out, int seq_len, i
 // ---------------------------------------------------------------------------------- RMSNorm (+ residual) + quantise
 // h = x (+ residual) for 4 consecutive elements
 __device__ __forceinline__ float4 load_h4(const float* x, const uint16_t* res, size_t off) {
-    float4 h = *reinterpret_cast<const float4*>(x + off);
+    float4 h = ld128f(x + off);
     if (res) {
         const uint2 r = *reinterpret_cast<const uint2*>(res + off);
         h.x += __uint_as_float(r.x << 16);
@@ -195,18 +199,18 @@ __device__ __forceinline__ void block_sum_max(float& s, float& m, float* sh) {  
 }
 
 // pass 1, any hidden (multiple of 16): one CTA per row (grid-stride): h_out, rstd per row, amax
-__global__ void __launch_bounds__(THREADS) rms_stats_kernel(const float* __restrict__ x, const uint16_t* __restrict__ res,
-                                                            float* h_out, const float* __restrict__ gamma,
-                                                            float* __restrict__ rstd_ws, float* amax, int rows, int hidden,
-                                                            float eps) {
+__global__ void __launch_bounds__(THREADS) rms_stats_kernel(const float* x, const uint16_t* res, float* h_out, const float* gamma,
+                                                            float* rstd_ws, float* amax, int rows, int hidden, float eps) {
     __shared__ float sh[2 * THREADS / 32];
+    pdl_wait();
+    pdl_trigger();
     float run_max = 0.f;
     for (int row = blockIdx.x; row < rows; row += gridDim.x) {
         const size_t base = (size_t)row * hidden;
         float ss = 0.f, m1 = 0.f;
         for (int c = threadIdx.x * 4; c < hidden; c += THREADS * 4) {
             const float4 h = load_h4(x, res, base + c);
-            if (res && h_out) *reinterpret_cast<float4*>(h_out + base + c) = h;
+            if (h_out) *reinterpret_cast<float4*>(h_out + base + c) = h;
             const float4 g = *reinterpret_cast<const float4*>(gamma + c);
             ss = fmaf(h.x, h.x, ss);
             ss = fmaf(h.y, h.y, ss);
@@ -242,19 +246,21 @@ __device__ __forceinline__ void load_row(RowRegs<N, HAS_RES>& t, const float* x,
     for (int k = 0; k < N; k++) {
         const size_t off = base + (size_t)k * (THREADS * 8) + threadIdx.x * 8;
         t.x[k] = ld256(x + off);
-        if (HAS_RES) t.r[k] = __ldg(reinterpret_cast<const uint4*>(res + off));
+        if (HAS_RES) t.r[k] = ld128(res + off);
     }
 }
 template <int N, bool HAS_RES>
-__global__ void __launch_bounds__(THREADS) rms_stats_regs_kernel(const float* __restrict__ x, const uint16_t* __restrict__ res, float* h_out,
-                                                                 const float* __restrict__ gamma, float* __restrict__ rstd_ws, float* amax,
+__global__ void __launch_bounds__(THREADS) rms_stats_regs_kernel(const float* x, const uint16_t* res, float* h_out,
+                                                                 const float* gamma, float* rstd_ws, float* amax,
                                                                  int rows, float eps) {
     constexpr int hidden = N * THREADS * 8;
     __shared__ float sh[2 * THREADS / 32];
+    pdl_wait();
+    pdl_trigger();
     float run_max = 0.f;
     U8 g[N];
 #pragma unroll
-    for (int k = 0; k < N; k++) g[k] = ldg256(gamma + k * (THREADS * 8) + threadIdx.x * 8);
+    for (int k = 0; k < N; k++) g[k] = ld256(gamma + k * (THREADS * 8) + threadIdx.x * 8);
     RowRegs<N, HAS_RES> cur, nxt;
     int row = blockIdx.x;
     if (row < rows) load_row<N, HAS_RES>(cur, x, res, (size_t)row * hidden);
@@ -275,7 +281,7 @@ __global__ void __launch_bounds__(THREADS) rms_stats_regs_kernel(const float* __
                 ss = fmaf(h, h, ss);
                 m1 = fmaxf(m1, fabsf(__fmul_rn(h, __uint_as_float(g[k].v[i]))));
             }
-            if (HAS_RES && h_out) st256(h_out + (size_t)row * hidden + (size_t)k * (THREADS * 8) + threadIdx.x * 8, o);
+            if (h_out) st256(h_out + (size_t)row * hidden + (size_t)k * (THREADS * 8) + threadIdx.x * 8, o);
         }
         block_sum_max(ss, m1, sh);
         const float rstd = __frsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)hidden), eps));
@@ -287,12 +293,12 @@ __global__ void __launch_bounds__(THREADS) rms_stats_regs_kernel(const float* __
 }
 
 // pass 2: 16 elements per thread per step
-__global__ void __launch_bounds__(THREADS) rms_quant_kernel(const float* __restrict__ h_src, const uint16_t* __restrict__ res,
-                                                            const float* __restrict__ gamma, const float* __restrict__ rstd_ws,
-                                                            const float* __restrict__ amax_ptr, float* scale_out,
-                                                            uint8_t* __restrict__ q, uint32_t items, int hidden,
-                                                            const FastDiv per_row) {
-    const float scale = scale_from_amax(*amax_ptr);
+__global__ void __launch_bounds__(THREADS) rms_quant_kernel(const float* h_src, const uint16_t* res, const float* gamma, const float* rstd_ws,
+                                                            const float* amax_ptr, float* scale_out, uint8_t* q, uint32_t items,
+                                                            int hidden, const FastDiv per_row) {
+    pdl_wait();
+    pdl_trigger();
+    const float scale = scale_from_amax(ld_f32(amax_ptr));
     const float inv = __fdiv_rn(1.0f, scale);
     if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = scale;
     // two items per step, all loads issued before the first use: twice the bytes in flight per thread
@@ -309,11 +315,11 @@ __global__ void __launch_bounds__(THREADS) rms_quant_kernel(const float* __restr
             per_row.divmod(items - 1 - (live[u] ? i : it), row[u], c[u]);  // backwards: the rows pass 1 finished with are still in L2
             c[u] *= 16;
             const size_t off = (size_t)row[u] * hidden + c[u];
-            hv[u][0] = ldg256(h_src + off);
-            hv[u][1] = ldg256(h_src + off + 8);
-            gv[u][0] = ldg256(gamma + c[u]);
-            gv[u][1] = ldg256(gamma + c[u] + 8);
-            rstd[u] = rstd_ws[row[u]];
+            hv[u][0] = ld256(h_src + off);
+            hv[u][1] = ld256(h_src + off + 8);
+            gv[u][0] = ld256(gamma + c[u]);
+            gv[u][1] = ld256(gamma + c[u] + 8);
+            rstd[u] = ld_f32(rstd_ws + row[u]);
         }
 #pragma unroll
         for (int u = 0; u < 2; u++) {
@@ -333,6 +339,135 @@ __global__ void __launch_bounds__(THREADS) rms_quant_kernel(const float* __restr
         }
     }
 }
+
+// both passes in one cluster: a row belongs to a group of 16, 4 or 1 warps of one CTA, the same in both passes
+struct RmsOp {
+    static constexpr int N = 1;
+    const float* x;
+    const uint16_t* res;
+    float* h_out;   // nullptr: h is not stored
+    const float* gamma;
+    uint8_t* q;
+    float* scale_out;
+    float* amax_out;
+    float* rstd_ws;
+    float* zero_word;
+    int rows, hidden;
+    float eps;
+    int lw;         // log2 of the warps per row
+
+    // h of 16 consecutive elements; from_h: pass 1 has stored them
+    __device__ __forceinline__ void load16(size_t off, bool from_h, float* h) const {
+        const float* src = from_h ? h_out : x;
+        const U8 a = ld256(src + off), b = ld256(src + off + 8);
+        uint4 r0 = make_uint4(0, 0, 0, 0), r1 = r0;
+        const bool add = res && !from_h;
+        if (add) {
+            r0 = ld128(res + off);
+            r1 = ld128(res + off + 8);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            h[i] = __uint_as_float(a.v[i]);
+            h[8 + i] = __uint_as_float(b.v[i]);
+        }
+        if (add) {
+            float rf[16];
+            bf16x8_to_f32(r0, rf);
+            bf16x8_to_f32(r1, rf + 8);
+#pragma unroll
+            for (int i = 0; i < 16; i++) h[i] += rf[i];
+        }
+    }
+    __device__ __forceinline__ int row_of(int it) const {   // neighbouring rows go to different CTAs
+        const int groups = (OC_THREADS / 32) >> lw, g = (int)(threadIdx.x >> 5) >> lw;
+        return (it * groups + g) * OC_CTAS + oc_rank();
+    }
+    __device__ __forceinline__ int rounds() const {
+        const int per_round = ((OC_THREADS / 32) >> lw) * OC_CTAS;
+        return (rows + per_round - 1) / per_round;
+    }
+    __device__ void pass1(float (&m)[1]) const {
+        __shared__ float2 part[2][OC_THREADS / 32];
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpr = 1 << lw, wi = warp & (wpr - 1);
+        if (zero_word && oc_tid() == 0) *zero_word = 0.f;
+        const int n = rounds();
+        for (int it = 0; it < n; it++) {
+            const int row = row_of(it);
+            float ss = 0.f, m1 = 0.f;
+            if (row < rows) {
+                const size_t base = (size_t)row * hidden;
+#pragma unroll 2
+                for (int c = (wi * 32 + lane) * 16; c < hidden; c += wpr * 512) {
+                    float h[16];
+                    load16(base + c, false, h);
+                    const U8 g0 = ld256(gamma + c), g1 = ld256(gamma + c + 8);
+                    if (h_out) {
+                        U8 o0, o1;
+#pragma unroll
+                        for (int i = 0; i < 8; i++) {
+                            o0.v[i] = __float_as_uint(h[i]);
+                            o1.v[i] = __float_as_uint(h[8 + i]);
+                        }
+                        st256(h_out + base + c, o0);
+                        st256(h_out + base + c + 8, o1);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 16; i++) {
+                        ss = fmaf(h[i], h[i], ss);
+                        m1 = fmaxf(m1, fabsf(__fmul_rn(h[i], __uint_as_float(i < 8 ? g0.v[i & 7] : g1.v[i & 7]))));
+                    }
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+            }
+            if (lw > 0) {   // uniform: every warp takes every round
+                if (lane == 0) part[it & 1][warp] = make_float2(ss, m1);
+                __syncthreads();
+                ss = 0.f;
+                for (int w = 0; w < wpr; w++) {
+                    const float2 t = part[it & 1][warp - wi + w];
+                    ss += t.x;
+                    m1 = fmaxf(m1, t.y);
+                }
+            }
+            const float rstd = __frsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)hidden), eps));
+            if (row < rows) {
+                if (wi == 0 && lane == 0) rstd_ws[row] = rstd;
+                m[0] = fmaxf(m[0], __fmul_rn(m1, rstd));
+            }
+        }
+    }
+    __device__ void pass2(const float (&m)[1]) const {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpr = 1 << lw, wi = warp & (wpr - 1);
+        const float scale = scale_from_amax(m[0]);
+        const float inv = __fdiv_rn(1.0f, scale);
+        if (oc_tid() == 0) {
+            *scale_out = scale;
+            *amax_out = m[0];
+        }
+        const int n = rounds();
+        for (int it = 0; it < n; it++) {
+            const int row = row_of(it);
+            if (row >= rows) continue;
+            const size_t base = (size_t)row * hidden;
+            const float rstd = ld_f32(rstd_ws + row);
+#pragma unroll 2
+            for (int c = (wi * 32 + lane) * 16; c < hidden; c += wpr * 512) {
+                float h[16], y[16];
+                load16(base + c, h_out != nullptr, h);
+                const U8 g0 = ld256(gamma + c), g1 = ld256(gamma + c + 8);
+#pragma unroll
+                for (int i = 0; i < 16; i++) y[i] = __fmul_rn(__fmul_rn(h[i], __uint_as_float(i < 8 ? g0.v[i & 7] : g1.v[i & 7])), rstd);
+                *reinterpret_cast<uint4*>(q + base + c) = quant16(y, inv);
+            }
+        }
+    }
+};
 
 // ---------------------------------------------------------------------------------- RoPE + permute + quantise of Q, K, V
 // One item = 32 elements of one (token, tensor, head): for Q and K the 16 rotation pairs
@@ -358,29 +493,29 @@ __device__ __forceinline__ QkvItem decode_qkv(uint32_t it, const QkvDivs& dv) {
     return r;
 }
 // y[0..15] = first-half results (or V elements 0..15), y[16..31] = second-half results (or V 16..31)
-__device__ __forceinline__ void qkv_values(const uint16_t* __restrict__ qkv, const float* __restrict__ cos_tab,
-                                           const float* __restrict__ sin_tab, const QkvItem& t, int seq_len, int heads, int hd,
+__device__ __forceinline__ void qkv_values(const uint16_t* qkv, const float* cos_tab, const float* sin_tab,
+                                           const QkvItem& t, int seq_len, int heads, int hd,
                                            float* y) {
     const int half = hd / 2;
     const size_t row = ((size_t)t.b * seq_len + t.s) * 3 * heads * hd + ((size_t)t.which * heads + t.h) * hd;
     if (t.which == 2) {
         const uint4* src = reinterpret_cast<const uint4*>(qkv + row + 32 * t.c);
 #pragma unroll
-        for (int v = 0; v < 4; v++) bf16x8_to_f32(__ldg(src + v), y + 8 * v);
+        for (int v = 0; v < 4; v++) bf16x8_to_f32(ld128(src + v), y + 8 * v);
         return;
     }
     float x0[16], x1[16];
     const uint4* s0 = reinterpret_cast<const uint4*>(qkv + row + 16 * t.c);
     const uint4* s1 = reinterpret_cast<const uint4*>(qkv + row + half + 16 * t.c);
-    bf16x8_to_f32(__ldg(s0), x0);
-    bf16x8_to_f32(__ldg(s0 + 1), x0 + 8);
-    bf16x8_to_f32(__ldg(s1), x1);
-    bf16x8_to_f32(__ldg(s1 + 1), x1 + 8);
+    bf16x8_to_f32(ld128(s0), x0);
+    bf16x8_to_f32(ld128(s0 + 1), x0 + 8);
+    bf16x8_to_f32(ld128(s1), x1);
+    bf16x8_to_f32(ld128(s1 + 1), x1 + 8);
     const float4* ct = reinterpret_cast<const float4*>(cos_tab + (size_t)t.s * half + 16 * t.c);
     const float4* st = reinterpret_cast<const float4*>(sin_tab + (size_t)t.s * half + 16 * t.c);
 #pragma unroll
     for (int v = 0; v < 4; v++) {
-        const float4 c4 = __ldg(ct + v), s4 = __ldg(st + v);
+        const float4 c4 = ld128f(ct + v), s4 = ld128f(st + v);
         const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
 #pragma unroll
         for (int e = 0; e < 4; e++) {
@@ -392,55 +527,92 @@ __device__ __forceinline__ void qkv_values(const uint16_t* __restrict__ qkv, con
     }
 }
 
-__global__ void __launch_bounds__(THREADS) qkv_amax_kernel(const uint16_t* __restrict__ qkv, const float* __restrict__ cos_tab,
-                                                           const float* __restrict__ sin_tab, float* amaxes, uint32_t items,
-                                                           int seq_len, int heads, int hd, const QkvDivs dv) {
-    __shared__ float sh[THREADS / 32];
-    float m[3] = {0.f, 0.f, 0.f};
-    for (uint32_t it = blockIdx.x * blockDim.x + threadIdx.x; it < items; it += gridDim.x * blockDim.x) {
-        const QkvItem t = decode_qkv(it, dv);
+struct QkvArgs {
+    const uint16_t* qkv;
+    const float* cos_tab;
+    const float* sin_tab;
+    float* scales;
+    float* amaxes;
+    uint8_t* q_out;
+    uint8_t* k_out;
+    uint8_t* v_out;
+    // with k_cache set: the K and V codes also into a cache [batch, heads, s_max, hd], their scales and the lengths beside it
+    uint8_t* k_cache;
+    uint8_t* v_cache;
+    float* cache_scales;
+    int* cache_lens;
+    int s_max;
+    uint32_t items;
+    int batch, seq_len, heads, hd;
+    QkvDivs dv;
+};
+__device__ __forceinline__ void qkv_amax_items(const QkvArgs& a, uint32_t tid, uint32_t step, float (&m)[3]) {
+    for (uint32_t it = tid; it < a.items; it += step) {
+        const QkvItem t = decode_qkv(it, a.dv);
         float y[32];
-        qkv_values(qkv, cos_tab, sin_tab, t, seq_len, heads, hd, y);
-        const float a = absmax16(y + 16, absmax16(y, 0.f));
-        if (t.which == 0) m[0] = fmaxf(m[0], a);
-        else if (t.which == 1) m[1] = fmaxf(m[1], a);
-        else m[2] = fmaxf(m[2], a);
-    }
-#pragma unroll
-    for (int w = 0; w < 3; w++) {
-        const float r = block_max(m[w], sh);
-        if (threadIdx.x == 0) atomic_amax(amaxes + w, r);
+        qkv_values(a.qkv, a.cos_tab, a.sin_tab, t, a.seq_len, a.heads, a.hd, y);
+        const float v = absmax16(y + 16, absmax16(y, 0.f));
+        if (t.which == 0) m[0] = fmaxf(m[0], v);
+        else if (t.which == 1) m[1] = fmaxf(m[1], v);
+        else m[2] = fmaxf(m[2], v);
     }
 }
-
-__global__ void __launch_bounds__(THREADS) qkv_quant_kernel(const uint16_t* __restrict__ qkv, const float* __restrict__ cos_tab,
-                                                            const float* __restrict__ sin_tab, const float* __restrict__ amaxes,
-                                                            float* scales, uint8_t* __restrict__ q_out, uint8_t* __restrict__ k_out,
-                                                            uint8_t* __restrict__ v_out, uint32_t items, int seq_len, int heads, int hd,
-                                                            const QkvDivs dv) {
+__device__ __forceinline__ void qkv_store(uint8_t* dst, const QkvItem& t, int half, const uint4& lo, const uint4& hi) {
+    *reinterpret_cast<uint4*>(dst + (t.which == 2 ? 32 : 16) * t.c) = lo;
+    *reinterpret_cast<uint4*>(dst + (t.which == 2 ? 32 * t.c + 16 : half + 16 * t.c)) = hi;
+}
+__device__ __forceinline__ void qkv_quant_items(const QkvArgs& a, uint32_t tid, uint32_t step, const float (&m)[3]) {
     float inv[3];
 #pragma unroll
     for (int w = 0; w < 3; w++) {
-        const float sc = scale_from_amax(amaxes[w]);
+        const float sc = scale_from_amax(m[w]);
         inv[w] = __fdiv_rn(1.0f, sc);
-        if (blockIdx.x == 0 && threadIdx.x == 0) scales[w] = sc;
-    }
-    const int half = hd / 2;
-    for (uint32_t it = blockIdx.x * blockDim.x + threadIdx.x; it < items; it += gridDim.x * blockDim.x) {
-        const QkvItem t = decode_qkv(items - 1 - it, dv);  // backwards: see the file header
-        float y[32];
-        qkv_values(qkv, cos_tab, sin_tab, t, seq_len, heads, hd, y);
-        uint8_t* dst = (t.which == 0 ? q_out : t.which == 1 ? k_out : v_out) + (((size_t)t.b * heads + t.h) * seq_len + t.s) * hd;
-        const float iv = t.which == 0 ? inv[0] : t.which == 1 ? inv[1] : inv[2];
-        if (t.which == 2) {
-            *reinterpret_cast<uint4*>(dst + 32 * t.c) = quant16(y, iv);
-            *reinterpret_cast<uint4*>(dst + 32 * t.c + 16) = quant16(y + 16, iv);
-        } else {
-            *reinterpret_cast<uint4*>(dst + 16 * t.c) = quant16(y, iv);
-            *reinterpret_cast<uint4*>(dst + half + 16 * t.c) = quant16(y + 16, iv);
+        if (tid == 0) {
+            a.scales[w] = sc;
+            if (w > 0 && a.k_cache) a.cache_scales[w - 1] = sc;
         }
     }
+    if (a.k_cache)
+        for (uint32_t b = tid; b < (uint32_t)a.batch; b += step) a.cache_lens[b] = a.seq_len;
+    const int half = a.hd / 2;
+    for (uint32_t it = tid; it < a.items; it += step) {
+        const QkvItem t = decode_qkv(a.items - 1 - it, a.dv);  // backwards: see the file header
+        float y[32];
+        qkv_values(a.qkv, a.cos_tab, a.sin_tab, t, a.seq_len, a.heads, a.hd, y);
+        const size_t head = (size_t)t.b * a.heads + t.h;
+        const float iv = t.which == 0 ? inv[0] : t.which == 1 ? inv[1] : inv[2];
+        const uint4 lo = quant16(y, iv), hi = quant16(y + 16, iv);
+        qkv_store((t.which == 0 ? a.q_out : t.which == 1 ? a.k_out : a.v_out) + (head * a.seq_len + t.s) * a.hd, t, half, lo, hi);
+        if (t.which > 0 && a.k_cache) qkv_store((t.which == 1 ? a.k_cache : a.v_cache) + (head * a.s_max + t.s) * a.hd, t, half, lo, hi);
+    }
 }
+__global__ void __launch_bounds__(THREADS) qkv_amax_kernel(const QkvArgs a) {
+    __shared__ float sh[THREADS / 32];
+    pdl_wait();
+    pdl_trigger();
+    float m[3] = {0.f, 0.f, 0.f};
+    qkv_amax_items(a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, m);
+#pragma unroll
+    for (int w = 0; w < 3; w++) {
+        const float r = block_max(m[w], sh);
+        if (threadIdx.x == 0) atomic_amax(a.amaxes + w, r);
+    }
+}
+__global__ void __launch_bounds__(THREADS) qkv_quant_kernel(const QkvArgs a) {
+    pdl_wait();
+    pdl_trigger();
+    const float m[3] = {ld_f32(a.amaxes), ld_f32(a.amaxes + 1), ld_f32(a.amaxes + 2)};
+    qkv_quant_items(a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, m);
+}
+struct QkvOp {
+    static constexpr int N = 3;
+    QkvArgs a;
+    __device__ void pass1(float (&m)[3]) const { qkv_amax_items(a, oc_tid(), OC_STEP, m); }
+    __device__ void pass2(const float (&m)[3]) const {
+        if (oc_tid() < 3) a.amaxes[oc_tid()] = oc_tid() == 0 ? m[0] : oc_tid() == 1 ? m[1] : m[2];
+        qkv_quant_items(a, oc_tid(), OC_STEP, m);
+    }
+};
 
 // ---------------------------------------------------------------------------------- decode step: RoPE + quantise + cache append
 // One item = 32 elements of one (sequence, head slot): slots [0, Hq) are query heads, [Hq, Hq+Hkv) key heads,
@@ -460,12 +632,13 @@ struct DecAppend {
     int* seq_lens_out;
     const int* block_table;
     int batch, hq, hkv, hd, s_max, table_rows, page_size, max_pages, num_pages;
+    int tab_vec;   // the RoPE tables are 16-byte aligned
     uint32_t items;
     FastDiv cph, slots;
 };
 // position of sequence b's new token, or -1 when it cannot be placed (an inactive slot, a full cache, no RoPE row)
 __device__ __forceinline__ int dec_position(const DecAppend& a, int b) {
-    const int pos = __ldg(a.positions + b);
+    const int pos = ld_s32(a.positions + b);
     const int cap = a.block_table ? a.page_size * a.max_pages : a.s_max;
     return (pos >= 0 && pos < cap && pos < a.table_rows) ? pos : -1;
 }
@@ -475,29 +648,42 @@ __device__ __forceinline__ void dec_values(const DecAppend& a, int b, int slot, 
     if (slot >= a.hq + a.hkv) {
         const uint4* src = reinterpret_cast<const uint4*>(a.qkv + row + 32 * c);
 #pragma unroll
-        for (int v = 0; v < 4; v++) bf16x8_to_f32(__ldg(src + v), y + 8 * v);
+        for (int v = 0; v < 4; v++) bf16x8_to_f32(ld128(src + v), y + 8 * v);
         return;
     }
     float x0[16], x1[16];
     const uint4* s0 = reinterpret_cast<const uint4*>(a.qkv + row + 16 * c);
     const uint4* s1 = reinterpret_cast<const uint4*>(a.qkv + row + half + 16 * c);
-    bf16x8_to_f32(__ldg(s0), x0);
-    bf16x8_to_f32(__ldg(s0 + 1), x0 + 8);
-    bf16x8_to_f32(__ldg(s1), x1);
-    bf16x8_to_f32(__ldg(s1 + 1), x1 + 8);
+    bf16x8_to_f32(ld128(s0), x0);
+    bf16x8_to_f32(ld128(s0 + 1), x0 + 8);
+    bf16x8_to_f32(ld128(s1), x1);
+    bf16x8_to_f32(ld128(s1 + 1), x1 + 8);
     const float* ct = a.cos_tab + (size_t)pos * half + 16 * c;
     const float* st = a.sin_tab + (size_t)pos * half + 16 * c;
+    float cc[16], ss[16];
+    if (a.tab_vec) {
+#pragma unroll
+        for (int v = 0; v < 4; v++) {
+            const float4 c4 = ld128f(ct + 4 * v), s4 = ld128f(st + 4 * v);
+            cc[4 * v] = c4.x; cc[4 * v + 1] = c4.y; cc[4 * v + 2] = c4.z; cc[4 * v + 3] = c4.w;
+            ss[4 * v] = s4.x; ss[4 * v + 1] = s4.y; ss[4 * v + 2] = s4.z; ss[4 * v + 3] = s4.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            cc[i] = ld_f32(ct + i);
+            ss[i] = ld_f32(st + i);
+        }
+    }
 #pragma unroll
     for (int i = 0; i < 16; i++) {
-        const float cc = __ldg(ct + i), ss = __ldg(st + i);
-        y[i] = __fsub_rn(__fmul_rn(x0[i], cc), __fmul_rn(x1[i], ss));
-        y[16 + i] = __fadd_rn(__fmul_rn(x0[i], ss), __fmul_rn(x1[i], cc));
+        y[i] = __fsub_rn(__fmul_rn(x0[i], cc[i]), __fmul_rn(x1[i], ss[i]));
+        y[16 + i] = __fadd_rn(__fmul_rn(x0[i], ss[i]), __fmul_rn(x1[i], cc[i]));
     }
 }
-__global__ void __launch_bounds__(THREADS) dec_q_amax_kernel(const DecAppend a) {
-    __shared__ float sh[THREADS / 32];
+__device__ __forceinline__ float dec_q_amax_items(const DecAppend& a, uint32_t tid, uint32_t step) {
     float m = 0.f;
-    for (uint32_t it = blockIdx.x * blockDim.x + threadIdx.x; it < a.items; it += gridDim.x * blockDim.x) {
+    for (uint32_t it = tid; it < a.items; it += step) {
         uint32_t q, c, b, slot;
         a.cph.divmod(it, q, c);
         a.slots.divmod(q, b, slot);
@@ -508,23 +694,22 @@ __global__ void __launch_bounds__(THREADS) dec_q_amax_kernel(const DecAppend a) 
         dec_values(a, (int)b, (int)slot, (int)c, pos, y);
         m = absmax16(y + 16, absmax16(y, m));
     }
-    m = block_max(m, sh);
-    if (threadIdx.x == 0) atomic_amax(a.q_amax, m);
+    return m;
 }
-__global__ void __launch_bounds__(THREADS) dec_append_kernel(const DecAppend a) {
-    const float q_sc = scale_from_amax(*a.q_amax);
+__device__ __forceinline__ void dec_append_items(const DecAppend& a, uint32_t tid, uint32_t step, float q_amax) {
+    const float q_sc = scale_from_amax(q_amax);
     const float inv_q = __fdiv_rn(1.0f, q_sc);
-    const float inv_k = __fdiv_rn(1.0f, __ldg(a.k_scale)), inv_v = __fdiv_rn(1.0f, __ldg(a.v_scale));
-    if (blockIdx.x == 0 && threadIdx.x == 0) *a.q_scale = q_sc;
+    const float inv_k = __fdiv_rn(1.0f, ld_f32(a.k_scale)), inv_v = __fdiv_rn(1.0f, ld_f32(a.v_scale));
+    if (tid == 0) *a.q_scale = q_sc;
     const int half = a.hd / 2;
-    for (uint32_t it = blockIdx.x * blockDim.x + threadIdx.x; it < a.items; it += gridDim.x * blockDim.x) {
+    for (uint32_t it = tid; it < a.items; it += step) {
         uint32_t q, c, b, slot;
         a.cph.divmod(it, q, c);
         a.slots.divmod(q, b, slot);
         const int pos = dec_position(a, (int)b);
         if (slot == 0 && c == 0 && a.seq_lens_out) {
             // an inactive slot keeps its length: 0 for a negative position, the capacity for a full cache
-            const int raw = __ldg(a.positions + b);
+            const int raw = ld_s32(a.positions + b);
             const int cap = a.block_table ? a.page_size * a.max_pages : a.s_max;
             a.seq_lens_out[b] = pos >= 0 ? pos + 1 : (raw < 0 ? 0 : min(raw, cap));
         }
@@ -547,7 +732,7 @@ __global__ void __launch_bounds__(THREADS) dec_append_kernel(const DecAppend a) 
         size_t key_row;   // index of this (sequence, kv head, position) among the cache's rows of hd codes
         if (a.block_table) {
             const int pg = pos / a.page_size;
-            const int page = __ldg(a.block_table + (size_t)b * a.max_pages + pg);
+            const int page = ld_s32(a.block_table + (size_t)b * a.max_pages + pg);
             if (page < 0 || page >= a.num_pages) continue;   // no page behind this position: nothing is written
             key_row = ((size_t)page * a.hkv + h) * a.page_size + (pos - pg * a.page_size);
         } else {
@@ -566,6 +751,28 @@ __global__ void __launch_bounds__(THREADS) dec_append_kernel(const DecAppend a) 
     }
 }
 
+__global__ void __launch_bounds__(THREADS) dec_q_amax_kernel(const DecAppend a) {
+    __shared__ float sh[THREADS / 32];
+    pdl_wait();
+    pdl_trigger();
+    const float m = block_max(dec_q_amax_items(a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x), sh);
+    if (threadIdx.x == 0) atomic_amax(a.q_amax, m);
+}
+__global__ void __launch_bounds__(THREADS) dec_append_kernel(const DecAppend a) {
+    pdl_wait();
+    pdl_trigger();
+    dec_append_items(a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, ld_f32(a.q_amax));
+}
+struct DecOp {
+    static constexpr int N = 1;
+    DecAppend a;
+    __device__ void pass1(float (&m)[1]) const { m[0] = dec_q_amax_items(a, oc_tid(), OC_STEP); }
+    __device__ void pass2(const float (&m)[1]) const {
+        if (oc_tid() == 0) *a.q_amax = m[0];
+        dec_append_items(a, oc_tid(), OC_STEP, m[0]);
+    }
+};
+
 // ---------------------------------------------------------------------------------- attention output: permute + quantise
 // item = 16 consecutive elements of one (token, head); out index order so that stores are contiguous
 struct ODivs {
@@ -578,34 +785,60 @@ __device__ __forceinline__ size_t o_src_offset(uint32_t it, int seq_len, int hea
     dv.seq.divmod(q, q, s);  // q = batch index
     return (((size_t)q * heads + h) * seq_len + s) * hd + 16 * c;
 }
-__global__ void __launch_bounds__(THREADS) o_amax_kernel(const uint16_t* __restrict__ o, float* amax, size_t n16) {
-    __shared__ float sh[THREADS / 32];
+struct OArgs {
+    const uint16_t* o;
+    uint8_t* q;
+    float* scale_out;
+    float* amax_out;
+    uint32_t n16;
+    int seq_len, heads, hd;
+    ODivs dv;
+};
+__device__ __forceinline__ float o_amax_items(const OArgs& a, uint32_t tid, uint32_t step) {
     float m = 0.f;
-    const uint4* src = reinterpret_cast<const uint4*>(o);
-    for (size_t it = (size_t)blockIdx.x * blockDim.x + threadIdx.x; it < n16; it += (size_t)gridDim.x * blockDim.x) {
+#pragma unroll 2
+    for (uint32_t it = tid; it < a.n16; it += step) {
         float y[16];
-        f16x8_to_f32(__ldg(src + 2 * it), y);
-        f16x8_to_f32(__ldg(src + 2 * it + 1), y + 8);
+        f16x8_to_f32(ld128(a.o + (size_t)it * 16), y);
+        f16x8_to_f32(ld128(a.o + (size_t)it * 16 + 8), y + 8);
         m = absmax16(y, m);
     }
-    m = block_max(m, sh);
-    if (threadIdx.x == 0) atomic_amax(amax, m);
+    return m;
 }
-__global__ void __launch_bounds__(THREADS) o_quant_kernel(const uint16_t* __restrict__ o, const float* __restrict__ amax_ptr,
-                                                          float* scale_out, uint8_t* __restrict__ q, uint32_t n16, int seq_len,
-                                                          int heads, int hd, const ODivs dv) {
-    const float scale = scale_from_amax(*amax_ptr);
+__device__ __forceinline__ void o_quant_items(const OArgs& a, uint32_t tid, uint32_t step, float amax) {
+    const float scale = scale_from_amax(amax);
     const float inv = __fdiv_rn(1.0f, scale);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = scale;
-    for (uint32_t it = blockIdx.x * blockDim.x + threadIdx.x; it < n16; it += gridDim.x * blockDim.x) {
-        const uint32_t rit = n16 - 1 - it;   // destination order (token-major), walked backwards
-        const uint4* sp = reinterpret_cast<const uint4*>(o + o_src_offset(rit, seq_len, heads, hd, dv));
+    if (tid == 0) *a.scale_out = scale;
+    for (uint32_t it = tid; it < a.n16; it += step) {
+        const uint32_t rit = a.n16 - 1 - it;   // destination order (token-major), walked backwards
+        const uint16_t* sp = a.o + o_src_offset(rit, a.seq_len, a.heads, a.hd, a.dv);
         float y[16];
-        f16x8_to_f32(__ldg(sp), y);
-        f16x8_to_f32(__ldg(sp + 1), y + 8);
-        *reinterpret_cast<uint4*>(q + (size_t)rit * 16) = quant16(y, inv);
+        f16x8_to_f32(ld128(sp), y);
+        f16x8_to_f32(ld128(sp + 8), y + 8);
+        *reinterpret_cast<uint4*>(a.q + (size_t)rit * 16) = quant16(y, inv);
     }
 }
+__global__ void __launch_bounds__(THREADS) o_amax_kernel(const OArgs a) {
+    __shared__ float sh[THREADS / 32];
+    pdl_wait();
+    pdl_trigger();
+    const float m = block_max(o_amax_items(a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x), sh);
+    if (threadIdx.x == 0) atomic_amax(a.amax_out, m);
+}
+__global__ void __launch_bounds__(THREADS) o_quant_kernel(const OArgs a) {
+    pdl_wait();
+    pdl_trigger();
+    o_quant_items(a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, ld_f32(a.amax_out));
+}
+struct OOp {
+    static constexpr int N = 1;
+    OArgs a;
+    __device__ void pass1(float (&m)[1]) const { m[0] = o_amax_items(a, oc_tid(), OC_STEP); }
+    __device__ void pass2(const float (&m)[1]) const {
+        if (oc_tid() == 0) *a.amax_out = m[0];
+        o_quant_items(a, oc_tid(), OC_STEP, m[0]);
+    }
+};
 
 // ---------------------------------------------------------------------------------- SwiGLU + quantise
 __device__ __forceinline__ float rcp_approx(float x) {
@@ -636,8 +869,8 @@ __global__ void __launch_bounds__(THREADS) swiglu_amax_kernel(const uint16_t* __
             uint32_t row, c;
             per_row.divmod(live[u] ? i : it, row, c);
             const uint16_t* gp = gu + (size_t)row * 2 * F + c * 16;
-            gv[u] = ldg256(gp);
-            uv[u] = ldg256(gp + F);
+            gv[u] = ld256(gp);
+            uv[u] = ld256(gp + F);
         }
 #pragma unroll
         for (int u = 0; u < 2; u++) {
@@ -652,7 +885,7 @@ __global__ void __launch_bounds__(THREADS) swiglu_amax_kernel(const uint16_t* __
 __global__ void __launch_bounds__(THREADS) swiglu_quant_kernel(const uint16_t* __restrict__ gu, const float* __restrict__ amax_ptr,
                                                                float* scale_out, uint8_t* __restrict__ q, uint32_t items, int F,
                                                                const FastDiv per_row) {
-    const float scale = scale_from_amax(*amax_ptr);
+    const float scale = scale_from_amax(ld_f32(amax_ptr));
     const float inv = __fdiv_rn(1.0f, scale);
     if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = scale;
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -667,8 +900,8 @@ __global__ void __launch_bounds__(THREADS) swiglu_quant_kernel(const uint16_t* _
             uint32_t row, c;
             per_row.divmod(items - 1 - (live[u] ? i : it), row, c);  // backwards: see the file header
             const uint16_t* gp = gu + (size_t)row * 2 * F + c * 16;
-            gv[u] = ldg256(gp);
-            uv[u] = ldg256(gp + F);
+            gv[u] = ld256(gp);
+            uv[u] = ld256(gp + F);
             dst[u] = (size_t)row * F + c * 16;
         }
 #pragma unroll
@@ -682,16 +915,17 @@ __global__ void __launch_bounds__(THREADS) swiglu_quant_kernel(const uint16_t* _
 
 // ---------------------------------------------------------------------------------- quantise bf16 with a known amax
 // single pass: the producer (the SwiGLU GEMM epilogue) already reduced max|x|
-__global__ void __launch_bounds__(THREADS) quant_bf16_kernel(const uint16_t* __restrict__ x, const float* __restrict__ amax_ptr,
-                                                             float* scale_out, uint8_t* __restrict__ q, size_t n16) {
-    const float scale = scale_from_amax(*amax_ptr);
+__global__ void __launch_bounds__(THREADS) quant_bf16_kernel(const uint16_t* x, const float* amax_ptr, float* scale_out, uint8_t* q, size_t n16) {
+    pdl_wait();
+    pdl_trigger();
+    const float scale = scale_from_amax(ld_f32(amax_ptr));
     const float inv = __fdiv_rn(1.0f, scale);
     if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = scale;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t it = (size_t)blockIdx.x * blockDim.x + threadIdx.x; it < n16; it += 2 * stride) {  // two items per step, loads first
         const bool second = it + stride < n16;
-        const U8 a = ldg256(x + it * 16);
-        const U8 b = ldg256(x + (second ? it + stride : it) * 16);
+        const U8 a = ld256(x + it * 16);
+        const U8 b = ld256(x + (second ? it + stride : it) * 16);
         float y[16];
         bf16x16_to_f32(a, y);
         *reinterpret_cast<uint4*>(q + it * 16) = quant16(y, inv);
@@ -706,7 +940,7 @@ __global__ void __launch_bounds__(THREADS) quant_bf16_kernel(const uint16_t* __r
 __global__ void __launch_bounds__(THREADS) residual_add_kernel(float* __restrict__ x, const uint16_t* __restrict__ y, size_t n8) {
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (size_t)gridDim.x * blockDim.x) {
         float f[8];
-        bf16x8_to_f32(__ldg(reinterpret_cast<const uint4*>(y) + i), f);
+        bf16x8_to_f32(ld128(reinterpret_cast<const uint4*>(y) + i), f);
         float4* xp = reinterpret_cast<float4*>(x) + 2 * i;
         float4 a = xp[0], b = xp[1];
         a.x += f[0]; a.y += f[1]; a.z += f[2]; a.w += f[3];
@@ -728,60 +962,103 @@ int fp8_rope_table(float* cos_out, float* sin_out, int seq_len, int head_dim, fl
     return (int)cudaGetLastError();
 }
 
-int fp8_rmsnorm_quantize(const float* x, const void* residual_bf16, float* h_out, const float* gamma, uint8_t* q,
-                         float* scale_out, float* amax_out, float* rstd_ws, int rows, int hidden, float eps, void* stream) {
+}  // extern "C"
+
+namespace {
+
+int rmsnorm_quantize(const float* x, const void* residual_bf16, float* h_out, bool store_h, const float* gamma, uint8_t* q, float* scale_out,
+                     float* amax_out, float* rstd_ws, float* zero_word, int rows, int hidden, float eps, cudaStream_t s) {
     if (!x || !gamma || !q || !scale_out || !amax_out || !rstd_ws) return (int)cudaErrorInvalidValue;
     if (rows < 0 || hidden <= 0 || (hidden % 16) != 0) return (int)cudaErrorInvalidValue;
     if (misaligned32(x) || misaligned(residual_bf16) || misaligned32(h_out) || misaligned32(gamma) || misaligned(q)) return (int)cudaErrorInvalidValue;
-    cudaStream_t s = (cudaStream_t)stream;
-    cudaError_t e = cudaMemsetAsync(amax_out, 0, sizeof(float), s);
-    if (e != cudaSuccess) return (int)e;
+    const size_t items = (size_t)rows * (hidden / 16);
+    if (items >= (1ull << 31)) return (int)cudaErrorInvalidValue;
     const uint16_t* res = reinterpret_cast<const uint16_t*>(residual_bf16);
+    float* h = store_h ? h_out : nullptr;
+    if (items * 64 <= OC_BYTES_RMS && oc_fits<RmsOp>()) {
+        RmsOp op{x, res, h, gamma, q, scale_out, amax_out, rstd_ws, zero_word, rows, hidden, eps, rows <= OC_CTAS ? 4 : rows <= 4 * OC_CTAS ? 2 : 0};
+        return (int)oc_launch(op, s);
+    }
+    cudaError_t e = clear_words(amax_out, 1, s);
+    if (e == cudaSuccess && zero_word) e = clear_words(zero_word, 1, s);
+    if (e != cudaSuccess) return (int)e;
     if (rows > 0) {
         int dev = 0, sms = 148;
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int grid = rows < sms * 8 ? rows : sms * 8;
-#define RMS_STATS_REGS(N)                                                                                               \
-    (res ? rms_stats_regs_kernel<N, true><<<grid, THREADS, 0, s>>>(x, res, h_out, gamma, rstd_ws, amax_out, rows, eps) \
-         : rms_stats_regs_kernel<N, false><<<grid, THREADS, 0, s>>>(x, res, h_out, gamma, rstd_ws, amax_out, rows, eps))
-        if (hidden == 2048) RMS_STATS_REGS(1);
-        else if (hidden == 4096) RMS_STATS_REGS(2);
-        else if (hidden == 8192) RMS_STATS_REGS(4);
-        else rms_stats_kernel<<<grid, THREADS, 0, s>>>(x, res, h_out, gamma, rstd_ws, amax_out, rows, hidden, eps);
+        const dim3 grid(rows < sms * 8 ? rows : sms * 8), block(THREADS);
+#define RMS_STATS_REGS(N)                                                                                                        \
+    (res ? launch_pdl(rms_stats_regs_kernel<N, true>, grid, block, 0, s, x, res, h, gamma, rstd_ws, amax_out, rows, eps) \
+         : launch_pdl(rms_stats_regs_kernel<N, false>, grid, block, 0, s, x, res, h, gamma, rstd_ws, amax_out, rows, eps))
+        if (hidden == 2048) e = RMS_STATS_REGS(1);
+        else if (hidden == 4096) e = RMS_STATS_REGS(2);
+        else if (hidden == 8192) e = RMS_STATS_REGS(4);
+        else e = launch_pdl(rms_stats_kernel, grid, block, 0, s, x, res, h, gamma, rstd_ws, amax_out, rows, hidden, eps);
 #undef RMS_STATS_REGS
+        if (e != cudaSuccess) return (int)e;
     }
-    // pass 2 reads the updated stream where pass 1 stored it
-    const bool from_h = res && h_out;
-    const size_t items = (size_t)rows * (hidden / 16);
+    // pass 2 reads the stream where pass 1 stored it
+    return (int)launch_pdl(rms_quant_kernel, dim3(grid_for(items)), dim3(THREADS), 0, s, h ? h : x, h ? nullptr : res, gamma, rstd_ws,
+                           amax_out, scale_out, q, (uint32_t)items, hidden, FastDiv(hidden / 16));
+}
+
+int rope_quantize_qkv(QkvArgs a, cudaStream_t s) {
+    if (!a.qkv || !a.cos_tab || !a.sin_tab || !a.q_out || !a.k_out || !a.v_out || !a.scales || !a.amaxes) return (int)cudaErrorInvalidValue;
+    if (a.batch < 0 || a.seq_len <= 0 || a.heads <= 0 || (a.hd != 64 && a.hd != 128)) return (int)cudaErrorInvalidValue;
+    if (misaligned(a.qkv) || misaligned(a.cos_tab) || misaligned(a.sin_tab) || misaligned(a.q_out) || misaligned(a.k_out) || misaligned(a.v_out))
+        return (int)cudaErrorInvalidValue;
+    const size_t items = (size_t)a.batch * a.seq_len * 3 * a.heads * (a.hd / 32);
     if (items >= (1ull << 31)) return (int)cudaErrorInvalidValue;
-    rms_quant_kernel<<<grid_for(items), THREADS, 0, s>>>(from_h ? h_out : x, from_h ? nullptr : res, gamma, rstd_ws, amax_out, scale_out, q,
-                                                         (uint32_t)items, hidden, FastDiv(hidden / 16));
-    return (int)cudaGetLastError();
+    a.items = (uint32_t)items;
+    a.dv.cph = FastDiv(a.hd / 32);
+    a.dv.heads = FastDiv(a.heads);
+    a.dv.three = FastDiv(3);
+    a.dv.seq = FastDiv(a.seq_len);
+    if (items * 64 <= OC_BYTES_QKV && oc_fits<QkvOp>()) return (int)oc_launch(QkvOp{a}, s);
+    cudaError_t e = clear_words(a.amaxes, 3, s);
+    if (e == cudaSuccess && items > 0) e = launch_pdl(qkv_amax_kernel, dim3(grid_for(items)), dim3(THREADS), 0, s, a);
+    if (e == cudaSuccess) e = launch_pdl(qkv_quant_kernel, dim3(grid_for(items)), dim3(THREADS), 0, s, a);
+    return (int)e;
+}
+
+}  // namespace
+
+extern "C" {
+
+int fp8_rmsnorm_quantize(const float* x, const void* residual_bf16, float* h_out, const float* gamma, uint8_t* q,
+                         float* scale_out, float* amax_out, float* rstd_ws, int rows, int hidden, float eps, void* stream) {
+    return rmsnorm_quantize(x, residual_bf16, h_out, residual_bf16 && h_out, gamma, q, scale_out, amax_out, rstd_ws, nullptr, rows, hidden, eps,
+                            (cudaStream_t)stream);
+}
+
+int fp8_rmsnorm_quantize_into(const float* x, float* h_out, const float* gamma, uint8_t* q, float* scale_out, float* amax_out, float* rstd_ws,
+                              float* zero_word, int rows, int hidden, float eps, void* stream) {
+    return rmsnorm_quantize(x, nullptr, h_out, h_out != nullptr, gamma, q, scale_out, amax_out, rstd_ws, zero_word, rows, hidden, eps,
+                            (cudaStream_t)stream);
 }
 
 int fp8_rope_quantize_qkv(const void* qkv_bf16, const float* cos_tab, const float* sin_tab, uint8_t* q_out, uint8_t* k_out,
                           uint8_t* v_out, float* scales, float* amaxes, int batch, int seq_len, int heads, int head_dim,
                           void* stream) {
-    if (!qkv_bf16 || !cos_tab || !sin_tab || !q_out || !k_out || !v_out || !scales || !amaxes) return (int)cudaErrorInvalidValue;
-    if (batch < 0 || seq_len <= 0 || heads <= 0 || (head_dim != 64 && head_dim != 128)) return (int)cudaErrorInvalidValue;
-    if (misaligned(qkv_bf16) || misaligned(cos_tab) || misaligned(sin_tab) || misaligned(q_out) || misaligned(k_out) || misaligned(v_out))
+    QkvArgs a{};
+    a.qkv = reinterpret_cast<const uint16_t*>(qkv_bf16);
+    a.cos_tab = cos_tab; a.sin_tab = sin_tab; a.scales = scales; a.amaxes = amaxes;
+    a.q_out = q_out; a.k_out = k_out; a.v_out = v_out;
+    a.batch = batch; a.seq_len = seq_len; a.heads = heads; a.hd = head_dim;
+    return rope_quantize_qkv(a, (cudaStream_t)stream);
+}
+
+int fp8_rope_quantize_qkv_cache(const void* qkv_bf16, const float* cos_tab, const float* sin_tab, uint8_t* q_out, uint8_t* k_out,
+                                uint8_t* v_out, float* scales, float* amaxes, uint8_t* k_cache, uint8_t* v_cache, float* cache_scales,
+                                int32_t* cache_lens, int batch, int seq_len, int s_max, int heads, int head_dim, void* stream) {
+    if (!k_cache || !v_cache || !cache_scales || !cache_lens || s_max < seq_len || misaligned(k_cache) || misaligned(v_cache))
         return (int)cudaErrorInvalidValue;
-    cudaStream_t s = (cudaStream_t)stream;
-    cudaError_t e = cudaMemsetAsync(amaxes, 0, 3 * sizeof(float), s);
-    if (e != cudaSuccess) return (int)e;
-    const size_t items = (size_t)batch * seq_len * 3 * heads * (head_dim / 32);
-    if (items >= (1ull << 31)) return (int)cudaErrorInvalidValue;
-    const uint16_t* src = reinterpret_cast<const uint16_t*>(qkv_bf16);
-    QkvDivs dv;
-    dv.cph = FastDiv(head_dim / 32);
-    dv.heads = FastDiv(heads);
-    dv.three = FastDiv(3);
-    dv.seq = FastDiv(seq_len);
-    if (items > 0)
-        qkv_amax_kernel<<<grid_for(items), THREADS, 0, s>>>(src, cos_tab, sin_tab, amaxes, (uint32_t)items, seq_len, heads, head_dim, dv);
-    qkv_quant_kernel<<<grid_for(items), THREADS, 0, s>>>(src, cos_tab, sin_tab, amaxes, scales, q_out, k_out, v_out, (uint32_t)items, seq_len,
-                                                         heads, head_dim, dv);
-    return (int)cudaGetLastError();
+    QkvArgs a{};
+    a.qkv = reinterpret_cast<const uint16_t*>(qkv_bf16);
+    a.cos_tab = cos_tab; a.sin_tab = sin_tab; a.scales = scales; a.amaxes = amaxes;
+    a.q_out = q_out; a.k_out = k_out; a.v_out = v_out;
+    a.k_cache = k_cache; a.v_cache = v_cache; a.cache_scales = cache_scales; a.cache_lens = cache_lens; a.s_max = s_max;
+    a.batch = batch; a.seq_len = seq_len; a.heads = heads; a.hd = head_dim;
+    return rope_quantize_qkv(a, (cudaStream_t)stream);
 }
 
 int fp8_decode_rope_append(const fp8_decode_append_args_t* g) {
@@ -799,8 +1076,6 @@ int fp8_decode_rope_append(const fp8_decode_append_args_t* g) {
     }
     if (misaligned(g->qkv_bf16) || misaligned(g->q_out) || misaligned(g->k_cache) || misaligned(g->v_cache)) return (int)cudaErrorInvalidValue;
     cudaStream_t s = (cudaStream_t)g->stream;
-    cudaError_t e = cudaMemsetAsync(g->q_amax_out, 0, sizeof(float), s);
-    if (e != cudaSuccess) return (int)e;
     const int slots = g->q_heads + 2 * g->kv_heads;
     const size_t items = (size_t)g->batch * slots * (g->head_dim / 32);
     if (items >= (1ull << 31)) return (int)cudaErrorInvalidValue;
@@ -813,11 +1088,14 @@ int fp8_decode_rope_append(const fp8_decode_append_args_t* g) {
     a.batch = g->batch; a.hq = g->q_heads; a.hkv = g->kv_heads; a.hd = g->head_dim; a.s_max = g->s_max;
     a.table_rows = g->rope_rows; a.page_size = g->page_size; a.max_pages = g->max_pages_per_seq; a.num_pages = g->num_pages;
     a.items = (uint32_t)items;
+    a.tab_vec = !misaligned(g->cos_tab) && !misaligned(g->sin_tab);
     a.cph = FastDiv(g->head_dim / 32);
     a.slots = FastDiv(slots);
-    if (items > 0) dec_q_amax_kernel<<<grid_for(items), THREADS, 0, s>>>(a);
-    dec_append_kernel<<<grid_for(items), THREADS, 0, s>>>(a);
-    return (int)cudaGetLastError();
+    if (items * 64 <= OC_BYTES_DEC && oc_fits<DecOp>()) return (int)oc_launch(DecOp{a}, s);
+    cudaError_t e = clear_words(a.q_amax, 1, s);
+    if (e == cudaSuccess && items > 0) e = launch_pdl(dec_q_amax_kernel, dim3(grid_for(items)), dim3(THREADS), 0, s, a);
+    if (e == cudaSuccess) e = launch_pdl(dec_append_kernel, dim3(grid_for(items)), dim3(THREADS), 0, s, a);
+    return (int)e;
 }
 
 int fp8_permute_quantize_heads(const void* o_fp16, uint8_t* q, float* scale_out, float* amax_out, int batch, int seq_len,
@@ -826,18 +1104,20 @@ int fp8_permute_quantize_heads(const void* o_fp16, uint8_t* q, float* scale_out,
     if (batch < 0 || seq_len <= 0 || heads <= 0 || head_dim <= 0 || (head_dim % 16) != 0) return (int)cudaErrorInvalidValue;
     if (misaligned(o_fp16) || misaligned(q)) return (int)cudaErrorInvalidValue;
     cudaStream_t s = (cudaStream_t)stream;
-    cudaError_t e = cudaMemsetAsync(amax_out, 0, sizeof(float), s);
-    if (e != cudaSuccess) return (int)e;
     const size_t n16 = (size_t)batch * seq_len * heads * (head_dim / 16);
     if (n16 >= (1ull << 31)) return (int)cudaErrorInvalidValue;
-    const uint16_t* src = reinterpret_cast<const uint16_t*>(o_fp16);
-    ODivs dv;
-    dv.cph = FastDiv(head_dim / 16);
-    dv.heads = FastDiv(heads);
-    dv.seq = FastDiv(seq_len);
-    if (n16 > 0) o_amax_kernel<<<grid_for(n16), THREADS, 0, s>>>(src, amax_out, n16);
-    o_quant_kernel<<<grid_for(n16), THREADS, 0, s>>>(src, amax_out, scale_out, q, (uint32_t)n16, seq_len, heads, head_dim, dv);
-    return (int)cudaGetLastError();
+    OArgs a{};
+    a.o = reinterpret_cast<const uint16_t*>(o_fp16);
+    a.q = q; a.scale_out = scale_out; a.amax_out = amax_out;
+    a.n16 = (uint32_t)n16; a.seq_len = seq_len; a.heads = heads; a.hd = head_dim;
+    a.dv.cph = FastDiv(head_dim / 16);
+    a.dv.heads = FastDiv(heads);
+    a.dv.seq = FastDiv(seq_len);
+    if (n16 * 32 <= OC_BYTES_O && oc_fits<OOp>()) return (int)oc_launch(OOp{a}, s);
+    cudaError_t e = clear_words(amax_out, 1, s);
+    if (e == cudaSuccess && n16 > 0) e = launch_pdl(o_amax_kernel, dim3(grid_for(n16)), dim3(THREADS), 0, s, a);
+    if (e == cudaSuccess) e = launch_pdl(o_quant_kernel, dim3(grid_for(n16)), dim3(THREADS), 0, s, a);
+    return (int)e;
 }
 
 int fp8_swiglu_quantize(const void* gate_up_bf16, uint8_t* q, float* scale_out, float* amax_out, int rows, int ffn_hidden,
@@ -859,9 +1139,8 @@ int fp8_swiglu_quantize(const void* gate_up_bf16, uint8_t* q, float* scale_out, 
 
 int fp8_quantize_bf16(const void* x_bf16, uint8_t* q, float* scale_out, const float* amax_in, size_t n, void* stream) {
     if (!x_bf16 || !q || !scale_out || !amax_in || (n % 16) != 0 || misaligned32(x_bf16) || misaligned(q)) return (int)cudaErrorInvalidValue;
-    quant_bf16_kernel<<<grid_for(n / 32 + 1), THREADS, 0, (cudaStream_t)stream>>>(reinterpret_cast<const uint16_t*>(x_bf16), amax_in, scale_out, q,
-                                                                                 n / 16);
-    return (int)cudaGetLastError();
+    return (int)launch_pdl(quant_bf16_kernel, dim3(grid_for(n / 32 + 1)), dim3(THREADS), 0, (cudaStream_t)stream,
+                           reinterpret_cast<const uint16_t*>(x_bf16), amax_in, scale_out, q, n / 16);
 }
 
 int fp8_residual_add(float* x, const void* y_bf16, size_t n, void* stream) {

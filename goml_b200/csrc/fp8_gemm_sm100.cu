@@ -793,13 +793,19 @@ int fp8_gemm_accumulate_f32(int M, int N, int K, const void* A, const void* B, f
     return launch(M, N, K, A, B, nullptr, alpha, scale_a, scale_b, 0, (cudaStream_t)stream, X);
 }
 
+int fp8_gemm_swiglu_raise(int M, int F, int K, const void* A, const void* B_interleaved, void* H, float alpha, const float* scale_a,
+                          const float* scale_b, float* amax, void* stream) {
+    if (!H || !amax || F <= 0) return (int)cudaErrorInvalidValue;
+    const int n = 2 * ((F + 31) / 32) * 32;
+    return launch(M, n, K, A, B_interleaved, nullptr, alpha, scale_a, scale_b, 1, (cudaStream_t)stream, nullptr, H, F, amax);
+}
+
 int fp8_gemm_swiglu(int M, int F, int K, const void* A, const void* B_interleaved, void* H, float alpha, const float* scale_a,
                     const float* scale_b, float* amax_out, void* stream) {
     if (!H || !amax_out || F <= 0) return (int)cudaErrorInvalidValue;
     cudaError_t e = cudaMemsetAsync(amax_out, 0, sizeof(float), (cudaStream_t)stream);
     if (e != cudaSuccess) return (int)e;
-    const int n = 2 * ((F + 31) / 32) * 32;
-    return launch(M, n, K, A, B_interleaved, nullptr, alpha, scale_a, scale_b, 1, (cudaStream_t)stream, nullptr, H, F, amax_out);
+    return fp8_gemm_swiglu_raise(M, F, K, A, B_interleaved, H, alpha, scale_a, scale_b, amax_out, stream);
 }
 
 int fp8_gemm_fp8out(int M, int N, int K, const void* A, const void* B, void* D, float alpha, const float* scale_a,

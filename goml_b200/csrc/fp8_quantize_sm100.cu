@@ -3,28 +3,55 @@
 // HBM-bound: the amax pass reads 4 B/element, the conversion pass reads 4 B and
 // writes 1 B per element (the second read is served from L2 when the tensor
 // fits).  128-bit loads, one 128-bit store per 16 elements, grid sized to a
-// multiple of the SM count.
+// multiple of the SM count.  A small tensor is done by one cluster in one kernel
+// (one_cluster.cuh).
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "../../include/fp8_quantize.h"
+#include "one_cluster.cuh"
 
 namespace {
 
-constexpr int THREADS = 256;
+using namespace sm100;
 
-__global__ void __launch_bounds__(THREADS) amax_kernel(const float* __restrict__ x, size_t n, float* amax) {
+constexpr int THREADS = 256;
+// Input bytes up to which one cluster does both passes: rows of 4096, 1 / 40 / 96 rows 2.4 / 4.0 / 5.0 us; two kernels behind a
+// clearing one, as overlapped launches, 4.1 at 128 rows; behind a memset and in turn, as it was, 7.1 to 8.2.
+constexpr size_t OC_BYTES = 768 << 10;
+
+__global__ void clear_word_kernel(float* w) {
+    pdl_wait();
+    pdl_trigger();
+    *w = 0.f;
+}
+
+// |x| maximum of this thread's share of n values
+__device__ __forceinline__ float amax_items(const float* x, size_t n, size_t tid, size_t step) {
     const size_t n4 = n / 4;
-    const float4* x4 = reinterpret_cast<const float4*>(x);
     float m = 0.f;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
-        const float4 v = __ldg(x4 + i);
+    size_t i = tid;
+    for (; i + 3 * step < n4; i += 4 * step) {   // four loads in flight
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = ld128f(x + 4 * (i + u * step));
+#pragma unroll
+        for (int u = 0; u < 4; u++) m = fmaxf(fmaxf(m, fabsf(v[u].x)), fmaxf(fabsf(v[u].y), fmaxf(fabsf(v[u].z), fabsf(v[u].w))));
+    }
+    for (; i < n4; i += step) {
+        const float4 v = ld128f(x + 4 * i);
         m = fmaxf(fmaxf(m, fabsf(v.x)), fmaxf(fabsf(v.y), fmaxf(fabsf(v.z), fabsf(v.w))));  // NaN never wins
     }
-    if (blockIdx.x == 0 && threadIdx.x < (n & 3)) m = fmaxf(m, fabsf(x[n4 * 4 + threadIdx.x]));
+    if (tid < (n & 3)) m = fmaxf(m, fabsf(ld_f32(x + n4 * 4 + tid)));
+    return m;
+}
+
+__global__ void __launch_bounds__(THREADS) amax_kernel(const float* x, size_t n, float* amax) {
+    pdl_wait();
+    pdl_trigger();
+    float m = amax_items(x, n, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     __shared__ float wm[THREADS / 32];
@@ -50,28 +77,46 @@ __device__ __forceinline__ uint32_t quant4(float4 v, float inv) {
     return lo | (hi << 16);
 }
 
-__global__ void __launch_bounds__(THREADS) quant_kernel(const float* __restrict__ x, uint8_t* __restrict__ q, size_t n,
-                                                        const float* __restrict__ amax_ptr, float* scale_out,
-                                                        float divisor) {
-    const float amax = *amax_ptr;
+__device__ __forceinline__ void quant_items(const float* x, uint8_t* q, size_t n, size_t tid, size_t step, float amax, float* scale_out,
+                                            float divisor) {
     const float scale = (amax > 1e-12f) ? __fdiv_rn(amax, divisor) : 1.0f;
     const float inv = __fdiv_rn(1.0f, scale);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = scale;
+    if (tid == 0) *scale_out = scale;
     const size_t n16 = n / 16;
-    const float4* x4 = reinterpret_cast<const float4*>(x);
     uint4* q16 = reinterpret_cast<uint4*>(q);
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += stride) {
-        const float4 a = __ldg(x4 + 4 * i), b = __ldg(x4 + 4 * i + 1), c = __ldg(x4 + 4 * i + 2), d = __ldg(x4 + 4 * i + 3);
+    for (size_t it = tid; it < n16; it += step) {
+        const size_t i = n16 - 1 - it;   // backwards: what pass 1 read last is still in L2
+        const float4 a = ld128f(x + 16 * i), b = ld128f(x + 16 * i + 4), c = ld128f(x + 16 * i + 8), d = ld128f(x + 16 * i + 12);
         q16[i] = make_uint4(quant4(a, inv), quant4(b, inv), quant4(c, inv), quant4(d, inv));
     }
-    if (blockIdx.x == 0) {
-        for (size_t i = n16 * 16 + threadIdx.x; i < n; i += blockDim.x) {
-            const float v = fminf(fmaxf(__fmul_rn(x[i], inv), -448.f), 448.f);
-            q[i] = (uint8_t)__nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
-        }
+    if (tid < (n & 15)) {
+        const size_t i = n16 * 16 + tid;
+        const float v = fminf(fmaxf(__fmul_rn(ld_f32(x + i), inv), -448.f), 448.f);
+        q[i] = (uint8_t)__nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
     }
 }
+
+__global__ void __launch_bounds__(THREADS) quant_kernel(const float* x, uint8_t* q, size_t n, const float* amax_ptr, float* scale_out,
+                                                        float divisor) {
+    pdl_wait();
+    pdl_trigger();
+    quant_items(x, q, n, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x, ld_f32(amax_ptr), scale_out, divisor);
+}
+
+struct QuantOp {
+    static constexpr int N = 1;
+    const float* x;
+    uint8_t* q;
+    size_t n;
+    float* scale_out;
+    float* amax_out;
+    float divisor;
+    __device__ void pass1(float (&m)[1]) const { m[0] = amax_items(x, n, oc_tid(), OC_STEP); }
+    __device__ void pass2(const float (&m)[1]) const {
+        if (oc_tid() == 0) *amax_out = m[0];
+        quant_items(x, q, n, oc_tid(), OC_STEP, m[0], scale_out, divisor);
+    }
+};
 
 __global__ void __launch_bounds__(THREADS) dequant_kernel(const uint8_t* __restrict__ q, __half* __restrict__ out,
                                                           const float* __restrict__ scale_in, int n) {
@@ -217,12 +262,12 @@ int fp8_quantize_f32(const float* x, uint8_t* q, float* scale_out, float* amax_o
     if (convention != FP8_QUANT_AMAX_OVER_448 && convention != FP8_QUANT_UNIT) return (int)cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(q) & 15)) return (int)cudaErrorInvalidValue;
     cudaStream_t s = (cudaStream_t)stream;
-    cudaError_t e = cudaMemsetAsync(amax_out, 0, sizeof(float), s);
-    if (e != cudaSuccess) return (int)e;
-    if (n > 0) amax_kernel<<<grid_for(n / 4 + 1), THREADS, 0, s>>>(x, n, amax_out);
-    quant_kernel<<<grid_for(n / 16 + 1), THREADS, 0, s>>>(x, q, n, amax_out, scale_out,
-                                                           convention == FP8_QUANT_UNIT ? 1.0f : 448.0f);
-    return (int)cudaGetLastError();
+    const float divisor = convention == FP8_QUANT_UNIT ? 1.0f : 448.0f;
+    if (n * 4 <= OC_BYTES && oc_fits<QuantOp>()) return (int)oc_launch(QuantOp{x, q, n, scale_out, amax_out, divisor}, s);
+    cudaError_t e = launch_pdl(clear_word_kernel, dim3(1), dim3(1), 0, s, amax_out);
+    if (e == cudaSuccess) e = launch_pdl(amax_kernel, dim3(grid_for(n / 4 + 1)), dim3(THREADS), 0, s, x, n, amax_out);
+    if (e == cudaSuccess) e = launch_pdl(quant_kernel, dim3(grid_for(n / 16 + 1)), dim3(THREADS), 0, s, x, q, n, amax_out, scale_out, divisor);
+    return (int)e;
 }
 
 int fp8_dequantize_to_fp16(const void* input_fp8, void* output_fp16, const float* scale_in, int n) {

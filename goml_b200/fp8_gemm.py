@@ -46,6 +46,8 @@ def _init():
                 lib.fp8_gemm_accumulate_f32.argtypes = [i, i, i, p, p, p, f, p, p, p]
                 lib.fp8_gemm_swiglu.restype = i
                 lib.fp8_gemm_swiglu.argtypes = [i, i, i, p, p, p, f, p, p, p, p]
+                lib.fp8_gemm_swiglu_raise.restype = i
+                lib.fp8_gemm_swiglu_raise.argtypes = [i, i, i, p, p, p, f, p, p, p, p]
                 lib.fp8_gemm_fp8out.restype = i
                 lib.fp8_gemm_fp8out.argtypes = [i, i, i, p, p, p, f, p, p, p, p, p]
                 lib.fp8_gemm_device_status.restype = i
@@ -105,6 +107,13 @@ def FP8GEMMSwiGLU(M, F, K, A, B_interleaved, H, alpha=1.0, scale_a=0, scale_b=0,
     rc = _init().fp8_gemm_swiglu(M, F, K, A, B_interleaved, H, alpha, scale_a or None, scale_b or None, amax_out, stream or None)
     if rc != 0:
         raise FP8GEMMError(f"fp8_gemm_swiglu: CUDA error {rc}")
+
+
+def FP8GEMMSwiGLURaise(M, F, K, A, B_interleaved, H, alpha=1.0, scale_a=0, scale_b=0, amax=0, stream=0) -> None:
+    """FP8GEMMSwiGLU that raises *amax instead of clearing it first: the caller has zeroed the word."""
+    rc = _init().fp8_gemm_swiglu_raise(M, F, K, A, B_interleaved, H, alpha, scale_a or None, scale_b or None, amax, stream or None)
+    if rc != 0:
+        raise FP8GEMMError(f"fp8_gemm_swiglu_raise: CUDA error {rc}")
 
 
 def FP8GEMMFP8Out(M, N, K, A, B, D, alpha=1.0, scale_a=0, scale_b=0, scale_d=0, amax_d=0, stream=0) -> None:

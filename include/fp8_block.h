@@ -20,7 +20,7 @@
  *
  * Every op is two passes over its input (the per-tensor amax must be known before
  * the first code is written): pass 1 reduces amax (and the row statistics), pass 2
- * recomputes the values and writes codes.  Nothing but the codes, one scale and one
+ * recomputes the values and writes codes; two kernels, or one for a small tensor.  Nothing but the codes, one scale and one
  * amax per tensor (and, where stated, the updated residual stream) is written.
  *
  * All pointers are device pointers owned by the caller; calls are asynchronous on
@@ -58,6 +58,13 @@ FP8BLOCK_API int fp8_rmsnorm_quantize(const float* x, const void* residual_bf16,
                                       uint8_t* q, float* scale_out, float* amax_out, float* rstd_ws, int rows,
                                       int hidden, float eps, void* stream);
 
+/* The same without a residual, for the start of a block that updates its stream in place: h_out (NULL, x itself, or a
+ * buffer of its own) receives a copy of x while pass 1 reads it, and *zero_word (NULL or any fp32 word) is set to 0 for
+ * a later op of the chain that raises a maximum in it (fp8_gemm_swiglu_raise). */
+FP8BLOCK_API int fp8_rmsnorm_quantize_into(const float* x, float* h_out, const float* gamma, uint8_t* q, float* scale_out,
+                                           float* amax_out, float* rstd_ws, float* zero_word, int rows, int hidden, float eps,
+                                           void* stream);
+
 /* qkv [batch*seq_len, 3, heads, head_dim] bf16 (the QKV projection's output rows)
  *   -> RoPE on Q and K -> q_out, k_out, v_out [batch*heads, seq_len, head_dim] e4m3,
  * each with its own per-tensor scale: scales[3], amaxes[3] (order Q, K, V).
@@ -65,6 +72,14 @@ FP8BLOCK_API int fp8_rmsnorm_quantize(const float* x, const void* residual_bf16,
 FP8BLOCK_API int fp8_rope_quantize_qkv(const void* qkv_bf16, const float* cos_tab, const float* sin_tab,
                                        uint8_t* q_out, uint8_t* k_out, uint8_t* v_out, float* scales, float* amaxes,
                                        int batch, int seq_len, int heads, int head_dim, void* stream);
+
+/* The same, with the K and V codes also stored into a KV cache: k_cache, v_cache [batch, heads, s_max, head_dim]
+ * (positions 0 .. seq_len-1; s_max >= seq_len, 16-byte aligned), cache_scales[2] = the K and V scales, cache_lens[batch] =
+ * seq_len. */
+FP8BLOCK_API int fp8_rope_quantize_qkv_cache(const void* qkv_bf16, const float* cos_tab, const float* sin_tab,
+                                             uint8_t* q_out, uint8_t* k_out, uint8_t* v_out, float* scales, float* amaxes,
+                                             uint8_t* k_cache, uint8_t* v_cache, float* cache_scales, int32_t* cache_lens,
+                                             int batch, int seq_len, int s_max, int heads, int head_dim, void* stream);
 
 /* Attention output o [batch*heads, seq_len, head_dim] fp16 -> token-major codes
  * q [batch*seq_len, heads*head_dim] e4m3 (the O projection's A operand).

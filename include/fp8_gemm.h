@@ -79,6 +79,12 @@ FP8GEMM_API int fp8_gemm_accumulate_f32(int M, int N, int K, const void* A, cons
 FP8GEMM_API int fp8_gemm_swiglu(int M, int F, int K, const void* A, const void* B_interleaved, void* H, float alpha,
                                 const float* scale_a, const float* scale_b, float* amax_out, void* stream);
 
+/* The same, but *amax is only raised: it holds zero, or a maximum that is to be kept, when the call is made.  Spares the
+ * clearing (a memset between two kernels) where an earlier call of the chain zeroes the word anyway
+ * (fp8_rmsnorm_quantize_into). */
+FP8GEMM_API int fp8_gemm_swiglu_raise(int M, int F, int K, const void* A, const void* B_interleaved, void* H, float alpha,
+                                      const float* scale_a, const float* scale_b, float* amax, void* stream);
+
 /* Additive extension: e4m3 output with delayed scaling, the epilogue of the reference's cuBLASLt wrapper
  * (fp8_matmul_fp8out, libs1/cublas_lt_wrapper_v3.c:157-229: D type CUDA_R_8F_E4M3 with D_SCALE_POINTER and
  * AMAX_D_POINTER):

@@ -140,3 +140,65 @@ def test_rejects_bad_arguments(cuda, built_libs):
         BG.SwiGLUQuantize(p, p, p, p, 2, 40)                                 # ffn_hidden not a multiple of 16
     with pytest.raises(BG.BlockGlueError):
         BG.ResidualAdd(p, p, 12)                                             # n not a multiple of 8
+
+
+@pytest.mark.parametrize("rows,hidden", [(1, 16), (16, 1040), (17, 2048), (64, 528), (65, 2512), (20, 4096), (21, 4096), (300, 2064)])
+def test_rmsnorm_into_copies_the_stream_and_zeroes_the_word(cuda, built_libs, rows, hidden):
+    # rows per warp group (16 / 64 rows), and both sides of the size up to which one cluster does the op
+    from goml_b200 import block_glue as BG
+    cfg = f"rmsinto{rows}_{hidden}"
+    x = O.seeded_normal("x", (rows, hidden), config=cfg).astype(np.float32)
+    gamma = (1.0 + 0.1 * O.seeded_normal("g", (hidden,), config=cfg)).astype(np.float32)
+    xd, gd = dev(x), dev(gamma)
+    h = torch.full((rows + 1, hidden), 5.0, device="cuda")
+    q = torch.full((rows + 1, hidden), 0xAA, dtype=torch.uint8, device="cuda")
+    sa = torch.full((3,), 7.0, device="cuda")
+    rstd = torch.empty(rows, device="cuda")
+    BG.RMSNormQuantizeInto(xd.data_ptr(), h.data_ptr(), gd.data_ptr(), q.data_ptr(), sa.data_ptr(), sa.data_ptr() + 4, rstd.data_ptr(),
+                           sa.data_ptr() + 8, rows, hidden, 1e-5)
+    torch.cuda.synchronize()
+    codes, scale, amax, _, _ = glue.rmsnorm_quantize(x, None, gamma, 1e-5)
+    assert abs(sa[0].item() - scale) <= 1e-6 * scale and abs(sa[1].item() - amax) <= 1e-6 * amax and sa[2].item() == 0.0
+    nearly_same_codes(q.cpu().numpy()[:rows], codes, frac=max(1e-4, 1.5 / codes.size))   # one code of a tensor too small for the share
+    assert np.array_equal(h.cpu().numpy()[:rows], x) and torch.all(h[rows] == 5.0) and torch.all(q[rows] == 0xAA)
+
+
+@pytest.mark.parametrize("B,S,H,hd", [(1, 1, 1, 64), (2, 72, 4, 128), (2, 73, 8, 128), (3, 130, 5, 64)])
+def test_rope_quantize_into_cache(cuda, built_libs, B, S, H, hd):
+    from goml_b200 import block_glue as BG
+    cfg = f"ropecache{B}_{S}_{H}_{hd}"
+    s_max = S + 5
+    qkv = glue.bf16_values(O.seeded_normal("qkv", (B * S, 3, H, hd), config=cfg) * np.array([1.0, 3.0, 0.25])[None, :, None, None])
+    c_ref, s_ref = glue.rope_table(S, hd, 10000.0)
+    cos, sin, qkv_d = dev(c_ref), dev(s_ref), dev(qkv, torch.bfloat16)
+    out = [torch.full((B * H, S, hd), 0xAA, dtype=torch.uint8, device="cuda") for _ in range(3)]
+    cache = [torch.full((B, H, s_max, hd), 0xAA, dtype=torch.uint8, device="cuda") for _ in range(2)]
+    s6, cs = torch.full((6,), 9.0, device="cuda"), torch.full((2,), 9.0, device="cuda")
+    lens = torch.full((B,), -1, dtype=torch.int32, device="cuda")
+    BG.RopeQuantizeQKVCache(qkv_d.data_ptr(), cos.data_ptr(), sin.data_ptr(), *[t.data_ptr() for t in out], s6.data_ptr(), s6.data_ptr() + 12,
+                            *[t.data_ptr() for t in cache], cs.data_ptr(), lens.data_ptr(), B, S, s_max, H, hd)
+    torch.cuda.synchronize()
+    want = glue.rope_quantize_qkv(qkv, c_ref, s_ref, B, S, H, hd)
+    for w in range(3):
+        assert s6[w].item() == want[w][1] and s6[3 + w].item() == want[w][2]
+        assert np.array_equal(out[w].cpu().numpy(), want[w][0]), w
+    for w in range(2):
+        assert torch.equal(cache[w][:, :, :S].reshape(B * H, S, hd), out[1 + w]) and torch.all(cache[w][:, :, S:] == 0xAA)
+        assert cs[w].item() == want[1 + w][1]
+    assert lens.tolist() == [S] * B
+    with pytest.raises(BG.BlockGlueError):   # a cache shorter than the prompt
+        BG.RopeQuantizeQKVCache(qkv_d.data_ptr(), cos.data_ptr(), sin.data_ptr(), *[t.data_ptr() for t in out], s6.data_ptr(), s6.data_ptr() + 12,
+                                *[t.data_ptr() for t in cache], cs.data_ptr(), lens.data_ptr(), B, S, S - 1, H, hd)
+
+
+@pytest.mark.parametrize("B,S,H,hd", [(1, 1, 1, 16), (2, 64, 16, 128), (1, 129, 16, 128), (3, 50, 7, 80)])
+def test_permute_quantize_on_both_sides_of_one_cluster(cuda, built_libs, B, S, H, hd):
+    from goml_b200 import block_glue as BG
+    o = O.round_fp16(O.seeded_normal("o", (B * H, S, hd), config=f"permoc{B}_{S}_{H}_{hd}")).astype(np.float32)
+    q = torch.full((B * S, H * hd), 0xAA, dtype=torch.uint8, device="cuda")
+    sa = torch.full((2,), 9.0, device="cuda")
+    od = dev(o, torch.float16)
+    BG.PermuteQuantizeHeads(od.data_ptr(), q.data_ptr(), sa.data_ptr(), sa.data_ptr() + 4, B, S, H, hd)
+    torch.cuda.synchronize()
+    codes, scale, amax = glue.permute_quantize_heads(o, B, S, H, hd)
+    assert sa.tolist() == [scale, amax] and np.array_equal(q.cpu().numpy(), codes)

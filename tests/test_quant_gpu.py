@@ -95,3 +95,25 @@ def test_codes_and_scale_equal_the_reference_quantiser_kernel(cuda, built_libs, 
     # and the CPU restatement agrees with all three
     oq, oscale, _ = O.quantize_f32(x.astype(np.float32), 0)
     assert np.float32(wscale.item()) == oscale and np.array_equal(want[:n].cpu().numpy(), oq)
+
+
+@pytest.mark.parametrize("n", [1, 15, 17, 4099, 131072 + 3, 196608, 196608 + 1, 1 << 20])
+@pytest.mark.parametrize("where", ["first", "last"])
+def test_one_cluster_and_two_kernels_give_the_oracles_codes(cuda, built_libs, n, where):
+    # both sides of the size up to which one cluster does both passes (196608 values); the maximum at either end, and a NaN,
+    # which never becomes the maximum
+    from goml_b200 import quantize as Q
+    x = O.seeded_normal("x", (n,), config=f"oc{n}").astype(np.float32)
+    x[0 if where == "first" else -1] = -9.5
+    xd = torch.from_numpy(x).cuda()
+    q = torch.full((n + 16,), 0xAA, dtype=torch.uint8, device="cuda")
+    sa = torch.full((2,), 99.0, device="cuda")
+    Q.QuantizeF32ToF8E4M3(xd.data_ptr(), q.data_ptr(), sa.data_ptr(), sa.data_ptr() + 4, n, 0)
+    torch.cuda.synchronize()
+    codes, scale, amax = O.quantize_f32(x)
+    assert sa.tolist() == [scale, amax] and np.array_equal(q.cpu().numpy()[:n], codes) and torch.all(q[n:] == 0xAA)
+    if n > 2:
+        xd[n // 2] = float("nan")
+        Q.QuantizeF32ToF8E4M3(xd.data_ptr(), q.data_ptr(), sa.data_ptr(), sa.data_ptr() + 4, n, 0)
+        torch.cuda.synchronize()
+        assert sa.tolist() == [scale, amax]
