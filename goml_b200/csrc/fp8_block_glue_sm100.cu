@@ -642,6 +642,12 @@ __device__ __forceinline__ int dec_position(const DecAppend& a, int b) {
     const int cap = a.block_table ? a.page_size * a.max_pages : a.s_max;
     return (pos >= 0 && pos < cap && pos < a.table_rows) ? pos : -1;
 }
+// length of sequence b after the step; an inactive slot keeps its length: 0 for a negative position, the capacity for a full cache
+__device__ __forceinline__ int dec_length(const DecAppend& a, int b) {
+    const int raw = ld_s32(a.positions + b);
+    const int cap = a.block_table ? a.page_size * a.max_pages : a.s_max;
+    return dec_position(a, b) >= 0 ? raw + 1 : (raw < 0 ? 0 : min(raw, cap));
+}
 __device__ __forceinline__ void dec_values(const DecAppend& a, int b, int slot, int c, int pos, float* y) {
     const int half = a.hd / 2;
     const size_t row = ((size_t)b * (a.hq + 2 * a.hkv) + slot) * a.hd;
@@ -707,12 +713,7 @@ __device__ __forceinline__ void dec_append_items(const DecAppend& a, uint32_t ti
         a.cph.divmod(it, q, c);
         a.slots.divmod(q, b, slot);
         const int pos = dec_position(a, (int)b);
-        if (slot == 0 && c == 0 && a.seq_lens_out) {
-            // an inactive slot keeps its length: 0 for a negative position, the capacity for a full cache
-            const int raw = ld_s32(a.positions + b);
-            const int cap = a.block_table ? a.page_size * a.max_pages : a.s_max;
-            a.seq_lens_out[b] = pos >= 0 ? pos + 1 : (raw < 0 ? 0 : min(raw, cap));
-        }
+        if (slot == 0 && c == 0 && a.seq_lens_out && a.seq_lens_out != a.positions) a.seq_lens_out[b] = dec_length(a, (int)b);
         if ((int)slot < a.hq) {
             uint8_t* dst = a.q_out + ((size_t)b * a.hq + slot) * a.hd;
             if (pos < 0) {  // an inactive sequence: zero codes, nothing appended
@@ -770,8 +771,19 @@ struct DecOp {
     __device__ void pass2(const float (&m)[1]) const {
         if (oc_tid() == 0) *a.q_amax = m[0];
         dec_append_items(a, oc_tid(), OC_STEP, m[0]);
+        if (a.seq_lens_out == a.positions) {   // in place: once no thread reads a position any more
+            __syncwarp();
+            oc_arrive();
+            oc_wait();
+            for (uint32_t b = oc_tid(); b < (uint32_t)a.batch; b += OC_STEP) a.seq_lens_out[b] = dec_length(a, (int)b);
+        }
     }
 };
+__global__ void __launch_bounds__(THREADS) dec_lengths_kernel(const DecAppend a) {
+    pdl_wait();
+    pdl_trigger();
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < a.batch; b += gridDim.x * blockDim.x) a.seq_lens_out[b] = dec_length(a, b);
+}
 
 // ---------------------------------------------------------------------------------- attention output: permute + quantise
 // item = 16 consecutive elements of one (token, head); out index order so that stores are contiguous
@@ -1095,6 +1107,8 @@ int fp8_decode_rope_append(const fp8_decode_append_args_t* g) {
     cudaError_t e = clear_words(a.q_amax, 1, s);
     if (e == cudaSuccess && items > 0) e = launch_pdl(dec_q_amax_kernel, dim3(grid_for(items)), dim3(THREADS), 0, s, a);
     if (e == cudaSuccess) e = launch_pdl(dec_append_kernel, dim3(grid_for(items)), dim3(THREADS), 0, s, a);
+    if (e == cudaSuccess && a.seq_lens_out == a.positions && a.batch > 0)
+        e = launch_pdl(dec_lengths_kernel, dim3(grid_for((size_t)a.batch)), dim3(THREADS), 0, s, a);
     return (int)e;
 }
 

@@ -98,7 +98,14 @@ class FP8KVCache:
         self.v = torch.zeros_like(self.k)
         self.scales = torch.ones(2, dtype=torch.float32, device=device)      # k_scale, v_scale
         self.lens = torch.zeros(batch, dtype=torch.int32, device=device)     # keys cached per sequence
-        self._lens_next = torch.zeros_like(self.lens)
+
+    def takes(self, batch: int, heads: int, S: int, hd: int) -> bool:
+        """Whether a prompt's codes can be written straight into this cache: dense buffers of the shapes it was made with."""
+        shape = (batch, heads, self.s_max, hd)
+        return (S <= self.s_max and all(t.shape == shape and t.dtype == torch.uint8 and t.is_contiguous() and t.is_cuda and t.data_ptr() % 16 == 0
+                                        for t in (self.k, self.v))
+                and self.scales.dtype == torch.float32 and self.scales.shape == (2,) and self.scales.is_contiguous() and self.scales.is_cuda
+                and self.lens.dtype == torch.int32 and self.lens.shape == (batch,) and self.lens.is_contiguous() and self.lens.is_cuda)
 
     def fill(self, k_codes, v_codes, scales, S: int) -> None:
         """Prompt phase: K/V codes [batch*heads, S, hd] as the prefill quantiser wrote them, and their two scales."""
@@ -106,6 +113,28 @@ class FP8KVCache:
         self.v[:, :, :S].copy_(v_codes.view(self.B, self.H, S, self.hd))
         self.scales.copy_(scales)
         self.lens.fill_(S)
+
+
+def _scratch(dev, *sizes):
+    """One allocation cut into 256-byte aligned pieces: (the buffer, their addresses).  A call has a dozen temporaries, and
+    drawing each from the allocator took about a third of a decode step's host time."""
+    offsets, total = [], 0
+    for n in sizes:
+        offsets.append(total)
+        total += (n + 255) & -256
+    buf = torch.empty(total, dtype=torch.uint8, device=dev)
+    base = buf.data_ptr()
+    return (buf, *[base + o for o in offsets])
+
+
+def _stream_start(x: torch.Tensor, rows: int, d: int):
+    """(source, h) of a block's residual stream: h is written by the first RMSNorm while it reads x, or is a copy already
+    (source = h) where x is not what that kernel reads."""
+    if (x.dtype == torch.float32 and x.is_contiguous() and x.data_ptr() % 32 == 0 and x.numel() == rows * d
+            and not (x.requires_grad and torch.is_grad_enabled())):
+        return x, torch.empty_like(x)
+    h = x.float().clone()
+    return h, h
 
 
 class FP8DecoderBlock:
@@ -148,29 +177,30 @@ class FP8DecoderBlock:
         """The block with every glue op fused with the quantiser of its consumer and both residual adds done in
         the GEMM epilogues, SwiGLU in the gate/up GEMM's epilogue: 9 library calls, no torch math.
         With `cache`, the K and V codes of the prompt and their scales are also stored there for decode_step."""
-        dev, T, d, H, hd, Fh = x.device, B * S, self.d, self.H, self.hd, self.F
+        T, d, H, hd = B * S, self.d, self.H, self.hd
         sh = torch.cuda.current_stream().cuda_stream
-        u8 = lambda *shape: torch.empty(shape, dtype=torch.uint8, device=dev)
-        sa = lambda n=2: torch.empty(n, dtype=torch.float32, device=dev)   # scale and amax words: every entry point clears its own amax
-        h = x.float().clone()                                   # residual stream, updated in place
-        rstd = torch.empty(T, dtype=torch.float32, device=dev)
-        cos, sin = self.rope_tables(S, dev)
+        n = T * d
+        # codes of the normed input, QKV projection, codes of Q, K and V, attention output, its codes, rstd, scales and maxima
+        buf, xc, qkv, qc, kc, vc, o, oc, rstd, sc = _scratch(x.device, n, 6 * n, n, n, n, 2 * n, n, 4 * T, 40)
+        src, h = _stream_start(x, T, d)                         # residual stream, updated in place
+        cos, sin = self.rope_tables(S, x.device)
         # attention half
-        xq = FP8Tensor(u8(T, d), sa())
-        BG.RMSNormQuantize(h.data_ptr(), 0, 0, self.norm1.data_ptr(), xq.codes.data_ptr(), xq.sa.data_ptr(), xq.sa.data_ptr() + 4,
-                           rstd.data_ptr(), T, d, self.eps, sh)
-        qkv = self.qkv.forward_codes(xq, T)                      # [T, 3, H, hd] bf16
-        qc, kc, vc, s3 = u8(B * H, S, hd), u8(B * H, S, hd), u8(B * H, S, hd), sa(6)   # scales[3], amaxes[3]
-        BG.RopeQuantizeQKV(qkv.data_ptr(), cos.data_ptr(), sin.data_ptr(), qc.data_ptr(), kc.data_ptr(), vc.data_ptr(),
-                           s3.data_ptr(), s3.data_ptr() + 12, B, S, H, hd, sh)
-        if cache is not None:
-            cache.fill(kc, vc, s3[1:3], S)
-        o = torch.empty((B * H, S, hd), dtype=torch.float16, device=dev)
-        self.fa.ForwardEx(qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), o.data_ptr(), 0, B * H, S, hd, 1, 0, 1.0 / math.sqrt(hd), 1.0,
-                          s3.data_ptr(), s3.data_ptr() + 4, s3.data_ptr() + 8, sh)
-        oq = FP8Tensor(u8(T, d), sa())
-        BG.PermuteQuantizeHeads(o.data_ptr(), oq.codes.data_ptr(), oq.sa.data_ptr(), oq.sa.data_ptr() + 4, B, S, H, hd, sh)
-        self.o.accumulate_into(oq, T, h)                         # h += attention projection, in the GEMM epilogue
+        BG.RMSNormQuantizeInto(src.data_ptr(), h.data_ptr(), self.norm1.data_ptr(), xc, sc, sc + 4, rstd, 0, T, d, self.eps, sh)
+        G.FP8GEMMScaled(T, 3 * d, d, xc, self.qkv.w.codes.data_ptr(), qkv, 1.0, sc, self.qkv.w.scale_ptr, G.OutBF16, sh)   # [T, 3, H, hd] bf16
+        s3 = sc + 8                                             # scales[3], amaxes[3]
+        if cache is not None and cache.takes(B, H, S, hd):
+            BG.RopeQuantizeQKVCache(qkv, cos.data_ptr(), sin.data_ptr(), qc, kc, vc, s3, s3 + 12, cache.k.data_ptr(), cache.v.data_ptr(),
+                                    cache.scales.data_ptr(), cache.lens.data_ptr(), B, S, cache.s_max, H, hd, sh)
+        else:
+            BG.RopeQuantizeQKV(qkv, cos.data_ptr(), sin.data_ptr(), qc, kc, vc, s3, s3 + 12, B, S, H, hd, sh)
+            if cache is not None:
+                view = lambda p, nbytes: buf[p - buf.data_ptr():p - buf.data_ptr() + nbytes]
+                cache.fill(view(kc, n), view(vc, n), view(s3 + 4, 8).view(torch.float32), S)
+        self.fa.ForwardEx(qc, kc, vc, o, 0, B * H, S, hd, 1, 0, 1.0 / math.sqrt(hd), 1.0, s3, s3 + 4, s3 + 8, sh)
+        BG.PermuteQuantizeHeads(o, oc, sc + 32, sc + 36, B, S, H, hd, sh)
+        # h += attention projection, in the GEMM epilogue
+        G.FP8GEMMAccumulateF32(T, d, d, oc, self.o.w.codes.data_ptr(), h.data_ptr(), 1.0, sc + 32, self.o.w.scale_ptr, sh)
+        del buf   # the feed-forward half may take its place: same stream
         return self._feed_forward(h, T)
 
     def decode_step(self, x: torch.Tensor, cache: FP8KVCache) -> torch.Tensor:
@@ -178,48 +208,37 @@ class FP8DecoderBlock:
         position cache.lens[b] (quantised with the cache's scales) and cache.lens advanced.  Ten library calls:
         RMSNorm+quantise -> QKV GEMM -> RoPE+quantise+append -> decode attention -> quantise -> O GEMM (residual in the
         epilogue) -> the feed-forward half of forward_fused."""
-        dev, B, d, H, hd = x.device, x.shape[0], self.d, self.H, self.hd
+        B, d, H, hd = x.shape[0], self.d, self.H, self.hd
         assert (B, H, hd) == (cache.B, cache.H, cache.hd)
         sh = torch.cuda.current_stream().cuda_stream
-        u8 = lambda *shape: torch.empty(shape, dtype=torch.uint8, device=dev)
-        sa = lambda n=2: torch.empty(n, dtype=torch.float32, device=dev)
-        h = x.float().clone()
-        rstd = torch.empty(B, dtype=torch.float32, device=dev)
-        cos, sin = self.rope_tables(cache.s_max, dev)
-        xq = FP8Tensor(u8(B, d), sa())
-        BG.RMSNormQuantize(h.data_ptr(), 0, 0, self.norm1.data_ptr(), xq.codes.data_ptr(), xq.sa.data_ptr(), xq.sa.data_ptr() + 4,
-                           rstd.data_ptr(), B, d, self.eps, sh)
-        qkv = self.qkv.forward_codes(xq, B)                      # [B, (H + 2H) * hd] bf16: Q heads, K heads, V heads
-        qc, qs = u8(B, H, hd), sa()
-        BG.DecodeRopeAppend(qkv.data_ptr(), cos.data_ptr(), sin.data_ptr(), cache.lens.data_ptr(), qc.data_ptr(), qs.data_ptr(),
-                            qs.data_ptr() + 4, cache.k.data_ptr(), cache.v.data_ptr(), cache.scales.data_ptr(), cache.scales.data_ptr() + 4,
-                            B, H, H, hd, cache.s_max, cache.s_max, seq_lens_out=cache._lens_next.data_ptr(), stream=sh)
-        cache.lens.copy_(cache._lens_next)    # a device copy, not a pointer swap: the step can be replayed from a CUDA graph
-        o = torch.empty((B, H, hd), dtype=torch.float16, device=dev)
-        self.fa.Decode(qc.data_ptr(), cache.k.data_ptr(), cache.v.data_ptr(), o.data_ptr(), 0, cache.lens.data_ptr(), B, H, H, hd,
-                       cache.s_max, 0, 1.0 / math.sqrt(hd), 1.0, qs.data_ptr(), cache.scales.data_ptr(), cache.scales.data_ptr() + 4, sh)
-        oq = FP8Tensor(u8(B, d), sa())
-        BG.PermuteQuantizeHeads(o.data_ptr(), oq.codes.data_ptr(), oq.sa.data_ptr(), oq.sa.data_ptr() + 4, B, 1, H, hd, sh)
-        self.o.accumulate_into(oq, B, h)
+        n = B * d
+        buf, xc, qkv, qc, o, oc, rstd, sc = _scratch(x.device, n, 6 * n, n, 2 * n, n, 4 * B, 24)
+        src, h = _stream_start(x, B, d)
+        cos, sin = self.rope_tables(cache.s_max, x.device)
+        BG.RMSNormQuantizeInto(src.data_ptr(), h.data_ptr(), self.norm1.data_ptr(), xc, sc, sc + 4, rstd, 0, B, d, self.eps, sh)
+        # [B, (H + 2H) * hd] bf16: Q heads, K heads, V heads
+        G.FP8GEMMScaled(B, 3 * d, d, xc, self.qkv.w.codes.data_ptr(), qkv, 1.0, sc, self.qkv.w.scale_ptr, G.OutBF16, sh)
+        k, v, lens, ks = cache.k.data_ptr(), cache.v.data_ptr(), cache.lens.data_ptr(), cache.scales.data_ptr()
+        # the lengths advance in place, on the device: the step can be replayed from a CUDA graph
+        BG.DecodeRopeAppend(qkv, cos.data_ptr(), sin.data_ptr(), lens, qc, sc + 8, sc + 12, k, v, ks, ks + 4, B, H, H, hd,
+                            cache.s_max, cache.s_max, seq_lens_out=lens, stream=sh)
+        self.fa.Decode(qc, k, v, o, 0, lens, B, H, H, hd, cache.s_max, 0, 1.0 / math.sqrt(hd), 1.0, sc + 8, ks, ks + 4, sh)
+        BG.PermuteQuantizeHeads(o, oc, sc + 16, sc + 20, B, 1, H, hd, sh)
+        G.FP8GEMMAccumulateF32(B, d, d, oc, self.o.w.codes.data_ptr(), h.data_ptr(), 1.0, sc + 16, self.o.w.scale_ptr, sh)
+        del buf
         return self._feed_forward(h, B)
 
     def _feed_forward(self, h: torch.Tensor, T: int) -> torch.Tensor:
         """h [T, d] fp32 += W_down(silu(W_gate n) * W_up n), n = RMSNorm(h): in place, three GEMM-library calls."""
-        dev, d, Fh = h.device, self.d, self.F
+        d, Fh = self.d, self.F
         sh = torch.cuda.current_stream().cuda_stream
-        u8 = lambda *shape: torch.empty(shape, dtype=torch.uint8, device=dev)
-        sa = lambda n=2: torch.empty(n, dtype=torch.float32, device=dev)
-        rstd = torch.empty(T, dtype=torch.float32, device=dev)
-        xq2 = FP8Tensor(u8(T, d), sa())
-        BG.RMSNormQuantize(h.data_ptr(), 0, 0, self.norm2.data_ptr(), xq2.codes.data_ptr(), xq2.sa.data_ptr(),
-                           xq2.sa.data_ptr() + 4, rstd.data_ptr(), T, d, self.eps, sh)
-        hq = FP8Tensor(u8(T, Fh), sa())
-        hb = torch.empty((T, Fh), dtype=torch.bfloat16, device=dev)
+        buf, xc, hb, hc, rstd, sc = _scratch(h.device, T * d, 2 * T * Fh, T * Fh, 4 * T, 16)
+        # the norm zeroes the word that the gate/up epilogue raises max|.| in
+        BG.RMSNormQuantizeInto(h.data_ptr(), 0, self.norm2.data_ptr(), xc, sc, sc + 4, rstd, sc + 12, T, d, self.eps, sh)
         # gate/up projections with silu(gate) * up and max|.| in the GEMM epilogue, then one quantiser pass
-        G.FP8GEMMSwiGLU(T, Fh, d, xq2.codes.data_ptr(), self.gate_up_interleaved.data_ptr(), hb.data_ptr(), 1.0, xq2.scale_ptr,
-                        self.gate_up.w.scale_ptr, hq.sa.data_ptr() + 4, sh)
-        BG.QuantizeBF16(hb.data_ptr(), hq.codes.data_ptr(), hq.sa.data_ptr(), hq.sa.data_ptr() + 4, T * Fh, sh)
-        self.down.accumulate_into(hq, T, h)                      # h += feed-forward output
+        G.FP8GEMMSwiGLURaise(T, Fh, d, xc, self.gate_up_interleaved.data_ptr(), hb, 1.0, sc, self.gate_up.w.scale_ptr, sc + 12, sh)
+        BG.QuantizeBF16(hb, hc, sc + 8, sc + 12, T * Fh, sh)
+        G.FP8GEMMAccumulateF32(T, d, Fh, hc, self.down.w.codes.data_ptr(), h.data_ptr(), 1.0, sc + 8, self.down.w.scale_ptr, sh)   # h += feed-forward output
         return h
 
     def __call__(self, x: torch.Tensor, B: int, S: int, cache: "FP8KVCache | None" = None) -> torch.Tensor:

@@ -118,7 +118,8 @@ FP8BLOCK_API int fp8_residual_add(float* x, const void* y_bf16, size_t n, void* 
  *   k_scale, v_scale: device pointers to the dequantisation scales the cache was written with; the new codes are
  *              e4m3_rn_satfinite(clamp(x / scale)), i.e. values beyond 448 * scale saturate;
  *   seq_lens_out [batch] int32 or NULL: positions[b] + 1 for active sequences, the lengths to pass to fa_decode
- *              next (and the next step's positions); must not alias positions.
+ *              next (and the next step's positions); may be `positions` itself (the lengths then advance in place)
+ *              but must not overlap it otherwise.
  * head_dim 64 or 128.  Two passes over the Q part (amax, then codes); K and V are written in the second. */
 typedef struct fp8_decode_append_args {
     const void* qkv_bf16;

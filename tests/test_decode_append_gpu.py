@@ -137,3 +137,30 @@ def test_generation_loop_append_then_decode(cuda, built_libs, fa_ctx):
         maxabs, meanrel = O.error_stats(o.double().cpu().numpy(), ref)
         assert maxabs <= 2e-2 and meanrel <= 1e-2 and np.abs(lse.double().cpu().numpy() - rl).max() <= 5e-3, (step, maxabs, meanrel)
         positions = positions + 1
+
+
+@pytest.mark.parametrize("B,Hq,Hkv", [(1, 1, 1), (3, 8, 2), (40, 32, 8)])
+def test_lengths_advance_in_place(cuda, built_libs, B, Hq, Hkv):
+    # seq_lens_out = positions, in the one-cluster kernel and in the two-kernel path (40 sequences of 48 head slots): the same
+    # codes and lengths as with a separate array, inactive and full sequences among them
+    from goml_b200 import block_glue as BG
+    Smax, hd = 64, 128
+    g = torch.Generator(device="cuda").manual_seed(B)
+    qkv = torch.randn(B, (Hq + 2 * Hkv) * hd, generator=g, device="cuda").bfloat16()
+    cos, sin = rope_tables(Smax, hd)
+    positions = ((torch.arange(B, device="cuda") * 7 + 5) % (Smax + 3) - 1).to(torch.int32)
+    sc = torch.tensor([0.0, 0.0, 0.01, 0.02], device="cuda")
+    res = []
+    for in_place in (False, True):
+        k, v = (torch.zeros(B, Hkv, Smax, hd, dtype=torch.uint8, device="cuda") for _ in range(2))
+        q = torch.zeros(B, Hq, hd, dtype=torch.uint8, device="cuda")
+        pos = positions.clone()
+        lens = pos if in_place else torch.full_like(pos, -7)
+        BG.DecodeRopeAppend(qkv.data_ptr(), cos.data_ptr(), sin.data_ptr(), pos.data_ptr(), q.data_ptr(), sc.data_ptr(), sc.data_ptr() + 4,
+                            k.data_ptr(), v.data_ptr(), sc.data_ptr() + 8, sc.data_ptr() + 12, B, Hq, Hkv, hd, Smax, Smax,
+                            seq_lens_out=lens.data_ptr())
+        torch.cuda.synchronize()
+        res.append((k, v, q, lens, sc.clone()))
+    assert all(torch.equal(a, b) for a, b in zip(*res))
+    p = positions.tolist()
+    assert res[0][3].tolist() == [0 if x < 0 else min(x + 1, Smax) for x in p]
