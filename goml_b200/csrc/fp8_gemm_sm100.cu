@@ -14,6 +14,7 @@
 //
 // One persistent CTA per SM walks output tiles in an order that keeps a band of
 // A rows and a few B panels resident in L2.  Every CTA loads its own tiles; no thread-block clusters.
+// Few rows of A go to the kernel of fp8_gemm_skinny.cuh.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -726,8 +727,8 @@ int launch(int M, int N, int K, const void* A, const void* B, void* C, float alp
     const bool split_tail = (bn == 256) && !pair && tiles > st.num_sms && rem > 0 && 2 * rem <= st.num_sms;
     p.split_from = (int)(split_tail ? tiles - rem : tiles);
     p.num_units = (int)(split_tail ? tiles + rem : tiles);
-    // Split-K: a problem with fewer tiles than half the SMs and a long K (the O and down projections of a decode
-    // step: 16 x 4096 x 11008 is 64 tiles) leaves most SMs idle while each busy one streams a long panel of B.
+    // Split-K: a problem with fewer tiles than half the SMs and a long K (the down projection of a 256-token prompt through a
+    // half-width block: 256 x 2048 x 5504) leaves most SMs idle while each busy one streams a long panel of B.
     // Where the result is added into X by TMA reduce anyway, slices of K go to different CTAs and each adds its
     // partial sum (the order of those fp32 additions is then not fixed from run to run).
     const int k_stages = (p.k_blocks + Tile_KSUB(bn) - 1) / Tile_KSUB(bn);
