@@ -9,12 +9,13 @@
 //    holds 16 KB of weights and only 128 bytes per token, and every weight byte is read once;
 //  * the K range of a 128-row tile is cut over a thread-block cluster of 1 to 8 CTAs; the fp32 partial sums meet in
 //    distributed shared memory and are added in rank order (no atomics: the result does not depend on timing);
-//  * all CTAs are resident at once, up to two to an SM, so the kernel is one wave of equal streams (an SM takes in about
+//  * all CTAs are resident at once, up to three to an SM, so the kernel is one wave of equal streams (an SM takes in about
 //    57 bytes a nanosecond, so weights have to be spread over nearly all of them to reach the 6.5 TB/s of HBM);
 //  * the kernel starts before its predecessor on the stream has drained and asks for its first weight tiles to be
 //    brought into L2 while the small kernel ahead (a quantiser, usually) still runs.
 // What is left is 3 us of start, fill and finish beside the stream: M = 16, 8192 x 8192 16.7 -> 13.7 us (floor 10.3),
-// 11008 x 4096 12.8 -> 10.3 (6.9), 4096 x 11008 12.9 -> 10.8 (6.9), 4096 x 4096 7.8 -> 6.1 (2.6).
+// 12288 x 4096 13.3 -> 11.1 (7.7), 22016 x 4096 with SwiGLU
+// 21.9 -> 19.0 (13.8), 11008 x 4096 12.8 -> 10.3 (6.9), 4096 x 11008 12.9 -> 10.8 (6.9), 4096 x 4096 7.8 -> 6.1 (2.6).
 #pragma once
 
 namespace skinny {
@@ -28,7 +29,8 @@ constexpr int PREFETCH_BLOCKS = 16;         // k-blocks per CTA asked for ahead 
 constexpr int THREADS = 192;                // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2-5: read the accumulators back
 constexpr int TAIL_BYTES = 1024 /*align*/ + 512 /*barriers*/;
 constexpr int SMEM_ONE = 227 * 1024;        // of one CTA when it has the SM to itself
-constexpr int SMEM_TWO = 112 * 1024;        // of one of two CTAs on an SM
+// shared memory of one of up to three CTAs on an SM (228 KB, 1 KB of it the system's for each CTA)
+constexpr int smem_of(int per_sm) { return per_sm == 1 ? SMEM_ONE : per_sm == 2 ? 112 * 1024 : 74 * 1024; }
 
 struct Params {
     GemmParams g;
@@ -334,7 +336,7 @@ inline Kernel kernel_for(int split) {
 }
 
 // clusters of each size that are resident at once with one CTA to an SM (a cluster stays inside one group of SMs, so this
-// is less than SMs / size); with two CTAs to an SM it is at least twice as many
+// is less than SMs / size); with n CTAs to an SM it is at least n times as many
 struct Fit {
     int one[MAX_SPLIT + 1] = {};
 };
@@ -371,7 +373,7 @@ inline cudaError_t init(Fit* fit) {
 // How a problem is cut, or split = 0 where the square kernel is the faster one.
 struct Plan {
     int split = 0;
-    bool two = false;   // two CTAs to an SM, each with half of its shared memory
+    int per_sm = 1;     // CTAs that share an SM and its shared memory
 };
 inline Plan plan(int M, int N, int K, int num_sms, const Fit& fit) {
     Plan r;
@@ -394,19 +396,32 @@ inline Plan plan(int M, int N, int K, int num_sms, const Fit& fit) {
     // Too few CTAs that way (or more tiles than SMs): two to an SM.  Four stages and the partial sums have to fit in half of
     // its shared memory (80 tokens), and with fewer than one and a half CTAs per SM the imbalance costs what the spread
     // gains (16 tokens: 11008 x 4096 3 slices 10.3 us / 1 slice 12.2, 12288 x 4096 2 slices 12.1 / 12.4).
-    const bool half_fits = 4 * (W_BYTES + tn * BK) <= SMEM_TWO - TAIL_BYTES && tn * W_ROWS * 4 <= SMEM_TWO - TAIL_BYTES;
+    const bool half_fits = 4 * (W_BYTES + tn * BK) <= smem_of(2) - TAIL_BYTES && tn * W_ROWS * 4 <= smem_of(2) - TAIL_BYTES;
     if (half_fits && split > 0 && k_blocks >= 24)
         for (int s = 4; s > split; s--)
-            if (tiles <= 2 * fit.one[s] && 2 * tiles * s >= 3 * num_sms) { r.split = s; r.two = true; return r; }
+            if (tiles <= 2 * fit.one[s] && 2 * tiles * s >= 3 * num_sms) { r.split = s; r.per_sm = 2; return r; }
+    // Three to an SM, with four stages each (three past 16 tokens): 12288 x 4096 in 4 slices 11.1 us / 1 slice 12.4 at 16 tokens,
+    // 12.3 / 12.9 at 48.
+    if (M <= 48 && split > 0 && k_blocks >= 24 && tiles <= 3 * fit.one[4] && 2 * tiles >= num_sms) { r.split = 4; r.per_sm = 3; return r; }
+    // With more tiles than SMs the same in two slices, instead of two whole tiles on a few SMs and one on the others, or of the
+    // square kernel's short second wave (16 tokens: 22016 x 4096 19.0 us / 20.8 / 21.9, 26880 x 4096 20.4 / 21.7 / 23.1).  Past 16
+    // tokens it stays ahead up to a quarter more tiles than SMs (24000 x 4096, 32 tokens 21.4 / 21.2), and with only an eighth
+    // more up to 32 tokens (20000 x 4096, 48 tokens 20.0 / - / 19.7).
+    if (M <= 48 && split == 0 && k_blocks >= 16 && tiles <= 3 * fit.one[2] && (M <= 16 || 4 * tiles <= 5 * num_sms) &&
+        (M <= 32 || 8 * tiles >= 9 * num_sms)) {
+        r.split = 2;
+        r.per_sm = 3;
+        return r;
+    }
     if (split > 0) {
         // a third of the SMs idle: still ahead of the square kernel up to 48 tokens (12288 x 4096, 40 / 64 / 96 tokens: 12.8 / 13.4 /
         // 13.8 us against 13.2 / 13.2 / 13.4), or where that one reads the weight twice
         if (M <= 48 || M > 128 || 4 * tiles < num_sms) r.split = split;
         return r;
     }
-    // More tiles than SMs: in one wave of two to an SM, unless only a few SMs would get a second one (16 tokens: 172 tiles
-    // of K = 4096 22.8 us against 25.4, 256 tiles 22.9 against 25.2; 157 tiles 20.0 against 19.7, 512 tiles 44.9 against 45.7)
-    if (half_fits && M <= 64 && tiles <= 2 * fit.one[1] && 8 * tiles >= 9 * num_sms) { r.split = 1; r.two = true; }
+    // Up to twice as many tiles as SMs otherwise: one wave of two to an SM (16 tokens of K = 4096: 256 tiles 22.9 us against 25.2
+    // for the square kernel, 512 tiles 44.9 against 45.7), with a long K up to 48 tokens (21376 x 8192, 64 tokens 37.4 / 36.5)
+    if (half_fits && M <= (k_blocks > 32 ? 48 : 64) && tiles <= 2 * fit.one[1] && 8 * tiles >= 9 * num_sms) { r.split = 1; r.per_sm = 2; }
     return r;
 }
 
@@ -421,7 +436,7 @@ inline int launch(GemmParams g, const Plan& plan, const void* A, const void* B, 
     const int tiles = (g.N + W_ROWS - 1) / W_ROWS;
     const int stage_bytes = W_BYTES + p.tn * BK, part_bytes = p.tn * W_ROWS * 4;
     const int slice = (g.k_blocks + plan.split - 1) / plan.split;
-    p.stages = ((plan.two ? SMEM_TWO : SMEM_ONE) - TAIL_BYTES) / stage_bytes;
+    p.stages = (smem_of(plan.per_sm) - TAIL_BYTES) / stage_bytes;
     if (p.stages > slice) p.stages = slice;
     if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
     int ring_bytes = p.stages * stage_bytes;

@@ -355,9 +355,10 @@ def test_skinny_shapes_in_full(cuda, built_libs, M):
 
 @pytest.mark.parametrize("M,N,K", [(1, 128, 16), (1, 1003, 144), (15, 4096, 512), (16, 5000, 1040), (17, 2048, 10256), (33, 11008, 3088),
                                    (64, 21440, 256), (65, 512, 4112), (80, 130, 2064), (96, 8192, 4096), (128, 8192, 4096), (129, 4099, 4096),
-                                   (173, 12288, 2048), (192, 8200, 2064), (193, 4096, 4096)])
+                                   (173, 12288, 2048), (192, 8200, 2064), (193, 4096, 4096), (16, 12288, 3088), (48, 12500, 3088), (49, 12288, 3088),
+                                   (16, 22016, 2064), (33, 22016, 2048), (17, 19072, 2048), (16, 28000, 2064), (48, 24000, 2048)])
 def test_few_rows_exact_on_integer_data(cuda, built_libs, M, N, K):
-    # every way the few-row kernel cuts a problem (1 to 7 slices of K, one or two CTAs to an SM, ragged M, N and K, the rows
+    # every way the few-row kernel cuts a problem (1 to 7 slices of K, one to three CTAs to an SM, ragged M, N and K, the rows
     # just past its range).  Codes of small integers: products and sums are exact in fp32 whatever their order, so the
     # accumulate mode has to match to the bit and the 16-bit output to its one rounding; stores stay inside the matrix.
     from goml_b200 import fp8_gemm as G
