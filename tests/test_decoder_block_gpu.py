@@ -305,7 +305,6 @@ def test_inputs_and_caches_that_take_the_copying_route(cuda, built_libs):
         out.append((y, cache.k[:, :, :S].clone(), cache.v[:, :, :S].clone(), cache.scales, cache.lens))
     for other in out[1:]:
         assert all(torch.equal(a, b) for a, b in zip(out[0][1:], other[1:]))
-        # the residual adds of the larger GEMM may meet in another order: fp32 last bits, seen through one e4m3 quantiser
         # sums of the larger GEMMs need not meet in one order: a last bit becomes an isolated neighbouring e4m3 code (2^-4 of a value
         # in fewer than one in forty of them: 2^-4 * sqrt(1/40) < 1e-2 in the norm)
         assert (out[0][0] - other[0]).norm() <= 1e-2 * out[0][0].norm()
