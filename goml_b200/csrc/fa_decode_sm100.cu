@@ -189,8 +189,8 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
     pdl_trigger();
 
     float scale_log2 = p.scale_log2;
-    if (p.sq) scale_log2 *= __ldg(p.sq);
-    if (p.sk) scale_log2 *= __ldg(p.sk);
+    if (p.sq) scale_log2 *= ld_f32(p.sq);
+    if (p.sk) scale_log2 *= ld_f32(p.sk);
 
     // a sequence with no visible key is on nobody's piece: O = 0, LSE = -inf
     auto empty_sequence = [&](int b) {
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
     uint32_t vr[C::TILES][4][C::VW];
     auto page_of = [&](int key) -> int { return (int)(__umulhi((uint32_t)key, p.page_mul) >> (p.page_shr - 1)); };
     auto entry = [&](const Segment& x, int c) -> int {   // table entry of chunk c
-        return PAGED && c < x.c_end ? __ldg(p.block_table + (size_t)x.b * p.max_pages + page_of(c * CHUNK)) : 0;
+        return PAGED && c < x.c_end ? ld_s32(p.block_table + (size_t)x.b * p.max_pages + page_of(c * CHUNK)) : 0;
     };
     // byte offset of chunk c (the same in K and V), or -1 where the table names no page of the pool: nothing is read
     // there, the keys count as zeros
@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
         // slots of a cut pair: its splits in order, or on the line the odd slot of the CTA that has its first piece and the
         // even slots of the CTAs after that
         const int slot = p.plan == SPLITS ? blockIdx.x : 2 * blockIdx.x + (seg.c_begin == 0 ? 1 : 0);
-        const float vds = p.sv ? p.v_descale * __ldg(p.sv) : p.v_descale;
+        const float vds = p.sv ? p.v_descale * ld_f32(p.sv) : p.v_descale;
         for (int idx = threadIdx.x; idx < p.group * (D / 4); idx += THREADS) {   // four columns per thread and step
             const int row = idx / (D / 4), col = idx % (D / 4) * 4;
             float M = -INFINITY;

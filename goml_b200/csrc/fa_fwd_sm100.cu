@@ -158,7 +158,7 @@ __device__ __forceinline__ void e4m3x16_to_f16(const uint4 c, uint4& lo, uint4& 
     hi = make_uint4(h[4], h[5], h[6], h[7]);
 }
 template <int HD>
-__global__ void __launch_bounds__(V_THREADS, 12) v_to_f16_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, int chunks,
+__global__ void __launch_bounds__(V_THREADS, 12) v_to_f16_kernel(const uint4* in, uint4* out, int chunks,
                                                                 int chunks_per_head, int sl, uint32_t* flags, uint32_t epoch) {
     pdl_wait();      // V may come from the kernel ahead, and the attention of an earlier call may still read `out`
     pdl_trigger();   // after the wait: the attention kernel reads Q and K without waiting for this kernel
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(V_THREADS, 12) v_to_f16_kernel(const uint4* __
 #pragma unroll
             for (int i = 0; i < BATCH; i++) {
                 const int at = (i0 + i) * V_THREADS + threadIdx.x;
-                if (at < pieces) v[i] = __ldg(in + base + at);
+                if (at < pieces) v[i] = ld128(in + base + at);
             }
 #pragma unroll
             for (int i = 0; i < BATCH; i++) {
@@ -412,8 +412,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         const int qi = q0 + r;                   // query index in the sequence
         const uint32_t lane_off = uint32_t(warp * 32) << 16;
         float scale_log2 = p.scale_log2;
-        if (p.sq) scale_log2 *= __ldg(p.sq);
-        if (p.sk) scale_log2 *= __ldg(p.sk);
+        if (p.sq) scale_log2 *= ld_f32(p.sq);
+        if (p.sk) scale_log2 *= ld_f32(p.sk);
         const bool neg = scale_log2 < 0.f;       // the row max is taken on sign-adjusted raw scores
         float ascale = fabsf(scale_log2);
         if (ascale == 0.f) ascale = 1e-30f;      // keeps -inf * scale = -inf for masked keys
@@ -534,7 +534,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         if (ok && __all_sync(0xffffffffu, mbar_wait(bar_pvdone + 8 * rs_prev, rph_prev, abort_flag, ST_TIMEOUT_SOFTMAX))) {
             tc_fence_after();
             const float l = (l0 + l1) + (l2 + l3);
-            const float vds = p.sv ? p.v_descale * __ldg(p.sv) : p.v_descale;
+            const float vds = p.sv ? p.v_descale * ld_f32(p.sv) : p.v_descale;
             const float inv = (l > 0.f) ? vds / l : 0.f;
             // O leaves through shared memory so that the global stores are coalesced: a thread owns one row (HD fp16 = ROWB
             // bytes), which written straight to global makes every store instruction of a warp touch 32 different lines.

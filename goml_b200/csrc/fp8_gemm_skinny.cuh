@@ -55,12 +55,6 @@ __device__ __forceinline__ void prefetch_l2_2d(const CUtensorMap* m, int x, int 
     asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];"
                  ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y) : "memory");
 }
-// a scalar that a kernel ahead on the stream may have written: a plain load behind the wait, never a read-only one
-__device__ __forceinline__ float ld_scalar(const float* p) {
-    float v;
-    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
-    return v;
-}
 // the cluster's partial results for weight rows [row, row + 4) and token j: loads, and their sum in rank order
 template <int SPLIT>
 __device__ __forceinline__ void gather(float4* v, uint32_t part, int j, int row) {
@@ -185,9 +179,9 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         const GemmParams& g = p.g;
         constexpr int STEP = SPLIT * THREADS;
         float alpha = g.alpha;
-        if (g.scale_a) alpha *= ld_scalar(g.scale_a);
-        if (g.scale_b) alpha *= ld_scalar(g.scale_b);
-        const float scale_d = (g.D8 && g.scale_d) ? ld_scalar(g.scale_d) : 1.0f;
+        if (g.scale_a) alpha *= ld_f32(g.scale_a);
+        if (g.scale_b) alpha *= ld_f32(g.scale_b);
+        const float scale_d = (g.D8 && g.scale_d) ? ld_f32(g.scale_d) : 1.0f;
         float tmax = 0.f;
         if (g.H) {
             // gate rows [64c, 64c + 32), up rows [64c + 32, 64c + 64) of the tile

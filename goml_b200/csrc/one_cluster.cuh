@@ -5,8 +5,7 @@
 // pass reads its input from L1 / L2.  One cluster draws about 0.9 TB/s, so larger tensors stay with the two kernels
 // (as overlapped launches, with a clearing kernel in the memset's place).
 //
-// The loads below are plain (coherent) ones: a kernel launched before its predecessor has drained must not use the
-// read-only path for what that predecessor writes.
+// Loads are the coherent ones of pdl.cuh.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -19,27 +18,6 @@ namespace sm100 {
 
 constexpr int OC_CTAS = 16;        // more than the portable 8: a cluster of 16 fits a group of SMs of the B200
 constexpr int OC_THREADS = 512;
-
-__device__ __forceinline__ uint4 ld128(const void* p) {
-    uint4 r;
-    asm volatile("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
-    return r;
-}
-__device__ __forceinline__ float4 ld128f(const void* p) {
-    float4 r;
-    asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(p) : "memory");
-    return r;
-}
-__device__ __forceinline__ float ld_f32(const float* p) {
-    float r;
-    asm volatile("ld.global.f32 %0, [%1];" : "=f"(r) : "l"(p) : "memory");
-    return r;
-}
-__device__ __forceinline__ int ld_s32(const int* p) {
-    int r;
-    asm volatile("ld.global.s32 %0, [%1];" : "=r"(r) : "l"(p) : "memory");
-    return r;
-}
 
 __device__ __forceinline__ int oc_rank() {
     uint32_t r;

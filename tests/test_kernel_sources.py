@@ -1,0 +1,44 @@
+"""Rules of the kernel sources that no output shows reliably: checked on the text of goml_b200/csrc."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "goml_b200", "csrc")
+
+
+def sources():
+    out = {}
+    for f in sorted(os.listdir(CSRC)):
+        if f.endswith((".cu", ".cuh")):
+            with open(os.path.join(CSRC, f)) as fh:
+                out[f] = re.sub(r"//[^\n]*|/\*.*?\*/", "", fh.read(), flags=re.S)
+    return out
+
+
+def functions(text):
+    """(name, signature + body) of every __global__ / __device__ function of a source."""
+    for m in re.finditer(r"__(?:global|device)__[^;{}=]*?(\w+)\s*\([^{};]*\)\s*(?:const\s*)?\{", text):
+        depth, at = 1, m.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[at], 0)
+            at += 1
+        name = re.sub(r"__launch_bounds__\s*\([^()]*(?:\([^()]*\))?[^()]*\)", "", m.group(0))
+        yield re.search(r"(\w+)\s*\(", name).group(1), text[m.start():at]
+
+
+def plain_launches(text):
+    return set(re.findall(r"(\w+)(?:<[^<>;]*>)?<<<", text))
+
+
+@pytest.mark.parametrize("name", [n for n, t in sources().items() if re.search(r"__global__|__device__", t)])
+def test_no_read_only_loads_in_overlapped_kernels(name):
+    # a kernel that may start before its predecessor on the stream has drained must not read through the read-only path: only
+    # kernels launched plainly (<<<>>>) may
+    text = sources()[name]
+    assert list(functions(text))
+    plain = plain_launches(text)
+    for fn, body in functions(text):
+        if re.search(r"__ldg\s*\(|__restrict__|ld\.global\.nc|ld\.global\.L1::no_allocate\.nc", body):
+            assert fn in plain, f"{name}: {fn} reads through the read-only path"
+    assert not plain & set(re.findall(r"launch_pdl\(\s*(\w+)", text))

@@ -1,0 +1,87 @@
+"""Kernels that start before their predecessor on the stream has drained: chains of dependent calls, queued without a
+synchronisation and over the same buffers, give what the same calls give one at a time."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+STEPS = 50
+
+
+def twice(step, out):
+    """step(i) -> None writes out[i]: once with a synchronisation behind every step, once queued behind a short pause so that
+    the whole chain runs back to back on the GPU."""
+    got = []
+    for queued in (False, True):
+        out.fill_(0)
+        torch.cuda.synchronize()
+        if queued:
+            torch.cuda._sleep(30_000_000)   # some 15 ms
+        for i in range(STEPS):
+            step(i)
+            if not queued:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        got.append(out.clone())
+    assert torch.equal(*got)
+    return got[0]
+
+
+@pytest.mark.parametrize("B,S,H,hd", [(1, 40, 2, 64), (2, 300, 8, 128), (1, 700, 6, 64)])
+def test_rope_quantise_then_attention(cuda, built_libs, fa_ctx, B, S, H, hd):
+    # V and the scales of every step are written by the kernel right ahead of the attention; one cluster and two kernels
+    from goml_b200 import block_glue as BG
+    g = torch.Generator(device="cuda").manual_seed(S)
+    qkv = [(torch.randn(B * S, 3, H, hd, generator=g, device="cuda") * (0.1 + i % 7)).bfloat16() for i in range(STEPS)]
+    cos, sin = (torch.empty(S, hd // 2, device="cuda") for _ in range(2))
+    BG.RopeTable(cos.data_ptr(), sin.data_ptr(), S, hd, 10000.0)
+    q, k, v = (torch.empty(B * H, S, hd, dtype=torch.uint8, device="cuda") for _ in range(3))
+    s6 = torch.empty(6, device="cuda")
+    out = torch.empty(STEPS, B * H, S, hd, dtype=torch.float16, device="cuda")
+    sp, stream = s6.data_ptr(), torch.cuda.current_stream().cuda_stream
+
+    def step(i):
+        BG.RopeQuantizeQKV(qkv[i].data_ptr(), cos.data_ptr(), sin.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), sp, sp + 12, B, S, H, hd, stream)
+        fa_ctx.ForwardEx(q.data_ptr(), k.data_ptr(), v.data_ptr(), out[i].data_ptr(), 0, B * H, S, hd, 1, 0, 1.0 / math.sqrt(hd), 1.0,
+                         sp, sp + 4, sp + 8, stream)
+
+    got = twice(step, out)
+    # the first query of a sequence sees one key: its output is that key's V, 2^-4 relative to a code and its fp16 rounding
+    want = torch.stack([x.view(B, S, 3, H, hd)[:, 0, 2].reshape(B * H, hd).float() for x in qkv])
+    assert ((got[:, :, 0].float() - want).abs() <= 0.07 * want.abs() + 2e-3 * want.abs().amax(dim=(1, 2), keepdim=True)).all()
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,hd,paged", [(2, 4, 4, 64, False), (3, 8, 2, 128, True), (30, 32, 32, 128, False), (24, 32, 8, 128, True)])
+def test_append_then_decode(cuda, built_libs, fa_ctx, B, Hq, Hkv, hd, paged):
+    # the q scale, the appended rows and the lengths of every step are written by the kernel right ahead of the decode attention
+    from goml_b200 import block_glue as BG
+    g = torch.Generator(device="cuda").manual_seed(B)
+    s_max, page = 256, 64
+    qkv = [(torch.randn(B, (Hq + 2 * Hkv) * hd, generator=g, device="cuda") * (0.1 + i % 7)).bfloat16() for i in range(STEPS)]
+    cos, sin = (torch.empty(s_max, hd // 2, device="cuda") for _ in range(2))
+    BG.RopeTable(cos.data_ptr(), sin.data_ptr(), s_max, hd, 10000.0)
+    per = s_max // page
+    table = torch.randperm(B * per, generator=g, device="cuda").to(torch.int32).view(B, per)
+    shape = (B * per, Hkv, page, hd) if paged else (B, Hkv, s_max, hd)
+    k, v = (torch.empty(shape, dtype=torch.uint8, device="cuda") for _ in range(2))
+    k0, v0 = (torch.randint(0, 0x60, shape, generator=g, dtype=torch.uint8, device="cuda") for _ in range(2))
+    lens0 = (torch.arange(B, device="cuda") * 17 % 150).to(torch.int32)
+    lens = torch.empty_like(lens0)
+    q = torch.empty(B, Hq, hd, dtype=torch.uint8, device="cuda")
+    qs, kvs = torch.empty(2, device="cuda"), torch.tensor([0.02, 0.03], device="cuda")
+    out = torch.empty(STEPS, B, Hq, hd, dtype=torch.float16, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    more = dict(block_table=table.data_ptr(), page_size=page, max_pages_per_seq=per, num_pages=B * per) if paged else {}
+
+    def step(i):
+        if i == 0:
+            k.copy_(k0), v.copy_(v0), lens.copy_(lens0)
+        BG.DecodeRopeAppend(qkv[i].data_ptr(), cos.data_ptr(), sin.data_ptr(), lens.data_ptr(), q.data_ptr(), qs.data_ptr(), qs.data_ptr() + 4,
+                            k.data_ptr(), v.data_ptr(), kvs.data_ptr(), kvs.data_ptr() + 4, B, Hq, Hkv, hd, 0 if paged else s_max, s_max,
+                            seq_lens_out=lens.data_ptr(), stream=stream, **more)
+        fa_ctx.Decode(q.data_ptr(), k.data_ptr(), v.data_ptr(), out[i].data_ptr(), 0, lens.data_ptr(), B, Hq, Hkv, hd, 0 if paged else s_max, 0,
+                      1.0 / math.sqrt(hd), 1.0, qs.data_ptr(), kvs.data_ptr(), kvs.data_ptr() + 4, stream, **more)
+
+    twice(step, out)
+    assert torch.isfinite(out).all() and lens.tolist() == [n + STEPS for n in lens0.tolist()]
