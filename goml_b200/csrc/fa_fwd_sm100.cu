@@ -216,6 +216,8 @@ __device__ __forceinline__ bool wait_v_chunk(const uint32_t* head_flags, int chu
         const int n = missing ? __ffs(missing) - 1 : 32;
         if (n > 0) {
             ready = c + n;
+            // the lane that issues the copy need not be the one that acquired the chunk's flag, and a vote orders no memory
+            __syncwarp();
             asm volatile("fence.proxy.async.global;" ::: "memory");
             return true;
         }

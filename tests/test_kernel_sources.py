@@ -42,3 +42,10 @@ def test_no_read_only_loads_in_overlapped_kernels(name):
         if re.search(r"__ldg\s*\(|__restrict__|ld\.global\.nc|ld\.global\.L1::no_allocate\.nc", body):
             assert fn in plain, f"{name}: {fn} reads through the read-only path"
     assert not plain & set(re.findall(r"launch_pdl\(\s*(\w+)", text))
+
+
+def test_the_lane_that_copies_v_is_ordered_behind_the_lane_that_saw_the_flag():
+    # the attention producer: every lane acquires a flag of its own and one elected lane issues the copies; between the vote and
+    # the proxy fence stands a warp barrier, which orders memory among the lanes (a vote does not)
+    body = dict(functions(sources()["fa_fwd_sm100.cu"]))["wait_v_chunk"]
+    assert re.search(r"ld\.acquire\.gpu.*__ballot_sync.*__syncwarp\(\);\s*asm volatile\(\"fence\.proxy\.async", body, flags=re.S)
