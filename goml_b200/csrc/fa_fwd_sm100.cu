@@ -203,9 +203,11 @@ __global__ void __launch_bounds__(V_THREADS, 12) v_to_f16_kernel(const uint4* in
 // Producer-side view of the pre-pass: how many leading chunks of this head (from chunk `c` on) are known to be ready.
 // The whole warp asks for 32 flags at a time, so a head of up to 4096 keys costs one load when it is complete.
 // Bounded like every wait of this file.
-__device__ __forceinline__ bool wait_v_chunk(const uint32_t* head_flags, int chunks_per_head, uint32_t epoch, int c, int& ready,
+// `ok` is each lane's outcome of the waits before; the lanes enter the polls together or not at all.
+__device__ __forceinline__ bool wait_v_chunk(bool ok, const uint32_t* head_flags, int chunks_per_head, uint32_t epoch, int c, int& ready,
                                              volatile uint32_t* abort_flag) {
-    if (c < ready) return true;
+    if (c < ready) return ok;
+    if (!__all_sync(0xffffffffu, ok)) return false;
     const int lane = threadIdx.x & 31;
     uint64_t t0 = 0;
     for (uint32_t polls = 1;; polls++) {
@@ -334,25 +336,25 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
             uint32_t ph = 1;  // "previous phase complete": the rings start empty
             for (int j = 0; j < nblk; j++) {
                 const int key0 = (blk0 + j) * BN;
-                if (!mbar_wait(bar_sfull + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD)) break;   // Q K^T three blocks back is done
-                if (leader) {
+                bool ok = mbar_wait(bar_sfull + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD);   // Q K^T three blocks back is done
+                if (leader && ok) {
                     mbar_arrive_expect_tx(bar_kfull + 8 * s, C::K_BYTES);
                     tma_load_3d(sbase + C::OFF_K + s * C::K_BYTES, &tmap_k, bar_kfull + 8 * s, 0, key0, head);
                 }
-                if (!mbar_wait(bar_pvdone + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD)) break;  // P V three blocks back is done
+                ok = ok && mbar_wait(bar_pvdone + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD);  // P V three blocks back is done
                 if (!head_flags) {
                     if (j == 0) pdl_wait();
-                } else if (!wait_v_chunk(head_flags, p.v_chunks, p.v_epoch, key0 / V_CHUNK, v_ready, abort_flag)) {
-                    break;
+                } else {
+                    ok = wait_v_chunk(ok, head_flags, p.v_chunks, p.v_epoch, key0 / V_CHUNK, v_ready, abort_flag);
                 }
-                if (leader) {
+                if (leader && ok) {
                     mbar_arrive_expect_tx(bar_vfull + 8 * s, C::V_BYTES);
 #pragma unroll
                     for (int h = 0; h < HD / 64; h++)  // one 64-column (128-byte) slab of d per copy
                         tma_load_3d(sbase + C::OFF_V + s * C::V_BYTES + h * C::V_HALF_BYTES, &tmap_v, bar_vfull + 8 * s,
                                     h * 64, key0, head);
                 }
-                __syncwarp();
+                if (!__all_sync(0xffffffffu, ok)) break;
                 if (++s == STAGES) { s = 0; ph ^= 1; }
             }
             pdl_wait();   // this kernel completes after the pre-pass
@@ -371,29 +373,27 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
             bool ok = true;
             auto issue_qk = [&](int j) {  // S[j & 1] = Q K(j)^T
                 ok = mbar_wait(bar_kfull + 8 * ks, kph, abort_flag, ST_TIMEOUT_MMA);
-                if (!ok) return;
                 tc_fence_after();
                 const uint64_t qd = qk_desc(sbase + C::OFF_Q);
                 const uint64_t kd = qk_desc(sbase + C::OFF_K + ks * C::K_BYTES);
-                if (leader) {
+                if (leader && ok) {
 #pragma unroll
                     for (int k = 0; k < HD / 32; k++)
                         mma_f8f6f4_ss(tmem_s + (j & 1) * BN, qd + 2 * k, kd + 2 * k, idesc_qk, k != 0);
                     mma_commit(bar_sfull + 8 * ks);
                 }
-                __syncwarp();
+                ok = __all_sync(0xffffffffu, ok);
                 if (++ks == STAGES) { ks = 0; kph ^= 1; }
             };
-            ok = mbar_wait(bar_q, 0, abort_flag, ST_TIMEOUT_MMA);
+            ok = mbar_wait_warp(bar_q, 0, abort_flag, ST_TIMEOUT_MMA);
             for (int j = 0; j < 2 && j < nblk && ok; j++) issue_qk(j);
             for (int j = 0; j < nblk && ok; j++) {
                 const int b = j & 1;
                 ok = mbar_wait(bar_vfull + 8 * vs, vph, abort_flag, ST_TIMEOUT_MMA) &&
                      mbar_wait(bar_pfull + 8 * b, (j >> 1) & 1, abort_flag, ST_TIMEOUT_MMA);
-                if (!ok) break;
                 tc_fence_after();
                 const uint32_t vaddr = sbase + C::OFF_V + vs * C::V_BYTES;
-                if (leader) {
+                if (leader && ok) {
 #pragma unroll
                     for (int k = 0; k < BN / 16; k++) {  // 16 keys per MMA: 8 TMEM columns of P, 16 rows of V
                         const uint64_t vd = mnmajor_desc_sw128(vaddr + k * 16 * 128, C::V_HALF_BYTES);
@@ -401,7 +401,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
                     }
                     mma_commit(bar_pvdone + 8 * vs);
                 }
-                __syncwarp();
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
                 if (++vs == STAGES) { vs = 0; vph ^= 1; }
                 // S[b] is rewritten by the Q K^T two blocks ahead; it is issued behind this P V on the
                 // same in-order tensor pipe, so P(j) has been read before S(j+2) lands on it
@@ -444,7 +445,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         for (int j = 0; j < nblk; j++) {
             const int key0 = (blk0 + j) * BN;
             const int b = j & 1;
-            if (!__all_sync(0xffffffffu, mbar_wait(bar_sfull + 8 * rs, rph, abort_flag, ST_TIMEOUT_SOFTMAX))) { ok = false; break; }
+            if (!mbar_wait_warp(bar_sfull + 8 * rs, rph, abort_flag, ST_TIMEOUT_SOFTMAX)) { ok = false; break; }
             tc_fence_after();
             uint32_t sreg[BN];
 #pragma unroll
@@ -490,7 +491,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
                 const float m_new = bump ? mx : m_ref;
                 if (j > 0) {
                     // O is final only once the previous P V has finished
-                    if (!__all_sync(0xffffffffu, mbar_wait(bar_pvdone + 8 * rs_prev, rph_prev, abort_flag, ST_TIMEOUT_SOFTMAX))) { ok = false; break; }
+                    if (!mbar_wait_warp(bar_pvdone + 8 * rs_prev, rph_prev, abort_flag, ST_TIMEOUT_SOFTMAX)) { ok = false; break; }
                     tc_fence_after();
                     const float f = bump ? ex2(m_ref - m_new) : 1.0f;  // m_ref = -inf -> 0
                     l0 *= f; l1 *= f; l2 *= f; l3 *= f;
@@ -533,7 +534,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         }
 
         // epilogue: O / l (times the V dequantisation scale) -> fp16
-        if (ok && __all_sync(0xffffffffu, mbar_wait(bar_pvdone + 8 * rs_prev, rph_prev, abort_flag, ST_TIMEOUT_SOFTMAX))) {
+        if (ok && mbar_wait_warp(bar_pvdone + 8 * rs_prev, rph_prev, abort_flag, ST_TIMEOUT_SOFTMAX)) {
             tc_fence_after();
             const float l = (l0 + l1) + (l2 + l3);
             const float vds = p.sv ? p.v_descale * ld_f32(p.sv) : p.v_descale;

@@ -86,6 +86,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
+// Every role of these kernels runs on whole warps, and a lane may run out of time, or see the abort word, where its neighbour
+// still sees the phase complete.  Leaving the role's loop without it, it would wait in the CTA's teardown barrier while the
+// others wait for it in the loop's next warp-wide operation.  So the lanes vote on the outcome before any of them leaves: here,
+// or, in the loops that feed the tensor core and the copy engine, at the end of the step, in the place of a __syncwarp() and
+// behind the elected lane's issue (a vote between the wait and the issue costs the GEMMs and the attention 0.3 to 1 %).
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t code) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, code));
+}
+
 // Self-test of the bounded wait, shared by the libraries: one warp waits, with a 1 ms budget, on a barrier that
 // nothing will ever arrive at.  The wait must give up, set the CTA's abort word to `code`, and the kernel then latches
 // the code into the library's device status word exactly as a production kernel's teardown does — and returns.

@@ -49,3 +49,21 @@ def test_the_lane_that_copies_v_is_ordered_behind_the_lane_that_saw_the_flag():
     # the proxy fence stands a warp barrier, which orders memory among the lanes (a vote does not)
     body = dict(functions(sources()["fa_fwd_sm100.cu"]))["wait_v_chunk"]
     assert re.search(r"ld\.acquire\.gpu.*__ballot_sync.*__syncwarp\(\);\s*asm volatile\(\"fence\.proxy\.async", body, flags=re.S)
+
+
+@pytest.mark.parametrize("name", [n for n, t in sources().items() if "mbar_wait" in t and n != "sm100_ptx.cuh"])
+def test_bounded_waits_are_left_by_whole_warps(name):
+    # roles run on whole warps: a lane that leaves a loop on its own outcome of a wait strands the others in the loop's next
+    # warp-wide operation.  So an outcome is either voted on inside the wait or kept in `ok`, and `ok` is voted on before
+    # any lane breaks or returns
+    text = sources()[name]
+    waits = [m.start() for m in re.finditer(r"\bmbar_wait\s*\(", text)]
+    assert len(waits) == sum(o.count("mbar_wait(") for o in re.findall(r"\bok = [^;]*;", text))
+    for at in waits:
+        leaves = re.search(r"\b(break|return|goto|continue)\b", text[at:])
+        assert "__all_sync(" in text[at:at + leaves.start()], text[at:at + leaves.start()]
+
+
+def test_the_warp_wait_votes():
+    body = dict(functions(sources()["sm100_ptx.cuh"]))["mbar_wait_warp"]
+    assert re.search(r"__all_sync\(0xffffffffu,\s*mbar_wait\(", body)
