@@ -121,7 +121,7 @@ fa_status_t validate(fa_ctx_t* c, const char* who, const void* q, const void* k,
 // One call's scratch: the stream's kept buffers where they serve, else blocks drawn from the pool for this call.
 struct Scratch {
     void* ptr = nullptr;
-    uint32_t* flags = nullptr;   // nullptr: none kept for this stream (a capture, more streams than slots)
+    uint32_t* flags = nullptr;   // nullptr: none kept for this stream (a capture, more streams than slots) and none needed
     uint32_t epoch = 0;
     uint32_t* zeros = nullptr;
     void* pooled[2] = {nullptr, nullptr};
@@ -145,7 +145,8 @@ struct Scratch {
         return cudaSuccess;
     }
 
-    cudaError_t take(fa_ctx_t* c, cudaStream_t s, size_t bytes, size_t flag_words, size_t zero_words) {
+    // need_flags: the call cannot do without flags (else they are given where the stream's kept ones serve)
+    cudaError_t take(fa_ctx_t* c, cudaStream_t s, size_t bytes, size_t flag_words, bool need_flags, size_t zero_words) {
         stream = s;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         cudaError_t e = cudaStreamIsCapturing(s, &cap);
@@ -185,10 +186,16 @@ struct Scratch {
             if ((e = cudaMallocFromPoolAsync(&pooled[0], bytes, c->shared->pool, s)) != cudaSuccess) return e;
             ptr = pooled[0];
         }
-        if (zero_words && !zeros) {
-            if ((e = cudaMallocFromPoolAsync(&pooled[1], zero_words * 4, c->shared->pool, s)) != cudaSuccess) { give_back(); return e; }
-            if ((e = cudaMemsetAsync(pooled[1], 0, zero_words * 4, s)) != cudaSuccess) { give_back(); return e; }
-            zeros = static_cast<uint32_t*>(pooled[1]);
+        const size_t more_zeros = zeros ? 0 : zero_words, more_flags = flags || !need_flags ? 0 : flag_words;
+        if (more_zeros + more_flags) {
+            const size_t n = (more_zeros + more_flags) * 4;
+            if ((e = cudaMallocFromPoolAsync(&pooled[1], n, c->shared->pool, s)) != cudaSuccess) { give_back(); return e; }
+            if ((e = cudaMemsetAsync(pooled[1], 0, n, s)) != cudaSuccess) { give_back(); return e; }
+            if (more_zeros) zeros = static_cast<uint32_t*>(pooled[1]);
+            if (more_flags) {
+                flags = static_cast<uint32_t*>(pooled[1]) + more_zeros;
+                epoch = 1;
+            }
         }
         return cudaSuccess;
     }
@@ -215,7 +222,7 @@ fa_status_t run(fa_ctx_t* c, const char* who, const fa_sm100::LaunchArgs& a) {
     }
     fa_sm100::LaunchArgs b = a;
     Scratch ws;
-    e = ws.take(c, a.stream, fa_sm100::workspace_bytes(a.bh, a.sl, a.hd), fa_sm100::v_flag_count(a.bh, a.sl), 0);
+    e = ws.take(c, a.stream, fa_sm100::workspace_bytes(a.bh, a.sl, a.hd), fa_sm100::v_flag_count(a.bh, a.sl), false, 0);
     if (e != cudaSuccess) {
         set_err(c, "%s: workspace allocation: %s", who, cudaGetErrorString(e));
         return e == cudaErrorMemoryAllocation ? FA_ERR_OOM : FA_ERR_CUDA;
@@ -373,7 +380,7 @@ fa_status_t fa_decode(fa_ctx_t* ctx, const fa_decode_args_t* g) {
     Scratch ws;
     const int span = fa_sm100::decode_span(a);
     e = ws.take(ctx, a.stream, fa_sm100::decode_workspace_bytes(a.batch, a.q_heads, a.kv_heads, a.hd, span),
-                fa_sm100::decode_flag_count(a.batch, a.q_heads, a.kv_heads, span), (size_t)a.batch * a.kv_heads);
+                fa_sm100::decode_flag_count(a.batch, a.q_heads, a.kv_heads, span), true, (size_t)a.batch * a.kv_heads);
     if (e != cudaSuccess) { set_err(ctx, "%s: workspace allocation: %s", who, cudaGetErrorString(e)); return e == cudaErrorMemoryAllocation ? FA_ERR_OOM : FA_ERR_CUDA; }
     a.workspace = ws.ptr;
     a.arrivals = ws.zeros;

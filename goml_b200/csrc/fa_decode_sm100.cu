@@ -22,8 +22,9 @@
 //    next block's scores (Little's law asks for about 45 KB in flight per SM).
 //
 // How the keys are divided (Plan below): a pair (sequence, kv head) may be cut between chunks; the pieces leave partial
-// states in a workspace and the CTA that finishes last merges them in a fixed order, so results do not depend on timing
-// and there is no second kernel.
+// states in a workspace and the CTA that finishes last merges them in a fixed order, so there is no second kernel and results
+// do not depend on timing: the same call gives the same bits, eager or in a graph, on whatever stream.  (One exception is
+// reported: a hand-over of maxima that does not come within the wait's budget, see LINE_HANDED.)
 //
 // STREAMS: the rounding of P to fp16 depends on the running maximum it is taken against, so which keys share a warp and
 // where a pair is cut show in the last bits of O.  A block that re-quantises its activations turns last bits into e4m3
@@ -38,6 +39,7 @@
 
 #include "fa_fwd_sm100.h"
 #include "pdl.cuh"
+#include "sm100_ptx.cuh"
 
 namespace fa_sm100 {
 
@@ -99,9 +101,12 @@ __device__ __forceinline__ void ldg64(uint32_t* r, const uint8_t* p) {
 //          different lengths load all SMs alike.
 //  LINE_HANDED: the same with pieces at least as long as the longest pair, so that a pair is cut at most once.  A CTA
 //          takes the pair that its piece ends in first, publishes the running maxima it ended with, and takes the pair its
-//          piece begins in last, starting from the maxima of the CTA before it.  Those were published about a piece ago;
-//          the wait for them is bounded and gives up to a start from scratch, which changes only roundings.
+//          piece begins in last, starting from the maxima of the CTA before it.  Those were published about a piece ago by a
+//          CTA that started earlier and waits for nobody before it publishes.  The wait for them is bounded all the same: when
+//          its budget runs out the status word is set and the pair starts from scratch, which changes only roundings.
 enum Plan : int { SPLITS, LINE, LINE_HANDED };
+constexpr uint32_t ST_TIMEOUT_HANDED = 0x204;   // beside the codes of the forward kernel
+__device__ uint32_t g_decode_status = 0;
 
 struct DecodeParams {
     const uint8_t* q;
@@ -126,7 +131,7 @@ struct DecodeParams {
     float* ws_ml;
     float* ws_handed;     // [CTA][WARPS][rows] running maxima
     uint32_t* arrivals;   // [B*Hkv], zero before and after every launch
-    uint32_t* handed;     // [CTA], set to epoch when the CTA's maxima are published; nullptr: nothing is handed on
+    uint32_t* handed;     // [CTA], set to epoch when the CTA's maxima are published
     uint32_t epoch;
 };
 
@@ -428,11 +433,21 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
 #pragma unroll
             for (int i = 0; i < C::MT; i++) acc[n][i][0] = acc[n][i][1] = acc[n][i][2] = acc[n][i][3] = 0.f;
         }
-        if (STREAMS && p.plan == LINE_HANDED && seg.c_begin > 0 && p.handed) {
-            uint32_t f = ~p.epoch;
-            for (int polls = 0; polls < 20000 && f != p.epoch; polls++)
+        if (STREAMS && p.plan == LINE_HANDED && seg.c_begin > 0) {
+            uint32_t f;
+            uint64_t t0 = 0;
+            for (uint32_t polls = 1;; polls++) {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(f) : "l"(p.handed + blockIdx.x - 1) : "memory");
-            if (__all_sync(0xffffffffu, f == p.epoch)) {
+                if (f == p.epoch) break;
+                if ((polls & 255u) == 0) {
+                    const uint64_t now = globaltimer_ns();
+                    if (t0 == 0) t0 = now;
+                    else if (now - t0 > SM100_WAIT_BUDGET_NS) break;
+                }
+            }
+            if (!__all_sync(0xffffffffu, f == p.epoch)) {
+                if (lane == 0) atomicCAS(&g_decode_status, 0u, ST_TIMEOUT_HANDED);
+            } else {
 #pragma unroll
                 for (int n = 0; n < NQ; n++)
 #pragma unroll
@@ -563,7 +578,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
 
         // ---- merge the four warps' states
         const bool whole = seg.c_begin == 0 && seg.c_end == seg.n_chunks;
-        const bool hand_on = STREAMS && p.plan == LINE_HANDED && p.handed && seg.c_end < seg.n_chunks;
+        const bool hand_on = STREAMS && p.plan == LINE_HANDED && seg.c_end < seg.n_chunks;
 #pragma unroll
         for (int n = 0; n < NQ; n++)
 #pragma unroll
@@ -727,6 +742,7 @@ cudaError_t launch_decode(const DecodeArgs& a) {
     if ((long long)a.batch * a.kv_heads * ((span + CHUNK - 1) / CHUNK) > 0x7fffffffLL) return cudaErrorInvalidValue;
     if (!a.workspace || !a.arrivals) return cudaErrorInvalidValue;
     const Layout x = layout_of(a.batch, a.q_heads, a.kv_heads, span);
+    if (x.plan == LINE_HANDED && !a.flags) return cudaErrorInvalidValue;
     DecodeParams p;
     p.q = static_cast<const uint8_t*>(a.q);
     p.k = static_cast<const uint8_t*>(a.k_cache);
@@ -764,6 +780,13 @@ cudaError_t launch_decode(const DecodeArgs& a) {
     return a.hd == 128 ? KERNELS(128) : KERNELS(64);
 #undef KERNELS
 #undef KERNEL
+}
+
+cudaError_t take_decode_status(uint32_t* code) {
+    const uint32_t zero = 0;
+    cudaError_t e = cudaMemcpyFromSymbol(code, g_decode_status, sizeof(*code));
+    if (e == cudaSuccess && *code != 0) e = cudaMemcpyToSymbol(g_decode_status, &zero, sizeof(zero));
+    return e;
 }
 
 }  // namespace fa_sm100

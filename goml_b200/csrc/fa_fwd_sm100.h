@@ -50,7 +50,7 @@ struct DecodeArgs {
     const float* scale_v_dev = nullptr;
     void* workspace = nullptr;      // decode_workspace_bytes(...) bytes, 16-byte aligned
     uint32_t* arrivals = nullptr;   // [batch * kv_heads] words that are zero; the launch leaves them zero
-    uint32_t* flags = nullptr;      // decode_flag_count(...) words none of which is `epoch`, or nullptr
+    uint32_t* flags = nullptr;      // decode_flag_count(...) words none of which is `epoch`
     uint32_t epoch = 0;
     cudaStream_t stream;
     // paged cache (block_table != nullptr): k_cache, v_cache are [num_pages, kv_heads, page_size, hd], page_size a
@@ -64,6 +64,8 @@ inline int decode_span(const DecodeArgs& a) { return a.seq_lens ? a.s_max : a.se
 size_t decode_workspace_bytes(int batch, int q_heads, int kv_heads, int head_dim, int span);
 size_t decode_flag_count(int batch, int q_heads, int kv_heads, int span);
 cudaError_t launch_decode(const DecodeArgs& a);
+// Status word of the decode kernels (0, or the code of a wait that ran out), which the read clears; synchronous.
+cudaError_t take_decode_status(uint32_t* code);
 
 // One warp that lets a 1 ms bounded wait run out on a barrier nothing arrives at and latches code 0x2F0.
 cudaError_t launch_wait_expiry_selftest(cudaStream_t stream);

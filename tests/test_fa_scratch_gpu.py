@@ -1,0 +1,107 @@
+"""The attention library's scratch: the same call gives the same bits whatever stream, thread, graph or context it comes from."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def codes(g, *shape):
+    x = torch.randn(*shape, generator=g, device="cuda").mul_(80.0).clamp_(-448, 448)
+    return x.to(torch.float8_e4m3fn).view(torch.uint8)
+
+
+class Decode:
+    """One decode call on buffers of its own; new(seed) puts other inputs and lengths into them."""
+
+    def __init__(self, B, Hq, Hkv, s_max, hd, seed=1):
+        self.dims = (B, Hq, Hkv, hd, s_max)
+        self.k, self.v = (torch.empty(B, Hkv, s_max, hd, dtype=torch.uint8, device="cuda") for _ in range(2))
+        self.q = torch.empty(B, Hq, hd, dtype=torch.uint8, device="cuda")
+        self.lens = torch.empty(B, dtype=torch.int32, device="cuda")
+        self.sc = torch.full((3,), 1 / 80.0, device="cuda")
+        self.o = torch.empty(B, Hq, hd, dtype=torch.float16, device="cuda")
+        self.new(seed)
+
+    def new(self, seed):
+        B, _, _, _, s_max = self.dims
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        for t in (self.k, self.v, self.q):
+            t.copy_(codes(g, *t.shape))
+        self.lens.copy_(torch.randint(s_max // 3, s_max + 1, (B,), generator=g, device="cuda"))
+        torch.cuda.synchronize()
+
+    def __call__(self, ctx, stream=None):
+        B, Hq, Hkv, hd, s_max = self.dims
+        stream = torch.cuda.current_stream() if stream is None else stream
+        s = self.sc.data_ptr()
+        ctx.Decode(self.q.data_ptr(), self.k.data_ptr(), self.v.data_ptr(), self.o.data_ptr(), 0, self.lens.data_ptr(), B, Hq, Hkv, hd, s_max, 0,
+                   1.0 / math.sqrt(hd), 1.0, s, s + 4, s + 8, stream.cuda_stream)
+
+    def result(self, ctx, stream=None):
+        self.o.fill_(float("nan"))
+        torch.cuda.synchronize()
+        self(ctx, stream)
+        torch.cuda.synchronize()
+        ctx.DeviceStatus()
+        assert torch.isfinite(self.o).all()
+        return self.o.clone()
+
+
+class Forward:
+    def __init__(self, bh, s, hd, causal=1, seed=1):
+        self.dims = (bh, s, hd, causal)
+        self.q, self.k, self.v = (torch.empty(bh, s, hd, dtype=torch.uint8, device="cuda") for _ in range(3))
+        self.sc = torch.full((3,), 1 / 80.0, device="cuda")
+        self.o = torch.empty(bh, s, hd, dtype=torch.float16, device="cuda")
+        self.new(seed)
+
+    def new(self, seed):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        for t in (self.q, self.k, self.v):
+            t.copy_(codes(g, *t.shape))
+        torch.cuda.synchronize()
+
+    def __call__(self, ctx, stream=None):
+        bh, s, hd, causal = self.dims
+        stream = torch.cuda.current_stream() if stream is None else stream
+        p = self.sc.data_ptr()
+        ctx.ForwardEx(self.q.data_ptr(), self.k.data_ptr(), self.v.data_ptr(), self.o.data_ptr(), 0, bh, s, hd, causal, 0, 1.0 / math.sqrt(hd), 1.0,
+                      p, p + 4, p + 8, stream.cuda_stream)
+
+    result = Decode.result
+
+
+# every plan of the decode kernel: fixed splits (cut and uncut pairs), the line with hand-over, the freely cut line
+CALLS = {"splits": lambda: Decode(1, 8, 8, 1000, 128), "one split": lambda: Decode(12, 32, 32, 300, 64), "handed": lambda: Decode(25, 32, 32, 500, 128),
+         "handed, hd 64": lambda: Decode(23, 30, 30, 900, 64), "line": lambda: Decode(5, 32, 8, 700, 128), "wide line": lambda: Decode(3, 24, 2, 900, 64),
+         "forward": lambda: Forward(8, 700, 128), "forward, hd 64": lambda: Forward(3, 300, 64, 0)}
+
+
+@pytest.mark.parametrize("name", CALLS)
+def test_a_graph_gives_the_bits_of_the_eager_call(cuda, built_libs, fa_ctx, name):
+    call = CALLS[name]()
+    call.result(fa_ctx)
+    side = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        call(fa_ctx)
+        call(fa_ctx)
+    for seed in (2, 3, 2):   # replayed with other inputs and lengths in the same buffers
+        call.new(seed)
+        want = call.result(fa_ctx)
+        for _ in range(2):
+            call.o.fill_(float("nan"))
+            graph.replay()
+            torch.cuda.synchronize()
+            fa_ctx.DeviceStatus()
+            assert torch.equal(call.o, want)
+
+
+@pytest.mark.parametrize("name", CALLS)
+def test_twenty_streams_give_the_same_bits(cuda, built_libs, fa_ctx, name):
+    call = CALLS[name]()
+    want = call.result(fa_ctx)
+    for stream in [torch.cuda.Stream() for _ in range(20)]:
+        assert torch.equal(call.result(fa_ctx, stream), want)
