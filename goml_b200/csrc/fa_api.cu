@@ -190,7 +190,7 @@ struct Scratch {
         if (more_zeros + more_flags) {
             const size_t n = (more_zeros + more_flags) * 4;
             if ((e = cudaMallocFromPoolAsync(&pooled[1], n, c->shared->pool, s)) != cudaSuccess) { give_back(); return e; }
-            if ((e = cudaMemsetAsync(pooled[1], 0, n, s)) != cudaSuccess) { give_back(); return e; }
+            if ((e = fa_sm100::launch_clear_words(static_cast<uint32_t*>(pooled[1]), more_zeros + more_flags, s)) != cudaSuccess) { give_back(); return e; }
             if (more_zeros) zeros = static_cast<uint32_t*>(pooled[1]);
             if (more_flags) {
                 flags = static_cast<uint32_t*>(pooled[1]) + more_zeros;
@@ -380,7 +380,8 @@ fa_status_t fa_decode(fa_ctx_t* ctx, const fa_decode_args_t* g) {
     Scratch ws;
     const int span = fa_sm100::decode_span(a);
     e = ws.take(ctx, a.stream, fa_sm100::decode_workspace_bytes(a.batch, a.q_heads, a.kv_heads, a.hd, span),
-                fa_sm100::decode_flag_count(a.batch, a.q_heads, a.kv_heads, span), true, (size_t)a.batch * a.kv_heads);
+                fa_sm100::decode_flag_count(a.batch, a.q_heads, a.kv_heads, span), true,
+                fa_sm100::decode_arrival_count(a.batch, a.q_heads, a.kv_heads, span));
     if (e != cudaSuccess) { set_err(ctx, "%s: workspace allocation: %s", who, cudaGetErrorString(e)); return e == cudaErrorMemoryAllocation ? FA_ERR_OOM : FA_ERR_CUDA; }
     a.workspace = ws.ptr;
     a.arrivals = ws.zeros;

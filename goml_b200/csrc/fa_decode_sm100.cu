@@ -697,8 +697,17 @@ int num_sms_of_current_device() {
     return sms;
 }
 
+// A kernel and not a memset node: in a graph the decode kernel is then launched behind it before it has drained (one sequence of
+// 32 heads and 100 keys: 8.8 us a captured call with the node).
+__global__ void clear_words_kernel(uint32_t* w, uint32_t n) {
+    pdl_wait();
+    pdl_trigger();
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) w[i] = 0;
+}
+
 struct Layout {
     int plan, splits, grid, rows;
+    bool cuts() const { return plan != SPLITS || splits > 1; }   // whether a pair may be cut
 };
 // One query head per kv head keeps the streams: fixed splits while the pairs leave room for them, else the line with
 // hand-over.  Groups take the freely cut line, which balances best (24 sequences of 3000 to 6000 keys, 8 kv heads: 45 us
@@ -730,7 +739,11 @@ Layout layout_of(int batch, int q_heads, int kv_heads, int span) {
 
 size_t decode_workspace_bytes(int batch, int q_heads, int kv_heads, int head_dim, int span) {
     const Layout x = layout_of(batch, q_heads, kv_heads, span);
+    if (!x.cuts()) return 0;
     return (size_t)x.grid * x.rows * (2 * (head_dim + 2) + WARPS) * sizeof(float);
+}
+size_t decode_arrival_count(int batch, int q_heads, int kv_heads, int span) {
+    return layout_of(batch, q_heads, kv_heads, span).cuts() ? (size_t)batch * kv_heads : 0;
 }
 size_t decode_flag_count(int batch, int q_heads, int kv_heads, int span) {
     const Layout x = layout_of(batch, q_heads, kv_heads, span);
@@ -740,8 +753,8 @@ size_t decode_flag_count(int batch, int q_heads, int kv_heads, int span) {
 cudaError_t launch_decode(const DecodeArgs& a) {
     const int span = decode_span(a);
     if ((long long)a.batch * a.kv_heads * ((span + CHUNK - 1) / CHUNK) > 0x7fffffffLL) return cudaErrorInvalidValue;
-    if (!a.workspace || !a.arrivals) return cudaErrorInvalidValue;
     const Layout x = layout_of(a.batch, a.q_heads, a.kv_heads, span);
+    if (x.cuts() && (!a.workspace || !a.arrivals)) return cudaErrorInvalidValue;
     if (x.plan == LINE_HANDED && !a.flags) return cudaErrorInvalidValue;
     DecodeParams p;
     p.q = static_cast<const uint8_t*>(a.q);
@@ -780,6 +793,12 @@ cudaError_t launch_decode(const DecodeArgs& a) {
     return a.hd == 128 ? KERNELS(128) : KERNELS(64);
 #undef KERNELS
 #undef KERNEL
+}
+
+cudaError_t launch_clear_words(uint32_t* w, size_t n, cudaStream_t stream) {
+    if (n > 0xffffffffu) return cudaErrorInvalidValue;
+    const unsigned blocks = (unsigned)((n + 1023) / 1024 < 64 ? (n + 1023) / 1024 : 64);
+    return launch_pdl(clear_words_kernel, dim3(blocks), dim3(256), 0, stream, w, (uint32_t)n);
 }
 
 cudaError_t take_decode_status(uint32_t* code) {

@@ -105,3 +105,34 @@ def test_twenty_streams_give_the_same_bits(cuda, built_libs, fa_ctx, name):
     want = call.result(fa_ctx)
     for stream in [torch.cuda.Stream() for _ in range(20)]:
         assert torch.equal(call.result(fa_ctx, stream), want)
+
+
+def node_types(graph):
+    import ctypes as C
+    cu = C.CDLL("libcuda.so.1")
+    n = C.c_size_t()
+    raw = C.c_void_p(graph.raw_cuda_graph())
+    assert cu.cuGraphGetNodes(raw, None, C.byref(n)) == 0
+    nodes = (C.c_void_p * n.value)()
+    assert cu.cuGraphGetNodes(raw, nodes, C.byref(n)) == 0
+    out = []
+    for node in nodes:
+        t = C.c_int()
+        assert cu.cuGraphNodeGetType(C.c_void_p(node), C.byref(t)) == 0
+        out.append(t.value)
+    return out
+
+
+@pytest.mark.parametrize("name,kernels,others", [("one split", 1, 0), ("splits", 2, 4), ("handed", 2, 4), ("line", 2, 4)])
+def test_nodes_of_a_captured_decode(cuda, built_libs, fa_ctx, name, kernels, others):
+    # no memset node, which would part the decode kernel from the kernel ahead; nothing but the kernel where no pair is cut, and
+    # else two allocations, their two frees and the kernel that clears the words
+    call = CALLS[name]()
+    call.result(fa_ctx)
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+        call(fa_ctx)
+    types = node_types(graph)
+    kernel, memset, alloc, free = 0, 2, 10, 11
+    assert types.count(kernel) == kernels and types.count(memset) == 0
+    assert sorted(t for t in types if t != kernel) == sorted([alloc, free] * (others // 2))
