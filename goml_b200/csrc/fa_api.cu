@@ -28,13 +28,23 @@ struct Kept {
     uint32_t* zeros = nullptr;     // words that every call finds zero and leaves zero
     size_t zero_words = 0;
     bool used = false;
+    std::mutex busy;               // held from the look-up until the kernels that use the buffers are on the stream: calls on one
+                                   // stream take turns, calls on others do not wait for them
+    void drop() {
+        if (scratch) cudaFree(scratch);
+        if (flags) cudaFree(flags);
+        if (zeros) cudaFree(zeros);
+        scratch = nullptr; flags = zeros = nullptr;
+        scratch_bytes = flag_words = zero_words = 0;
+        used = false;
+    }
 };
 constexpr int MAX_DEVICES = 64;
 constexpr int KEPT_STREAMS = 8;
 constexpr size_t KEPT_SCRATCH_MAX = (size_t)64 << 20;
 constexpr size_t KEPT_WORDS_MAX = (size_t)1 << 20;
 struct DeviceScratch {
-    std::mutex lock;               // held from looking a buffer up until the kernels that use it are on the stream
+    std::mutex lock;               // of the members here and of which slot belongs to which stream; never held over a launch
     int contexts = 0;
     cudaMemPool_t pool = nullptr;
     Kept kept[KEPT_STREAMS];
@@ -65,16 +75,25 @@ struct DeviceScratch {
             cudaGetDevice(&cur);
             if (cur != dev) cudaSetDevice(dev);
             cudaDeviceSynchronize();
-            for (Kept& k : kept) {
-                if (k.scratch) cudaFree(k.scratch);
-                if (k.flags) cudaFree(k.flags);
-                if (k.zeros) cudaFree(k.zeros);
-                k = Kept();
-            }
+            for (Kept& k : kept) k.drop();
             if (cur >= 0 && cur != dev) cudaSetDevice(cur);
         }
         cudaMemPoolDestroy(pool);  // pending frees complete first (stream-ordered)
         pool = nullptr;
+    }
+    // the slot of a stream, or nullptr when all belong to others
+    Kept* slot_of(unsigned long long stream_id) {
+        std::lock_guard<std::mutex> g(lock);
+        Kept* vacant = nullptr;
+        for (Kept& k : kept) {
+            if (k.used && k.stream_id == stream_id) return &k;
+            if (!k.used && !vacant) vacant = &k;
+        }
+        if (vacant) {
+            vacant->used = true;
+            vacant->stream_id = stream_id;
+        }
+        return vacant;
     }
 };
 DeviceScratch g_scratch[MAX_DEVICES];
@@ -153,14 +172,9 @@ struct Scratch {
         if (e != cudaSuccess) return e;
         unsigned long long id = 0;
         if (cap == cudaStreamCaptureStatusNone && cudaStreamGetId(s, &id) == cudaSuccess) {
-            lock = std::unique_lock<std::mutex>(c->shared->lock);
-            Kept* k = nullptr;
-            for (auto& x : c->shared->kept)
-                if (x.used && x.stream_id == id) { k = &x; break; }
-            if (!k)
-                for (auto& x : c->shared->kept)
-                    if (!x.used) { k = &x; k->used = true; k->stream_id = id; break; }
+            Kept* k = c->shared->slot_of(id);
             if (k) {
+                lock = std::unique_lock<std::mutex>(k->busy);
                 if (flag_words && flag_words <= KEPT_WORDS_MAX) {
                     const uint32_t* before = k->flags;
                     if ((e = grow(c->shared->pool, k->flags, k->flag_words, flag_words, 4096, true, s)) != cudaSuccess) return e;

@@ -136,3 +136,59 @@ def test_nodes_of_a_captured_decode(cuda, built_libs, fa_ctx, name, kernels, oth
     kernel, memset, alloc, free = 0, 2, 10, 11
     assert types.count(kernel) == kernels and types.count(memset) == 0
     assert sorted(t for t in types if t != kernel) == sorted([alloc, free] * (others // 2))
+
+
+def test_buffers_that_grow_and_serve_both_entry_points(cuda, built_libs, fa_ctx):
+    # large, small, large again and other plans in between, on one stream, queued without a synchronisation
+    calls = [Forward(16, 3000, 128), Forward(1, 40, 64, 0), Decode(1, 8, 8, 1000, 128), Decode(25, 32, 32, 500, 128), Forward(64, 2048, 128),
+             Decode(40, 32, 8, 900, 128), Forward(2, 129, 64), Decode(1, 16, 1, 9000, 64)]
+    want = [c.result(fa_ctx) for c in calls]
+    stream = torch.cuda.Stream()
+    for order in (range(len(calls)), reversed(range(len(calls)))):
+        for c in calls:
+            c.o.fill_(float("nan"))
+        torch.cuda.synchronize()
+        for i in order:
+            calls[i](fa_ctx, stream)
+        torch.cuda.synchronize()
+        fa_ctx.DeviceStatus()
+        assert all(torch.equal(c.o, w) for c, w in zip(calls, want))
+
+
+@pytest.mark.parametrize("streams,contexts", [(4, 4), (1, 4), (1, 1), (4, 1)])
+def test_threads(cuda, built_libs, fa_ctx, streams, contexts):
+    # four host threads, each with calls of its own: streams and contexts of their own or shared
+    import threading
+    from goml_b200 import fa_forward as F
+    make = [lambda: Decode(1, 8, 8, 1000, 128), lambda: Forward(8, 700, 128), lambda: Decode(25, 32, 32, 200, 128), lambda: Decode(5, 32, 8, 700, 128)]
+    calls = [[make[(t + i) % 4]() for i in range(3)] for t in range(4)]
+    want = [[c.result(fa_ctx) for c in cs] for cs in calls]
+    ss = [torch.cuda.Stream() for _ in range(streams)]
+    ctxs = [F.FACreate() for _ in range(contexts)]
+    for cs in calls:
+        for c in cs:
+            c.o.fill_(float("nan"))
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(t):
+        try:
+            torch.cuda.set_device(0)
+            for _ in range(100):
+                for c in calls[t]:
+                    c(ctxs[t % contexts], ss[t % streams])
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    torch.cuda.synchronize()
+    assert not errors, errors
+    fa_ctx.DeviceStatus()
+    for cs, ws in zip(calls, want):
+        assert all(torch.equal(c.o, w) for c, w in zip(cs, ws))
+    for c in ctxs:
+        c.Destroy()

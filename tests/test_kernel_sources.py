@@ -67,3 +67,10 @@ def test_bounded_waits_are_left_by_whole_warps(name):
 def test_the_warp_wait_votes():
     body = dict(functions(sources()["sm100_ptx.cuh"]))["mbar_wait_warp"]
     assert re.search(r"__all_sync\(0xffffffffu,\s*mbar_wait\(", body)
+
+
+def test_calls_on_different_streams_do_not_hold_one_lock_over_their_launches():
+    # the lock of a GPU's table of kept buffers guards the look-up; what is held over the launches belongs to the stream
+    text = sources()["fa_api.cu"]
+    assert re.search(r"lock = std::unique_lock<std::mutex>\(k->busy\)", text)
+    assert not re.search(r"unique_lock<std::mutex>\([^)]*shared", text)
