@@ -12,6 +12,14 @@
 
 namespace {
 
+// While it lives, a stream capture that another thread has begun does not forbid this thread's allocations and frees (they are
+// on streams that are not being captured).
+struct BesideCaptures {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // What all contexts of one GPU share: the stream-ordered pool their scratch is drawn from (freed blocks stay cached in it,
 // so steady-state calls do not reach the driver allocator) and, per stream, scratch kept between calls.  Work on one
 // stream is ordered, so consecutive calls there can use the same buffers and a call costs no allocation.  Kept: small
@@ -30,11 +38,18 @@ struct Kept {
     bool used = false;
     std::mutex busy;               // held from the look-up until the kernels that use the buffers are on the stream: calls on one
                                    // stream take turns, calls on others do not wait for them
-    void drop() {
-        if (scratch) cudaFree(scratch);
-        if (flags) cudaFree(flags);
-        if (zeros) cudaFree(zeros);
-        scratch = nullptr; flags = zeros = nullptr;
+    cudaEvent_t done = nullptr;    // recorded behind every call: the stream itself may be gone when the buffers are given back
+
+    // gives the buffers back behind the slot's last call, without waiting for it here; `s` is a stream of the library's own
+    void give_back(cudaStream_t s) {
+        if (done) {
+            cudaStreamWaitEvent(s, done, 0);
+            cudaEventDestroy(done);
+        }
+        if (scratch) cudaFreeAsync(scratch, s);
+        if (flags) cudaFreeAsync(flags, s);
+        if (zeros) cudaFreeAsync(zeros, s);
+        scratch = nullptr; flags = zeros = nullptr; done = nullptr;
         scratch_bytes = flag_words = zero_words = 0;
         used = false;
     }
@@ -47,17 +62,20 @@ struct DeviceScratch {
     std::mutex lock;               // of the members here and of which slot belongs to which stream; never held over a launch
     int contexts = 0;
     cudaMemPool_t pool = nullptr;
+    cudaStream_t reaper = nullptr; // where kept buffers are given back
     Kept kept[KEPT_STREAMS];
 
     cudaError_t acquire(int dev) {
         std::lock_guard<std::mutex> g(lock);
         if (contexts == 0) {
+            BesideCaptures relaxed;
             cudaMemPoolProps props = {};
             props.allocType = cudaMemAllocationTypePinned;
             props.handleTypes = cudaMemHandleTypeNone;
             props.location.type = cudaMemLocationTypeDevice;
             props.location.id = dev;
-            const cudaError_t e = cudaMemPoolCreate(&pool, &props);
+            cudaError_t e = cudaMemPoolCreate(&pool, &props);
+            if (e == cudaSuccess && (e = cudaStreamCreateWithFlags(&reaper, cudaStreamNonBlocking)) != cudaSuccess) cudaMemPoolDestroy(pool);
             if (e != cudaSuccess) return e;
             unsigned long long keep = ~0ull;  // keep freed scratch cached in the pool
             cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
@@ -68,18 +86,18 @@ struct DeviceScratch {
     void release(int dev) {
         std::lock_guard<std::mutex> g(lock);
         if (--contexts > 0) return;
-        bool any = false;
-        for (Kept& k : kept) any = any || k.scratch || k.flags || k.zeros;
-        if (any) {   // kernels that still use a kept buffer finish first
-            int cur = -1;
-            cudaGetDevice(&cur);
-            if (cur != dev) cudaSetDevice(dev);
-            cudaDeviceSynchronize();
-            for (Kept& k : kept) k.drop();
-            if (cur >= 0 && cur != dev) cudaSetDevice(cur);
-        }
-        cudaMemPoolDestroy(pool);  // pending frees complete first (stream-ordered)
+        // All of it is ordered behind the work that uses it and waits for nothing: kernels may still run, and a synchronising
+        // call would break a capture that some other thread has begun.
+        BesideCaptures relaxed;
+        int cur = -1;
+        cudaGetDevice(&cur);
+        if (cur != dev) cudaSetDevice(dev);
+        for (Kept& k : kept) k.give_back(reaper);
+        cudaMemPoolDestroy(pool);      // pending frees complete first (stream-ordered)
+        cudaStreamDestroy(reaper);     // likewise
+        if (cur >= 0 && cur != dev) cudaSetDevice(cur);
         pool = nullptr;
+        reaper = nullptr;
     }
     // the slot of a stream, or nullptr when all belong to others
     Kept* slot_of(unsigned long long stream_id) {
@@ -145,6 +163,7 @@ struct Scratch {
     uint32_t* zeros = nullptr;
     void* pooled[2] = {nullptr, nullptr};
     cudaStream_t stream = nullptr;
+    cudaEvent_t done = nullptr;
     std::unique_lock<std::mutex> lock;
 
     // grows one kept buffer of a stream; a block that is replaced is released behind the kernels that use it
@@ -166,6 +185,11 @@ struct Scratch {
 
     // need_flags: the call cannot do without flags (else they are given where the stream's kept ones serve)
     cudaError_t take(fa_ctx_t* c, cudaStream_t s, size_t bytes, size_t flag_words, bool need_flags, size_t zero_words) {
+        const cudaError_t e = take_from(c, s, bytes, flag_words, need_flags, zero_words);
+        if (e != cudaSuccess) give_back();
+        return e;
+    }
+    cudaError_t take_from(fa_ctx_t* c, cudaStream_t s, size_t bytes, size_t flag_words, bool need_flags, size_t zero_words) {
         stream = s;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         cudaError_t e = cudaStreamIsCapturing(s, &cap);
@@ -175,6 +199,8 @@ struct Scratch {
             Kept* k = c->shared->slot_of(id);
             if (k) {
                 lock = std::unique_lock<std::mutex>(k->busy);
+                if (!k->done && (e = cudaEventCreateWithFlags(&k->done, cudaEventDisableTiming)) != cudaSuccess) return e;
+                done = k->done;
                 if (flag_words && flag_words <= KEPT_WORDS_MAX) {
                     const uint32_t* before = k->flags;
                     if ((e = grow(c->shared->pool, k->flags, k->flag_words, flag_words, 4096, true, s)) != cudaSuccess) return e;
@@ -203,8 +229,8 @@ struct Scratch {
         const size_t more_zeros = zeros ? 0 : zero_words, more_flags = flags || !need_flags ? 0 : flag_words;
         if (more_zeros + more_flags) {
             const size_t n = (more_zeros + more_flags) * 4;
-            if ((e = cudaMallocFromPoolAsync(&pooled[1], n, c->shared->pool, s)) != cudaSuccess) { give_back(); return e; }
-            if ((e = fa_sm100::launch_clear_words(static_cast<uint32_t*>(pooled[1]), more_zeros + more_flags, s)) != cudaSuccess) { give_back(); return e; }
+            if ((e = cudaMallocFromPoolAsync(&pooled[1], n, c->shared->pool, s)) != cudaSuccess) return e;
+            if ((e = fa_sm100::launch_clear_words(static_cast<uint32_t*>(pooled[1]), more_zeros + more_flags, s)) != cudaSuccess) return e;
             if (more_zeros) zeros = static_cast<uint32_t*>(pooled[1]);
             if (more_flags) {
                 flags = static_cast<uint32_t*>(pooled[1]) + more_zeros;
@@ -213,8 +239,9 @@ struct Scratch {
         }
         return cudaSuccess;
     }
+    // behind the call's kernels, or behind what a failed call has queued
     cudaError_t give_back() {
-        cudaError_t r = cudaSuccess;
+        cudaError_t r = done ? cudaEventRecord(done, stream) : cudaSuccess;
         for (void*& p : pooled)
             if (p) {
                 const cudaError_t e = cudaFreeAsync(p, stream);

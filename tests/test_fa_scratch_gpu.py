@@ -192,3 +192,61 @@ def test_threads(cuda, built_libs, fa_ctx, streams, contexts):
         assert all(torch.equal(c.o, w) for c, w in zip(cs, ws))
     for c in ctxs:
         c.Destroy()
+
+
+LAST_CONTEXT = '''
+import threading, time
+import torch
+from goml_b200 import fa_forward as F
+codes = lambda *s: torch.randint(0, 0x60, s, dtype=torch.uint8, device="cuda")
+q, k, v = codes(64, 2048, 64), codes(64, 2048, 64), codes(64, 2048, 64)
+o = torch.empty(64, 2048, 64, dtype=torch.float16, device="cuda")
+call = lambda ctx, s: ctx.ForwardEx(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), 0, 64, 2048, 64, 1, 0, 0.1, 0.0125, 0, 0, 0, s.cuda_stream)
+x = torch.zeros(1 << 20, device="cuda")
+streams = [torch.cuda.Stream() for _ in range(3)]
+ctx = F.FACreate()
+call(ctx, streams[0])
+torch.cuda.synchronize()
+ctx.DeviceStatus()
+want = o.clone()
+ctx.Destroy()
+for again in range(3):
+    ctx, other = F.FACreate(), F.FACreate()
+    call(other, streams[1])
+    o.zero_()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(streams[0]):
+        torch.cuda._sleep(800_000_000)   # some 0.4 s
+    call(ctx, streams[0])
+    graph = torch.cuda.CUDAGraph()
+    took = []
+    def work():
+        torch.cuda.set_device(0)
+        t = time.perf_counter()
+        ctx.Destroy()
+        other.Destroy()                  # the last one
+        took.append(time.perf_counter() - t)
+    with torch.cuda.graph(graph, stream=streams[2]):
+        x.add_(1)
+        th = threading.Thread(target=work)
+        th.start()
+        th.join()
+        x.add_(1)
+    assert took and took[0] < 0.2, took
+    x.zero_()
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert (x == 2).all() and torch.equal(o, want)
+print("fine")
+'''
+
+
+def test_the_last_context_goes_while_work_is_queued_and_a_capture_is_open(cuda, built_libs):
+    # in a process of its own: no other context of the GPU is left
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", LAST_CONTEXT], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "fine" in r.stdout, r.stdout + r.stderr
