@@ -23,7 +23,8 @@ struct BesideCaptures {
 // What all contexts of one GPU share: the stream-ordered pool their scratch is drawn from (freed blocks stay cached in it,
 // so steady-state calls do not reach the driver allocator) and, per stream, scratch kept between calls.  Work on one
 // stream is ordered, so consecutive calls there can use the same buffers and a call costs no allocation.  Kept: small
-// buffers only (a large one is drawn from the pool per call, where the 2 us do not show), for a fixed number of streams.
+// buffers only (a large one is drawn from the pool per call, where the 2 us do not show), for a fixed number of streams;
+// a stream that has not called for KEPT_AGE calls of others, or is gone, gives its place and buffers up to a new one.
 // Streams are told apart by their id, which the driver never reuses.  Calls that are being captured into a graph do not
 // use it: a graph may be replayed on any stream.  Created with the first context of the GPU, released with the last.
 struct Kept {
@@ -36,12 +37,15 @@ struct Kept {
     uint32_t* zeros = nullptr;     // words that every call finds zero and leaves zero
     size_t zero_words = 0;
     bool used = false;
+    int users = 0;                 // calls that hold the slot or wait for it
+    unsigned long long last = 0;   // number of the slot's last call
     std::mutex busy;               // held from the look-up until the kernels that use the buffers are on the stream: calls on one
                                    // stream take turns, calls on others do not wait for them
     cudaEvent_t done = nullptr;    // recorded behind every call: the stream itself may be gone when the buffers are given back
 
     // gives the buffers back behind the slot's last call, without waiting for it here; `s` is a stream of the library's own
     void give_back(cudaStream_t s) {
+        BesideCaptures relaxed;
         if (done) {
             cudaStreamWaitEvent(s, done, 0);
             cudaEventDestroy(done);
@@ -56,6 +60,8 @@ struct Kept {
 };
 constexpr int MAX_DEVICES = 64;
 constexpr int KEPT_STREAMS = 8;
+// well above KEPT_STREAMS: more streams than places that call in turn do not chase each other's buffers
+constexpr unsigned long long KEPT_AGE = 64;
 constexpr size_t KEPT_SCRATCH_MAX = (size_t)64 << 20;
 constexpr size_t KEPT_WORDS_MAX = (size_t)1 << 20;
 struct DeviceScratch {
@@ -63,6 +69,7 @@ struct DeviceScratch {
     int contexts = 0;
     cudaMemPool_t pool = nullptr;
     cudaStream_t reaper = nullptr; // where kept buffers are given back
+    unsigned long long calls = 0;
     Kept kept[KEPT_STREAMS];
 
     cudaError_t acquire(int dev) {
@@ -99,19 +106,31 @@ struct DeviceScratch {
         pool = nullptr;
         reaper = nullptr;
     }
-    // the slot of a stream, or nullptr when all belong to others
-    Kept* slot_of(unsigned long long stream_id) {
+    // the slot of a stream, or nullptr when all belong to streams that still call; leave() follows
+    Kept* enter(unsigned long long stream_id) {
         std::lock_guard<std::mutex> g(lock);
-        Kept* vacant = nullptr;
+        calls++;
+        Kept* mine = nullptr;
+        Kept* oldest = nullptr;    // a vacant slot, or the one unused for longest
         for (Kept& k : kept) {
-            if (k.used && k.stream_id == stream_id) return &k;
-            if (!k.used && !vacant) vacant = &k;
+            if (k.used && k.stream_id == stream_id) { mine = &k; break; }
+            if (k.users == 0 && (!oldest || (oldest->used && (!k.used || k.last < oldest->last)))) oldest = &k;
         }
-        if (vacant) {
-            vacant->used = true;
-            vacant->stream_id = stream_id;
+        if (!mine && oldest && (!oldest->used || calls - oldest->last > KEPT_AGE)) {
+            if (oldest->used) oldest->give_back(reaper);
+            mine = oldest;
+            mine->used = true;
+            mine->stream_id = stream_id;
         }
-        return vacant;
+        if (mine) {
+            mine->users++;
+            mine->last = calls;
+        }
+        return mine;
+    }
+    void leave(Kept* k) {
+        std::lock_guard<std::mutex> g(lock);
+        k->users--;
     }
 };
 DeviceScratch g_scratch[MAX_DEVICES];
@@ -163,8 +182,15 @@ struct Scratch {
     uint32_t* zeros = nullptr;
     void* pooled[2] = {nullptr, nullptr};
     cudaStream_t stream = nullptr;
-    cudaEvent_t done = nullptr;
+    DeviceScratch* owner = nullptr;
+    Kept* slot = nullptr;
     std::unique_lock<std::mutex> lock;
+
+    ~Scratch() {
+        if (!slot) return;
+        lock.unlock();
+        owner->leave(slot);
+    }
 
     // grows one kept buffer of a stream; a block that is replaced is released behind the kernels that use it
     template <typename T>
@@ -196,11 +222,12 @@ struct Scratch {
         if (e != cudaSuccess) return e;
         unsigned long long id = 0;
         if (cap == cudaStreamCaptureStatusNone && cudaStreamGetId(s, &id) == cudaSuccess) {
-            Kept* k = c->shared->slot_of(id);
+            Kept* k = c->shared->enter(id);
             if (k) {
                 lock = std::unique_lock<std::mutex>(k->busy);
+                owner = c->shared;
+                slot = k;
                 if (!k->done && (e = cudaEventCreateWithFlags(&k->done, cudaEventDisableTiming)) != cudaSuccess) return e;
-                done = k->done;
                 if (flag_words && flag_words <= KEPT_WORDS_MAX) {
                     const uint32_t* before = k->flags;
                     if ((e = grow(c->shared->pool, k->flags, k->flag_words, flag_words, 4096, true, s)) != cudaSuccess) return e;
@@ -241,7 +268,7 @@ struct Scratch {
     }
     // behind the call's kernels, or behind what a failed call has queued
     cudaError_t give_back() {
-        cudaError_t r = done ? cudaEventRecord(done, stream) : cudaSuccess;
+        cudaError_t r = slot && slot->done ? cudaEventRecord(slot->done, stream) : cudaSuccess;
         for (void*& p : pooled)
             if (p) {
                 const cudaError_t e = cudaFreeAsync(p, stream);

@@ -79,3 +79,42 @@ def test_what_a_failed_call_has_queued_is_covered_too(library):
     lines = ctx.forward(7, ok=False)
     assert [x.split()[0] for x in lines] == ["alloc", "memset", "record"]
     ctx.destroy()
+
+
+def kept(lines):
+    """Whether a call used buffers that it did not draw."""
+    return not [x for x in lines if x.startswith("alloc")]
+
+
+def test_streams_that_are_gone_give_their_place_up(library):
+    # a stream per request: each finds a place again, and what it displaces is freed behind the displaced stream's last call
+    ctx = Context(library)
+    event = {}
+    for stream in range(1, 9):
+        event[stream] = field(ctx.forward(stream), "record", "event")[0]
+    lines = ctx.forward(9)
+    assert not field(lines, "record", "event") and not [x for x in lines if x.startswith("wait")]   # all places are in use
+    for _ in range(70):
+        assert kept(ctx.forward(8))
+    lines = ctx.forward(10)           # in the place of stream 1
+    freed = [x for x in lines if x.startswith("free")]
+    assert len(freed) == 2 and lines.index(next(x for x in lines if x.startswith("wait"))) < lines.index(freed[0])
+    assert field(lines, "wait", "event") == [event[1]] and not set(field(freed, "free", "stream")) & {str(s) for s in range(1, 11)}
+    assert kept(ctx.forward(10)) and kept(ctx.forward(8))
+    lines = ctx.forward(1)            # stream 1 is a new one again, in the place of stream 2
+    assert field(lines, "wait", "event") == [event[2]] and kept(ctx.forward(1))
+    ctx.destroy()
+
+
+def test_more_streams_than_places_in_turn(library):
+    # ten streams that call in turn: eight keep their buffers, two draw theirs for each call, nobody is displaced
+    ctx = Context(library)
+    for turn in range(30):
+        for stream in range(1, 11):
+            lines = ctx.forward(stream)
+            assert not [x for x in lines if x.startswith("wait")]
+            if turn:
+                assert kept(lines) == (stream <= 8)
+            if stream > 8:
+                assert len([x for x in lines if x.startswith("free")]) == len([x for x in lines if x.startswith("alloc")]) == 1
+    ctx.destroy()

@@ -107,6 +107,25 @@ def test_twenty_streams_give_the_same_bits(cuda, built_libs, fa_ctx, name):
         assert torch.equal(call.result(fa_ctx, stream), want)
 
 
+@pytest.mark.parametrize("name", ["handed", "line", "forward"])
+def test_streams_that_come_and_go(cuda, built_libs, fa_ctx, name):
+    # each of twenty streams calls a few times, among many calls of another, so that they take each other's places; queued
+    make = CALLS[name]
+    busy, calls = make(), [make() for _ in range(20)]
+    want = busy.result(fa_ctx)
+    for c in calls:
+        c.o.fill_(float("nan"))
+    torch.cuda.synchronize()
+    for stream, c in zip([torch.cuda.Stream() for _ in calls], calls):
+        for _ in range(3):
+            c(fa_ctx, stream)
+        for _ in range(70):
+            busy(fa_ctx)
+    torch.cuda.synchronize()
+    fa_ctx.DeviceStatus()
+    assert all(torch.equal(c.o, want) for c in [busy, *calls])
+
+
 def node_types(graph):
     import ctypes as C
     cu = C.CDLL("libcuda.so.1")
