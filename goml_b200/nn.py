@@ -99,13 +99,27 @@ class FP8KVCache:
         self.scales = torch.ones(2, dtype=torch.float32, device=device)      # k_scale, v_scale
         self.lens = torch.zeros(batch, dtype=torch.int32, device=device)     # keys cached per sequence
 
-    def takes(self, batch: int, heads: int, S: int, hd: int) -> bool:
-        """Whether a prompt's codes can be written straight into this cache: dense buffers of the shapes it was made with."""
+    def dense_on(self, device: torch.device) -> bool:
+        """Whether kernels of `device` that are given the buffers' pointers find the cache there: codes [batch, heads, s_max, hd]
+        without gaps, two scales and the lengths, all on that device."""
+        k, v, scales, lens = self.k, self.v, self.scales, self.lens
+        if not (k.device == v.device == scales.device == lens.device == device and scales.dtype is torch.float32 and lens.dtype is torch.int32
+                and k.is_contiguous() and v.is_contiguous() and scales.is_contiguous() and lens.is_contiguous()):
+            return False
+        if k.shape == v.shape == (self.B, self.H, self.s_max, self.hd) and k.dtype is v.dtype is torch.uint8 and lens.shape == (self.B,):
+            return scales.numel() >= 2
+        # other views of the same bytes
+        codes = self.B * self.H * self.s_max * self.hd
+        return (all(t.element_size() == 1 and t.numel() >= codes and (t.dim() == 1 or t.shape[-2:] == (self.s_max, self.hd)) for t in (k, v))
+                and scales.numel() >= 2 and lens.numel() >= self.B)
+
+    def takes(self, batch: int, heads: int, S: int, hd: int, device: "torch.device | None" = None) -> bool:
+        """Whether a prompt's codes can be written straight into this cache by a kernel of `device` (the codes' own by default)."""
+        device = self.k.device if device is None else device
         shape = (batch, heads, self.s_max, hd)
-        return (S <= self.s_max and all(t.shape == shape and t.dtype == torch.uint8 and t.is_contiguous() and t.is_cuda and t.data_ptr() % 16 == 0
-                                        for t in (self.k, self.v))
-                and self.scales.dtype == torch.float32 and self.scales.shape == (2,) and self.scales.is_contiguous() and self.scales.is_cuda
-                and self.lens.dtype == torch.int32 and self.lens.shape == (batch,) and self.lens.is_contiguous() and self.lens.is_cuda)
+        return ((batch, heads, hd) == (self.B, self.H, self.hd) and S <= self.s_max and self.dense_on(device)
+                and all(t.shape == shape and t.dtype == torch.uint8 and t.data_ptr() % 16 == 0 for t in (self.k, self.v))
+                and self.scales.shape == (2,) and self.lens.shape == (batch,))
 
     def fill(self, k_codes, v_codes, scales, S: int) -> None:
         """Prompt phase: K/V codes [batch*heads, S, hd] as the prefill quantiser wrote them, and their two scales."""
@@ -188,7 +202,7 @@ class FP8DecoderBlock:
         BG.RMSNormQuantizeInto(src.data_ptr(), h.data_ptr(), self.norm1.data_ptr(), xc, sc, sc + 4, rstd, 0, T, d, self.eps, sh)
         G.FP8GEMMScaled(T, 3 * d, d, xc, self.qkv.w.codes.data_ptr(), qkv, 1.0, sc, self.qkv.w.scale_ptr, G.OutBF16, sh)   # [T, 3, H, hd] bf16
         s3 = sc + 8                                             # scales[3], amaxes[3]
-        if cache is not None and cache.takes(B, H, S, hd):
+        if cache is not None and cache.takes(B, H, S, hd, x.device):
             BG.RopeQuantizeQKVCache(qkv, cos.data_ptr(), sin.data_ptr(), qc, kc, vc, s3, s3 + 12, cache.k.data_ptr(), cache.v.data_ptr(),
                                     cache.scales.data_ptr(), cache.lens.data_ptr(), B, S, cache.s_max, H, hd, sh)
         else:
@@ -210,6 +224,8 @@ class FP8DecoderBlock:
         epilogue) -> the feed-forward half of forward_fused."""
         B, d, H, hd = x.shape[0], self.d, self.H, self.hd
         assert (B, H, hd) == (cache.B, cache.H, cache.hd)
+        if not cache.dense_on(x.device):
+            raise ValueError(f"decode_step: the cache's buffers must lie without gaps, in the shapes it was made with, on {x.device}")
         sh = torch.cuda.current_stream().cuda_stream
         n = B * d
         buf, xc, qkv, qc, o, oc, rstd, sc = _scratch(x.device, n, 6 * n, n, 2 * n, n, 4 * B, 24)

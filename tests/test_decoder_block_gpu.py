@@ -302,6 +302,9 @@ def test_inputs_and_caches_that_take_the_copying_route(cuda, built_libs):
         y = blk(xin, B, S, cache)
         torch.cuda.synchronize()
         assert torch.equal(xin, before) and y.data_ptr() != xin.data_ptr()
+        if not dense:   # the prompt is copied in; the step, which is given pointers, does not take such a cache
+            with pytest.raises(ValueError):
+                blk.decode_step(x[:B], cache)
         out.append((y, cache.k[:, :, :S].clone(), cache.v[:, :, :S].clone(), cache.scales, cache.lens))
     for other in out[1:]:
         assert all(torch.equal(a, b) for a, b in zip(out[0][1:], other[1:]))
