@@ -143,11 +143,14 @@ def _scratch(dev, *sizes):
 
 def _stream_start(x: torch.Tensor, rows: int, d: int):
     """(source, h) of a block's residual stream: h is written by the first RMSNorm while it reads x, or is a copy already
-    (source = h) where x is not what that kernel reads."""
-    if (x.dtype == torch.float32 and x.is_contiguous() and x.data_ptr() % 32 == 0 and x.numel() == rows * d
+    (source = h) where x is not what that kernel reads.  The kernels behind it address h as rows of d values without gaps, so
+    what its copy does not turn into that (a clone keeps the order of strides) is refused."""
+    assert x.shape == (rows, d), f"the block takes [{rows}, {d}], not {list(x.shape)}"
+    if (x.dtype == torch.float32 and x.is_contiguous() and x.data_ptr() % 32 == 0
             and not (x.requires_grad and torch.is_grad_enabled())):
         return x, torch.empty_like(x)
     h = x.float().clone()
+    assert h.is_contiguous(), f"the block takes rows of {d} values, not strides {x.stride()}"
     return h, h
 
 

@@ -293,7 +293,8 @@ def test_inputs_and_caches_that_take_the_copying_route(cuda, built_libs):
     shifted = room[1:].view(B * S, d)
     shifted.copy_(x)
     out = []
-    for xin, dense in ((x, True), (shifted, True), (x.bfloat16(), True), (x, False)):
+    wide = torch.cat([x, -x], dim=1)[:, :d]
+    for xin, dense in ((x, True), (shifted, True), (x.bfloat16(), True), (wide, True), (x, False)):
         before = xin.clone()
         cache = nn.FP8KVCache(B, H, S + 8, d // H)
         if not dense:
@@ -306,6 +307,12 @@ def test_inputs_and_caches_that_take_the_copying_route(cuda, built_libs):
             with pytest.raises(ValueError):
                 blk.decode_step(x[:B], cache)
         out.append((y, cache.k[:, :, :S].clone(), cache.v[:, :, :S].clone(), cache.scales, cache.lens))
+    for refused in (x.t().contiguous().t(), x.view(B, S, d), torch.cat([x, x[:1]]), x[1:]):
+        with pytest.raises(AssertionError):
+            blk(refused, B, S)
+    for refused in (x[:B].t().contiguous().t(), x[:B].view(B, 1, d)):
+        with pytest.raises(AssertionError):
+            blk.decode_step(refused, nn.FP8KVCache(B, H, S + 8, d // H))
     for other in out[1:]:
         assert all(torch.equal(a, b) for a, b in zip(out[0][1:], other[1:]))
         # sums of the larger GEMMs need not meet in one order: a last bit becomes an isolated neighbouring e4m3 code (2^-4 of a value

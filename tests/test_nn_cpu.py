@@ -52,3 +52,44 @@ def test_caches_that_they_can():
     # what a step reads through its pointer, and a prompt is copied into
     for other in (dict(k=u8(B, H, S_MAX, HD).view(torch.float8_e4m3fn)), dict(lens=torch.zeros(B + 1, dtype=torch.int32))):
         assert cache(**other).dense_on(CPU) and not cache(**other).takes(B, H, 8, HD, CPU)
+
+
+T, D = 6, 32
+
+
+def rows_of(n, d, offset=0):
+    room = torch.zeros(n * d + 64)
+    start = -room.data_ptr() // 4 % 8 + offset      # 32-byte aligned, and `offset` values past that
+    x = room[start:start + n * d].view(n, d)
+    x.copy_(torch.arange(n * d, dtype=torch.float32).view(n, d))
+    return x
+
+
+INPUTS = {   # the input, and whether the first kernel can read it where it is
+    "dense": (lambda: rows_of(T, D), True),
+    "misaligned": (lambda: rows_of(T, D, 1), False),
+    "rows of a wider tensor": (lambda: rows_of(T, 2 * D)[:, :D], False),
+    "every other row": (lambda: rows_of(2 * T, D)[::2], False),
+    "one row for all": (lambda: rows_of(1, D).expand(T, D), False),
+    "bf16": (lambda: rows_of(T, D).bfloat16(), False),
+    "double": (lambda: rows_of(T, D).double(), False),
+    "needs a gradient": (lambda: rows_of(T, D).requires_grad_(), False),
+}
+
+
+@pytest.mark.parametrize("name", INPUTS)
+def test_the_streams_start(name):
+    make, direct = INPUTS[name]
+    x = make()
+    src, h = nn._stream_start(x, T, D)
+    assert (src is x) == direct and (src is h) != direct
+    assert h.shape == (T, D) and h.is_contiguous() and h.dtype == torch.float32 and h.data_ptr() != x.data_ptr()
+    assert torch.equal(src, x.float())
+
+
+@pytest.mark.parametrize("name,x", [("columns", rows_of(D, T).t()), ("sequences behind one another", rows_of(T, D).view(3, 2, D).transpose(0, 1)),
+                                    ("three dimensions", rows_of(T, D).view(2, 3, D)), ("a row too few", rows_of(T - 1, D)),
+                                    ("a row too many", rows_of(T + 1, D)), ("shorter rows", rows_of(2 * T, D // 2))])
+def test_inputs_that_are_no_rows_are_refused(name, x):
+    with pytest.raises(AssertionError):
+        nn._stream_start(x, T, D)
