@@ -315,7 +315,5 @@ def test_inputs_and_caches_that_take_the_copying_route(cuda, built_libs):
             blk.decode_step(refused, nn.FP8KVCache(B, H, S + 8, d // H))
     for other in out[1:]:
         assert all(torch.equal(a, b) for a, b in zip(out[0][1:], other[1:]))
-        # sums of the larger GEMMs need not meet in one order: a last bit becomes an isolated neighbouring e4m3 code (2^-4 of a value
-        # in fewer than one in forty of them: 2^-4 * sqrt(1/40) < 1e-2 in the norm)
-        assert (out[0][0] - other[0]).norm() <= 1e-2 * out[0][0].norm()
+        assert torch.equal(out[0][0], other[0])   # 80 rows: every GEMM adds its partial sums in a fixed order
     blk.close()
