@@ -129,6 +129,11 @@ class FP8KVCache:
         self.lens.fill_(S)
 
 
+def _writes_directly(cache, B: int, H: int, S: int, hd: int, device: torch.device) -> bool:
+    """Whether the prompt's codes go straight into the cache; a cache with a `fill` of its own has that called."""
+    return isinstance(cache, FP8KVCache) and type(cache).fill is FP8KVCache.fill and "fill" not in vars(cache) and cache.takes(B, H, S, hd, device)
+
+
 def _scratch(dev, *sizes):
     """One allocation cut into 256-byte aligned pieces: (the buffer, their addresses).  A call has a dozen temporaries, and
     drawing each from the allocator took about a third of a decode step's host time."""
@@ -205,7 +210,7 @@ class FP8DecoderBlock:
         BG.RMSNormQuantizeInto(src.data_ptr(), h.data_ptr(), self.norm1.data_ptr(), xc, sc, sc + 4, rstd, 0, T, d, self.eps, sh)
         G.FP8GEMMScaled(T, 3 * d, d, xc, self.qkv.w.codes.data_ptr(), qkv, 1.0, sc, self.qkv.w.scale_ptr, G.OutBF16, sh)   # [T, 3, H, hd] bf16
         s3 = sc + 8                                             # scales[3], amaxes[3]
-        if cache is not None and cache.takes(B, H, S, hd, x.device):
+        if _writes_directly(cache, B, H, S, hd, x.device):
             BG.RopeQuantizeQKVCache(qkv, cos.data_ptr(), sin.data_ptr(), qc, kc, vc, s3, s3 + 12, cache.k.data_ptr(), cache.v.data_ptr(),
                                     cache.scales.data_ptr(), cache.lens.data_ptr(), B, S, cache.s_max, H, hd, sh)
         else:

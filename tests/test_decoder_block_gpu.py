@@ -307,6 +307,15 @@ def test_inputs_and_caches_that_take_the_copying_route(cuda, built_libs):
             with pytest.raises(ValueError):
                 blk.decode_step(x[:B], cache)
         out.append((y, cache.k[:, :, :S].clone(), cache.v[:, :, :S].clone(), cache.scales, cache.lens))
+    calls = []
+
+    class Duck:   # a cache that only has a fill gets the same codes, scales and length
+        def fill(self, k_codes, v_codes, scales, n):
+            calls.append((k_codes.view(B, H, S, d // H).clone(), v_codes.view(B, H, S, d // H).clone(), scales.clone(), n))
+
+    y = blk(x, B, S, Duck())
+    (k, v, scales, n), = calls
+    assert n == S and all(torch.equal(a, b) for a, b in zip(out[0][:4], (y, k, v, scales)))
     for refused in (x.t().contiguous().t(), x.view(B, S, d), torch.cat([x, x[:1]]), x[1:]):
         with pytest.raises(AssertionError):
             blk(refused, B, S)

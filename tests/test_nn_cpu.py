@@ -93,3 +93,19 @@ def test_the_streams_start(name):
 def test_inputs_that_are_no_rows_are_refused(name, x):
     with pytest.raises(AssertionError):
         nn._stream_start(x, T, D)
+
+
+def test_a_cache_with_a_fill_of_its_own_has_it_called():
+    class Counting(nn.FP8KVCache):
+        def fill(self, *args):
+            super().fill(*args)
+
+    class Duck:   # anything with a fill was good enough for the prompt
+        def fill(self, k_codes, v_codes, scales, S):
+            pass
+
+    patched = cache()
+    patched.fill = lambda *args: None
+    assert nn._writes_directly(cache(), B, H, 8, HD, CPU)
+    for c in (Counting(B, H, S_MAX, HD, device="cpu"), Duck(), patched, None):
+        assert not nn._writes_directly(c, B, H, 8, HD, CPU)
