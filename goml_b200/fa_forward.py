@@ -76,6 +76,15 @@ _PACK_FORWARD = struct.Struct("@5P5i2f4P").pack
 _PACK_DECODE = struct.Struct("@6P6i2f5P3i0P").pack
 assert struct.calcsize("@5P5i2f4P") == C.sizeof(ForwardArgs) and struct.calcsize("@6P6i2f5P3i0P") == C.sizeof(DecodeArgs)
 
+
+def _pack(pack, block, *args) -> bytes:
+    """The argument block's bytes; values that struct.pack has no format for (a c_void_p, a float out of range) go through
+    the ctypes structure, which takes or refuses them."""
+    try:
+        return pack(*args)
+    except (struct.error, OverflowError):
+        return bytes(block(*args))
+
 _lock = threading.Lock()
 _lib = None
 _lib_err = None
@@ -206,8 +215,8 @@ class FAContext:
                   scale_q_dev=0, scale_k_dev=0, scale_v_dev=0, stream=0) -> None:
         if not self.ptr:
             raise FAError("FAContext.ForwardEx: nil ctx", FA_ERR_INVALID_ARG)
-        st = _forward_ex(self.ptr, _PACK_FORWARD(q or 0, k or 0, v or 0, o or 0, lOut or 0, bh, sl, hd, causal, window, scale, v_descale,
-                                                 scale_q_dev or 0, scale_k_dev or 0, scale_v_dev or 0, stream or 0))
+        st = _forward_ex(self.ptr, _pack(_PACK_FORWARD, ForwardArgs, q or 0, k or 0, v or 0, o or 0, lOut or 0, bh, sl, hd, causal, window,
+                                         scale, v_descale, scale_q_dev or 0, scale_k_dev or 0, scale_v_dev or 0, stream or 0))
         if st != FA_OK:
             raise FAError("fa_forward_ex", st, self._msg())
 
@@ -220,9 +229,9 @@ class FAContext:
         hd] and s_max is ignored."""
         if not self.ptr:
             raise FAError("FAContext.Decode: nil ctx", FA_ERR_INVALID_ARG)
-        st = _decode(self.ptr, _PACK_DECODE(q or 0, k_cache or 0, v_cache or 0, o or 0, lOut or 0, seq_lens or 0, batch, q_heads, kv_heads, hd,
-                                            s_max, seq_len, scale, v_descale, scale_q_dev or 0, scale_k_dev or 0, scale_v_dev or 0, stream or 0,
-                                            block_table or 0, page_size, max_pages_per_seq, num_pages))
+        st = _decode(self.ptr, _pack(_PACK_DECODE, DecodeArgs, q or 0, k_cache or 0, v_cache or 0, o or 0, lOut or 0, seq_lens or 0, batch, q_heads,
+                                     kv_heads, hd, s_max, seq_len, scale, v_descale, scale_q_dev or 0, scale_k_dev or 0, scale_v_dev or 0,
+                                     stream or 0, block_table or 0, page_size, max_pages_per_seq, num_pages))
         if st != FA_OK:
             raise FAError("fa_decode", st, self._msg())
 

@@ -96,3 +96,41 @@ def test_decode_append_restatement_properties():
 def test_fixed_scale_quantiser_saturates():
     codes = glue.quantize_fixed_scale(np.array([1e6, -1e6, 0.0, 448.0, 0.5], np.float32), 1.0)
     assert list(codes) == [0x7E, 0xFE, 0x00, 0x7E, 0x30]
+
+
+def test_argument_blocks_are_packed_as_the_ctypes_structures():
+    # whatever the structures take, the packed block takes, with the same bytes; what they refuse it refuses with their error
+    import ctypes as C
+
+    import pytest
+    from goml_b200 import fa_forward as F
+    forward = (16, 32, 48, 64, 0, 4, 256, 64, 1, 0, 0.125, 1.0, 80, 0, 96, 2 ** 48)
+    decode = (16, 32, 48, 64, 0, 80, 3, 8, 2, 128, 300, 0, 0.25, 1.0, 0, 96, 112, 7, 0, 64, 5, 9)
+    for pack, block, base in ((F._PACK_FORWARD, F.ForwardArgs, forward), (F._PACK_DECODE, F.DecodeArgs, decode)):
+        pointers = [i for i, (_, t) in enumerate(block._fields_) if t is C.c_void_p]
+        ints = [i for i, (_, t) in enumerate(block._fields_) if t is C.c_int]
+        floats = [i for i, (_, t) in enumerate(block._fields_) if t is C.c_float]
+        changes = [(0, 16)] + [(i, v) for i in pointers for v in (C.c_void_p(4096), 2 ** 63 + 5, -16)]
+        changes += [(i, v) for i in ints for v in (-1, True, 2 ** 31, 2 ** 40 + 3, np.int64(5))]
+        changes += [(i, v) for i in floats for v in (3, -0.0, np.float32(0.1), float("inf"), float("nan"), 1e300)]
+        for i, v in changes:
+            args = base[:i] + (v,) + base[i + 1:]
+            want = None
+            try:
+                want = bytes(block(*args))
+            except TypeError:
+                pass
+            if want is None:
+                try:
+                    F._pack(pack, block, *args)
+                except TypeError:
+                    continue
+                assert isinstance(v, np.integer), (i, v)   # an integer all the same
+            else:
+                assert F._pack(pack, block, *args) == want, (i, v)
+        for i, v in [(i, "x") for i in pointers] + [(i, 1.5) for i in ints] + [(i, "x") for i in floats]:
+            args = base[:i] + (v,) + base[i + 1:]
+            with pytest.raises(TypeError):
+                bytes(block(*args))
+            with pytest.raises(TypeError):
+                F._pack(pack, block, *args)
