@@ -707,6 +707,7 @@ __global__ void clear_words_kernel(uint32_t* w, uint32_t n) {
 
 struct Layout {
     int plan, splits, grid, rows;
+    bool streams;
     bool cuts() const { return plan != SPLITS || splits > 1; }   // whether a pair may be cut
 };
 // One query head per kv head keeps the streams: fixed splits while the pairs leave room for them, else the line with
@@ -716,18 +717,24 @@ Layout layout_of(int batch, int q_heads, int kv_heads, int span) {
     Layout x;
     const int group = q_heads / kv_heads;
     x.rows = group <= 8 ? 8 : 16;
-    const long long pairs = (long long)batch * kv_heads, chunks = (span + CHUNK - 1) / CHUNK;
+    x.streams = group == 1;
+    const long long pairs = (long long)batch * kv_heads, chunks = ((long long)span + CHUNK - 1) / CHUNK;
     const long long narrow = (long long)ctas_per_sm(1, false) * num_sms_of_current_device();
     long long splits = narrow / pairs;
     if (splits > chunks) splits = chunks;
     if (splits > 64) splits = 64;
     if (splits < 1) splits = 1;
     x.splits = (int)splits;
-    if (group == 1 && pairs * splits <= narrow) {
+    if (x.streams && pairs * splits <= narrow) {
         x.plan = SPLITS;
         x.grid = (int)(pairs * splits);
+    } else if (pairs * chunks > 0x7fffffffLL) {
+        // a line of more chunks than an int counts (a paged cache whose capacity is far above what it holds): a CTA per pair
+        x.plan = SPLITS;
+        x.splits = 1;
+        x.grid = (int)pairs;
     } else {
-        x.plan = group == 1 ? LINE_HANDED : LINE;
+        x.plan = x.streams ? LINE_HANDED : LINE;
         const long long slots = (long long)ctas_per_sm(x.rows / 8, true) * num_sms_of_current_device();
         const long long units = pairs * chunks;
         x.grid = (int)(units < slots ? (units > 0 ? units : 1) : slots);
@@ -752,7 +759,7 @@ size_t decode_flag_count(int batch, int q_heads, int kv_heads, int span) {
 
 cudaError_t launch_decode(const DecodeArgs& a) {
     const int span = decode_span(a);
-    if ((long long)a.batch * a.kv_heads * ((span + CHUNK - 1) / CHUNK) > 0x7fffffffLL) return cudaErrorInvalidValue;
+    if ((long long)a.batch * a.kv_heads > 0x7fffffffLL) return cudaErrorInvalidValue;
     const Layout x = layout_of(a.batch, a.q_heads, a.kv_heads, span);
     if (x.cuts() && (!a.workspace || !a.arrivals)) return cudaErrorInvalidValue;
     if (x.plan == LINE_HANDED && !a.flags) return cudaErrorInvalidValue;
@@ -769,7 +776,7 @@ cudaError_t launch_decode(const DecodeArgs& a) {
     p.v_descale = a.v_descale;
     p.sq = a.scale_q_dev; p.sk = a.scale_k_dev; p.sv = a.scale_v_dev;
     p.plan = x.plan; p.splits = x.splits;
-    p.chunks_per_split = ((span + CHUNK - 1) / CHUNK + x.splits - 1) / x.splits;
+    p.chunks_per_split = (int)((((long long)span + CHUNK - 1) / CHUNK + x.splits - 1) / x.splits);
     p.block_table = a.block_table;
     p.page_mul = p.page_shr = 0;
     if (a.block_table) {   // page_size >= 64; exact for numerators below 2^31, and the multiplier fits 32 bits
@@ -786,10 +793,10 @@ cudaError_t launch_decode(const DecodeArgs& a) {
     p.handed = a.flags; p.epoch = a.epoch;
     auto run = [&](auto contiguous, auto paged) { return launch_pdl(a.block_table ? paged : contiguous, x.grid, THREADS, 0, a.stream, p); };
 #define KERNEL(D, NQ, WIDE, STREAMS) run(fa_decode_kernel<D, NQ, WIDE, STREAMS, false>, fa_decode_kernel<D, NQ, WIDE, STREAMS, true>)
-#define KERNELS(D)                                                    \
-    (x.plan == SPLITS        ? KERNEL(D, 1, false, true)              \
-     : x.plan == LINE_HANDED ? KERNEL(D, 1, true, true)               \
-     : x.rows == 8           ? KERNEL(D, 1, true, false) : KERNEL(D, 2, true, false))
+#define KERNELS(D)                                             \
+    (x.streams && x.plan == SPLITS ? KERNEL(D, 1, false, true) \
+     : x.streams                   ? KERNEL(D, 1, true, true)  \
+     : x.rows == 8                 ? KERNEL(D, 1, true, false) : KERNEL(D, 2, true, false))
     return a.hd == 128 ? KERNELS(128) : KERNELS(64);
 #undef KERNELS
 #undef KERNEL

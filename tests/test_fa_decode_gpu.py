@@ -202,3 +202,34 @@ def test_decode_work_split(cuda, built_libs, fa_ctx, B, Hq, Hkv, Smax, D, lens):
     maxabs, meanrel = O.error_stats(got[some], ref[some])
     assert maxabs <= 2e-2 and meanrel <= 1e-2, (maxabs, meanrel)
     assert np.abs(lse[some] - rl[some]).max() <= 5e-3
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,D", [(256, 1, 1, 64), (64, 8, 4, 128), (128, 10, 2, 64), (3, 2, 2, 64)])
+def test_capacity_far_above_what_is_held(cuda, built_libs, fa_ctx, B, Hq, Hkv, D):
+    # 2^30 rows a sequence in the block table (2^24 chunks of 64 keys: with 256 pairs more than an int counts), few of them
+    # held; unused entries name no page
+    page, max_pages, held = 65536, 16384, 3
+    name = f"decode-capacity{B}_{Hq}_{Hkv}_{D}"
+    q, k, v, sq, sk, sv = make_case(name, B, Hq, Hkv, 150, D)
+    seq_lens = np.arange(B) % 151
+    kd, vd = (torch.zeros(held, Hkv, page, D, dtype=torch.uint8, device="cuda") for _ in range(2))
+    for i in range(held):    # sequence b lives in page b % 3: the content of the first three sequences
+        kd[i, :, :150], vd[i, :, :150] = torch.from_numpy(k[i % B]).cuda(), torch.from_numpy(v[i % B]).cuda()
+    table = torch.full((B, max_pages), -1, dtype=torch.int32, device="cuda")
+    table[:, 0] = torch.arange(B, device="cuda") % held
+    scale = sq * sk / math.sqrt(D)
+    qd, sl = torch.from_numpy(q).cuda(), torch.from_numpy(seq_lens.astype(np.int32)).cuda()
+    o = torch.full((B, Hq, D), float("nan"), dtype=torch.float16, device="cuda")
+    lse = torch.full((B, Hq), float("nan"), dtype=torch.float32, device="cuda")
+    fa_ctx.Decode(qd.data_ptr(), kd.data_ptr(), vd.data_ptr(), o.data_ptr(), lse.data_ptr(), sl.data_ptr(), B, Hq, Hkv, D, 0, 0, scale, sv,
+                  block_table=table.data_ptr(), page_size=page, max_pages_per_seq=max_pages, num_pages=held)
+    torch.cuda.synchronize()
+    fa_ctx.DeviceStatus()
+    src = np.arange(B) % held % B
+    ref, rl = glue.decode_attention_f64(q, k[src], v[src], seq_lens, scale, sv)
+    some = seq_lens > 0
+    got, glse = o.double().cpu().numpy(), lse.double().cpu().numpy()
+    assert np.all(got[~some] == 0) and np.all(np.isneginf(glse[~some]))
+    maxabs, meanrel = O.error_stats(got[some], ref[some])
+    assert maxabs <= 2e-2 and meanrel <= 1e-2, (maxabs, meanrel)
+    assert np.abs(glse[some] - rl[some]).max() <= 5e-3
