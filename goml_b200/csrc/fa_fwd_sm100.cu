@@ -203,11 +203,9 @@ __global__ void __launch_bounds__(V_THREADS, 12) v_to_f16_kernel(const uint4* in
 // Producer-side view of the pre-pass: how many leading chunks of this head (from chunk `c` on) are known to be ready.
 // The whole warp asks for 32 flags at a time, so a head of up to 4096 keys costs one load when it is complete.
 // Bounded like every wait of this file.
-// `ok` is each lane's outcome of the waits before; the lanes enter the polls together or not at all.
-__device__ __forceinline__ bool wait_v_chunk(bool ok, const uint32_t* head_flags, int chunks_per_head, uint32_t epoch, int c, int& ready,
+__device__ __forceinline__ bool wait_v_chunk(const uint32_t* head_flags, int chunks_per_head, uint32_t epoch, int c, int& ready,
                                              volatile uint32_t* abort_flag) {
-    if (c < ready) return ok;
-    if (!__all_sync(0xffffffffu, ok)) return false;
+    if (c < ready) return true;
     const int lane = threadIdx.x & 31;
     uint64_t t0 = 0;
     for (uint32_t polls = 1;; polls++) {
@@ -336,25 +334,25 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
             uint32_t ph = 1;  // "previous phase complete": the rings start empty
             for (int j = 0; j < nblk; j++) {
                 const int key0 = (blk0 + j) * BN;
-                bool ok = mbar_wait(bar_sfull + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD);   // Q K^T three blocks back is done
-                if (leader && ok) {
+                if (!mbar_wait_warp(bar_sfull + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD)) break;   // Q K^T three blocks back is done
+                if (leader) {
                     mbar_arrive_expect_tx(bar_kfull + 8 * s, C::K_BYTES);
                     tma_load_3d(sbase + C::OFF_K + s * C::K_BYTES, &tmap_k, bar_kfull + 8 * s, 0, key0, head);
                 }
-                ok = ok && mbar_wait(bar_pvdone + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD);  // P V three blocks back is done
+                if (!mbar_wait_warp(bar_pvdone + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD)) break;  // P V three blocks back is done
                 if (!head_flags) {
                     if (j == 0) pdl_wait();
-                } else {
-                    ok = wait_v_chunk(ok, head_flags, p.v_chunks, p.v_epoch, key0 / V_CHUNK, v_ready, abort_flag);
+                } else if (!wait_v_chunk(head_flags, p.v_chunks, p.v_epoch, key0 / V_CHUNK, v_ready, abort_flag)) {
+                    break;
                 }
-                if (leader && ok) {
+                if (leader) {
                     mbar_arrive_expect_tx(bar_vfull + 8 * s, C::V_BYTES);
 #pragma unroll
                     for (int h = 0; h < HD / 64; h++)  // one 64-column (128-byte) slab of d per copy
                         tma_load_3d(sbase + C::OFF_V + s * C::V_BYTES + h * C::V_HALF_BYTES, &tmap_v, bar_vfull + 8 * s,
                                     h * 64, key0, head);
                 }
-                if (!__all_sync(0xffffffffu, ok)) break;
+                __syncwarp();
                 if (++s == STAGES) { s = 0; ph ^= 1; }
             }
             pdl_wait();   // this kernel completes after the pre-pass
@@ -372,28 +370,30 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
             uint32_t kph = 0, vph = 0;
             bool ok = true;
             auto issue_qk = [&](int j) {  // S[j & 1] = Q K(j)^T
-                ok = mbar_wait(bar_kfull + 8 * ks, kph, abort_flag, ST_TIMEOUT_MMA);
+                ok = mbar_wait_warp(bar_kfull + 8 * ks, kph, abort_flag, ST_TIMEOUT_MMA);
+                if (!ok) return;
                 tc_fence_after();
                 const uint64_t qd = qk_desc(sbase + C::OFF_Q);
                 const uint64_t kd = qk_desc(sbase + C::OFF_K + ks * C::K_BYTES);
-                if (leader && ok) {
+                if (leader) {
 #pragma unroll
                     for (int k = 0; k < HD / 32; k++)
                         mma_f8f6f4_ss(tmem_s + (j & 1) * BN, qd + 2 * k, kd + 2 * k, idesc_qk, k != 0);
                     mma_commit(bar_sfull + 8 * ks);
                 }
-                ok = __all_sync(0xffffffffu, ok);
+                __syncwarp();
                 if (++ks == STAGES) { ks = 0; kph ^= 1; }
             };
             ok = mbar_wait_warp(bar_q, 0, abort_flag, ST_TIMEOUT_MMA);
             for (int j = 0; j < 2 && j < nblk && ok; j++) issue_qk(j);
             for (int j = 0; j < nblk && ok; j++) {
                 const int b = j & 1;
-                ok = mbar_wait(bar_vfull + 8 * vs, vph, abort_flag, ST_TIMEOUT_MMA) &&
-                     mbar_wait(bar_pfull + 8 * b, (j >> 1) & 1, abort_flag, ST_TIMEOUT_MMA);
+                ok = mbar_wait_warp(bar_vfull + 8 * vs, vph, abort_flag, ST_TIMEOUT_MMA) &&
+                     mbar_wait_warp(bar_pfull + 8 * b, (j >> 1) & 1, abort_flag, ST_TIMEOUT_MMA);
+                if (!ok) break;
                 tc_fence_after();
                 const uint32_t vaddr = sbase + C::OFF_V + vs * C::V_BYTES;
-                if (leader && ok) {
+                if (leader) {
 #pragma unroll
                     for (int k = 0; k < BN / 16; k++) {  // 16 keys per MMA: 8 TMEM columns of P, 16 rows of V
                         const uint64_t vd = mnmajor_desc_sw128(vaddr + k * 16 * 128, C::V_HALF_BYTES);
@@ -401,8 +401,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
                     }
                     mma_commit(bar_pvdone + 8 * vs);
                 }
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
+                __syncwarp();
                 if (++vs == STAGES) { vs = 0; vph ^= 1; }
                 // S[b] is rewritten by the Q K^T two blocks ahead; it is issued behind this P V on the
                 // same in-order tensor pipe, so P(j) has been read before S(j+2) lands on it

@@ -139,10 +139,10 @@ fp8_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                 if (it.nh == 0) continue;
                 const uint32_t tx = (uint32_t)it.nh * (A_BYTES + SF_BYTES) + B_BYTES + SF_BYTES;
                 for (int ks = 0; ks < p.k_stages; ks++) {
-                    ok = mbar_wait(bar_empty + 8 * stage, phase, abort_flag, ST_TIMEOUT_PRODUCER);
+                    if (!mbar_wait_warp(bar_empty + 8 * stage, phase, abort_flag, ST_TIMEOUT_PRODUCER)) { ok = false; break; }
                     const uint32_t fb = bar_full + 8 * stage;
                     const uint32_t sa = smem_base + stage * STAGE_BYTES;
-                    if (leader && ok) {
+                    if (leader) {
                         mbar_arrive_expect_tx(fb, tx);
                         for (int h = 0; h < it.nh; h++) {
                             tma_load_2d(sa + h * A_BYTES, &tmap_a, fb, ks * BK, (it.rt + h) * BM);   // rows past M: zero-filled
@@ -151,8 +151,7 @@ fp8_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                         tma_load_2d(sa + OFF_B, &tmap_b, fb, ks * BK, it.tn * BN);
                         bulk_load(sa + OFF_SF + 2 * SF_BYTES, p.sfb + ((size_t)it.tn * p.k_stages + ks) * SF_BYTES, SF_BYTES, fb);
                     }
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
+                    __syncwarp();
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
             }
@@ -169,7 +168,7 @@ fp8_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                 const Item it = decode_item(p, idx);
                 if (it.nh == 0) continue;
                 for (int ks = 0; ks < p.k_stages && ok; ks++) {
-                    ok = mbar_wait(bar_full + 8 * stage, phase, abort_flag, ST_TIMEOUT_MMA);
+                    if (!mbar_wait_warp(bar_full + 8 * stage, phase, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t sa = smem_base + stage * STAGE_BYTES;
                     const uint32_t sf_tmem = tmem_base + SF_COL + 16 * stage;
@@ -177,24 +176,24 @@ fp8_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                     // below run in issue order, so a stage's scales are in place before its MMAs and are not overwritten
                     // before the MMAs of the ring's previous lap have read them
                     for (int h = 0; h < it.nh; h++)
-                        if (leader && ok) tmem_cp_32x128b_warpx4(sf_tmem + 4 * h, make_smem_desc(sa + OFF_SF + h * SF_BYTES, 128, 128, LAYOUT_NONE));
-                    if (leader && ok) tmem_cp_32x128b_warpx4(sf_tmem + 8, make_smem_desc(sa + OFF_SF + 2 * SF_BYTES, 128, 128, LAYOUT_NONE));
+                        if (leader) tmem_cp_32x128b_warpx4(sf_tmem + 4 * h, make_smem_desc(sa + OFF_SF + h * SF_BYTES, 128, 128, LAYOUT_NONE));
+                    if (leader) tmem_cp_32x128b_warpx4(sf_tmem + 8, make_smem_desc(sa + OFF_SF + 2 * SF_BYTES, 128, 128, LAYOUT_NONE));
                     const uint64_t bdesc = kmajor_desc_sw128(sa + OFF_B);
                     for (int h = 0; h < it.nh; h++) {
                         const uint32_t c = cnt + h, slot = c % ACC_SLOTS;
                         if (ks == 0) {   // the slot's previous contents must have been read out
-                            ok = ok && mbar_wait(bar_tempty + 8 * slot, ((c / ACC_SLOTS) & 1) ^ 1, abort_flag, ST_TIMEOUT_MMA);
+                            if (!mbar_wait_warp(bar_tempty + 8 * slot, ((c / ACC_SLOTS) & 1) ^ 1, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
                             tc_fence_after();
                         }
                         const uint32_t d_tmem = tmem_base + slot * BN;
                         const uint64_t adesc = kmajor_desc_sw128(sa + h * A_BYTES);
 #pragma unroll
                         for (int k = 0; k < BK / 32; k++)   // +32 bytes along K inside the swizzle span = +2 in the address field
-                            if (leader && ok) mma_mx(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc_mx(k), sf_tmem + 4 * h, sf_tmem + 8, (ks | k) != 0);
+                            if (leader) mma_mx(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc_mx(k), sf_tmem + 4 * h, sf_tmem + 8, (ks | k) != 0);
                     }
-                    if (leader && ok) mma_commit(bar_empty + 8 * stage);  // stage reusable once these MMAs retire
-                    ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
+                    if (leader) mma_commit(bar_empty + 8 * stage);  // stage reusable once these MMAs retire
+                    __syncwarp();
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
                 if (ok)

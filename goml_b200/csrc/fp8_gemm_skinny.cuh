@@ -121,14 +121,14 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         int stage = 0;
         uint32_t phase = 1;
         for (int kb = kb0; kb < kb1; kb++) {
-            const bool ok = mbar_wait(bar_empty + 8 * stage, phase, abort_flag, ST_TIMEOUT_PRODUCER);
-            if (leader && ok) {
+            if (!mbar_wait_warp(bar_empty + 8 * stage, phase, abort_flag, ST_TIMEOUT_PRODUCER)) break;
+            if (leader) {
                 const uint32_t fb = bar_full + 8 * stage, sw = ring + stage * stage_bytes;
                 mbar_arrive_expect_tx(fb, stage_bytes);   // parts of a box outside the matrix are zero-filled and counted
                 tma_load_2d(sw, &tmap_w, fb, kb * BK, n0);
                 tma_load_2d(sw + W_BYTES, &tmap_t, fb, kb * BK, 0);
             }
-            if (!__all_sync(0xffffffffu, ok)) break;
+            __syncwarp();
             if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
     } else if (warp == 1) {
@@ -137,16 +137,15 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         uint32_t phase = 0;
         bool ok = true;
         for (int kb = kb0; kb < kb1; kb++) {
-            ok = mbar_wait(bar_full + 8 * stage, phase, abort_flag, ST_TIMEOUT_MMA);
+            if (!mbar_wait_warp(bar_full + 8 * stage, phase, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
             tc_fence_after();
             const uint32_t sw = ring + stage * stage_bytes;
             const uint64_t wdesc = kmajor_desc_sw128(sw), tdesc = kmajor_desc_sw128(sw + W_BYTES);
 #pragma unroll
             for (int k = 0; k < BK / 32; k++)
-                if (leader && ok) mma_f8f6f4_ss(tmem, wdesc + 2 * k, tdesc + 2 * k, p.idesc, ((kb - kb0) | k) != 0);
-            if (leader && ok) mma_commit(bar_empty + 8 * stage);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
+                if (leader) mma_f8f6f4_ss(tmem, wdesc + 2 * k, tdesc + 2 * k, p.idesc, ((kb - kb0) | k) != 0);
+            if (leader) mma_commit(bar_empty + 8 * stage);
+            __syncwarp();
             if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
         if (ok && leader) mma_commit(bar_done);

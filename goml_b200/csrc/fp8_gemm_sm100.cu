@@ -215,9 +215,9 @@ fp8_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                 unit_coords<BN>(t, p, tm, n0, bn);
                 const CUtensorMap* tb = (bn == BN) ? &tmap_b : &tmap_b_half;
                 for (int ks = ks0; ks < ks1; ks++) {
-                    ok = mbar_wait(bar_empty + 8 * stage, phase, abort_flag, ST_TIMEOUT_PRODUCER);
+                    if (!mbar_wait_warp(bar_empty + 8 * stage, phase, abort_flag, ST_TIMEOUT_PRODUCER)) { ok = false; break; }
                     const uint32_t fb = bar_full + 8 * stage;
-                    if (leader && ok) {
+                    if (leader) {
                         mbar_arrive_expect_tx(fb, KSUB * (MT * p.a_rows * BK + bn * BK));
 #pragma unroll
                         for (int sub = 0; sub < KSUB; sub++) {
@@ -229,8 +229,7 @@ fp8_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                             tma_load_2d(sa + MT * A_BYTES, tb, fb, kb * BK, n0);
                         }
                     }
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
+                    __syncwarp();
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
             }
@@ -255,7 +254,7 @@ fp8_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * BN;
                 for (int ks = ks0; ks < ks1; ks++) {
-                    ok = mbar_wait(bar_full + 8 * stage, phase, abort_flag, ST_TIMEOUT_MMA);
+                    if (!mbar_wait_warp(bar_full + 8 * stage, phase, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
                     tc_fence_after();
 #pragma unroll
                     for (int sub = 0; sub < KSUB; sub++) {
@@ -265,26 +264,26 @@ fp8_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
 #pragma unroll
                         for (int k = 0; k < BK / 32; k++) {
                             // +32 bytes along K inside the swizzle span = +2 in the address field
-                            if (leader && ok) mma_f8f6f4_ss(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, ((ks - ks0) | sub | k) != 0);
+                            if (leader) mma_f8f6f4_ss(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, ((ks - ks0) | sub | k) != 0);
                         }
                         if (MT == 2) {
                             // lower half of the pair: the other accumulator buffer, the same B operand.  Its buffer is
                             // waited for only here, so the epilogue of the previous pair's lower half overlaps the
                             // first MMAs of this pair's upper half.
                             if (ks == ks0 && sub == 0) {
-                                ok = ok && mbar_wait(bar_tempty + 8, tphase[1], abort_flag, ST_TIMEOUT_MMA);
+                                if (!mbar_wait_warp(bar_tempty + 8, tphase[1], abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
                                 tphase[1] ^= 1;
                                 tc_fence_after();
                             }
                             const uint64_t adesc2 = kmajor_desc_sw128(sa + A_BYTES);
 #pragma unroll
                             for (int k = 0; k < BK / 32; k++)
-                                if (leader && ok) mma_f8f6f4_ss(tmem_base + BN, adesc2 + 2 * k, bdesc + 2 * k, idesc, ((ks - ks0) | sub | k) != 0);
+                                if (leader) mma_f8f6f4_ss(tmem_base + BN, adesc2 + 2 * k, bdesc + 2 * k, idesc, ((ks - ks0) | sub | k) != 0);
                         }
                     }
-                    if (leader && ok) mma_commit(bar_empty + 8 * stage);  // stage reusable once these MMAs retire
-                    ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
+                    if (leader) mma_commit(bar_empty + 8 * stage);  // stage reusable once these MMAs retire
+                    __syncwarp();
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
                 if (ok && leader) mma_commit(bar_tfull + 8 * buf);  // accumulator complete

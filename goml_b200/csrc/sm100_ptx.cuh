@@ -86,13 +86,23 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
-// Every role of these kernels runs on whole warps, and a lane may run out of time, or see the abort word, where its neighbour
-// still sees the phase complete.  Leaving the role's loop without it, it would wait in the CTA's teardown barrier while the
-// others wait for it in the loop's next warp-wide operation.  So the lanes vote on the outcome before any of them leaves: here,
-// or, in the loops that feed the tensor core and the copy engine, at the end of the step, in the place of a __syncwarp() and
-// behind the elected lane's issue (a vote between the wait and the issue costs the GEMMs and the attention 0.3 to 1 %).
+// The wait of a role that runs on a whole warp, which is every role of these kernels: each poll is voted on, so the lanes leave
+// it together and with one outcome.  With an outcome of its own a lane may run out of time, or see the abort word, where its
+// neighbour still sees the phase complete; leaving the role's loop without it, it would wait in the CTA's teardown barrier
+// while the others wait for it in the loop's next warp-wide operation.  (The vote is here and not behind the issue of the step:
+// `leader && ok` in front of the MMAs costs a 256 x 4096 x 4096 product 7 %, this nothing.)
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t code) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, code));
+    uint64_t t0 = 0;
+    for (uint32_t polls = 1; !__all_sync(0xffffffffu, mbar_try_wait(bar, parity)); polls++) {
+        if ((polls & 2047u) == 0) {
+            const uint64_t now = globaltimer_ns();
+            if (t0 == 0) t0 = now;
+            const bool late = now - t0 > SM100_WAIT_BUDGET_NS;
+            if (late) atomicCAS((uint32_t*)abort_flag, 0u, code);
+            if (__any_sync(0xffffffffu, late || *abort_flag != 0)) return false;
+        }
+    }
+    return true;
 }
 
 // Self-test of the bounded wait, shared by the libraries: one warp waits, with a 1 ms budget, on a barrier that

@@ -54,19 +54,15 @@ def test_the_lane_that_copies_v_is_ordered_behind_the_lane_that_saw_the_flag():
 @pytest.mark.parametrize("name", [n for n, t in sources().items() if "mbar_wait" in t and n != "sm100_ptx.cuh"])
 def test_bounded_waits_are_left_by_whole_warps(name):
     # roles run on whole warps: a lane that leaves a loop on its own outcome of a wait strands the others in the loop's next
-    # warp-wide operation.  So an outcome is either voted on inside the wait or kept in `ok`, and `ok` is voted on before
-    # any lane breaks or returns
-    text = sources()[name]
-    waits = [m.start() for m in re.finditer(r"\bmbar_wait\s*\(", text)]
-    assert len(waits) == sum(o.count("mbar_wait(") for o in re.findall(r"\bok = [^;]*;", text))
-    for at in waits:
-        leaves = re.search(r"\b(break|return|goto|continue)\b", text[at:])
-        assert "__all_sync(" in text[at:at + leaves.start()], text[at:at + leaves.start()]
+    # warp-wide operation
+    assert not re.search(r"\bmbar_(try_)?wait\s*[(<]", sources()[name])
 
 
 def test_the_warp_wait_votes():
     body = dict(functions(sources()["sm100_ptx.cuh"]))["mbar_wait_warp"]
-    assert re.search(r"__all_sync\(0xffffffffu,\s*mbar_wait\(", body)
+    assert re.search(r"__all_sync\(0xffffffffu,\s*mbar_try_wait\(", body) and "mbar_wait(" not in body
+    # the only other way out is voted on as well
+    assert body.count("return") == 2 and re.search(r"if \(__any_sync\([^;]*\) return false;", body)
 
 
 def test_calls_on_different_streams_do_not_hold_one_lock_over_their_launches():
