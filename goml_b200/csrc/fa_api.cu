@@ -177,7 +177,7 @@ fa_status_t validate(fa_ctx_t* c, const char* who, const void* q, const void* k,
 // One call's scratch: the stream's kept buffers where they serve, else blocks drawn from the pool for this call.
 struct Scratch {
     void* ptr = nullptr;
-    uint32_t* flags = nullptr;   // nullptr: none kept for this stream (a capture, more streams than slots) and none needed
+    uint32_t* flags = nullptr;   // nullptr: none kept for this stream (a capture, more streams than slots)
     uint32_t epoch = 0;
     uint32_t* zeros = nullptr;
     void* pooled[2] = {nullptr, nullptr};
@@ -209,13 +209,12 @@ struct Scratch {
         return cudaSuccess;
     }
 
-    // need_flags: the call cannot do without flags (else they are given where the stream's kept ones serve)
-    cudaError_t take(fa_ctx_t* c, cudaStream_t s, size_t bytes, size_t flag_words, bool need_flags, size_t zero_words) {
-        const cudaError_t e = take_from(c, s, bytes, flag_words, need_flags, zero_words);
+    cudaError_t take(fa_ctx_t* c, cudaStream_t s, size_t bytes, size_t flag_words, size_t zero_words) {
+        const cudaError_t e = take_from(c, s, bytes, flag_words, zero_words);
         if (e != cudaSuccess) give_back();
         return e;
     }
-    cudaError_t take_from(fa_ctx_t* c, cudaStream_t s, size_t bytes, size_t flag_words, bool need_flags, size_t zero_words) {
+    cudaError_t take_from(fa_ctx_t* c, cudaStream_t s, size_t bytes, size_t flag_words, size_t zero_words) {
         stream = s;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         cudaError_t e = cudaStreamIsCapturing(s, &cap);
@@ -253,16 +252,10 @@ struct Scratch {
             if ((e = cudaMallocFromPoolAsync(&pooled[0], bytes, c->shared->pool, s)) != cudaSuccess) return e;
             ptr = pooled[0];
         }
-        const size_t more_zeros = zeros ? 0 : zero_words, more_flags = flags || !need_flags ? 0 : flag_words;
-        if (more_zeros + more_flags) {
-            const size_t n = (more_zeros + more_flags) * 4;
-            if ((e = cudaMallocFromPoolAsync(&pooled[1], n, c->shared->pool, s)) != cudaSuccess) return e;
-            if ((e = fa_sm100::launch_clear_words(static_cast<uint32_t*>(pooled[1]), more_zeros + more_flags, s)) != cudaSuccess) return e;
-            if (more_zeros) zeros = static_cast<uint32_t*>(pooled[1]);
-            if (more_flags) {
-                flags = static_cast<uint32_t*>(pooled[1]) + more_zeros;
-                epoch = 1;
-            }
+        if (zero_words && !zeros) {
+            if ((e = cudaMallocFromPoolAsync(&pooled[1], zero_words * 4, c->shared->pool, s)) != cudaSuccess) return e;
+            if ((e = fa_sm100::launch_clear_words(static_cast<uint32_t*>(pooled[1]), zero_words, s)) != cudaSuccess) return e;
+            zeros = static_cast<uint32_t*>(pooled[1]);
         }
         return cudaSuccess;
     }
@@ -290,7 +283,7 @@ fa_status_t run(fa_ctx_t* c, const char* who, const fa_sm100::LaunchArgs& a) {
     }
     fa_sm100::LaunchArgs b = a;
     Scratch ws;
-    e = ws.take(c, a.stream, fa_sm100::workspace_bytes(a.bh, a.sl, a.hd), fa_sm100::v_flag_count(a.bh, a.sl), false, 0);
+    e = ws.take(c, a.stream, fa_sm100::workspace_bytes(a.bh, a.sl, a.hd), fa_sm100::v_flag_count(a.bh, a.sl), 0);
     if (e != cudaSuccess) {
         set_err(c, "%s: workspace allocation: %s", who, cudaGetErrorString(e));
         return e == cudaErrorMemoryAllocation ? FA_ERR_OOM : FA_ERR_CUDA;
@@ -447,14 +440,11 @@ fa_status_t fa_decode(fa_ctx_t* ctx, const fa_decode_args_t* g) {
     a.stream = reinterpret_cast<cudaStream_t>(g->stream);
     Scratch ws;
     const int span = fa_sm100::decode_span(a);
-    e = ws.take(ctx, a.stream, fa_sm100::decode_workspace_bytes(a.batch, a.q_heads, a.kv_heads, a.hd, span),
-                fa_sm100::decode_flag_count(a.batch, a.q_heads, a.kv_heads, span), true,
-                fa_sm100::decode_arrival_count(a.batch, a.q_heads, a.kv_heads, span));
+    e = ws.take(ctx, a.stream, fa_sm100::decode_workspace_bytes(a.batch, a.q_heads, a.kv_heads, a.hd, span), 0,
+                fa_sm100::decode_arrival_count(a.batch, a.q_heads, a.kv_heads, a.hd, span));
     if (e != cudaSuccess) { set_err(ctx, "%s: workspace allocation: %s", who, cudaGetErrorString(e)); return e == cudaErrorMemoryAllocation ? FA_ERR_OOM : FA_ERR_CUDA; }
     a.workspace = ws.ptr;
     a.arrivals = ws.zeros;
-    a.flags = ws.flags;
-    a.epoch = ws.epoch;
     e = fa_sm100::launch_decode(a);
     const cudaError_t fe = ws.give_back();  // stream-ordered: released after the kernels
     if (e != cudaSuccess) { set_err(ctx, "%s: launch: %s", who, cudaGetErrorString(e)); return FA_ERR_CUDA; }

@@ -23,15 +23,14 @@
 //
 // How the keys are divided (Plan below): a pair (sequence, kv head) may be cut between chunks; the pieces leave partial
 // states in a workspace and the CTA that finishes last merges them in a fixed order, so there is no second kernel and results
-// do not depend on timing: the same call gives the same bits, eager or in a graph, on whatever stream.  (One exception is
-// reported: a hand-over of maxima that does not come within the wait's budget, see LINE_HANDED.)
+// do not depend on timing: the same call gives the same bits, eager or in a graph, on whatever stream.
 //
 // STREAMS: the rounding of P to fp16 depends on the running maximum it is taken against, so which keys share a warp and
 // where a pair is cut show in the last bits of O.  A block that re-quantises its activations turns last bits into e4m3
 // steps further on.  For one query head per kv head (what the decoder block runs) warp w therefore always takes keys
-// 16w .. 16w + 15 of every 64-key chunk, and the plans keep each such stream's maximum what an uncut walk over the pair
-// (or over a fixed split of it) gives.  Grouped heads are free of that: the maximum may lag by 2^LAG, a warp takes 32
-// (D = 64: 64) contiguous keys, pairs are cut anywhere.
+// 16w .. 16w + 15 of every 64-key chunk, and each such stream's maximum is what a walk over the pair (or over a fixed split of
+// it) gives.  Grouped heads are free of that: the maximum may lag by 2^LAG, a warp takes 32 (D = 64: 64) contiguous keys,
+// pairs are cut anywhere.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -39,7 +38,6 @@
 
 #include "fa_fwd_sm100.h"
 #include "pdl.cuh"
-#include "sm100_ptx.cuh"
 
 namespace fa_sm100 {
 
@@ -96,17 +94,10 @@ __device__ __forceinline__ void ldg64(uint32_t* r, const uint8_t* p) {
 
 // Plans.
 //  SPLITS: CTA i is split i % splits of pair i / splits; a split is chunks_per_split chunks.  Few pairs: one resident CTA
-//          per split.
+//          per split.  Many: one CTA per pair.
 //  LINE:   the chunks of all pairs form one line that is cut into equal pieces, one per resident CTA, so sequences of very
 //          different lengths load all SMs alike.
-//  LINE_HANDED: the same with pieces at least as long as the longest pair, so that a pair is cut at most once.  A CTA
-//          takes the pair that its piece ends in first, publishes the running maxima it ended with, and takes the pair its
-//          piece begins in last, starting from the maxima of the CTA before it.  Those were published about a piece ago by a
-//          CTA that started earlier and waits for nobody before it publishes.  The wait for them is bounded all the same: when
-//          its budget runs out the status word is set and the pair starts from scratch, which changes only roundings.
-enum Plan : int { SPLITS, LINE, LINE_HANDED };
-constexpr uint32_t ST_TIMEOUT_HANDED = 0x204;   // beside the codes of the forward kernel
-__device__ uint32_t g_decode_status = 0;
+enum Plan : int { SPLITS, LINE };
 
 struct DecodeParams {
     const uint8_t* q;
@@ -129,10 +120,7 @@ struct DecodeParams {
     // partial states, two slots per CTA: [slot][rows][D] un-normalised outputs, then [slot][rows][2] (m in log2 units, l)
     float* ws_o;
     float* ws_ml;
-    float* ws_handed;     // [CTA][WARPS][rows] running maxima
     uint32_t* arrivals;   // [B*Hkv], zero before and after every launch
-    uint32_t* handed;     // [CTA], set to epoch when the CTA's maxima are published
-    uint32_t epoch;
 };
 
 template <int D, int NQ, bool WIDE>
@@ -209,7 +197,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
     constexpr int LENS = 4;
     int lens[LENS];
 #pragma unroll
-    for (int i = 0; i < LENS; i++) lens[i] = p.plan != SPLITS && 32 * i + lane < p.batch ? seq_len_of(p, 32 * i + lane) : 0;
+    for (int i = 0; i < LENS; i++) lens[i] = !STREAMS && p.plan == LINE && 32 * i + lane < p.batch ? seq_len_of(p, 32 * i + lane) : 0;
     auto lane_len = [&](int b0) -> int {   // length of sequence b0 + lane, b0 a multiple of 32
         if (b0 < 32 * LENS) {
             int x = lens[0];
@@ -253,10 +241,10 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
     };
 
     Segment seg;
-    int u_begin = 0, u_end = 0, cut_q = 0, cut_r = 0;
+    int cut_q = 0, cut_r = 0;
     int mid = 0, mid_end = 0;    // units of the segments still to come in line order
-    bool head_last = false;      // the cut pair this piece begins in is still to come, behind them
-    if (p.plan == SPLITS) {
+    const bool line = !STREAMS && p.plan == LINE;   // streams are not cut along a line: that code is not compiled for them
+    if (!line) {
         const int pair = blockIdx.x / p.splits, split = blockIdx.x - pair * p.splits;
         seg.b = pair / p.hkv;
         seg.kvh = pair - seg.b * p.hkv;
@@ -268,39 +256,22 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
         if (seg.n_chunks == 0 && seg.kvh == 0 && split == 0 && threadIdx.x == 0) empty_sequence(seg.b);
         if (seg.c_begin >= seg.c_end) return;
     } else {
-        int total = 0, longest = 1;
+        int total = 0;
         for (int b0 = 0; b0 < p.batch; b0 += 32) {
             const int b = b0 + lane, n = chunks_of(lane_len(b0));
             if (n == 0 && b < p.batch && warp == 0 && b % gridDim.x == blockIdx.x) empty_sequence(b);
             total += __reduce_add_sync(0xffffffffu, n);
-            longest = max(longest, __reduce_max_sync(0xffffffffu, n));
         }
         total *= p.hkv;
-        int pieces = gridDim.x;
-        if (p.plan == LINE_HANDED) pieces = max(1, min(pieces, total / longest));
-        if ((int)blockIdx.x >= pieces) return;
+        const int pieces = gridDim.x;
         cut_q = total / pieces;
         cut_r = total - cut_q * pieces;
         const Cut cut(cut_q, cut_r);
-        u_begin = cut.begin(blockIdx.x);
-        u_end = cut.begin(blockIdx.x + 1);
-        if (u_begin >= u_end) return;
-        mid = u_begin;
-        mid_end = u_end;
-        if (p.plan == LINE_HANDED) {
-            const Segment head = segment_at(u_begin, u_end), tail = segment_at(u_end - 1, u_end);
-            if (head.c_begin > 0) {
-                head_last = true;
-                mid = min(u_end, head.pair_u0 + head.n_chunks);
-            }
-            if (tail.c_end < tail.n_chunks && tail.pair_u0 >= u_begin) mid_end = tail.pair_u0;
-            if (mid_end < u_end) seg = segment_at(mid_end, u_end);
-            else if (mid < mid_end) { seg = segment_at(mid, mid_end); mid += seg.c_end - seg.c_begin; }
-            else { seg = head; head_last = false; }
-        } else {
-            seg = segment_at(mid, mid_end);
-            mid += seg.c_end - seg.c_begin;
-        }
+        mid = cut.begin(blockIdx.x);
+        mid_end = cut.begin(blockIdx.x + 1);
+        if (mid >= mid_end) return;
+        seg = segment_at(mid, mid_end);
+        mid += seg.c_end - seg.c_begin;
     }
     const Cut cut(cut_q, cut_r);
 
@@ -390,18 +361,14 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
         for (int j = 0; j < OFFS; j++) page_next[j] = entry(seg, seg.c_begin + C::TILES + chunk_at(j));
 
         // the segment behind this one waits in shared memory (a copy per warp: no barrier)
-        bool more = true;
+        bool more;
         int next_entry[OFFS];
         {
             Segment next;
-            if (mid < mid_end) {
+            more = line && mid < mid_end;
+            if (more) {
                 next = segment_at(mid, mid_end);
                 mid += next.c_end - next.c_begin;
-            } else if (head_last) {
-                next = segment_at(u_begin, u_end);
-                head_last = false;
-            } else {
-                more = false;
             }
             if (more) {
 #pragma unroll
@@ -432,28 +399,6 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
             for (int e = 0; e < 2; e++) { m[n][e] = -INFINITY; l[n][e] = 0.f; }
 #pragma unroll
             for (int i = 0; i < C::MT; i++) acc[n][i][0] = acc[n][i][1] = acc[n][i][2] = acc[n][i][3] = 0.f;
-        }
-        if (STREAMS && p.plan == LINE_HANDED && seg.c_begin > 0) {
-            uint32_t f;
-            uint64_t t0 = 0;
-            for (uint32_t polls = 1;; polls++) {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(f) : "l"(p.handed + blockIdx.x - 1) : "memory");
-                if (f == p.epoch) break;
-                if ((polls & 255u) == 0) {
-                    const uint64_t now = globaltimer_ns();
-                    if (t0 == 0) t0 = now;
-                    else if (now - t0 > SM100_WAIT_BUDGET_NS) break;
-                }
-            }
-            if (!__all_sync(0xffffffffu, f == p.epoch)) {
-                if (lane == 0) atomicCAS(&g_decode_status, 0u, ST_TIMEOUT_HANDED);
-            } else {
-#pragma unroll
-                for (int n = 0; n < NQ; n++)
-#pragma unroll
-                    for (int e = 0; e < 2; e++)
-                        m[n][e] = __ldcg(p.ws_handed + ((size_t)(blockIdx.x - 1) * WARPS + warp) * C::ROWS + 8 * n + 2 * t + e);
-            }
         }
 
         for (int c = seg.c_begin; c < seg.c_end; c += C::TILES) {
@@ -578,7 +523,6 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
 
         // ---- merge the four warps' states
         const bool whole = seg.c_begin == 0 && seg.c_end == seg.n_chunks;
-        const bool hand_on = STREAMS && p.plan == LINE_HANDED && seg.c_end < seg.n_chunks;
 #pragma unroll
         for (int n = 0; n < NQ; n++)
 #pragma unroll
@@ -589,7 +533,6 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
                 if (g == 0) {
                     s_m[warp][row] = m[n][e];
                     s_l[warp][row] = l[n][e];
-                    if (hand_on) __stcg(p.ws_handed + ((size_t)blockIdx.x * WARPS + warp) * C::ROWS + row, m[n][e]);
                 }
                 if (row < p.group) {
 #pragma unroll
@@ -597,13 +540,10 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
                         *reinterpret_cast<float2*>(&s_o[warp][row][(D / 8) * g + 2 * j]) = make_float2(acc[n][j][e], acc[n][j][e + 2]);
                 }
             }
-        if (hand_on) __threadfence();
         __syncthreads();
-        if (hand_on && threadIdx.x == 0)
-            asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p.handed + blockIdx.x), "r"(p.epoch) : "memory");
         // slots of a cut pair: its splits in order, or on the line the odd slot of the CTA that has its first piece and the
         // even slots of the CTAs after that
-        const int slot = p.plan == SPLITS ? blockIdx.x : 2 * blockIdx.x + (seg.c_begin == 0 ? 1 : 0);
+        const int slot = !line ? blockIdx.x : 2 * blockIdx.x + (seg.c_begin == 0 ? 1 : 0);
         const float vds = p.sv ? p.v_descale * ld_f32(p.sv) : p.v_descale;
         for (int idx = threadIdx.x; idx < p.group * (D / 4); idx += THREADS) {   // four columns per thread and step
             const int row = idx / (D / 4), col = idx % (D / 4) * 4;
@@ -627,7 +567,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
         }
         if (!whole) {
             int parts, slot0, slot_step;   // the pair's pieces: slot0, then slot0 + 1 + i * slot_step
-            if (p.plan == SPLITS) {
+            if (!line) {
                 parts = (seg.n_chunks + p.chunks_per_split - 1) / p.chunks_per_split;
                 slot0 = (blockIdx.x / p.splits) * p.splits;
                 slot_step = 1;
@@ -707,37 +647,47 @@ __global__ void clear_words_kernel(uint32_t* w, uint32_t n) {
 
 struct Layout {
     int plan, splits, grid, rows;
-    bool streams;
+    bool streams, wide;
     bool cuts() const { return plan != SPLITS || splits > 1; }   // whether a pair may be cut
 };
-// One query head per kv head keeps the streams: fixed splits while the pairs leave room for them, else the line with
-// hand-over.  Groups take the freely cut line, which balances best (24 sequences of 3000 to 6000 keys, 8 kv heads: 45 us
-// against 70 with fixed splits and a merging kernel).
-Layout layout_of(int batch, int q_heads, int kv_heads, int span) {
+// One query head per kv head keeps the streams: fixed splits while the pairs leave room for them, else a CTA per pair, which
+// the hardware hands out as CTAs end, so uneven lengths balance by themselves.  (The freely cut line, with a CTA taking up the
+// running maxima of the one before it, was 10 to 30 % faster where all sequences are equally long and the pairs fill the
+// SMs badly, and up to twice as slow for short or very uneven ones: 24 sequences of 32 heads of 128, lengths random up to
+// 2048, 100 us against 56, 64 of up to 4160 255 against 205.)
+//
+// Wide steps pay once there is something to stream (from 2048 keys on; 300 keys of 64 x 32 pairs 51 us against 47), for head
+// dim 128 (64 takes 256 keys a step: up to 1.4 times as slow on short sequences in a long cache), and unless the fewer
+// CTAs they leave resident need more rounds than that (keys of equal length, 4160 of them: 80 x 16 pairs, 3 rounds of 444
+// against 3 of 592, 221 us against 262; 30 x 32 pairs, 3 rounds against 2, 202 against 186).
+//
+// Groups take the freely cut line, which balances best (24 sequences of 3000 to 6000 keys, 8 kv heads: 45 us against 70 with
+// fixed splits and a merging kernel), unless it has more chunks than an int counts (a paged cache whose capacity is far above
+// what it holds).
+Layout layout_of(int batch, int q_heads, int kv_heads, int head_dim, int span) {
     Layout x;
-    const int group = q_heads / kv_heads;
+    const int group = q_heads / kv_heads, sms = num_sms_of_current_device();
     x.rows = group <= 8 ? 8 : 16;
     x.streams = group == 1;
     const long long pairs = (long long)batch * kv_heads, chunks = ((long long)span + CHUNK - 1) / CHUNK;
-    const long long narrow = (long long)ctas_per_sm(1, false) * num_sms_of_current_device();
-    long long splits = narrow / pairs;
-    if (splits > chunks) splits = chunks;
-    if (splits > 64) splits = 64;
-    if (splits < 1) splits = 1;
-    x.splits = (int)splits;
-    if (x.streams && pairs * splits <= narrow) {
+    const long long narrow = (long long)ctas_per_sm(1, false) * sms, wide = (long long)ctas_per_sm(x.rows / 8, true) * sms;
+    x.splits = 1;
+    x.wide = !x.streams;
+    if (x.streams && pairs <= narrow) {
+        long long splits = narrow / pairs;
+        if (splits > chunks) splits = chunks;
+        if (splits > 64) splits = 64;
+        x.splits = splits < 1 ? 1 : (int)splits;
         x.plan = SPLITS;
-        x.grid = (int)(pairs * splits);
-    } else if (pairs * chunks > 0x7fffffffLL) {
-        // a line of more chunks than an int counts (a paged cache whose capacity is far above what it holds): a CTA per pair
+        x.grid = (int)(pairs * x.splits);
+    } else if (x.streams || pairs * chunks > 0x7fffffffLL) {
         x.plan = SPLITS;
-        x.splits = 1;
         x.grid = (int)pairs;
+        if (x.streams) x.wide = head_dim == 128 && chunks >= 32 && (pairs + wide - 1) / wide * wide <= (pairs + narrow - 1) / narrow * narrow;
     } else {
-        x.plan = x.streams ? LINE_HANDED : LINE;
-        const long long slots = (long long)ctas_per_sm(x.rows / 8, true) * num_sms_of_current_device();
+        x.plan = LINE;
         const long long units = pairs * chunks;
-        x.grid = (int)(units < slots ? (units > 0 ? units : 1) : slots);
+        x.grid = (int)(units < wide ? (units > 0 ? units : 1) : wide);
     }
     return x;
 }
@@ -745,24 +695,18 @@ Layout layout_of(int batch, int q_heads, int kv_heads, int span) {
 }  // namespace
 
 size_t decode_workspace_bytes(int batch, int q_heads, int kv_heads, int head_dim, int span) {
-    const Layout x = layout_of(batch, q_heads, kv_heads, span);
-    if (!x.cuts()) return 0;
-    return (size_t)x.grid * x.rows * (2 * (head_dim + 2) + WARPS) * sizeof(float);
+    const Layout x = layout_of(batch, q_heads, kv_heads, head_dim, span);
+    return x.cuts() ? (size_t)x.grid * x.rows * 2 * (head_dim + 2) * sizeof(float) : 0;
 }
-size_t decode_arrival_count(int batch, int q_heads, int kv_heads, int span) {
-    return layout_of(batch, q_heads, kv_heads, span).cuts() ? (size_t)batch * kv_heads : 0;
-}
-size_t decode_flag_count(int batch, int q_heads, int kv_heads, int span) {
-    const Layout x = layout_of(batch, q_heads, kv_heads, span);
-    return x.plan == LINE_HANDED ? (size_t)x.grid : 0;
+size_t decode_arrival_count(int batch, int q_heads, int kv_heads, int head_dim, int span) {
+    return layout_of(batch, q_heads, kv_heads, head_dim, span).cuts() ? (size_t)batch * kv_heads : 0;
 }
 
 cudaError_t launch_decode(const DecodeArgs& a) {
     const int span = decode_span(a);
     if ((long long)a.batch * a.kv_heads > 0x7fffffffLL) return cudaErrorInvalidValue;
-    const Layout x = layout_of(a.batch, a.q_heads, a.kv_heads, span);
+    const Layout x = layout_of(a.batch, a.q_heads, a.kv_heads, a.hd, span);
     if (x.cuts() && (!a.workspace || !a.arrivals)) return cudaErrorInvalidValue;
-    if (x.plan == LINE_HANDED && !a.flags) return cudaErrorInvalidValue;
     DecodeParams p;
     p.q = static_cast<const uint8_t*>(a.q);
     p.k = static_cast<const uint8_t*>(a.k_cache);
@@ -788,17 +732,12 @@ cudaError_t launch_decode(const DecodeArgs& a) {
     p.page_size = a.page_size; p.max_pages = a.max_pages; p.num_pages = a.num_pages;
     p.ws_o = static_cast<float*>(a.workspace);
     p.ws_ml = p.ws_o + (size_t)x.grid * 2 * x.rows * a.hd;
-    p.ws_handed = p.ws_ml + (size_t)x.grid * 2 * x.rows * 2;
     p.arrivals = a.arrivals;
-    p.handed = a.flags; p.epoch = a.epoch;
     auto run = [&](auto contiguous, auto paged) { return launch_pdl(a.block_table ? paged : contiguous, x.grid, THREADS, 0, a.stream, p); };
 #define KERNEL(D, NQ, WIDE, STREAMS) run(fa_decode_kernel<D, NQ, WIDE, STREAMS, false>, fa_decode_kernel<D, NQ, WIDE, STREAMS, true>)
-#define KERNELS(D)                                             \
-    (x.streams && x.plan == SPLITS ? KERNEL(D, 1, false, true) \
-     : x.streams                   ? KERNEL(D, 1, true, true)  \
-     : x.rows == 8                 ? KERNEL(D, 1, true, false) : KERNEL(D, 2, true, false))
-    return a.hd == 128 ? KERNELS(128) : KERNELS(64);
-#undef KERNELS
+    if (x.streams) return a.hd == 64 ? KERNEL(64, 1, false, true) : x.wide ? KERNEL(128, 1, true, true) : KERNEL(128, 1, false, true);
+    if (x.rows == 8) return a.hd == 64 ? KERNEL(64, 1, true, false) : KERNEL(128, 1, true, false);
+    return a.hd == 64 ? KERNEL(64, 2, true, false) : KERNEL(128, 2, true, false);
 #undef KERNEL
 }
 
@@ -806,13 +745,6 @@ cudaError_t launch_clear_words(uint32_t* w, size_t n, cudaStream_t stream) {
     if (n > 0xffffffffu) return cudaErrorInvalidValue;
     const unsigned blocks = (unsigned)((n + 1023) / 1024 < 64 ? (n + 1023) / 1024 : 64);
     return launch_pdl(clear_words_kernel, dim3(blocks), dim3(256), 0, stream, w, (uint32_t)n);
-}
-
-cudaError_t take_decode_status(uint32_t* code) {
-    const uint32_t zero = 0;
-    cudaError_t e = cudaMemcpyFromSymbol(code, g_decode_status, sizeof(*code));
-    if (e == cudaSuccess && *code != 0) e = cudaMemcpyToSymbol(g_decode_status, &zero, sizeof(zero));
-    return e;
 }
 
 }  // namespace fa_sm100

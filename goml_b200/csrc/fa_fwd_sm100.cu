@@ -682,9 +682,7 @@ int device_status() {
     e = cudaMemcpyFromSymbol(&code, g_fa_status, sizeof(code));
     if (e != cudaSuccess) return -(int)e;
     if (code != 0) cudaMemcpyToSymbol(g_fa_status, &zero, sizeof(zero));
-    uint32_t decode = 0;
-    if ((e = take_decode_status(&decode)) != cudaSuccess) return -(int)e;
-    return (int)(code != 0 ? code : decode);
+    return (int)code;
 }
 
 // ----------------------------------------------------------------------------------------

@@ -50,8 +50,6 @@ struct DecodeArgs {
     const float* scale_v_dev = nullptr;
     void* workspace = nullptr;      // decode_workspace_bytes(...) bytes, 16-byte aligned
     uint32_t* arrivals = nullptr;   // decode_arrival_count(...) words that are zero; the launch leaves them zero
-    uint32_t* flags = nullptr;      // decode_flag_count(...) words none of which is `epoch`
-    uint32_t epoch = 0;
     cudaStream_t stream;
     // paged cache (block_table != nullptr): k_cache, v_cache are [num_pages, kv_heads, page_size, hd], page_size a
     // multiple of 64; block_table [batch, max_pages] holds the page of each page_size-key range of a sequence and
@@ -62,13 +60,10 @@ struct DecodeArgs {
 // Longest key range any sequence can have in this call (s_max with per-sequence lengths, else seq_len).
 inline int decode_span(const DecodeArgs& a) { return a.seq_lens ? a.s_max : a.seq_len; }
 size_t decode_workspace_bytes(int batch, int q_heads, int kv_heads, int head_dim, int span);
-size_t decode_arrival_count(int batch, int q_heads, int kv_heads, int span);
-size_t decode_flag_count(int batch, int q_heads, int kv_heads, int span);
+size_t decode_arrival_count(int batch, int q_heads, int kv_heads, int head_dim, int span);
 cudaError_t launch_decode(const DecodeArgs& a);
 // Sets n words to zero; an overlapped launch like the kernel behind it.
 cudaError_t launch_clear_words(uint32_t* w, size_t n, cudaStream_t stream);
-// Status word of the decode kernels (0, or the code of a wait that ran out), which the read clears; synchronous.
-cudaError_t take_decode_status(uint32_t* code);
 
 // One warp that lets a 1 ms bounded wait run out on a barrier nothing arrives at and latches code 0x2F0.
 cudaError_t launch_wait_expiry_selftest(cudaStream_t stream);

@@ -62,10 +62,9 @@ size_t workspace_bytes(int bh, int sl, int hd) { return (size_t)bh * sl * hd * 2
 size_t v_flag_count(int bh, int) { return bh; }
 cudaError_t launch(const LaunchArgs& a) { note("launch stream " + n(a.stream) + " scratch " + n(a.v16_workspace) + " flags " + n(a.v_flags)); return cudaSuccess; }
 size_t decode_workspace_bytes(int, int, int, int, int) { return 1 << 20; }
-size_t decode_arrival_count(int batch, int, int kv_heads, int) { return (size_t)batch * kv_heads; }
-size_t decode_flag_count(int, int, int, int) { return 444; }
+size_t decode_arrival_count(int batch, int, int kv_heads, int, int) { return (size_t)batch * kv_heads; }
 cudaError_t launch_decode(const DecodeArgs& a) {
-    note("launch stream " + n(a.stream) + " scratch " + n(a.workspace) + " flags " + n(a.flags) + " zeros " + n(a.arrivals));
+    note("launch stream " + n(a.stream) + " scratch " + n(a.workspace) + " zeros " + n(a.arrivals));
     return cudaSuccess;
 }
 cudaError_t launch_clear_words(uint32_t* w, size_t, cudaStream_t s) { note("clear " + n(w) + " stream " + n(s)); return cudaSuccess; }

@@ -186,6 +186,9 @@ def test_paged_rejects_bad_page_size(cuda, built_libs, fa_ctx):
     (7, 4, 2, 1500, 128, "one long"),    # one long sequence among very short ones
     (25, 32, 32, 200, 128, "ramp"),      # one query head per kv head, more pairs than CTAs: each pair cut at most once
     (23, 30, 30, 1100, 64, "one long"),
+    (40, 32, 32, 2050, 128, "ramp"),     # a CTA per pair: wide steps, empty sequences among them, one key in the last chunk
+    (70, 16, 16, 2047, 128, "one long"),
+    (19, 32, 32, 2049, 64, "ramp"),
 ])
 def test_decode_work_split(cuda, built_libs, fa_ctx, B, Hq, Hkv, Smax, D, lens):
     # the key range is cut at chunk borders wherever the pieces of the work line end, whatever the lengths are

@@ -73,9 +73,9 @@ class Forward:
     result = Decode.result
 
 
-# every plan of the decode kernel: fixed splits (cut and uncut pairs), the line with hand-over, the freely cut line
-CALLS = {"splits": lambda: Decode(1, 8, 8, 1000, 128), "one split": lambda: Decode(12, 32, 32, 300, 64), "handed": lambda: Decode(25, 32, 32, 500, 128),
-         "handed, hd 64": lambda: Decode(23, 30, 30, 900, 64), "line": lambda: Decode(5, 32, 8, 700, 128), "wide line": lambda: Decode(3, 24, 2, 900, 64),
+# every plan of the decode kernel: fixed splits (cut and uncut pairs), a CTA per pair, the freely cut line
+CALLS = {"splits": lambda: Decode(1, 8, 8, 1000, 128), "one split": lambda: Decode(12, 32, 32, 300, 64), "a CTA a pair": lambda: Decode(25, 32, 32, 500, 128),
+         "a CTA a pair, hd 64": lambda: Decode(23, 30, 30, 900, 64), "line": lambda: Decode(5, 32, 8, 700, 128), "wide line": lambda: Decode(3, 24, 2, 900, 64),
          "forward": lambda: Forward(8, 700, 128), "forward, hd 64": lambda: Forward(3, 300, 64, 0)}
 
 
@@ -107,7 +107,7 @@ def test_twenty_streams_give_the_same_bits(cuda, built_libs, fa_ctx, name):
         assert torch.equal(call.result(fa_ctx, stream), want)
 
 
-@pytest.mark.parametrize("name", ["handed", "line", "forward"])
+@pytest.mark.parametrize("name", ["a CTA a pair", "line", "forward"])
 def test_streams_that_come_and_go(cuda, built_libs, fa_ctx, name):
     # each of twenty streams calls a few times, among many calls of another, so that they take each other's places; queued
     make = CALLS[name]
@@ -142,7 +142,7 @@ def node_types(graph):
     return out
 
 
-@pytest.mark.parametrize("name,kernels,others", [("one split", 1, 0), ("splits", 2, 4), ("handed", 2, 4), ("line", 2, 4)])
+@pytest.mark.parametrize("name,kernels,others", [("one split", 1, 0), ("splits", 2, 4), ("a CTA a pair", 1, 0), ("line", 2, 4)])
 def test_nodes_of_a_captured_decode(cuda, built_libs, fa_ctx, name, kernels, others):
     # no memset node, which would part the decode kernel from the kernel ahead; nothing but the kernel where no pair is cut, and
     # else two allocations, their two frees and the kernel that clears the words
