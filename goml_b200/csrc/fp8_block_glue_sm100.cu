@@ -162,7 +162,7 @@ __global__ void rope_table_kernel(float* cos_out, float* sin_out, int seq_len, i
 // ---------------------------------------------------------------------------------- RMSNorm (+ residual) + quantise
 // h = x (+ residual) for 4 consecutive elements
 __device__ __forceinline__ float4 load_h4(const float* x, const uint16_t* res, size_t off) {
-    float4 h = ld128f(x + off);
+    float4 h = *reinterpret_cast<const float4*>(x + off);   // a plain load: the compiler may have several in flight
     if (res) {
         const uint2 r = *reinterpret_cast<const uint2*>(res + off);
         h.x += __uint_as_float(r.x << 16);
