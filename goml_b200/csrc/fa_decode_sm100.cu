@@ -208,14 +208,14 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
         }
         return b0 + lane < p.batch ? seq_len_of(p, b0 + lane) : 0;
     };
-    auto len_of = [&](int b) -> int { return b < 32 * LENS ? __shfl_sync(0xffffffffu, lane_len(b & ~31), b & 31) : seq_len_of(p, b); };
-    // the part of one pair that starts at unit u and ends at unit end or with the pair
+    // the part of one pair that starts at unit u and ends at unit end or with the pair.  The sequence, its length and what lies
+    // before it come from one reading of the lengths: nothing is addressed from two that disagree (a caller that rewrites them
+    // while the kernel runs gets wrong results, and an empty part where the line has become shorter than u).
     auto segment_at = [&](int u, int end) {
         Segment x;
-        int seq_u0 = 0;
-        x.b = 0;
+        x.b = x.kvh = x.len = x.n_chunks = x.c_begin = x.c_end = x.pair_u0 = 0;
         for (int b0 = 0, before = 0; b0 < p.batch; b0 += 32) {
-            const int n = chunks_of(lane_len(b0)) * p.hkv;
+            const int len = lane_len(b0), n = chunks_of(len) * p.hkv;
             int incl = n;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -224,19 +224,18 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
             }
             const uint32_t past = __ballot_sync(0xffffffffu, before + incl > u);   // first lane whose sequence ends past u
             if (past) {
-                const int at = __ffs(past) - 1;
+                const int at = __ffs(past) - 1, seq_u0 = before + __shfl_sync(0xffffffffu, incl - n, at);
                 x.b = b0 + at;
-                seq_u0 = before + __shfl_sync(0xffffffffu, incl - n, at);
+                x.len = __shfl_sync(0xffffffffu, len, at);
+                x.n_chunks = chunks_of(x.len);
+                x.kvh = (u - seq_u0) / x.n_chunks;
+                x.pair_u0 = seq_u0 + x.kvh * x.n_chunks;
+                x.c_begin = u - x.pair_u0;
+                x.c_end = min(x.n_chunks, x.c_begin + (end - u));
                 break;
             }
             before += __shfl_sync(0xffffffffu, incl, 31);
         }
-        x.len = len_of(x.b);
-        x.n_chunks = chunks_of(x.len);
-        x.kvh = (u - seq_u0) / x.n_chunks;
-        x.pair_u0 = seq_u0 + x.kvh * x.n_chunks;
-        x.c_begin = u - x.pair_u0;
-        x.c_end = min(x.n_chunks, x.c_begin + (end - u));
         return x;
     };
 
@@ -271,6 +270,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
         mid_end = cut.begin(blockIdx.x + 1);
         if (mid >= mid_end) return;
         seg = segment_at(mid, mid_end);
+        if (seg.c_begin >= seg.c_end) return;
         mid += seg.c_end - seg.c_begin;
     }
     const Cut cut(cut_q, cut_r);
@@ -368,6 +368,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kern
             more = line && mid < mid_end;
             if (more) {
                 next = segment_at(mid, mid_end);
+                more = next.c_begin < next.c_end;
                 mid += next.c_end - next.c_begin;
             }
             if (more) {

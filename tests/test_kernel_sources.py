@@ -70,3 +70,10 @@ def test_calls_on_different_streams_do_not_hold_one_lock_over_their_launches():
     text = sources()["fa_api.cu"]
     assert re.search(r"lock = std::unique_lock<std::mutex>\(k->busy\)", text)
     assert not re.search(r"unique_lock<std::mutex>\([^)]*shared", text)
+
+
+def test_a_part_of_the_decode_line_comes_from_one_reading_of_the_lengths():
+    # two readings that disagree (a caller that rewrites the lengths while the kernel runs) must not make an address: the sequence
+    # that a unit falls in, its length and the units before it are taken from the same values
+    body = re.search(r"auto segment_at = .*?\n    \};", sources()["fa_decode_sm100.cu"], flags=re.S).group(0)
+    assert body.count("lane_len(") == 1 and "seq_len_of" not in body and "len_of(" not in body.replace("lane_len(", "")
