@@ -50,9 +50,9 @@ constexpr int THREADS = 128;
 constexpr int WARPS = THREADS / 32;
 constexpr float LAG = 6.0f;      // log2 units
 // A wide warp step takes twice the keys of a narrow one (8 against 4 KB in flight per warp) and leaves registers for 12
-// warps per SM instead of 16 (8 with two column tiles).  It streams faster (0.8 GB of cache: 137 us against 146); the
+// warps per SM instead of 16 (two column tiles: 8 instead of 12, or of 16 for D = 64).  It streams faster (0.8 GB of cache: 137 us against 146); the
 // narrow one lets more CTAs be resident.
-constexpr int ctas_per_sm(int nq, bool wide) { return nq == 2 ? 2 : wide ? 3 : 4; }
+constexpr int ctas_per_sm(int d, int nq, bool wide) { return nq == 2 ? (wide ? 2 : d == 64 ? 4 : 3) : wide ? 3 : 4; }
 
 // D = A B with a zero accumulator input
 __device__ __forceinline__ void mma_e4m3_m16n8k32_zero(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -169,7 +169,7 @@ struct Segment {
 };
 
 template <int D, int NQ, bool WIDE, bool STREAMS, bool PAGED>
-__global__ void __launch_bounds__(THREADS, ctas_per_sm(NQ, WIDE)) fa_decode_kernel(const DecodeParams p) {
+__global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_kernel(const DecodeParams p) {
     using C = Cfg<D, NQ, WIDE>;
     __shared__ float s_o[WARPS][C::ROWS][C::PITCH];
     __shared__ float s_m[WARPS][C::ROWS], s_l[WARPS][C::ROWS];
@@ -663,15 +663,21 @@ struct Layout {
 // against 3 of 592, 221 us against 262; 30 x 32 pairs, 3 rounds against 2, 202 against 186).
 //
 // Groups take the freely cut line, which balances best (24 sequences of 3000 to 6000 keys, 8 kv heads: 45 us against 70 with
-// fixed splits and a merging kernel), unless it has more chunks than an int counts (a paged cache whose capacity is far above
-// what it holds).
+// fixed splits and a merging kernel).  But each piece of a pair costs some 5 us of latency that nothing hides, so once the
+// pairs nearly fill the SMs (four fifths of the resident CTAs) a CTA per pair is faster for short sequences, and with several
+// pairs to a CTA for long ones too.  8 kv heads of 64 / of 128, lengths random up to the span, line against CTA per pair: 64
+// sequences of 1000 30 against 13 us / 32 against 20, 400 of 300 133 against 30 / 145 against 44, 400 of 4160 264 against 165 /
+// 392 against 306; but 64 of 8256 74 against 72 / 114 against 131.  Groups of 9 to 16 have fewer CTAs resident, so "several" is
+// one and a half there, and short sequences take narrow steps, which leave room for more (300 sequences of 64 keys, 16 heads on
+// one kv head of 64: 9.2 against 7 us; 500 of 1000 on one of 128 the other way, 39 against 62).  Last, a line has to have no more chunks than an int
+// counts (a paged cache whose capacity is far above what it holds).
 Layout layout_of(int batch, int q_heads, int kv_heads, int head_dim, int span) {
     Layout x;
     const int group = q_heads / kv_heads, sms = num_sms_of_current_device();
     x.rows = group <= 8 ? 8 : 16;
     x.streams = group == 1;
     const long long pairs = (long long)batch * kv_heads, chunks = ((long long)span + CHUNK - 1) / CHUNK;
-    const long long narrow = (long long)ctas_per_sm(1, false) * sms, wide = (long long)ctas_per_sm(x.rows / 8, true) * sms;
+    const long long narrow = (long long)ctas_per_sm(head_dim, 1, false) * sms, wide = (long long)ctas_per_sm(head_dim, x.rows / 8, true) * sms;
     x.splits = 1;
     x.wide = !x.streams;
     if (x.streams && pairs <= narrow) {
@@ -681,9 +687,10 @@ Layout layout_of(int batch, int q_heads, int kv_heads, int head_dim, int span) {
         x.splits = splits < 1 ? 1 : (int)splits;
         x.plan = SPLITS;
         x.grid = (int)(pairs * x.splits);
-    } else if (x.streams || pairs * chunks > 0x7fffffffLL) {
+    } else if (x.streams || 2 * pairs >= (x.rows == 8 ? 6 : 3) * wide || (chunks <= 32 && 5 * pairs >= 4 * wide) || pairs * chunks > 0x7fffffffLL) {
         x.plan = SPLITS;
         x.grid = (int)pairs;
+        if (x.rows == 16) x.wide = chunks > (head_dim == 64 ? 16 : 8);
         if (x.streams) x.wide = head_dim == 128 && chunks >= 32 && (pairs + wide - 1) / wide * wide <= (pairs + narrow - 1) / narrow * narrow;
     } else {
         x.plan = LINE;
@@ -738,7 +745,8 @@ cudaError_t launch_decode(const DecodeArgs& a) {
 #define KERNEL(D, NQ, WIDE, STREAMS) run(fa_decode_kernel<D, NQ, WIDE, STREAMS, false>, fa_decode_kernel<D, NQ, WIDE, STREAMS, true>)
     if (x.streams) return a.hd == 64 ? KERNEL(64, 1, false, true) : x.wide ? KERNEL(128, 1, true, true) : KERNEL(128, 1, false, true);
     if (x.rows == 8) return a.hd == 64 ? KERNEL(64, 1, true, false) : KERNEL(128, 1, true, false);
-    return a.hd == 64 ? KERNEL(64, 2, true, false) : KERNEL(128, 2, true, false);
+    if (x.wide) return a.hd == 64 ? KERNEL(64, 2, true, false) : KERNEL(128, 2, true, false);
+    return a.hd == 64 ? KERNEL(64, 2, false, false) : KERNEL(128, 2, false, false);
 #undef KERNEL
 }
 

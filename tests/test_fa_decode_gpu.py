@@ -189,6 +189,13 @@ def test_paged_rejects_bad_page_size(cuda, built_libs, fa_ctx):
     (40, 32, 32, 2050, 128, "ramp"),     # a CTA per pair: wide steps, empty sequences among them, one key in the last chunk
     (70, 16, 16, 2047, 128, "one long"),
     (19, 32, 32, 2049, 64, "ramp"),
+    (60, 32, 8, 900, 128, "ramp"),       # groups with a CTA per pair
+    (180, 8, 8, 65, 64, "one long"),
+    (200, 32, 8, 130, 64, "ramp"),
+    (61, 64, 4, 1025, 64, "one long"),   # two column tiles, a CTA per pair: wide and narrow steps
+    (70, 40, 4, 500, 128, "ramp"),
+    (300, 9, 1, 70, 64, "ramp"),
+    (130, 48, 4, 600, 128, "one long"),
 ])
 def test_decode_work_split(cuda, built_libs, fa_ctx, B, Hq, Hkv, Smax, D, lens):
     # the key range is cut at chunk borders wherever the pieces of the work line end, whatever the lengths are
