@@ -116,10 +116,10 @@ class FP8KVCache:
     def takes(self, batch: int, heads: int, S: int, hd: int, device: "torch.device | None" = None) -> bool:
         """Whether a prompt's codes can be written straight into this cache by a kernel of `device` (the codes' own by default)."""
         device = self.k.device if device is None else device
-        shape = (batch, heads, self.s_max, hd)
-        return ((batch, heads, hd) == (self.B, self.H, self.hd) and S <= self.s_max and self.dense_on(device)
-                and all(t.shape == shape and t.dtype == torch.uint8 and t.data_ptr() % 16 == 0 for t in (self.k, self.v))
-                and self.scales.shape == (2,) and self.lens.shape == (batch,))
+        k, v = self.k, self.v
+        return (batch == self.B and heads == self.H and hd == self.hd and S <= self.s_max and self.dense_on(device)
+                and k.shape == v.shape == (batch, heads, self.s_max, hd) and k.dtype is v.dtype is torch.uint8
+                and (k.data_ptr() | v.data_ptr()) % 16 == 0 and self.scales.shape == (2,) and self.lens.shape == (batch,))
 
     def fill(self, k_codes, v_codes, scales, S: int) -> None:
         """Prompt phase: K/V codes [batch*heads, S, hd] as the prefill quantiser wrote them, and their two scales."""
