@@ -5,8 +5,9 @@
 // O = softmax(scale * Q K^T + mask) V with an online (blockwise) softmax, fp16 output
 // and optional natural-log LSE — rebuilt around the Blackwell data path:
 //
-//   pre-pass       : V (e4m3) -> fp16 copy in a caller-provided workspace (exact:
-//                    every e4m3 value is an fp16 value; HBM-bound, <2% of the time)
+//   V in fp16      : exact (every e4m3 value is an fp16 value).  Long sequences: a pre-pass makes an fp16 copy in a
+//                    caller-provided workspace (HBM-bound, <2% of the time).  Short ones and narrow windows, where
+//                    few query tiles share a key: the kernel converts each tile in shared memory (VRAW below)
 //   TMA            : swizzled tiles, 3-D maps over [BH,S,D] so a tile never crosses a head
 //   S = Q K^T      : tcgen05.mma kind::f8f6f4 on the e4m3 codes, 128x64 fp32
 //                    accumulator in TMEM, double buffered so the next block's scores are
@@ -74,7 +75,7 @@ __device__ uint32_t g_fa_status = 0;
 // Shared memory holds only TMA-written operand tiles.  Both MMAs are limited by how fast the
 // tensor core can read its shared-memory operands (128 B/clk/SM), so P never goes through
 // shared memory: it is written to tensor memory and read from there as the A operand.
-template <int HD>
+template <int HD, bool VRAW>
 struct Cfg {
     static constexpr int Q_BYTES = BM * HD;
     static constexpr int K_BYTES = BN * HD;
@@ -83,7 +84,8 @@ struct Cfg {
     static constexpr int OFF_Q = 0;
     static constexpr int OFF_K = OFF_Q + Q_BYTES;
     static constexpr int OFF_V = OFF_K + STAGES * K_BYTES;
-    static constexpr int OFF_BAR = OFF_V + STAGES * V_BYTES;
+    static constexpr int OFF_VRAW = OFF_V + STAGES * V_BYTES;   // codes of V, where the kernel converts them itself
+    static constexpr int OFF_BAR = OFF_VRAW + (VRAW ? STAGES * K_BYTES : 0);
     static constexpr int SMEM_BYTES = OFF_BAR + 256;
     // TMEM: S[0], S[1] (64 fp32 columns each; P of the same block, 32 columns of packed fp16
     //       pairs, overwrites the first half of its S buffer)   O at [128, 128 + HD)
@@ -152,8 +154,7 @@ __device__ __forceinline__ void e4m3x16_to_f16(const uint4 c, uint4& lo, uint4& 
     uint32_t h[8];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h[2 * k]) : "h"((uint16_t)(w[k] & 0xffffu)));
-        asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h[2 * k + 1]) : "h"((uint16_t)(w[k] >> 16)));
+        asm("{\n\t.reg .b16 l, u;\n\tmov.b32 {l, u}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, l;\n\tcvt.rn.f16x2.e4m3x2 %1, u;\n\t}" : "=r"(h[2 * k]), "=r"(h[2 * k + 1]) : "r"(w[k]));
     }
     lo = make_uint4(h[0], h[1], h[2], h[3]);
     hi = make_uint4(h[4], h[5], h[6], h[7]);
@@ -235,20 +236,67 @@ __device__ __forceinline__ bool wait_v_chunk(const uint32_t* head_flags, int chu
     }
 }
 
+// One 64-key tile of V in shared memory: codes -> fp16 in the order of a TMA load with 128-byte swizzle, one 64-column slab of
+// d after the other.  By one warp, which takes 16 codes of a lane at a time; eight neighbouring lanes, whose 16-byte accesses
+// share a wavefront, meet eight different bank groups on both sides.
+//  D = 128 (codes swizzled too): they take four neighbouring pieces of one slab of two keys k and k ^ 5 — bit 2 of the key puts the
+//   loads in different halves of the 128 bytes, bit 0 the stores on chunks of different parity;
+//  D = 64 (codes as they lie in global memory): the four pieces of two neighbouring keys, 128 bytes in a row.
+// Unrolled in full: a loop of four steps cost 2 % at S = 8192.
+template <int HD>
+__device__ __forceinline__ void convert_v(uint32_t raw, uint32_t dst) {
+    constexpr int STEPS = BN * HD / 512, BATCH = 8;   // steps of the warp, loads in flight
+    const int lane = threadIdx.x & 31;
+    const int slab = HD == 128 ? (lane >> 3) & 1 : 0;
+    const int key = HD == 128 ? (lane >> 4) ^ ((lane & 4) ? 5 : 0) : lane >> 2;   // of step 0, below 8
+    const int chunk = ((lane & 3) * 2) ^ key;
+    // D = 128: a step takes four keys, {0, 5, 1, 4} and then {2, 7, 3, 6} of eight: key + 2 is key ^ 2.  D = 64: eight
+    constexpr int TURN = HD == 128 ? 2 : 1;           // steps per eight keys
+    uint32_t src[TURN], lo_at[TURN], hi_at[TURN];
+#pragma unroll
+    for (int t = 0; t < TURN; t++) {
+        const int row = (key ^ (2 * t)) * 128;
+        src[t] = raw + (HD == 128 ? row + (((slab * 4 + (lane & 3)) ^ key ^ (2 * t)) << 4) : lane * 16);
+        lo_at[t] = dst + slab * (BN * 128) + row + ((chunk ^ (2 * t)) << 4);
+        hi_at[t] = dst + slab * (BN * 128) + row + ((chunk ^ (2 * t) ^ 1) << 4);
+    }
+#pragma unroll
+    for (int i0 = 0; i0 < STEPS; i0 += BATCH) {
+        uint4 v[BATCH];
+#pragma unroll
+        for (int i = 0; i < BATCH; i++)
+            asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[i].x), "=r"(v[i].y), "=r"(v[i].z), "=r"(v[i].w)
+                         : "r"(src[i % TURN] + (i0 + i) / TURN * (8 * HD)) : "memory");
+#pragma unroll
+        for (int i = 0; i < BATCH; i++) {
+            uint4 lo, hi;
+            e4m3x16_to_f16(v[i], lo, hi);
+            const int at = (i0 + i) / TURN * 1024;
+            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(lo_at[i % TURN] + at), "r"(lo.x), "r"(lo.y), "r"(lo.z), "r"(lo.w) : "memory");
+            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(hi_at[i % TURN] + at), "r"(hi.x), "r"(hi.y), "r"(hi.z), "r"(hi.w) : "memory");
+        }
+    }
+}
+
 // Sign flip of one row of raw scores for a negative scale (the row max is taken on sign-adjusted scores).
 // Rare, so it is kept out of line: the common path pays one not-taken branch instead of 64 predicated ops.
 __device__ __noinline__ void negate_scores(uint32_t* s) {
     for (int c = 0; c < BN; c++) s[c] ^= 0x80000000u;
 }
 
+// VRAW = true: V arrives as codes, and the producer warp converts each tile in shared memory while it waits for the ring.  That
+// costs a tile 0.04 us per key block (D = 128; the producer shares its scheduler with one softmax warp of the CTA, and
+// shared memory carries 24 KB more per block) and saves the pre-pass: 3 bytes per element of traffic, a launch, the scratch, and
+// the CTAs of the pre-pass, which the attention's first CTAs wait for.  Bit for bit the same results.
+//
 // MASKED = false: no key of the launch is masked (non-causal, no window, S a multiple of the block) and the host-side scale
 // is positive: neither the masking code nor the sign flip of a negative scale is compiled into the softmax loop.  (The
 // device-side scale factors are quantiser outputs, amax / 448: never negative.)
-template <int HD, bool MASKED>
+template <int HD, bool MASKED, bool VRAW>
 __global__ void __launch_bounds__(NUM_THREADS, 2)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
               const __grid_constant__ CUtensorMap tmap_v, const Params p) {
-    using C = Cfg<HD>;
+    using C = Cfg<HD, VRAW>;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem);
     const uint32_t bars = sbase + C::OFF_BAR;
@@ -260,6 +308,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     const uint32_t bar_sfull = bar_vfull + 8 * STAGES;    // [STAGES] S = Q K^T of that block complete (K stage reusable)
     const uint32_t bar_pvdone = bar_sfull + 8 * STAGES;   // [STAGES] O += P V of that block complete (V stage reusable)
     const uint32_t bar_pfull = bar_pvdone + 8 * STAGES;   // [2] softmax wrote P into S[b] (and rescaled O if needed)
+    const uint32_t bar_vraw = bar_pfull + 16;             // [STAGES] codes of a V tile landed
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_BAR + 240);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
@@ -296,6 +345,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
             mbar_init(bar_vfull + 8 * s, 1);
             mbar_init(bar_sfull + 8 * s, 1);
             mbar_init(bar_pvdone + 8 * s, 1);
+            mbar_init(bar_vraw + 8 * s, 1);
         }
         for (int b = 0; b < 2; b++) mbar_init(bar_pfull + 8 * b, NUM_SOFTMAX_WARPS * 32);
         *abort_flag = (sbase & 1023u) ? ST_BAD_SMEM_ALIGN : 0u;
@@ -312,6 +362,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     const uint32_t tmem_s = tmem_base;
     const uint32_t tmem_o = tmem_base + C::O_COL;
     const bool bad_start = (*abort_flag != 0);
+    if (VRAW) pdl_wait();   // no pre-pass has waited for what is ahead
 
     if (bad_start) {
         // fall through to teardown
@@ -327,36 +378,77 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
                 mbar_arrive_expect_tx(bar_q, C::Q_BYTES);
                 tma_load_3d(sbase + C::OFF_Q, &tmap_q, bar_q, 0, q0, head);
             }
-            // Q and K are complete when this kernel starts (the pre-pass triggered it after its own wait); the fp16 copy
-            // of V is waited for chunk by chunk, or as a whole when the launch has no flags
-            int v_ready = 0;
-            const uint32_t* head_flags = p.v_flags ? p.v_flags + (size_t)head * p.v_chunks : nullptr;
-            int s = 0;
-            uint32_t ph = 1;  // "previous phase complete": the rings start empty
-            for (int j = 0; j < nblk; j++) {
-                const int key0 = (blk0 + j) * BN;
-                if (!mbar_wait_warp(bar_sfull + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD)) break;   // Q K^T three blocks back is done
-                if (leader) {
+            if (VRAW) {
+                auto load_k = [&](int j) {
+                    const int s = j % STAGES;
                     mbar_arrive_expect_tx(bar_kfull + 8 * s, C::K_BYTES);
-                    tma_load_3d(sbase + C::OFF_K + s * C::K_BYTES, &tmap_k, bar_kfull + 8 * s, 0, key0, head);
-                }
-                if (!mbar_wait_warp(bar_pvdone + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD)) break;  // P V three blocks back is done
-                if (!head_flags) {
-                    if (j == 0) pdl_wait();
-                } else if (!wait_v_chunk(head_flags, p.v_chunks, p.v_epoch, key0 / V_CHUNK, v_ready, abort_flag)) {
-                    break;
-                }
+                    tma_load_3d(sbase + C::OFF_K + s * C::K_BYTES, &tmap_k, bar_kfull + 8 * s, 0, (blk0 + j) * BN, head);
+                };
+                auto load_v = [&](int j) {
+                    const int s = j % STAGES;
+                    mbar_arrive_expect_tx(bar_vraw + 8 * s, C::K_BYTES);
+                    tma_load_3d(sbase + C::OFF_VRAW + s * C::K_BYTES, &tmap_v, bar_vraw + 8 * s, 0, (blk0 + j) * BN, head);
+                };
                 if (leader) {
-                    mbar_arrive_expect_tx(bar_vfull + 8 * s, C::V_BYTES);
-#pragma unroll
-                    for (int h = 0; h < HD / 64; h++)  // one 64-column (128-byte) slab of d per copy
-                        tma_load_3d(sbase + C::OFF_V + s * C::V_BYTES + h * C::V_HALF_BYTES, &tmap_v, bar_vfull + 8 * s,
-                                    h * 64, key0, head);
+                    for (int j = 0; j < STAGES && j < nblk; j++) {
+                        load_k(j);
+                        load_v(j);
+                    }
                 }
                 __syncwarp();
-                if (++s == STAGES) { s = 0; ph ^= 1; }
+                int s = 0;         // ring stage of block j, of K, of the codes of V and of V alike
+                uint32_t ph = 0;   // phase of block j
+                for (int j = 0; j < nblk; j++) {
+                    if (!mbar_wait_warp(bar_vraw + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD)) break;
+                    if (!mbar_wait_warp(bar_pvdone + 8 * s, ph ^ 1, abort_flag, ST_TIMEOUT_LOAD)) break;   // P V three blocks back is done
+                    // and with it every MMA issued before it, Q K^T two blocks back among them: its K stage is free.  (In the third
+                    // block nothing has been waited for yet: there the first Q K^T is.)
+                    if (j + 1 >= STAGES && j + 1 < nblk) {
+                        if (j + 1 == STAGES && !mbar_wait_warp(bar_sfull, 0, abort_flag, ST_TIMEOUT_LOAD)) break;
+                        if (leader) load_k(j + 1);
+                    }
+                    convert_v<HD>(sbase + C::OFF_VRAW + s * C::K_BYTES, sbase + C::OFF_V + s * C::V_BYTES);
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (leader) {
+                        mbar_arrive(bar_vfull + 8 * s);
+                        if (j + STAGES < nblk) load_v(j + STAGES);
+                    }
+                    __syncwarp();
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
+                }
+            } else {
+                // Q and K are complete when this kernel starts (the pre-pass triggered it after its own wait); the fp16 copy
+                // of V is waited for chunk by chunk, or as a whole when the launch has no flags
+                int v_ready = 0;
+                const uint32_t* head_flags = p.v_flags ? p.v_flags + (size_t)head * p.v_chunks : nullptr;
+                int s = 0;
+                uint32_t ph = 1;  // "previous phase complete": the rings start empty
+                for (int j = 0; j < nblk; j++) {
+                    const int key0 = (blk0 + j) * BN;
+                    if (!mbar_wait_warp(bar_sfull + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD)) break;   // Q K^T three blocks back is done
+                    if (leader) {
+                        mbar_arrive_expect_tx(bar_kfull + 8 * s, C::K_BYTES);
+                        tma_load_3d(sbase + C::OFF_K + s * C::K_BYTES, &tmap_k, bar_kfull + 8 * s, 0, key0, head);
+                    }
+                    if (!mbar_wait_warp(bar_pvdone + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD)) break;  // P V three blocks back is done
+                    if (!head_flags) {
+                        if (j == 0) pdl_wait();
+                    } else if (!wait_v_chunk(head_flags, p.v_chunks, p.v_epoch, key0 / V_CHUNK, v_ready, abort_flag)) {
+                        break;
+                    }
+                    if (leader) {
+                        mbar_arrive_expect_tx(bar_vfull + 8 * s, C::V_BYTES);
+#pragma unroll
+                        for (int h = 0; h < HD / 64; h++)  // one 64-column (128-byte) slab of d per copy
+                            tma_load_3d(sbase + C::OFF_V + s * C::V_BYTES + h * C::V_HALF_BYTES, &tmap_v, bar_vfull + 8 * s,
+                                        h * 64, key0, head);
+                    }
+                    __syncwarp();
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
+                }
+                pdl_wait();   // this kernel completes after the pre-pass
             }
-            pdl_wait();   // this kernel completes after the pre-pass
         }
     } else if (warp == MMA_WARP) {
         // -------------------------------------------------------------- MMA issuer
@@ -653,9 +745,25 @@ DeviceState g_dev[64];
 
 void init_device(DeviceState* st, int dev);
 
-template <int HD>
+// Whether the kernel converts V itself.  What a tile's conversion costs is paid once for every query tile that reads the key
+// block, what the pre-pass costs once per key block: the line lies at a number of queries per key.  Measured with the pre-pass /
+// in the kernel (us): D = 128, not causal, 128 heads of 1024 77.9 / 73.6, 64 of 1536 82 / 77, 64 of 2048 129.7 / 131.5, 24 of 4096
+// 186 / 188, 128 of 8192 3446 / 3563; causal, half of whose queries see a key, but the last ones of every sequence see all: 512
+// heads of 512 94 / 76, 256 of 2048 339 / 311, 60 of 3000 163 / 156 but 20 of 3000 71 / 74; window 1300, 20 heads of 8000, 129 / 122.
+// D = 64 converts half as much per block: 64 of 2048 101 / 98, 42 of 3072 143 / 142, 32 of 4096 185 / 186; causal 40 of 4000 147 /
+// 140; window 512 of 3000, 64 heads, 71.2 / 65.0.  Where no more than half of the SMs have a tile, nothing hides the conversion
+// behind another CTA and its cost adds up along the longest tile: 8 heads of 1024 15.4 / 14.0, 4 of 1280 16.8 / 17.4, 1 of 8192 75 / 92.
+bool converts_v(const LaunchArgs& a, int num_sms) {
+    const int limit = a.hd == 128 ? 1536 : 2560;
+    const int span = a.causal && a.window > 0 && a.window < a.sl - BM ? a.window + BM : a.sl;   // keys of the longest tile
+    const long long tiles = (long long)a.bh * ((a.sl + BM - 1) / BM);
+    if (2 * tiles <= num_sms) return span <= 1024;
+    return (a.causal && span == a.sl ? (long long)a.sl * 3 / 5 : span) <= limit;
+}
+
+template <int HD, bool VRAW>
 cudaError_t launch_hd(const LaunchArgs& a, int num_sms) {
-    using C = Cfg<HD>;
+    using C = Cfg<HD, VRAW>;
     const long long grid = (long long)a.bh * ((a.sl + BM - 1) / BM);
     const int v_chunks = (a.sl + V_CHUNK - 1) / V_CHUNK;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
@@ -663,7 +771,8 @@ cudaError_t launch_hd(const LaunchArgs& a, int num_sms) {
     const CUtensorMapSwizzle swz = (HD == 128) ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
     if (!make_tmap_u8_3d(&tq, a.q, a.bh, a.sl, HD, BM, HD, swz) ||
         !make_tmap_u8_3d(&tk, a.k, a.bh, a.sl, HD, BN, HD, swz) ||
-        !make_tmap_u16_3d(&tv, a.v16_workspace, a.bh, a.sl, HD, BN, 64, CU_TENSOR_MAP_SWIZZLE_128B))
+        !(VRAW ? make_tmap_u8_3d(&tv, a.v, a.bh, a.sl, HD, BN, HD, HD == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE)
+               : make_tmap_u16_3d(&tv, a.v16_workspace, a.bh, a.sl, HD, BN, 64, CU_TENSOR_MAP_SWIZZLE_128B)))
         return cudaErrorInvalidValue;
     Params p;
     p.bh = a.bh; p.sl = a.sl; p.n_qtiles = (a.sl + BM - 1) / BM;
@@ -674,30 +783,46 @@ cudaError_t launch_hd(const LaunchArgs& a, int num_sms) {
     p.o = reinterpret_cast<__half*>(a.o);
     p.lse = a.lse;
     p.v_flags = a.v_flags; p.v_epoch = a.v_epoch; p.v_chunks = v_chunks;
-    // pre-pass: V codes -> fp16 workspace
-    const long long chunks = (long long)a.bh * v_chunks, cap = (long long)num_sms * V_CTAS_PER_SM;
-    const cudaError_t e = launch_pdl(v_to_f16_kernel<HD>, (unsigned)(chunks < cap ? chunks : cap), V_THREADS, 0, a.stream,
-                                     reinterpret_cast<const uint4*>(a.v), reinterpret_cast<uint4*>(a.v16_workspace), (int)chunks, v_chunks,
-                                     a.sl, a.v_flags, a.v_epoch);
-    if (e != cudaSuccess) return e;
+    if (!VRAW) {
+        // pre-pass: V codes -> fp16 workspace
+        const long long chunks = (long long)a.bh * v_chunks, cap = (long long)num_sms * V_CTAS_PER_SM;
+        const cudaError_t e = launch_pdl(v_to_f16_kernel<HD>, (unsigned)(chunks < cap ? chunks : cap), V_THREADS, 0, a.stream,
+                                         reinterpret_cast<const uint4*>(a.v), reinterpret_cast<uint4*>(a.v16_workspace), (int)chunks, v_chunks,
+                                         a.sl, a.v_flags, a.v_epoch);
+        if (e != cudaSuccess) return e;
+    }
     const bool masked = a.causal || a.window > 0 || (a.sl % BN) != 0 || !(a.scale > 0.f);
-    return masked ? launch_pdl(fa_fwd_kernel<HD, true>, (unsigned)grid, NUM_THREADS, C::SMEM_BYTES, a.stream, tq, tk, tv, p)
-                  : launch_pdl(fa_fwd_kernel<HD, false>, (unsigned)grid, NUM_THREADS, C::SMEM_BYTES, a.stream, tq, tk, tv, p);
+    return masked ? launch_pdl(fa_fwd_kernel<HD, true, VRAW>, (unsigned)grid, NUM_THREADS, C::SMEM_BYTES, a.stream, tq, tk, tv, p)
+                  : launch_pdl(fa_fwd_kernel<HD, false, VRAW>, (unsigned)grid, NUM_THREADS, C::SMEM_BYTES, a.stream, tq, tk, tv, p);
 }
 
 }  // namespace
 
 namespace {
 void init_device(DeviceState* st, int dev) {
-    cudaError_t e = cudaFuncSetAttribute(fa_fwd_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<128>::SMEM_BYTES);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fa_fwd_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<128>::SMEM_BYTES);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fa_fwd_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<64>::SMEM_BYTES);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fa_fwd_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<64>::SMEM_BYTES);
+    cudaError_t e = cudaSuccess;
+    auto set = [&](auto kernel, int bytes) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    };
+    set(fa_fwd_kernel<128, true, false>, Cfg<128, false>::SMEM_BYTES);
+    set(fa_fwd_kernel<128, false, false>, Cfg<128, false>::SMEM_BYTES);
+    set(fa_fwd_kernel<64, true, false>, Cfg<64, false>::SMEM_BYTES);
+    set(fa_fwd_kernel<64, false, false>, Cfg<64, false>::SMEM_BYTES);
+    set(fa_fwd_kernel<128, true, true>, Cfg<128, true>::SMEM_BYTES);
+    set(fa_fwd_kernel<128, false, true>, Cfg<128, true>::SMEM_BYTES);
+    set(fa_fwd_kernel<64, true, true>, Cfg<64, true>::SMEM_BYTES);
+    set(fa_fwd_kernel<64, false, true>, Cfg<64, true>::SMEM_BYTES);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&st->num_sms, cudaDevAttrMultiProcessorCount, dev);
     st->init_error = e;
 }
 }  // namespace
 
+bool needs_no_scratch(const LaunchArgs& a) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    std::call_once(g_dev[dev].once, init_device, &g_dev[dev], dev);
+    return g_dev[dev].init_error == cudaSuccess && converts_v(a, g_dev[dev].num_sms);
+}
 size_t workspace_bytes(int bh, int sl, int hd) { return (size_t)bh * sl * hd * 2; }
 size_t v_flag_count(int bh, int sl) { return (size_t)bh * ((sl + V_CHUNK - 1) / V_CHUNK); }
 
@@ -706,10 +831,11 @@ cudaError_t launch(const LaunchArgs& a) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    if (!a.v16_workspace || (reinterpret_cast<uintptr_t>(a.v16_workspace) & 127)) return cudaErrorInvalidValue;
     std::call_once(g_dev[dev].once, init_device, &g_dev[dev], dev);
     if (g_dev[dev].init_error != cudaSuccess) return g_dev[dev].init_error;
-    return a.hd == 128 ? launch_hd<128>(a, g_dev[dev].num_sms) : launch_hd<64>(a, g_dev[dev].num_sms);
+    if (converts_v(a, g_dev[dev].num_sms)) return a.hd == 128 ? launch_hd<128, true>(a, g_dev[dev].num_sms) : launch_hd<64, true>(a, g_dev[dev].num_sms);
+    if (!a.v16_workspace || (reinterpret_cast<uintptr_t>(a.v16_workspace) & 127)) return cudaErrorInvalidValue;
+    return a.hd == 128 ? launch_hd<128, false>(a, g_dev[dev].num_sms) : launch_hd<64, false>(a, g_dev[dev].num_sms);
 }
 
 cudaError_t launch_wait_expiry_selftest(cudaStream_t stream) {

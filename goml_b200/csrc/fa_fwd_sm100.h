@@ -12,7 +12,7 @@ struct LaunchArgs {
     const void* v;
     void* o;            // [bh, sl, hd] fp16
     float* lse;         // [bh, sl] fp32 natural-log LSE, or nullptr
-    void* v16_workspace = nullptr;  // workspace_bytes(bh, sl, hd) bytes, 128-byte aligned: fp16 copy of V
+    void* v16_workspace = nullptr;  // workspace_bytes(bh, sl, hd) bytes, 128-byte aligned: fp16 copy of V (see needs_no_scratch)
     int bh, sl, hd;     // hd in {64, 128}
     int causal, window;
     float scale;        // softmax_scale * scale_q * scale_k
@@ -28,7 +28,10 @@ struct LaunchArgs {
     uint32_t v_epoch = 0;
 };
 
-// Scratch the forward needs (an fp16 copy of V made by a pre-pass on the same stream).
+// Whether this call's kernel converts V itself: v16_workspace and v_flags may then be null.  Weak, so that the host side can be
+// linked without the kernels (the test of the scratch table), where every call takes scratch.
+__attribute__((weak)) bool needs_no_scratch(const LaunchArgs& a);
+// Scratch the forward needs otherwise (an fp16 copy of V made by a pre-pass on the same stream).
 size_t workspace_bytes(int bh, int sl, int hd);
 size_t v_flag_count(int bh, int sl);
 

@@ -1,4 +1,5 @@
-"""Attention forward where masks cut key blocks: every 32-key chunk of a block is masked, left alone or skipped per warp."""
+"""Attention forward where masks cut key blocks (every 32-key chunk of a block is masked, left alone or skipped per warp), and
+where V is converted: by a pre-pass or in the kernel."""
 import math
 
 import numpy as np
@@ -32,3 +33,45 @@ def test_masks_that_cut_chunks(fa_ctx, s, hd, scale):
         for window in sorted({w for w in (0, 1, 2, 31, 32, 33, 63, 64, 65, 96, 127, 128, 129, 160, s - 1, s) if 0 <= w <= s}):
             o, lse = run_attention(fa_ctx, q, k, v, causal, window, scale)
             near(o, lse, q, k, v, causal, window, scale)
+
+
+@pytest.mark.parametrize("s,hd,causal,window", [(1025, 128, 0, 0), (1536, 128, 0, 0), (1500, 128, 1, 0), (1500, 128, 1, 1000), (1400, 64, 0, 0), (1100, 64, 1, 0),
+                                                (1279, 64, 0, 700)])
+def test_v_converted_ahead_and_in_the_kernel_gives_the_same_bits(cuda, built_libs, fa_ctx, s, hd, causal, window):
+    # few heads have V converted by a pre-pass, more of them in the kernel; a head's result does not depend on the others
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(s)
+    q, k, v = (torch.randint(0, 0x70, (13, s, hd), generator=g, dtype=torch.uint8, device="cuda") for _ in range(3))
+    for t in (q, k, v):
+        t ^= torch.randint(0, 2, t.shape, generator=g, dtype=torch.uint8, device="cuda") << 7
+    v[2, s - 1, 3] = 0x7f   # NaN
+    out = []
+    for heads in (3, 13):
+        o = torch.zeros(heads, s, hd, dtype=torch.float16, device="cuda")
+        lse = torch.zeros(heads, s, device="cuda")
+        fa_ctx.ForwardEx(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), heads, s, hd, causal, window, 1e-5, 1.0)
+        torch.cuda.synchronize()
+        fa_ctx.DeviceStatus()
+        out.append((o[:3], lse[:3]))
+    assert torch.isnan(out[0][0][2, s - 1, 3]) and not torch.isnan(out[0][0][:2]).any()
+    assert torch.equal(out[0][0].view(torch.int16), out[1][0].view(torch.int16)) and torch.equal(out[0][1], out[1][1])
+
+
+# calls whose V is converted ahead, with scratch
+AHEAD = {"few tiles": (4, 1300, 128, 0), "hd 64": (6, 2700, 64, 0), "causal": (9, 2700, 128, 1)}
+
+
+@pytest.mark.parametrize("name", AHEAD)
+def test_scratch_of_the_pre_pass(cuda, built_libs, fa_ctx, monkeypatch, name):
+    # the promises of the scratch table, for calls that take the pre-pass
+    from tests import test_fa_scratch_gpu as scratch
+    monkeypatch.setitem(scratch.CALLS, name, lambda: scratch.Forward(*AHEAD[name]))
+    scratch.test_a_graph_gives_the_bits_of_the_eager_call(cuda, built_libs, fa_ctx, name)
+    scratch.test_twenty_streams_give_the_same_bits(cuda, built_libs, fa_ctx, name)
+    scratch.test_streams_that_come_and_go(cuda, built_libs, fa_ctx, name)
+
+
+def test_the_last_context_goes_while_a_pre_pass_is_queued(cuda, built_libs, monkeypatch):
+    from tests import test_fa_scratch_gpu as scratch
+    monkeypatch.setattr(scratch, "LAST_CONTEXT", scratch.LAST_CONTEXT.replace("2048", "4608"))
+    scratch.test_the_last_context_goes_while_work_is_queued_and_a_capture_is_open(cuda, built_libs)
