@@ -10,12 +10,14 @@ other binding of this package; each call is asynchronous on `stream`.
 from __future__ import annotations
 
 import ctypes as C
+import struct
 import threading
 
 from . import loader
 
 _lock = threading.Lock()
 _lib = None
+_run = None   # fp8_block_run taking the packed block
 
 
 class BlockGlueError(RuntimeError):
@@ -36,6 +38,40 @@ class DecodeAppendArgs(C.Structure):
     ]
 
 
+class BlockRunArgs(C.Structure):
+    """fp8_block_run_args_t (include/fp8_block.h)."""
+    _fields_ = ([(name, C.c_void_p) for name in (
+        "gemm_scaled", "gemm_accumulate_f32", "gemm_swiglu_raise", "attention", "attention_ctx", "x", "h", "norm1", "norm2",
+        "wqkv", "wo", "wgate_up", "wdown", "wqkv_scale", "wo_scale", "wgate_up_scale", "wdown_scale", "cos_tab", "sin_tab",
+        "k_cache", "v_cache", "cache_scales", "cache_lens", "words", "rstd", "codes", "k_codes", "v_codes", "region")]
+        + [("region_bytes", C.c_size_t), ("stream", C.c_void_p)]
+        + [(name, C.c_int32) for name in ("batch", "seq_len", "d_model", "heads", "ffn_hidden", "s_max", "rope_rows", "decode")]
+        + [("eps", C.c_float), ("softmax_scale", C.c_float)])
+
+
+_PACK_RUN = struct.Struct("@29PNP8i2f").pack
+assert struct.calcsize("@29PNP8i2f") == C.sizeof(BlockRunArgs)
+
+
+def BlockRun(*args) -> int:
+    """fp8_block_run with the fields of BlockRunArgs in order; its return code."""
+    run = _run or _load_run()
+    try:
+        block = _PACK_RUN(*args)
+    except (struct.error, OverflowError):   # values that only ctypes takes
+        block = bytes(BlockRunArgs(*args))
+    return run(block)
+
+
+def _load_run():
+    global _run
+    lib = _init()
+    fn = lib["fp8_block_run"]
+    fn.restype, fn.argtypes = C.c_int, [C.c_char_p]
+    _run = fn
+    return fn
+
+
 def _init():
     global _lib
     with _lock:
@@ -53,6 +89,7 @@ def _init():
                 "fp8_quantize_bf16": [p, p, p, p, z, p],
                 "fp8_residual_add": [p, p, z, p],
                 "fp8_decode_rope_append": [C.POINTER(DecodeAppendArgs)],
+                "fp8_block_run": [C.POINTER(BlockRunArgs)],
             }.items():
                 fn = getattr(lib, name)
                 fn.restype = C.c_int

@@ -14,6 +14,7 @@
 #include <stdint.h>
 
 #include "../../include/fp8_block.h"
+#include "fp8_block_glue.h"
 #include "one_cluster.cuh"
 
 namespace {
@@ -351,7 +352,8 @@ struct RmsOp {
     float* scale_out;
     float* amax_out;
     float* rstd_ws;
-    float* zero_word;
+    float* zero;    // words set to 0 first (its own maximum may be among them)
+    int zeros;
     int rows, hidden;
     float eps;
     int lw;         // log2 of the warps per row
@@ -390,7 +392,7 @@ struct RmsOp {
     __device__ void pass1(float (&m)[1]) const {
         __shared__ float2 part[2][OC_THREADS / 32];
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpr = 1 << lw, wi = warp & (wpr - 1);
-        if (zero_word && oc_tid() == 0) *zero_word = 0.f;
+        if (oc_tid() < (uint32_t)zeros) zero[oc_tid()] = 0.f;   // ahead of the cluster barrier in front of pass 2
         const int n = rounds();
         for (int it = 0; it < n; it++) {
             const int row = row_of(it);
@@ -976,10 +978,10 @@ int fp8_rope_table(float* cos_out, float* sin_out, int seq_len, int head_dim, fl
 
 }  // extern "C"
 
-namespace {
+namespace fp8_block {
 
-int rmsnorm_quantize(const float* x, const void* residual_bf16, float* h_out, bool store_h, const float* gamma, uint8_t* q, float* scale_out,
-                     float* amax_out, float* rstd_ws, float* zero_word, int rows, int hidden, float eps, cudaStream_t s) {
+int rmsnorm(const float* x, const void* residual_bf16, float* h_out, bool store_h, const float* gamma, uint8_t* q, float* scale_out, float* amax_out,
+            float* rstd_ws, const Words& words, int rows, int hidden, float eps, cudaStream_t s) {
     if (!x || !gamma || !q || !scale_out || !amax_out || !rstd_ws) return (int)cudaErrorInvalidValue;
     if (rows < 0 || hidden <= 0 || (hidden % 16) != 0) return (int)cudaErrorInvalidValue;
     if (misaligned32(x) || misaligned(residual_bf16) || misaligned32(h_out) || misaligned32(gamma) || misaligned(q)) return (int)cudaErrorInvalidValue;
@@ -988,11 +990,11 @@ int rmsnorm_quantize(const float* x, const void* residual_bf16, float* h_out, bo
     const uint16_t* res = reinterpret_cast<const uint16_t*>(residual_bf16);
     float* h = store_h ? h_out : nullptr;
     if (items * 64 <= OC_BYTES_RMS && oc_fits<RmsOp>()) {
-        RmsOp op{x, res, h, gamma, q, scale_out, amax_out, rstd_ws, zero_word, rows, hidden, eps, rows <= OC_CTAS ? 4 : rows <= 4 * OC_CTAS ? 2 : 0};
+        RmsOp op{x, res, h, gamma, q, scale_out, amax_out, rstd_ws, words.first, words.n, rows, hidden, eps, rows <= OC_CTAS ? 4 : rows <= 4 * OC_CTAS ? 2 : 0};
         return (int)oc_launch(op, s);
     }
-    cudaError_t e = clear_words(amax_out, 1, s);
-    if (e == cudaSuccess && zero_word) e = clear_words(zero_word, 1, s);
+    cudaError_t e = words.cleared ? cudaSuccess : clear_words(amax_out, 1, s);
+    if (e == cudaSuccess && words.n > 0) e = clear_words(words.first, words.n, s);
     if (e != cudaSuccess) return (int)e;
     if (rows > 0) {
         int dev = 0, sms = 148;
@@ -1013,7 +1015,14 @@ int rmsnorm_quantize(const float* x, const void* residual_bf16, float* h_out, bo
                            amax_out, scale_out, q, (uint32_t)items, hidden, FastDiv(hidden / 16));
 }
 
-int rope_quantize_qkv(QkvArgs a, cudaStream_t s) {
+int rope_qkv(const Rope& r, bool cleared, cudaStream_t s) {
+    QkvArgs a{};
+    a.qkv = reinterpret_cast<const uint16_t*>(r.qkv_bf16);
+    a.cos_tab = r.cos_tab; a.sin_tab = r.sin_tab; a.scales = r.scales; a.amaxes = r.amaxes;
+    a.q_out = r.q_out; a.k_out = r.k_out; a.v_out = r.v_out;
+    a.k_cache = r.k_cache; a.v_cache = r.v_cache; a.cache_scales = r.cache_scales; a.cache_lens = r.cache_lens; a.s_max = r.s_max;
+    a.batch = r.batch; a.seq_len = r.seq_len; a.heads = r.heads; a.hd = r.head_dim;
+    if (a.k_cache && (misaligned(a.k_cache) || misaligned(a.v_cache))) return (int)cudaErrorInvalidValue;
     if (!a.qkv || !a.cos_tab || !a.sin_tab || !a.q_out || !a.k_out || !a.v_out || !a.scales || !a.amaxes) return (int)cudaErrorInvalidValue;
     if (a.batch < 0 || a.seq_len <= 0 || a.heads <= 0 || (a.hd != 64 && a.hd != 128)) return (int)cudaErrorInvalidValue;
     if (misaligned(a.qkv) || misaligned(a.cos_tab) || misaligned(a.sin_tab) || misaligned(a.q_out) || misaligned(a.k_out) || misaligned(a.v_out))
@@ -1026,54 +1035,13 @@ int rope_quantize_qkv(QkvArgs a, cudaStream_t s) {
     a.dv.three = FastDiv(3);
     a.dv.seq = FastDiv(a.seq_len);
     if (items * 64 <= OC_BYTES_QKV && oc_fits<QkvOp>()) return (int)oc_launch(QkvOp{a}, s);
-    cudaError_t e = clear_words(a.amaxes, 3, s);
+    cudaError_t e = cleared ? cudaSuccess : clear_words(a.amaxes, 3, s);
     if (e == cudaSuccess && items > 0) e = launch_pdl(qkv_amax_kernel, dim3(grid_for(items)), dim3(THREADS), 0, s, a);
     if (e == cudaSuccess) e = launch_pdl(qkv_quant_kernel, dim3(grid_for(items)), dim3(THREADS), 0, s, a);
     return (int)e;
 }
 
-}  // namespace
-
-extern "C" {
-
-int fp8_rmsnorm_quantize(const float* x, const void* residual_bf16, float* h_out, const float* gamma, uint8_t* q,
-                         float* scale_out, float* amax_out, float* rstd_ws, int rows, int hidden, float eps, void* stream) {
-    return rmsnorm_quantize(x, residual_bf16, h_out, residual_bf16 && h_out, gamma, q, scale_out, amax_out, rstd_ws, nullptr, rows, hidden, eps,
-                            (cudaStream_t)stream);
-}
-
-int fp8_rmsnorm_quantize_into(const float* x, float* h_out, const float* gamma, uint8_t* q, float* scale_out, float* amax_out, float* rstd_ws,
-                              float* zero_word, int rows, int hidden, float eps, void* stream) {
-    return rmsnorm_quantize(x, nullptr, h_out, h_out != nullptr, gamma, q, scale_out, amax_out, rstd_ws, zero_word, rows, hidden, eps,
-                            (cudaStream_t)stream);
-}
-
-int fp8_rope_quantize_qkv(const void* qkv_bf16, const float* cos_tab, const float* sin_tab, uint8_t* q_out, uint8_t* k_out,
-                          uint8_t* v_out, float* scales, float* amaxes, int batch, int seq_len, int heads, int head_dim,
-                          void* stream) {
-    QkvArgs a{};
-    a.qkv = reinterpret_cast<const uint16_t*>(qkv_bf16);
-    a.cos_tab = cos_tab; a.sin_tab = sin_tab; a.scales = scales; a.amaxes = amaxes;
-    a.q_out = q_out; a.k_out = k_out; a.v_out = v_out;
-    a.batch = batch; a.seq_len = seq_len; a.heads = heads; a.hd = head_dim;
-    return rope_quantize_qkv(a, (cudaStream_t)stream);
-}
-
-int fp8_rope_quantize_qkv_cache(const void* qkv_bf16, const float* cos_tab, const float* sin_tab, uint8_t* q_out, uint8_t* k_out,
-                                uint8_t* v_out, float* scales, float* amaxes, uint8_t* k_cache, uint8_t* v_cache, float* cache_scales,
-                                int32_t* cache_lens, int batch, int seq_len, int s_max, int heads, int head_dim, void* stream) {
-    if (!k_cache || !v_cache || !cache_scales || !cache_lens || s_max < seq_len || misaligned(k_cache) || misaligned(v_cache))
-        return (int)cudaErrorInvalidValue;
-    QkvArgs a{};
-    a.qkv = reinterpret_cast<const uint16_t*>(qkv_bf16);
-    a.cos_tab = cos_tab; a.sin_tab = sin_tab; a.scales = scales; a.amaxes = amaxes;
-    a.q_out = q_out; a.k_out = k_out; a.v_out = v_out;
-    a.k_cache = k_cache; a.v_cache = v_cache; a.cache_scales = cache_scales; a.cache_lens = cache_lens; a.s_max = s_max;
-    a.batch = batch; a.seq_len = seq_len; a.heads = heads; a.hd = head_dim;
-    return rope_quantize_qkv(a, (cudaStream_t)stream);
-}
-
-int fp8_decode_rope_append(const fp8_decode_append_args_t* g) {
+int append(const fp8_decode_append_args_t* g, bool cleared) {
     if (!g || !g->qkv_bf16 || !g->cos_tab || !g->sin_tab || !g->positions || !g->q_out || !g->q_scale_out || !g->q_amax_out ||
         !g->k_cache || !g->v_cache || !g->k_scale || !g->v_scale)
         return (int)cudaErrorInvalidValue;
@@ -1104,7 +1072,7 @@ int fp8_decode_rope_append(const fp8_decode_append_args_t* g) {
     a.cph = FastDiv(g->head_dim / 32);
     a.slots = FastDiv(slots);
     if (items * 64 <= OC_BYTES_DEC && oc_fits<DecOp>()) return (int)oc_launch(DecOp{a}, s);
-    cudaError_t e = clear_words(a.q_amax, 1, s);
+    cudaError_t e = cleared ? cudaSuccess : clear_words(a.q_amax, 1, s);
     if (e == cudaSuccess && items > 0) e = launch_pdl(dec_q_amax_kernel, dim3(grid_for(items)), dim3(THREADS), 0, s, a);
     if (e == cudaSuccess) e = launch_pdl(dec_append_kernel, dim3(grid_for(items)), dim3(THREADS), 0, s, a);
     if (e == cudaSuccess && a.seq_lens_out == a.positions && a.batch > 0)
@@ -1112,12 +1080,11 @@ int fp8_decode_rope_append(const fp8_decode_append_args_t* g) {
     return (int)e;
 }
 
-int fp8_permute_quantize_heads(const void* o_fp16, uint8_t* q, float* scale_out, float* amax_out, int batch, int seq_len,
-                               int heads, int head_dim, void* stream) {
+int permute_heads(const void* o_fp16, uint8_t* q, float* scale_out, float* amax_out, int batch, int seq_len, int heads, int head_dim, bool cleared,
+                  cudaStream_t s) {
     if (!o_fp16 || !q || !scale_out || !amax_out) return (int)cudaErrorInvalidValue;
     if (batch < 0 || seq_len <= 0 || heads <= 0 || head_dim <= 0 || (head_dim % 16) != 0) return (int)cudaErrorInvalidValue;
     if (misaligned(o_fp16) || misaligned(q)) return (int)cudaErrorInvalidValue;
-    cudaStream_t s = (cudaStream_t)stream;
     const size_t n16 = (size_t)batch * seq_len * heads * (head_dim / 16);
     if (n16 >= (1ull << 31)) return (int)cudaErrorInvalidValue;
     OArgs a{};
@@ -1128,10 +1095,48 @@ int fp8_permute_quantize_heads(const void* o_fp16, uint8_t* q, float* scale_out,
     a.dv.heads = FastDiv(heads);
     a.dv.seq = FastDiv(seq_len);
     if (n16 * 32 <= OC_BYTES_O && oc_fits<OOp>()) return (int)oc_launch(OOp{a}, s);
-    cudaError_t e = clear_words(amax_out, 1, s);
+    cudaError_t e = cleared ? cudaSuccess : clear_words(amax_out, 1, s);
     if (e == cudaSuccess && n16 > 0) e = launch_pdl(o_amax_kernel, dim3(grid_for(n16)), dim3(THREADS), 0, s, a);
     if (e == cudaSuccess) e = launch_pdl(o_quant_kernel, dim3(grid_for(n16)), dim3(THREADS), 0, s, a);
     return (int)e;
+}
+
+}  // namespace fp8_block
+
+extern "C" {
+
+int fp8_rmsnorm_quantize(const float* x, const void* residual_bf16, float* h_out, const float* gamma, uint8_t* q,
+                         float* scale_out, float* amax_out, float* rstd_ws, int rows, int hidden, float eps, void* stream) {
+    return fp8_block::rmsnorm(x, residual_bf16, h_out, residual_bf16 && h_out, gamma, q, scale_out, amax_out, rstd_ws, {}, rows, hidden, eps,
+                              (cudaStream_t)stream);
+}
+
+int fp8_rmsnorm_quantize_into(const float* x, float* h_out, const float* gamma, uint8_t* q, float* scale_out, float* amax_out, float* rstd_ws,
+                              float* zero_word, int rows, int hidden, float eps, void* stream) {
+    return fp8_block::rmsnorm(x, nullptr, h_out, h_out != nullptr, gamma, q, scale_out, amax_out, rstd_ws, {zero_word, zero_word ? 1 : 0, false},
+                              rows, hidden, eps, (cudaStream_t)stream);
+}
+
+int fp8_rope_quantize_qkv(const void* qkv_bf16, const float* cos_tab, const float* sin_tab, uint8_t* q_out, uint8_t* k_out,
+                          uint8_t* v_out, float* scales, float* amaxes, int batch, int seq_len, int heads, int head_dim,
+                          void* stream) {
+    return fp8_block::rope_qkv({qkv_bf16, cos_tab, sin_tab, q_out, k_out, v_out, scales, amaxes, nullptr, nullptr, nullptr, nullptr, batch, seq_len, 0,
+                                heads, head_dim}, false, (cudaStream_t)stream);
+}
+
+int fp8_rope_quantize_qkv_cache(const void* qkv_bf16, const float* cos_tab, const float* sin_tab, uint8_t* q_out, uint8_t* k_out,
+                                uint8_t* v_out, float* scales, float* amaxes, uint8_t* k_cache, uint8_t* v_cache, float* cache_scales,
+                                int32_t* cache_lens, int batch, int seq_len, int s_max, int heads, int head_dim, void* stream) {
+    if (!k_cache || !v_cache || !cache_scales || !cache_lens || s_max < seq_len) return (int)cudaErrorInvalidValue;
+    return fp8_block::rope_qkv({qkv_bf16, cos_tab, sin_tab, q_out, k_out, v_out, scales, amaxes, k_cache, v_cache, cache_scales, cache_lens, batch, seq_len,
+                                s_max, heads, head_dim}, false, (cudaStream_t)stream);
+}
+
+int fp8_decode_rope_append(const fp8_decode_append_args_t* g) { return fp8_block::append(g, false); }
+
+int fp8_permute_quantize_heads(const void* o_fp16, uint8_t* q, float* scale_out, float* amax_out, int batch, int seq_len,
+                               int heads, int head_dim, void* stream) {
+    return fp8_block::permute_heads(o_fp16, q, scale_out, amax_out, batch, seq_len, heads, head_dim, false, (cudaStream_t)stream);
 }
 
 int fp8_swiglu_quantize(const void* gate_up_bf16, uint8_t* q, float* scale_out, float* amax_out, int rows, int ffn_hidden,

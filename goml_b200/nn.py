@@ -16,6 +16,7 @@ torch tensors are used as device buffers; all heavy kernels are reached through 
 """
 from __future__ import annotations
 
+import ctypes
 import math
 
 import torch
@@ -146,6 +147,19 @@ def _scratch(dev, *sizes):
     return (buf, *[base + o for o in offsets])
 
 
+_entries = None
+
+
+def _entry_points():
+    """Addresses of the library entry points that fp8_block_run calls."""
+    global _entries
+    if _entries is None:
+        gemm, fa = G._init(), F.FALoad()
+        _entries = tuple(ctypes.cast(fn, ctypes.c_void_p).value for fn in (gemm.fp8_gemm_scaled, gemm.fp8_gemm_accumulate_f32, gemm.fp8_gemm_swiglu_raise,
+                                                                           fa.fa_forward_ex, fa.fa_decode))
+    return _entries
+
+
 def _stream_start(x: torch.Tensor, rows: int, d: int):
     """(source, h) of a block's residual stream: h is written by the first RMSNorm while it reads x, or is a copy already
     (source = h) where x is not what that kernel reads.  The kernels behind it address h as rows of d values without gaps, so
@@ -195,75 +209,69 @@ class FP8DecoderBlock:
             self._rope[S] = (cos, sin)
         return self._rope[S]
 
+    def _run(self, x: torch.Tensor, B: int, S: int, tables: int, cache: "FP8KVCache | None", decode: bool):
+        """The block's library calls (fp8_block_run): the new stream, and the scratch with the addresses of the prompt's K and V
+        codes and of their scales."""
+        T, d, H, Fh = B * S, self.d, self.H, self.F
+        n = T * d
+        up = lambda size: (size + 255) & -256
+        # what the attention half needs (projections, Q codes, attention output, its codes) and then the feed-forward half
+        # (activations, their codes) in the same place
+        region_bytes = max(up(6 * n) + 2 * up(n) + up(2 * n), up(2 * T * Fh) + up(T * Fh))
+        kv = 0 if decode else n
+        buf, words, rstd, codes, kc, vc, region = _scratch(x.device, 256, 4 * T, n, kv, kv, region_bytes)
+        src, h = _stream_start(x, T, d)                         # residual stream, updated in place
+        cos, sin = self.rope_tables(tables, x.device)
+        if not self.fa.ptr:
+            raise F.FAError("FP8DecoderBlock: nil ctx", F.FA_ERR_INVALID_ARG)
+        gemm, accumulate, swiglu, forward, step = _entry_points()
+        k = v = ks = lens = s_max = 0
+        if cache is not None:
+            k, v, ks, lens, s_max = cache.k.data_ptr(), cache.v.data_ptr(), cache.scales.data_ptr(), cache.lens.data_ptr(), cache.s_max
+        qkv, o, gate_up, down = self.qkv.w, self.o.w, self.gate_up.w, self.down.w
+        rc = BG.BlockRun(gemm, accumulate, swiglu, step if decode else forward, self.fa.ptr, src.data_ptr(), h.data_ptr(), self.norm1.data_ptr(),
+                         self.norm2.data_ptr(), qkv.codes.data_ptr(), o.codes.data_ptr(), self.gate_up_interleaved.data_ptr(), down.codes.data_ptr(),
+                         qkv.scale_ptr, o.scale_ptr, gate_up.scale_ptr, down.scale_ptr, cos.data_ptr(), sin.data_ptr(), k, v, ks, lens,
+                         words, rstd, codes, kc, vc, region, region_bytes, torch.cuda.current_stream().cuda_stream,
+                         B, S, d, H, Fh, s_max, tables, int(decode), self.eps, 1.0 / math.sqrt(self.hd))
+        if rc:
+            self._raise(rc)
+        return h, buf, kc, vc, words + 72
+
+    def _raise(self, rc: int) -> None:
+        """The error of the library call that fp8_block_run stopped at, as its own binding raises it."""
+        place, code = rc >> 16, rc & 0xffff
+        if place == 4:
+            raise F.FAError("attention", code, self.fa._msg())
+        name = ("fp8_block_run", "fp8_rmsnorm_quantize_into", "fp8_gemm_scaled", "fp8_rope_quantize_qkv", "", "fp8_permute_quantize_heads",
+                "fp8_gemm_accumulate_f32", "fp8_rmsnorm_quantize_into", "fp8_gemm_swiglu_raise", "fp8_quantize_bf16", "fp8_gemm_accumulate_f32")[place]
+        if name.startswith("fp8_gemm"):
+            raise G.FP8GEMMError(f"{name}: CUDA error {code}")
+        raise BG.BlockGlueError(f"{name}: CUDA error {code}")
+
     def forward_fused(self, x: torch.Tensor, B: int, S: int, cache: "FP8KVCache | None" = None) -> torch.Tensor:
         """The block with every glue op fused with the quantiser of its consumer and both residual adds done in
-        the GEMM epilogues, SwiGLU in the gate/up GEMM's epilogue: 9 library calls, no torch math.
+        the GEMM epilogues, SwiGLU in the gate/up GEMM's epilogue: 10 library calls, issued in native code, no torch math.
         With `cache`, the K and V codes of the prompt and their scales are also stored there for decode_step."""
-        T, d, H, hd = B * S, self.d, self.H, self.hd
-        sh = torch.cuda.current_stream().cuda_stream
-        n = T * d
-        # codes of the normed input, QKV projection, codes of Q, K and V, attention output, its codes, rstd, scales and maxima
-        buf, xc, qkv, qc, kc, vc, o, oc, rstd, sc = _scratch(x.device, n, 6 * n, n, n, n, 2 * n, n, 4 * T, 40)
-        src, h = _stream_start(x, T, d)                         # residual stream, updated in place
-        cos, sin = self.rope_tables(S, x.device)
-        # attention half
-        BG.RMSNormQuantizeInto(src.data_ptr(), h.data_ptr(), self.norm1.data_ptr(), xc, sc, sc + 4, rstd, 0, T, d, self.eps, sh)
-        G.FP8GEMMScaled(T, 3 * d, d, xc, self.qkv.w.codes.data_ptr(), qkv, 1.0, sc, self.qkv.w.scale_ptr, G.OutBF16, sh)   # [T, 3, H, hd] bf16
-        s3 = sc + 8                                             # scales[3], amaxes[3]
-        if _writes_directly(cache, B, H, S, hd, x.device):
-            BG.RopeQuantizeQKVCache(qkv, cos.data_ptr(), sin.data_ptr(), qc, kc, vc, s3, s3 + 12, cache.k.data_ptr(), cache.v.data_ptr(),
-                                    cache.scales.data_ptr(), cache.lens.data_ptr(), B, S, cache.s_max, H, hd, sh)
-        else:
-            BG.RopeQuantizeQKV(qkv, cos.data_ptr(), sin.data_ptr(), qc, kc, vc, s3, s3 + 12, B, S, H, hd, sh)
-            if cache is not None:
-                view = lambda p, nbytes: buf[p - buf.data_ptr():p - buf.data_ptr() + nbytes]
-                cache.fill(view(kc, n), view(vc, n), view(s3 + 4, 8).view(torch.float32), S)
-        self.fa.ForwardEx(qc, kc, vc, o, 0, B * H, S, hd, 1, 0, 1.0 / math.sqrt(hd), 1.0, s3, s3 + 4, s3 + 8, sh)
-        BG.PermuteQuantizeHeads(o, oc, sc + 32, sc + 36, B, S, H, hd, sh)
-        # h += attention projection, in the GEMM epilogue
-        G.FP8GEMMAccumulateF32(T, d, d, oc, self.o.w.codes.data_ptr(), h.data_ptr(), 1.0, sc + 32, self.o.w.scale_ptr, sh)
-        del buf   # the feed-forward half may take its place: same stream
-        return self._feed_forward(h, T)
+        direct = _writes_directly(cache, B, self.H, S, self.hd, x.device)
+        h, buf, kc, vc, kv_scales = self._run(x, B, S, S, cache if direct else None, False)
+        if cache is not None and not direct:
+            view = lambda p, nbytes: buf[p - buf.data_ptr():p - buf.data_ptr() + nbytes]
+            n = B * S * self.d
+            cache.fill(view(kc, n), view(vc, n), view(kv_scales, 8).view(torch.float32), S)
+        return h
 
     def decode_step(self, x: torch.Tensor, cache: FP8KVCache) -> torch.Tensor:
         """One new token per sequence: x [batch, d] fp32 -> [batch, d] fp32, the token's K and V appended to `cache` at
         position cache.lens[b] (quantised with the cache's scales) and cache.lens advanced.  Ten library calls:
         RMSNorm+quantise -> QKV GEMM -> RoPE+quantise+append -> decode attention -> quantise -> O GEMM (residual in the
         epilogue) -> the feed-forward half of forward_fused."""
-        B, d, H, hd = x.shape[0], self.d, self.H, self.hd
-        assert (B, H, hd) == (cache.B, cache.H, cache.hd)
+        B = x.shape[0]
+        assert (B, self.H, self.hd) == (cache.B, cache.H, cache.hd)
         if not cache.dense_on(x.device):
             raise ValueError(f"decode_step: the cache's buffers must lie without gaps, in the shapes it was made with, on {x.device}")
-        sh = torch.cuda.current_stream().cuda_stream
-        n = B * d
-        buf, xc, qkv, qc, o, oc, rstd, sc = _scratch(x.device, n, 6 * n, n, 2 * n, n, 4 * B, 24)
-        src, h = _stream_start(x, B, d)
-        cos, sin = self.rope_tables(cache.s_max, x.device)
-        BG.RMSNormQuantizeInto(src.data_ptr(), h.data_ptr(), self.norm1.data_ptr(), xc, sc, sc + 4, rstd, 0, B, d, self.eps, sh)
-        # [B, (H + 2H) * hd] bf16: Q heads, K heads, V heads
-        G.FP8GEMMScaled(B, 3 * d, d, xc, self.qkv.w.codes.data_ptr(), qkv, 1.0, sc, self.qkv.w.scale_ptr, G.OutBF16, sh)
-        k, v, lens, ks = cache.k.data_ptr(), cache.v.data_ptr(), cache.lens.data_ptr(), cache.scales.data_ptr()
         # the lengths advance in place, on the device: the step can be replayed from a CUDA graph
-        BG.DecodeRopeAppend(qkv, cos.data_ptr(), sin.data_ptr(), lens, qc, sc + 8, sc + 12, k, v, ks, ks + 4, B, H, H, hd,
-                            cache.s_max, cache.s_max, seq_lens_out=lens, stream=sh)
-        self.fa.Decode(qc, k, v, o, 0, lens, B, H, H, hd, cache.s_max, 0, 1.0 / math.sqrt(hd), 1.0, sc + 8, ks, ks + 4, sh)
-        BG.PermuteQuantizeHeads(o, oc, sc + 16, sc + 20, B, 1, H, hd, sh)
-        G.FP8GEMMAccumulateF32(B, d, d, oc, self.o.w.codes.data_ptr(), h.data_ptr(), 1.0, sc + 16, self.o.w.scale_ptr, sh)
-        del buf
-        return self._feed_forward(h, B)
-
-    def _feed_forward(self, h: torch.Tensor, T: int) -> torch.Tensor:
-        """h [T, d] fp32 += W_down(silu(W_gate n) * W_up n), n = RMSNorm(h): in place, three GEMM-library calls."""
-        d, Fh = self.d, self.F
-        sh = torch.cuda.current_stream().cuda_stream
-        buf, xc, hb, hc, rstd, sc = _scratch(h.device, T * d, 2 * T * Fh, T * Fh, 4 * T, 16)
-        # the norm zeroes the word that the gate/up epilogue raises max|.| in
-        BG.RMSNormQuantizeInto(h.data_ptr(), 0, self.norm2.data_ptr(), xc, sc, sc + 4, rstd, sc + 12, T, d, self.eps, sh)
-        # gate/up projections with silu(gate) * up and max|.| in the GEMM epilogue, then one quantiser pass
-        G.FP8GEMMSwiGLURaise(T, Fh, d, xc, self.gate_up_interleaved.data_ptr(), hb, 1.0, sc, self.gate_up.w.scale_ptr, sc + 12, sh)
-        BG.QuantizeBF16(hb, hc, sc + 8, sc + 12, T * Fh, sh)
-        G.FP8GEMMAccumulateF32(T, d, Fh, hc, self.down.w.codes.data_ptr(), h.data_ptr(), 1.0, sc + 8, self.down.w.scale_ptr, sh)   # h += feed-forward output
-        return h
+        return self._run(x, B, 1, cache.s_max, cache, True)[0]
 
     def __call__(self, x: torch.Tensor, B: int, S: int, cache: "FP8KVCache | None" = None) -> torch.Tensor:
         """x [B*S, d] fp32 -> [B*S, d] fp32."""

@@ -35,6 +35,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "fa_sm120.h"
+
 #ifdef __cplusplus
 extern "C" {
 #endif
@@ -143,6 +145,46 @@ typedef struct fp8_decode_append_args {
 } fp8_decode_append_args_t;
 
 FP8BLOCK_API int fp8_decode_rope_append(const fp8_decode_append_args_t* args);
+
+/* A whole decoder block as one call: the sequence of library calls of a prompt (decode = 0: h = x + O(attention), then
+ * h += W_down(silu(W_gate n) * W_up n), n the RMSNorm of h) or of one new token per sequence (decode = 1, seq_len 1: K and V
+ * appended to the cache at cache_lens, which advances in place), issued in native code.
+ * The GEMM and attention entry points come as function pointers, so this library links to neither of the others:
+ * fp8_gemm_scaled, fp8_gemm_accumulate_f32, fp8_gemm_swiglu_raise, and fa_forward_ex (prompt) or fa_decode with its context.
+ *   x, h     [batch*seq_len, d_model] fp32: input and output stream; h may be x (then it is updated in place);
+ *   w*       e4m3 weights and their device scales; wgate_up interleaved as fp8_gemm_swiglu reads it; norm1, norm2 fp32;
+ *   cos_tab, sin_tab  [rope_rows, d_model/heads/2] (at least seq_len rows for a prompt, s_max for a step);
+ *   k_cache ... s_max  the KV cache [batch, heads, s_max, head_dim]; for a prompt it may be NULL;
+ * and scratch of the caller: words (64 floats), rstd (batch*seq_len floats), codes (batch*seq_len*d_model bytes, 16-byte aligned),
+ * k_codes, v_codes (the same; a prompt's K and V codes, left there with their scales in words[18], words[19]), region
+ * (fp8_block_region_bytes, 256-byte aligned).
+ * Returns 0, or (place of the call in the sequence, from 1) << 16 | its error; errors of fp8_block_run's own arguments have place 0. */
+typedef struct fp8_block_run_args {
+    int (*gemm_scaled)(int, int, int, const void*, const void*, void*, float, const float*, const float*, int, void*);
+    int (*gemm_accumulate_f32)(int, int, int, const void*, const void*, float*, float, const float*, const float*, void*);
+    int (*gemm_swiglu_raise)(int, int, int, const void*, const void*, void*, float, const float*, const float*, float*, void*);
+    int (*attention)(void* ctx, const void* args);
+    void* attention_ctx;
+    const float* x;
+    float* h;
+    const float *norm1, *norm2;
+    const uint8_t *wqkv, *wo, *wgate_up, *wdown;
+    const float *wqkv_scale, *wo_scale, *wgate_up_scale, *wdown_scale;
+    const float *cos_tab, *sin_tab;
+    uint8_t *k_cache, *v_cache;
+    float* cache_scales;
+    int32_t* cache_lens;
+    float* words;
+    float* rstd;
+    uint8_t *codes, *k_codes, *v_codes, *region;
+    size_t region_bytes;
+    void* stream;
+    int32_t batch, seq_len, d_model, heads, ffn_hidden, s_max, rope_rows, decode;
+    float eps, softmax_scale;
+} fp8_block_run_args_t;
+
+FP8BLOCK_API size_t fp8_block_region_bytes(int rows, int d_model, int ffn_hidden);
+FP8BLOCK_API int fp8_block_run(const fp8_block_run_args_t* args);
 
 #ifdef __cplusplus
 }
