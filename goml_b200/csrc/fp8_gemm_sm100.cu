@@ -200,6 +200,10 @@ fp8_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    // overlapped with the kernel ahead up to here (barriers, tensor memory, descriptors), usually the quantiser of A: 1.5 to 2 us
+    // between the two, and as much to the kernel behind (8 x 2048 tokens of a block: eight such gaps)
+    pdl_wait();
+    pdl_trigger();
 
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer
@@ -296,12 +300,12 @@ fp8_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         const int quad = warp & 3;                 // TMEM lane quadrant this warp may read
         const int row_in_tile = quad * 32 + lane;  // TMEM lane = row of the tile
         float alpha = p.alpha;
-        if (p.scale_a) alpha *= __ldg(p.scale_a);
-        if (p.scale_b) alpha *= __ldg(p.scale_b);
+        if (p.scale_a) alpha *= ld_f32(p.scale_a);
+        if (p.scale_b) alpha *= ld_f32(p.scale_b);
         const bool vec_ok = (p.N % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
         const bool xvec_ok = (p.N % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.X) & 15) == 0);
         const bool dvec_ok = (p.N % 16 == 0) && ((reinterpret_cast<uintptr_t>(p.D8) & 15) == 0);
-        const float scale_d = (p.D8 && p.scale_d) ? __ldg(p.scale_d) : 1.0f;
+        const float scale_d = (p.D8 && p.scale_d) ? ld_f32(p.scale_d) : 1.0f;
         uint32_t tphase[2] = {0, 0};
         int buf = 0;
         int sbuf = 0;  // staging box in use (accumulate mode)
@@ -758,11 +762,11 @@ int launch(int M, int N, int K, const void* A, const void* B, void* C, float alp
     if (p.d_tma && !make_tmap_u8_2d(&tx, D8, (uint64_t)M, (uint64_t)N, 32, 128, CU_TENSOR_MAP_SWIZZLE_128B)) return (int)cudaErrorInvalidValue;
 
     const int grid = (int)(p.num_units < st.num_sms ? p.num_units : st.num_sms);
-    if (pair) fp8_gemm_tcgen05_kernel<256, 2><<<grid, NUM_THREADS, Tile<256, 2>::SMEM_BYTES, stream>>>(ta, tb, tbh, tx, p);
-    else if (bn == 256) fp8_gemm_tcgen05_kernel<256><<<grid, NUM_THREADS, Tile<256>::SMEM_BYTES, stream>>>(ta, tb, tbh, tx, p);
-    else if (bn == 128) fp8_gemm_tcgen05_kernel<128><<<grid, NUM_THREADS, Tile<128>::SMEM_BYTES, stream>>>(ta, tb, tbh, tx, p);
-    else fp8_gemm_tcgen05_kernel<64><<<grid, NUM_THREADS, Tile<64>::SMEM_BYTES, stream>>>(ta, tb, tbh, tx, p);
-    return (int)cudaGetLastError();
+    auto start = [&](auto kernel, size_t smem) { return (int)launch_pdl(kernel, dim3(grid), dim3(NUM_THREADS), smem, stream, ta, tb, tbh, tx, p); };
+    if (pair) return start(fp8_gemm_tcgen05_kernel<256, 2>, Tile<256, 2>::SMEM_BYTES);
+    if (bn == 256) return start(fp8_gemm_tcgen05_kernel<256>, Tile<256>::SMEM_BYTES);
+    if (bn == 128) return start(fp8_gemm_tcgen05_kernel<128>, Tile<128>::SMEM_BYTES);
+    return start(fp8_gemm_tcgen05_kernel<64>, Tile<64>::SMEM_BYTES);
 }
 
 }  // namespace
