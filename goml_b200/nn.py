@@ -41,7 +41,7 @@ def quantize(x: torch.Tensor, unit: bool = False) -> FP8Tensor:
     x = x.contiguous()
     assert x.dtype == torch.float32 and x.is_cuda
     codes = torch.empty(x.shape, dtype=torch.uint8, device=x.device)
-    sa = torch.zeros(2, dtype=torch.float32, device=x.device)
+    sa = torch.empty(2, dtype=torch.float32, device=x.device)   # both written by the quantiser
     fn = Q.QuantizeF32ToF8E4M3Unit if unit else Q.QuantizeF32ToF8E4M3
     fn(x.data_ptr(), codes.data_ptr(), sa.data_ptr(), sa.data_ptr() + 4, x.numel(), torch.cuda.current_stream().cuda_stream)
     return FP8Tensor(codes, sa)
