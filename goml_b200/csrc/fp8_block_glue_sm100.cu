@@ -1001,17 +1001,17 @@ int rmsnorm(const float* x, const void* residual_bf16, float* h_out, bool store_
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const dim3 grid(rows < sms * 8 ? rows : sms * 8), block(THREADS);
 #define RMS_STATS_REGS(N)                                                                                                        \
-    (res ? launch_pdl_stream<rms_stats_regs_kernel<N, true>>(grid, block, s, x, res, h, gamma, rstd_ws, amax_out, rows, eps) \
-         : launch_pdl_stream<rms_stats_regs_kernel<N, false>>(grid, block, s, x, res, h, gamma, rstd_ws, amax_out, rows, eps))
+    (res ? launch_pdl_stream(items * 64, rms_stats_regs_kernel<N, true>, grid, block, s, x, res, h, gamma, rstd_ws, amax_out, rows, eps) \
+         : launch_pdl_stream(items * 64, rms_stats_regs_kernel<N, false>, grid, block, s, x, res, h, gamma, rstd_ws, amax_out, rows, eps))
         if (hidden == 2048) e = RMS_STATS_REGS(1);
         else if (hidden == 4096) e = RMS_STATS_REGS(2);
         else if (hidden == 8192) e = RMS_STATS_REGS(4);
-        else e = launch_pdl_stream<rms_stats_kernel>(grid, block, s, x, res, h, gamma, rstd_ws, amax_out, rows, hidden, eps);
+        else e = launch_pdl_stream(items * 64, rms_stats_kernel, grid, block, s, x, res, h, gamma, rstd_ws, amax_out, rows, hidden, eps);
 #undef RMS_STATS_REGS
         if (e != cudaSuccess) return (int)e;
     }
     // pass 2 reads the stream where pass 1 stored it
-    return (int)launch_pdl_stream<rms_quant_kernel>(dim3(grid_for(items)), dim3(THREADS), s, h ? h : x, h ? nullptr : res, gamma, rstd_ws,
+    return (int)launch_pdl_stream(items * 64, rms_quant_kernel, dim3(grid_for(items)), dim3(THREADS), s, h ? h : x, h ? nullptr : res, gamma, rstd_ws,
                            amax_out, scale_out, q, (uint32_t)items, hidden, FastDiv(hidden / 16));
 }
 
@@ -1036,8 +1036,8 @@ int rope_qkv(const Rope& r, bool cleared, cudaStream_t s) {
     a.dv.seq = FastDiv(a.seq_len);
     if (items * 64 <= OC_BYTES_QKV && oc_fits<QkvOp>()) return (int)oc_launch(QkvOp{a}, s);
     cudaError_t e = cleared ? cudaSuccess : clear_words(a.amaxes, 3, s);
-    if (e == cudaSuccess && items > 0) e = launch_pdl_stream<qkv_amax_kernel>(dim3(grid_for(items)), dim3(THREADS), s, a);
-    if (e == cudaSuccess) e = launch_pdl_stream<qkv_quant_kernel>(dim3(grid_for(items)), dim3(THREADS), s, a);
+    if (e == cudaSuccess && items > 0) e = launch_pdl_stream(items * 64, qkv_amax_kernel, dim3(grid_for(items)), dim3(THREADS), s, a);
+    if (e == cudaSuccess) e = launch_pdl_stream(items * 64, qkv_quant_kernel, dim3(grid_for(items)), dim3(THREADS), s, a);
     return (int)e;
 }
 
@@ -1096,8 +1096,8 @@ int permute_heads(const void* o_fp16, uint8_t* q, float* scale_out, float* amax_
     a.dv.seq = FastDiv(seq_len);
     if (n16 * 32 <= OC_BYTES_O && oc_fits<OOp>()) return (int)oc_launch(OOp{a}, s);
     cudaError_t e = cleared ? cudaSuccess : clear_words(amax_out, 1, s);
-    if (e == cudaSuccess && n16 > 0) e = launch_pdl_stream<o_amax_kernel>(dim3(grid_for(n16)), dim3(THREADS), s, a);
-    if (e == cudaSuccess) e = launch_pdl_stream<o_quant_kernel>(dim3(grid_for(n16)), dim3(THREADS), s, a);
+    if (e == cudaSuccess && n16 > 0) e = launch_pdl_stream(n16 * 32, o_amax_kernel, dim3(grid_for(n16)), dim3(THREADS), s, a);
+    if (e == cudaSuccess) e = launch_pdl_stream(n16 * 32, o_quant_kernel, dim3(grid_for(n16)), dim3(THREADS), s, a);
     return (int)e;
 }
 
@@ -1158,7 +1158,7 @@ int fp8_swiglu_quantize(const void* gate_up_bf16, uint8_t* q, float* scale_out, 
 
 int fp8_quantize_bf16(const void* x_bf16, uint8_t* q, float* scale_out, const float* amax_in, size_t n, void* stream) {
     if (!x_bf16 || !q || !scale_out || !amax_in || (n % 16) != 0 || misaligned32(x_bf16) || misaligned(q)) return (int)cudaErrorInvalidValue;
-    return (int)launch_pdl_stream<quant_bf16_kernel>(dim3(grid_for(n / 32 + 1)), dim3(THREADS), (cudaStream_t)stream,
+    return (int)launch_pdl_stream(n * 2, quant_bf16_kernel, dim3(grid_for(n / 32 + 1)), dim3(THREADS), (cudaStream_t)stream,
                            reinterpret_cast<const uint16_t*>(x_bf16), amax_in, scale_out, q, n / 16);
 }
 

@@ -25,7 +25,6 @@ constexpr int W_BYTES = W_ROWS * BK;        // of one k-block
 constexpr int MAX_TOKENS = 192;
 constexpr int MAX_STAGES = 16;
 constexpr int MAX_SPLIT = 8;                // portable cluster size
-constexpr int PREFETCH_BLOCKS = 16;         // k-blocks per CTA asked for ahead of the wait
 constexpr int THREADS = 192;                // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2-5: read the accumulators back
 constexpr int TAIL_BYTES = 1024 /*align*/ + 512 /*barriers*/;
 constexpr int SMEM_ONE = 227 * 1024;        // of one CTA when it has the SM to itself
@@ -38,6 +37,7 @@ struct Params {
     int tmem_cols;
     uint32_t idesc;
     int stages;
+    int prefetch;      // k-blocks per CTA asked for ahead of the wait
     int vec;           // four neighbouring outputs of a token may be stored at once
 };
 
@@ -102,7 +102,7 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     }
     __syncwarp();
     if (warp == 0) {
-        const int pf1 = min(kb1, kb0 + PREFETCH_BLOCKS);
+        const int pf1 = min(kb1, kb0 + p.prefetch);
         for (int kb = kb0 + lane; kb < pf1; kb += 32) prefetch_l2_2d(&tmap_w, kb * BK, n0);
         __syncwarp();
     } else if (warp == 1) {
@@ -434,7 +434,15 @@ inline int launch(GemmParams g, const Plan& plan, const void* A, const void* B, 
     if (p.stages > slice) p.stages = slice;
     if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
     int ring_bytes = p.stages * stage_bytes;
-    while (ring_bytes < part_bytes) { p.stages++; ring_bytes += stage_bytes; }   // the partial sums take the ring's place
+    // How much of the weight is asked for ahead of the wait.  It helps as far as memory is idle until then; past that a CTA's first
+    // loads stand behind hints for its last ones.  Half of a CTA's blocks up to 16 (all of up to 8), with several CTAs to an SM no more than 20 MB in
+    // all, and four blocks past 80 tokens, whose first loads bring as much again in tokens, which no hint has fetched.  All / as
+    // here, us: 22016 x 4096 with SwiGLU, 1 token 19.4 / 18.0, 40 tokens 21.4 / 19.3; 12288 x 4096 10.8 / 10.4; 4096 x 11008
+    // 11.2 / 10.8, 173 tokens 16.7 / 16.1; a block over 40 tokens 83.2 / 80.2, a step of one sequence 79.9 / 78.3.
+    p.prefetch = slice <= 8 ? slice : (slice + 1) / 2;
+    if (plan.per_sm > 1 && p.prefetch > (20 << 20) / (W_BYTES * tiles * plan.split)) p.prefetch = (20 << 20) / (W_BYTES * tiles * plan.split);
+    if (p.prefetch > 16) p.prefetch = 16;
+    if (g.M > 80) p.prefetch = 4;
     p.vec = g.H ? (g.F % 4 == 0 && (reinterpret_cast<uintptr_t>(g.H) & 7) == 0)
           : g.X ? (g.N % 4 == 0 && (reinterpret_cast<uintptr_t>(g.X) & 15) == 0)
           : g.D8 ? (g.N % 4 == 0 && (reinterpret_cast<uintptr_t>(g.D8) & 3) == 0)

@@ -282,8 +282,8 @@ int quantize_f32(const float* x, uint8_t* q, float* scale_out, float* amax_out, 
     // the first pass to that of the GEMM behind the second 26.2 -> 18.4 us, 2 of them the GEMM's earlier start.
     const dim3 grid(grid_for(n / (8 * BATCH) + 1, 32));
     cudaError_t e = launch_pdl(clear_word_kernel, dim3(1), dim3(1), 0, s, amax_out);
-    if (e == cudaSuccess) e = launch_pdl_stream<amax_kernel<WIDE>>(grid, dim3(THREADS), s, x, n, amax_out);
-    if (e == cudaSuccess) e = launch_pdl_stream<quant_kernel<WIDE>>(grid, dim3(THREADS), s, x, q, n, amax_out, scale_out, divisor);
+    if (e == cudaSuccess) e = launch_pdl_stream(n * 4, amax_kernel<WIDE>, grid, dim3(THREADS), s, x, n, amax_out);
+    if (e == cudaSuccess) e = launch_pdl_stream(n * 4, quant_kernel<WIDE>, grid, dim3(THREADS), s, x, q, n, amax_out, scale_out, divisor);
     return (int)e;
 }
 

@@ -20,8 +20,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <atomic>
-
 namespace sm100 {
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -64,20 +62,24 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// The same for a kernel that streams memory behind one that takes most of an SM's shared memory.  Launched early it would find the
-// SM's storage given to shared memory, and loads in flight need lines of what is left: 28 KB hold it to two thirds of the
-// memory's rate (and the kernels behind it, as long as no SM runs empty).  Asking for L1 keeps its CTAs off an SM until that can be had.
-template <auto KERNEL, typename... Args>
-inline cudaError_t launch_pdl_stream(dim3 grid, dim3 block, cudaStream_t stream, Args&&... args) {
-    static std::atomic<bool> known[64];
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < 64 && !known[dev].load(std::memory_order_acquire)) {
-        if ((e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1)) != cudaSuccess) return e;
-        known[dev].store(true, std::memory_order_release);
-    }
-    return launch_pdl(KERNEL, grid, block, 0, stream, static_cast<Args&&>(args)...);
+// The same for a kernel that streams `bytes`.  Launched early behind one that takes most of an SM's shared memory it would find the
+// SM's storage given to that, and loads in flight need lines of what is left: 28 KB hold it to two thirds of the memory's
+// rate (and the kernels behind it, as long as no SM runs empty).  A large one asks for L1, which keeps its CTAs off an SM until
+// that can be had; for a small one being there early is worth more (16384 rows behind a GEMM 111 -> 79 us, 16 rows 1 us slower).
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl_stream(size_t bytes, void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t stream, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[1].val.sharedMemCarveout = cudaSharedmemCarveoutMaxL1;
+    cfg.attrs = attr;
+    cfg.numAttrs = bytes >= ((size_t)16 << 20) ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
 }  // namespace sm100
