@@ -41,7 +41,7 @@ class DecodeAppendArgs(C.Structure):
 class BlockRunArgs(C.Structure):
     """fp8_block_run_args_t (include/fp8_block.h)."""
     _fields_ = ([(name, C.c_void_p) for name in (
-        "gemm_scaled", "gemm_accumulate_f32", "gemm_swiglu_raise", "attention", "attention_ctx", "x", "h", "norm1", "norm2",
+        "gemm_scaled", "gemm_accumulate_f32", "gemm_swiglu_raise", "attention_raise", "attention_decode", "attention_ctx", "x", "h", "norm1", "norm2",
         "wqkv", "wo", "wgate_up", "wdown", "wqkv_scale", "wo_scale", "wgate_up_scale", "wdown_scale", "cos_tab", "sin_tab",
         "k_cache", "v_cache", "cache_scales", "cache_lens", "words", "rstd", "codes", "k_codes", "v_codes", "region")]
         + [("region_bytes", C.c_size_t), ("stream", C.c_void_p)]
@@ -49,8 +49,8 @@ class BlockRunArgs(C.Structure):
         + [("eps", C.c_float), ("softmax_scale", C.c_float)])
 
 
-_PACK_RUN = struct.Struct("@29PNP8i2f").pack
-assert struct.calcsize("@29PNP8i2f") == C.sizeof(BlockRunArgs)
+_PACK_RUN = struct.Struct("@30PNP8i2f").pack
+assert struct.calcsize("@30PNP8i2f") == C.sizeof(BlockRunArgs)
 
 
 def BlockRun(*args) -> int:

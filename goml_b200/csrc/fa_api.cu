@@ -391,10 +391,10 @@ fa_status_t fa_forward(fa_ctx_t* ctx, const void* q, const void* k, const void* 
     return run(ctx, "fa_forward", a);
 }
 
-fa_status_t fa_forward_ex(fa_ctx_t* ctx, const fa_forward_args_t* g) {
+static fa_status_t forward_ex(fa_ctx_t* ctx, const fa_forward_args_t* g, float* o_amax, const char* who) {
     if (!ctx) return FA_ERR_INVALID_ARG;
-    if (!g) { set_err(ctx, "%s: null argument block", "fa_forward_ex"); return FA_ERR_INVALID_ARG; }
-    fa_status_t s = validate(ctx, "fa_forward_ex", g->q, g->k, g->v, g->o, g->batch_heads, g->seq_len, g->head_dim,
+    if (!g) { set_err(ctx, "%s: null argument block", who); return FA_ERR_INVALID_ARG; }
+    fa_status_t s = validate(ctx, who, g->q, g->k, g->v, g->o, g->batch_heads, g->seq_len, g->head_dim,
                              g->causal, g->window, g->l_out);
     if (s != FA_OK) return s;
     fa_sm100::LaunchArgs a{};
@@ -403,7 +403,18 @@ fa_status_t fa_forward_ex(fa_ctx_t* ctx, const fa_forward_args_t* g) {
     a.scale = g->scale; a.v_descale = (g->v_descale == 0.0f) ? 1.0f : g->v_descale;
     a.scale_q_dev = g->scale_q_dev; a.scale_k_dev = g->scale_k_dev; a.scale_v_dev = g->scale_v_dev;
     a.stream = reinterpret_cast<cudaStream_t>(g->stream);
-    return run(ctx, "fa_forward_ex", a);
+    a.o_amax = o_amax;
+    return run(ctx, who, a);
+}
+
+fa_status_t fa_forward_ex(fa_ctx_t* ctx, const fa_forward_args_t* g) { return forward_ex(ctx, g, nullptr, "fa_forward_ex"); }
+
+fa_status_t fa_forward_raise(fa_ctx_t* ctx, const fa_forward_args_t* g, float* o_amax) {
+    if (ctx && (!o_amax || (reinterpret_cast<uintptr_t>(o_amax) & 3))) {
+        set_err(ctx, "%s: o_amax must be a 4-byte aligned device pointer", "fa_forward_raise");
+        return FA_ERR_INVALID_ARG;
+    }
+    return forward_ex(ctx, g, o_amax, "fa_forward_raise");
 }
 
 fa_status_t fa_decode(fa_ctx_t* ctx, const fa_decode_args_t* g) {

@@ -103,7 +103,8 @@ struct Params {
     const float* sv;
     __half* o;
     float* lse;
-    const uint32_t* v_flags;   // see LaunchArgs
+    float* o_amax;             // see LaunchArgs
+    const uint32_t* v_flags;
     uint32_t v_epoch;
     int v_chunks;              // chunks per head
 };
@@ -292,7 +293,9 @@ __device__ __noinline__ void negate_scores(uint32_t* s) {
 // MASKED = false: no key of the launch is masked (non-causal, no window, S a multiple of the block) and the host-side scale
 // is positive: neither the masking code nor the sign flip of a negative scale is compiled into the softmax loop.  (The
 // device-side scale factors are quantiser outputs, amax / 448: never negative.)
-template <int HD, bool MASKED, bool VRAW>
+//
+// AMAX = true: the largest |O| also goes to p.o_amax, for the quantiser behind (a variant of its own: the others keep their code).
+template <int HD, bool MASKED, bool VRAW, bool AMAX>
 __global__ void __launch_bounds__(NUM_THREADS, 2)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
               const __grid_constant__ CUtensorMap tmap_v, const Params p) {
@@ -681,6 +684,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
             constexpr int CPR = ROWB / 16;          // 16-byte chunks per row: 16 (D = 128) or 8 (D = 64)
             uint8_t* stage = smem + C::OFF_K + warp * (32 * ROWB);
             const int lane = threadIdx.x & 31;
+            __half2 top = __float2half2_rn(0.f);
 #pragma unroll
             for (int c = 0; c < HD / 16; c++) {
                 uint32_t o[16];
@@ -693,6 +697,11 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
                     w.y = pack_half2(__uint_as_float(o[8 * v + 2]) * inv, __uint_as_float(o[8 * v + 3]) * inv);
                     w.z = pack_half2(__uint_as_float(o[8 * v + 4]) * inv, __uint_as_float(o[8 * v + 5]) * inv);
                     w.w = pack_half2(__uint_as_float(o[8 * v + 6]) * inv, __uint_as_float(o[8 * v + 7]) * inv);
+                    if (AMAX) {   // of the rounded values; NaN never wins
+                        const uint32_t x[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                        for (int i = 0; i < 4; i++) top = __hmax2(top, __habs2(*reinterpret_cast<const __half2*>(&x[i])));
+                    }
                     const int ch = 2 * c + v;
                     *reinterpret_cast<uint4*>(stage + lane * ROWB + ((ch ^ (lane % CPR)) << 4)) = w;
                 }
@@ -708,6 +717,12 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
                     const uint4 w = *reinterpret_cast<const uint4*>(stage + rr * ROWB + ((ch ^ (rr % CPR)) << 4));
                     if (rr < rows_left) *reinterpret_cast<uint4*>(obase + (size_t)rr * ROWB + (ch << 4)) = w;
                 }
+            }
+            if (AMAX) {
+                float m = qi < p.sl ? fmaxf(__low2float(top), __high2float(top)) : 0.f;
+#pragma unroll
+                for (int i = 16; i > 0; i >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, i));
+                if (lane == 0) atomicMax(reinterpret_cast<unsigned int*>(p.o_amax), __float_as_uint(m));   // ordered like their bits
             }
             if (p.lse && qi < p.sl) {
                 // sum_j exp(s_j) = l * 2^(m_ref - POFF)  ->  natural-log LSE
@@ -782,6 +797,7 @@ cudaError_t launch_hd(const LaunchArgs& a, int num_sms) {
     p.sq = a.scale_q_dev; p.sk = a.scale_k_dev; p.sv = a.scale_v_dev;
     p.o = reinterpret_cast<__half*>(a.o);
     p.lse = a.lse;
+    p.o_amax = a.o_amax;
     p.v_flags = a.v_flags; p.v_epoch = a.v_epoch; p.v_chunks = v_chunks;
     if (!VRAW) {
         // pre-pass: V codes -> fp16 workspace
@@ -792,8 +808,9 @@ cudaError_t launch_hd(const LaunchArgs& a, int num_sms) {
         if (e != cudaSuccess) return e;
     }
     const bool masked = a.causal || a.window > 0 || (a.sl % BN) != 0 || !(a.scale > 0.f);
-    return masked ? launch_pdl(fa_fwd_kernel<HD, true, VRAW>, (unsigned)grid, NUM_THREADS, C::SMEM_BYTES, a.stream, tq, tk, tv, p)
-                  : launch_pdl(fa_fwd_kernel<HD, false, VRAW>, (unsigned)grid, NUM_THREADS, C::SMEM_BYTES, a.stream, tq, tk, tv, p);
+    auto start = [&](auto kernel) { return launch_pdl(kernel, (unsigned)grid, NUM_THREADS, C::SMEM_BYTES, a.stream, tq, tk, tv, p); };
+    if (a.o_amax) return start(fa_fwd_kernel<HD, true, VRAW, true>);   // the masked kernel serves every call
+    return masked ? start(fa_fwd_kernel<HD, true, VRAW, false>) : start(fa_fwd_kernel<HD, false, VRAW, false>);
 }
 
 }  // namespace
@@ -804,14 +821,18 @@ void init_device(DeviceState* st, int dev) {
     auto set = [&](auto kernel, int bytes) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     };
-    set(fa_fwd_kernel<128, true, false>, Cfg<128, false>::SMEM_BYTES);
-    set(fa_fwd_kernel<128, false, false>, Cfg<128, false>::SMEM_BYTES);
-    set(fa_fwd_kernel<64, true, false>, Cfg<64, false>::SMEM_BYTES);
-    set(fa_fwd_kernel<64, false, false>, Cfg<64, false>::SMEM_BYTES);
-    set(fa_fwd_kernel<128, true, true>, Cfg<128, true>::SMEM_BYTES);
-    set(fa_fwd_kernel<128, false, true>, Cfg<128, true>::SMEM_BYTES);
-    set(fa_fwd_kernel<64, true, true>, Cfg<64, true>::SMEM_BYTES);
-    set(fa_fwd_kernel<64, false, true>, Cfg<64, true>::SMEM_BYTES);
+    set(fa_fwd_kernel<128, true, false, false>, Cfg<128, false>::SMEM_BYTES);
+    set(fa_fwd_kernel<128, false, false, false>, Cfg<128, false>::SMEM_BYTES);
+    set(fa_fwd_kernel<128, true, false, true>, Cfg<128, false>::SMEM_BYTES);
+    set(fa_fwd_kernel<128, true, true, false>, Cfg<128, true>::SMEM_BYTES);
+    set(fa_fwd_kernel<128, false, true, false>, Cfg<128, true>::SMEM_BYTES);
+    set(fa_fwd_kernel<128, true, true, true>, Cfg<128, true>::SMEM_BYTES);
+    set(fa_fwd_kernel<64, true, false, false>, Cfg<64, false>::SMEM_BYTES);
+    set(fa_fwd_kernel<64, false, false, false>, Cfg<64, false>::SMEM_BYTES);
+    set(fa_fwd_kernel<64, true, false, true>, Cfg<64, false>::SMEM_BYTES);
+    set(fa_fwd_kernel<64, true, true, false>, Cfg<64, true>::SMEM_BYTES);
+    set(fa_fwd_kernel<64, false, true, false>, Cfg<64, true>::SMEM_BYTES);
+    set(fa_fwd_kernel<64, true, true, true>, Cfg<64, true>::SMEM_BYTES);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&st->num_sms, cudaDevAttrMultiProcessorCount, dev);
     st->init_error = e;
 }

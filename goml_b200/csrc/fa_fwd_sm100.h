@@ -12,6 +12,7 @@ struct LaunchArgs {
     const void* v;
     void* o;            // [bh, sl, hd] fp16
     float* lse;         // [bh, sl] fp32 natural-log LSE, or nullptr
+    float* o_amax = nullptr;   // raised to the largest |o| (a word that holds a non-negative value), or nullptr
     void* v16_workspace = nullptr;  // workspace_bytes(bh, sl, hd) bytes, 128-byte aligned: fp16 copy of V (see needs_no_scratch)
     int bh, sl, hd;     // hd in {64, 128}
     int causal, window;

@@ -33,7 +33,7 @@ size_t fp8_block_region_bytes(int rows, int d_model, int ffn_hidden) {
 }
 
 int fp8_block_run(const fp8_block_run_args_t* a) {
-    if (!a || !a->gemm_scaled || !a->gemm_accumulate_f32 || !a->gemm_swiglu_raise || !a->attention || !a->attention_ctx) return (int)cudaErrorInvalidValue;
+    if (!a || !a->gemm_scaled || !a->gemm_accumulate_f32 || !a->gemm_swiglu_raise || !a->attention_raise || !a->attention_decode || !a->attention_ctx) return (int)cudaErrorInvalidValue;
     if (!a->x || !a->h || !a->wqkv || !a->wo || !a->wgate_up || !a->wdown || !a->words || !a->rstd || !a->codes || !a->region)
         return (int)cudaErrorInvalidValue;
     const bool decode = a->decode != 0;
@@ -75,7 +75,7 @@ int fp8_block_run(const fp8_block_run_args_t* a) {
         t.scale = a->softmax_scale; t.v_descale = 1.0f;
         t.scale_q_dev = scale + Q; t.scale_k_dev = a->cache_scales; t.scale_v_dev = a->cache_scales + 1;
         t.stream = (fa_stream_t)stream;
-        if ((rc = step(a->attention(a->attention_ctx, &t)))) return rc;
+        if ((rc = step(a->attention_decode(a->attention_ctx, &t)))) return rc;
     } else {
         fp8_block::Rope r{};
         r.qkv_bf16 = qkv; r.cos_tab = a->cos_tab; r.sin_tab = a->sin_tab;
@@ -89,9 +89,10 @@ int fp8_block_run(const fp8_block_run_args_t* a) {
         t.scale = a->softmax_scale; t.v_descale = 1.0f;
         t.scale_q_dev = scale + Q; t.scale_k_dev = scale + K; t.scale_v_dev = scale + V;
         t.stream = (fa_stream_t)stream;
-        if ((rc = step(a->attention(a->attention_ctx, &t)))) return rc;
+        if ((rc = step(a->attention_raise(a->attention_ctx, &t, amax + O)))) return rc;
     }
-    if ((rc = step(fp8_block::permute_heads(o, oc, scale + O, amax + O, a->batch, a->seq_len, H, hd, true, s)))) return rc;
+    const fp8_block::Max known = decode ? fp8_block::Max::ZERO : fp8_block::Max::KNOWN;
+    if ((rc = step(fp8_block::permute_heads(o, oc, scale + O, amax + O, a->batch, a->seq_len, H, hd, known, s)))) return rc;
     // h += attention projection, in the GEMM epilogue
     if ((rc = step(a->gemm_accumulate_f32(T, d, d, oc, a->wo, a->h, 1.0f, scale + O, a->wo_scale, stream)))) return rc;
     // feed-forward half

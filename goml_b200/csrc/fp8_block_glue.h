@@ -30,7 +30,9 @@ struct Rope {
 };
 int rope_qkv(const Rope& r, bool cleared, cudaStream_t s);
 int append(const fp8_decode_append_args_t* g, bool cleared);
-int permute_heads(const void* o_fp16, uint8_t* q, float* scale_out, float* amax_out, int batch, int seq_len, int heads, int head_dim, bool cleared,
+// state of a maximum's word when an op is called: any value, zero, or the maximum itself (no pass over the input for it)
+enum class Max { ANY, ZERO, KNOWN };
+int permute_heads(const void* o_fp16, uint8_t* q, float* scale_out, float* amax, int batch, int seq_len, int heads, int head_dim, Max state,
                   cudaStream_t s);
 
 }  // namespace fp8_block

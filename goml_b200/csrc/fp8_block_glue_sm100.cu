@@ -1080,7 +1080,7 @@ int append(const fp8_decode_append_args_t* g, bool cleared) {
     return (int)e;
 }
 
-int permute_heads(const void* o_fp16, uint8_t* q, float* scale_out, float* amax_out, int batch, int seq_len, int heads, int head_dim, bool cleared,
+int permute_heads(const void* o_fp16, uint8_t* q, float* scale_out, float* amax_out, int batch, int seq_len, int heads, int head_dim, Max state,
                   cudaStream_t s) {
     if (!o_fp16 || !q || !scale_out || !amax_out) return (int)cudaErrorInvalidValue;
     if (batch < 0 || seq_len <= 0 || heads <= 0 || head_dim <= 0 || (head_dim % 16) != 0) return (int)cudaErrorInvalidValue;
@@ -1094,9 +1094,9 @@ int permute_heads(const void* o_fp16, uint8_t* q, float* scale_out, float* amax_
     a.dv.cph = FastDiv(head_dim / 16);
     a.dv.heads = FastDiv(heads);
     a.dv.seq = FastDiv(seq_len);
-    if (n16 * 32 <= OC_BYTES_O && oc_fits<OOp>()) return (int)oc_launch(OOp{a}, s);
-    cudaError_t e = cleared ? cudaSuccess : clear_words(amax_out, 1, s);
-    if (e == cudaSuccess && n16 > 0) e = launch_pdl_stream(n16 * 32, o_amax_kernel, dim3(grid_for(n16)), dim3(THREADS), s, a);
+    if (state != Max::KNOWN && n16 * 32 <= OC_BYTES_O && oc_fits<OOp>()) return (int)oc_launch(OOp{a}, s);
+    cudaError_t e = state == Max::ANY ? clear_words(amax_out, 1, s) : cudaSuccess;
+    if (e == cudaSuccess && n16 > 0 && state != Max::KNOWN) e = launch_pdl_stream(n16 * 32, o_amax_kernel, dim3(grid_for(n16)), dim3(THREADS), s, a);
     if (e == cudaSuccess) e = launch_pdl_stream(n16 * 32, o_quant_kernel, dim3(grid_for(n16)), dim3(THREADS), s, a);
     return (int)e;
 }
@@ -1136,7 +1136,7 @@ int fp8_decode_rope_append(const fp8_decode_append_args_t* g) { return fp8_block
 
 int fp8_permute_quantize_heads(const void* o_fp16, uint8_t* q, float* scale_out, float* amax_out, int batch, int seq_len,
                                int heads, int head_dim, void* stream) {
-    return fp8_block::permute_heads(o_fp16, q, scale_out, amax_out, batch, seq_len, heads, head_dim, false, (cudaStream_t)stream);
+    return fp8_block::permute_heads(o_fp16, q, scale_out, amax_out, batch, seq_len, heads, head_dim, fp8_block::Max::ANY, (cudaStream_t)stream);
 }
 
 int fp8_swiglu_quantize(const void* gate_up_bf16, uint8_t* q, float* scale_out, float* amax_out, int rows, int ffn_hidden,

@@ -138,6 +138,8 @@ def FALoad():
                 lib.fa_kernel_name.argtypes = [i]
                 lib.fa_forward_ex.restype = i
                 lib.fa_forward_ex.argtypes = [p, C.POINTER(ForwardArgs)]
+                lib.fa_forward_raise.restype = i
+                lib.fa_forward_raise.argtypes = [p, C.POINTER(ForwardArgs), p]
                 lib.fa_forward_noalloc.restype = i
                 lib.fa_forward_noalloc.argtypes = [C.POINTER(ForwardArgs), C.c_char_p, i]
                 lib.fa_decode.restype = i

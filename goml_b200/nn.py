@@ -156,7 +156,7 @@ def _entry_points():
     if _entries is None:
         gemm, fa = G._init(), F.FALoad()
         _entries = tuple(ctypes.cast(fn, ctypes.c_void_p).value for fn in (gemm.fp8_gemm_scaled, gemm.fp8_gemm_accumulate_f32, gemm.fp8_gemm_swiglu_raise,
-                                                                           fa.fa_forward_ex, fa.fa_decode))
+                                                                           fa.fa_forward_raise, fa.fa_decode))
     return _entries
 
 
@@ -224,12 +224,11 @@ class FP8DecoderBlock:
         cos, sin = self.rope_tables(tables, x.device)
         if not self.fa.ptr:
             raise F.FAError("FP8DecoderBlock: nil ctx", F.FA_ERR_INVALID_ARG)
-        gemm, accumulate, swiglu, forward, step = _entry_points()
         k = v = ks = lens = s_max = 0
         if cache is not None:
             k, v, ks, lens, s_max = cache.k.data_ptr(), cache.v.data_ptr(), cache.scales.data_ptr(), cache.lens.data_ptr(), cache.s_max
         qkv, o, gate_up, down = self.qkv.w, self.o.w, self.gate_up.w, self.down.w
-        rc = BG.BlockRun(gemm, accumulate, swiglu, step if decode else forward, self.fa.ptr, src.data_ptr(), h.data_ptr(), self.norm1.data_ptr(),
+        rc = BG.BlockRun(*_entry_points(), self.fa.ptr, src.data_ptr(), h.data_ptr(), self.norm1.data_ptr(),
                          self.norm2.data_ptr(), qkv.codes.data_ptr(), o.codes.data_ptr(), self.gate_up_interleaved.data_ptr(), down.codes.data_ptr(),
                          qkv.scale_ptr, o.scale_ptr, gate_up.scale_ptr, down.scale_ptr, cos.data_ptr(), sin.data_ptr(), k, v, ks, lens,
                          words, rstd, codes, kc, vc, region, region_bytes, torch.cuda.current_stream().cuda_stream,

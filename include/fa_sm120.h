@@ -147,6 +147,10 @@ typedef struct {
 
 FA_API fa_status_t fa_forward_ex(fa_ctx_t* ctx, const fa_forward_args_t* args);
 
+/* fa_forward_ex that also raises *o_amax (a device word that holds a non-negative value) to the largest |O| of the call, as
+ * written (fp16; NaN never wins): the maximum that a quantiser of O needs, without a pass over it. */
+FA_API fa_status_t fa_forward_raise(fa_ctx_t* ctx, const fa_forward_args_t* args, float* o_amax);
+
 /* No counterpart in the reference: an attention forward that allocates nothing.
  * The other entry points draw their scratch (an fp16 copy of V, 2*BH*S*D bytes) from a
  * memory pool.  This one is for callers that may not touch the allocator at all — code

@@ -150,7 +150,7 @@ FP8BLOCK_API int fp8_decode_rope_append(const fp8_decode_append_args_t* args);
  * h += W_down(silu(W_gate n) * W_up n), n the RMSNorm of h) or of one new token per sequence (decode = 1, seq_len 1: K and V
  * appended to the cache at cache_lens, which advances in place), issued in native code.
  * The GEMM and attention entry points come as function pointers, so this library links to neither of the others:
- * fp8_gemm_scaled, fp8_gemm_accumulate_f32, fp8_gemm_swiglu_raise, and fa_forward_ex (prompt) or fa_decode with its context.
+ * fp8_gemm_scaled, fp8_gemm_accumulate_f32, fp8_gemm_swiglu_raise, and fa_forward_raise and fa_decode with their context.
  *   x, h     [batch*seq_len, d_model] fp32: input and output stream; h may be x (then it is updated in place);
  *   w*       e4m3 weights and their device scales; wgate_up interleaved as fp8_gemm_swiglu reads it; norm1, norm2 fp32;
  *   cos_tab, sin_tab  [rope_rows, d_model/heads/2] (at least seq_len rows for a prompt, s_max for a step);
@@ -163,7 +163,8 @@ typedef struct fp8_block_run_args {
     int (*gemm_scaled)(int, int, int, const void*, const void*, void*, float, const float*, const float*, int, void*);
     int (*gemm_accumulate_f32)(int, int, int, const void*, const void*, float*, float, const float*, const float*, void*);
     int (*gemm_swiglu_raise)(int, int, int, const void*, const void*, void*, float, const float*, const float*, float*, void*);
-    int (*attention)(void* ctx, const void* args);
+    int (*attention_raise)(void* ctx, const void* args, float* o_amax);
+    int (*attention_decode)(void* ctx, const void* args);
     void* attention_ctx;
     const float* x;
     float* h;

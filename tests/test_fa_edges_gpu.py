@@ -75,3 +75,27 @@ def test_the_last_context_goes_while_a_pre_pass_is_queued(cuda, built_libs, monk
     from tests import test_fa_scratch_gpu as scratch
     monkeypatch.setattr(scratch, "LAST_CONTEXT", scratch.LAST_CONTEXT.replace("2048", "4608"))
     scratch.test_the_last_context_goes_while_work_is_queued_and_a_capture_is_open(cuda, built_libs)
+
+
+@pytest.mark.parametrize("s,hd,causal,window", [(1, 64, 1, 0), (127, 128, 1, 0), (129, 64, 1, 0), (300, 128, 0, 0), (2700, 128, 1, 0), (2700, 64, 0, 0), (256, 128, 0, 0),
+                                                (500, 64, 1, 33)])
+def test_the_largest_output(cuda, built_libs, fa_ctx, s, hd, causal, window):
+    # raised, not set; of the rows of the sequences alone; the output itself is the other entry point's (its kernel of masked launches
+    # serves the unmasked ones here)
+    import ctypes as C
+    import torch
+    from goml_b200 import fa_forward as F
+    g = torch.Generator(device="cuda").manual_seed(s)
+    q, k, v = (torch.randint(0, 0x70, (5, s, hd), generator=g, dtype=torch.uint8, device="cuda") for _ in range(3))
+    v ^= torch.randint(0, 2, v.shape, generator=g, dtype=torch.uint8, device="cuda") << 7
+    want, o = (torch.zeros(5, s, hd, dtype=torch.float16, device="cuda") for _ in range(2))
+    fa_ctx.ForwardEx(q.data_ptr(), k.data_ptr(), v.data_ptr(), want.data_ptr(), 0, 5, s, hd, causal, window, 1e-5, 1.0)
+    args = F.ForwardArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), None, 5, s, hd, causal, window, 1e-5, 1.0, None, None, None, None)
+    top = want.float().abs().max().item()
+    for start in (0.0, 2 * top):
+        word = torch.tensor([start], device="cuda")
+        assert F.FALoad().fa_forward_raise(fa_ctx.ptr, C.byref(args), word.data_ptr()) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(o, want) and word.item() == max(start, top)
+    fa_ctx.DeviceStatus()
+    assert F.FALoad().fa_forward_raise(fa_ctx.ptr, C.byref(args), None) == F.FA_ERR_INVALID_ARG
