@@ -434,6 +434,7 @@ inline int launch(GemmParams g, const Plan& plan, const void* A, const void* B, 
     if (p.stages > slice) p.stages = slice;
     if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
     int ring_bytes = p.stages * stage_bytes;
+    while (ring_bytes < part_bytes) { p.stages++; ring_bytes += stage_bytes; }   // the partial sums take the ring's place
     // How much of the weight is asked for ahead of the wait.  It helps as far as memory is idle until then; past that a CTA's first
     // loads stand behind hints for its last ones.  Half of a CTA's blocks up to 16 (all of up to 8), with several CTAs to an SM no more than 20 MB in
     // all, and four blocks past 80 tokens, whose first loads bring as much again in tokens, which no hint has fetched.  All / as
