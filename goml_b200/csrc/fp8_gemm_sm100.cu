@@ -141,6 +141,46 @@ __device__ __forceinline__ uint32_t pack_out(float a, float b, int bf16) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// A 32 x 64 box of 16-bit values (128-byte rows, swizzled) to a matrix whose rows start on multiples of UNIT bytes, by one warp: a
+// row is 128 bytes in a row.  `cols` is a multiple of UNIT / 2.  UNIT 2: rows may start on odd multiples of 2 bytes; there a lane
+// takes the second half of its word and the first of the next lane's.
+template <int UNIT>
+__device__ __forceinline__ void store_box(uint32_t box, uint16_t* out, int n, int rows, int cols, int lane) {
+    constexpr int RPI = UNIT == 8 ? 2 : 1, BATCH = 8;   // rows per step, steps whose loads are in flight
+    const int sub = RPI == 2 ? lane >> 4 : 0, c = RPI == 2 ? (lane & 15) * 4 : lane * 2;
+#pragma unroll 1
+    for (int r0 = 0; r0 < rows; r0 += BATCH * RPI) {
+        uint32_t w[BATCH][UNIT == 8 ? 2 : 1];
+#pragma unroll
+        for (int i = 0; i < BATCH; i++) {
+            const int r = r0 + i * RPI + sub;
+            const uint32_t src = box + r * 128 + (((c >> 3) ^ (r & 7)) << 4) + (c & 7) * 2;
+            if (UNIT == 8) asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(w[i][0]), "=r"(w[i][UNIT == 8 ? 1 : 0]) : "r"(src) : "memory");
+            else asm volatile("ld.shared.b32 %0, [%1];" : "=r"(w[i][0]) : "r"(src) : "memory");
+        }
+#pragma unroll
+        for (int i = 0; i < BATCH; i++) {
+            const int r = r0 + i * RPI + sub;
+            if (UNIT == 2) {
+                const uint32_t next = __shfl_down_sync(0xffffffffu, w[i][0], 1);
+                if (r >= rows) continue;            // the same in every lane
+                uint16_t* dst = out + (size_t)r * n;
+                const int odd = (int)((reinterpret_cast<uintptr_t>(dst) >> 1) & 1), e = c + odd;
+                const uint32_t v = odd ? __byte_perm(w[i][0], next, 0x5432) : w[i][0];
+                if (e + 1 < cols) *reinterpret_cast<uint32_t*>(dst + e) = v;
+                // what the pairs leave out: the first value of an odd row, the last one of a row that ends within a pair
+                const bool head = odd && lane == 0;
+                if (head || e + 1 == cols) dst[head ? 0 : e] = (uint16_t)(head ? w[i][0] : v);
+                if (cols == 2 && head) dst[1] = (uint16_t)v;   // both in one lane
+            } else if (r < rows && c < cols) {
+                uint16_t* dst = out + (size_t)r * n + c;
+                if (UNIT == 8) *reinterpret_cast<uint2*>(dst) = make_uint2(w[i][0], w[i][UNIT == 8 ? 1 : 0]);
+                else *reinterpret_cast<uint32_t*>(dst) = w[i][0];
+            }
+        }
+    }
+}
+
 // four fp32 -> four e4m3 codes (round to nearest even, saturate to +-448, NaN -> 0x7f), a in the lowest byte
 __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float d) {
     uint16_t lo, hi;
@@ -302,7 +342,8 @@ fp8_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         float alpha = p.alpha;
         if (p.scale_a) alpha *= ld_f32(p.scale_a);
         if (p.scale_b) alpha *= ld_f32(p.scale_b);
-        const bool vec_ok = (p.N % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
+        // bytes of C that a lane may store at once: rows start on multiples of it
+        const int c_unit = (p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 7) == 0) ? 8 : (p.N % 2 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 3) == 0) ? 4 : 2;
         const bool xvec_ok = (p.N % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.X) & 15) == 0);
         const bool dvec_ok = (p.N % 16 == 0) && ((reinterpret_cast<uintptr_t>(p.D8) & 15) == 0);
         const float scale_d = (p.D8 && p.scale_d) ? ld_f32(p.scale_d) : 1.0f;
@@ -319,7 +360,6 @@ fp8_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
             tc_fence_after();
             const int row = tm * BM + row_in_tile;
             const uint32_t taddr = tmem_base + buf * BN + (uint32_t(quad * 32) << 16);
-            uint16_t* crow = reinterpret_cast<uint16_t*>(p.C) + (size_t)row * p.N;
             float tmax = 0.f;  // running max of this thread's row (SwiGLU and e4m3-output modes)
             if (tm * BM + quad * 32 >= p.M) {
                 // all 32 rows of this warp lie past M (a skinny problem uses 16 of a tile's 128 rows): nothing to
@@ -464,6 +504,39 @@ fp8_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                     }
                     sbuf ^= 1;
                 }
+            } else if (p.C) {
+                // 16-bit C that no tensor map describes (N % 8 != 0 or misaligned): a thread's own row would leave as 2-byte stores to 32
+                // rows at a time.  The same boxes as above instead, stored row by row, 128 bytes in a row (us, before / now, and with
+                // a length that takes the map: 2500 x 1500 x 5008 70 / 30 / 28, 700 x 5556 x 1024 52 / 11, 8192 x 3002 x 3008 313 / 87,
+                // x 3001 321 / 131, x 3000 62: odd rows still pay for a second store and for sectors written in halves).
+#pragma unroll 1
+                for (int c2 = 0; c2 < bn / 64; c2++) {
+                    const int col0 = n0 + c2 * 64;
+                    if (col0 >= p.N) break;  // uniform across the CTA
+                    const uint32_t box = staging + quad * 2 * STAGING_BOX;
+                    __syncwarp();            // the rows of the box before have been read
+#pragma unroll
+                    for (int hf = 0; hf < 2; hf++) {
+                        uint32_t acc[32];
+                        tmem_ld_32x32b_x32(taddr + c2 * 64 + hf * 32, acc);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int v = 0; v < 4; v++) {
+                            uint32_t w[4];
+#pragma unroll
+                            for (int i = 0; i < 4; i++)
+                                w[i] = pack_out(__uint_as_float(acc[8 * v + 2 * i]) * alpha, __uint_as_float(acc[8 * v + 2 * i + 1]) * alpha, p.out_bf16);
+                            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(box + lane * 128 + (((hf * 4 + v) ^ (lane & 7)) << 4)),
+                                         "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+                        }
+                    }
+                    __syncwarp();
+                    const int row0 = tm * BM + quad * 32, rows = min(32, p.M - row0), cols = min(64, p.N - col0);
+                    uint16_t* out = reinterpret_cast<uint16_t*>(p.C) + (size_t)row0 * p.N + col0;
+                    if (c_unit == 8) store_box<8>(box, out, p.N, rows, cols, lane);
+                    else if (c_unit == 4) store_box<4>(box, out, p.N, rows, cols, lane);
+                    else store_box<2>(box, out, p.N, rows, cols, lane);
+                }
             } else
 #pragma unroll 1
             for (int c = 0; c < bn / 32; c++) {
@@ -539,30 +612,6 @@ fp8_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
 #pragma unroll
                         for (int j = 0; j < 32; j++)
                             if (col0 + j < p.N) xrow[j] = fmaf(__uint_as_float(acc[j]), alpha, xrow[j]);
-                    }
-                } else if (row < p.M) {
-                    if (vec_ok && col0 + 32 <= p.N) {
-                        uint4* dst = reinterpret_cast<uint4*>(crow + col0);
-#pragma unroll
-                        for (int v = 0; v < 4; v++) {
-                            uint4 o;
-                            o.x = pack_out(__uint_as_float(acc[8 * v + 0]) * alpha, __uint_as_float(acc[8 * v + 1]) * alpha, p.out_bf16);
-                            o.y = pack_out(__uint_as_float(acc[8 * v + 2]) * alpha, __uint_as_float(acc[8 * v + 3]) * alpha, p.out_bf16);
-                            o.z = pack_out(__uint_as_float(acc[8 * v + 4]) * alpha, __uint_as_float(acc[8 * v + 5]) * alpha, p.out_bf16);
-                            o.w = pack_out(__uint_as_float(acc[8 * v + 6]) * alpha, __uint_as_float(acc[8 * v + 7]) * alpha, p.out_bf16);
-                            __stcs(dst + v, o);  // streaming store: C is not read again, keep A and B panels in L2
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; j++) {
-                            if (col0 + j < p.N) {
-                                const float f = __uint_as_float(acc[j]) * alpha;
-                                uint16_t bits;
-                                if (p.out_bf16) { __nv_bfloat16 h = __float2bfloat16_rn(f); bits = *reinterpret_cast<uint16_t*>(&h); }
-                                else { __half h = __float2half_rn(f); bits = *reinterpret_cast<uint16_t*>(&h); }
-                                crow[col0 + j] = bits;
-                            }
-                        }
                     }
                 }
             }

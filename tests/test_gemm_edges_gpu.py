@@ -1,0 +1,43 @@
+"""FP8 GEMM where the output's rows are not whole 16-byte pieces, and on both sides of the few-row kernel's lines: products of
+-1, 0 and 1, whose sums are whole numbers that fp16 holds, so every element is compared exactly."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def exact(M, N, K, offset=0, out="fp16", seed=0):
+    from goml_b200 import fp8_gemm as G
+    g = torch.Generator(device="cuda").manual_seed(seed + 1000 * M + N)
+    a, b = (torch.randint(-1, 2, (rows, K), generator=g, device="cuda") for rows in (M, N))
+    codes = lambda x: torch.tensor([0xb8, 0x00, 0x38], dtype=torch.uint8, device="cuda")[x + 1].contiguous()
+    ad, bd = codes(a), codes(b)
+    dtype = torch.float16 if out == "fp16" else torch.bfloat16
+    room = torch.full((M * N + 64,), 7.0, dtype=dtype, device="cuda")
+    c = room[16 + offset:16 + offset + M * N]
+    G.FP8GEMMScaled(M, N, K, ad.data_ptr(), bd.data_ptr(), c.data_ptr(), 1.0, 0, 0, G.OutFP16 if out == "fp16" else G.OutBF16, 0)
+    torch.cuda.synchronize()
+    assert G.device_status() == 0
+    want = a.double() @ b.double().t()
+    assert torch.equal(c.view(M, N).double(), want.to(dtype).double())
+    assert (room[:16 + offset] == 7).all() and (room[16 + offset + M * N:] == 7).all()   # nothing around it
+
+
+@pytest.mark.parametrize("N", [1, 2, 3, 5, 31, 62, 63, 64, 65, 66, 67, 127, 130, 191, 252, 255, 257, 260, 513, 1001])
+@pytest.mark.parametrize("M", [193, 257])
+def test_rows_of_any_length(cuda, built_libs, M, N):
+    for offset in (0, 1, 2, 4):   # elements past a 16-byte boundary
+        exact(M, N, 64, offset)
+    exact(M, N, 64, 0, "bf16")
+
+
+@pytest.mark.parametrize("M,N,K", [(4097, 517, 128), (700, 5555, 256), (300, 20003, 2048), (5000, 2001, 2048)])
+def test_many_tiles_with_rows_of_any_length(cuda, built_libs, M, N, K):
+    # tiles of every width, halves of a short last wave and tile pairs
+    exact(M, N, K)
+
+
+@pytest.mark.parametrize("M", [81, 100, 128, 129, 150, 192])
+@pytest.mark.parametrize("N,K", [(1024, 2992), (1024, 3008), (1501, 4784), (1501, 4800), (130, 8192)])
+def test_few_rows_on_both_sides_of_the_lines(cuda, built_libs, M, N, K):
+    exact(M, N, K)
