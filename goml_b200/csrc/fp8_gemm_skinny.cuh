@@ -376,9 +376,10 @@ inline Plan plan(int M, int N, int K, int num_sms, const Fit& fit) {
     const long long tiles = ((long long)N + W_ROWS - 1) / W_ROWS;
     const int k_blocks = (K + BK - 1) / BK, tn = (M + 15) / 16 * 16;
     // Past 80 tokens the tokens' own traffic and the longer finish (2 us more at 128) weigh against a square kernel that
-    // needs one row of tiles: 4096 x 4096, 112 tokens 8.4 / 8.0 us, but 8192 x 8192 16.2 / 17.1.  Past 128 that one reads
-    // the weight twice: 144 tokens, 4096 x 4096 8.7 / 10.1 us, 2048 x 2048 6.3 / 6.2.
-    if (M > 80 && weights < (M > 128 ? 1ll << 24 : 1ll << 25)) return r;
+    // needs one row of tiles, for small weights whose K is short: 100 tokens, 2048 x 2048 6.7 / 6.3 us, 8192 x 2048 (128) 9.0 / 7.6, but
+    // 4096 x 4096 8.4 / 9.3, 2000 x 3008 7.3 / 7.9, 1024 x 8192 8.4 / 13.6.  Past 128 that one reads the weight twice: 150 tokens, 2048
+    // x 2048 7.5 / 6.5, 4096 x 4000 9.9 / 10.0, 2000 x 5008 10.4 / 14.6; 190 tokens, 1504 x 6000 12.1 / 16.5.
+    if (M > 128 ? weights < 1ll << 24 && K < 4800 : M > 80 && weights < 1ll << 25 && K < 3000) return r;
     // the K range is cut as long as all slices are resident, one to an SM, and two k-blocks are left to each (16 tokens, 1 / 2 /
     // 3 / 4 slices: 8192 x 8192 17.4 / 13.9 / 14.8 / 13.7 us, of which 2 fit; 4096 x 4096 9.9 / 7.0 / 6.3 / 6.2);
     // past four slices the finish grows faster than the stream shrinks, unless less than three fifths of the SMs are in use and
