@@ -295,7 +295,10 @@ __device__ __noinline__ void negate_scores(uint32_t* s) {
 // device-side scale factors are quantiser outputs, amax / 448: never negative.)
 //
 // AMAX = true: the largest |O| also goes to p.o_amax, for the quantiser behind (a variant of its own: the others keep their code).
-template <int HD, bool MASKED, bool VRAW, bool AMAX>
+// COPY = true: the rows of O leave as one copy each.  That takes the stores off the softmax warps but ends later: with more than
+// two waves of tiles the first counts (256 heads of 2048, causal, 308 -> 302 us, 150 of 512 25.3 -> 24.7), else the second (100 of
+// 300 14.6 -> 15.0, 64 of 700 20.2 -> 20.5).  Not for D = 64, whose copies are of 128 bytes (64 heads of 3000, window 512, 64.8 -> 67.8).
+template <int HD, bool MASKED, bool VRAW, bool AMAX, bool COPY = false>
 __global__ void __launch_bounds__(NUM_THREADS, 2)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
               const __grid_constant__ CUtensorMap tmap_v, const Params p) {
@@ -675,13 +678,18 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
             const float l = (l0 + l1) + (l2 + l3);
             const float vds = p.sv ? p.v_descale * ld_f32(p.sv) : p.v_descale;
             const float inv = (l > 0.f) ? vds / l : 0.f;
-            // O leaves through shared memory so that the global stores are coalesced: a thread owns one row (HD fp16 = ROWB
-            // bytes), which written straight to global makes every store instruction of a warp touch 32 different lines.
-            // Each warp stages its 32 rows in the (by now idle) K ring — 16-byte chunk c of row r at chunk c ^ (r % CPR), so
-            // that both the row-wise writes and the read-back are free of bank conflicts — and stores them back as whole
-            // 512-byte runs.  Only this warp touches its staging area: a __syncwarp() orders the two passes.
+            // O leaves through shared memory: a thread owns one row (HD fp16 = ROWB bytes), which written straight to global makes
+            // every store instruction of a warp touch 32 different lines.  Its place is the (by now idle) rings.
+            //  COPY: each thread stages its row, rows 16 bytes more than their length apart so that eight neighbouring lanes meet
+            //   different banks, and has it copied out whole.
+            //  Else each warp stages its 32 rows — 16-byte chunk c of row r at chunk c ^ (r % CPR), so that both the row-wise writes
+            //   and the read-back are free of bank conflicts — and stores them back as whole 512-byte runs.  Only this warp touches
+            //   its staging area: a __syncwarp() orders the two passes.
             constexpr int ROWB = HD * 2;            // bytes per output row
             constexpr int CPR = ROWB / 16;          // 16-byte chunks per row: 16 (D = 128) or 8 (D = 64)
+            constexpr int PITCH = ROWB + 16;
+            const uint32_t own = sbase + C::OFF_K + r * PITCH;
+            static_assert(C::OFF_K + BM * PITCH <= C::OFF_BAR, "the rows fit the rings");
             uint8_t* stage = smem + C::OFF_K + warp * (32 * ROWB);
             const int lane = threadIdx.x & 31;
             __half2 top = __float2half2_rn(0.f);
@@ -703,12 +711,21 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
                         for (int i = 0; i < 4; i++) top = __hmax2(top, __habs2(*reinterpret_cast<const __half2*>(&x[i])));
                     }
                     const int ch = 2 * c + v;
-                    *reinterpret_cast<uint4*>(stage + lane * ROWB + ((ch ^ (lane % CPR)) << 4)) = w;
+                    if (COPY)
+                        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(own + ch * 16), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w) : "memory");
+                    else
+                        *reinterpret_cast<uint4*>(stage + lane * ROWB + ((ch ^ (lane % CPR)) << 4)) = w;
                 }
             }
-            __syncwarp();
-            {
-                constexpr int RPI = 32 / CPR;       // rows per store instruction: 2 (D = 128) or 4 (D = 64)
+            if (COPY) {
+                fence_proxy_async_smem();
+                if (qi < p.sl)
+                    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                                 ::"l"(p.o + ((size_t)head * p.sl + qi) * HD), "r"(own), "n"(ROWB) : "memory");
+                tma_store_commit();
+            } else {
+                __syncwarp();
+                constexpr int RPI = 32 / CPR;       // rows per store instruction
                 uint8_t* obase = reinterpret_cast<uint8_t*>(p.o + ((size_t)head * p.sl + q0 + warp * 32) * HD);
                 const int rows_left = p.sl - (q0 + warp * 32);   // rows of this warp inside the sequence
 #pragma unroll
@@ -729,6 +746,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
                 p.lse[(size_t)head * p.sl + qi] =
                     (l > 0.f) ? (m_ref - POFF + log2f(l)) * 0.6931471805599453f : -INFINITY;
             }
+            if (COPY) tma_store_wait_read<0>();   // shared memory outlives the copies' reads
         }
     }
 
@@ -810,6 +828,8 @@ cudaError_t launch_hd(const LaunchArgs& a, int num_sms) {
     const bool masked = a.causal || a.window > 0 || (a.sl % BN) != 0 || !(a.scale > 0.f);
     auto start = [&](auto kernel) { return launch_pdl(kernel, (unsigned)grid, NUM_THREADS, C::SMEM_BYTES, a.stream, tq, tk, tv, p); };
     if (a.o_amax) return start(fa_fwd_kernel<HD, true, VRAW, true>);   // the masked kernel serves every call
+    if constexpr (HD == 128)
+        if (grid > 4ll * num_sms) return masked ? start(fa_fwd_kernel<HD, true, VRAW, false, true>) : start(fa_fwd_kernel<HD, false, VRAW, false, true>);
     return masked ? start(fa_fwd_kernel<HD, true, VRAW, false>) : start(fa_fwd_kernel<HD, false, VRAW, false>);
 }
 
@@ -833,6 +853,10 @@ void init_device(DeviceState* st, int dev) {
     set(fa_fwd_kernel<64, true, true, false>, Cfg<64, true>::SMEM_BYTES);
     set(fa_fwd_kernel<64, false, true, false>, Cfg<64, true>::SMEM_BYTES);
     set(fa_fwd_kernel<64, true, true, true>, Cfg<64, true>::SMEM_BYTES);
+    set(fa_fwd_kernel<128, true, false, false, true>, Cfg<128, false>::SMEM_BYTES);
+    set(fa_fwd_kernel<128, false, false, false, true>, Cfg<128, false>::SMEM_BYTES);
+    set(fa_fwd_kernel<128, true, true, false, true>, Cfg<128, true>::SMEM_BYTES);
+    set(fa_fwd_kernel<128, false, true, false, true>, Cfg<128, true>::SMEM_BYTES);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&st->num_sms, cudaDevAttrMultiProcessorCount, dev);
     st->init_error = e;
 }

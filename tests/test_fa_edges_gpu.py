@@ -99,3 +99,22 @@ def test_the_largest_output(cuda, built_libs, fa_ctx, s, hd, causal, window):
         assert torch.equal(o, want) and word.item() == max(start, top)
     fa_ctx.DeviceStatus()
     assert F.FALoad().fa_forward_raise(fa_ctx.ptr, C.byref(args), None) == F.FA_ERR_INVALID_ARG
+
+
+@pytest.mark.parametrize("s,heads,causal,window", [(129, 300, 0, 0), (1, 600, 1, 0), (255, 301, 1, 77), (64, 600, 0, 0), (2600, 30, 1, 0)])
+def test_output_rows_copied_whole(cuda, built_libs, fa_ctx, s, heads, causal, window):
+    # with many tiles the rows leave as copies of their own, with few as runs of a warp: the same bits, and nothing around them
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(s)
+    q, k, v = (torch.randint(0, 0x70, (heads, s, 128), generator=g, dtype=torch.uint8, device="cuda") for _ in range(3))
+    room = torch.full((heads * s * 128 + 128,), 7.0, dtype=torch.float16, device="cuda")
+    o = room[64:-64].view(heads, s, 128)
+    run = lambda i, n, out: fa_ctx.ForwardEx(q[i:].data_ptr(), k[i:].data_ptr(), v[i:].data_ptr(), out.data_ptr(), 0, n, s, 128, causal, window, 1e-5, 1.0)
+    run(0, heads, o)
+    for i in (0, heads - 2):
+        few = torch.zeros(2, s, 128, dtype=torch.float16, device="cuda")
+        run(i, 2, few)
+        torch.cuda.synchronize()
+        assert torch.equal(few, o[i:i + 2])
+    fa_ctx.DeviceStatus()
+    assert torch.isfinite(o).all() and (room[:64] == 7).all() and (room[-64:] == 7).all()
