@@ -15,7 +15,7 @@
 //    brought into L2 while the small kernel ahead (a quantiser, usually) still runs.
 // What is left is 3 us of start, fill and finish beside the stream: M = 16, 8192 x 8192 16.7 -> 13.7 us (floor 10.3),
 // 12288 x 4096 13.3 -> 11.1 (7.7), 22016 x 4096 with SwiGLU
-// 21.9 -> 19.0 (13.8), 11008 x 4096 12.8 -> 10.3 (6.9), 4096 x 11008 12.9 -> 10.8 (6.9), 4096 x 4096 7.8 -> 6.1 (2.6).
+// 21.9 -> 18.4 (13.8), 11008 x 4096 12.8 -> 10.3 (6.9), 4096 x 11008 12.9 -> 10.8 (6.9), 4096 x 4096 7.8 -> 6.1 (2.6).
 #pragma once
 
 namespace skinny {
