@@ -223,7 +223,7 @@ class FP8DecoderBlock:
         src, h = _stream_start(x, T, d)                         # residual stream, updated in place
         cos, sin = self.rope_tables(tables, x.device)
         if not self.fa.ptr:
-            raise F.FAError("FP8DecoderBlock: nil ctx", F.FA_ERR_INVALID_ARG)
+            raise F.FAError(f"FAContext.{'Decode' if decode else 'ForwardEx'}: nil ctx", F.FA_ERR_INVALID_ARG)
         k = v = ks = lens = s_max = 0
         if cache is not None:
             k, v, ks, lens, s_max = cache.k.data_ptr(), cache.v.data_ptr(), cache.scales.data_ptr(), cache.lens.data_ptr(), cache.s_max
@@ -234,15 +234,16 @@ class FP8DecoderBlock:
                          words, rstd, codes, kc, vc, region, region_bytes, torch.cuda.current_stream().cuda_stream,
                          B, S, d, H, Fh, s_max, tables, int(decode), self.eps, 1.0 / math.sqrt(self.hd))
         if rc:
-            self._raise(rc)
+            self._raise(rc, decode, cache is not None)
         return h, buf, kc, vc, words + 72
 
-    def _raise(self, rc: int) -> None:
+    def _raise(self, rc: int, decode: bool, cached: bool) -> None:
         """The error of the library call that fp8_block_run stopped at, as its own binding raises it."""
         place, code = rc >> 16, rc & 0xffff
         if place == 4:
-            raise F.FAError("attention", code, self.fa._msg())
-        name = ("fp8_block_run", "fp8_rmsnorm_quantize_into", "fp8_gemm_scaled", "fp8_rope_quantize_qkv", "", "fp8_permute_quantize_heads",
+            raise F.FAError("fa_decode" if decode else "fa_forward_raise", code, self.fa._msg())
+        rope = "fp8_decode_rope_append" if decode else "fp8_rope_quantize_qkv_cache" if cached else "fp8_rope_quantize_qkv"
+        name = ("fp8_block_run", "fp8_rmsnorm_quantize_into", "fp8_gemm_scaled", rope, "", "fp8_permute_quantize_heads",
                 "fp8_gemm_accumulate_f32", "fp8_rmsnorm_quantize_into", "fp8_gemm_swiglu_raise", "fp8_quantize_bf16", "fp8_gemm_accumulate_f32")[place]
         if name.startswith("fp8_gemm"):
             raise G.FP8GEMMError(f"{name}: CUDA error {code}")

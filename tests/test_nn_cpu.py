@@ -109,3 +109,36 @@ def test_a_cache_with_a_fill_of_its_own_has_it_called():
     assert nn._writes_directly(cache(), B, H, 8, HD, CPU)
     for c in (Counting(B, H, S_MAX, HD, device="cpu"), Duck(), patched, None):
         assert not nn._writes_directly(c, B, H, 8, HD, CPU)
+
+
+# the calls of a block in their order, and what their bindings raise
+CALLS = ["fp8_rmsnorm_quantize_into", "fp8_gemm_scaled", None, None, "fp8_permute_quantize_heads", "fp8_gemm_accumulate_f32", "fp8_rmsnorm_quantize_into",
+         "fp8_gemm_swiglu_raise", "fp8_quantize_bf16", "fp8_gemm_accumulate_f32"]
+
+
+@pytest.mark.parametrize("kind", ["step", "prompt", "prompt into a cache"])
+def test_a_failed_call_is_named(monkeypatch, kind):
+    from goml_b200 import block_glue as BG, fa_forward as F, fp8_gemm as G
+    calls = list(CALLS)
+    calls[2:4] = {"step": ["fp8_decode_rope_append", "fa_decode"], "prompt": ["fp8_rope_quantize_qkv", "fa_forward_raise"],
+                  "prompt into a cache": ["fp8_rope_quantize_qkv_cache", "fa_forward_raise"]}[kind]
+    blk = block()
+    blk.eps, blk.norm1, blk.norm2 = 1e-5, torch.ones(H * HD), torch.ones(H * HD)
+    blk.gate_up_interleaved = u8(1)
+    blk.qkv = blk.o = blk.gate_up = blk.down = type("Layer", (), {"w": nn.FP8Tensor(u8(1), torch.ones(2))})
+    blk.rope_tables = lambda S, dev: (torch.ones(S, HD // 2), torch.ones(S, HD // 2))
+    blk.fa = type("Context", (), {"ptr": 1, "_msg": lambda self: "why"})()
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: type("Stream", (), {"cuda_stream": 0}))
+    monkeypatch.setattr(nn, "_entry_points", lambda: (1,) * 5)
+    monkeypatch.setattr(F, "FAStatusString", lambda status: f"status {status}")
+    run = {"step": lambda: blk.decode_step(torch.zeros(B, H * HD), cache()), "prompt": lambda: blk.forward_fused(torch.zeros(B * 8, H * HD), B, 8),
+           "prompt into a cache": lambda: blk.forward_fused(torch.zeros(B * 8, H * HD), B, 8, cache())}[kind]
+    for place, name in enumerate(["fp8_block_run", *calls]):
+        monkeypatch.setattr(BG, "BlockRun", lambda *args: place << 16 | 5)
+        error = F.FAError if name.startswith("fa") else G.FP8GEMMError if name.startswith("fp8_gemm") else BG.BlockGlueError
+        with pytest.raises(error) as e:
+            run()
+        assert type(e.value) is error and str(e.value) == (f"{name}: status 5 (why)" if error is F.FAError else f"{name}: CUDA error 5")
+    blk.fa.ptr = 0
+    with pytest.raises(F.FAError, match="FAContext.Decode: nil ctx" if kind == "step" else "FAContext.ForwardEx: nil ctx"):
+        run()
