@@ -38,7 +38,8 @@ int fp8_block_run(const fp8_block_run_args_t* a) {
         return (int)cudaErrorInvalidValue;
     const bool decode = a->decode != 0;
     if (a->batch <= 0 || a->heads <= 0 || a->d_model <= 0 || a->d_model % a->heads != 0 || a->ffn_hidden <= 0) return (int)cudaErrorInvalidValue;
-    if (decode ? a->seq_len != 1 || !a->k_cache : a->seq_len <= 0 || !a->k_codes || !a->v_codes) return (int)cudaErrorInvalidValue;
+    // a prompt's positions are 0 .. seq_len - 1, each of which must have its row of the tables (a step looks at rope_rows itself)
+    if (decode ? a->seq_len != 1 || !a->k_cache : a->seq_len <= 0 || a->rope_rows < a->seq_len || !a->k_codes || !a->v_codes) return (int)cudaErrorInvalidValue;
     if (a->k_cache && (!a->v_cache || !a->cache_scales || !a->cache_lens || a->s_max < a->seq_len)) return (int)cudaErrorInvalidValue;
     if ((long long)a->batch * a->seq_len > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
     const int T = a->batch * a->seq_len, d = a->d_model, H = a->heads, hd = d / H, F = a->ffn_hidden;
