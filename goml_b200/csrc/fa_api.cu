@@ -281,7 +281,7 @@ fa_status_t run(fa_ctx_t* c, const char* who, const fa_sm100::LaunchArgs& a) {
         set_err(c, "%s: the calling thread's current device differs from the context's device", who);
         return FA_ERR_INVALID_ARG;
     }
-    if (fa_sm100::needs_no_scratch && fa_sm100::needs_no_scratch(a)) {
+    if (fa_sm100::needs_no_scratch(a)) {
         e = fa_sm100::launch(a);
         if (e != cudaSuccess) { set_err(c, "%s: launch: %s", who, cudaGetErrorString(e)); return FA_ERR_CUDA; }
         return FA_OK;

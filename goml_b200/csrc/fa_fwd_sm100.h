@@ -29,9 +29,8 @@ struct LaunchArgs {
     uint32_t v_epoch = 0;
 };
 
-// Whether this call's kernel converts V itself: v16_workspace and v_flags may then be null.  Weak, so that the host side can be
-// linked without the kernels (the test of the scratch table), where every call takes scratch.
-__attribute__((weak)) bool needs_no_scratch(const LaunchArgs& a);
+// Whether this call's kernel converts V itself: v16_workspace and v_flags may then be null.
+bool needs_no_scratch(const LaunchArgs& a);
 // Scratch the forward needs otherwise (an fp16 copy of V made by a pre-pass on the same stream).
 size_t workspace_bytes(int bh, int sl, int hd);
 size_t v_flag_count(int bh, int sl);

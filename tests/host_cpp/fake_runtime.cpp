@@ -13,6 +13,7 @@ static std::mutex lock_;
 static std::string log_;
 static size_t next_ = 0x1000;
 static size_t fail_allocation_ = 0;   // the n-th allocation from now on fails
+static int rows_with_scratch_ = 0;    // forwards of shorter sequences take none
 static void note(const std::string& s) {
     std::lock_guard<std::mutex> g(lock_);
     log_ += s + "\n";
@@ -28,6 +29,7 @@ extern "C" {
 const char* fake_log(void) { return log_.c_str(); }
 void fake_clear(void) { log_.clear(); }
 void fake_fail_allocation(size_t nth) { fail_allocation_ = nth; }
+void fake_rows_with_scratch(int rows) { rows_with_scratch_ = rows; }
 
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
@@ -58,6 +60,7 @@ cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 }
 
 namespace fa_sm100 {
+bool needs_no_scratch(const LaunchArgs& a) { return a.sl < rows_with_scratch_; }
 size_t workspace_bytes(int bh, int sl, int hd) { return (size_t)bh * sl * hd * 2; }
 size_t v_flag_count(int bh, int) { return bh; }
 cudaError_t launch(const LaunchArgs& a) { note("launch stream " + n(a.stream) + " scratch " + n(a.v16_workspace) + " flags " + n(a.v_flags)); return cudaSuccess; }

@@ -118,3 +118,17 @@ def test_more_streams_than_places_in_turn(library):
             if stream > 8:
                 assert len([x for x in lines if x.startswith("free")]) == len([x for x in lines if x.startswith("alloc")]) == 1
     ctx.destroy()
+
+
+def test_calls_without_scratch_leave_no_trace(library):
+    # nothing drawn, kept, cleared or recorded; calls with scratch on the same stream go on as they were
+    ctx = Context(library)
+    ctx.forward(3)
+    library.fake_rows_with_scratch(1000)
+    try:
+        for stream in (3, 4):
+            assert ctx.forward(stream) == [f"launch stream {stream} scratch 0 flags 0"]
+    finally:
+        library.fake_rows_with_scratch(0)
+    assert kept(ctx.forward(3)) and not kept(ctx.forward(4))
+    ctx.destroy()
