@@ -31,6 +31,24 @@ def plain_launches(text):
     return set(re.findall(r"(\w+)(?:<[^<>;]*>)?<<<", text))
 
 
+def other_uses(text):
+    """The kernels of a source that are named anywhere but in their definition, a plain launch and an attribute: handed to one of
+    the overlapped launches (launch_pdl, launch_pdl_stream, a lambda around them, cudaLaunchKernelEx)."""
+    rest = re.sub(r"cudaFuncSetAttribute\([^;]*;|\w+(?:<[^<>;]*>)?<<<", "", text)
+    kernels = {fn for fn, body in functions(text) if body.startswith("__global__")}
+    return {k for k in kernels if len(re.findall(rf"\b{k}\b", rest)) > 1}
+
+
+# every kernel of a chain of calls, by source
+OVERLAPPED = {
+    "fa_fwd_sm100.cu": {"fa_fwd_kernel", "v_to_f16_kernel"}, "fa_decode_sm100.cu": {"fa_decode_kernel", "clear_words_kernel"},
+    "fp8_gemm_sm100.cu": {"fp8_gemm_tcgen05_kernel"}, "fp8_gemm_skinny.cuh": {"fp8_gemm_skinny_kernel"}, "one_cluster.cuh": {"one_cluster_kernel"},
+    "fp8_quantize_sm100.cu": {"clear_word_kernel", "amax_kernel", "quant_kernel"},
+    "fp8_block_glue_sm100.cu": {"clear_words_kernel", "rms_stats_kernel", "rms_stats_regs_kernel", "rms_quant_kernel", "qkv_amax_kernel", "qkv_quant_kernel",
+                                "dec_q_amax_kernel", "dec_append_kernel", "dec_lengths_kernel", "o_amax_kernel", "o_quant_kernel", "quant_bf16_kernel"},
+}
+
+
 @pytest.mark.parametrize("name", [n for n, t in sources().items() if re.search(r"__global__|__device__", t)])
 def test_no_read_only_loads_in_overlapped_kernels(name):
     # a kernel that may start before its predecessor on the stream has drained must not read through the read-only path: only
@@ -41,7 +59,16 @@ def test_no_read_only_loads_in_overlapped_kernels(name):
     for fn, body in functions(text):
         if re.search(r"__ldg\s*\(|__restrict__|ld\.global\.nc|ld\.global\.L1::no_allocate\.nc", body):
             assert fn in plain, f"{name}: {fn} reads through the read-only path"
-    assert not plain & set(re.findall(r"launch_pdl\(\s*(\w+)", text))
+    assert not plain & other_uses(text)
+
+
+@pytest.mark.parametrize("name", OVERLAPPED)
+def test_overlapped_kernels_are_seen(name):
+    text = sources()[name]
+    assert other_uses(text) == OVERLAPPED[name]
+    # a plain launch added to any of them is one the test above objects to
+    for kernel in OVERLAPPED[name]:
+        assert plain_launches(f"{text}\n{kernel}<<<1, 1>>>();") & other_uses(f"{text}\n{kernel}<<<1, 1>>>();") == {kernel}
 
 
 def test_the_lane_that_copies_v_is_ordered_behind_the_lane_that_saw_the_flag():
