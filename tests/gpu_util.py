@@ -1,4 +1,6 @@
 """Helpers for the GPU parity tests: torch is used for device memory only."""
+import ctypes as C
+
 import numpy as np
 import torch
 
@@ -47,3 +49,45 @@ def run_attention(ctx, q, k, v, causal=0, window=0, scale=None, v_descale=1.0, e
     torch.cuda.synchronize()
     ctx.DeviceStatus()
     return o.double().cpu().numpy(), (lse.double().cpu().numpy() if want_lse and entry != "forward" else None)
+
+
+class _KernelParams(C.Structure):   # CUDA_KERNEL_NODE_PARAMS_v2
+    _fields_ = [("func", C.c_void_p)] + [(n, C.c_uint) for n in ("gx", "gy", "gz", "bx", "by", "bz", "smem")] + \
+               [(n, C.c_void_p) for n in ("params", "extra", "kern", "ctx")]
+
+
+def captured_nodes(call):
+    """The nodes that call() leaves in a graph: (CUgraphNodeType, name of the kernel or None) each."""
+    cu = C.CDLL("libcuda.so.1")
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+        call()
+    n = C.c_size_t()
+    raw = C.c_void_p(graph.raw_cuda_graph())
+    assert cu.cuGraphGetNodes(raw, None, C.byref(n)) == 0
+    nodes = (C.c_void_p * n.value)()
+    assert cu.cuGraphGetNodes(raw, nodes, C.byref(n)) == 0
+    out = []
+    for node in nodes:
+        t, name = C.c_int(), None
+        assert cu.cuGraphNodeGetType(C.c_void_p(node), C.byref(t)) == 0
+        if t.value == 0:
+            p, text = _KernelParams(), C.c_char_p()
+            assert cu.cuGraphKernelNodeGetParams_v2(C.c_void_p(node), C.byref(p)) == 0
+            got = cu.cuFuncGetName(C.byref(text), C.c_void_p(p.func)) if p.func else cu.cuKernelGetName(C.byref(text), C.c_void_p(p.kern))
+            assert got == 0
+            name = text.value.decode()
+        out.append((t.value, name))
+    return out
+
+
+def kernels(call):
+    """Names (as the linker knows them) of the kernels that call() launches."""
+    return [name for _, name in captured_nodes(call) if name]
+
+
+def has_pre_pass(call):
+    """Whether an attention call has V converted ahead of its kernel."""
+    names = kernels(call)
+    assert sum("fa_fwd_kernel" in n for n in names) == 1
+    return any("v_to_f16_kernel" in n for n in names)

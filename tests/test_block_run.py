@@ -69,3 +69,44 @@ def test_the_same_arguments_unchanged_reach_the_first_call(lib, decode):
     for more in ({}, {} if decode else dict(k_cache=None, v_cache=None, cache_scales=None, cache_lens=None, s_max=0)):
         assert lib.fp8_block_run(C.byref(block(lib, decode, lambda name, n: 0x10000, norm1=0x10001, **more))) == 1 << 16 | INVALID
     assert lib.fp8_block_run(None) == INVALID
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("decode", [False, True])
+def test_place_and_code_of_a_failed_call(cuda, lib, decode):
+    # the other libraries' calls are stand-ins, of which one fails; this library's own are real, and refuse a misaligned or missing
+    # operand.  What stands behind a failed call is not issued
+    import torch
+    real = {}
+
+    def pointer(name, n):
+        real[name] = torch.zeros(n, dtype=torch.uint8, device="cuda")
+        return real[name].data_ptr()
+
+    T, d = B * (1 if decode else S), H * HD
+    attention = "attention_decode" if decode else "attention_raise"
+    order = [("gemm_scaled", 2), (attention, 4), ("gemm_accumulate_f32", 6), ("gemm_swiglu_raise", 8), ("gemm_accumulate_f32", 10)]
+    shapes = {2: (T, 3 * d, d), 6: (T, d, d), 8: (T, F, d), 10: (T, d, F)}
+
+    def run(fails=0, **changed):
+        seen = []
+
+        def entry(name, *args):
+            expected, place = order[len(seen)]
+            seen.append(place)
+            assert name == expected and args[:3] == shapes.get(place, args[:3])
+            return 7 if place == fails else 0
+
+        rc = lib.fp8_block_run(C.byref(block(lib, decode, pointer, entry, **changed)))
+        torch.cuda.synchronize()
+        return rc, seen
+
+    assert run() == (0, [2, 4, 6, 8, 10])
+    for place in (2, 4, 6, 8, 10):
+        assert run(place) == (place << 16 | 7, [p for p in (2, 4, 6, 8, 10) if p <= place])
+    assert run(norm1=None) == (1 << 16 | INVALID, [])
+    assert run(cos_tab=None) == (3 << 16 | INVALID, [2])
+    assert run(norm2=None) == (7 << 16 | INVALID, [2, 4, 6])
+    if decode:   # an odd number of values to quantise
+        shapes[8], shapes[10] = (T, 20, d), (T, d, 20)
+        assert run(ffn_hidden=20) == (9 << 16 | INVALID, [2, 4, 6, 8])

@@ -1,12 +1,13 @@
 """Attention forward where masks cut key blocks (every 32-key chunk of a block is masked, left alone or skipped per warp), and
 where V is converted: by a pre-pass or in the kernel."""
 import math
+import re
 
 import numpy as np
 import pytest
 
 import oracle as O
-from tests.gpu_util import run_attention
+from tests.gpu_util import has_pre_pass, kernels, run_attention
 
 pytestmark = pytest.mark.gpu
 
@@ -49,32 +50,15 @@ def test_v_converted_ahead_and_in_the_kernel_gives_the_same_bits(cuda, built_lib
     for heads in (3, 13):
         o = torch.zeros(heads, s, hd, dtype=torch.float16, device="cuda")
         lse = torch.zeros(heads, s, device="cuda")
-        fa_ctx.ForwardEx(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), heads, s, hd, causal, window, 1e-5, 1.0)
+        call = lambda: fa_ctx.ForwardEx(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), heads, s, hd, causal, window, 1e-5, 1.0, 0, 0, 0,
+                                        torch.cuda.current_stream().cuda_stream)
+        call()
         torch.cuda.synchronize()
+        assert has_pre_pass(call) == (heads == 3)
         fa_ctx.DeviceStatus()
         out.append((o[:3], lse[:3]))
     assert torch.isnan(out[0][0][2, s - 1, 3]) and not torch.isnan(out[0][0][:2]).any()
     assert torch.equal(out[0][0].view(torch.int16), out[1][0].view(torch.int16)) and torch.equal(out[0][1], out[1][1])
-
-
-# calls whose V is converted ahead, with scratch
-AHEAD = {"few tiles": (4, 1300, 128, 0), "hd 64": (6, 2700, 64, 0), "causal": (9, 2700, 128, 1)}
-
-
-@pytest.mark.parametrize("name", AHEAD)
-def test_scratch_of_the_pre_pass(cuda, built_libs, fa_ctx, monkeypatch, name):
-    # the promises of the scratch table, for calls that take the pre-pass
-    from tests import test_fa_scratch_gpu as scratch
-    monkeypatch.setitem(scratch.CALLS, name, lambda: scratch.Forward(*AHEAD[name]))
-    scratch.test_a_graph_gives_the_bits_of_the_eager_call(cuda, built_libs, fa_ctx, name)
-    scratch.test_twenty_streams_give_the_same_bits(cuda, built_libs, fa_ctx, name)
-    scratch.test_streams_that_come_and_go(cuda, built_libs, fa_ctx, name)
-
-
-def test_the_last_context_goes_while_a_pre_pass_is_queued(cuda, built_libs, monkeypatch):
-    from tests import test_fa_scratch_gpu as scratch
-    monkeypatch.setattr(scratch, "LAST_CONTEXT", scratch.LAST_CONTEXT.replace("2048", "4608"))
-    scratch.test_the_last_context_goes_while_work_is_queued_and_a_capture_is_open(cuda, built_libs)
 
 
 @pytest.mark.parametrize("s,hd,causal,window", [(1, 64, 1, 0), (127, 128, 1, 0), (129, 64, 1, 0), (300, 128, 0, 0), (2700, 128, 1, 0), (2700, 64, 0, 0), (256, 128, 0, 0),
@@ -109,7 +93,10 @@ def test_output_rows_copied_whole(cuda, built_libs, fa_ctx, s, heads, causal, wi
     q, k, v = (torch.randint(0, 0x70, (heads, s, 128), generator=g, dtype=torch.uint8, device="cuda") for _ in range(3))
     room = torch.full((heads * s * 128 + 128,), 7.0, dtype=torch.float16, device="cuda")
     o = room[64:-64].view(heads, s, 128)
-    run = lambda i, n, out: fa_ctx.ForwardEx(q[i:].data_ptr(), k[i:].data_ptr(), v[i:].data_ptr(), out.data_ptr(), 0, n, s, 128, causal, window, 1e-5, 1.0)
+    run = lambda i, n, out: fa_ctx.ForwardEx(q[i:].data_ptr(), k[i:].data_ptr(), v[i:].data_ptr(), out.data_ptr(), 0, n, s, 128, causal, window, 1e-5, 1.0, 0, 0, 0,
+                                             torch.cuda.current_stream().cuda_stream)
+    copies = lambda n: any(re.search(r"fa_fwd_kernelILi128ELb[01]ELb[01]ELb0ELb1E", name) for name in kernels(lambda: run(0, n, o)))   # <128, .., .., false, COPY>
+    assert copies(heads) and not copies(2)
     run(0, heads, o)
     for i in (0, heads - 2):
         few = torch.zeros(2, s, 128, dtype=torch.float16, device="cuda")

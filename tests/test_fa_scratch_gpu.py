@@ -4,6 +4,8 @@ import math
 import pytest
 import torch
 
+from tests.gpu_util import captured_nodes, has_pre_pass
+
 pytestmark = pytest.mark.gpu
 
 
@@ -76,7 +78,16 @@ class Forward:
 # every plan of the decode kernel: fixed splits (cut and uncut pairs), a CTA per pair, the freely cut line
 CALLS = {"splits": lambda: Decode(1, 8, 8, 1000, 128), "one split": lambda: Decode(12, 32, 32, 300, 64), "a CTA a pair": lambda: Decode(25, 32, 32, 500, 128),
          "a CTA a pair, hd 64": lambda: Decode(23, 30, 30, 900, 64), "line": lambda: Decode(5, 32, 8, 700, 128), "wide line": lambda: Decode(3, 24, 2, 900, 64),
-         "forward": lambda: Forward(8, 700, 128), "forward, hd 64": lambda: Forward(3, 300, 64, 0)}
+         "forward": lambda: Forward(8, 700, 128), "forward, hd 64": lambda: Forward(3, 300, 64, 0),
+         # V converted ahead, with scratch and flags
+         "ahead, few tiles": lambda: Forward(4, 1300, 128, 0), "ahead, hd 64": lambda: Forward(6, 2700, 64, 0), "ahead, causal": lambda: Forward(9, 2700, 128)}
+
+
+@pytest.mark.parametrize("name", [n for n in CALLS if "forward" in n or "ahead" in n])
+def test_which_forwards_take_scratch(cuda, built_libs, fa_ctx, name):
+    call = CALLS[name]()
+    call.result(fa_ctx)
+    assert has_pre_pass(lambda: call(fa_ctx)) == ("ahead" in name)
 
 
 @pytest.mark.parametrize("name", CALLS)
@@ -107,7 +118,7 @@ def test_twenty_streams_give_the_same_bits(cuda, built_libs, fa_ctx, name):
         assert torch.equal(call.result(fa_ctx, stream), want)
 
 
-@pytest.mark.parametrize("name", ["a CTA a pair", "line", "forward"])
+@pytest.mark.parametrize("name", ["a CTA a pair", "line", "forward", "ahead, few tiles", "ahead, hd 64", "ahead, causal"])
 def test_streams_that_come_and_go(cuda, built_libs, fa_ctx, name):
     # each of twenty streams calls a few times, among many calls of another, so that they take each other's places; queued
     make = CALLS[name]
@@ -126,32 +137,13 @@ def test_streams_that_come_and_go(cuda, built_libs, fa_ctx, name):
     assert all(torch.equal(c.o, want) for c in [busy, *calls])
 
 
-def node_types(graph):
-    import ctypes as C
-    cu = C.CDLL("libcuda.so.1")
-    n = C.c_size_t()
-    raw = C.c_void_p(graph.raw_cuda_graph())
-    assert cu.cuGraphGetNodes(raw, None, C.byref(n)) == 0
-    nodes = (C.c_void_p * n.value)()
-    assert cu.cuGraphGetNodes(raw, nodes, C.byref(n)) == 0
-    out = []
-    for node in nodes:
-        t = C.c_int()
-        assert cu.cuGraphNodeGetType(C.c_void_p(node), C.byref(t)) == 0
-        out.append(t.value)
-    return out
-
-
 @pytest.mark.parametrize("name,kernels,others", [("one split", 1, 0), ("splits", 2, 4), ("a CTA a pair", 1, 0), ("line", 2, 4)])
 def test_nodes_of_a_captured_decode(cuda, built_libs, fa_ctx, name, kernels, others):
     # no memset node, which would part the decode kernel from the kernel ahead; nothing but the kernel where no pair is cut, and
     # else two allocations, their two frees and the kernel that clears the words
     call = CALLS[name]()
     call.result(fa_ctx)
-    graph = torch.cuda.CUDAGraph(keep_graph=True)
-    with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
-        call(fa_ctx)
-    types = node_types(graph)
+    types = [t for t, _ in captured_nodes(lambda: call(fa_ctx))]
     kernel, memset, alloc, free = 0, 2, 10, 11
     assert types.count(kernel) == kernels and types.count(memset) == 0
     assert sorted(t for t in types if t != kernel) == sorted([alloc, free] * (others // 2))
@@ -159,9 +151,11 @@ def test_nodes_of_a_captured_decode(cuda, built_libs, fa_ctx, name, kernels, oth
 
 def test_buffers_that_grow_and_serve_both_entry_points(cuda, built_libs, fa_ctx):
     # large, small, large again and other plans in between, on one stream, queued without a synchronisation
-    calls = [Forward(16, 3000, 128), Forward(1, 40, 64, 0), Decode(1, 8, 8, 1000, 128), Decode(25, 32, 32, 500, 128), Forward(64, 2048, 128),
-             Decode(40, 32, 8, 900, 128), Forward(2, 129, 64), Decode(1, 16, 1, 9000, 64)]
+    ahead = [Forward(16, 3000, 128), Forward(4, 1300, 128, 0), Forward(70, 4000, 128), Forward(6, 2700, 64, 0), Forward(9, 2700, 128)]   # the third: more than is kept
+    calls = [ahead[0], Forward(1, 40, 64, 0), Decode(1, 8, 8, 1000, 128), ahead[1], Decode(25, 32, 32, 500, 128), Forward(64, 2048, 128), ahead[2],
+             Decode(40, 32, 8, 900, 128), ahead[3], Forward(2, 129, 64), ahead[4], Decode(1, 16, 1, 9000, 64)]
     want = [c.result(fa_ctx) for c in calls]
+    assert all(has_pre_pass(lambda: c(fa_ctx)) for c in ahead)
     stream = torch.cuda.Stream()
     for order in (range(len(calls)), reversed(range(len(calls)))):
         for c in calls:
@@ -175,11 +169,14 @@ def test_buffers_that_grow_and_serve_both_entry_points(cuda, built_libs, fa_ctx)
 
 
 @pytest.mark.parametrize("streams,contexts", [(4, 4), (1, 4), (1, 1), (4, 1)])
-def test_threads(cuda, built_libs, fa_ctx, streams, contexts):
+@pytest.mark.parametrize("ahead", [False, True])
+def test_threads(cuda, built_libs, fa_ctx, streams, contexts, ahead):
     # four host threads, each with calls of its own: streams and contexts of their own or shared
     import threading
     from goml_b200 import fa_forward as F
     make = [lambda: Decode(1, 8, 8, 1000, 128), lambda: Forward(8, 700, 128), lambda: Decode(25, 32, 32, 200, 128), lambda: Decode(5, 32, 8, 700, 128)]
+    if ahead:   # forwards that share kept scratch, flags and epoch, one of them larger than another and one beside a decode call
+        make = [CALLS["ahead, few tiles"], CALLS["ahead, hd 64"], lambda: Decode(5, 32, 8, 700, 128), CALLS["ahead, causal"]]
     calls = [[make[(t + i) % 4]() for i in range(3)] for t in range(4)]
     want = [[c.result(fa_ctx) for c in cs] for cs in calls]
     ss = [torch.cuda.Stream() for _ in range(streams)]
@@ -214,13 +211,15 @@ def test_threads(cuda, built_libs, fa_ctx, streams, contexts):
 
 
 LAST_CONTEXT = '''
-import threading, time
+import sys, threading, time
 import torch
 from goml_b200 import fa_forward as F
+from tests.gpu_util import has_pre_pass
+keys, ahead = int(sys.argv[1]), sys.argv[2] == "True"
 codes = lambda *s: torch.randint(0, 0x60, s, dtype=torch.uint8, device="cuda")
-q, k, v = codes(64, 2048, 64), codes(64, 2048, 64), codes(64, 2048, 64)
-o = torch.empty(64, 2048, 64, dtype=torch.float16, device="cuda")
-call = lambda ctx, s: ctx.ForwardEx(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), 0, 64, 2048, 64, 1, 0, 0.1, 0.0125, 0, 0, 0, s.cuda_stream)
+q, k, v = codes(64, keys, 64), codes(64, keys, 64), codes(64, keys, 64)
+o = torch.empty(64, keys, 64, dtype=torch.float16, device="cuda")
+call = lambda ctx, s: ctx.ForwardEx(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), 0, 64, keys, 64, 1, 0, 0.1, 0.0125, 0, 0, 0, s.cuda_stream)
 x = torch.zeros(1 << 20, device="cuda")
 streams = [torch.cuda.Stream() for _ in range(3)]
 ctx = F.FACreate()
@@ -228,6 +227,7 @@ call(ctx, streams[0])
 torch.cuda.synchronize()
 ctx.DeviceStatus()
 want = o.clone()
+assert has_pre_pass(lambda: call(ctx, torch.cuda.current_stream())) == ahead
 ctx.Destroy()
 for again in range(3):
     ctx, other = F.FACreate(), F.FACreate()
@@ -261,11 +261,12 @@ print("fine")
 '''
 
 
-def test_the_last_context_goes_while_work_is_queued_and_a_capture_is_open(cuda, built_libs):
+@pytest.mark.parametrize("keys,ahead", [(2048, False), (4608, True)])
+def test_the_last_context_goes_while_work_is_queued_and_a_capture_is_open(cuda, built_libs, keys, ahead):
     # in a process of its own: no other context of the GPU is left
     import os
     import subprocess
     import sys
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    r = subprocess.run([sys.executable, "-c", LAST_CONTEXT], cwd=root, capture_output=True, text=True, timeout=300)
+    r = subprocess.run([sys.executable, "-c", LAST_CONTEXT, str(keys), str(ahead)], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "fine" in r.stdout, r.stdout + r.stderr

@@ -5,6 +5,8 @@ import math
 import pytest
 import torch
 
+from tests.gpu_util import has_pre_pass, kernels
+
 pytestmark = pytest.mark.gpu
 STEPS = 50
 
@@ -28,9 +30,11 @@ def twice(step, out):
     return got[0]
 
 
-@pytest.mark.parametrize("B,S,H,hd", [(1, 40, 2, 64), (2, 300, 8, 128), (1, 700, 6, 64)])
-def test_rope_quantise_then_attention(cuda, built_libs, fa_ctx, B, S, H, hd):
-    # V and the scales of every step are written by the kernel right ahead of the attention; one cluster and two kernels
+@pytest.mark.parametrize("B,S,H,hd,ahead", [(1, 40, 2, 64, False), (2, 300, 8, 128, False), (1, 700, 6, 64, False), (1, 1300, 4, 128, True), (1, 1100, 2, 64, True),
+                                            (1, 2700, 9, 128, True)])
+def test_rope_quantise_then_attention(cuda, built_libs, fa_ctx, B, S, H, hd, ahead):
+    # V and the scales of every step are written by the kernel right ahead of the attention, one cluster or two kernels; with V
+    # converted in the attention's kernel, and by a pre-pass that hands it on chunk by chunk
     from goml_b200 import block_glue as BG
     g = torch.Generator(device="cuda").manual_seed(S)
     qkv = [(torch.randn(B * S, 3, H, hd, generator=g, device="cuda") * (0.1 + i % 7)).bfloat16() for i in range(STEPS)]
@@ -47,6 +51,8 @@ def test_rope_quantise_then_attention(cuda, built_libs, fa_ctx, B, S, H, hd):
                          sp, sp + 4, sp + 8, stream)
 
     got = twice(step, out)
+    assert has_pre_pass(lambda: fa_ctx.ForwardEx(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), 0, B * H, S, hd, 1, 0, 1.0, 1.0, 0, 0, 0,
+                                                 torch.cuda.current_stream().cuda_stream)) == ahead
     # the first query of a sequence sees one key: its output is that key's V, 2^-4 relative to a code and its fp16 rounding
     want = torch.stack([x.view(B, S, 3, H, hd)[:, 0, 2].reshape(B * H, hd).float() for x in qkv])
     assert ((got[:, :, 0].float() - want).abs() <= 0.07 * want.abs() + 2e-3 * want.abs().amax(dim=(1, 2), keepdim=True)).all()
@@ -85,3 +91,36 @@ def test_append_then_decode(cuda, built_libs, fa_ctx, B, Hq, Hkv, hd, paged):
 
     twice(step, out)
     assert torch.isfinite(out).all() and lens.tolist() == [n + STEPS for n in lens0.tolist()]
+
+
+@pytest.mark.parametrize("M,K,F,N,variant", [(300, 512, 704, 520, "Li64ELi1"), (1000, 1024, 1376, 517, "Li256ELi1"), (2048, 2048, 4736, 520, "Li256ELi2")])
+def test_quantise_then_square_gemm(cuda, built_libs, M, K, F, N, variant):
+    # norm + quantiser -> gate/up GEMM -> quantiser -> GEMM into 16 bits, rows of whole pieces and odd ones -> and the next step's norm
+    # into the codes that the first GEMM has just read; every kernel overlaps the one ahead
+    from goml_b200 import block_glue as BG, fp8_gemm as G
+    g = torch.Generator(device="cuda").manual_seed(M)
+    xs = [torch.randn(M, K, generator=g, device="cuda") * (0.1 + i) for i in range(5)]
+    code = lambda rows, k: torch.randn(rows, k, generator=g, device="cuda").mul_(2).to(torch.float8_e4m3fn).view(torch.uint8)
+    w1, w2 = G.interleave_gate_up(code(2 * F, K), F), code(N, F)
+    gamma = [1 + torch.randn(K, generator=g, device="cuda") * 0.3 for _ in range(STEPS)]
+    empty = lambda *shape, dtype=torch.uint8: torch.empty(shape, dtype=dtype, device="cuda")
+    codes, hb, hc, rstd, w = empty(M, K), empty(M, F, dtype=torch.bfloat16), empty(M, F), empty(M, dtype=torch.float32), empty(5, dtype=torch.float32)
+    out = empty(STEPS, M, N, dtype=torch.bfloat16)
+    p, stream = w.data_ptr(), torch.cuda.current_stream().cuda_stream
+    weight_scale = torch.full((1,), 2.0 ** -7, device="cuda")
+    up = lambda: G.FP8GEMMSwiGLURaise(M, F, K, codes.data_ptr(), w1.data_ptr(), hb.data_ptr(), 1.0, p, weight_scale.data_ptr(), p + 8,
+                                      torch.cuda.current_stream().cuda_stream)
+
+    def step(i):
+        BG.RMSNormQuantizeInto(xs[i % 5].data_ptr(), 0, gamma[i].data_ptr(), codes.data_ptr(), p, p + 4, rstd.data_ptr(), p + 8, M, K, 1e-5, stream)
+        up()
+        BG.QuantizeBF16(hb.data_ptr(), hc.data_ptr(), p + 12, p + 8, M * F, stream)
+        G.FP8GEMMScaled(M, N, F, hc.data_ptr(), w2.data_ptr(), out[i].data_ptr(), 1.0, p + 12, weight_scale.data_ptr(), G.OutBF16, stream)
+
+    got = twice(step, out)
+    assert G.device_status() == 0
+    name, = kernels(up)
+    assert f"fp8_gemm_tcgen05_kernelI{variant}E" in name
+    # the last step against its own codes: bf16 rounding of the result, and of the sums' last bits
+    want = hc.view(torch.float8_e4m3fn).double() @ w2.view(torch.float8_e4m3fn).double().t() * w[3].double() * 2.0 ** -7
+    assert ((got[-1].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * want.abs().max()).all()
