@@ -86,7 +86,12 @@ struct Cfg {
     static constexpr int OFF_V = OFF_K + STAGES * K_BYTES;
     static constexpr int OFF_VRAW = OFF_V + STAGES * V_BYTES;   // codes of V, where the kernel converts them itself
     static constexpr int OFF_BAR = OFF_VRAW + (VRAW ? STAGES * K_BYTES : 0);
-    static constexpr int SMEM_BYTES = OFF_BAR + 256;
+    // Behind a pre-pass a CTA asks for half of an SM's 228 KB (1 KB of which the system takes per CTA): while any CTA of the pre-pass
+    // is left on an SM, no second one fits there, so that the tiles in front, a causal launch's longest, spread over all
+    // SMs first.  With two to an SM from the start (88 KB, and registers for both beside a CTA of the pre-pass) one call behind
+    // another took, D = 128, causal, 4 heads of 4700 65.3 us, 6 of 4790 66.1, 10 of 4608 62.0, now 52.4, 56.9, 58.1.
+    static constexpr int SMEM_BYTES = VRAW ? OFF_BAR + 256 : 113 * 1024;
+    static_assert(OFF_BAR + 256 <= SMEM_BYTES, "everything fits");
     // TMEM: S[0], S[1] (64 fp32 columns each; P of the same block, 32 columns of packed fp16
     //       pairs, overwrites the first half of its S buffer)   O at [128, 128 + HD)
     static constexpr int TMEM_COLS = 256;

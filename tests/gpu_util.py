@@ -57,7 +57,7 @@ class _KernelParams(C.Structure):   # CUDA_KERNEL_NODE_PARAMS_v2
 
 
 def captured_nodes(call):
-    """The nodes that call() leaves in a graph: (CUgraphNodeType, name of the kernel or None) each."""
+    """The nodes that call() leaves in a graph: (CUgraphNodeType, name of the kernel or None, its dynamic shared memory) each."""
     cu = C.CDLL("libcuda.so.1")
     graph = torch.cuda.CUDAGraph(keep_graph=True)
     with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
@@ -69,21 +69,21 @@ def captured_nodes(call):
     assert cu.cuGraphGetNodes(raw, nodes, C.byref(n)) == 0
     out = []
     for node in nodes:
-        t, name = C.c_int(), None
+        t, name, p = C.c_int(), None, _KernelParams()
         assert cu.cuGraphNodeGetType(C.c_void_p(node), C.byref(t)) == 0
         if t.value == 0:
-            p, text = _KernelParams(), C.c_char_p()
+            text = C.c_char_p()
             assert cu.cuGraphKernelNodeGetParams_v2(C.c_void_p(node), C.byref(p)) == 0
             got = cu.cuFuncGetName(C.byref(text), C.c_void_p(p.func)) if p.func else cu.cuKernelGetName(C.byref(text), C.c_void_p(p.kern))
             assert got == 0
             name = text.value.decode()
-        out.append((t.value, name))
+        out.append((t.value, name, p.smem))
     return out
 
 
 def kernels(call):
     """Names (as the linker knows them) of the kernels that call() launches."""
-    return [name for _, name in captured_nodes(call) if name]
+    return [name for _, name, _ in captured_nodes(call) if name]
 
 
 def has_pre_pass(call):

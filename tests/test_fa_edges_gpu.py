@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import oracle as O
-from tests.gpu_util import has_pre_pass, kernels, run_attention
+from tests.gpu_util import captured_nodes, has_pre_pass, kernels, run_attention
 
 pytestmark = pytest.mark.gpu
 
@@ -105,3 +105,23 @@ def test_output_rows_copied_whole(cuda, built_libs, fa_ctx, s, heads, causal, wi
         assert torch.equal(few, o[i:i + 2])
     fa_ctx.DeviceStatus()
     assert torch.isfinite(o).all() and (room[:64] == 7).all() and (room[-64:] == 7).all()
+
+
+def placed(fa_ctx, heads, s, hd, causal, window=0):
+    """Whether V is converted ahead, and how many CTAs of the attention's kernel an SM holds: alone, and beside a CTA of another kernel."""
+    import torch
+    q = torch.zeros(heads, s, hd, dtype=torch.uint8, device="cuda")
+    o = torch.empty(heads, s, hd, dtype=torch.float16, device="cuda")
+    p = q.data_ptr()
+    nodes = captured_nodes(lambda: fa_ctx.ForwardEx(p, p, p, o.data_ptr(), 0, heads, s, hd, causal, window, 1.0, 1.0, 0, 0, 0,
+                                                    torch.cuda.current_stream().cuda_stream))
+    smem, = [bytes_ for _, name, bytes_ in nodes if name and "fa_fwd_kernel" in name]
+    total, taken = torch.cuda.get_device_properties(0).shared_memory_per_multiprocessor, 1024   # what every CTA takes besides
+    fit = lambda room: min(2, room // (smem + taken))   # registers for two
+    return any(name and "v_to_f16" in name for _, name, _ in nodes), fit(total), fit(total - taken)
+
+
+@pytest.mark.parametrize("heads,s,hd,causal,window", [(4, 4700, 128, 1, 0), (10, 5500, 128, 1, 0), (8, 4790, 64, 1, 0), (24, 4096, 128, 0, 0), (70, 8192, 64, 0, 0)])
+def test_tiles_in_front_are_spread_while_the_pre_pass_runs(cuda, built_libs, fa_ctx, heads, s, hd, causal, window):
+    ahead, alone, beside = placed(fa_ctx, heads, s, hd, causal, window)
+    assert ahead and beside == 1 and alone in (1, 2)

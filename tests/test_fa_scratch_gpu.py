@@ -143,7 +143,7 @@ def test_nodes_of_a_captured_decode(cuda, built_libs, fa_ctx, name, kernels, oth
     # else two allocations, their two frees and the kernel that clears the words
     call = CALLS[name]()
     call.result(fa_ctx)
-    types = [t for t, _ in captured_nodes(lambda: call(fa_ctx))]
+    types = [t for t, _, _ in captured_nodes(lambda: call(fa_ctx))]
     kernel, memset, alloc, free = 0, 2, 10, 11
     assert types.count(kernel) == kernels and types.count(memset) == 0
     assert sorted(t for t in types if t != kernel) == sorted([alloc, free] * (others // 2))
