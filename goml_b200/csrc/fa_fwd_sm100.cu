@@ -55,6 +55,7 @@ constexpr int BM = 128;  // query rows per CTA (= TMEM lanes)
 constexpr int BN = 64;   // keys per block
 constexpr int STAGES = 3; // K / V shared-memory ring depth
 constexpr int NUM_SOFTMAX_WARPS = 4;   // one thread per query row
+constexpr int SMEM_ONE = 120 * 1024;   // dynamic shared memory of a CTA that is to have an SM to itself
 constexpr int HEAD_GROUP = 16;         // heads whose tiles are interleaved when tiles differ in length (48 MB of K/V at S = 8192, D = 128)
 constexpr int NUM_THREADS = (NUM_SOFTMAX_WARPS + 2) * 32;
 constexpr int MMA_WARP = NUM_SOFTMAX_WARPS;
@@ -799,6 +800,18 @@ bool converts_v(const LaunchArgs& a, int num_sms) {
     return (a.causal && span == a.sl ? (long long)a.sl * 3 / 5 : span) <= limit;
 }
 
+// Whether a CTA asks for more than half of an SM's shared memory, so that no two share one.  The CTAs of an early launch go where
+// the kernel ahead has drained first, two to such an SM, and with few more tiles than SMs the longest ones of a causal launch, in
+// front, then pair up while other SMs have a short one.  One to an SM, the short ones start where middle ones have finished.  Up to
+// one and a half tiles per SM that was the faster form or level for up to 16 heads; with more heads a sequence has so few tiles that
+// their start and finish count, which two to an SM hide (32 heads of 700 keys of 64, 192 tiles: 11 / 13 us).
+// Behind the kernel that writes Q, K and V, us for both kernels, before V was converted in here / since / one to an SM: D = 64, 5
+// heads of 4000 54.9 / 61.2 / 48.7, 6 of 3500 51.0 / 56.7 / 44.6, 8 of 3000 47.7 / 50.0 / 40.2.  One call behind another: the same
+// 45.9 / 39.6 / 39.3, 42.1 / 35.5 / 35.2, 38.2 / 31.3 / 30.7; D = 128, 6 of 3500 50.7 / 49.8 / 37.8, 8 of 2000 30.4 / 25.7 / 25.7.
+bool one_to_an_sm(const LaunchArgs& a, long long tiles, int num_sms) {
+    return a.causal && (a.window <= 0 || a.window >= a.sl) && a.bh <= HEAD_GROUP && 2 * tiles <= 3ll * num_sms;
+}
+
 template <int HD, bool VRAW>
 cudaError_t launch_hd(const LaunchArgs& a, int num_sms) {
     using C = Cfg<HD, VRAW>;
@@ -831,7 +844,8 @@ cudaError_t launch_hd(const LaunchArgs& a, int num_sms) {
         if (e != cudaSuccess) return e;
     }
     const bool masked = a.causal || a.window > 0 || (a.sl % BN) != 0 || !(a.scale > 0.f);
-    auto start = [&](auto kernel) { return launch_pdl(kernel, (unsigned)grid, NUM_THREADS, C::SMEM_BYTES, a.stream, tq, tk, tv, p); };
+    const size_t smem = one_to_an_sm(a, grid, num_sms) ? SMEM_ONE : C::SMEM_BYTES;
+    auto start = [&](auto kernel) { return launch_pdl(kernel, (unsigned)grid, NUM_THREADS, smem, a.stream, tq, tk, tv, p); };
     if (a.o_amax) return start(fa_fwd_kernel<HD, true, VRAW, true>);   // the masked kernel serves every call
     if constexpr (HD == 128)
         if (grid > 4ll * num_sms) return masked ? start(fa_fwd_kernel<HD, true, VRAW, false, true>) : start(fa_fwd_kernel<HD, false, VRAW, false, true>);
@@ -844,7 +858,7 @@ namespace {
 void init_device(DeviceState* st, int dev) {
     cudaError_t e = cudaSuccess;
     auto set = [&](auto kernel, int bytes) {
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes > SMEM_ONE ? bytes : SMEM_ONE);
     };
     set(fa_fwd_kernel<128, true, false, false>, Cfg<128, false>::SMEM_BYTES);
     set(fa_fwd_kernel<128, false, false, false>, Cfg<128, false>::SMEM_BYTES);

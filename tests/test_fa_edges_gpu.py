@@ -125,3 +125,24 @@ def placed(fa_ctx, heads, s, hd, causal, window=0):
 def test_tiles_in_front_are_spread_while_the_pre_pass_runs(cuda, built_libs, fa_ctx, heads, s, hd, causal, window):
     ahead, alone, beside = placed(fa_ctx, heads, s, hd, causal, window)
     assert ahead and beside == 1 and alone in (1, 2)
+
+
+@pytest.mark.parametrize("heads,s,hd,causal,window,alone", [(5, 4000, 64, 1, 0, 1), (8, 3000, 64, 1, 3000, 1), (4, 4700, 128, 1, 0, 1), (1, 1, 64, 1, 0, 1),
+                                                            (16, 1664, 64, 1, 0, 1), (16, 1792, 64, 1, 0, 2), (17, 1000, 128, 1, 0, 2), (8, 2500, 64, 1, 500, 2),
+                                                            (8, 2500, 128, 0, 0, 2)])
+def test_few_long_tiles_have_an_sm_each(cuda, built_libs, fa_ctx, heads, s, hd, causal, window, alone):
+    # 148 SMs: up to 222 tiles of up to 16 heads; and the same bits either way, one head at a time among them
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert sms == 148
+    assert placed(fa_ctx, heads, s, hd, causal, window)[1] == alone
+    g = torch.Generator(device="cuda").manual_seed(s)
+    q, k, v = (torch.randint(0, 0x70, (heads, s, hd), generator=g, dtype=torch.uint8, device="cuda") for _ in range(3))
+    o, one = torch.empty(heads, s, hd, dtype=torch.float16, device="cuda"), torch.empty(s, hd, dtype=torch.float16, device="cuda")
+    run = lambda n, i, out: fa_ctx.ForwardEx(q[i:].data_ptr(), k[i:].data_ptr(), v[i:].data_ptr(), out.data_ptr(), 0, n, s, hd, causal, window, 1e-5, 1.0)
+    run(heads, 0, o)
+    for i in (0, heads - 1):
+        run(1, i, one)
+        torch.cuda.synchronize()
+        assert torch.equal(one, o[i])
+    fa_ctx.DeviceStatus()
