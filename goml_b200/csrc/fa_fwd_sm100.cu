@@ -57,6 +57,7 @@ constexpr int STAGES = 3; // K / V shared-memory ring depth
 constexpr int NUM_SOFTMAX_WARPS = 4;   // one thread per query row
 constexpr int SMEM_ONE = 120 * 1024;   // dynamic shared memory of a CTA that is to have an SM to itself
 constexpr int HEAD_GROUP = 16;         // heads whose tiles are interleaved when tiles differ in length (48 MB of K/V at S = 8192, D = 128)
+constexpr long long GROUP_ELEMS = 1ll << 24;   // S * D of a larger group: as much K/V
 constexpr int NUM_THREADS = (NUM_SOFTMAX_WARPS + 2) * 32;
 constexpr int MMA_WARP = NUM_SOFTMAX_WARPS;
 constexpr int TMA_WARP = NUM_SOFTMAX_WARPS + 1;
@@ -113,6 +114,7 @@ struct Params {
     const uint32_t* v_flags;
     uint32_t v_epoch;
     int v_chunks;              // chunks per head
+    int group;                 // heads whose tiles are interleaved
 };
 
 __device__ __forceinline__ float ex2(float x) {
@@ -328,16 +330,16 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
 
     // tile -> (head, query tile).  Tiles of equal cost go head by head, so that the CTAs in
     // flight share a few heads' K/V in L2.  When the key range depends on the query tile
-    // (causal, window) the heads are taken in groups of HEAD_GROUP, and inside a group the
+    // (causal, window) the heads are taken in groups (heads_together), and inside a group the
     // tiles with the most keys come first across all its heads: the last CTAs of the launch
     // are then the short tiles of a whole group, not the long tiles of the last head.
     int head, qt;
     if (p.causal || p.window > 0) {
-        const int per_group = HEAD_GROUP * p.n_qtiles;
+        const int per_group = p.group * p.n_qtiles;
         const int g = blockIdx.x / per_group;
         const int r = blockIdx.x - g * per_group;
-        const int heads_here = min(HEAD_GROUP, p.bh - g * HEAD_GROUP);
-        head = g * HEAD_GROUP + r % heads_here;
+        const int heads_here = min(p.group, p.bh - g * p.group);
+        head = g * p.group + r % heads_here;
         qt = p.n_qtiles - 1 - r / heads_here;
     } else {
         head = blockIdx.x / p.n_qtiles;
@@ -800,6 +802,20 @@ bool converts_v(const LaunchArgs& a, int num_sms) {
     return (a.causal && span == a.sl ? (long long)a.sl * 3 / 5 : span) <= limit;
 }
 
+// Heads whose tiles are interleaved, the longest of all of them first, where tiles differ in length.  With 17 to 24 heads in groups of 16
+// the long tiles of the last few heads ended the launch, and converting V made them longer.  So it is one group, or
+// equal ones, of as many heads as 48 MB of K and V allow; but up to three tiles per SM two or more full groups of 16 stay (32 heads
+// of 1300 23.0 us / 24.4 in one, 32 of 1600 30.2 / 30.9).  D = 128, causal, one call behind another, before V was converted in here /
+// since, in groups of 16 / now: 17 heads of 2560 47.9 / 54.5 / 36.2, 20 of 2200 44.3 / 48.6 / 33.3, 24 of 2048 37.3 / 39.1 / 32.9, 32 of 2048
+// 43.3 / 44.2 / 41.0, 40 of 2048 61.9 / 56.5 / 45.7, 256 of 2048 298 / 272 / 267; a window of 300, 128 of 2500 134.7 / 106.0 / 107.2.
+int heads_together(const LaunchArgs& a, long long tiles, int num_sms) {
+    const bool full = a.bh % HEAD_GROUP == 0 || a.bh % HEAD_GROUP >= HEAD_GROUP - 2;
+    long long most = GROUP_ELEMS / ((long long)a.sl * a.hd);
+    if (most < HEAD_GROUP || (full && tiles <= 3ll * num_sms)) most = HEAD_GROUP;
+    const long long groups = (a.bh + most - 1) / most;
+    return (int)((a.bh + groups - 1) / groups);
+}
+
 // Whether a CTA asks for more than half of an SM's shared memory, so that no two share one.  The CTAs of an early launch go where
 // the kernel ahead has drained first, two to such an SM, and with few more tiles than SMs the longest ones of a causal launch, in
 // front, then pair up while other SMs have a short one.  One to an SM, the short ones start where middle ones have finished.  Up to
@@ -826,6 +842,7 @@ cudaError_t launch_hd(const LaunchArgs& a, int num_sms) {
                : make_tmap_u16_3d(&tv, a.v16_workspace, a.bh, a.sl, HD, BN, 64, CU_TENSOR_MAP_SWIZZLE_128B)))
         return cudaErrorInvalidValue;
     Params p;
+    p.group = heads_together(a, grid, num_sms);
     p.bh = a.bh; p.sl = a.sl; p.n_qtiles = (a.sl + BM - 1) / BM;
     p.causal = a.causal; p.window = a.window;
     p.scale_log2 = a.scale * 1.4426950408889634f;

@@ -146,3 +146,22 @@ def test_few_long_tiles_have_an_sm_each(cuda, built_libs, fa_ctx, heads, s, hd, 
         torch.cuda.synchronize()
         assert torch.equal(one, o[i])
     fa_ctx.DeviceStatus()
+
+
+@pytest.mark.parametrize("heads", [15, 16, 17, 29, 30, 32, 33, 47, 300])
+@pytest.mark.parametrize("s,hd,window", [(129, 128, 0), (400, 64, 0), (400, 128, 100), (1800, 64, 0)])
+def test_tiles_of_heads_in_one_group_or_several(cuda, built_libs, fa_ctx, heads, s, hd, window):
+    # every tile of every head once: a head's bits do not depend on the heads beside it
+    import torch
+    if heads * s > 100_000:
+        heads = 100_000 // s
+    g = torch.Generator(device="cuda").manual_seed(heads)
+    q, k, v = (torch.randint(0, 0x70, (heads, s, hd), generator=g, dtype=torch.uint8, device="cuda") for _ in range(3))
+    o, few = (torch.full((heads, s, hd), 7.0, dtype=torch.float16, device="cuda") for _ in range(2))
+    run = lambda i, n, out: fa_ctx.ForwardEx(q[i:].data_ptr(), k[i:].data_ptr(), v[i:].data_ptr(), out[i:].data_ptr(), 0, n, s, hd, 1, window, 1e-5, 1.0)
+    run(0, heads, o)
+    for i in range(0, heads, 5):
+        run(i, min(5, heads - i), few)
+    torch.cuda.synchronize()
+    fa_ctx.DeviceStatus()
+    assert torch.equal(o, few)

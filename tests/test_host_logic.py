@@ -134,3 +134,18 @@ def test_argument_blocks_are_packed_as_the_ctypes_structures():
                 bytes(block(*args))
             with pytest.raises(TypeError):
                 F._pack(pack, block, *args)
+
+
+def test_groups_of_heads_cover_the_tiles():
+    # the kernel's arithmetic for the tile of a CTA, over the group sizes that the host may choose
+    for heads in (1, 2, 15, 16, 17, 30, 33, 47, 100):
+        for tiles in (1, 2, 7):
+            for groups in range(1, heads + 1):
+                group = -(-heads // groups)
+                seen = set()
+                for cta in range(heads * tiles):
+                    first = cta // (group * tiles) * group
+                    r, here = cta % (group * tiles), min(group, heads - first)
+                    assert here > 0
+                    seen.add((first + r % here, tiles - 1 - r // here))
+                assert seen == {(h, t) for h in range(heads) for t in range(tiles)}
