@@ -364,12 +364,13 @@ inline cudaError_t init(Fit* fit) {
     return cudaSuccess;
 }
 
-// How a problem is cut, or split = 0 where the square kernel is the faster one.
+// How a problem is cut, or split = 0 where the square kernel is the faster one.  added: the output is added to an fp32 matrix by
+// the copy engine, so that the square kernel cuts a long K as well; codes: it is e4m3.
 struct Plan {
     int split = 0;
     int per_sm = 1;     // CTAs that share an SM and its shared memory
 };
-inline Plan plan(int M, int N, int K, int num_sms, const Fit& fit) {
+inline Plan plan(int M, int N, int K, bool added, bool codes, int num_sms, const Fit& fit) {
     Plan r;
     if (M > MAX_TOKENS) return r;
     const long long weights = (long long)N * K;
@@ -379,7 +380,11 @@ inline Plan plan(int M, int N, int K, int num_sms, const Fit& fit) {
     // needs one row of tiles, for small weights whose K is short: 100 tokens, 2048 x 2048 6.7 / 6.3 us, 8192 x 2048 (128) 9.0 / 7.6, but
     // 4096 x 4096 8.4 / 9.3, 2000 x 3008 7.3 / 7.9, 1024 x 8192 8.4 / 13.6.  Past 128 that one reads the weight twice: 150 tokens, 2048
     // x 2048 7.5 / 6.5, 4096 x 4000 9.9 / 10.0, 2000 x 5008 10.4 / 14.6; 190 tokens, 1504 x 6000 12.1 / 16.5.
-    if (M > 128 ? weights < 1ll << 24 && K < 4800 : M > 80 && weights < 1ll << 25 && K < 3000) return r;
+    // Codes cost this kernel's finish more: 100 tokens, 2048 x 3008 10.8 / 10.3, 3504 long 12.4 / 14.4.  Where the square kernel cuts K
+    // too, it is ahead for all small weights: 100 tokens, 1024 x 8192 7.8 / 5.4 (behind a quantiser 9.5 / 8.2), 2048 x 11008 10.1 / 8.4,
+    // 192, 512 x 8192 9.3 / 5.3, 2048 x 5504 9.8 / 8.1; 4096 x 6000 alone is not (100 tokens 10.7 / 11.9).
+    const int short_k = M > 128 ? 4800 : codes ? 3500 : 3000;
+    if (M > 80 && weights < (M > 128 ? 1ll << 24 : 1ll << 25) && (added || K < short_k)) return r;
     // the K range is cut as long as all slices are resident, one to an SM, and two k-blocks are left to each (16 tokens, 1 / 2 /
     // 3 / 4 slices: 8192 x 8192 17.4 / 13.9 / 14.8 / 13.7 us, of which 2 fit; 4096 x 4096 9.9 / 7.0 / 6.3 / 6.2);
     // past four slices the finish grows faster than the stream shrinks, unless less than three fifths of the SMs are in use and

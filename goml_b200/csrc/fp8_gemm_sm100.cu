@@ -726,7 +726,8 @@ int launch(int M, int N, int K, const void* A, const void* B, void* C, float alp
     p.H = H; p.F = F; p.amax = amax;
     p.D8 = D8; p.scale_d = scale_d;
     // few rows of A: a kernel of its own, without tile pairs or their policy
-    const skinny::Plan few = skinny::plan(M, N, K, st.num_sms, st.skinny_fit);
+    p.x_tma = (X && (N % 4) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0) ? 1 : 0;
+    const skinny::Plan few = skinny::plan(M, N, K, p.x_tma != 0, D8 != nullptr, st.num_sms, st.skinny_fit);
     if (few.split > 0) return skinny::launch(p, few, A, B, stream);
 
     // Tile width: 256 unless a narrower tile cuts (waves x per-k-block MMA time) by more than a quarter —
@@ -764,7 +765,6 @@ int launch(int M, int N, int K, const void* A, const void* B, void* C, float alp
         const long long pair_cost = ((pairs + st.num_sms - 1) / st.num_sms) * 2 * 92;
         if (pair_cost > single_cost) pair = false;
     }
-    p.x_tma = (X && (N % 4) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0) ? 1 : 0;
     p.c_tma = (C && !X && !H && !D8 && (N % 8) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) ? 1 : 0;
     p.h_tma = (H && bn >= 128 && (F % 8) == 0 && (reinterpret_cast<uintptr_t>(H) & 15) == 0) ? 1 : 0;
     p.d_tma = (D8 && !H && !X && bn >= 128 && (N % 16) == 0 && (reinterpret_cast<uintptr_t>(D8) & 15) == 0) ? 1 : 0;

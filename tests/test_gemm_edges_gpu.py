@@ -3,6 +3,8 @@
 import pytest
 import torch
 
+from tests.gpu_util import kernels
+
 pytestmark = pytest.mark.gpu
 
 
@@ -41,3 +43,44 @@ def test_many_tiles_with_rows_of_any_length(cuda, built_libs, M, N, K):
 @pytest.mark.parametrize("N,K", [(1024, 2992), (1024, 3008), (1501, 4784), (1501, 4800), (130, 8192)])
 def test_few_rows_on_both_sides_of_the_lines(cuda, built_libs, M, N, K):
     exact(M, N, K)
+
+
+@pytest.mark.parametrize("M,N,K,offset,few", [(100, 1024, 8192, 0, False), (150, 2048, 5504, 0, False), (192, 512, 8192, 0, False), (81, 2048, 3008, 0, False),
+                                              (80, 1024, 8192, 0, True), (100, 1023, 8192, 0, True), (100, 1024, 8192, 1, True), (128, 4096, 11008, 0, True),
+                                              (150, 3008, 8000, 0, True), (193, 512, 8192, 0, False)])
+def test_added_to_fp32_by_the_kernel_that_cuts_a_long_k_best(cuda, built_libs, M, N, K, offset, few):
+    # offset: values past a 16-byte boundary, where the copy engine cannot add and the square kernel does not cut K
+    from goml_b200 import fp8_gemm as G
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a, b = (torch.randint(-1, 2, (rows, K), generator=g, device="cuda") for rows in (M, N))
+    codes = lambda x: torch.tensor([0xb8, 0x00, 0x38], dtype=torch.uint8, device="cuda")[x + 1].contiguous()
+    ad, bd = codes(a), codes(b)
+    room = torch.full((M * N + 64,), 7.0, device="cuda")
+    x = room[16 + offset:16 + offset + M * N].view(M, N)
+    x.copy_(torch.randint(-9, 10, (M, N), generator=g, device="cuda").float())
+    want = x.double() + a.double() @ b.double().t()
+    call = lambda: G.FP8GEMMAccumulateF32(M, N, K, ad.data_ptr(), bd.data_ptr(), x.data_ptr(), 1.0, 0, 0, torch.cuda.current_stream().cuda_stream)
+    name, = kernels(call)
+    assert ("skinny" in name) == few
+    call()
+    torch.cuda.synchronize()
+    assert G.device_status() == 0 and torch.equal(x.double(), want)
+    assert (room[:16 + offset] == 7).all() and (room[16 + offset + M * N:] == 7).all()
+
+
+@pytest.mark.parametrize("M,K,few", [(80, 3008, True), (100, 3008, False), (128, 3488, False), (128, 3504, True), (150, 4784, False), (150, 4800, True)])
+def test_codes_on_both_sides_of_the_line(cuda, built_libs, M, K, few):
+    from goml_b200 import fp8_gemm as G
+    N = 1024
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a, b = (torch.randint(-1, 2, (rows, K), generator=g, device="cuda") for rows in (M, N))
+    codes = lambda x: torch.tensor([0xb8, 0x00, 0x38], dtype=torch.uint8, device="cuda")[x + 1].contiguous()
+    ad, bd = codes(a), codes(b)
+    d, amax = torch.empty(M, N, dtype=torch.uint8, device="cuda"), torch.zeros(1, device="cuda")
+    call = lambda: G.FP8GEMMFP8Out(M, N, K, ad.data_ptr(), bd.data_ptr(), d.data_ptr(), 1.0, 0, 0, 0, amax.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert ("skinny" in "".join(kernels(call))) == few
+    call()
+    torch.cuda.synchronize()
+    want = (a.double() @ b.double().t())
+    assert amax.item() == want.abs().max().item()
+    assert torch.equal(d.view(torch.float8_e4m3fn).float(), want.float().to(torch.float8_e4m3fn).float())
