@@ -44,9 +44,9 @@ __device__ __forceinline__ void load8(const float* x, float (&v)[8]) {
         v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
     }
 }
-constexpr int BATCH = 4;   // loads of 8 values in flight per thread
 
-template <bool WIDE>
+// BATCH: groups of 8 values in flight per thread
+template <bool WIDE, int BATCH>
 __device__ __forceinline__ float amax_items(const float* x, size_t n, size_t tid, size_t step) {
     const size_t n8 = n / 8;
     float m = 0.f;
@@ -63,11 +63,11 @@ __device__ __forceinline__ float amax_items(const float* x, size_t n, size_t tid
     return m;
 }
 
-template <bool WIDE>
+template <bool WIDE, int BATCH>
 __global__ void __launch_bounds__(THREADS) amax_kernel(const float* x, size_t n, float* amax) {
     pdl_wait();
     pdl_trigger();
-    float m = amax_items<WIDE>(x, n, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x);
+    float m = amax_items<WIDE, BATCH>(x, n, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     __shared__ float wm[THREADS / 32];
@@ -93,7 +93,7 @@ __device__ __forceinline__ uint32_t quant4(const float* v, float inv) {
     return lo | (hi << 16);
 }
 
-template <bool WIDE>
+template <bool WIDE, int BATCH>
 __device__ __forceinline__ void quant_items(const float* x, uint8_t* q, size_t n, size_t tid, size_t step, float amax, float* scale_out,
                                             float divisor) {
     const float scale = (amax > 1e-12f) ? __fdiv_rn(amax, divisor) : 1.0f;
@@ -116,15 +116,15 @@ __device__ __forceinline__ void quant_items(const float* x, uint8_t* q, size_t n
     }
 }
 
-template <bool WIDE>
+template <bool WIDE, int BATCH>
 __global__ void __launch_bounds__(THREADS) quant_kernel(const float* x, uint8_t* q, size_t n, const float* amax_ptr, float* scale_out,
                                                         float divisor) {
     pdl_wait();
     pdl_trigger();
-    quant_items<WIDE>(x, q, n, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x, ld_f32(amax_ptr), scale_out, divisor);
+    quant_items<WIDE, BATCH>(x, q, n, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x, ld_f32(amax_ptr), scale_out, divisor);
 }
 
-template <bool WIDE>
+template <bool WIDE, int BATCH>
 struct QuantOp {
     static constexpr int N = 1;
     const float* x;
@@ -133,10 +133,10 @@ struct QuantOp {
     float* scale_out;
     float* amax_out;
     float divisor;
-    __device__ void pass1(float (&m)[1]) const { m[0] = amax_items<WIDE>(x, n, oc_tid(), OC_STEP); }
+    __device__ void pass1(float (&m)[1]) const { m[0] = amax_items<WIDE, BATCH>(x, n, oc_tid(), OC_STEP); }
     __device__ void pass2(const float (&m)[1]) const {
         if (oc_tid() == 0) *amax_out = m[0];
-        quant_items<WIDE>(x, q, n, oc_tid(), OC_STEP, m[0], scale_out, divisor);
+        quant_items<WIDE, BATCH>(x, q, n, oc_tid(), OC_STEP, m[0], scale_out, divisor);
     }
 };
 
@@ -274,17 +274,31 @@ int grid_for(size_t work_items, int per_sm = 8) {
     return (int)blocks;
 }
 
+template <bool WIDE, int BATCH>
+int quantize_in_two(const float* x, uint8_t* q, float* scale_out, float* amax_out, size_t n, float divisor, dim3 grid, cudaStream_t s) {
+    cudaError_t e = launch_pdl(clear_word_kernel, dim3(1), dim3(1), 0, s, amax_out);
+    if (e == cudaSuccess) e = launch_pdl_stream(n * 4, amax_kernel<WIDE, BATCH>, grid, dim3(THREADS), s, x, n, amax_out);
+    if (e == cudaSuccess) e = launch_pdl_stream(n * 4, quant_kernel<WIDE, BATCH>, grid, dim3(THREADS), s, x, q, n, amax_out, scale_out, divisor);
+    return (int)e;
+}
+
+// Loads past the end are made all the same, of values that the thread has: a small tensor waits for them in vain.  So a thread has
+// as many groups in flight as it has to take.  Before the loads were four / with four / now, us: 4096 values 2.5 / 2.9 / 2.4, of an input
+// that is only 16-byte aligned 2.5 / 3.5 / 2.5; 131072 3.1 / 3.3 / 3.0 and 3.1 / 3.8 / 3.0; 230000 4.6 / 4.5 / 4.1.
 template <bool WIDE>
 int quantize_f32(const float* x, uint8_t* q, float* scale_out, float* amax_out, size_t n, float divisor, cudaStream_t s) {
-    if (n * 4 <= OC_BYTES && oc_fits<QuantOp<WIDE>>()) return (int)oc_launch(QuantOp<WIDE>{x, q, n, scale_out, amax_out, divisor}, s);
-    // One round of BATCH loads per thread, up to four waves of CTAs: with a fixed grid the last round of 3001 rows of 4096 was half
+    const size_t n8 = n / 8;
+    if (n * 4 <= OC_BYTES) {
+        if (n8 <= OC_STEP && oc_fits<QuantOp<WIDE, 1>>()) return (int)oc_launch(QuantOp<WIDE, 1>{x, q, n, scale_out, amax_out, divisor}, s);
+        if ((!WIDE || n8 <= 2 * OC_STEP) && oc_fits<QuantOp<WIDE, 2>>()) return (int)oc_launch(QuantOp<WIDE, 2>{x, q, n, scale_out, amax_out, divisor}, s);
+        if (oc_fits<QuantOp<WIDE, 4>>()) return (int)oc_launch(QuantOp<WIDE, 4>{x, q, n, scale_out, amax_out, divisor}, s);
+    }
+    const size_t one = n8 / THREADS + 1;   // CTAs of one group per thread
+    if ((size_t)grid_for(n8 + 1, 1) >= one) return quantize_in_two<WIDE, 1>(x, q, scale_out, amax_out, n, divisor, dim3((unsigned)one), s);
+    // One round of loads per thread, up to four waves of CTAs: with a fixed grid the last round of 3001 rows of 4096 was half
     // empty.  With loads and stores that are contiguous over a warp (16 values a lane before, 64 bytes apart) from the start of
     // the first pass to that of the GEMM behind the second 26.2 -> 18.4 us, 2 of them the GEMM's earlier start.
-    const dim3 grid(grid_for(n / (8 * BATCH) + 1, 32));
-    cudaError_t e = launch_pdl(clear_word_kernel, dim3(1), dim3(1), 0, s, amax_out);
-    if (e == cudaSuccess) e = launch_pdl_stream(n * 4, amax_kernel<WIDE>, grid, dim3(THREADS), s, x, n, amax_out);
-    if (e == cudaSuccess) e = launch_pdl_stream(n * 4, quant_kernel<WIDE>, grid, dim3(THREADS), s, x, q, n, amax_out, scale_out, divisor);
-    return (int)e;
+    return quantize_in_two<WIDE, 4>(x, q, scale_out, amax_out, n, divisor, dim3(grid_for(n / (8 * 4) + 1, 32)), s);
 }
 
 }  // namespace

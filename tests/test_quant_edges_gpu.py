@@ -7,10 +7,10 @@ import oracle as O
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 7, 8, 9, 4097, 196608, 196609, 300000, 1048583])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 4097, 65543, 65544, 131079, 131080, 196608, 196609, 300000, 303103, 303104, 1048583])
 @pytest.mark.parametrize("offset", [0, 4])
 def test_any_alignment_and_size(cuda, built_libs, n, offset):
-    # one cluster up to 196608 values, two kernels above; offset 4: 16-byte but not 32-byte aligned
+    # one cluster up to 196608 values, two kernels above; one, two or four groups of 8 values in flight; offset 4: 16-byte but not 32-byte aligned
     from goml_b200 import quantize as Q
     g = torch.Generator(device="cuda").manual_seed(n)
     room = torch.randn(n + 16, generator=g, device="cuda") * 3
