@@ -89,7 +89,6 @@ def _init():
                 "fp8_quantize_bf16": [p, p, p, p, z, p],
                 "fp8_residual_add": [p, p, z, p],
                 "fp8_decode_rope_append": [C.POINTER(DecodeAppendArgs)],
-                "fp8_block_run": [C.POINTER(BlockRunArgs)],
             }.items():
                 fn = getattr(lib, name)
                 fn.restype = C.c_int

@@ -74,7 +74,8 @@ enum : uint32_t {
 
 __device__ uint32_t g_fa_status = 0;
 
-// Shared memory holds only TMA-written operand tiles.  Both MMAs are limited by how fast the
+// Shared memory holds the operand tiles: Q, K and the fp16 V, or (VRAW) the codes of V beside the fp16 tiles that the producer warp
+// makes of them; two CTAs an SM either way.  Both MMAs are limited by how fast the
 // tensor core can read its shared-memory operands (128 B/clk/SM), so P never goes through
 // shared memory: it is written to tensor memory and read from there as the A operand.
 template <int HD, bool VRAW>
@@ -305,7 +306,7 @@ __device__ __noinline__ void negate_scores(uint32_t* s) {
 // AMAX = true: the largest |O| also goes to p.o_amax, for the quantiser behind (a variant of its own: the others keep their code).
 // COPY = true: the rows of O leave as one copy each.  That takes the stores off the softmax warps but ends later: with more than
 // two waves of tiles the first counts (256 heads of 2048, causal, 308 -> 302 us, 150 of 512 25.3 -> 24.7), else the second (100 of
-// 300 14.6 -> 15.0, 64 of 700 20.2 -> 20.5).  Not for D = 64, whose copies are of 128 bytes (64 heads of 3000, window 512, 64.8 -> 67.8).
+// 300 14.6 -> 15.0, 64 of 700 20.2 -> 20.5).  The two together are not instantiated: not measured.  Not for D = 64, whose copies are of 128 bytes (64 heads of 3000, window 512, 64.8 -> 67.8).
 template <int HD, bool MASKED, bool VRAW, bool AMAX, bool COPY = false>
 __global__ void __launch_bounds__(NUM_THREADS, 2)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -794,6 +795,8 @@ void init_device(DeviceState* st, int dev);
 // D = 64 converts half as much per block: 64 of 2048 101 / 98, 42 of 3072 143 / 142, 32 of 4096 185 / 186; causal 40 of 4000 147 /
 // 140; window 512 of 3000, 64 heads, 71.2 / 65.0.  Where no more than half of the SMs have a tile, nothing hides the conversion
 // behind another CTA and its cost adds up along the longest tile: 8 heads of 1024 15.4 / 14.0, 4 of 1280 16.8 / 17.4, 1 of 8192 75 / 92.
+// All in a loop of the call; behind the kernel that has just written V the pre-pass costs more, so where both differ little the line
+// is drawn for that: D = 128, not causal, 32 heads of 1536 42.5 / 45.2, but both kernels behind one another 74.5 / 68.8.
 bool converts_v(const LaunchArgs& a, int num_sms) {
     const int limit = a.hd == 128 ? 1536 : 2560;
     const int span = a.causal && a.window > 0 && a.window < a.sl - BM ? a.window + BM : a.sl;   // keys of the longest tile

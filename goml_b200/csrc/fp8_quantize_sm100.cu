@@ -2,9 +2,9 @@
 // (amax reduction + scale + round-to-nearest-even, saturating conversion).
 // HBM-bound: the amax pass reads 4 B/element, the conversion pass reads 4 B and
 // writes 1 B per element (the second read is served from L2 when the tensor
-// fits).  128-bit loads, one 128-bit store per 16 elements, grid sized to a
-// multiple of the SM count.  A small tensor is done by one cluster in one kernel
-// (one_cluster.cuh).
+// fits).  32-byte loads (two of 16 where the input is not 32-byte aligned), an
+// 8-byte store per 8 elements, contiguous over a warp.  A small tensor is done by one
+// cluster in one kernel (one_cluster.cuh).
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
@@ -28,7 +28,6 @@ __global__ void clear_word_kernel(float* w) {
     *w = 0.f;
 }
 
-// |x| maximum of this thread's share of n values
 // Eight neighbouring values: one 32-byte load where x allows it, so that a warp's load is 1 KB in a row.
 template <bool WIDE>
 __device__ __forceinline__ void load8(const float* x, float (&v)[8]) {

@@ -152,8 +152,9 @@ FA_API fa_status_t fa_forward_ex(fa_ctx_t* ctx, const fa_forward_args_t* args);
 FA_API fa_status_t fa_forward_raise(fa_ctx_t* ctx, const fa_forward_args_t* args, float* o_amax);
 
 /* No counterpart in the reference: an attention forward that allocates nothing.
- * The other entry points draw their scratch (an fp16 copy of V, 2*BH*S*D bytes) from a
- * memory pool.  This one is for callers that may not touch the allocator at all — code
+ * Where many queries share a key (long sequences) the other entry points draw scratch (an fp16
+ * copy of V, 2*BH*S*D bytes) from a memory pool; calls whose kernel converts V itself draw none.
+ * This one is for callers that may not touch the allocator at all — code
  * embedded in a framework that reserved the whole GPU up front and forbids later
  * cudaMalloc-family calls, or real-time / safety-certified processes whose device memory
  * map is frozen after start-up.  Its scratch is a fixed 32 MiB device array inside the
