@@ -274,16 +274,22 @@ int grid_for(size_t work_items, int per_sm = 8) {
 }
 
 template <bool WIDE, int BATCH>
-int quantize_in_two(const float* x, uint8_t* q, float* scale_out, float* amax_out, size_t n, float divisor, dim3 grid, cudaStream_t s) {
+int quantize_in_two(const float* x, uint8_t* q, float* scale_out, float* amax_out, size_t n, float divisor, cudaStream_t s) {
+    // One round of BATCH loads per thread, up to four waves of CTAs: with a fixed grid the last round of 3001 rows of 4096 was half
+    // empty.  With loads and stores that are contiguous over a warp (16 values a lane before, 64 bytes apart) from the start of
+    // the first pass to that of the GEMM behind the second 26.2 -> 18.4 us, 2 of them the GEMM's earlier start.
+    const dim3 grid(grid_for(n / (8 * BATCH) + 1, 32));
     cudaError_t e = launch_pdl(clear_word_kernel, dim3(1), dim3(1), 0, s, amax_out);
     if (e == cudaSuccess) e = launch_pdl_stream(n * 4, amax_kernel<WIDE, BATCH>, grid, dim3(THREADS), s, x, n, amax_out);
     if (e == cudaSuccess) e = launch_pdl_stream(n * 4, quant_kernel<WIDE, BATCH>, grid, dim3(THREADS), s, x, q, n, amax_out, scale_out, divisor);
     return (int)e;
 }
 
-// Loads past the end are made all the same, of values that the thread has: a small tensor waits for them in vain.  So a thread has
-// as many groups in flight as it has to take.  Before the loads were four / with four / now, us: 4096 values 2.5 / 2.9 / 2.4, of an input
-// that is only 16-byte aligned 2.5 / 3.5 / 2.5; 131072 3.1 / 3.3 / 3.0 and 3.1 / 3.8 / 3.0; 230000 4.6 / 4.5 / 4.1.
+// Loads past the end are made all the same, of values that the thread has: a small tensor waits for them in vain.  So in one cluster a
+// thread has as many groups in flight as it has to take.  Before the loads were four / with four / now, us: 4096 values 2.5 / 2.9 /
+// 2.4, of an input that is only 16-byte aligned 2.5 / 3.5 / 2.5; 131072 3.1 / 3.3 / 3.0 and 3.1 / 3.8 / 3.0.  In two kernels such an
+// input, whose group is two loads, has two in flight up to a million values (230000 4.5 / 4.7 / 4.3).  One per thread there, in more
+// CTAs, is 0.4 us faster alone, but the few-row GEMM behind it starts late (58 x 2520 x 4528, both: 12.1 / 12.6).
 template <bool WIDE>
 int quantize_f32(const float* x, uint8_t* q, float* scale_out, float* amax_out, size_t n, float divisor, cudaStream_t s) {
     const size_t n8 = n / 8;
@@ -292,12 +298,8 @@ int quantize_f32(const float* x, uint8_t* q, float* scale_out, float* amax_out, 
         if ((!WIDE || n8 <= 2 * OC_STEP) && oc_fits<QuantOp<WIDE, 2>>()) return (int)oc_launch(QuantOp<WIDE, 2>{x, q, n, scale_out, amax_out, divisor}, s);
         if (oc_fits<QuantOp<WIDE, 4>>()) return (int)oc_launch(QuantOp<WIDE, 4>{x, q, n, scale_out, amax_out, divisor}, s);
     }
-    const size_t one = n8 / THREADS + 1;   // CTAs of one group per thread
-    if ((size_t)grid_for(n8 + 1, 1) >= one) return quantize_in_two<WIDE, 1>(x, q, scale_out, amax_out, n, divisor, dim3((unsigned)one), s);
-    // One round of loads per thread, up to four waves of CTAs: with a fixed grid the last round of 3001 rows of 4096 was half
-    // empty.  With loads and stores that are contiguous over a warp (16 values a lane before, 64 bytes apart) from the start of
-    // the first pass to that of the GEMM behind the second 26.2 -> 18.4 us, 2 of them the GEMM's earlier start.
-    return quantize_in_two<WIDE, 4>(x, q, scale_out, amax_out, n, divisor, dim3(grid_for(n / (8 * 4) + 1, 32)), s);
+    if (!WIDE && n < ((size_t)1 << 20)) return quantize_in_two<WIDE, 2>(x, q, scale_out, amax_out, n, divisor, s);
+    return quantize_in_two<WIDE, 4>(x, q, scale_out, amax_out, n, divisor, s);
 }
 
 }  // namespace

@@ -7,7 +7,7 @@ import oracle as O
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 7, 8, 9, 4097, 65543, 65544, 131079, 131080, 196608, 196609, 300000, 303103, 303104, 1048583])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 4097, 65543, 65544, 131079, 131080, 196608, 196609, 300000, 1048575, 1048576, 1048583])
 @pytest.mark.parametrize("offset", [0, 4])
 def test_any_alignment_and_size(cuda, built_libs, n, offset):
     # one cluster up to 196608 values, two kernels above; one, two or four groups of 8 values in flight; offset 4: 16-byte but not 32-byte aligned
