@@ -49,6 +49,7 @@ constexpr int CHUNK = 64;        // keys per unit of work (page sizes are multip
 constexpr int THREADS = 128;
 constexpr int WARPS = THREADS / 32;
 constexpr float LAG = 6.0f;      // log2 units
+constexpr int HINTS = 2;         // chunks a CTA asks for ahead of the wait
 // A wide warp step takes twice the keys of a narrow one (8 against 4 KB in flight per warp) and leaves registers for 12
 // warps per SM instead of 16 (two column tiles: 8 instead of 12, or of 16 for D = 64).  It streams faster (0.8 GB of cache: 137 us against 146); the
 // narrow one lets more CTAs be resident.
@@ -162,6 +163,16 @@ __device__ __forceinline__ void store_out(const DecodeParams& p, size_t row, int
     if (col == 0 && p.lse) p.lse[row] = (L > 0.f) ? (M + log2f(L)) * 0.6931471805599453f : -INFINITY;
 }
 
+// What a hint ahead of the wait is addressed by: read past L1, which the wait does not invalidate.
+__device__ __forceinline__ int peek_s32(const int* p) {
+    int r;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(r) : "l"(p) : "memory");
+    return r;
+}
+__device__ __forceinline__ void prefetch_l2(const uint8_t* p, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 struct Segment {
     int b, kvh, len;                // sequence, kv head, keys of the sequence
     int n_chunks, c_begin, c_end;   // chunks of the pair, and those of them this CTA takes
@@ -178,12 +189,6 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;              // MMA fragment coordinates
-    pdl_wait();
-    pdl_trigger();
-
-    float scale_log2 = p.scale_log2;
-    if (p.sq) scale_log2 *= ld_f32(p.sq);
-    if (p.sk) scale_log2 *= ld_f32(p.sk);
 
     // a sequence with no visible key is on nobody's piece: O = 0, LSE = -inf
     auto empty_sequence = [&](int b) {
@@ -195,9 +200,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
     // ---- this CTA's piece of the line.  Every warp adds the lengths up for itself (no barrier); lane i keeps those of
     // sequences i, i + 32, .. of the first 32 * LENS, larger batches read theirs again where they need them.
     constexpr int LENS = 4;
-    int lens[LENS];
-#pragma unroll
-    for (int i = 0; i < LENS; i++) lens[i] = !STREAMS && p.plan == LINE && 32 * i + lane < p.batch ? seq_len_of(p, 32 * i + lane) : 0;
+    int lens[LENS] = {};
     auto lane_len = [&](int b0) -> int {   // length of sequence b0 + lane, b0 a multiple of 32
         if (b0 < 32 * LENS) {
             int x = lens[0];
@@ -239,40 +242,74 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
         return x;
     };
 
+    auto page_of = [&](int key) -> int { return (int)(__umulhi((uint32_t)key, p.page_mul) >> (p.page_shr - 1)); };
+    // byte offset of chunk c (the same in K and V), or -1 where the table names no page of the pool: nothing is read
+    // there, the keys count as zeros
+    auto offset = [&](const Segment& x, int c, int page) -> long long {
+        if (!PAGED) return (((long long)x.b * p.hkv + x.kvh) * p.s_max + (long long)c * CHUNK) * D;
+        if (page < 0 || page >= p.num_pages) return -1;
+        const int key = c * CHUNK;
+        return (((long long)page * p.hkv + x.kvh) * p.page_size + (key - page_of(key) * p.page_size)) * D;
+    };
+
+    // On the line the first trip is made while the kernel ahead still runs (the append of the new token, usually), which leaves memory idle: this
+    // CTA's first chunks are asked for from L2, by the lengths and the table as they then are.  Those may still be the last step's,
+    // or anything: they are bounded like the ones read behind the wait, and nothing but hints comes of them.  Two chunks for each of 444 CTAs are 14 MB: append and
+    // attention of 24 sequences of 3000 to 6000 keys, 8 kv heads, paged, 49.9 -> 48.8 us (four 49.1, eight 49.8).  A CTA per pair or
+    // split gains nothing (a step of 64 sequences 336 / 341 us, of one 78.1 / 77.7) and makes one trip.
     Segment seg;
     int cut_q = 0, cut_r = 0;
     int mid = 0, mid_end = 0;    // units of the segments still to come in line order
     const bool line = !STREAMS && p.plan == LINE;   // streams are not cut along a line: that code is not compiled for them
-    if (!line) {
-        const int pair = blockIdx.x / p.splits, split = blockIdx.x - pair * p.splits;
-        seg.b = pair / p.hkv;
-        seg.kvh = pair - seg.b * p.hkv;
-        seg.len = seq_len_of(p, seg.b);
-        seg.n_chunks = chunks_of(seg.len);
-        seg.pair_u0 = 0;
-        seg.c_begin = split * p.chunks_per_split;
-        seg.c_end = min(seg.n_chunks, seg.c_begin + p.chunks_per_split);
-        if (seg.n_chunks == 0 && seg.kvh == 0 && split == 0 && threadIdx.x == 0) empty_sequence(seg.b);
-        if (seg.c_begin >= seg.c_end) return;
-    } else {
-        int total = 0;
-        for (int b0 = 0; b0 < p.batch; b0 += 32) {
-            const int b = b0 + lane, n = chunks_of(lane_len(b0));
-            if (n == 0 && b < p.batch && warp == 0 && b % gridDim.x == blockIdx.x) empty_sequence(b);
-            total += __reduce_add_sync(0xffffffffu, n);
+#pragma unroll 1
+    for (int trip = line ? 0 : 1; trip < 2; trip++) {
+        const bool early = !STREAMS && trip == 0;
+        if (!early) {
+            pdl_wait();
+            pdl_trigger();
         }
-        total *= p.hkv;
-        const int pieces = gridDim.x;
-        cut_q = total / pieces;
-        cut_r = total - cut_q * pieces;
-        const Cut cut(cut_q, cut_r);
-        mid = cut.begin(blockIdx.x);
-        mid_end = cut.begin(blockIdx.x + 1);
-        if (mid >= mid_end) return;
-        seg = segment_at(mid, mid_end);
-        if (seg.c_begin >= seg.c_end) return;
-        mid += seg.c_end - seg.c_begin;
+        seg.b = seg.kvh = seg.len = seg.n_chunks = seg.c_begin = seg.c_end = seg.pair_u0 = 0;
+        if (!line) {
+            const int pair = blockIdx.x / p.splits, split = blockIdx.x - pair * p.splits;
+            seg.b = pair / p.hkv;
+            seg.kvh = pair - seg.b * p.hkv;
+            seg.len = seq_len_of(p, seg.b);
+            seg.n_chunks = chunks_of(seg.len);
+            seg.c_begin = split * p.chunks_per_split;
+            seg.c_end = min(seg.n_chunks, seg.c_begin + p.chunks_per_split);
+            if (!early && seg.n_chunks == 0 && seg.kvh == 0 && split == 0 && threadIdx.x == 0) empty_sequence(seg.b);
+        } else {
+#pragma unroll
+            for (int i = 0; i < LENS; i++) lens[i] = 32 * i + lane < p.batch ? seq_len_of(p, 32 * i + lane) : 0;
+            int total = 0;
+            for (int b0 = 0; b0 < p.batch; b0 += 32) {
+                const int b = b0 + lane, n = chunks_of(lane_len(b0));
+                if (!early && n == 0 && b < p.batch && warp == 0 && b % gridDim.x == blockIdx.x) empty_sequence(b);
+                total += __reduce_add_sync(0xffffffffu, n);
+            }
+            total *= p.hkv;
+            const int pieces = gridDim.x;
+            cut_q = total / pieces;
+            cut_r = total - cut_q * pieces;
+            const Cut cut(cut_q, cut_r);
+            mid = cut.begin(blockIdx.x);
+            mid_end = cut.begin(blockIdx.x + 1);
+            if (mid < mid_end) seg = segment_at(mid, mid_end);
+            mid += seg.c_end - seg.c_begin;
+        }
+        if (early) {
+            const int c = seg.c_begin + lane;
+            if (warp < 2 && lane < HINTS && c < seg.c_end) {
+                const long long off = offset(seg, c, PAGED ? peek_s32(p.block_table + (size_t)seg.b * p.max_pages + page_of(c * CHUNK)) : 0);
+                if (off >= 0) prefetch_l2((warp == 0 ? p.k : p.v) + off, (PAGED ? CHUNK : min(CHUNK, p.s_max - c * CHUNK)) * D);
+            }
+            __syncwarp();
+        }
     }
+    if (seg.c_begin >= seg.c_end) return;
+    float scale_log2 = p.scale_log2;
+    if (p.sq) scale_log2 *= ld_f32(p.sq);
+    if (p.sk) scale_log2 *= ld_f32(p.sk);
     const Cut cut(cut_q, cut_r);
 
     // A CTA step is TILES chunks.  Tile i of warp w: keys 16w.. of chunk i (STREAMS), or 16i.. of the warp's own contiguous
@@ -284,17 +321,8 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
     const uint32_t k_lane = g * D + (D / 4) * t, v_lane = 2 * t * D + (D / 8) * g;
     uint32_t kr[C::TILES][2][C::KW];    // [tile][row g / g + 8][words]
     uint32_t vr[C::TILES][4][C::VW];
-    auto page_of = [&](int key) -> int { return (int)(__umulhi((uint32_t)key, p.page_mul) >> (p.page_shr - 1)); };
     auto entry = [&](const Segment& x, int c) -> int {   // table entry of chunk c
         return PAGED && c < x.c_end ? ld_s32(p.block_table + (size_t)x.b * p.max_pages + page_of(c * CHUNK)) : 0;
-    };
-    // byte offset of chunk c (the same in K and V), or -1 where the table names no page of the pool: nothing is read
-    // there, the keys count as zeros
-    auto offset = [&](const Segment& x, int c, int page) -> long long {
-        if (!PAGED) return (((long long)x.b * p.hkv + x.kvh) * p.s_max + (long long)c * CHUNK) * D;
-        if (page < 0 || page >= p.num_pages) return -1;
-        const int key = c * CHUNK;
-        return (((long long)page * p.hkv + x.kvh) * p.page_size + (key - page_of(key) * p.page_size)) * D;
     };
     // left: keys from the chunk's first one to the end of the sequence.  Keys past it are not read but taken as zeros: they
     // may hold anything (0 x NaN would poison O)

@@ -9,7 +9,8 @@
 //  * a kernel whose successor reads before its own wait (the attention forward, behind its V pre-pass) calls
 //    pdl_trigger() only after pdl_wait(): everything ahead of the pair has then completed;
 //  * what any kernel may do before its wait is to ask for lines of an operand to be brought into L2: a hint moves no
-//    data into the SM, and L2 is where stores of the kernel ahead land, so it cannot be stale;
+//    data into the SM, and L2 is where stores of the kernel ahead land, so it cannot be stale.  What only says where a hint goes
+//    (lengths, a block table) may be read for it as well, past L1, if any value leads to an address inside the operand;
 //  * no load of such a kernel takes the read-only path (__ldg, a const __restrict__ pointer): that is for data that nobody
 //    writes while the kernel exists, so it may be served from before the wait, by the compiler or by an L1 line that the
 //    wait does not invalidate.  Plain loads and the ones below are ordered behind the wait.
