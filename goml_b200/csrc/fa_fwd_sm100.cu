@@ -22,13 +22,14 @@
 //   O += P V       : tcgen05.mma kind::f16, A = P read from TMEM, B = V consumed MN-major
 //                    straight from the TMA tile (no shared-memory transpose), fp32
 //                    accumulator in TMEM
-//   epilogue       : O * (v_descale / l) -> fp16, 128-bit stores; LSE.
+//   epilogue       : O * (v_descale / l) -> fp16, staged per warp, 128-bit stores; LSE.
 //
 // The tensor core reads shared-memory operands at 128 B/clk/SM, which is what bounds both
 // MMAs here; keeping P out of shared memory keeps that traffic near the exponential-unit
-// time, which is the next bound (16 ex2 per clock per SM).  One CTA = one 128-row query tile of one head; 6 warps (4 softmax,
-// 1 MMA issuer, 1 TMA producer); two CTAs share an SM so one CTA's softmax overlaps the
-// other's MMAs.  Every mbarrier wait is bounded.
+// time, which is the next bound (16 ex2 per clock per SM).  A CTA works on one 128-row query tile of one head at a time; 6 warps
+// (4 softmax, 1 MMA issuer, 1 TMA producer), or 8 where one converts V; two CTAs share an SM so one CTA's softmax overlaps the
+// other's MMAs.  With more tiles than CTAs fit, a CTA that is about to finish takes over the tile of one that has not been
+// launched yet (cluster launch control), so the order and the balance are the hardware's.  Every mbarrier wait is bounded.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -58,9 +59,11 @@ constexpr int NUM_SOFTMAX_WARPS = 4;   // one thread per query row
 constexpr int SMEM_ONE = 120 * 1024;   // dynamic shared memory of a CTA that is to have an SM to itself
 constexpr int HEAD_GROUP = 16;         // heads whose tiles are interleaved when tiles differ in length (48 MB of K/V at S = 8192, D = 128)
 constexpr long long GROUP_ELEMS = 1ll << 24;   // S * D of a larger group: as much K/V
-constexpr int NUM_THREADS = (NUM_SOFTMAX_WARPS + 2) * 32;
 constexpr int MMA_WARP = NUM_SOFTMAX_WARPS;
 constexpr int TMA_WARP = NUM_SOFTMAX_WARPS + 1;
+constexpr int CONVERT_WARP = NUM_SOFTMAX_WARPS + 2;   // where V has a warp of its own (Cfg::CONVERTER)
+// registers of a thread there: at launch (8 warps, two CTAs an SM), then of a softmax thread; the other half of the CTA gives them up
+constexpr int LAUNCH_REGS = 128, SOFTMAX_REGS = 160, OTHER_REGS = 2 * LAUNCH_REGS - SOFTMAX_REGS;
 constexpr float TAU = 6.0f;   // lazy-rescale threshold (log2 units)
 constexpr float POFF = 2.0f;  // P is carried as P * 2^POFF (max 2^(TAU+POFF) = 256, far inside fp16)
 
@@ -84,11 +87,19 @@ struct Cfg {
     static constexpr int K_BYTES = BN * HD;
     static constexpr int V_BYTES = BN * HD * 2;       // fp16
     static constexpr int V_HALF_BYTES = BN * 128;     // one 64-wide (128-byte) slab of d
+    // A warp of its own converts V, else the producer does.  For D = 128 a block costs a warp 900 of the 1500 clk it may take, and a
+    // producer that also loads and walks falls behind at every tile's start (256 heads of 2048, causal: 310 us, with the warp 284);
+    // for D = 64 it costs 500, and the eighth warp more than it brings (64 of 3000, window 512: 57 us, with the warp 60).
+    static constexpr bool CONVERTER = VRAW && HD == 128;
+    static constexpr int RAW_STAGES = !VRAW ? 0 : HD == 128 ? 2 : 3;
+    static constexpr int STAGE_BYTES = 2048;          // of a softmax warp, for its rows on their way out
+    static constexpr int NUM_THREADS = (CONVERTER ? 8 : NUM_SOFTMAX_WARPS + 2) * 32;
     static constexpr int OFF_Q = 0;
     static constexpr int OFF_K = OFF_Q + Q_BYTES;
     static constexpr int OFF_V = OFF_K + STAGES * K_BYTES;
-    static constexpr int OFF_VRAW = OFF_V + STAGES * V_BYTES;   // codes of V, where the kernel converts them itself
-    static constexpr int OFF_BAR = OFF_VRAW + (VRAW ? STAGES * K_BYTES : 0);
+    static constexpr int OFF_VRAW = OFF_V + STAGES * V_BYTES;   // codes of V, where the kernel converts them itself (D = 128: two stages, all that fits)
+    static constexpr int OFF_STAGE = OFF_VRAW + RAW_STAGES * K_BYTES;
+    static constexpr int OFF_BAR = OFF_STAGE + NUM_SOFTMAX_WARPS * STAGE_BYTES;
     // Behind a pre-pass a CTA asks for half of an SM's 228 KB (1 KB of which the system takes per CTA): while any CTA of the pre-pass
     // is left on an SM, no second one fits there, so that the tiles in front, a causal launch's longest, spread over all
     // SMs first.  With two to an SM from the start (88 KB, and registers for both beside a CTA of the pre-pass) one call behind
@@ -288,10 +299,53 @@ __device__ __forceinline__ void convert_v(uint32_t raw, uint32_t dst) {
     }
 }
 
-// Sign flip of one row of raw scores for a negative scale (the row max is taken on sign-adjusted scores).
-// Rare, so it is kept out of line: the common path pays one not-taken branch instead of 64 predicated ops.
-__device__ __noinline__ void negate_scores(uint32_t* s) {
-    for (int c = 0; c < BN; c++) s[c] ^= 0x80000000u;
+// tile -> (head, query tile).  Tiles of equal cost go head by head, so that the CTAs in
+// flight share a few heads' K/V in L2.  When the key range depends on the query tile
+// (causal, window) the heads are taken in groups (heads_together), and inside a group the
+// tiles with the most keys come first across all its heads: the last CTAs of the launch
+// are then the short tiles of a whole group, not the long tiles of the last head.
+struct Tile {
+    int head, q0;
+    int blk0, nblk;   // key blocks this tile can see: nblk >= 1, or 0 for no tile
+    __device__ __forceinline__ Tile(int4 r) : head(r.x), q0(r.y), blk0(r.z), nblk(r.w) {}
+    __device__ __forceinline__ Tile(const Params& p, int index) {
+        int qt;
+        if (p.causal || p.window > 0) {
+            const int per_group = p.group * p.n_qtiles;
+            const int g = index / per_group;
+            const int r = index - g * per_group;
+            const int heads_here = min(p.group, p.bh - g * p.group);
+            head = g * p.group + r % heads_here;
+            qt = p.n_qtiles - 1 - r / heads_here;
+        } else {
+            head = index / p.n_qtiles;
+            qt = p.n_qtiles - 1 - (index % p.n_qtiles);
+        }
+        q0 = qt * BM;
+        const int kv_hi = p.causal ? min(p.sl, q0 + BM) : p.sl;
+        const int kv_lo = (p.window > 0) ? max(0, q0 - p.window + 1) : 0;
+        blk0 = kv_lo / BN;
+        nblk = (kv_hi + BN - 1) / BN - blk0;
+    }
+};
+
+// The index of the tile that a request of this CTA has taken over from a CTA that had not been launched yet (its blockIdx.x), or
+// -1 where none was left.  By a whole warp, once per request.
+__device__ __forceinline__ int taken_tile(uint32_t response) {
+    int canceled, index;
+    asm volatile("{\n\t.reg .b64 lo, hi;\n\t.reg .b128 r;\n\t.reg .pred p;\n\t"
+                 "ld.shared.v2.b64 {lo, hi}, [%2];\n\tmov.b128 r, {lo, hi};\n\t"
+                 "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\tselp.s32 %0, 1, 0, p;\n\tmov.s32 %1, -1;\n\t"
+                 "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, r;\n\t}"
+                 : "=r"(canceled), "=r"(index) : "r"(response) : "memory");
+    fence_proxy_async_smem();   // the next response overwrites this one
+    __syncwarp();
+    return canceled ? index : -1;
+}
+__device__ __forceinline__ Tile tile_record(uint32_t at) {
+    int4 r;
+    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(at) : "memory");
+    return Tile(r);
 }
 
 // VRAW = true: V arrives as codes, and the producer warp converts each tile in shared memory while it waits for the ring.  That
@@ -304,11 +358,11 @@ __device__ __noinline__ void negate_scores(uint32_t* s) {
 // device-side scale factors are quantiser outputs, amax / 448: never negative.)
 //
 // AMAX = true: the largest |O| also goes to p.o_amax, for the quantiser behind (a variant of its own: the others keep their code).
-// COPY = true: the rows of O leave as one copy each.  That takes the stores off the softmax warps but ends later: with more than
-// two waves of tiles the first counts (256 heads of 2048, causal, 308 -> 302 us, 150 of 512 25.3 -> 24.7), else the second (100 of
-// 300 14.6 -> 15.0, 64 of 700 20.2 -> 20.5).  The two together are not instantiated: not measured.  Not for D = 64, whose copies are of 128 bytes (64 heads of 3000, window 512, 64.8 -> 67.8).
-template <int HD, bool MASKED, bool VRAW, bool AMAX, bool COPY = false>
-__global__ void __launch_bounds__(NUM_THREADS, 2)
+// WALK = true: the CTA goes on to further tiles (walks() has the line).  The roles run through one sequence of blocks across them: the
+// producer asks for a tile with the last block of the one before on its way, loads Q once the last Q K^T has read the old one, and the rings
+// and the two S buffers just go on.
+template <int HD, bool MASKED, bool VRAW, bool AMAX, bool WALK>
+__global__ void __launch_bounds__(Cfg<HD, VRAW>::NUM_THREADS, 2)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
               const __grid_constant__ CUtensorMap tmap_v, const Params p) {
     using C = Cfg<HD, VRAW>;
@@ -322,36 +376,17 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     const uint32_t bar_vfull = bar_kfull + 8 * STAGES;    // [STAGES] V tile landed
     const uint32_t bar_sfull = bar_vfull + 8 * STAGES;    // [STAGES] S = Q K^T of that block complete (K stage reusable)
     const uint32_t bar_pvdone = bar_sfull + 8 * STAGES;   // [STAGES] O += P V of that block complete (V stage reusable)
-    const uint32_t bar_pfull = bar_pvdone + 8 * STAGES;   // [2] softmax wrote P into S[b] (and rescaled O if needed)
-    const uint32_t bar_vraw = bar_pfull + 16;             // [STAGES] codes of a V tile landed
+    const uint32_t bar_pfull = bars + 112;                // [2] softmax wrote P into S[b] (and rescaled O if needed); 16-byte aligned
+    const uint32_t bar_vraw = bar_pfull + 16;             // [RAW_STAGES] codes of a V tile landed
+    const uint32_t bar_vfree = bar_vraw + 8 * STAGES;     // [RAW_STAGES] ... and are converted
+    const uint32_t bar_answer = bar_vfree + 8 * STAGES;   // the answer to a request for another tile is there
+    const uint32_t bar_next = bar_answer + 8;             // the producer has written that tile's record
+    const uint32_t bar_seen = bar_next + 8;               // the other warps have read it
+    const uint32_t response = bars + 208, record = bars + 224;   // 16 bytes each
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_BAR + 240);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const int warp = threadIdx.x >> 5;
-
-    // tile -> (head, query tile).  Tiles of equal cost go head by head, so that the CTAs in
-    // flight share a few heads' K/V in L2.  When the key range depends on the query tile
-    // (causal, window) the heads are taken in groups (heads_together), and inside a group the
-    // tiles with the most keys come first across all its heads: the last CTAs of the launch
-    // are then the short tiles of a whole group, not the long tiles of the last head.
-    int head, qt;
-    if (p.causal || p.window > 0) {
-        const int per_group = p.group * p.n_qtiles;
-        const int g = blockIdx.x / per_group;
-        const int r = blockIdx.x - g * per_group;
-        const int heads_here = min(p.group, p.bh - g * p.group);
-        head = g * p.group + r % heads_here;
-        qt = p.n_qtiles - 1 - r / heads_here;
-    } else {
-        head = blockIdx.x / p.n_qtiles;
-        qt = p.n_qtiles - 1 - (blockIdx.x % p.n_qtiles);
-    }
-    const int q0 = qt * BM;
-    // keys this tile can see: [kv_lo, kv_hi)
-    const int kv_hi = p.causal ? min(p.sl, q0 + BM) : p.sl;
-    const int kv_lo = (p.window > 0) ? max(0, q0 - p.window + 1) : 0;
-    const int blk0 = kv_lo / BN;
-    const int nblk = (kv_hi + BN - 1) / BN - blk0;  // >= 1
 
     if (threadIdx.x == 0) {
         mbar_init(bar_q, 1);
@@ -361,7 +396,11 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
             mbar_init(bar_sfull + 8 * s, 1);
             mbar_init(bar_pvdone + 8 * s, 1);
             mbar_init(bar_vraw + 8 * s, 1);
+            mbar_init(bar_vfree + 8 * s, 1);
         }
+        mbar_init(bar_answer, 1);
+        mbar_init(bar_next, 1);
+        mbar_init(bar_seen, NUM_SOFTMAX_WARPS + 1 + C::CONVERTER);
         for (int b = 0; b < 2; b++) mbar_init(bar_pfull + 8 * b, NUM_SOFTMAX_WARPS * 32);
         *abort_flag = (sbase & 1023u) ? ST_BAD_SMEM_ALIGN : 0u;
         fence_mbar_init();
@@ -378,10 +417,15 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     const uint32_t tmem_o = tmem_base + C::O_COL;
     const bool bad_start = (*abort_flag != 0);
     if (VRAW) pdl_wait();   // no pre-pass has waited for what is ahead
-
+    // Both halves of the CTA take part, the idle warp included.  (In each role's branch: in front of them the compiler gives every
+    // role what the smaller share allows.)
+    auto give_registers = []() {
+        if constexpr (C::CONVERTER) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(OTHER_REGS));
+    };
     if (bad_start) {
         // fall through to teardown
     } else if (warp == TMA_WARP) {
+        give_registers();
         // ------------------------------------------------------------- TMA producer
         // The whole warp runs the loop and one elected lane issues: addresses and coordinates stay warp-uniform.
         {
@@ -390,82 +434,174 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
                 prefetch_tmap(&tmap_q);
                 prefetch_tmap(&tmap_k);
                 prefetch_tmap(&tmap_v);
-                mbar_arrive_expect_tx(bar_q, C::Q_BYTES);
-                tma_load_3d(sbase + C::OFF_Q, &tmap_q, bar_q, 0, q0, head);
             }
-            if (VRAW) {
-                auto load_k = [&](int j) {
-                    const int s = j % STAGES;
-                    mbar_arrive_expect_tx(bar_kfull + 8 * s, C::K_BYTES);
-                    tma_load_3d(sbase + C::OFF_K + s * C::K_BYTES, &tmap_k, bar_kfull + 8 * s, 0, (blk0 + j) * BN, head);
+            bool ok = true;
+            int s = 0, raw = 0;            // ring stages of the next block, of K and V and of the codes of V
+            uint32_t ph = 0, raw_ph = 0;   // their phases
+            uint32_t tph = 0;              // phase of the tile
+            Tile t(p, blockIdx.x);
+            for (bool first = true;; first = false) {          // first tile of this CTA: the rings are empty
+                const int before = s == 0 ? STAGES - 1 : s - 1;
+                const uint32_t before_ph = s == 0 ? ph ^ 1 : ph;
+                auto load_q = [&]() {
+                    mbar_arrive_expect_tx(bar_q, C::Q_BYTES);
+                    tma_load_3d(sbase + C::OFF_Q, &tmap_q, bar_q, 0, t.q0, t.head);
                 };
-                auto load_v = [&](int j) {
-                    const int s = j % STAGES;
-                    mbar_arrive_expect_tx(bar_vraw + 8 * s, C::K_BYTES);
-                    tma_load_3d(sbase + C::OFF_VRAW + s * C::K_BYTES, &tmap_v, bar_vraw + 8 * s, 0, (blk0 + j) * BN, head);
-                };
-                if (leader) {
-                    for (int j = 0; j < STAGES && j < nblk; j++) {
-                        load_k(j);
-                        load_v(j);
+                if (first && leader) load_q();
+                if constexpr (VRAW && !C::CONVERTER) {
+                    auto load_k = [&](int j, int at) {
+                        mbar_arrive_expect_tx(bar_kfull + 8 * at, C::K_BYTES);
+                        tma_load_3d(sbase + C::OFF_K + at * C::K_BYTES, &tmap_k, bar_kfull + 8 * at, 0, (t.blk0 + j) * BN, t.head);
+                    };
+                    auto load_v = [&](int j, int at) {
+                        mbar_arrive_expect_tx(bar_vraw + 8 * at, C::K_BYTES);
+                        tma_load_3d(sbase + C::OFF_VRAW + at * C::K_BYTES, &tmap_v, bar_vraw + 8 * at, 0, (t.blk0 + j) * BN, t.head);
+                    };
+                    const int s0 = s;
+                    const uint32_t ph0 = ph;
+                    if (!first) {
+                        // with the last Q K^T of the tile before, Q and all stages of the K ring are free
+                        ok = mbar_wait_warp(bar_sfull + 8 * before, before_ph, abort_flag, ST_TIMEOUT_LOAD);
+                        if (!ok) break;
+                        if (leader) load_q();
+                    }
+                    if (leader) {
+                        for (int j = 0; j < STAGES && j < t.nblk; j++) {
+                            const int at = s0 + j < STAGES ? s0 + j : s0 + j - STAGES;
+                            load_k(j, at);
+                            load_v(j, at);
+                        }
+                    }
+                    __syncwarp();
+                    for (int j = 0; j < t.nblk; j++) {
+                        ok = mbar_wait_warp(bar_vraw + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD) &&
+                             mbar_wait_warp(bar_pvdone + 8 * s, ph ^ 1, abort_flag, ST_TIMEOUT_LOAD);   // P V three blocks back is done
+                        if (!ok) break;
+                        // and with it every MMA issued before it, Q K^T two blocks back among them: its K stage is free.  (In the third
+                        // block of a tile only the tile before has been waited for: there the first Q K^T is.)
+                        if (j + 1 >= STAGES && j + 1 < t.nblk) {
+                            if (j + 1 == STAGES) ok = mbar_wait_warp(bar_sfull + 8 * s0, ph0, abort_flag, ST_TIMEOUT_LOAD);
+                            if (!ok) break;
+                            if (leader) load_k(j + 1, s + 1 < STAGES ? s + 1 : 0);
+                        }
+                        convert_v<HD>(sbase + C::OFF_VRAW + s * C::K_BYTES, sbase + C::OFF_V + s * C::V_BYTES);
+                        fence_proxy_async_smem();
+                        __syncwarp();
+                        if (leader) {
+                            mbar_arrive(bar_vfull + 8 * s);
+                            if (j + STAGES < t.nblk) load_v(j + STAGES, s);
+                        }
+                        __syncwarp();
+                        if (++s == STAGES) { s = 0; ph ^= 1; }
+                    }
+                } else {
+                    // Q and K are complete when this kernel starts (a pre-pass triggers it after its own wait); the fp16 copy
+                    // of V is waited for chunk by chunk, or as a whole when the launch has no flags
+                    int v_ready = 0;
+                    const uint32_t* head_flags = !VRAW && p.v_flags ? p.v_flags + (size_t)t.head * p.v_chunks : nullptr;
+                    for (int j = 0; j < t.nblk; j++) {
+                        const int key0 = (t.blk0 + j) * BN;
+                        const bool fresh = first && j < STAGES;
+                        ok = fresh || mbar_wait_warp(bar_sfull + 8 * s, ph ^ 1, abort_flag, ST_TIMEOUT_LOAD);   // Q K^T three blocks back is done
+                        if (!ok) break;
+                        if (leader) {
+                            mbar_arrive_expect_tx(bar_kfull + 8 * s, C::K_BYTES);
+                            tma_load_3d(sbase + C::OFF_K + s * C::K_BYTES, &tmap_k, bar_kfull + 8 * s, 0, key0, t.head);
+                        }
+                        if (VRAW) {
+                            ok = (first && j < C::RAW_STAGES) || mbar_wait_warp(bar_vfree + 8 * raw, raw_ph ^ 1, abort_flag, ST_TIMEOUT_LOAD);
+                            if (!ok) break;
+                            if (leader) {
+                                mbar_arrive_expect_tx(bar_vraw + 8 * raw, C::K_BYTES);
+                                tma_load_3d(sbase + C::OFF_VRAW + raw * C::K_BYTES, &tmap_v, bar_vraw + 8 * raw, 0, key0, t.head);
+                            }
+                            if (++raw == C::RAW_STAGES) { raw = 0; raw_ph ^= 1; }
+                        }
+                        if (!first && j == 0) {
+                            // with the last Q K^T of the tile before, Q is free
+                            ok = mbar_wait_warp(bar_sfull + 8 * before, before_ph, abort_flag, ST_TIMEOUT_LOAD);
+                            if (!ok) break;
+                            if (leader) load_q();
+                        }
+                        if (!VRAW) {
+                            ok = fresh || mbar_wait_warp(bar_pvdone + 8 * s, ph ^ 1, abort_flag, ST_TIMEOUT_LOAD);  // P V three blocks back is done
+                            if (!ok) break;
+                            if (!head_flags) {
+                                if (j == 0) pdl_wait();
+                            } else {
+                                ok = wait_v_chunk(head_flags, p.v_chunks, p.v_epoch, key0 / V_CHUNK, v_ready, abort_flag);
+                                if (!ok) break;
+                            }
+                            if (leader) {
+                                mbar_arrive_expect_tx(bar_vfull + 8 * s, C::V_BYTES);
+#pragma unroll
+                                for (int h = 0; h < HD / 64; h++)  // one 64-column (128-byte) slab of d per copy
+                                    tma_load_3d(sbase + C::OFF_V + s * C::V_BYTES + h * C::V_HALF_BYTES, &tmap_v, bar_vfull + 8 * s,
+                                                h * 64, key0, t.head);
+                            }
+                        }
+                        __syncwarp();
+                        if (++s == STAGES) { s = 0; ph ^= 1; }
                     }
                 }
+                if (!ok || !WALK) break;
+                // Another tile is asked for with this one's last block on its way, some three before the softmax warps finish: earlier, the
+                // launch's last tiles would go to whoever asks and not to whoever is done first.
+                if (!first && !mbar_wait_warp(bar_seen, tph ^ 1, abort_flag, ST_TIMEOUT_LOAD)) break;
+                if (leader) {
+                    mbar_arrive_expect_tx(bar_answer, 16);
+                    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+                                 ::"r"(response), "r"(bar_answer) : "memory");
+                }
                 __syncwarp();
-                int s = 0;         // ring stage of block j, of K, of the codes of V and of V alike
-                uint32_t ph = 0;   // phase of block j
+                if (!mbar_wait_warp(bar_answer, tph, abort_flag, ST_TIMEOUT_LOAD)) break;
+                const int index = taken_tile(response);
+                if (index < 0) t.nblk = 0;
+                else t = Tile(p, index);
+                if (leader) {
+                    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(record), "r"(t.head), "r"(t.q0), "r"(t.blk0), "r"(t.nblk) : "memory");
+                    mbar_arrive(bar_next);
+                }
+                __syncwarp();
+                tph ^= 1;
+                if (t.nblk == 0) break;
+            }
+            if (!VRAW) pdl_wait();   // this kernel completes after the pre-pass
+        }
+    } else if (C::CONVERTER && warp == CONVERT_WARP) {
+        give_registers();
+        // ------------------------------------------------------------- V: codes -> fp16
+        if constexpr (C::CONVERTER) {
+            const bool leader = elect_one();
+            bool ok = true;
+            int s = 0, raw = 0;
+            uint32_t ph = 0, raw_ph = 0, tph = 0;
+            for (int nblk = Tile(p, blockIdx.x).nblk;;) {
                 for (int j = 0; j < nblk; j++) {
-                    if (!mbar_wait_warp(bar_vraw + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD)) break;
-                    if (!mbar_wait_warp(bar_pvdone + 8 * s, ph ^ 1, abort_flag, ST_TIMEOUT_LOAD)) break;   // P V three blocks back is done
-                    // and with it every MMA issued before it, Q K^T two blocks back among them: its K stage is free.  (In the third
-                    // block nothing has been waited for yet: there the first Q K^T is.)
-                    if (j + 1 >= STAGES && j + 1 < nblk) {
-                        if (j + 1 == STAGES && !mbar_wait_warp(bar_sfull, 0, abort_flag, ST_TIMEOUT_LOAD)) break;
-                        if (leader) load_k(j + 1);
-                    }
-                    convert_v<HD>(sbase + C::OFF_VRAW + s * C::K_BYTES, sbase + C::OFF_V + s * C::V_BYTES);
+                    ok = mbar_wait_warp(bar_vraw + 8 * raw, raw_ph, abort_flag, ST_TIMEOUT_LOAD) &&
+                         mbar_wait_warp(bar_pvdone + 8 * s, ph ^ 1, abort_flag, ST_TIMEOUT_LOAD);   // P V three blocks back is done
+                    if (!ok) break;
+                    convert_v<HD>(sbase + C::OFF_VRAW + raw * C::K_BYTES, sbase + C::OFF_V + s * C::V_BYTES);
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (leader) {
                         mbar_arrive(bar_vfull + 8 * s);
-                        if (j + STAGES < nblk) load_v(j + STAGES);
+                        mbar_arrive(bar_vfree + 8 * raw);
                     }
                     __syncwarp();
                     if (++s == STAGES) { s = 0; ph ^= 1; }
+                    if (++raw == C::RAW_STAGES) { raw = 0; raw_ph ^= 1; }
                 }
-            } else {
-                // Q and K are complete when this kernel starts (the pre-pass triggered it after its own wait); the fp16 copy
-                // of V is waited for chunk by chunk, or as a whole when the launch has no flags
-                int v_ready = 0;
-                const uint32_t* head_flags = p.v_flags ? p.v_flags + (size_t)head * p.v_chunks : nullptr;
-                int s = 0;
-                uint32_t ph = 1;  // "previous phase complete": the rings start empty
-                for (int j = 0; j < nblk; j++) {
-                    const int key0 = (blk0 + j) * BN;
-                    if (!mbar_wait_warp(bar_sfull + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD)) break;   // Q K^T three blocks back is done
-                    if (leader) {
-                        mbar_arrive_expect_tx(bar_kfull + 8 * s, C::K_BYTES);
-                        tma_load_3d(sbase + C::OFF_K + s * C::K_BYTES, &tmap_k, bar_kfull + 8 * s, 0, key0, head);
-                    }
-                    if (!mbar_wait_warp(bar_pvdone + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD)) break;  // P V three blocks back is done
-                    if (!head_flags) {
-                        if (j == 0) pdl_wait();
-                    } else if (!wait_v_chunk(head_flags, p.v_chunks, p.v_epoch, key0 / V_CHUNK, v_ready, abort_flag)) {
-                        break;
-                    }
-                    if (leader) {
-                        mbar_arrive_expect_tx(bar_vfull + 8 * s, C::V_BYTES);
-#pragma unroll
-                        for (int h = 0; h < HD / 64; h++)  // one 64-column (128-byte) slab of d per copy
-                            tma_load_3d(sbase + C::OFF_V + s * C::V_BYTES + h * C::V_HALF_BYTES, &tmap_v, bar_vfull + 8 * s,
-                                        h * 64, key0, head);
-                    }
-                    __syncwarp();
-                    if (++s == STAGES) { s = 0; ph ^= 1; }
-                }
-                pdl_wait();   // this kernel completes after the pre-pass
+                if (!ok || !WALK || !mbar_wait_warp(bar_next, tph, abort_flag, ST_TIMEOUT_LOAD)) break;
+                nblk = tile_record(record).nblk;
+                __syncwarp();
+                if (leader) mbar_arrive(bar_seen);
+                tph ^= 1;
+                if (nblk == 0) break;
             }
         }
     } else if (warp == MMA_WARP) {
+        give_registers();
         // -------------------------------------------------------------- MMA issuer
         // Whole warp, one elected lane issues (descriptors stay in uniform registers).
         {
@@ -477,7 +613,10 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
             int ks = 0, vs = 0;
             uint32_t kph = 0, vph = 0;
             bool ok = true;
-            auto issue_qk = [&](int j) {  // S[j & 1] = Q K(j)^T
+            uint32_t kb = 0, vb = 0;      // S buffers of the next Q K^T and of the next P V
+            uint32_t pph = 0;             // bit b: phase of P in S[b]
+            uint32_t tph = 0, qph = 0;    // phases of the next tile's record and of Q
+            auto issue_qk = [&]() {       // S[kb] = Q K^T of the next block
                 ok = mbar_wait_warp(bar_kfull + 8 * ks, kph, abort_flag, ST_TIMEOUT_MMA);
                 if (!ok) return;
                 tc_fence_after();
@@ -486,88 +625,120 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
                 if (leader) {
 #pragma unroll
                     for (int k = 0; k < HD / 32; k++)
-                        mma_f8f6f4_ss(tmem_s + (j & 1) * BN, qd + 2 * k, kd + 2 * k, idesc_qk, k != 0);
+                        mma_f8f6f4_ss(tmem_s + kb * BN, qd + 2 * k, kd + 2 * k, idesc_qk, k != 0);
                     mma_commit(bar_sfull + 8 * ks);
                 }
                 __syncwarp();
+                kb ^= 1;
                 if (++ks == STAGES) { ks = 0; kph ^= 1; }
             };
+            // Two blocks' scores are ahead of the P V, across the end of a tile too: behind this tile's last but one P V follows the
+            // next one's first Q K^T, so that the softmax warps have its scores to work on until the last P V is done.
+            int nblk = Tile(p, blockIdx.x).nblk, next = -1;   // blocks of this tile and of the next (-1: not known yet, 0: none)
+            int qk = 0;                                       // Q K^T issued of this tile or, once next >= 0, of the next
             ok = mbar_wait_warp(bar_q, 0, abort_flag, ST_TIMEOUT_MMA);
-            for (int j = 0; j < 2 && j < nblk && ok; j++) issue_qk(j);
-            for (int j = 0; j < nblk && ok; j++) {
-                const int b = j & 1;
-                ok = mbar_wait_warp(bar_vfull + 8 * vs, vph, abort_flag, ST_TIMEOUT_MMA) &&
-                     mbar_wait_warp(bar_pfull + 8 * b, (j >> 1) & 1, abort_flag, ST_TIMEOUT_MMA);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t vaddr = sbase + C::OFF_V + vs * C::V_BYTES;
-                if (leader) {
-#pragma unroll
-                    for (int k = 0; k < BN / 16; k++) {  // 16 keys per MMA: 8 TMEM columns of P, 16 rows of V
-                        const uint64_t vd = mnmajor_desc_sw128(vaddr + k * 16 * 128, C::V_HALF_BYTES);
-                        mma_f16_ts(tmem_o, tmem_s + b * BN + 8 * k, vd, idesc_pv, (j | k) != 0);
+            for (; nblk > 0 && ok;) {
+                for (int j = 0; j < nblk && ok; j++) {
+                    while (ok && (next < 0 ? qk : nblk + qk) < j + 2) {
+                        if (next < 0 && qk == nblk) {
+                            if (!WALK) { next = 0; break; }
+                            ok = mbar_wait_warp(bar_next, tph, abort_flag, ST_TIMEOUT_MMA);
+                            if (!ok) break;
+                            next = tile_record(record).nblk;
+                            __syncwarp();
+                            if (leader) mbar_arrive(bar_seen);
+                            tph ^= 1;
+                            qk = 0;
+                            if (next > 0) {
+                                qph ^= 1;
+                                ok = mbar_wait_warp(bar_q, qph, abort_flag, ST_TIMEOUT_MMA);
+                            }
+                        }
+                        if (!ok || (next >= 0 && qk == next)) break;
+                        issue_qk();
+                        qk++;
                     }
-                    mma_commit(bar_pvdone + 8 * vs);
+                    if (!ok) break;
+                    const uint32_t b = vb;
+                    ok = mbar_wait_warp(bar_vfull + 8 * vs, vph, abort_flag, ST_TIMEOUT_MMA) &&
+                         mbar_wait_warp(bar_pfull + 8 * b, (pph >> b) & 1, abort_flag, ST_TIMEOUT_MMA);
+                    if (!ok) break;
+                    pph ^= 1u << b;
+                    vb ^= 1;
+                    tc_fence_after();
+                    const uint32_t vaddr = sbase + C::OFF_V + vs * C::V_BYTES;
+                    if (leader) {
+#pragma unroll
+                        for (int k = 0; k < BN / 16; k++) {  // 16 keys per MMA: 8 TMEM columns of P, 16 rows of V
+                            const uint64_t vd = mnmajor_desc_sw128(vaddr + k * 16 * 128, C::V_HALF_BYTES);
+                            mma_f16_ts(tmem_o, tmem_s + b * BN + 8 * k, vd, idesc_pv, (j | k) != 0);
+                        }
+                        mma_commit(bar_pvdone + 8 * vs);
+                    }
+                    __syncwarp();
+                    if (++vs == STAGES) { vs = 0; vph ^= 1; }
+                    // S[b] is rewritten by the Q K^T two blocks ahead; it is issued behind this P V on the
+                    // same in-order tensor pipe, so P(j) has been read before S(j+2) lands on it
                 }
-                __syncwarp();
-                if (++vs == STAGES) { vs = 0; vph ^= 1; }
-                // S[b] is rewritten by the Q K^T two blocks ahead; it is issued behind this P V on the
-                // same in-order tensor pipe, so P(j) has been read before S(j+2) lands on it
-                if (j + 2 < nblk) issue_qk(j + 2);
+                nblk = next;   // its first P V, which overwrites O, waits for a P that is published after O has been read
+                next = -1;
             }
         }
-    } else {
+    } else if (warp < NUM_SOFTMAX_WARPS) {
+        if constexpr (C::CONVERTER) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SOFTMAX_REGS));
         // ------------------------------------------- softmax / correction / epilogue
         const int r = threadIdx.x;               // row of the tile = TMEM lane (one thread per row)
-        const int qi = q0 + r;                   // query index in the sequence
         const uint32_t lane_off = uint32_t(warp * 32) << 16;
         float scale_log2 = p.scale_log2;
         if (p.sq) scale_log2 *= ld_f32(p.sq);
         if (p.sk) scale_log2 *= ld_f32(p.sk);
+        const float vds = p.sv ? p.v_descale * ld_f32(p.sv) : p.v_descale;
         const bool neg = scale_log2 < 0.f;       // the row max is taken on sign-adjusted raw scores
         float ascale = fabsf(scale_log2);
         if (ascale == 0.f) ascale = 1e-30f;      // keeps -inf * scale = -inf for masked keys
-        float m_ref = -INFINITY;                 // reference max used in the exponent (log2 units)
-        float m_thr = -INFINITY;                 // m_ref + TAU
-        float nmsub = 0.f;                       // POFF - m_ref (0 while no finite score has been seen)
-        float l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;   // running sum of P * 2^POFF, in four partial sums
-        bool ok = true;
-        int rs = 0;           // ring stage of block j (j % STAGES) and its phase; those of block j-1
+        int rs = 0;           // ring stage of the next block and its phase; those of the block before
         uint32_t rph = 0;
         int rs_prev = 0;
         uint32_t rph_prev = 0;
-        const int hi_key = p.causal ? min(qi, p.sl - 1) : p.sl - 1;   // last visible key of this row
-        const int lo_key = (p.window > 0) ? qi - p.window + 1 : 0;    // first visible key
-        // the same of the first and the last row of this warp
-        const int wq0 = q0 + warp * 32;
-        const int hi_key_first = p.causal ? min(wq0, p.sl - 1) : p.sl - 1, hi_key_last = p.causal ? min(wq0 + 31, p.sl - 1) : p.sl - 1;
-        const int lo_key_first = (p.window > 0) ? wq0 - p.window + 1 : 0, lo_key_last = (p.window > 0) ? lo_key_first + 31 : 0;
+        uint32_t tph = 0;     // phase of the next tile's record
+        uint32_t s_addr = tmem_s + lane_off, p_bar = bar_pfull;   // S buffer of the next block and the barrier of its P (^ BN, ^ 8: the other one)
+        float m_ref, m_thr, nmsub, l0, l1, l2, l3;
+        auto start_tile = [&]() {
+            m_ref = -INFINITY;                   // reference max used in the exponent (log2 units)
+            m_thr = -INFINITY;                   // m_ref + TAU
+            nmsub = 0.f;                         // POFF - m_ref (0 while no finite score has been seen)
+            l0 = l1 = l2 = l3 = 0.f;             // running sum of P * 2^POFF, in four partial sums
+        };
+        Tile t(p, blockIdx.x);
 
-        // One key block, its scores in S[b].  EDGE: the block may hold masked keys, or the scale is negative.
-        auto block = [&](const int j, const int b, auto edge) -> bool {
+        // The scores of key block j of the tile, in the S buffer at sa, and what they do to the reference.  EDGE: the block may hold
+        // masked keys, or the scale is negative.
+        uint32_t sreg[BN];
+        bool hidden[BN / 32];                    // no row of this warp sees these 32 keys: their P is zero
+        auto scores = [&](const int j, const uint32_t sa, auto edge) -> bool {
             constexpr bool EDGE = decltype(edge)::value;
             if (!mbar_wait_warp(bar_sfull + 8 * rs, rph, abort_flag, ST_TIMEOUT_SOFTMAX)) return false;
             tc_fence_after();
-            uint32_t sreg[BN];
 #pragma unroll
-            for (int c = 0; c < BN / 32; c++) tmem_ld_32x32b_x32(tmem_s + lane_off + b * BN + c * 32, sreg + c * 32);
+            for (int c = 0; c < BN / 32; c++) tmem_ld_32x32b_x32(sa + c * 32, sreg + c * 32);
             tmem_ld_wait();
 
-            bool hidden[BN / 32] = {};   // no row of this warp sees these 32 keys: their P is zero
+            hidden[0] = hidden[1] = false;
             if (EDGE) {
-                if (neg) {  // out of line, on a local copy so that sreg stays in registers
-                    uint32_t tmp[BN];
+                if (neg) {
 #pragma unroll
-                    for (int c = 0; c < BN; c++) tmp[c] = sreg[c];
-                    negate_scores(tmp);
-#pragma unroll
-                    for (int c = 0; c < BN; c++) sreg[c] = tmp[c];
+                    for (int c = 0; c < BN; c++) sreg[c] ^= 0x80000000u;   // the row max is taken on sign-adjusted scores
                 }
+                // last and first visible key of this row, and the same of the first and the last row of its warp
+                const int wq0 = t.q0 + warp * 32;
+                const int hi_key = p.causal ? min(t.q0 + r, p.sl - 1) : p.sl - 1, lo_key = p.window > 0 ? t.q0 + r - p.window + 1 : 0;
+                const int hi_key_first = p.causal ? min(wq0, p.sl - 1) : p.sl - 1, hi_key_last = p.causal ? min(wq0 + 31, p.sl - 1) : p.sl - 1;
+                const int lo_key_first = p.window > 0 ? wq0 - p.window + 1 : 0, lo_key_last = p.window > 0 ? lo_key_first + 31 : 0;
                 // What an edge leaves to do is decided per warp and 32 keys: most such chunks are visible to all rows of the
                 // warp or to none, and only those cut by the edge are masked key by key.
 #pragma unroll
                 for (int g = 0; g < BN / 32; g++) {
-                    const int k0 = (blk0 + j) * BN + g * 32;
+                    const int k0 = (t.blk0 + j) * BN + g * 32;
                     hidden[g] = k0 > hi_key_last || k0 + 31 < lo_key_first;
                     if (hidden[g]) {
 #pragma unroll
@@ -620,145 +791,182 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
                 m_thr = m_ref + TAU;
                 nmsub = (m_ref == -INFINITY) ? 0.f : POFF - m_ref;
             }
-
+            return true;
+        };
+        // P of 32 keys of the block: 16 words of packed fp16 pairs, and their part of the row sum
+        auto exponentials = [&](const int g, uint32_t* w, auto edge) {
+            if (decltype(edge)::value && hidden[g]) {
 #pragma unroll
-            for (int g = 0; g < BN / 32; g++) {  // 32 keys -> 16 TMEM columns of packed fp16 pairs
-                uint32_t w[16];
-                if (EDGE && hidden[g]) {
+                for (int q = 0; q < 16; q++) w[q] = 0;
+            } else {
 #pragma unroll
-                    for (int q = 0; q < 16; q++) w[q] = 0;
-                } else {
-#pragma unroll
-                    for (int q = 0; q < 16; q++) {
-                        float x0, x1;
-                        ffma2(x0, x1, __uint_as_float(sreg[g * 32 + q * 2 + 0]), __uint_as_float(sreg[g * 32 + q * 2 + 1]),
-                              ascale, ascale, nmsub, nmsub);
-                        const float p0 = ex2(x0);
-                        const float p1 = ex2(x1);
-                        if (q & 1) fadd2(l2, l3, p0, p1); else fadd2(l0, l1, p0, p1);
-                        w[q] = pack_half2(p0, p1);
-                    }
+                for (int q = 0; q < 16; q++) {
+                    float x0, x1;
+                    ffma2(x0, x1, __uint_as_float(sreg[g * 32 + q * 2 + 0]), __uint_as_float(sreg[g * 32 + q * 2 + 1]),
+                          ascale, ascale, nmsub, nmsub);
+                    const float p0 = ex2(x0);
+                    const float p1 = ex2(x1);
+                    if (q & 1) fadd2(l2, l3, p0, p1); else fadd2(l0, l1, p0, p1);
+                    w[q] = pack_half2(p0, p1);
                 }
-                tmem_st_32x32b_x16(tmem_s + lane_off + b * BN + g * 16, w);  // P overwrites the first half of S[b]
             }
+        };
+        auto publish = [&](const uint32_t pb) {   // P is in tensor memory
             tmem_st_wait();
             tc_fence_before();
-            mbar_arrive(bar_pfull + 8 * b);
+            mbar_arrive(pb);
             rs_prev = rs;
             rph_prev = rph;
             if (++rs == STAGES) { rs = 0; rph ^= 1; }
+        };
+        auto block = [&](const int j, const uint32_t sa, const uint32_t pb, auto edge) -> bool {
+            if (!scores(j, sa, edge)) return false;
+#pragma unroll
+            for (int g = 0; g < BN / 32; g++) {  // 32 keys -> 16 TMEM columns
+                uint32_t w[16];
+                exponentials(g, w, edge);
+                tmem_st_32x32b_x16(sa + g * 16, w);  // P overwrites the first half of its S buffer
+            }
+            publish(pb);
             return true;
         };
-        // Blocks without masked keys (uniform across the CTA) lie between those that start before the window of the tile's
-        // last query, below j_lo, and those that reach past the sequence end or past the tile's first query (causal), from
-        // j_hi on.  They run in a loop of their own, two to a trip, so that the S buffer index and everything derived from it
-        // are constants (it starts at an even block: one more at the window's edge is taken as an edge block if need be).
-        // (One loop with the test in it, masking key by key: 75.4 us for 64 heads of 3000 keys of 64, window 512, now 71.2; 8192
-        // keys causal 477 / 475.  The form of the clear loop matters: `j + 2 <= n` with two calls in its body is 2 % slower.)
-        // With 64-key blocks and 128-query tiles: (blk0 + j + 1) * BN > sl  <=>  j >= sl / BN - blk0;
-        // (blk0 + j + 1) * BN - 1 > q0  <=>  j >= q0 / BN - blk0;  (blk0 + j) * BN < q0 + BM - window  <=>  j < ceil(..) - blk0.
-        if (!MASKED) {
-#pragma unroll 2
-            for (int j = 0; j < nblk; j++)
-                if (!block(j, j & 1, std::false_type())) { ok = false; break; }
-        } else {
-            int j_hi = p.sl / BN - blk0;
-            if (p.causal) j_hi = min(j_hi, q0 / BN - blk0);
-            int j_lo = (p.window > 0 && q0 + BM - p.window > 0) ? (q0 + BM - p.window + BN - 1) / BN - blk0 : 0;
-            j_lo = neg ? nblk : min((j_lo + 1) & ~1, nblk);
-            int j = 0;
-            for (int stop = j_lo;; stop = nblk) {
+        // blocks [j, end), two to a trip where they are clear, so that the S buffer is a constant in each copy.  (The form of this loop
+        // matters: `j + 2 <= n` with two calls in its body is 2 % slower.)
+        auto edge_blocks = [&](int& j, const int end) -> bool {
 #pragma unroll 1
-                for (; j < stop; j++)
-                    if (!block(j, j & 1, std::true_type())) { ok = false; break; }
-                if (!ok || j == nblk) break;
-                const int clear = max(j_hi - j, 0);
+            for (; j < end; j++) {
+                if (!block(j, s_addr, p_bar, std::true_type())) return false;
+                s_addr ^= BN;
+                p_bar ^= 8;
+            }
+            return true;
+        };
+        auto clear_blocks = [&](int& j, const int end) -> bool {
+            const int n = max(end - j, 0);
 #pragma unroll 2
-                for (int i = 0; i < clear; i++)
-                    if (!block(j + i, i & 1, std::false_type())) { ok = false; break; }
-                if (!ok) break;
-                j += clear;
-            }
-        }
+            for (int i = 0; i < n; i++)
+                if (!block(j + i, s_addr ^ (i & 1) * BN, p_bar ^ (i & 1) * 8, std::false_type())) return false;
+            s_addr ^= (n & 1) * BN;
+            p_bar ^= (n & 1) * 8;
+            j += n;
+            return true;
+        };
 
-        // epilogue: O / l (times the V dequantisation scale) -> fp16
-        if (ok && mbar_wait_warp(bar_pvdone + 8 * rs_prev, rph_prev, abort_flag, ST_TIMEOUT_SOFTMAX)) {
+        // O / l (times the V dequantisation scale) -> fp16, and the LSE, of a tile whose last P V has this ring stage
+        auto epilogue = [&](const int head, const int q0, const float l, const float m, const int stage_pv, const uint32_t phase_pv) -> bool {
+            if (!mbar_wait_warp(bar_pvdone + 8 * stage_pv, phase_pv, abort_flag, ST_TIMEOUT_SOFTMAX)) return false;
             tc_fence_after();
-            const float l = (l0 + l1) + (l2 + l3);
-            const float vds = p.sv ? p.v_descale * ld_f32(p.sv) : p.v_descale;
+            const int qi = q0 + r;
             const float inv = (l > 0.f) ? vds / l : 0.f;
-            // O leaves through shared memory: a thread owns one row (HD fp16 = ROWB bytes), which written straight to global makes
-            // every store instruction of a warp touch 32 different lines.  Its place is the (by now idle) rings.
-            //  COPY: each thread stages its row, rows 16 bytes more than their length apart so that eight neighbouring lanes meet
-            //   different banks, and has it copied out whole.
-            //  Else each warp stages its 32 rows — 16-byte chunk c of row r at chunk c ^ (r % CPR), so that both the row-wise writes
-            //   and the read-back are free of bank conflicts — and stores them back as whole 512-byte runs.  Only this warp touches
-            //   its staging area: a __syncwarp() orders the two passes.
-            constexpr int ROWB = HD * 2;            // bytes per output row
-            constexpr int CPR = ROWB / 16;          // 16-byte chunks per row: 16 (D = 128) or 8 (D = 64)
-            constexpr int PITCH = ROWB + 16;
-            const uint32_t own = sbase + C::OFF_K + r * PITCH;
-            static_assert(C::OFF_K + BM * PITCH <= C::OFF_BAR, "the rows fit the rings");
-            uint8_t* stage = smem + C::OFF_K + warp * (32 * ROWB);
-            const int lane = threadIdx.x & 31;
             __half2 top = __float2half2_rn(0.f);
+            // O leaves through shared memory: a thread owns one row, which written straight to global makes every store instruction of a
+            // warp touch 32 lines.  32 columns at a time, each warp stages its 32 rows of 64 bytes — 16-byte
+            // chunk c of row r at chunk c ^ (r / 2 % 4), so that both the row-wise writes and the read-back are free of bank conflicts —
+            // and stores 8 rows an instruction.
+            uint8_t* stage = smem + C::OFF_STAGE + warp * C::STAGE_BYTES;
+            const int lane = threadIdx.x & 31;
+            __half* obase = p.o + ((size_t)head * p.sl + q0 + warp * 32 + (lane >> 2)) * HD + (lane & 3) * 8;
+            const int rows_left = p.sl - (q0 + warp * 32 + (lane >> 2));   // rows of this warp inside the sequence, from the lane's first on
 #pragma unroll
-            for (int c = 0; c < HD / 16; c++) {
-                uint32_t o[16];
-                tmem_ld_32x32b_x16(tmem_o + lane_off + c * 16, o);
+            for (int c = 0; c < HD / 32; c++) {
+                uint32_t o[32];
+                tmem_ld_32x32b_x32(tmem_o + lane_off + c * 32, o);
                 tmem_ld_wait();
+                if (c > 0) __syncwarp();   // the columns before have been read back
 #pragma unroll
-                for (int v = 0; v < 2; v++) {
-                    uint4 w;
-                    w.x = pack_half2(__uint_as_float(o[8 * v + 0]) * inv, __uint_as_float(o[8 * v + 1]) * inv);
-                    w.y = pack_half2(__uint_as_float(o[8 * v + 2]) * inv, __uint_as_float(o[8 * v + 3]) * inv);
-                    w.z = pack_half2(__uint_as_float(o[8 * v + 4]) * inv, __uint_as_float(o[8 * v + 5]) * inv);
-                    w.w = pack_half2(__uint_as_float(o[8 * v + 6]) * inv, __uint_as_float(o[8 * v + 7]) * inv);
-                    if (AMAX) {   // of the rounded values; NaN never wins
-                        const uint32_t x[4] = {w.x, w.y, w.z, w.w};
+                for (int v = 0; v < 4; v++) {
+                    uint32_t w[4];
 #pragma unroll
-                        for (int i = 0; i < 4; i++) top = __hmax2(top, __habs2(*reinterpret_cast<const __half2*>(&x[i])));
+                    for (int i = 0; i < 4; i++) {
+                        w[i] = pack_half2(__uint_as_float(o[8 * v + 2 * i]) * inv, __uint_as_float(o[8 * v + 2 * i + 1]) * inv);
+                        if (AMAX) top = __hmax2(top, __habs2(*reinterpret_cast<const __half2*>(&w[i])));   // of the rounded values; NaN never wins
                     }
-                    const int ch = 2 * c + v;
-                    if (COPY)
-                        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(own + ch * 16), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w) : "memory");
-                    else
-                        *reinterpret_cast<uint4*>(stage + lane * ROWB + ((ch ^ (lane % CPR)) << 4)) = w;
+                    *reinterpret_cast<uint4*>(stage + lane * 64 + ((v ^ ((lane >> 1) & 3)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
                 }
-            }
-            if (COPY) {
-                fence_proxy_async_smem();
-                if (qi < p.sl)
-                    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
-                                 ::"l"(p.o + ((size_t)head * p.sl + qi) * HD), "r"(own), "n"(ROWB) : "memory");
-                tma_store_commit();
-            } else {
                 __syncwarp();
-                constexpr int RPI = 32 / CPR;       // rows per store instruction
-                uint8_t* obase = reinterpret_cast<uint8_t*>(p.o + ((size_t)head * p.sl + q0 + warp * 32) * HD);
-                const int rows_left = p.sl - (q0 + warp * 32);   // rows of this warp inside the sequence
 #pragma unroll
-                for (int i = 0; i < 32 / RPI; i++) {
-                    const int rr = i * RPI + lane / CPR, ch = lane % CPR;
-                    const uint4 w = *reinterpret_cast<const uint4*>(stage + rr * ROWB + ((ch ^ (rr % CPR)) << 4));
-                    if (rr < rows_left) *reinterpret_cast<uint4*>(obase + (size_t)rr * ROWB + (ch << 4)) = w;
+                for (int i = 0; i < 4; i++) {
+                    const int rr = i * 8 + (lane >> 2);
+                    const uint4 w = *reinterpret_cast<const uint4*>(stage + rr * 64 + (((lane & 3) ^ ((rr >> 1) & 3)) << 4));
+                    if (i * 8 < rows_left) *reinterpret_cast<uint4*>(obase + (size_t)i * 8 * HD + c * 32) = w;
                 }
             }
+            if (WALK) __syncwarp();   // the next tile's rows are staged here too
             if (AMAX) {
-                float m = qi < p.sl ? fmaxf(__low2float(top), __high2float(top)) : 0.f;
+                float top1 = qi < p.sl ? fmaxf(__low2float(top), __high2float(top)) : 0.f;
 #pragma unroll
-                for (int i = 16; i > 0; i >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, i));
-                if (lane == 0) atomicMax(reinterpret_cast<unsigned int*>(p.o_amax), __float_as_uint(m));   // ordered like their bits
+                for (int i = 16; i > 0; i >>= 1) top1 = fmaxf(top1, __shfl_xor_sync(0xffffffffu, top1, i));
+                if (lane == 0) atomicMax(reinterpret_cast<unsigned int*>(p.o_amax), __float_as_uint(top1));   // ordered like their bits
             }
             if (p.lse && qi < p.sl) {
                 // sum_j exp(s_j) = l * 2^(m_ref - POFF)  ->  natural-log LSE
-                p.lse[(size_t)head * p.sl + qi] =
-                    (l > 0.f) ? (m_ref - POFF + log2f(l)) * 0.6931471805599453f : -INFINITY;
+                p.lse[(size_t)head * p.sl + qi] = (l > 0.f) ? (m - POFF + log2f(l)) * 0.6931471805599453f : -INFINITY;
             }
-            if (COPY) tma_store_wait_read<0>();   // shared memory outlives the copies' reads
+            return true;
+        };
+
+        start_tile();
+        for (int j = 0;;) {   // one tile per trip, from block j on
+            // Blocks without masked keys (uniform across the CTA) lie between those that start before the window of the tile's
+            // last query, below j_lo, and those that reach past the sequence end or past the tile's first query (causal), from
+            // j_hi on.  They run in a loop of their own.  (One loop with the test in it, masking key by key: 75.4 us for 64 heads of 3000 keys
+            // of 64, window 512, then 71.2; 8192 keys causal 477 / 475.)
+            // With 64-key blocks and 128-query tiles: (blk0 + j + 1) * BN > sl  <=>  j >= sl / BN - blk0;
+            // (blk0 + j + 1) * BN - 1 > q0  <=>  j >= q0 / BN - blk0;  (blk0 + j) * BN < q0 + BM - window  <=>  j < ceil(..) - blk0.
+            bool ok;
+            if (!MASKED) {
+                ok = clear_blocks(j, t.nblk);
+            } else {
+                int j_hi = p.sl / BN - t.blk0;
+                if (p.causal) j_hi = min(j_hi, t.q0 / BN - t.blk0);
+                int j_lo = (p.window > 0 && t.q0 + BM - p.window > 0) ? (t.q0 + BM - p.window + BN - 1) / BN - t.blk0 : 0;
+                j_lo = neg ? t.nblk : min(j_lo, t.nblk);
+                // one copy of each loop: edge, clear, edge
+                ok = true;
+                for (int stop = j_lo;; stop = t.nblk) {
+                    ok = edge_blocks(j, stop);
+                    if (!ok || j == t.nblk) break;
+                    ok = clear_blocks(j, j_hi);
+                    if (!ok) break;
+                }
+            }
+            if (!ok) break;
+            const float l = (l0 + l1) + (l2 + l3), m = m_ref;
+            const int head = t.head, q0 = t.q0, stage_pv = rs_prev;
+            const uint32_t phase_pv = rph_prev;
+            if (WALK) {
+                if (!mbar_wait_warp(bar_next, tph, abort_flag, ST_TIMEOUT_SOFTMAX)) break;
+                t = tile_record(record);
+                __syncwarp();
+                if ((threadIdx.x & 31) == 0) mbar_arrive(bar_seen);
+                tph ^= 1;
+            }
+            if (!WALK || MASKED || t.nblk == 0) {
+                if (!epilogue(head, q0, l, m, stage_pv, phase_pv) || !WALK || t.nblk == 0) break;
+                start_tile();
+                j = 0;
+                continue;
+            }
+            // The next tile's first block is worked on while this tile's last P V runs; its P is published once O has been read.  (512 heads
+            // of 512, D = 64, 61.6 -> 51.8 us, of which this is 3.  With it the masked kernel, whose loops are twice the code, loses 2 to 17 %.)
+            start_tile();
+            if (!scores(0, s_addr, std::false_type())) break;
+            uint32_t w[BN / 2];
+#pragma unroll
+            for (int g = 0; g < BN / 32; g++) exponentials(g, w + 16 * g, std::false_type());
+            if (!epilogue(head, q0, l, m, stage_pv, phase_pv)) break;
+#pragma unroll
+            for (int g = 0; g < BN / 32; g++) tmem_st_32x32b_x16(s_addr + g * 16, w + 16 * g);
+            publish(p_bar);
+            s_addr ^= BN;
+            p_bar ^= 8;
+            j = 1;
         }
     }
 
+    else {
+        give_registers();
+    }
     // ----------------------------------------------------------------- teardown
     __syncwarp();
     tc_fence_before();
@@ -831,6 +1039,15 @@ bool one_to_an_sm(const LaunchArgs& a, long long tiles, int num_sms) {
     return a.causal && (a.window <= 0 || a.window >= a.sl) && a.bh <= HEAD_GROUP && 2 * tiles <= 3ll * num_sms;
 }
 
+// Whether a CTA goes on to further tiles.  That saves a tile its CTA's start (barriers, tensor memory, the first loads' latency: 3000 clk)
+// and part of its end, which the other CTA of the SM hides in part.  Start of a CTA per tile / a walk, us, both in a loop: D = 128, causal,
+// 1024 heads of 512 136 / 119, 256 of 2048 298 / 284; not causal 256 of 1000 140 / 132, 128 of 1024 70 / 64; D = 64, 512 of 512 61.6 / 51.8, 64 of
+// 3000, window 512, 61.4 / 55.9; 64 of 8192 of 128, window 1024, 305 / 304.  Long causal tiles gain nothing: 64 of 8192 930 / 939.
+bool walks(const LaunchArgs& a, long long tiles, int num_sms) {
+    const bool window = a.window > 0 && a.window < a.sl;
+    return tiles > 2ll * num_sms && !(a.causal && !window && a.sl > 6144);
+}
+
 template <int HD, bool VRAW>
 cudaError_t launch_hd(const LaunchArgs& a, int num_sms) {
     using C = Cfg<HD, VRAW>;
@@ -865,11 +1082,11 @@ cudaError_t launch_hd(const LaunchArgs& a, int num_sms) {
     }
     const bool masked = a.causal || a.window > 0 || (a.sl % BN) != 0 || !(a.scale > 0.f);
     const size_t smem = one_to_an_sm(a, grid, num_sms) ? SMEM_ONE : C::SMEM_BYTES;
-    auto start = [&](auto kernel) { return launch_pdl(kernel, (unsigned)grid, NUM_THREADS, smem, a.stream, tq, tk, tv, p); };
-    if (a.o_amax) return start(fa_fwd_kernel<HD, true, VRAW, true>);   // the masked kernel serves every call
-    if constexpr (HD == 128)
-        if (grid > 4ll * num_sms) return masked ? start(fa_fwd_kernel<HD, true, VRAW, false, true>) : start(fa_fwd_kernel<HD, false, VRAW, false, true>);
-    return masked ? start(fa_fwd_kernel<HD, true, VRAW, false>) : start(fa_fwd_kernel<HD, false, VRAW, false>);
+    auto start = [&](auto kernel) { return launch_pdl(kernel, (unsigned)grid, C::NUM_THREADS, smem, a.stream, tq, tk, tv, p); };
+    const bool walk = walks(a, grid, num_sms);
+    if (a.o_amax) return walk ? start(fa_fwd_kernel<HD, true, VRAW, true, true>) : start(fa_fwd_kernel<HD, true, VRAW, true, false>);   // the masked kernel serves every call
+    if (walk) return masked ? start(fa_fwd_kernel<HD, true, VRAW, false, true>) : start(fa_fwd_kernel<HD, false, VRAW, false, true>);
+    return masked ? start(fa_fwd_kernel<HD, true, VRAW, false, false>) : start(fa_fwd_kernel<HD, false, VRAW, false, false>);
 }
 
 }  // namespace
@@ -880,22 +1097,33 @@ void init_device(DeviceState* st, int dev) {
     auto set = [&](auto kernel, int bytes) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes > SMEM_ONE ? bytes : SMEM_ONE);
     };
-    set(fa_fwd_kernel<128, true, false, false>, Cfg<128, false>::SMEM_BYTES);
-    set(fa_fwd_kernel<128, false, false, false>, Cfg<128, false>::SMEM_BYTES);
-    set(fa_fwd_kernel<128, true, false, true>, Cfg<128, false>::SMEM_BYTES);
-    set(fa_fwd_kernel<128, true, true, false>, Cfg<128, true>::SMEM_BYTES);
-    set(fa_fwd_kernel<128, false, true, false>, Cfg<128, true>::SMEM_BYTES);
-    set(fa_fwd_kernel<128, true, true, true>, Cfg<128, true>::SMEM_BYTES);
-    set(fa_fwd_kernel<64, true, false, false>, Cfg<64, false>::SMEM_BYTES);
-    set(fa_fwd_kernel<64, false, false, false>, Cfg<64, false>::SMEM_BYTES);
-    set(fa_fwd_kernel<64, true, false, true>, Cfg<64, false>::SMEM_BYTES);
-    set(fa_fwd_kernel<64, true, true, false>, Cfg<64, true>::SMEM_BYTES);
-    set(fa_fwd_kernel<64, false, true, false>, Cfg<64, true>::SMEM_BYTES);
-    set(fa_fwd_kernel<64, true, true, true>, Cfg<64, true>::SMEM_BYTES);
-    set(fa_fwd_kernel<128, true, false, false, true>, Cfg<128, false>::SMEM_BYTES);
-    set(fa_fwd_kernel<128, false, false, false, true>, Cfg<128, false>::SMEM_BYTES);
-    set(fa_fwd_kernel<128, true, true, false, true>, Cfg<128, true>::SMEM_BYTES);
-    set(fa_fwd_kernel<128, false, true, false, true>, Cfg<128, true>::SMEM_BYTES);
+    auto set_hd = [&](auto hd, auto vraw, auto walk) {
+        constexpr int HD = decltype(hd)::value;
+        constexpr bool VRAW = decltype(vraw)::value, WALK = decltype(walk)::value;
+        set(fa_fwd_kernel<HD, true, VRAW, false, WALK>, Cfg<HD, VRAW>::SMEM_BYTES);
+        set(fa_fwd_kernel<HD, false, VRAW, false, WALK>, Cfg<HD, VRAW>::SMEM_BYTES);
+        set(fa_fwd_kernel<HD, true, VRAW, true, WALK>, Cfg<HD, VRAW>::SMEM_BYTES);
+    };
+    auto set_all = [&](auto vraw, auto walk) {
+        set_hd(std::integral_constant<int, 128>(), vraw, walk);
+        set_hd(std::integral_constant<int, 64>(), vraw, walk);
+    };
+    set_all(std::false_type(), std::false_type());
+    set_all(std::false_type(), std::true_type());
+    set_all(std::true_type(), std::false_type());
+    set_all(std::true_type(), std::true_type());
+    // the registers that the softmax warps of these take are those that the others were launched with and give up
+    auto check = [&](auto kernel) {
+        cudaFuncAttributes f;
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&f, kernel);
+        if (e == cudaSuccess && f.numRegs != LAUNCH_REGS) e = cudaErrorInvalidKernelImage;
+    };
+    check(fa_fwd_kernel<128, true, true, false, false>);
+    check(fa_fwd_kernel<128, true, true, false, true>);
+    check(fa_fwd_kernel<128, false, true, false, false>);
+    check(fa_fwd_kernel<128, false, true, false, true>);
+    check(fa_fwd_kernel<128, true, true, true, false>);
+    check(fa_fwd_kernel<128, true, true, true, true>);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&st->num_sms, cudaDevAttrMultiProcessorCount, dev);
     st->init_error = e;
 }

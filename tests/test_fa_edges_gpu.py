@@ -165,3 +165,35 @@ def test_tiles_of_heads_in_one_group_or_several(cuda, built_libs, fa_ctx, heads,
     torch.cuda.synchronize()
     fa_ctx.DeviceStatus()
     assert torch.equal(o, few)
+
+
+@pytest.mark.parametrize("s,hd,causal,window", [(64, 64, 0, 0), (64, 128, 0, 0), (192, 128, 0, 0), (256, 64, 0, 0), (320, 64, 0, 0), (1600, 128, 0, 0), (2752, 64, 0, 0),
+                                                (1, 64, 1, 0), (130, 128, 1, 0), (1000, 128, 1, 200), (2700, 128, 1, 0), (4300, 64, 1, 0)])
+def test_a_walk_over_tiles_gives_what_single_tiles_give(cuda, built_libs, fa_ctx, s, hd, causal, window):
+    # more tiles than CTAs fit: tiles of one block, of an odd number and of many, behind one another in a CTA; both signs of the scale.  A few
+    # heads at a time have a CTA per tile: the same bits, LSE and largest output
+    import ctypes as C
+    import torch
+    from goml_b200 import fa_forward as F
+    tiles = (s + 127) // 128
+    heads = 900 // tiles + 1
+    g = torch.Generator(device="cuda").manual_seed(s + hd)
+    q, k, v = (torch.randint(0, 0x70, (heads, s, hd), generator=g, dtype=torch.uint8, device="cuda") for _ in range(3))
+    q ^= torch.randint(0, 2, q.shape, generator=g, dtype=torch.uint8, device="cuda") << 7
+    o, few, raised = (torch.full((heads, s, hd), 7.0, dtype=torch.float16, device="cuda") for _ in range(3))
+    lse, few_lse = (torch.full((heads, s), 7.0, device="cuda") for _ in range(2))
+    run = lambda i, n, out, l, scale: fa_ctx.ForwardEx(q[i:].data_ptr(), k[i:].data_ptr(), v[i:].data_ptr(), out[i:].data_ptr(), l[i:].data_ptr(), n, s, hd, causal,
+                                                       window, scale, 1.0, 0, 0, 0, torch.cuda.current_stream().cuda_stream)
+    walking = lambda n: any(re.search(r"fa_fwd_kernelILi\d+ELb[01]ELb[01]ELb0ELb1E", name) for name in kernels(lambda: run(0, n, o, lse, 1.0)))   # <.., false, WALK>
+    step = max(1, 200 // tiles)
+    assert walking(heads) and not walking(step)
+    for scale in (1e-4, -1e-4):
+        run(0, heads, o, lse, scale)
+        for i in range(0, heads, step):
+            run(i, min(step, heads - i), few, few_lse, scale)
+        args = F.ForwardArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), raised.data_ptr(), None, heads, s, hd, causal, window, scale, 1.0, None, None, None, None)
+        word = torch.zeros(1, device="cuda")
+        assert F.FALoad().fa_forward_raise(fa_ctx.ptr, C.byref(args), word.data_ptr()) == 0
+        torch.cuda.synchronize()
+        fa_ctx.DeviceStatus()
+        assert torch.equal(o, few) and torch.equal(lse, few_lse) and torch.equal(o, raised) and word.item() == o.float().abs().max().item()
