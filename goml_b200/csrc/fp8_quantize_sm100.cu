@@ -132,8 +132,10 @@ struct QuantOp {
     float* scale_out;
     float* amax_out;
     float divisor;
-    __device__ void pass1(float (&m)[1]) const { m[0] = amax_items<WIDE, BATCH>(x, n, oc_tid(), OC_STEP); }
-    __device__ void pass2(const float (&m)[1]) const {
+    using State = NoState;
+    __device__ void ahead() const {}
+    __device__ void pass1(float (&m)[1], State&) const { m[0] = amax_items<WIDE, BATCH>(x, n, oc_tid(), OC_STEP); }
+    __device__ void pass2(const float (&m)[1], State&) const {
         if (oc_tid() == 0) *amax_out = m[0];
         quant_items<WIDE, BATCH>(x, q, n, oc_tid(), OC_STEP, m[0], scale_out, divisor);
     }

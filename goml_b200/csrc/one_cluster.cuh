@@ -66,18 +66,22 @@ __device__ __forceinline__ void oc_max(float (&m)[N]) {
     }
 }
 
-// Op: N maxima; pass1(m) leaves this thread's maxima of non-negative values, pass2(m) is called with the tensor's
+// Op: N maxima; ahead() runs ahead of the wait and may only ask for lines of operands; pass1(m, state) leaves this thread's maxima of
+// non-negative values, pass2(m, state) is called with the tensor's; State is what a thread keeps from the one to the other
+struct NoState {};
 template <class Op>
 __global__ void __launch_bounds__(OC_THREADS) one_cluster_kernel(const Op op) {
     oc_arrive();
+    op.ahead();
     pdl_wait();
     pdl_trigger();
+    typename Op::State state;
     float m[Op::N];
 #pragma unroll
     for (int n = 0; n < Op::N; n++) m[n] = 0.f;
-    op.pass1(m);
+    op.pass1(m, state);
     oc_max(m);
-    op.pass2(m);
+    op.pass2(m, state);
 }
 __device__ __forceinline__ uint32_t oc_tid() { return (uint32_t)oc_rank() * OC_THREADS + threadIdx.x; }
 constexpr uint32_t OC_STEP = OC_CTAS * OC_THREADS;
