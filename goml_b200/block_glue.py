@@ -17,7 +17,7 @@ from . import loader
 
 _lock = threading.Lock()
 _lib = None
-_run = None   # fp8_block_run taking the packed block
+_run = None   # fp8_block_run_rows taking the packed block
 
 
 class BlockGlueError(RuntimeError):
@@ -53,21 +53,21 @@ _PACK_RUN = struct.Struct("@30PNP8i2f").pack
 assert struct.calcsize("@30PNP8i2f") == C.sizeof(BlockRunArgs)
 
 
-def BlockRun(*args) -> int:
-    """fp8_block_run with the fields of BlockRunArgs in order; its return code."""
+def BlockRun(*args, gemm_rows: int = 0) -> int:
+    """fp8_block_run with the fields of BlockRunArgs in order, or fp8_block_run_rows with the address of its gemm_rows; the return code."""
     run = _run or _load_run()
     try:
         block = _PACK_RUN(*args)
     except (struct.error, OverflowError):   # values that only ctypes takes
         block = bytes(BlockRunArgs(*args))
-    return run(block)
+    return run(block, gemm_rows)
 
 
 def _load_run():
     global _run
     lib = _init()
-    fn = lib["fp8_block_run"]
-    fn.restype, fn.argtypes = C.c_int, [C.c_char_p]
+    fn = lib["fp8_block_run_rows"]
+    fn.restype, fn.argtypes = C.c_int, [C.c_char_p, C.c_void_p]
     _run = fn
     return fn
 

@@ -31,12 +31,33 @@ constexpr int SMEM_ONE = 227 * 1024;        // of one CTA when it has the SM to 
 // shared memory of one of up to three CTAs on an SM (228 KB, 1 KB of it the system's for each CTA)
 constexpr int smem_of(int per_sm) { return per_sm == 1 ? SMEM_ONE : per_sm == 2 ? 112 * 1024 : 74 * 1024; }
 
+// Where the codes of the tokens come from: a matrix of them, or (a step of a few sequences) the values that they are made of, which
+// every CTA quantises for itself.  Values of at most MAX_ROWS tokens, of all of K, have one scale, max|value| / 448.  A row costs the
+// four products of a block 4 to 5 us, the quantisers ahead of them 15 to 18 however few rows there are: a step of one sequence 81.2 ->
+// 73.0 us, two 81.7 / 78.5, three 81.9 / 82.8, four 86 / 92.
+constexpr int MAX_ROWS = 2;
+enum Source : int { CODES = 0, RMS_F32 = 1, F16 = 2, BF16_KNOWN = 3 };   // RMSNorm of fp32 rows; fp16 values; bf16 values whose maximum is known
+struct Rows {
+    int source;
+    const void* x;         // [M, K]
+    const float* gamma;    // RMS_F32
+    float eps;
+    const float* amax;     // BF16_KNOWN
+    const float* x_in;     // accumulate mode: X = x_in + alpha A B^T
+    float* zero;           // words set to 0 for later kernels
+    int zeros;
+    int early;             // the weight is complete when this kernel starts: its first tiles are loaded ahead of the wait
+};
+constexpr int TOKEN_BYTES = 8 * BK;   // a k-block of such codes: one swizzle atom of eight rows
+
 struct Params {
     GemmParams g;
+    Rows r;
     int tn;            // tokens rounded up to 16: MMA N
     int tmem_cols;
     uint32_t idesc;
     int stages;
+    int slice;         // most k-blocks of a CTA
     int prefetch;      // k-blocks per CTA asked for ahead of the wait
     int vec;           // four neighbouring outputs of a token may be stored at once
 };
@@ -73,18 +94,162 @@ __device__ __forceinline__ void add_up(const float4* v, float* r) {
     for (int s = 1; s < SPLIT; s++) { r[0] += v[s].x; r[1] += v[s].y; r[2] += v[s].z; r[3] += v[s].w; }
 }
 
-template <int SPLIT>
+__device__ __forceinline__ uint32_t rows_quant4(float a, float b, float c, float d, float inv) {   // the quantiser's formula
+    const float x[4] = {a, b, c, d};
+    float y[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) y[i] = fminf(fmaxf(__fmul_rn(x[i], inv), -448.f), 448.f);
+    return pack_e4m3x4(y[0], y[1], y[2], y[3]);
+}
+// The codes of k-blocks [kb0, kb1) of all tokens, as a TMA load with 128-byte swizzle would leave them, and their scale.  By the four
+// warps that wait for the accumulators otherwise (tid 0 .. 127); every CTA goes over all of K for the maximum, which for a few tokens is
+// less than a second meeting of CTAs costs.  red: 4 * 2 * MAX_ROWS floats of shared memory.
+__device__ __forceinline__ void quantise_rows(const Params& p, uint32_t tok, float* red, float* scale_out, int kb0, int kb1, int tid) {
+    const Rows& r = p.r;
+    const int M = p.g.M, K = p.g.K, warp = tid >> 5, lane = tid & 31;
+    const float* xf = static_cast<const float*>(r.x);
+    const uint8_t* xh = static_cast<const uint8_t*>(r.x);
+    float amax = 0.f;
+    if (r.source == BF16_KNOWN) {
+        amax = ld_f32(r.amax);
+    } else {
+#pragma unroll 1
+        for (int j = 0; j < M; j++) {
+            float ss = 0.f, top = 0.f;
+            if (r.source == RMS_F32) {
+                const float* row = xf + (size_t)j * K;
+                constexpr int U = 8;   // loads in flight: one latency for 4096 values
+#pragma unroll 1
+                for (int c0 = tid * 4; c0 < K; c0 += 512 * U) {
+                    float4 h[U], g[U];
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const int c = c0 + u * 512;
+                        h[u] = g[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (c < K) { h[u] = ld128f(row + c); g[u] = ld128f(r.gamma + c); }
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        ss = fmaf(h[u].x, h[u].x, ss); ss = fmaf(h[u].y, h[u].y, ss);
+                        ss = fmaf(h[u].z, h[u].z, ss); ss = fmaf(h[u].w, h[u].w, ss);
+                        top = fmaxf(fmaxf(top, fmaxf(fabsf(__fmul_rn(h[u].x, g[u].x)), fabsf(__fmul_rn(h[u].y, g[u].y)))),
+                                    fmaxf(fabsf(__fmul_rn(h[u].z, g[u].z)), fabsf(__fmul_rn(h[u].w, g[u].w))));
+                    }
+                }
+            } else {
+                constexpr int U = 4;
+#pragma unroll 1
+                for (int c0 = tid * 8; c0 < K; c0 += 1024 * U) {
+                    uint4 v[U];
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const int c = c0 + u * 1024;
+                        v[u] = make_uint4(0u, 0u, 0u, 0u);
+                        if (c < K) v[u] = ld128(xh + ((size_t)j * K + c) * 2);
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+                            top = fmaxf(top, fmaxf(fabsf(f.x), fabsf(f.y)));   // NaN never wins
+                        }
+                    }
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+            }
+            if (lane == 0) {
+                red[(j * 4 + warp) * 2] = ss;
+                red[(j * 4 + warp) * 2 + 1] = top;
+            }
+        }
+        named_bar_sync(1, 128);
+    }
+    // of row j, from the four warps' parts in a fixed order: the same in every CTA
+    auto rstd_of = [&](int j) {
+        return __frsqrt_rn(__fadd_rn(__fdiv_rn(((red[j * 8] + red[j * 8 + 2]) + red[j * 8 + 4]) + red[j * 8 + 6], (float)K), r.eps));
+    };
+    float rstd0 = 1.f;
+    if (r.source != BF16_KNOWN)
+        for (int j = 0; j < M; j++) {
+            const float top = fmaxf(fmaxf(red[j * 8 + 1], red[j * 8 + 3]), fmaxf(red[j * 8 + 5], red[j * 8 + 7]));
+            const float rstd = r.source == RMS_F32 ? rstd_of(j) : 1.f;
+            if (j == 0) rstd0 = rstd;
+            amax = fmaxf(amax, r.source == RMS_F32 ? __fmul_rn(top, rstd) : top);
+        }
+    const float scale = amax > 1e-12f ? __fdiv_rn(amax, 448.0f) : 1.0f;
+    const float inv = __fdiv_rn(1.0f, scale);
+    if (tid == 0) *scale_out = scale;
+    const int chunks = (kb1 - kb0) * (BK / 16);   // of 16 codes; those past K are zeros
+#pragma unroll 1
+    for (int j = 0; j < M; j++) {
+        const float rstd = r.source != RMS_F32 ? 1.f : j == 0 ? rstd0 : rstd_of(j);
+        for (int it = tid; it < chunks; it += 128) {
+            const int col = kb0 * BK + it * 16;
+            uint4 q = make_uint4(0u, 0u, 0u, 0u);
+            if (col < K) {
+                float y[16];
+                if (r.source == RMS_F32) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const float4 h = ld128f(xf + (size_t)j * K + col + 4 * i), g = ld128f(r.gamma + col + 4 * i);
+                        y[4 * i] = __fmul_rn(__fmul_rn(h.x, g.x), rstd);
+                        y[4 * i + 1] = __fmul_rn(__fmul_rn(h.y, g.y), rstd);
+                        y[4 * i + 2] = __fmul_rn(__fmul_rn(h.z, g.z), rstd);
+                        y[4 * i + 3] = __fmul_rn(__fmul_rn(h.w, g.w), rstd);
+                    }
+                } else {
+                    const uint8_t* src = xh + ((size_t)j * K + col) * 2;
+                    const uint4 v0 = ld128(src), v1 = ld128(src + 16);
+                    const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        if (r.source == F16) {
+                            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+                            y[2 * i] = f.x;
+                            y[2 * i + 1] = f.y;
+                        } else {
+                            y[2 * i] = __uint_as_float(w[i] << 16);
+                            y[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+                        }
+                    }
+                }
+                q = make_uint4(rows_quant4(y[0], y[1], y[2], y[3], inv), rows_quant4(y[4], y[5], y[6], y[7], inv),
+                               rows_quant4(y[8], y[9], y[10], y[11], inv), rows_quant4(y[12], y[13], y[14], y[15], inv));
+            }
+            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(tok + (it >> 3) * TOKEN_BYTES + j * BK + (((it & 7) ^ j) << 4)),
+                         "r"(q.x), "r"(q.y), "r"(q.z), "r"(q.w) : "memory");
+        }
+    }
+}
+
+// VALUES: the tokens come as values (Rows), else as codes
+template <int SPLIT, bool VALUES>
 __global__ void __launch_bounds__(THREADS, 2)
 fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_t, const Params p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;   // swizzle atoms are 1024 bytes
     uint8_t* ring_gen = smem_raw + (ring - smem_u32(smem_raw));
-    const int stage_bytes = W_BYTES + p.tn * BK;                   // a multiple of 2048
-    const uint32_t bar_full = ring + p.stages * stage_bytes;
+    const int stage_bytes = VALUES ? W_BYTES : W_BYTES + p.tn * BK;   // a multiple of 2048
+    // VALUES: the codes of this CTA's k-blocks, eight rows each.  The MMA takes sixteen tokens; the other eight, which nobody looks at, it
+    // finds in the block behind, so that there is one block more
+    const uint32_t tok = ring + p.stages * stage_bytes;
+    const uint32_t tok_bytes = VALUES ? (p.slice + 1) * TOKEN_BYTES : 0;
+    const uint32_t bar_full = tok + tok_bytes;
     const uint32_t bar_empty = bar_full + 8 * MAX_STAGES;
     const uint32_t bar_done = bar_empty + 8 * MAX_STAGES;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ring_gen + p.stages * stage_bytes + 16 * MAX_STAGES + 8);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ring_gen + p.stages * stage_bytes + tok_bytes + 16 * MAX_STAGES + 8);
     volatile uint32_t* abort_flag = tmem_slot + 1;
+    const uint32_t bar_tok = bar_done + 16;
+    float* scale_slot = reinterpret_cast<float*>(tmem_slot + 4);
+    float* red = scale_slot + 2;                                      // 8 * MAX_ROWS floats
+    static_assert(16 * MAX_STAGES + 8 + 24 + 32 * MAX_ROWS <= 512, "barriers and words fit the tail");
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = (int)blockIdx.x % SPLIT;
@@ -97,6 +262,7 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
             mbar_init(bar_empty + 8 * s, 1);
         }
         mbar_init(bar_done, 1);
+        if (VALUES) mbar_init(bar_tok, 128);
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -113,20 +279,32 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    int kb_next = kb0;   // first k-block of the weight that is not on its way yet
+    if (VALUES && p.r.early && warp == 0) {
+        const bool leader = elect_one();
+        for (int i = 0; i < p.stages && kb_next < kb1; i++, kb_next++) {
+            if (leader) {
+                mbar_arrive_expect_tx(bar_full + 8 * i, W_BYTES);
+                tma_load_2d(ring + i * W_BYTES, &tmap_w, bar_full + 8 * i, kb_next * BK, n0);
+            }
+        }
+        __syncwarp();
+    }
     pdl_wait();
     pdl_trigger();
+    if (VALUES && blockIdx.x == 0 && (int)threadIdx.x < p.r.zeros) p.r.zero[threadIdx.x] = 0.f;
 
     if (warp == 0) {
         const bool leader = elect_one();
-        int stage = 0;
-        uint32_t phase = 1;
-        for (int kb = kb0; kb < kb1; kb++) {
+        int stage = (kb_next - kb0) % p.stages;
+        uint32_t phase = kb_next - kb0 == p.stages ? 0 : 1;
+        for (int kb = kb_next; kb < kb1; kb++) {
             if (!mbar_wait_warp(bar_empty + 8 * stage, phase, abort_flag, ST_TIMEOUT_PRODUCER)) break;
             if (leader) {
                 const uint32_t fb = bar_full + 8 * stage, sw = ring + stage * stage_bytes;
                 mbar_arrive_expect_tx(fb, stage_bytes);   // parts of a box outside the matrix are zero-filled and counted
                 tma_load_2d(sw, &tmap_w, fb, kb * BK, n0);
-                tma_load_2d(sw + W_BYTES, &tmap_t, fb, kb * BK, 0);
+                if (!VALUES) tma_load_2d(sw + W_BYTES, &tmap_t, fb, kb * BK, 0);
             }
             __syncwarp();
             if (++stage == p.stages) { stage = 0; phase ^= 1; }
@@ -135,12 +313,12 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         const bool leader = elect_one();
         int stage = 0;
         uint32_t phase = 0;
-        bool ok = true;
-        for (int kb = kb0; kb < kb1; kb++) {
+        bool ok = !VALUES || mbar_wait_warp(bar_tok, 0, abort_flag, ST_TIMEOUT_MMA);
+        for (int kb = kb0; kb < kb1 && ok; kb++) {
             if (!mbar_wait_warp(bar_full + 8 * stage, phase, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
             tc_fence_after();
             const uint32_t sw = ring + stage * stage_bytes;
-            const uint64_t wdesc = kmajor_desc_sw128(sw), tdesc = kmajor_desc_sw128(sw + W_BYTES);
+            const uint64_t wdesc = kmajor_desc_sw128(sw), tdesc = kmajor_desc_sw128(VALUES ? tok + (kb - kb0) * TOKEN_BYTES : sw + W_BYTES);
 #pragma unroll
             for (int k = 0; k < BK / 32; k++)
                 if (leader) mma_f8f6f4_ss(tmem, wdesc + 2 * k, tdesc + 2 * k, p.idesc, ((kb - kb0) | k) != 0);
@@ -154,6 +332,12 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         // accumulators -> shared memory, token-major ([token][128 weight rows] fp32): lanes write neighbouring words.  The
         // ring is free by then: every load that was issued has been consumed by an MMA that has retired.
         const int quad = warp & 3;
+        if (VALUES) {
+            quantise_rows(p, tok, red, scale_slot, kb0, kb1, (int)threadIdx.x - 64);
+            fence_proxy_async_smem();
+            mbar_arrive(bar_tok);
+            __syncwarp();
+        }
         if (mbar_wait_warp(bar_done, 0, abort_flag, ST_TIMEOUT_EPILOGUE)) {
             tc_fence_after();
             for (int j0 = 0; j0 < p.tn; j0 += 16) {
@@ -179,7 +363,8 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         const GemmParams& g = p.g;
         constexpr int STEP = SPLIT * THREADS;
         float alpha = g.alpha;
-        if (g.scale_a) alpha *= ld_f32(g.scale_a);
+        if (VALUES) alpha *= *scale_slot;
+        else if (g.scale_a) alpha *= ld_f32(g.scale_a);
         if (g.scale_b) alpha *= ld_f32(g.scale_b);
         const float scale_d = (g.D8 && g.scale_d) ? ld_f32(g.scale_d) : 1.0f;
         float tmax = 0.f;
@@ -238,7 +423,7 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
                 for (int u = 0; u < U; u++) {
                     const int it = min(it0 + u * STEP, items - 1), j = it / QUADS, row = (it % QUADS) * 4, col = n0 + row;
                     if (g.X) {
-                        const float* src = g.X + (size_t)j * g.N + col;
+                        const float* src = (VALUES ? p.r.x_in : g.X) + (size_t)j * g.N + col;
                         if (p.vec && col + 4 <= g.N) {
                             const float4 t = *reinterpret_cast<const float4*>(src);
                             x[u][0] = t.x; x[u][1] = t.y; x[u][2] = t.z; x[u][3] = t.w;
@@ -323,10 +508,13 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
 }
 
 using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const Params);
-inline Kernel kernel_for(int split) {
-    static const Kernel table[MAX_SPLIT] = {fp8_gemm_skinny_kernel<1>, fp8_gemm_skinny_kernel<2>, fp8_gemm_skinny_kernel<3>, fp8_gemm_skinny_kernel<4>,
-                                            fp8_gemm_skinny_kernel<5>, fp8_gemm_skinny_kernel<6>, fp8_gemm_skinny_kernel<7>, fp8_gemm_skinny_kernel<8>};
-    return table[split - 1];
+inline Kernel kernel_for(int split, bool values) {
+    static const Kernel table[2][MAX_SPLIT] = {
+        {fp8_gemm_skinny_kernel<1, false>, fp8_gemm_skinny_kernel<2, false>, fp8_gemm_skinny_kernel<3, false>, fp8_gemm_skinny_kernel<4, false>,
+         fp8_gemm_skinny_kernel<5, false>, fp8_gemm_skinny_kernel<6, false>, fp8_gemm_skinny_kernel<7, false>, fp8_gemm_skinny_kernel<8, false>},
+        {fp8_gemm_skinny_kernel<1, true>, fp8_gemm_skinny_kernel<2, true>, fp8_gemm_skinny_kernel<3, true>, fp8_gemm_skinny_kernel<4, true>,
+         fp8_gemm_skinny_kernel<5, true>, fp8_gemm_skinny_kernel<6, true>, fp8_gemm_skinny_kernel<7, true>, fp8_gemm_skinny_kernel<8, true>}};
+    return table[values][split - 1];
 }
 
 // clusters of each size that are resident at once with one CTA to an SM (a cluster stays inside one group of SMs, so this
@@ -352,13 +540,16 @@ inline void configure(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int ti
 
 inline cudaError_t init(Fit* fit) {
     for (int split = 1; split <= MAX_SPLIT; split++) {
-        cudaError_t e = cudaFuncSetAttribute(kernel_for(split), cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_ONE);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel_for(split), cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        cudaError_t e = cudaSuccess;
+        for (bool values : {false, true}) {
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel_for(split, values), cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_ONE);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel_for(split, values), cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        }
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[2];
         configure(cfg, attr, 1, split, SMEM_ONE, nullptr);
         cfg.numAttrs = 1;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fit->one[split], kernel_for(split), &cfg);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fit->one[split], kernel_for(split, false), &cfg);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -425,18 +616,22 @@ inline Plan plan(int M, int N, int K, bool added, bool codes, int num_sms, const
     return r;
 }
 
-// A: tokens [M, K], B: weights [N, K]; g is complete but for k_blocks
-inline int launch(GemmParams g, const Plan& plan, const void* A, const void* B, cudaStream_t stream) {
+// A: tokens [M, K] (their codes; rows = nullptr) or nothing, B: weights [N, K]; g is complete but for k_blocks
+inline int launch(GemmParams g, const Plan& plan, const void* A, const void* B, cudaStream_t stream, const Rows* rows = nullptr) {
     Params p;
+    p.r = rows ? *rows : Rows{};
     g.k_blocks = (g.K + BK - 1) / BK;
     p.tn = (g.M + 15) / 16 * 16;
     p.tmem_cols = 32;
     while (p.tmem_cols < p.tn) p.tmem_cols *= 2;
     p.idesc = make_idesc_e4m3_f32(W_ROWS, p.tn, 0, 0);
     const int tiles = (g.N + W_ROWS - 1) / W_ROWS;
-    const int stage_bytes = W_BYTES + p.tn * BK, part_bytes = p.tn * W_ROWS * 4;
     const int slice = (g.k_blocks + plan.split - 1) / plan.split;
-    p.stages = (smem_of(plan.per_sm) - TAIL_BYTES) / stage_bytes;
+    const int stage_bytes = rows ? W_BYTES : W_BYTES + p.tn * BK, part_bytes = p.tn * W_ROWS * 4;
+    const int tok_bytes = rows ? (slice + 1) * TOKEN_BYTES : 0;
+    p.slice = slice;
+    p.stages = (smem_of(plan.per_sm) - TAIL_BYTES - tok_bytes) / stage_bytes;
+    if (rows && p.stages < 2) return (int)cudaErrorNotSupported;
     if (p.stages > slice) p.stages = slice;
     if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
     int ring_bytes = p.stages * stage_bytes;
@@ -450,6 +645,7 @@ inline int launch(GemmParams g, const Plan& plan, const void* A, const void* B, 
     if (plan.per_sm > 1 && p.prefetch > (20 << 20) / (W_BYTES * tiles * plan.split)) p.prefetch = (20 << 20) / (W_BYTES * tiles * plan.split);
     if (p.prefetch > 16) p.prefetch = 16;
     if (g.M > 80) p.prefetch = 4;
+    if (p.r.early) p.prefetch = 0;
     p.vec = g.H ? (g.F % 4 == 0 && (reinterpret_cast<uintptr_t>(g.H) & 7) == 0)
           : g.X ? (g.N % 4 == 0 && (reinterpret_cast<uintptr_t>(g.X) & 15) == 0)
           : g.D8 ? (g.N % 4 == 0 && (reinterpret_cast<uintptr_t>(g.D8) & 3) == 0)
@@ -457,12 +653,13 @@ inline int launch(GemmParams g, const Plan& plan, const void* A, const void* B, 
     p.g = g;
     CUtensorMap tw, tt;
     if (!make_tmap_u8_2d(&tw, B, (uint64_t)g.N, (uint64_t)g.K, W_ROWS, BK, CU_TENSOR_MAP_SWIZZLE_128B) ||
-        !make_tmap_u8_2d(&tt, A, (uint64_t)g.M, (uint64_t)g.K, (uint32_t)p.tn, BK, CU_TENSOR_MAP_SWIZZLE_128B))
+        (!rows && !make_tmap_u8_2d(&tt, A, (uint64_t)g.M, (uint64_t)g.K, (uint32_t)p.tn, BK, CU_TENSOR_MAP_SWIZZLE_128B)))
         return (int)cudaErrorInvalidValue;
+    if (rows) tt = tw;   // not looked at
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
-    configure(cfg, attr, tiles, plan.split, (size_t)ring_bytes + TAIL_BYTES, stream);
-    return (int)cudaLaunchKernelEx(&cfg, kernel_for(plan.split), tw, tt, p);
+    configure(cfg, attr, tiles, plan.split, (size_t)ring_bytes + tok_bytes + TAIL_BYTES, stream);
+    return (int)cudaLaunchKernelEx(&cfg, kernel_for(plan.split, rows != nullptr), tw, tt, p);
 }
 
 }  // namespace skinny

@@ -699,6 +699,17 @@ void init_device(DeviceState* st, int dev) {
     st->num_sms = sms;
 }
 
+// the device's state, made on its first call
+cudaError_t device_state(DeviceState** out) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= MAX_DEVICES) return cudaErrorInvalidDevice;
+    *out = &g_dev[dev];
+    std::call_once(g_dev[dev].once, init_device, &g_dev[dev], dev);
+    return g_dev[dev].init_error;
+}
+
 int launch(int M, int N, int K, const void* A, const void* B, void* C, float alpha, const float* sa, const float* sb,
            int out_bf16, cudaStream_t stream, float* X = nullptr, void* H = nullptr, int F = 0, float* amax = nullptr,
            uint8_t* D8 = nullptr, const float* scale_d = nullptr) {
@@ -711,13 +722,9 @@ int launch(int M, int N, int K, const void* A, const void* B, void* C, float alp
         (reinterpret_cast<uintptr_t>(C) & 1) || (reinterpret_cast<uintptr_t>(X) & 3))
         return (int)cudaErrorInvalidValue;
 
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return (int)e;
-    if (dev < 0 || dev >= MAX_DEVICES) return (int)cudaErrorInvalidDevice;
-    DeviceState& st = g_dev[dev];
-    std::call_once(st.once, init_device, &st, dev);
-    if (st.init_error != cudaSuccess) return (int)st.init_error;
+    DeviceState* state = nullptr;
+    if (const cudaError_t e = device_state(&state)) return (int)e;
+    const DeviceState& st = *state;
 
     GemmParams p{};
     p.M = M; p.N = N; p.K = K; p.C = C;
@@ -871,6 +878,33 @@ int fp8_gemm_fp8out(int M, int N, int K, const void* A, const void* B, void* D, 
     }
     return launch(M, N, K, A, B, nullptr, alpha, scale_a, scale_b, 0, (cudaStream_t)stream, nullptr, nullptr, 0, amax_d,
                   reinterpret_cast<uint8_t*>(D), scale_d);
+}
+
+int fp8_gemm_rows(const fp8_gemm_rows_args_t* a) {
+    if (!a || a->m < 0 || a->n < 0 || a->k <= 0 || a->k % 16 != 0 || a->zeros < 0 || a->zeros > 64) return (int)cudaErrorInvalidValue;
+    if (a->source < FP8_ROWS_RMSNORM_F32 || a->source > FP8_ROWS_BF16) return (int)cudaErrorInvalidValue;
+    if (a->m > skinny::MAX_ROWS) return (int)cudaErrorNotSupported;
+    if (a->m == 0 || a->n == 0) return a->zeros == 0 ? 0 : (int)cudaErrorNotSupported;
+    const uintptr_t sixteen = reinterpret_cast<uintptr_t>(a->rows) | reinterpret_cast<uintptr_t>(a->b) | reinterpret_cast<uintptr_t>(a->gamma);
+    const uintptr_t four = reinterpret_cast<uintptr_t>(a->x) | reinterpret_cast<uintptr_t>(a->x_in) | reinterpret_cast<uintptr_t>(a->amax) |
+                           reinterpret_cast<uintptr_t>(a->h_amax) | reinterpret_cast<uintptr_t>(a->zero) | reinterpret_cast<uintptr_t>(a->scale_b);
+    if (!a->rows || !a->b || (sixteen & 15) || (four & 3) || ((reinterpret_cast<uintptr_t>(a->c) | reinterpret_cast<uintptr_t>(a->h)) & 1))
+        return (int)cudaErrorInvalidValue;
+    if ((a->source == FP8_ROWS_RMSNORM_F32 && !a->gamma) || (a->source == FP8_ROWS_BF16 && !a->amax) || (a->zeros > 0 && !a->zero))
+        return (int)cudaErrorInvalidValue;
+    if (!!a->c + !!a->x + !!a->h != 1 || (a->x && !a->x_in) || (a->h && !a->h_amax)) return (int)cudaErrorInvalidValue;
+    DeviceState* st = nullptr;
+    if (const cudaError_t e = device_state(&st)) return (int)e;
+    GemmParams p{};
+    p.M = a->m; p.K = a->k;
+    p.N = a->h ? 2 * ((a->n + 31) / 32) * 32 : a->n;
+    p.alpha = 1.0f; p.scale_b = a->scale_b; p.out_bf16 = 1;
+    p.C = a->c; p.X = a->x;
+    p.H = a->h; p.F = a->h ? a->n : 0; p.amax = a->h_amax;
+    const skinny::Plan plan = skinny::plan(p.M, p.N, p.K, a->x != nullptr, false, st->num_sms, st->skinny_fit);
+    if (plan.split == 0) return (int)cudaErrorNotSupported;
+    const skinny::Rows rows{a->source, a->rows, a->gamma, a->eps, a->amax, a->x_in, a->zero, a->zeros, a->b_complete};
+    return skinny::launch(p, plan, nullptr, a->b, (cudaStream_t)a->stream, &rows);
 }
 
 int fp8_gemm_device_status(void) {

@@ -23,6 +23,15 @@ class FP8GEMMError(RuntimeError):
     pass
 
 
+RowsRMSNormF32, RowsF16, RowsBF16 = 1, 2, 3
+
+
+class RowsArgs(C.Structure):
+    """fp8_gemm_rows_args_t (include/fp8_gemm.h)."""
+    _fields_ = ([(name, C.c_void_p) for name in ("rows", "gamma", "amax", "b", "scale_b", "c", "x", "x_in", "h", "h_amax", "zero", "stream")]
+                + [(name, C.c_int32) for name in ("m", "n", "k", "source", "zeros", "b_complete")] + [("eps", C.c_float), ("reserved", C.c_int32)])
+
+
 _state = {"lib": None, "err": None}
 _once = threading.Lock()
 
@@ -48,6 +57,8 @@ def _init():
                 lib.fp8_gemm_swiglu.argtypes = [i, i, i, p, p, p, f, p, p, p, p]
                 lib.fp8_gemm_swiglu_raise.restype = i
                 lib.fp8_gemm_swiglu_raise.argtypes = [i, i, i, p, p, p, f, p, p, p, p]
+                lib.fp8_gemm_rows.restype = i
+                lib.fp8_gemm_rows.argtypes = [C.POINTER(RowsArgs)]
                 lib.fp8_gemm_fp8out.restype = i
                 lib.fp8_gemm_fp8out.argtypes = [i, i, i, p, p, p, f, p, p, p, p, p]
                 lib.fp8_gemm_device_status.restype = i

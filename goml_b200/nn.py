@@ -156,7 +156,7 @@ def _entry_points():
     if _entries is None:
         gemm, fa = G._init(), F.FALoad()
         _entries = tuple(ctypes.cast(fn, ctypes.c_void_p).value for fn in (gemm.fp8_gemm_scaled, gemm.fp8_gemm_accumulate_f32, gemm.fp8_gemm_swiglu_raise,
-                                                                           fa.fa_forward_raise, fa.fa_decode))
+                                                                           fa.fa_forward_raise, fa.fa_decode, gemm.fp8_gemm_rows))
     return _entries
 
 
@@ -228,11 +228,12 @@ class FP8DecoderBlock:
         if cache is not None:
             k, v, ks, lens, s_max = cache.k.data_ptr(), cache.v.data_ptr(), cache.scales.data_ptr(), cache.lens.data_ptr(), cache.s_max
         qkv, o, gate_up, down = self.qkv.w, self.o.w, self.gate_up.w, self.down.w
-        rc = BG.BlockRun(*_entry_points(), self.fa.ptr, src.data_ptr(), h.data_ptr(), self.norm1.data_ptr(),
+        *entries, gemm_rows = _entry_points()
+        rc = BG.BlockRun(*entries, self.fa.ptr, src.data_ptr(), h.data_ptr(), self.norm1.data_ptr(),
                          self.norm2.data_ptr(), qkv.codes.data_ptr(), o.codes.data_ptr(), self.gate_up_interleaved.data_ptr(), down.codes.data_ptr(),
                          qkv.scale_ptr, o.scale_ptr, gate_up.scale_ptr, down.scale_ptr, cos.data_ptr(), sin.data_ptr(), k, v, ks, lens,
                          words, rstd, codes, kc, vc, region, region_bytes, torch.cuda.current_stream().cuda_stream,
-                         B, S, d, H, Fh, s_max, tables, int(decode), self.eps, 1.0 / math.sqrt(self.hd))
+                         B, S, d, H, Fh, s_max, tables, int(decode), self.eps, 1.0 / math.sqrt(self.hd), gemm_rows=gemm_rows)
         if rc:
             self._raise(rc, decode, cache is not None)
         return h, buf, kc, vc, words + 72
@@ -242,6 +243,8 @@ class FP8DecoderBlock:
         place, code = rc >> 16, rc & 0xffff
         if place == 4:
             raise F.FAError("fa_decode" if decode else "fa_forward_raise", code, self.fa._msg())
+        if place > 10:
+            raise G.FP8GEMMError(f"fp8_gemm_rows: CUDA error {code}")
         rope = "fp8_decode_rope_append" if decode else "fp8_rope_quantize_qkv_cache" if cached else "fp8_rope_quantize_qkv"
         name = ("fp8_block_run", "fp8_rmsnorm_quantize_into", "fp8_gemm_scaled", rope, "", "fp8_permute_quantize_heads",
                 "fp8_gemm_accumulate_f32", "fp8_rmsnorm_quantize_into", "fp8_gemm_swiglu_raise", "fp8_quantize_bf16", "fp8_gemm_accumulate_f32")[place]
@@ -265,7 +268,7 @@ class FP8DecoderBlock:
         """One new token per sequence: x [batch, d] fp32 -> [batch, d] fp32, the token's K and V appended to `cache` at
         position cache.lens[b] (quantised with the cache's scales) and cache.lens advanced.  Ten library calls:
         RMSNorm+quantise -> QKV GEMM -> RoPE+quantise+append -> decode attention -> quantise -> O GEMM (residual in the
-        epilogue) -> the feed-forward half of forward_fused."""
+        epilogue) -> the feed-forward half of forward_fused; six for one or two sequences, whose GEMMs quantise their rows themselves."""
         B = x.shape[0]
         assert (B, self.H, self.hd) == (cache.B, cache.H, cache.hd)
         if not cache.dense_on(x.device):

@@ -187,6 +187,12 @@ typedef struct fp8_block_run_args {
 FP8BLOCK_API size_t fp8_block_region_bytes(int rows, int d_model, int ffn_hidden);
 FP8BLOCK_API int fp8_block_run(const fp8_block_run_args_t* args);
 
+/* The same, and a step's products take their rows as values, through gemm_rows (fp8_gemm_rows of libfp8gemm.so; NULL: none does),
+ * wherever that does not return cudaErrorNotSupported: the quantisers ahead of them are then not launched, and x is not copied to h.
+ * Results may differ from fp8_block_run's by the order in which an RMSNorm adds its squares.  Places of those four calls: 11 to 14. */
+struct fp8_gemm_rows_args;
+FP8BLOCK_API int fp8_block_run_rows(const fp8_block_run_args_t* args, int (*gemm_rows)(const struct fp8_gemm_rows_args*));
+
 #ifdef __cplusplus
 }
 #endif

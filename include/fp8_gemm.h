@@ -25,6 +25,7 @@
 #define GOML_FP8_GEMM_H_
 
 #include <stddef.h>
+#include <stdint.h>
 
 #ifdef __cplusplus
 extern "C" {
@@ -84,6 +85,42 @@ FP8GEMM_API int fp8_gemm_swiglu(int M, int F, int K, const void* A, const void* 
  * (fp8_rmsnorm_quantize_into). */
 FP8GEMM_API int fp8_gemm_swiglu_raise(int M, int F, int K, const void* A, const void* B_interleaved, void* H, float alpha,
                                       const float* scale_a, const float* scale_b, float* amax, void* stream);
+
+/* Additive: the product for one or two rows of A that are given as the values their codes are made of: every thread block
+ * quantises them for itself, while the weight's first tiles are on their way, instead of a quantiser ahead of the product (a step
+ * of one sequence: ten kernels, six this way).  One per-tensor scale, max|value| / 448, like the quantisers of this directory; the
+ * values, rows [M, K] without gaps, are
+ *   FP8_ROWS_RMSNORM_F32  the RMSNorm of fp32 rows: (x * gamma) * (1 / sqrt(mean(x^2) + eps)), gamma [K] fp32;
+ *   FP8_ROWS_F16          fp16 as they are;
+ *   FP8_ROWS_BF16         bf16, their largest magnitude known: *amax.
+ * The output, one of three, with s = scale of the rows * (*scale_b):
+ *   c   [M, N] bf16 = s * A . B^T;
+ *   x   [M, N] fp32 = x_in + s * A . B^T   (x_in: x itself or a matrix of its own);
+ *   h   [M, N] bf16 = silu(s * gate) * (s * up), B interleaved as fp8_gemm_swiglu reads it ([2 * N rounded up to 32, K]), *h_amax raised.
+ * zero[0 .. zeros) (zeros <= 64; may be NULL) is set to 0 for later calls of a chain.  b_complete != 0 promises that B and *scale_b are
+ * not written by work of the stream that the kernel just ahead of this call on the stream may overlap: B is then read before that
+ * kernel has ended.  None of the outputs may overlap the rows.  rows, gamma, B 16-byte aligned, x_in and x 4-byte, c and h 2-byte; K a
+ * multiple of 16.
+ * Returns cudaErrorNotSupported, with nothing launched, where M or the sizes are not ones this kernel takes. */
+enum { FP8_ROWS_RMSNORM_F32 = 1, FP8_ROWS_F16 = 2, FP8_ROWS_BF16 = 3 };
+typedef struct fp8_gemm_rows_args {
+    const void* rows;
+    const float* gamma;
+    const float* amax;
+    const void* b;
+    const float* scale_b;
+    void* c;
+    float* x;
+    const float* x_in;
+    void* h;
+    float* h_amax;
+    float* zero;
+    void* stream;
+    int32_t m, n, k, source, zeros, b_complete;
+    float eps;
+    int32_t reserved;
+} fp8_gemm_rows_args_t;
+FP8GEMM_API int fp8_gemm_rows(const fp8_gemm_rows_args_t* args);
 
 /* Additive extension: e4m3 output with delayed scaling, the epilogue of the reference's cuBLASLt wrapper
  * (fp8_matmul_fp8out, libs1/cublas_lt_wrapper_v3.c:157-229: D type CUDA_R_8F_E4M3 with D_SCALE_POINTER and
