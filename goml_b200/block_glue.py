@@ -53,9 +53,13 @@ _PACK_RUN = struct.Struct("@30PNP8i2f").pack
 assert struct.calcsize("@30PNP8i2f") == C.sizeof(BlockRunArgs)
 
 
-def BlockRun(*args, gemm_rows: int = 0) -> int:
-    """fp8_block_run with the fields of BlockRunArgs in order, or fp8_block_run_rows with the address of its gemm_rows; the return code."""
+def BlockRun(*args) -> int:
+    """fp8_block_run with the fields of BlockRunArgs in order, or fp8_block_run_rows with the address of its gemm_rows behind them; the
+    return code."""
     run = _run or _load_run()
+    gemm_rows = 0
+    if len(args) > len(BlockRunArgs._fields_):
+        *args, gemm_rows = args
     try:
         block = _PACK_RUN(*args)
     except (struct.error, OverflowError):   # values that only ctypes takes

@@ -233,7 +233,7 @@ class FP8DecoderBlock:
                          self.norm2.data_ptr(), qkv.codes.data_ptr(), o.codes.data_ptr(), self.gate_up_interleaved.data_ptr(), down.codes.data_ptr(),
                          qkv.scale_ptr, o.scale_ptr, gate_up.scale_ptr, down.scale_ptr, cos.data_ptr(), sin.data_ptr(), k, v, ks, lens,
                          words, rstd, codes, kc, vc, region, region_bytes, torch.cuda.current_stream().cuda_stream,
-                         B, S, d, H, Fh, s_max, tables, int(decode), self.eps, 1.0 / math.sqrt(self.hd), gemm_rows=gemm_rows)
+                         B, S, d, H, Fh, s_max, tables, int(decode), self.eps, 1.0 / math.sqrt(self.hd), gemm_rows)
         if rc:
             self._raise(rc, decode, cache is not None)
         return h, buf, kc, vc, words + 72
