@@ -417,274 +417,271 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     const uint32_t tmem_o = tmem_base + C::O_COL;
     const bool bad_start = (*abort_flag != 0);
     if (VRAW) pdl_wait();   // no pre-pass has waited for what is ahead
-    // Both halves of the CTA take part, the idle warp included.  (In each role's branch: in front of them the compiler gives every
-    // role what the smaller share allows.)
-    auto give_registers = []() {
-        if constexpr (C::CONVERTER) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(OTHER_REGS));
-    };
     if (bad_start) {
         // fall through to teardown
-    } else if (warp == TMA_WARP) {
-        give_registers();
-        // ------------------------------------------------------------- TMA producer
-        // The whole warp runs the loop and one elected lane issues: addresses and coordinates stay warp-uniform.
-        {
-            const bool leader = elect_one();
-            if (leader) {
-                prefetch_tmap(&tmap_q);
-                prefetch_tmap(&tmap_k);
-                prefetch_tmap(&tmap_v);
-            }
-            bool ok = true;
-            int s = 0, raw = 0;            // ring stages of the next block, of K and V and of the codes of V
-            uint32_t ph = 0, raw_ph = 0;   // their phases
-            uint32_t tph = 0;              // phase of the tile
-            Tile t(p, blockIdx.x);
-            for (bool first = true;; first = false) {          // first tile of this CTA: the rings are empty
-                const int before = s == 0 ? STAGES - 1 : s - 1;
-                const uint32_t before_ph = s == 0 ? ph ^ 1 : ph;
-                auto load_q = [&]() {
-                    mbar_arrive_expect_tx(bar_q, C::Q_BYTES);
-                    tma_load_3d(sbase + C::OFF_Q, &tmap_q, bar_q, 0, t.q0, t.head);
-                };
-                if (first && leader) load_q();
-                if constexpr (VRAW && !C::CONVERTER) {
-                    auto load_k = [&](int j, int at) {
-                        mbar_arrive_expect_tx(bar_kfull + 8 * at, C::K_BYTES);
-                        tma_load_3d(sbase + C::OFF_K + at * C::K_BYTES, &tmap_k, bar_kfull + 8 * at, 0, (t.blk0 + j) * BN, t.head);
+    } else if (warp >= NUM_SOFTMAX_WARPS) {
+        // One instruction for the whole warpgroup, the idle warp included, which must not part before it.  (In front of the branch between
+        // the two halves of the CTA the compiler would give both what the smaller share allows.)
+        if constexpr (C::CONVERTER) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(OTHER_REGS));
+        if (warp == TMA_WARP) {
+            // ------------------------------------------------------------- TMA producer
+            // The whole warp runs the loop and one elected lane issues: addresses and coordinates stay warp-uniform.
+            {
+                const bool leader = elect_one();
+                if (leader) {
+                    prefetch_tmap(&tmap_q);
+                    prefetch_tmap(&tmap_k);
+                    prefetch_tmap(&tmap_v);
+                }
+                bool ok = true;
+                int s = 0, raw = 0;            // ring stages of the next block, of K and V and of the codes of V
+                uint32_t ph = 0, raw_ph = 0;   // their phases
+                uint32_t tph = 0;              // phase of the tile
+                Tile t(p, blockIdx.x);
+                for (bool first = true;; first = false) {          // first tile of this CTA: the rings are empty
+                    const int before = s == 0 ? STAGES - 1 : s - 1;
+                    const uint32_t before_ph = s == 0 ? ph ^ 1 : ph;
+                    auto load_q = [&]() {
+                        mbar_arrive_expect_tx(bar_q, C::Q_BYTES);
+                        tma_load_3d(sbase + C::OFF_Q, &tmap_q, bar_q, 0, t.q0, t.head);
                     };
-                    auto load_v = [&](int j, int at) {
-                        mbar_arrive_expect_tx(bar_vraw + 8 * at, C::K_BYTES);
-                        tma_load_3d(sbase + C::OFF_VRAW + at * C::K_BYTES, &tmap_v, bar_vraw + 8 * at, 0, (t.blk0 + j) * BN, t.head);
-                    };
-                    const int s0 = s;
-                    const uint32_t ph0 = ph;
-                    if (!first) {
-                        // with the last Q K^T of the tile before, Q and all stages of the K ring are free
-                        ok = mbar_wait_warp(bar_sfull + 8 * before, before_ph, abort_flag, ST_TIMEOUT_LOAD);
-                        if (!ok) break;
-                        if (leader) load_q();
-                    }
-                    if (leader) {
-                        for (int j = 0; j < STAGES && j < t.nblk; j++) {
-                            const int at = s0 + j < STAGES ? s0 + j : s0 + j - STAGES;
-                            load_k(j, at);
-                            load_v(j, at);
-                        }
-                    }
-                    __syncwarp();
-                    for (int j = 0; j < t.nblk; j++) {
-                        ok = mbar_wait_warp(bar_vraw + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD) &&
-                             mbar_wait_warp(bar_pvdone + 8 * s, ph ^ 1, abort_flag, ST_TIMEOUT_LOAD);   // P V three blocks back is done
-                        if (!ok) break;
-                        // and with it every MMA issued before it, Q K^T two blocks back among them: its K stage is free.  (In the third
-                        // block of a tile only the tile before has been waited for: there the first Q K^T is.)
-                        if (j + 1 >= STAGES && j + 1 < t.nblk) {
-                            if (j + 1 == STAGES) ok = mbar_wait_warp(bar_sfull + 8 * s0, ph0, abort_flag, ST_TIMEOUT_LOAD);
-                            if (!ok) break;
-                            if (leader) load_k(j + 1, s + 1 < STAGES ? s + 1 : 0);
-                        }
-                        convert_v<HD>(sbase + C::OFF_VRAW + s * C::K_BYTES, sbase + C::OFF_V + s * C::V_BYTES);
-                        fence_proxy_async_smem();
-                        __syncwarp();
-                        if (leader) {
-                            mbar_arrive(bar_vfull + 8 * s);
-                            if (j + STAGES < t.nblk) load_v(j + STAGES, s);
-                        }
-                        __syncwarp();
-                        if (++s == STAGES) { s = 0; ph ^= 1; }
-                    }
-                } else {
-                    // Q and K are complete when this kernel starts (a pre-pass triggers it after its own wait); the fp16 copy
-                    // of V is waited for chunk by chunk, or as a whole when the launch has no flags
-                    int v_ready = 0;
-                    const uint32_t* head_flags = !VRAW && p.v_flags ? p.v_flags + (size_t)t.head * p.v_chunks : nullptr;
-                    for (int j = 0; j < t.nblk; j++) {
-                        const int key0 = (t.blk0 + j) * BN;
-                        const bool fresh = first && j < STAGES;
-                        ok = fresh || mbar_wait_warp(bar_sfull + 8 * s, ph ^ 1, abort_flag, ST_TIMEOUT_LOAD);   // Q K^T three blocks back is done
-                        if (!ok) break;
-                        if (leader) {
-                            mbar_arrive_expect_tx(bar_kfull + 8 * s, C::K_BYTES);
-                            tma_load_3d(sbase + C::OFF_K + s * C::K_BYTES, &tmap_k, bar_kfull + 8 * s, 0, key0, t.head);
-                        }
-                        if (VRAW) {
-                            ok = (first && j < C::RAW_STAGES) || mbar_wait_warp(bar_vfree + 8 * raw, raw_ph ^ 1, abort_flag, ST_TIMEOUT_LOAD);
-                            if (!ok) break;
-                            if (leader) {
-                                mbar_arrive_expect_tx(bar_vraw + 8 * raw, C::K_BYTES);
-                                tma_load_3d(sbase + C::OFF_VRAW + raw * C::K_BYTES, &tmap_v, bar_vraw + 8 * raw, 0, key0, t.head);
-                            }
-                            if (++raw == C::RAW_STAGES) { raw = 0; raw_ph ^= 1; }
-                        }
-                        if (!first && j == 0) {
-                            // with the last Q K^T of the tile before, Q is free
+                    if (first && leader) load_q();
+                    if constexpr (VRAW && !C::CONVERTER) {
+                        auto load_k = [&](int j, int at) {
+                            mbar_arrive_expect_tx(bar_kfull + 8 * at, C::K_BYTES);
+                            tma_load_3d(sbase + C::OFF_K + at * C::K_BYTES, &tmap_k, bar_kfull + 8 * at, 0, (t.blk0 + j) * BN, t.head);
+                        };
+                        auto load_v = [&](int j, int at) {
+                            mbar_arrive_expect_tx(bar_vraw + 8 * at, C::K_BYTES);
+                            tma_load_3d(sbase + C::OFF_VRAW + at * C::K_BYTES, &tmap_v, bar_vraw + 8 * at, 0, (t.blk0 + j) * BN, t.head);
+                        };
+                        const int s0 = s;
+                        const uint32_t ph0 = ph;
+                        if (!first) {
+                            // with the last Q K^T of the tile before, Q and all stages of the K ring are free
                             ok = mbar_wait_warp(bar_sfull + 8 * before, before_ph, abort_flag, ST_TIMEOUT_LOAD);
                             if (!ok) break;
                             if (leader) load_q();
                         }
-                        if (!VRAW) {
-                            ok = fresh || mbar_wait_warp(bar_pvdone + 8 * s, ph ^ 1, abort_flag, ST_TIMEOUT_LOAD);  // P V three blocks back is done
-                            if (!ok) break;
-                            if (!head_flags) {
-                                if (j == 0) pdl_wait();
-                            } else {
-                                ok = wait_v_chunk(head_flags, p.v_chunks, p.v_epoch, key0 / V_CHUNK, v_ready, abort_flag);
-                                if (!ok) break;
-                            }
-                            if (leader) {
-                                mbar_arrive_expect_tx(bar_vfull + 8 * s, C::V_BYTES);
-#pragma unroll
-                                for (int h = 0; h < HD / 64; h++)  // one 64-column (128-byte) slab of d per copy
-                                    tma_load_3d(sbase + C::OFF_V + s * C::V_BYTES + h * C::V_HALF_BYTES, &tmap_v, bar_vfull + 8 * s,
-                                                h * 64, key0, t.head);
+                        if (leader) {
+                            for (int j = 0; j < STAGES && j < t.nblk; j++) {
+                                const int at = s0 + j < STAGES ? s0 + j : s0 + j - STAGES;
+                                load_k(j, at);
+                                load_v(j, at);
                             }
                         }
                         __syncwarp();
-                        if (++s == STAGES) { s = 0; ph ^= 1; }
-                    }
-                }
-                if (!ok || !WALK) break;
-                // Another tile is asked for with this one's last block on its way, some three before the softmax warps finish: earlier, the
-                // launch's last tiles would go to whoever asks and not to whoever is done first.
-                if (!first && !mbar_wait_warp(bar_seen, tph ^ 1, abort_flag, ST_TIMEOUT_LOAD)) break;
-                if (leader) {
-                    mbar_arrive_expect_tx(bar_answer, 16);
-                    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
-                                 ::"r"(response), "r"(bar_answer) : "memory");
-                }
-                __syncwarp();
-                if (!mbar_wait_warp(bar_answer, tph, abort_flag, ST_TIMEOUT_LOAD)) break;
-                const int index = taken_tile(response);
-                if (index < 0) t.nblk = 0;
-                else t = Tile(p, index);
-                if (leader) {
-                    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(record), "r"(t.head), "r"(t.q0), "r"(t.blk0), "r"(t.nblk) : "memory");
-                    mbar_arrive(bar_next);
-                }
-                __syncwarp();
-                tph ^= 1;
-                if (t.nblk == 0) break;
-            }
-            if (!VRAW) pdl_wait();   // this kernel completes after the pre-pass
-        }
-    } else if (C::CONVERTER && warp == CONVERT_WARP) {
-        give_registers();
-        // ------------------------------------------------------------- V: codes -> fp16
-        if constexpr (C::CONVERTER) {
-            const bool leader = elect_one();
-            bool ok = true;
-            int s = 0, raw = 0;
-            uint32_t ph = 0, raw_ph = 0, tph = 0;
-            for (int nblk = Tile(p, blockIdx.x).nblk;;) {
-                for (int j = 0; j < nblk; j++) {
-                    ok = mbar_wait_warp(bar_vraw + 8 * raw, raw_ph, abort_flag, ST_TIMEOUT_LOAD) &&
-                         mbar_wait_warp(bar_pvdone + 8 * s, ph ^ 1, abort_flag, ST_TIMEOUT_LOAD);   // P V three blocks back is done
-                    if (!ok) break;
-                    convert_v<HD>(sbase + C::OFF_VRAW + raw * C::K_BYTES, sbase + C::OFF_V + s * C::V_BYTES);
-                    fence_proxy_async_smem();
-                    __syncwarp();
-                    if (leader) {
-                        mbar_arrive(bar_vfull + 8 * s);
-                        mbar_arrive(bar_vfree + 8 * raw);
-                    }
-                    __syncwarp();
-                    if (++s == STAGES) { s = 0; ph ^= 1; }
-                    if (++raw == C::RAW_STAGES) { raw = 0; raw_ph ^= 1; }
-                }
-                if (!ok || !WALK || !mbar_wait_warp(bar_next, tph, abort_flag, ST_TIMEOUT_LOAD)) break;
-                nblk = tile_record(record).nblk;
-                __syncwarp();
-                if (leader) mbar_arrive(bar_seen);
-                tph ^= 1;
-                if (nblk == 0) break;
-            }
-        }
-    } else if (warp == MMA_WARP) {
-        give_registers();
-        // -------------------------------------------------------------- MMA issuer
-        // Whole warp, one elected lane issues (descriptors stay in uniform registers).
-        {
-            const bool leader = elect_one();
-            constexpr uint32_t idesc_qk = make_idesc_e4m3_f32(BM, BN, 0, 0);
-            constexpr uint32_t idesc_pv = make_idesc_f16_f32(BM, HD, 0, 1);  // A = P from TMEM, V is MN-major
-            auto qk_desc = [&](uint32_t addr) { return HD == 128 ? kmajor_desc_sw128(addr) : kmajor_desc_sw64(addr); };
-            // K ring position of the next Q K^T, V ring position of the next P V
-            int ks = 0, vs = 0;
-            uint32_t kph = 0, vph = 0;
-            bool ok = true;
-            uint32_t kb = 0, vb = 0;      // S buffers of the next Q K^T and of the next P V
-            uint32_t pph = 0;             // bit b: phase of P in S[b]
-            uint32_t tph = 0, qph = 0;    // phases of the next tile's record and of Q
-            auto issue_qk = [&]() {       // S[kb] = Q K^T of the next block
-                ok = mbar_wait_warp(bar_kfull + 8 * ks, kph, abort_flag, ST_TIMEOUT_MMA);
-                if (!ok) return;
-                tc_fence_after();
-                const uint64_t qd = qk_desc(sbase + C::OFF_Q);
-                const uint64_t kd = qk_desc(sbase + C::OFF_K + ks * C::K_BYTES);
-                if (leader) {
-#pragma unroll
-                    for (int k = 0; k < HD / 32; k++)
-                        mma_f8f6f4_ss(tmem_s + kb * BN, qd + 2 * k, kd + 2 * k, idesc_qk, k != 0);
-                    mma_commit(bar_sfull + 8 * ks);
-                }
-                __syncwarp();
-                kb ^= 1;
-                if (++ks == STAGES) { ks = 0; kph ^= 1; }
-            };
-            // Two blocks' scores are ahead of the P V, across the end of a tile too: behind this tile's last but one P V follows the
-            // next one's first Q K^T, so that the softmax warps have its scores to work on until the last P V is done.
-            int nblk = Tile(p, blockIdx.x).nblk, next = -1;   // blocks of this tile and of the next (-1: not known yet, 0: none)
-            int qk = 0;                                       // Q K^T issued of this tile or, once next >= 0, of the next
-            ok = mbar_wait_warp(bar_q, 0, abort_flag, ST_TIMEOUT_MMA);
-            for (; nblk > 0 && ok;) {
-                for (int j = 0; j < nblk && ok; j++) {
-                    while (ok && (next < 0 ? qk : nblk + qk) < j + 2) {
-                        if (next < 0 && qk == nblk) {
-                            if (!WALK) { next = 0; break; }
-                            ok = mbar_wait_warp(bar_next, tph, abort_flag, ST_TIMEOUT_MMA);
+                        for (int j = 0; j < t.nblk; j++) {
+                            ok = mbar_wait_warp(bar_vraw + 8 * s, ph, abort_flag, ST_TIMEOUT_LOAD) &&
+                                 mbar_wait_warp(bar_pvdone + 8 * s, ph ^ 1, abort_flag, ST_TIMEOUT_LOAD);   // P V three blocks back is done
                             if (!ok) break;
-                            next = tile_record(record).nblk;
-                            __syncwarp();
-                            if (leader) mbar_arrive(bar_seen);
-                            tph ^= 1;
-                            qk = 0;
-                            if (next > 0) {
-                                qph ^= 1;
-                                ok = mbar_wait_warp(bar_q, qph, abort_flag, ST_TIMEOUT_MMA);
+                            // and with it every MMA issued before it, Q K^T two blocks back among them: its K stage is free.  (In the third
+                            // block of a tile only the tile before has been waited for: there the first Q K^T is.)
+                            if (j + 1 >= STAGES && j + 1 < t.nblk) {
+                                if (j + 1 == STAGES) ok = mbar_wait_warp(bar_sfull + 8 * s0, ph0, abort_flag, ST_TIMEOUT_LOAD);
+                                if (!ok) break;
+                                if (leader) load_k(j + 1, s + 1 < STAGES ? s + 1 : 0);
                             }
+                            convert_v<HD>(sbase + C::OFF_VRAW + s * C::K_BYTES, sbase + C::OFF_V + s * C::V_BYTES);
+                            fence_proxy_async_smem();
+                            __syncwarp();
+                            if (leader) {
+                                mbar_arrive(bar_vfull + 8 * s);
+                                if (j + STAGES < t.nblk) load_v(j + STAGES, s);
+                            }
+                            __syncwarp();
+                            if (++s == STAGES) { s = 0; ph ^= 1; }
                         }
-                        if (!ok || (next >= 0 && qk == next)) break;
-                        issue_qk();
-                        qk++;
-                    }
-                    if (!ok) break;
-                    const uint32_t b = vb;
-                    ok = mbar_wait_warp(bar_vfull + 8 * vs, vph, abort_flag, ST_TIMEOUT_MMA) &&
-                         mbar_wait_warp(bar_pfull + 8 * b, (pph >> b) & 1, abort_flag, ST_TIMEOUT_MMA);
-                    if (!ok) break;
-                    pph ^= 1u << b;
-                    vb ^= 1;
-                    tc_fence_after();
-                    const uint32_t vaddr = sbase + C::OFF_V + vs * C::V_BYTES;
-                    if (leader) {
+                    } else {
+                        // Q and K are complete when this kernel starts (a pre-pass triggers it after its own wait); the fp16 copy
+                        // of V is waited for chunk by chunk, or as a whole when the launch has no flags
+                        int v_ready = 0;
+                        const uint32_t* head_flags = !VRAW && p.v_flags ? p.v_flags + (size_t)t.head * p.v_chunks : nullptr;
+                        for (int j = 0; j < t.nblk; j++) {
+                            const int key0 = (t.blk0 + j) * BN;
+                            const bool fresh = first && j < STAGES;
+                            ok = fresh || mbar_wait_warp(bar_sfull + 8 * s, ph ^ 1, abort_flag, ST_TIMEOUT_LOAD);   // Q K^T three blocks back is done
+                            if (!ok) break;
+                            if (leader) {
+                                mbar_arrive_expect_tx(bar_kfull + 8 * s, C::K_BYTES);
+                                tma_load_3d(sbase + C::OFF_K + s * C::K_BYTES, &tmap_k, bar_kfull + 8 * s, 0, key0, t.head);
+                            }
+                            if (VRAW) {
+                                ok = (first && j < C::RAW_STAGES) || mbar_wait_warp(bar_vfree + 8 * raw, raw_ph ^ 1, abort_flag, ST_TIMEOUT_LOAD);
+                                if (!ok) break;
+                                if (leader) {
+                                    mbar_arrive_expect_tx(bar_vraw + 8 * raw, C::K_BYTES);
+                                    tma_load_3d(sbase + C::OFF_VRAW + raw * C::K_BYTES, &tmap_v, bar_vraw + 8 * raw, 0, key0, t.head);
+                                }
+                                if (++raw == C::RAW_STAGES) { raw = 0; raw_ph ^= 1; }
+                            }
+                            if (!first && j == 0) {
+                                // with the last Q K^T of the tile before, Q is free
+                                ok = mbar_wait_warp(bar_sfull + 8 * before, before_ph, abort_flag, ST_TIMEOUT_LOAD);
+                                if (!ok) break;
+                                if (leader) load_q();
+                            }
+                            if (!VRAW) {
+                                ok = fresh || mbar_wait_warp(bar_pvdone + 8 * s, ph ^ 1, abort_flag, ST_TIMEOUT_LOAD);  // P V three blocks back is done
+                                if (!ok) break;
+                                if (!head_flags) {
+                                    if (j == 0) pdl_wait();
+                                } else {
+                                    ok = wait_v_chunk(head_flags, p.v_chunks, p.v_epoch, key0 / V_CHUNK, v_ready, abort_flag);
+                                    if (!ok) break;
+                                }
+                                if (leader) {
+                                    mbar_arrive_expect_tx(bar_vfull + 8 * s, C::V_BYTES);
 #pragma unroll
-                        for (int k = 0; k < BN / 16; k++) {  // 16 keys per MMA: 8 TMEM columns of P, 16 rows of V
-                            const uint64_t vd = mnmajor_desc_sw128(vaddr + k * 16 * 128, C::V_HALF_BYTES);
-                            mma_f16_ts(tmem_o, tmem_s + b * BN + 8 * k, vd, idesc_pv, (j | k) != 0);
+                                    for (int h = 0; h < HD / 64; h++)  // one 64-column (128-byte) slab of d per copy
+                                        tma_load_3d(sbase + C::OFF_V + s * C::V_BYTES + h * C::V_HALF_BYTES, &tmap_v, bar_vfull + 8 * s,
+                                                    h * 64, key0, t.head);
+                                }
+                            }
+                            __syncwarp();
+                            if (++s == STAGES) { s = 0; ph ^= 1; }
                         }
-                        mma_commit(bar_pvdone + 8 * vs);
+                    }
+                    if (!ok || !WALK) break;
+                    // Another tile is asked for with this one's last block on its way, some three before the softmax warps finish: earlier, the
+                    // launch's last tiles would go to whoever asks and not to whoever is done first.
+                    if (!first && !mbar_wait_warp(bar_seen, tph ^ 1, abort_flag, ST_TIMEOUT_LOAD)) break;
+                    if (leader) {
+                        mbar_arrive_expect_tx(bar_answer, 16);
+                        asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+                                     ::"r"(response), "r"(bar_answer) : "memory");
                     }
                     __syncwarp();
-                    if (++vs == STAGES) { vs = 0; vph ^= 1; }
-                    // S[b] is rewritten by the Q K^T two blocks ahead; it is issued behind this P V on the
-                    // same in-order tensor pipe, so P(j) has been read before S(j+2) lands on it
+                    if (!mbar_wait_warp(bar_answer, tph, abort_flag, ST_TIMEOUT_LOAD)) break;
+                    const int index = taken_tile(response);
+                    if (index < 0) t.nblk = 0;
+                    else t = Tile(p, index);
+                    if (leader) {
+                        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(record), "r"(t.head), "r"(t.q0), "r"(t.blk0), "r"(t.nblk) : "memory");
+                        mbar_arrive(bar_next);
+                    }
+                    __syncwarp();
+                    tph ^= 1;
+                    if (t.nblk == 0) break;
                 }
-                nblk = next;   // its first P V, which overwrites O, waits for a P that is published after O has been read
-                next = -1;
+                if (!VRAW) pdl_wait();   // this kernel completes after the pre-pass
+            }
+        } else if (C::CONVERTER && warp == CONVERT_WARP) {
+            // ------------------------------------------------------------- V: codes -> fp16
+            if constexpr (C::CONVERTER) {
+                const bool leader = elect_one();
+                bool ok = true;
+                int s = 0, raw = 0;
+                uint32_t ph = 0, raw_ph = 0, tph = 0;
+                for (int nblk = Tile(p, blockIdx.x).nblk;;) {
+                    for (int j = 0; j < nblk; j++) {
+                        ok = mbar_wait_warp(bar_vraw + 8 * raw, raw_ph, abort_flag, ST_TIMEOUT_LOAD) &&
+                             mbar_wait_warp(bar_pvdone + 8 * s, ph ^ 1, abort_flag, ST_TIMEOUT_LOAD);   // P V three blocks back is done
+                        if (!ok) break;
+                        convert_v<HD>(sbase + C::OFF_VRAW + raw * C::K_BYTES, sbase + C::OFF_V + s * C::V_BYTES);
+                        fence_proxy_async_smem();
+                        __syncwarp();
+                        if (leader) {
+                            mbar_arrive(bar_vfull + 8 * s);
+                            mbar_arrive(bar_vfree + 8 * raw);
+                        }
+                        __syncwarp();
+                        if (++s == STAGES) { s = 0; ph ^= 1; }
+                        if (++raw == C::RAW_STAGES) { raw = 0; raw_ph ^= 1; }
+                    }
+                    if (!ok || !WALK || !mbar_wait_warp(bar_next, tph, abort_flag, ST_TIMEOUT_LOAD)) break;
+                    nblk = tile_record(record).nblk;
+                    __syncwarp();
+                    if (leader) mbar_arrive(bar_seen);
+                    tph ^= 1;
+                    if (nblk == 0) break;
+                }
+            }
+        } else if (warp == MMA_WARP) {
+            // -------------------------------------------------------------- MMA issuer
+            // Whole warp, one elected lane issues (descriptors stay in uniform registers).
+            {
+                const bool leader = elect_one();
+                constexpr uint32_t idesc_qk = make_idesc_e4m3_f32(BM, BN, 0, 0);
+                constexpr uint32_t idesc_pv = make_idesc_f16_f32(BM, HD, 0, 1);  // A = P from TMEM, V is MN-major
+                auto qk_desc = [&](uint32_t addr) { return HD == 128 ? kmajor_desc_sw128(addr) : kmajor_desc_sw64(addr); };
+                // K ring position of the next Q K^T, V ring position of the next P V
+                int ks = 0, vs = 0;
+                uint32_t kph = 0, vph = 0;
+                bool ok = true;
+                uint32_t kb = 0, vb = 0;      // S buffers of the next Q K^T and of the next P V
+                uint32_t pph = 0;             // bit b: phase of P in S[b]
+                uint32_t tph = 0, qph = 0;    // phases of the next tile's record and of Q
+                auto issue_qk = [&]() {       // S[kb] = Q K^T of the next block
+                    ok = mbar_wait_warp(bar_kfull + 8 * ks, kph, abort_flag, ST_TIMEOUT_MMA);
+                    if (!ok) return;
+                    tc_fence_after();
+                    const uint64_t qd = qk_desc(sbase + C::OFF_Q);
+                    const uint64_t kd = qk_desc(sbase + C::OFF_K + ks * C::K_BYTES);
+                    if (leader) {
+#pragma unroll
+                        for (int k = 0; k < HD / 32; k++)
+                            mma_f8f6f4_ss(tmem_s + kb * BN, qd + 2 * k, kd + 2 * k, idesc_qk, k != 0);
+                        mma_commit(bar_sfull + 8 * ks);
+                    }
+                    __syncwarp();
+                    kb ^= 1;
+                    if (++ks == STAGES) { ks = 0; kph ^= 1; }
+                };
+                // Two blocks' scores are ahead of the P V, across the end of a tile too: behind this tile's last but one P V follows the
+                // next one's first Q K^T, so that the softmax warps have its scores to work on until the last P V is done.
+                int nblk = Tile(p, blockIdx.x).nblk, next = -1;   // blocks of this tile and of the next (-1: not known yet, 0: none)
+                int qk = 0;                                       // Q K^T issued of this tile or, once next >= 0, of the next
+                ok = mbar_wait_warp(bar_q, 0, abort_flag, ST_TIMEOUT_MMA);
+                for (; nblk > 0 && ok;) {
+                    for (int j = 0; j < nblk && ok; j++) {
+                        while (ok && (next < 0 ? qk : nblk + qk) < j + 2) {
+                            if (next < 0 && qk == nblk) {
+                                if (!WALK) { next = 0; break; }
+                                ok = mbar_wait_warp(bar_next, tph, abort_flag, ST_TIMEOUT_MMA);
+                                if (!ok) break;
+                                next = tile_record(record).nblk;
+                                __syncwarp();
+                                if (leader) mbar_arrive(bar_seen);
+                                tph ^= 1;
+                                qk = 0;
+                                if (next > 0) {
+                                    qph ^= 1;
+                                    ok = mbar_wait_warp(bar_q, qph, abort_flag, ST_TIMEOUT_MMA);
+                                }
+                            }
+                            if (!ok || (next >= 0 && qk == next)) break;
+                            issue_qk();
+                            qk++;
+                        }
+                        if (!ok) break;
+                        const uint32_t b = vb;
+                        ok = mbar_wait_warp(bar_vfull + 8 * vs, vph, abort_flag, ST_TIMEOUT_MMA) &&
+                             mbar_wait_warp(bar_pfull + 8 * b, (pph >> b) & 1, abort_flag, ST_TIMEOUT_MMA);
+                        if (!ok) break;
+                        pph ^= 1u << b;
+                        vb ^= 1;
+                        tc_fence_after();
+                        const uint32_t vaddr = sbase + C::OFF_V + vs * C::V_BYTES;
+                        if (leader) {
+#pragma unroll
+                            for (int k = 0; k < BN / 16; k++) {  // 16 keys per MMA: 8 TMEM columns of P, 16 rows of V
+                                const uint64_t vd = mnmajor_desc_sw128(vaddr + k * 16 * 128, C::V_HALF_BYTES);
+                                mma_f16_ts(tmem_o, tmem_s + b * BN + 8 * k, vd, idesc_pv, (j | k) != 0);
+                            }
+                            mma_commit(bar_pvdone + 8 * vs);
+                        }
+                        __syncwarp();
+                        if (++vs == STAGES) { vs = 0; vph ^= 1; }
+                        // S[b] is rewritten by the Q K^T two blocks ahead; it is issued behind this P V on the
+                        // same in-order tensor pipe, so P(j) has been read before S(j+2) lands on it
+                    }
+                    nblk = next;   // its first P V, which overwrites O, waits for a P that is published after O has been read
+                    next = -1;
+                }
             }
         }
-    } else if (warp < NUM_SOFTMAX_WARPS) {
+    } else {
         if constexpr (C::CONVERTER) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SOFTMAX_REGS));
         // ------------------------------------------- softmax / correction / epilogue
         const int r = threadIdx.x;               // row of the tile = TMEM lane (one thread per row)
@@ -962,10 +959,6 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
             p_bar ^= 8;
             j = 1;
         }
-    }
-
-    else {
-        give_registers();
     }
     // ----------------------------------------------------------------- teardown
     __syncwarp();
