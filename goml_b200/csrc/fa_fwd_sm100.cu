@@ -64,6 +64,7 @@ constexpr int TMA_WARP = NUM_SOFTMAX_WARPS + 1;
 constexpr int CONVERT_WARP = NUM_SOFTMAX_WARPS + 2;   // where V has a warp of its own (Cfg::CONVERTER)
 // registers of a thread there: at launch (8 warps, two CTAs an SM), then of a softmax thread; the other half of the CTA gives them up
 constexpr int LAUNCH_REGS = 128, SOFTMAX_REGS = 160, OTHER_REGS = 2 * LAUNCH_REGS - SOFTMAX_REGS;
+constexpr uint32_t IDESC_NEGATE_A = 1u << 13;   // of the instruction descriptor
 constexpr float TAU = 6.0f;   // lazy-rescale threshold (log2 units)
 constexpr float POFF = 2.0f;  // P is carried as P * 2^POFF (max 2^(TAU+POFF) = 256, far inside fp16)
 
@@ -263,7 +264,7 @@ __device__ __forceinline__ bool wait_v_chunk(const uint32_t* head_flags, int chu
 //  D = 128 (codes swizzled too): they take four neighbouring pieces of one slab of two keys k and k ^ 5 — bit 2 of the key puts the
 //   loads in different halves of the 128 bytes, bit 0 the stores on chunks of different parity;
 //  D = 64 (codes as they lie in global memory): the four pieces of two neighbouring keys, 128 bytes in a row.
-// Unrolled in full: a loop of four steps cost 2 % at S = 8192.
+// In rounds of eight steps: code that is not there is not fetched (see the loops of the softmax warps).
 template <int HD>
 __device__ __forceinline__ void convert_v(uint32_t raw, uint32_t dst) {
     constexpr int STEPS = BN * HD / 512, BATCH = 8;   // steps of the warp, loads in flight
@@ -281,7 +282,7 @@ __device__ __forceinline__ void convert_v(uint32_t raw, uint32_t dst) {
         lo_at[t] = dst + slab * (BN * 128) + row + ((chunk ^ (2 * t)) << 4);
         hi_at[t] = dst + slab * (BN * 128) + row + ((chunk ^ (2 * t) ^ 1) << 4);
     }
-#pragma unroll
+#pragma unroll 1
     for (int i0 = 0; i0 < STEPS; i0 += BATCH) {
         uint4 v[BATCH];
 #pragma unroll
@@ -354,7 +355,7 @@ __device__ __forceinline__ Tile tile_record(uint32_t at) {
 // the CTAs of the pre-pass, which the attention's first CTAs wait for.  Bit for bit the same results.
 //
 // MASKED = false: no key of the launch is masked (non-causal, no window, S a multiple of the block) and the host-side scale
-// is positive: neither the masking code nor the sign flip of a negative scale is compiled into the softmax loop.  (The
+// is positive: the masking code is not compiled into the softmax loop, and Q K^T is not asked for with a sign.  (The
 // device-side scale factors are quantiser outputs, amax / 448: never negative.)
 //
 // AMAX = true: the largest |O| also goes to p.o_amax, for the quantiser behind (a variant of its own: the others keep their code).
@@ -602,7 +603,11 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
             // Whole warp, one elected lane issues (descriptors stay in uniform registers).
             {
                 const bool leader = elect_one();
-                constexpr uint32_t idesc_qk = make_idesc_e4m3_f32(BM, BN, 0, 0);
+                // a negative scale: the scores come out of the tensor core with the sign that their maximum is taken with
+            float sign = p.scale_log2;
+            if (MASKED && p.sq) sign *= ld_f32(p.sq);
+            if (MASKED && p.sk) sign *= ld_f32(p.sk);
+            const uint32_t idesc_qk = make_idesc_e4m3_f32(BM, BN, 0, 0) | (MASKED && sign < 0.f ? IDESC_NEGATE_A : 0u);
                 constexpr uint32_t idesc_pv = make_idesc_f16_f32(BM, HD, 0, 1);  // A = P from TMEM, V is MN-major
                 auto qk_desc = [&](uint32_t addr) { return HD == 128 ? kmajor_desc_sw128(addr) : kmajor_desc_sw64(addr); };
                 // K ring position of the next Q K^T, V ring position of the next P V
@@ -690,8 +695,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         if (p.sq) scale_log2 *= ld_f32(p.sq);
         if (p.sk) scale_log2 *= ld_f32(p.sk);
         const float vds = p.sv ? p.v_descale * ld_f32(p.sv) : p.v_descale;
-        const bool neg = scale_log2 < 0.f;       // the row max is taken on sign-adjusted raw scores
-        float ascale = fabsf(scale_log2);
+        float ascale = fabsf(scale_log2);        // the scores have the scale's sign already
         if (ascale == 0.f) ascale = 1e-30f;      // keeps -inf * scale = -inf for masked keys
         int rs = 0;           // ring stage of the next block and its phase; those of the block before
         uint32_t rph = 0;
@@ -709,7 +713,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         Tile t(p, blockIdx.x);
 
         // The scores of key block j of the tile, in the S buffer at sa, and what they do to the reference.  EDGE: the block may hold
-        // masked keys, or the scale is negative.
+        // masked keys.  (The loop over O in the rare branch stays unrolled: as a loop it made the form with a converting warp fault.)
         uint32_t sreg[BN];
         bool hidden[BN / 32];                    // no row of this warp sees these 32 keys: their P is zero
         auto scores = [&](const int j, const uint32_t sa, auto edge) -> bool {
@@ -722,10 +726,6 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
 
             hidden[0] = hidden[1] = false;
             if (EDGE) {
-                if (neg) {
-#pragma unroll
-                    for (int c = 0; c < BN; c++) sreg[c] ^= 0x80000000u;   // the row max is taken on sign-adjusted scores
-                }
                 // last and first visible key of this row, and the same of the first and the last row of its warp
                 const int wq0 = t.q0 + warp * 32;
                 const int hi_key = p.causal ? min(t.q0 + r, p.sl - 1) : p.sl - 1, lo_key = p.window > 0 ? t.q0 + r - p.window + 1 : 0;
@@ -827,8 +827,11 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
             publish(pb);
             return true;
         };
-        // blocks [j, end), two to a trip where they are clear, so that the S buffer is a constant in each copy.  (The form of this loop
-        // matters: `j + 2 <= n` with two calls in its body is 2 % slower.)
+        // Blocks [j, end) of one kind.  What these loops cost is also their code: four warps run through it in turn with the other roles', and
+        // past the instruction cache it is fetched again and again.  With the clear loop unrolled by two, a sign flip of 64 instructions
+        // in the edge loop and the conversion of V unrolled in full, us: 256 heads of 2048 of 128, causal, 298 (now 279), 64 of 8192, window
+        // 1024, 327 (287), 64 of 3000 of 64, window 512, 57.1 (52.9), 256 of 1000 of 128, not causal, 139 (131).  One loop with the edge
+        // as a test in it keeps more registers alive: 300, 305, 57.5, 143.
         auto edge_blocks = [&](int& j, const int end) -> bool {
 #pragma unroll 1
             for (; j < end; j++) {
@@ -840,11 +843,12 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         };
         auto clear_blocks = [&](int& j, const int end) -> bool {
             const int n = max(end - j, 0);
-#pragma unroll 2
-            for (int i = 0; i < n; i++)
-                if (!block(j + i, s_addr ^ (i & 1) * BN, p_bar ^ (i & 1) * 8, std::false_type())) return false;
-            s_addr ^= (n & 1) * BN;
-            p_bar ^= (n & 1) * 8;
+#pragma unroll 1
+            for (int i = 0; i < n; i++) {
+                if (!block(j + i, s_addr, p_bar, std::false_type())) return false;
+                s_addr ^= BN;
+                p_bar ^= 8;
+            }
             j += n;
             return true;
         };
@@ -917,7 +921,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
                 int j_hi = p.sl / BN - t.blk0;
                 if (p.causal) j_hi = min(j_hi, t.q0 / BN - t.blk0);
                 int j_lo = (p.window > 0 && t.q0 + BM - p.window > 0) ? (t.q0 + BM - p.window + BN - 1) / BN - t.blk0 : 0;
-                j_lo = neg ? t.nblk : min(j_lo, t.nblk);
+                j_lo = min(j_lo, t.nblk);
                 // one copy of each loop: edge, clear, edge
                 ok = true;
                 for (int stop = j_lo;; stop = t.nblk) {
