@@ -832,6 +832,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         // in the edge loop and the conversion of V unrolled in full, us: 256 heads of 2048 of 128, causal, 298 (now 279), 64 of 8192, window
         // 1024, 327 (287), 64 of 3000 of 64, window 512, 57.1 (52.9), 256 of 1000 of 128, not causal, 139 (131).  One loop with the edge
         // as a test in it keeps more registers alive: 300, 305, 57.5, 143.
+        // A CTA with a tile of its own keeps the clear loop unrolled by two: its calls are few and long (1 head of 8192 of 128, causal, 92.8 / 85.7).
         auto edge_blocks = [&](int& j, const int end) -> bool {
 #pragma unroll 1
             for (; j < end; j++) {
@@ -843,7 +844,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         };
         auto clear_blocks = [&](int& j, const int end) -> bool {
             const int n = max(end - j, 0);
-#pragma unroll 1
+            constexpr int UNROLL = WALK ? 1 : 2;
+#pragma unroll UNROLL
             for (int i = 0; i < n; i++) {
                 if (!block(j + i, s_addr, p_bar, std::false_type())) return false;
                 s_addr ^= BN;
@@ -1036,14 +1038,13 @@ bool one_to_an_sm(const LaunchArgs& a, long long tiles, int num_sms) {
     return a.causal && (a.window <= 0 || a.window >= a.sl) && a.bh <= HEAD_GROUP && 2 * tiles <= 3ll * num_sms;
 }
 
-// Whether a CTA goes on to further tiles.  That saves a tile its CTA's start (barriers, tensor memory, the first loads' latency: 3000 clk)
-// and part of its end, which the other CTA of the SM hides in part.  Start of a CTA per tile / a walk, us, both in a loop: D = 128, causal,
-// 1024 heads of 512 136 / 119, 256 of 2048 298 / 284; not causal 256 of 1000 140 / 132, 128 of 1024 70 / 64; D = 64, 512 of 512 61.6 / 51.8, 64 of
-// 3000, window 512, 61.4 / 55.9; 64 of 8192 of 128, window 1024, 305 / 304.  Long causal tiles gain nothing: 64 of 8192 930 / 939.
-bool walks(const LaunchArgs& a, long long tiles, int num_sms) {
-    const bool window = a.window > 0 && a.window < a.sl;
-    return tiles > 2ll * num_sms && !(a.causal && !window && a.sl > 6144);
-}
+// Whether a CTA goes on to further tiles: as soon as there are more than fit at once.  That saves a tile its CTA's start (barriers,
+// tensor memory, the first loads' latency: 3000 clk) and part of its end, which the other CTA of the SM hides in part.  Start of a CTA per
+// tile, as it was / a walk, us, both in a loop: D = 128, causal, 1024 heads of 512 136 / 117, 256 of 2048 293 / 274, 64 of 8192 784 / 771; not
+// causal 256 of 1000 140 / 131, 64 of 8192 1550 / 1499; D = 64, 448 of 179, causal, 19.9 / 14.8, 512 of 512 61.6 / 51.8, 64 of 3000, window
+// 512, 63.8 / 54.3, 32 of 8192, causal, 360 / 349.  Just past that line a few causal calls lose (32 of 1300 of 128 22.7 / 23.2, a CTA per
+// tile 22.7) and most gain (28 of 1700 30.4 / 24.1, a CTA per tile 26.5; 300 of 100 11.0 / 8.5 and 10.4).
+bool walks(long long tiles, int num_sms) { return tiles > 2ll * num_sms; }
 
 template <int HD, bool VRAW>
 cudaError_t launch_hd(const LaunchArgs& a, int num_sms) {
@@ -1080,7 +1081,7 @@ cudaError_t launch_hd(const LaunchArgs& a, int num_sms) {
     const bool masked = a.causal || a.window > 0 || (a.sl % BN) != 0 || !(a.scale > 0.f);
     const size_t smem = one_to_an_sm(a, grid, num_sms) ? SMEM_ONE : C::SMEM_BYTES;
     auto start = [&](auto kernel) { return launch_pdl(kernel, (unsigned)grid, C::NUM_THREADS, smem, a.stream, tq, tk, tv, p); };
-    const bool walk = walks(a, grid, num_sms);
+    const bool walk = walks(grid, num_sms);
     if (a.o_amax) return walk ? start(fa_fwd_kernel<HD, true, VRAW, true, true>) : start(fa_fwd_kernel<HD, true, VRAW, true, false>);   // the masked kernel serves every call
     if (walk) return masked ? start(fa_fwd_kernel<HD, true, VRAW, false, true>) : start(fa_fwd_kernel<HD, false, VRAW, false, true>);
     return masked ? start(fa_fwd_kernel<HD, true, VRAW, false, false>) : start(fa_fwd_kernel<HD, false, VRAW, false, false>);
