@@ -101,7 +101,7 @@ def FP8GEMMSinglesync(M, N, K, A, B, Cptr, stream=0) -> None:
 
 def FP8GEMMScaled(M, N, K, A, B, Cptr, alpha=1.0, scale_a=0, scale_b=0, out_dtype=OutBF16, stream=0) -> None:
     """C = alpha * (*scale_a) * (*scale_b) * A x B^T; scale pointers are device pointers or 0."""
-    rc = _init().fp8_gemm_scaled(M, N, K, A, B, Cptr, alpha, scale_a or None, scale_b or None, out_dtype, stream)
+    rc = (_state["lib"] or _init()).fp8_gemm_scaled(M, N, K, A, B, Cptr, alpha, scale_a or None, scale_b or None, out_dtype, stream)
     if rc != 0:
         raise FP8GEMMError(f"fp8_gemm_scaled: CUDA error {rc}")
 

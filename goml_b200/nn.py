@@ -55,8 +55,16 @@ class FP8Linear:
         self.w = quantize(weight.float())
 
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
-        M = x.numel() // self.in_features
-        return self.forward_codes(quantize(x.reshape(M, self.in_features).float()), M)
+        M, K, N = x.numel() // self.in_features, self.in_features, self.out_features
+        if x.dtype is not torch.float32 or not x.is_cuda or x.numel() != M * K or not x.is_contiguous():
+            return self.forward_codes(quantize(x.reshape(M, K).float()), M)
+        # codes, scale and amax in one allocation and no views: for a few rows a call is its host time (28.7 us with a tensor for each)
+        buf, codes, sa = _scratch(x.device, M * K, 8)
+        y = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
+        stream = torch.cuda.current_stream().cuda_stream
+        Q.QuantizeF32ToF8E4M3(x.data_ptr(), codes, sa, sa + 4, M * K, stream)
+        G.FP8GEMMScaled(M, N, K, codes, self.w.codes.data_ptr(), y.data_ptr(), 1.0, sa, self.w.scale_ptr, G.OutBF16, stream)
+        return y
 
     def accumulate_into(self, xq: FP8Tensor, M: int, x: torch.Tensor) -> None:
         """x (fp32 [M, out]) += this layer's output, added in the GEMM epilogue (no 16-bit intermediate)."""

@@ -44,7 +44,7 @@ def _init():
 
 
 def QuantizeF32ToF8E4M3(src: int, dst: int, scale: int, amax: int, n: int, stream: int = 0) -> None:
-    rc = _init().fp8_quantize_f32(src, dst, scale, amax, n, AMAX_OVER_448, stream or None)
+    rc = (_lib or _init()).fp8_quantize_f32(src, dst, scale, amax, n, AMAX_OVER_448, stream or None)
     if rc != 0:
         raise QuantizeError(f"fp8_quantize_f32: CUDA error {rc}")
 

@@ -84,3 +84,24 @@ def test_codes_on_both_sides_of_the_line(cuda, built_libs, M, K, few):
     want = (a.double() @ b.double().t())
     assert amax.item() == want.abs().max().item()
     assert torch.equal(d.view(torch.float8_e4m3fn).float(), want.float().to(torch.float8_e4m3fn).float())
+
+
+@pytest.mark.parametrize("shape", [(1, 64), (3, 5, 64), (64,), (200, 64)])
+def test_linear_layer_takes_any_tensor(cuda, built_libs, shape):
+    # contiguous fp32 goes straight to the libraries, everything else through views and copies: the same bits
+    import torch
+    from goml_b200 import nn
+    g = torch.Generator(device="cuda").manual_seed(len(shape))
+    layer = nn.FP8Linear(torch.randn(40, 64, generator=g, device="cuda"))
+    x = torch.randn(shape, generator=g, device="cuda").bfloat16().float()
+    want = layer.forward_codes(nn.quantize(x.reshape(-1, 64)), x.numel() // 64)
+    strided = torch.stack([x, x + 1], -1)[..., 0]
+    assert not strided.is_contiguous() and want.shape == (x.numel() // 64, 40)
+    for same in (x, strided, x.bfloat16(), x.double(), x.clone().requires_grad_()):
+        assert torch.equal(layer(same), want)
+    with pytest.raises(RuntimeError):
+        layer(torch.zeros(65, device="cuda"))
+    with pytest.raises(AssertionError):
+        layer(x.cpu())
+    with pytest.raises(Exception):
+        layer(torch.zeros(0, 64, device="cuda"))
