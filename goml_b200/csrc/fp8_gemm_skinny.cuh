@@ -647,7 +647,7 @@ inline int launch(GemmParams g, const Plan& plan, const void* A, const void* B, 
     if (g.M > 80) p.prefetch = 4;
     if (p.r.early) p.prefetch = 0;
     p.vec = g.H ? (g.F % 4 == 0 && (reinterpret_cast<uintptr_t>(g.H) & 7) == 0)
-          : g.X ? (g.N % 4 == 0 && (reinterpret_cast<uintptr_t>(g.X) & 15) == 0)
+          : g.X ? (g.N % 4 == 0 && ((reinterpret_cast<uintptr_t>(g.X) | (rows ? reinterpret_cast<uintptr_t>(rows->x_in) : 0)) & 15) == 0)   // both are read or written whole
           : g.D8 ? (g.N % 4 == 0 && (reinterpret_cast<uintptr_t>(g.D8) & 3) == 0)
                  : (g.N % 4 == 0 && (reinterpret_cast<uintptr_t>(g.C) & 7) == 0);
     p.g = g;

@@ -74,6 +74,35 @@ def test_rows_against_quantiser_and_product(cuda, built_libs, m, n, k, source):
     assert G.device_status() == 0
 
 
+# n a multiple of four or not, whole and cut tiles; sizes that need four slices and one
+@pytest.mark.parametrize("m,n,k", [(1, 4096, 4096), (2, 1000, 2048), (2, 1001, 2000)])
+def test_the_stream_may_lie_on_any_four_bytes(cuda, built_libs, m, n, k):
+    # x_in and x each 0 to 12 bytes past a multiple of 16: the same bits, nothing written around x
+    import torch
+    from goml_b200 import fp8_gemm as G
+    lib = G._init()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    rows = torch.randn(m, k, generator=g, device="cuda").half()
+    w = torch.randint(0, 0x70, (n, k), generator=g, dtype=torch.uint8, device="cuda")
+    ws = torch.tensor([1e-3], device="cuda")
+    base = torch.randn(m, n, generator=g, device="cuda")
+    src, dst = (torch.empty(m * n + 8, device="cuda") for _ in range(2))
+    assert src.data_ptr() % 16 == dst.data_ptr() % 16 == 0
+    got = []
+    for i in range(4):
+        for j in range(4):
+            src.fill_(9.0)
+            src[i:i + m * n].copy_(base.view(-1))
+            dst.fill_(7.0)
+            assert call(lib, rows=rows.data_ptr(), b=w.data_ptr(), scale_b=ws.data_ptr(), x=dst.data_ptr() + 4 * j, x_in=src.data_ptr() + 4 * i, m=m, n=n, k=k,
+                        source=G.RowsF16) == 0
+            got.append(dst[j:j + m * n].clone())
+            assert (dst[:j] == 7).all() and (dst[j + m * n:] == 7).all()
+    torch.cuda.synchronize()
+    assert G.device_status() == 0
+    assert not torch.equal(got[0], base.view(-1)) and all(torch.equal(got[0], other) for other in got)
+
+
 def test_values_without_a_scale_and_beyond_numbers(cuda, built_libs):
     # all zeros: scale 1.  NaN never wins the maximum and gets the code that the quantiser's clamp makes of it, -448
     import torch
