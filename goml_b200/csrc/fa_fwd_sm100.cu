@@ -27,7 +27,7 @@
 // The tensor core reads shared-memory operands at 128 B/clk/SM, which is what bounds both
 // MMAs here; keeping P out of shared memory keeps that traffic near the exponential-unit
 // time, which is the next bound (16 ex2 per clock per SM).  A CTA works on one 128-row query tile of one head at a time; 6 warps
-// (4 softmax, 1 MMA issuer, 1 TMA producer), or 8 where one converts V; two CTAs share an SM so one CTA's softmax overlaps the
+// (4 softmax, 1 MMA issuer, 1 TMA producer), or 7 where one converts V; two CTAs share an SM so one CTA's softmax overlaps the
 // other's MMAs.  With more tiles than CTAs fit, a CTA that is about to finish takes over the tile of one that has not been
 // launched yet (cluster launch control), so the order and the balance are the hardware's.  Every mbarrier wait is bounded.
 #include <cuda_fp16.h>
@@ -62,8 +62,6 @@ constexpr long long GROUP_ELEMS = 1ll << 24;   // S * D of a larger group: as mu
 constexpr int MMA_WARP = NUM_SOFTMAX_WARPS;
 constexpr int TMA_WARP = NUM_SOFTMAX_WARPS + 1;
 constexpr int CONVERT_WARP = NUM_SOFTMAX_WARPS + 2;   // where V has a warp of its own (Cfg::CONVERTER)
-// registers of a thread there: at launch (8 warps, two CTAs an SM), then of a softmax thread; the other half of the CTA gives them up
-constexpr int LAUNCH_REGS = 128, SOFTMAX_REGS = 160, OTHER_REGS = 2 * LAUNCH_REGS - SOFTMAX_REGS;
 constexpr uint32_t IDESC_NEGATE_A = 1u << 13;   // of the instruction descriptor
 constexpr float TAU = 6.0f;   // lazy-rescale threshold (log2 units)
 constexpr float POFF = 2.0f;  // P is carried as P * 2^POFF (max 2^(TAU+POFF) = 256, far inside fp16)
@@ -89,12 +87,18 @@ struct Cfg {
     static constexpr int V_BYTES = BN * HD * 2;       // fp16
     static constexpr int V_HALF_BYTES = BN * 128;     // one 64-wide (128-byte) slab of d
     // A warp of its own converts V, else the producer does.  For D = 128 a block costs a warp 900 of the 1500 clk it may take, and a
-    // producer that also loads and walks falls behind at every tile's start (256 heads of 2048, causal: 310 us, with the warp 284);
-    // for D = 64 it costs 500, and the eighth warp more than it brings (64 of 3000, window 512: 57 us, with the warp 60).
+    // producer that also loads and walks falls behind at every tile's start (256 heads of 2048, causal: 291 us, with the warp 264); for
+    // D = 64 it costs 500, and the warp more than it brings (64 of 3000, window 512: 57 us, with the warp 60).
     static constexpr bool CONVERTER = VRAW && HD == 128;
     static constexpr int RAW_STAGES = !VRAW ? 0 : HD == 128 ? 2 : 3;
     static constexpr int STAGE_BYTES = 2048;          // of a softmax warp, for its rows on their way out
-    static constexpr int NUM_THREADS = (CONVERTER ? 8 : NUM_SOFTMAX_WARPS + 2) * 32;
+    static constexpr int NUM_THREADS = (NUM_SOFTMAX_WARPS + 2 + CONVERTER) * 32;
+    // Registers are those of eight warps, two CTAs to an SM: of fourteen warps one of its four schedulers has four, which leaves a thread
+    // 128.  Of the masked forms 72 to 80 bytes spill.  With 32 registers of every other thread moved to the softmax threads (setmaxnreg) none
+    // did, and 256 heads of 2048, causal, took 247 us (now 264), 1024 of 512 104 (119), 64 of 8192, window 1024, 262 (281), 256 of 1000, not
+    // causal, 119 (131), 40 of 2048 45.4 (46.7).  But beside that split a small change of code, the rescale of O as a loop, raised
+    // illegal accesses whose cause was not found, so registers stay where a launch puts them.
+    static constexpr int BOUND_THREADS = CONVERTER ? 256 : NUM_THREADS;
     static constexpr int OFF_Q = 0;
     static constexpr int OFF_K = OFF_Q + Q_BYTES;
     static constexpr int OFF_V = OFF_K + STAGES * K_BYTES;
@@ -376,7 +380,7 @@ __device__ __forceinline__ Tile tile_record(uint32_t at) {
 // producer asks for a tile with the last block of the one before on its way, loads Q once the last Q K^T has read the old one, and the rings
 // and the two S buffers just go on.
 template <int HD, bool MASKED, bool VRAW, bool AMAX, bool WALK>
-__global__ void __launch_bounds__(Cfg<HD, VRAW>::NUM_THREADS, 2)
+__global__ void __launch_bounds__(Cfg<HD, VRAW>::BOUND_THREADS, 2)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
               const __grid_constant__ CUtensorMap tmap_v, const Params p) {
     using C = Cfg<HD, VRAW>;
@@ -434,9 +438,6 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     if (bad_start) {
         // fall through to teardown
     } else if (warp >= NUM_SOFTMAX_WARPS) {
-        // One instruction for the whole warpgroup, the idle warp included, which must not part before it.  (In front of the branch between
-        // the two halves of the CTA the compiler would give both what the smaller share allows.)
-        if constexpr (C::CONVERTER) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(OTHER_REGS));
         if (warp == TMA_WARP) {
             // ------------------------------------------------------------- TMA producer
             // The whole warp runs the loop and one elected lane issues: addresses and coordinates stay warp-uniform.
@@ -700,7 +701,6 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
             }
         }
     } else {
-        if constexpr (C::CONVERTER) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SOFTMAX_REGS));
         // ------------------------------------------- softmax / correction / epilogue
         const int r = threadIdx.x;               // row of the tile = TMEM lane (one thread per row)
         const uint32_t lane_off = uint32_t(warp * 32) << 16;
@@ -726,7 +726,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         Tile t(p, blockIdx.x);
 
         // The scores of key block j of the tile, in the S buffer at sa, and what they do to the reference.  EDGE: the block may hold
-        // masked keys.  (The loop over O in the rare branch stays unrolled: as a loop it made the form with a converting warp fault.)
+        // masked keys.
         uint32_t sreg[BN];
         bool hidden[BN / 32];                    // no row of this warp sees these 32 keys: their P is zero
         auto scores = [&](const int j, const uint32_t sa, auto edge) -> bool {
@@ -1130,18 +1130,6 @@ void init_device(DeviceState* st, int dev) {
     set_all(std::false_type(), std::true_type());
     set_all(std::true_type(), std::false_type());
     set_all(std::true_type(), std::true_type());
-    // the registers that the softmax warps of these take are those that the others were launched with and give up
-    auto check = [&](auto kernel) {
-        cudaFuncAttributes f;
-        if (e == cudaSuccess) e = cudaFuncGetAttributes(&f, kernel);
-        if (e == cudaSuccess && f.numRegs != LAUNCH_REGS) e = cudaErrorInvalidKernelImage;
-    };
-    check(fa_fwd_kernel<128, true, true, false, false>);
-    check(fa_fwd_kernel<128, true, true, false, true>);
-    check(fa_fwd_kernel<128, false, true, false, false>);
-    check(fa_fwd_kernel<128, false, true, false, true>);
-    check(fa_fwd_kernel<128, true, true, true, false>);
-    check(fa_fwd_kernel<128, true, true, true, true>);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&st->num_sms, cudaDevAttrMultiProcessorCount, dev);
     st->init_error = e;
 }

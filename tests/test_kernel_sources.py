@@ -104,3 +104,10 @@ def test_a_part_of_the_decode_line_comes_from_one_reading_of_the_lengths():
     # that a unit falls in, its length and the units before it are taken from the same values
     body = re.search(r"auto segment_at = .*?\n    \};", sources()["fa_decode_sm100.cu"], flags=re.S).group(0)
     assert body.count("lane_len(") == 1 and "seq_len_of" not in body and "len_of(" not in body.replace("lane_len(", "")
+
+
+@pytest.mark.parametrize("name", sources())
+def test_registers_stay_where_a_launch_puts_them(name):
+    # an attention form that moved registers between its warps raised illegal accesses after a harmless change of its code, and the
+    # cause was not found
+    assert "setmaxnreg" not in sources()[name]
