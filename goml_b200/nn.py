@@ -55,16 +55,15 @@ class FP8Linear:
         self.w = quantize(weight.float())
 
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
-        M, K, N = x.numel() // self.in_features, self.in_features, self.out_features
-        if x.dtype is not torch.float32 or not x.is_cuda or x.numel() != M * K or not x.is_contiguous():
+        M, K = x.numel() // self.in_features, self.in_features
+        if (x.dtype is not torch.float32 or not x.is_cuda or x.numel() != M * K or not x.is_contiguous()
+                or type(self).forward_codes is not FP8Linear.forward_codes or "forward_codes" in vars(self)):   # a layer with a product of its own has it called
             return self.forward_codes(quantize(x.reshape(M, K).float()), M)
         # codes, scale and amax in one allocation and no views: for a few rows a call is its host time (28.7 us with a tensor for each)
         buf, codes, sa = _scratch(x.device, M * K, 8)
-        y = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
         stream = torch.cuda.current_stream().cuda_stream
         Q.QuantizeF32ToF8E4M3(x.data_ptr(), codes, sa, sa + 4, M * K, stream)
-        G.FP8GEMMScaled(M, N, K, codes, self.w.codes.data_ptr(), y.data_ptr(), 1.0, sa, self.w.scale_ptr, G.OutBF16, stream)
-        return y
+        return self._product(codes, sa, M, x.device, stream)
 
     def accumulate_into(self, xq: FP8Tensor, M: int, x: torch.Tensor) -> None:
         """x (fp32 [M, out]) += this layer's output, added in the GEMM epilogue (no 16-bit intermediate)."""
@@ -74,9 +73,12 @@ class FP8Linear:
 
     def forward_codes(self, xq: FP8Tensor, M: int) -> torch.Tensor:
         """The GEMM alone, on an activation that is already e4m3 codes + device scale."""
-        y = torch.empty((M, self.out_features), dtype=torch.bfloat16, device=xq.codes.device)
-        G.FP8GEMMScaled(M, self.out_features, self.in_features, xq.codes.data_ptr(), self.w.codes.data_ptr(), y.data_ptr(),
-                        1.0, xq.scale_ptr, self.w.scale_ptr, G.OutBF16, torch.cuda.current_stream().cuda_stream)
+        return self._product(xq.codes.data_ptr(), xq.scale_ptr, M, xq.codes.device, torch.cuda.current_stream().cuda_stream)
+
+    def _product(self, codes: int, scale: int, M: int, device: torch.device, stream: int) -> torch.Tensor:
+        y = torch.empty((M, self.out_features), dtype=torch.bfloat16, device=device)
+        G.FP8GEMMScaled(M, self.out_features, self.in_features, codes, self.w.codes.data_ptr(), y.data_ptr(),
+                        1.0, scale, self.w.scale_ptr, G.OutBF16, stream)
         return y
 
 

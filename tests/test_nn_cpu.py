@@ -111,6 +111,36 @@ def test_a_cache_with_a_fill_of_its_own_has_it_called():
         assert not nn._writes_directly(c, B, H, 8, HD, CPU)
 
 
+def test_a_layer_with_a_product_of_its_own_has_it_called(monkeypatch):
+    # for every kind of tensor, the one that goes straight to the libraries too
+    from goml_b200 import fp8_gemm as G, quantize as Q
+    calls = []
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: type("Stream", (), {"cuda_stream": 7}))
+    monkeypatch.setattr(Q, "QuantizeF32ToF8E4M3", lambda src, dst, scale, amax, n, stream: calls.append(("quantise", n, stream)))
+    monkeypatch.setattr(G, "FP8GEMMScaled", lambda m, n, k, *args: calls.append(("product", m, n, k)))
+
+    class OnGPU(torch.Tensor):
+        is_cuda = property(lambda self: True)
+
+    class Other(nn.FP8Linear):
+        def forward_codes(self, xq, M):
+            assert isinstance(xq, nn.FP8Tensor) and xq.codes.shape == (M, 32)
+            return "its own"
+
+    def layer(cls):
+        made = cls.__new__(cls)
+        made.out_features, made.in_features, made.w = 5, 32, nn.FP8Tensor(u8(5, 32), torch.ones(2))
+        return made
+
+    x = torch.ones(3, 2, 32).as_subclass(OnGPU)
+    for same in (x, x.bfloat16(), torch.ones(3, 2, 64).as_subclass(OnGPU)[..., ::2]):
+        assert layer(nn.FP8Linear)(same).shape == (6, 5) and calls == [("quantise", 6 * 32, 7), ("product", 6, 5, 32)]
+        patched = layer(nn.FP8Linear)
+        patched.forward_codes = lambda xq, M: ("patched", M)
+        assert layer(Other)(same) == "its own" and patched(same) == ("patched", 6)
+        calls.clear()
+
+
 # the calls of a block in their order, and what their bindings raise
 CALLS = ["fp8_rmsnorm_quantize_into", "fp8_gemm_scaled", None, None, "fp8_permute_quantize_heads", "fp8_gemm_accumulate_f32", "fp8_rmsnorm_quantize_into",
          "fp8_gemm_swiglu_raise", "fp8_quantize_bf16", "fp8_gemm_accumulate_f32"]
