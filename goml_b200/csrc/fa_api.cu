@@ -461,6 +461,7 @@ fa_status_t fa_decode(fa_ctx_t* ctx, const fa_decode_args_t* g) {
     if (e != cudaSuccess) { set_err(ctx, "%s: workspace allocation: %s", who, cudaGetErrorString(e)); return e == cudaErrorMemoryAllocation ? FA_ERR_OOM : FA_ERR_CUDA; }
     a.workspace = ws.ptr;
     a.arrivals = ws.zeros;
+    a.behind_clear = ws.pooled[1] != nullptr;
     e = fa_sm100::launch_decode(a);
     const cudaError_t fe = ws.give_back();  // stream-ordered: released after the kernels
     if (e != cudaSuccess) { set_err(ctx, "%s: launch: %s", who, cudaGetErrorString(e)); return FA_ERR_CUDA; }

@@ -113,6 +113,7 @@ struct DecodeParams {
     const float* sk;
     const float* sv;
     int plan, splits, chunks_per_split;
+    bool hints;   // on the line: ask for the first chunks ahead of the wait
     // paged cache: k, v are [num_pages, Hkv, page_size, D]; the chunk at key k0 of sequence b lives in page
     // block_table[b * max_pages + k0 / page_size]
     const int* block_table;
@@ -252,22 +253,20 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
         return (((long long)page * p.hkv + x.kvh) * p.page_size + (key - page_of(key) * p.page_size)) * D;
     };
 
-    // On the line the first trip is made while the kernel ahead still runs (the append of the new token, usually), which leaves memory idle: this
-    // CTA's first chunks are asked for from L2, by the lengths and the table as they then are.  Those may still be the last step's,
-    // or anything: they are bounded like the ones read behind the wait, and nothing but hints comes of them.  Two chunks for each of 444 CTAs are 14 MB: append and
-    // attention of 24 sequences of 3000 to 6000 keys, 8 kv heads, paged, 49.9 -> 48.8 us (four 49.1, eight 49.8).  A CTA per pair or
-    // split gains nothing (a step of 64 sequences 336 / 341 us, of one 78.1 / 77.7) and makes one trip.
+    // On the line the piece is found twice, the first time while the kernel ahead still runs (the append of the new token, usually), which leaves memory
+    // idle: this CTA's first chunks are asked for from L2, by the lengths and the table as they then are.  Those may still be the last
+    // step's, or anything: they are bounded like the ones read behind the wait, and nothing but hints comes of them.  Two chunks for each of
+    // 444 CTAs are 14 MB.  Append and attention, 8 kv heads, paged, without / with: 24 sequences of 3000 to 6000 keys 48.7 / 47.3 us, 12 of
+    // 1500 to 3000 24.1 / 23.0, one of 8000 18.0 / 17.3, one of 500 9.4 / 9.5; with the lengths and pages of other sequences in place until
+    // the append, the same 48.3 / 47.1, 27.4 / 26.7, 21.8 / 21.5, 14.4 / 14.4.  Not behind a kernel that clears the counters (captured calls):
+    // that one starts when the append has ended, and the hints cost a call 0.9 us.  (As two trips of one loop the search cost pieces of one to two
+    // chunks: one sequence of 4000 18.3, now 16.5, 16.6 without.)  A CTA per pair or split gains nothing (a step of 64 sequences 336 / 341, of one
+    // 78.1 / 77.7) and is found once.
     Segment seg;
     int cut_q = 0, cut_r = 0;
     int mid = 0, mid_end = 0;    // units of the segments still to come in line order
     const bool line = !STREAMS && p.plan == LINE;   // streams are not cut along a line: that code is not compiled for them
-#pragma unroll 1
-    for (int trip = line ? 0 : 1; trip < 2; trip++) {
-        const bool early = !STREAMS && trip == 0;
-        if (!early) {
-            pdl_wait();
-            pdl_trigger();
-        }
+    auto find_piece = [&](const bool early) {
         seg.b = seg.kvh = seg.len = seg.n_chunks = seg.c_begin = seg.c_end = seg.pair_u0 = 0;
         if (!line) {
             const int pair = blockIdx.x / p.splits, split = blockIdx.x - pair * p.splits;
@@ -277,7 +276,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
             seg.n_chunks = chunks_of(seg.len);
             seg.c_begin = split * p.chunks_per_split;
             seg.c_end = min(seg.n_chunks, seg.c_begin + p.chunks_per_split);
-            if (!early && seg.n_chunks == 0 && seg.kvh == 0 && split == 0 && threadIdx.x == 0) empty_sequence(seg.b);
+            if (seg.n_chunks == 0 && seg.kvh == 0 && split == 0 && threadIdx.x == 0) empty_sequence(seg.b);
         } else {
 #pragma unroll
             for (int i = 0; i < LENS; i++) lens[i] = 32 * i + lane < p.batch ? seq_len_of(p, 32 * i + lane) : 0;
@@ -297,15 +296,19 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
             if (mid < mid_end) seg = segment_at(mid, mid_end);
             mid += seg.c_end - seg.c_begin;
         }
-        if (early) {
-            const int c = seg.c_begin + lane;
-            if (warp < 2 && lane < HINTS && c < seg.c_end) {
-                const long long off = offset(seg, c, PAGED ? peek_s32(p.block_table + (size_t)seg.b * p.max_pages + page_of(c * CHUNK)) : 0);
-                if (off >= 0) prefetch_l2((warp == 0 ? p.k : p.v) + off, (PAGED ? CHUNK : min(CHUNK, p.s_max - c * CHUNK)) * D);
-            }
-            __syncwarp();
+    };
+    if (line && p.hints) {
+        find_piece(true);
+        const int c = seg.c_begin + lane;
+        if (warp < 2 && lane < HINTS && c < seg.c_end) {
+            const long long off = offset(seg, c, PAGED ? peek_s32(p.block_table + (size_t)seg.b * p.max_pages + page_of(c * CHUNK)) : 0);
+            if (off >= 0) prefetch_l2((warp == 0 ? p.k : p.v) + off, (PAGED ? CHUNK : min(CHUNK, p.s_max - c * CHUNK)) * D);
         }
+        __syncwarp();
     }
+    pdl_wait();
+    pdl_trigger();
+    find_piece(false);
     if (seg.c_begin >= seg.c_end) return;
     float scale_log2 = p.scale_log2;
     if (p.sq) scale_log2 *= ld_f32(p.sq);
@@ -755,7 +758,7 @@ cudaError_t launch_decode(const DecodeArgs& a) {
     p.scale_log2 = a.scale * 1.4426950408889634f;
     p.v_descale = a.v_descale;
     p.sq = a.scale_q_dev; p.sk = a.scale_k_dev; p.sv = a.scale_v_dev;
-    p.plan = x.plan; p.splits = x.splits;
+    p.plan = x.plan; p.splits = x.splits; p.hints = !a.behind_clear;
     p.chunks_per_split = (int)((((long long)span + CHUNK - 1) / CHUNK + x.splits - 1) / x.splits);
     p.block_table = a.block_table;
     p.page_mul = p.page_shr = 0;

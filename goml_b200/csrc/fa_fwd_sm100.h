@@ -53,6 +53,7 @@ struct DecodeArgs {
     const float* scale_v_dev = nullptr;
     void* workspace = nullptr;      // decode_workspace_bytes(...) bytes, 16-byte aligned
     uint32_t* arrivals = nullptr;   // decode_arrival_count(...) words that are zero; the launch leaves them zero
+    bool behind_clear = false;      // a kernel that clears them is the one ahead on the stream
     cudaStream_t stream;
     // paged cache (block_table != nullptr): k_cache, v_cache are [num_pages, kv_heads, page_size, hd], page_size a
     // multiple of 64; block_table [batch, max_pages] holds the page of each page_size-key range of a sequence and
