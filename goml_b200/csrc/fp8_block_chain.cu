@@ -4,7 +4,7 @@
 // it 7 us apiece (argument conversion, checks, the launch), more than the GPU needs; here they cost the launch.  The maxima of
 // all quantisers of the block are cleared once, by its first kernel, where every larger op had a clearing kernel in front.
 //
-// A step of one or two sequences has its quantisers inside the products that read their codes (fp8_gemm_rows): six kernels in the
+// A step of one or two sequences has its quantisers inside the products that read their codes (fp8_gemm_rows): six calls in the
 // place of ten.  Each of the four that this saved took 2 to 5 us with its hand-over, and the product behind it began to stream its
 // weight only then.
 #include "../../include/fp8_gemm.h"   // the argument block of fp8_gemm_rows; nothing of that library is linked

@@ -88,7 +88,7 @@ FP8GEMM_API int fp8_gemm_swiglu_raise(int M, int F, int K, const void* A, const 
 
 /* Additive: the product for one or two rows of A that are given as the values their codes are made of: every thread block
  * quantises them for itself, while the weight's first tiles are on their way, instead of a quantiser ahead of the product (a step
- * of one sequence: ten kernels, six this way).  One per-tensor scale, max|value| / 448, like the quantisers of this directory; the
+ * of one sequence: ten calls, six this way).  One per-tensor scale, max|value| / 448, like the quantisers of this directory; the
  * values, rows [M, K] without gaps, are
  *   FP8_ROWS_RMSNORM_F32  the RMSNorm of fp32 rows: (x * gamma) * (1 / sqrt(mean(x^2) + eps)), gamma [K] fp32;
  *   FP8_ROWS_F16          fp16 as they are;

@@ -3,7 +3,7 @@ import ctypes as C
 
 import pytest
 
-INVALID = 1   # cudaErrorInvalidValue
+INVALID, NOT_SUPPORTED = 1, 801   # cudaErrorInvalidValue, cudaErrorNotSupported
 GEMM = C.CFUNCTYPE(C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_float, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p)
 ADD = C.CFUNCTYPE(C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_float, C.c_void_p, C.c_void_p, C.c_void_p)
 SWIGLU = C.CFUNCTYPE(C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_float, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p)
@@ -20,6 +20,16 @@ def lib(built_libs):
     lib.fp8_block_region_bytes.restype, lib.fp8_block_region_bytes.argtypes = C.c_size_t, [C.c_int] * 3
     lib.fp8_block_run.restype, lib.fp8_block_run.argtypes = C.c_int, [C.POINTER(BG.BlockRunArgs)]
     return lib
+
+
+def run_rows(lib, args, rows):
+    """fp8_block_run_rows with rows(argument block) in fp8_gemm_rows' place (the same function object has other types elsewhere)."""
+    from goml_b200 import fp8_gemm as G
+    kind = C.CFUNCTYPE(C.c_int, C.POINTER(G.RowsArgs))
+    keep = kind(lambda block: rows(block.contents))
+    fn = lib["fp8_block_run_rows"]
+    fn.restype, fn.argtypes = C.c_int, [C.c_void_p, C.c_void_p]
+    return fn(C.addressof(args), C.cast(keep, C.c_void_p))
 
 
 def block(lib, decode, pointer, entry=lambda name, *args: 0, **changed):
@@ -110,3 +120,67 @@ def test_place_and_code_of_a_failed_call(cuda, lib, decode):
     if decode:   # an odd number of values to quantise
         shapes[8], shapes[10] = (T, 20, d), (T, d, 20)
         assert run(ffn_hidden=20) == (9 << 16 | INVALID, [2, 4, 6, 8])
+
+
+def test_a_step_whose_first_product_takes_rows(lib):
+    # it is the first call, and its failure the end; a prompt has no such products; the arguments are refused as without them
+    seen = []
+    refuse = lambda g: seen.append(g.source) or 7
+    assert run_rows(lib, block(lib, True, lambda name, n: 0x10000, norm1=0x10001), refuse) == 11 << 16 | 7 and seen == [1]
+    assert run_rows(lib, block(lib, False, lambda name, n: 0x10000, norm1=0x10001), refuse) == 1 << 16 | INVALID and seen == [1]
+    assert run_rows(lib, block(lib, True, lambda name, n: 0x10000, norm1=0x10001), lambda g: NOT_SUPPORTED) == 1 << 16 | INVALID
+    for changed in (dict(seq_len=2), dict(k_cache=None), dict(x=None), dict(region_bytes=0)):
+        assert run_rows(lib, block(lib, True, lambda name, n: 0x10000, **changed), refuse) == INVALID and seen == [1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("refused", [(), (11,), (12,), (13,), (14,), (11, 12), (11, 13), (12, 14), (11, 12, 13, 14)], ids=lambda r: "-".join(map(str, r)) or "none")
+def test_products_that_take_rows_and_those_that_do_not(cuda, lib, refused):
+    # each product by itself goes the one way or the other: which calls are made in which order, what they are given, and that the
+    # stream is in h where the product behind adds to it in place
+    import torch
+    d, real, g = H * HD, {}, torch.Generator(device="cuda").manual_seed(1)
+
+    def pointer(name, n):
+        real[name] = torch.zeros(n, dtype=torch.uint8, device="cuda")
+        return real[name].data_ptr()
+
+    def run(fails=0):
+        seen, blocks = [], {}
+
+        def entry(name, *args):
+            seen.append({"gemm_scaled": 2, "attention_decode": 4, "gemm_swiglu_raise": 8}.get(name) or (6 if args[2] == d else 10))
+            return 0
+
+        def rows(g):
+            place = 11 + len(blocks)
+            blocks[place] = {name: getattr(g, name) for name, _ in g._fields_}
+            if place in refused and place != fails:
+                return NOT_SUPPORTED
+            seen.append(place)
+            return 7 if place == fails else 0
+
+        args = block(lib, True, pointer, entry)
+        real["x"].copy_(torch.randn(B * d, generator=g, device="cuda").view(torch.uint8))
+        rc = run_rows(lib, args, rows)
+        torch.cuda.synchronize()
+        return rc, seen, blocks, args
+
+    order = [2 if 11 in refused else 11, 4, 6 if 12 in refused else 12, 8 if 13 in refused else 13, 10 if 14 in refused else 14]
+    rc, seen, got, a = run()
+    assert rc == 0 and seen == order
+    in_place = 11 in refused or 12 in refused   # the norm or a copy brings x to h; else the second product reads x itself
+    assert torch.equal(real["h"], real["x"] if in_place else torch.zeros_like(real["h"]))
+    hidden = a.words + 4 * 6   # the maximum of the hidden activations, the last of the seven words that the first kernel clears
+    none = dict(gamma=None, amax=None, c=None, x=None, x_in=None, h=None, h_amax=None, zero=None, zeros=0, b_complete=1, reserved=0)
+    common = lambda w, **more: {**none, "b": getattr(a, w), "scale_b": getattr(a, w + "_scale"), "m": B, "stream": a.stream, "eps": pytest.approx(1e-5), **more}
+    assert got[11] == common("wqkv", source=1, rows=a.x, gamma=a.norm1, c=got[11]["c"], n=3 * d, k=d, zero=a.words, zeros=7, b_complete=0)
+    assert got[12] == common("wo", source=2, rows=got[12]["rows"], x=a.h, x_in=a.h if 11 in refused else a.x, n=d, k=d)
+    assert got[13] == common("wgate_up", source=1, rows=a.h, gamma=a.norm2, h=got[13]["h"], h_amax=hidden, n=F, k=d)
+    assert got[14] == common("wdown", source=3, rows=got[13]["h"], amax=hidden, x=a.h, x_in=a.h, n=d, k=F)
+    inside = lambda p: a.region <= p < a.region + a.region_bytes and p % 16 == 0
+    assert inside(got[11]["c"]) and inside(got[12]["rows"]) and inside(got[13]["h"])
+    assert real["cache_lens"].view(torch.int32).tolist() == [1] * B
+    for place in (11, 12, 13, 14):
+        if place not in refused:
+            assert run(place)[:2] == (place << 16 | 7, order[:order.index(place) + 1])

@@ -13,9 +13,10 @@ def call(lib, **fields):
     return lib.fp8_gemm_rows(C.byref(G.RowsArgs(stream=torch.cuda.current_stream().cuda_stream, **fields)))
 
 
-# few and many tiles, slices of one to four, two and three CTAs to an SM; K ragged in 128 and 64; N ragged in 128 and 4
+# the blocks' products, with n as the width of the SwiGLU too; few and many tiles, slices of one to four, two and three CTAs to an SM; K ragged in 128 and 64; N ragged in 128 and 4
 @pytest.mark.parametrize("m,n,k", [(1, 12288, 4096), (2, 4096, 4096), (2, 22016, 4096), (2, 4096, 11008), (1, 2048, 5504), (2, 1001, 2000), (1, 128, 16), (1, 6144, 2048),
-                                   (2, 8192, 8192), (2, 11264, 2048), (1, 130, 272)])
+                                   (2, 8192, 8192), (2, 11264, 2048), (1, 130, 272), (1, 11008, 4096),
+                                   (2, 11008, 4096), (2, 5504, 2048), (1, 5632, 2048)])
 @pytest.mark.parametrize("source", [1, 2, 3])
 def test_rows_against_quantiser_and_product(cuda, built_libs, m, n, k, source):
     import torch
@@ -66,7 +67,7 @@ def test_rows_against_quantiser_and_product(cuda, built_libs, m, n, k, source):
     wh, h, top = torch.empty(m, n, dtype=torch.bfloat16, device="cuda"), torch.empty(m, n, dtype=torch.bfloat16, device="cuda"), torch.zeros(2, device="cuda")
     G.FP8GEMMSwiGLU(m, n, k, codes.data_ptr(), w.data_ptr(), wh.data_ptr(), 1.0, p, ws.data_ptr(), top.data_ptr(), st)
     rc = call(lib, h=h.data_ptr(), h_amax=top.data_ptr() + 4, n=n, b_complete=1, **more)
-    assert rc in (0, NOT_SUPPORTED)
+    assert rc == (NOT_SUPPORTED if (n, k) == (22016, 4096) else 0)   # 344 tiles of weight rows: more than two to an SM
     if rc == 0:
         close(h, wh, 4e-3 if source == 1 else 1e-3)
         assert top[1].item() == h.float().abs().max().item()

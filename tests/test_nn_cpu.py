@@ -159,12 +159,16 @@ def test_a_failed_call_is_named(monkeypatch, kind):
     blk.rope_tables = lambda S, dev: (torch.ones(S, HD // 2), torch.ones(S, HD // 2))
     blk.fa = type("Context", (), {"ptr": 1, "_msg": lambda self: "why"})()
     monkeypatch.setattr(torch.cuda, "current_stream", lambda: type("Stream", (), {"cuda_stream": 0}))
-    monkeypatch.setattr(nn, "_entry_points", lambda: (1,) * 5)
+    monkeypatch.setattr(nn, "_entry_points", lambda: (1, 2, 3, 4, 5, 6))
     monkeypatch.setattr(F, "FAStatusString", lambda status: f"status {status}")
     run = {"step": lambda: blk.decode_step(torch.zeros(B, H * HD), cache()), "prompt": lambda: blk.forward_fused(torch.zeros(B * 8, H * HD), B, 8),
            "prompt into a cache": lambda: blk.forward_fused(torch.zeros(B * 8, H * HD), B, 8, cache())}[kind]
-    for place, name in enumerate(["fp8_block_run", *calls]):
-        monkeypatch.setattr(BG, "BlockRun", lambda *args: place << 16 | 5)
+    for place, name in enumerate(["fp8_block_run", *calls, *["fp8_gemm_rows"] * 4 * (kind == "step")]):
+        def failing(*args):   # the entry points of the fields in front, that of the products of rows behind them
+            assert args[:5] == (1, 2, 3, 4, 5) and args[-1] == 6 and len(args) == len(BG.BlockRunArgs._fields_) + 1
+            return place << 16 | 5
+
+        monkeypatch.setattr(BG, "BlockRun", failing)
         error = F.FAError if name.startswith("fa") else G.FP8GEMMError if name.startswith("fp8_gemm") else BG.BlockGlueError
         with pytest.raises(error) as e:
             run()

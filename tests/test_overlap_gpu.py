@@ -124,3 +124,36 @@ def test_quantise_then_square_gemm(cuda, built_libs, M, K, F, N, variant):
     # the last step against its own codes: bf16 rounding of the result, and of the sums' last bits
     want = hc.view(torch.float8_e4m3fn).double() @ w2.view(torch.float8_e4m3fn).double().t() * w[3].double() * 2.0 ** -7
     assert ((got[-1].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * want.abs().max()).all()
+
+
+@pytest.mark.parametrize("B,d,H,Fh", [(1, 512, 4, 1376), (2, 512, 8, 1376), (1, 2048, 16, 5504)])
+def test_steps_behind_rewritten_weights(cuda, built_libs, B, d, H, Fh):
+    # the products of a step of one or two sequences load their weights ahead of the wait, all but the first one's: every step's weights
+    # and scales are written by the kernels right ahead of it, those of its last product last
+    from goml_b200 import fp8_gemm as G, nn
+    g = torch.Generator(device="cuda").manual_seed(d + B)
+    rn = lambda *shape: torch.randn(*shape, generator=g, device="cuda") * 0.02
+    blk = nn.FP8DecoderBlock(d, H, Fh, rn(3 * d, d), rn(d, d), rn(2 * Fh, d), rn(d, Fh), 1 + rn(d), 1 + rn(d))
+    held = lambda b: [b.qkv.w.codes, b.o.w.codes, b.gate_up_interleaved, b.qkv.w.sa, b.o.w.sa, b.gate_up.w.sa, b.down.w.sa, b.down.w.codes]
+    sets = []
+    for i in range(3):
+        other = nn.FP8DecoderBlock(d, H, Fh, *(rn(*shape) * (0.5 + i) for shape in ((3 * d, d), (d, d), (2 * Fh, d), (d, Fh))), 1 + rn(d), 1 + rn(d))
+        sets.append([w.clone() for w in held(other)])
+        other.close()
+    xs = torch.randn(STEPS, B, d, generator=g, device="cuda")
+    cache = nn.FP8KVCache(B, H, STEPS + 8, d // H)
+    cache.scales.fill_(0.02)
+    out = torch.empty(STEPS, B, d, device="cuda")
+
+    def step(i):
+        if i == 0:
+            for buf in (cache.k, cache.v, cache.lens):
+                buf.zero_()
+        for w, new in zip(held(blk), sets[i % 3]):
+            w.copy_(new)
+        out[i].copy_(blk.decode_step(xs[i], cache))
+
+    got = twice(step, out)
+    assert got.isfinite().all() and cache.lens.tolist() == [STEPS] * B and G.device_status() == 0
+    assert sum("fp8_gemm_skinny_kernel" in n and "ELb1E" in n for n in kernels(lambda: blk.decode_step(xs[0], cache))) == 4
+    blk.close()
