@@ -133,6 +133,16 @@ def test_a_step_whose_first_product_takes_rows(lib):
         assert run_rows(lib, block(lib, True, lambda name, n: 0x10000, **changed), refuse) == INVALID and seen == [1]
 
 
+@pytest.mark.parametrize("batch,heads,taken", [(1, 64, True), (2, 64, True), (4, 32, True), (1, 65, True), (2, 65, False), (3, 64, False), (64, 2, True), (65, 2, False),
+                                               (1, 128, True), (1, 130, False)])
+def test_long_rows_have_a_quantiser_ahead(lib, batch, heads, taken):
+    # past 8192 values the maximum that every thread block takes for itself costs more than a kernel that takes it once
+    d, seen = heads * HD, []
+    args = block(lib, True, lambda name, n: 0x10000, norm1=0x10001, batch=batch, heads=heads, d_model=d, region_bytes=lib.fp8_block_region_bytes(batch, d, F))
+    assert run_rows(lib, args, lambda g: seen.append((g.m, g.k)) or 7) == (11 << 16 | 7 if taken else 1 << 16 | INVALID)
+    assert seen == ([(batch, d)] if taken else []) and taken == (batch * d <= 8192)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("refused", [(), (11,), (12,), (13,), (14,), (11, 12), (11, 13), (12, 14), (11, 12, 13, 14)], ids=lambda r: "-".join(map(str, r)) or "none")
 def test_products_that_take_rows_and_those_that_do_not(cuda, lib, refused):
