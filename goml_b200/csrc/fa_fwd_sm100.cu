@@ -1032,16 +1032,16 @@ bool converts_v(const LaunchArgs& a, int num_sms) {
     return (a.causal && span == a.sl ? (long long)a.sl * 3 / 5 : span) <= limit;
 }
 
-// Heads whose tiles are interleaved, the longest of all of them first, where tiles differ in length.  With 17 to 24 heads in groups of 16
-// the long tiles of the last few heads ended the launch, and converting V made them longer.  So it is one group, or
-// equal ones, of as many heads as 48 MB of K and V allow; but up to three tiles per SM two or more full groups of 16 stay (32 heads
-// of 1300 23.0 us / 24.4 in one, 32 of 1600 30.2 / 30.9).  D = 128, causal, one call behind another, before V was converted in here /
-// since, in groups of 16 / now: 17 heads of 2560 47.9 / 54.5 / 36.2, 20 of 2200 44.3 / 48.6 / 33.3, 24 of 2048 37.3 / 39.1 / 32.9, 32 of 2048
-// 43.3 / 44.2 / 41.0, 40 of 2048 61.9 / 56.5 / 45.7, 256 of 2048 298 / 272 / 267; a window of 300, 128 of 2500 134.7 / 106.0 / 107.2.
+// Heads whose tiles are interleaved, the longest of all of them first, where tiles differ in length.  In groups of 16 the long tiles of
+// the last few heads end the launch, so it is one group, or equal ones, of as many heads as 48 MB of K and V allow.  Full groups stay
+// where there is little to balance, up to 1.6 tiles per SM.  Causal, one call behind another, in groups of 16 / in as few as that, us: D = 128, 17
+// heads of 2560 47.3 / 36.3, 24 of 2048 34.6 / 31.1, 40 of 2048 55.3 / 46.5, 256 of 2048 268 / 266, 32 of 1300 25.1 / 22.3, 48 of 1100 27.4 /
+// 23.8, 48 of 600 15.1 / 13.9, but 32 of 850 15.9 / 16.8, 48 of 500 11.3 / 12.2, 32 of 600 11.6 / 12.1; D = 64, 18 of 3000 58.2 / 37.1, 64 of 700 16.4 /
+// 13.7, 32 of 700 10.6 / 10.5; a window of 300, 128 of 2500 of 128 106.6 / 107.1.
 int heads_together(const LaunchArgs& a, long long tiles, int num_sms) {
     const bool full = a.bh % HEAD_GROUP == 0 || a.bh % HEAD_GROUP >= HEAD_GROUP - 2;
     long long most = GROUP_ELEMS / ((long long)a.sl * a.hd);
-    if (most < HEAD_GROUP || (full && tiles <= 3ll * num_sms)) most = HEAD_GROUP;
+    if (most < HEAD_GROUP || (full && 5 * tiles <= 8ll * num_sms)) most = HEAD_GROUP;
     const long long groups = (a.bh + most - 1) / most;
     return (int)((a.bh + groups - 1) / groups);
 }
