@@ -76,7 +76,7 @@ enum : uint32_t {
 
 __device__ uint32_t g_fa_status = 0;
 
-// Shared memory holds the operand tiles: Q, K and the fp16 V, or (VRAW) the codes of V beside the fp16 tiles that the producer warp
+// Shared memory holds the operand tiles: Q, K and the fp16 V, or (VRAW) the codes of V beside the fp16 tiles that a warp
 // makes of them; two CTAs an SM either way.  Both MMAs are limited by how fast the
 // tensor core can read its shared-memory operands (128 B/clk/SM), so P never goes through
 // shared memory: it is written to tensor memory and read from there as the A operand.
@@ -366,10 +366,10 @@ __device__ __forceinline__ Tile tile_record(uint32_t at) {
     return Tile(r);
 }
 
-// VRAW = true: V arrives as codes, and the producer warp converts each tile in shared memory while it waits for the ring.  That
-// costs a tile 0.04 us per key block (D = 128; the producer shares its scheduler with one softmax warp of the CTA, and
-// shared memory carries 24 KB more per block) and saves the pre-pass: 3 bytes per element of traffic, a launch, the scratch, and
-// the CTAs of the pre-pass, which the attention's first CTAs wait for.  Bit for bit the same results.
+// VRAW = true: V arrives as codes, and a warp converts each tile in shared memory (for D = 64 the producer, while it waits for the ring).
+// It shares its scheduler with one softmax warp of the CTA, and shared memory carries 24 KB more per block of D = 128; that saves the
+// pre-pass: 3 bytes per element of traffic, a launch, the scratch, and the CTAs of the pre-pass, which the attention's first CTAs wait
+// for.  Bit for bit the same results.
 //
 // MASKED = false: no key of the launch is masked (non-causal, no window, S a multiple of the block) and the host-side scale
 // is positive: the masking code is not compiled into the softmax loop, and Q K^T is not asked for with a sign.  (The
@@ -618,10 +618,10 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
             {
                 const bool leader = elect_one();
                 // a negative scale: the scores come out of the tensor core with the sign that their maximum is taken with
-            float sign = p.scale_log2;
-            if (MASKED && p.sq) sign *= ld_f32(p.sq);
-            if (MASKED && p.sk) sign *= ld_f32(p.sk);
-            const uint32_t idesc_qk = make_idesc_e4m3_f32(BM, BN, 0, 0) | (MASKED && sign < 0.f ? IDESC_NEGATE_A : 0u);
+                float sign = p.scale_log2;
+                if (MASKED && p.sq) sign *= ld_f32(p.sq);
+                if (MASKED && p.sk) sign *= ld_f32(p.sk);
+                const uint32_t idesc_qk = make_idesc_e4m3_f32(BM, BN, 0, 0) | (MASKED && sign < 0.f ? IDESC_NEGATE_A : 0u);
                 constexpr uint32_t idesc_pv = make_idesc_f16_f32(BM, HD, 0, 1);  // A = P from TMEM, V is MN-major
                 auto qk_desc = [&](uint32_t addr) { return HD == 128 ? kmajor_desc_sw128(addr) : kmajor_desc_sw64(addr); };
                 // K ring position of the next Q K^T, V ring position of the next P V
@@ -849,7 +849,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         // past the instruction cache it is fetched again and again.  With the clear loop unrolled by two, a sign flip of 64 instructions
         // in the edge loop and the conversion of V unrolled in full, us: 256 heads of 2048 of 128, causal, 298 (now 279), 64 of 8192, window
         // 1024, 327 (287), 64 of 3000 of 64, window 512, 57.1 (52.9), 256 of 1000 of 128, not causal, 139 (131).  One loop with the edge
-        // as a test in it keeps more registers alive: 300, 305, 57.5, 143.
+        // as a test in it keeps more registers alive: 300, 305, 57.5, 143.  (All at the power cap, and those of 128 with registers moved
+        // between the warps.)
         // A CTA with a tile of its own keeps the clear loop unrolled by two: its calls are few and long (1 head of 8192 of 128, causal, 92.8 / 85.7).
         auto edge_blocks = [&](int& j, const int end) -> bool {
 #pragma unroll 1
@@ -1016,14 +1017,15 @@ void init_device(DeviceState* st, int dev);
 
 // Whether the kernel converts V itself.  What a tile's conversion costs is paid once for every query tile that reads the key
 // block, what the pre-pass costs once per key block: the line lies at a number of queries per key.  Measured with the pre-pass /
-// in the kernel (us): D = 128, not causal, 128 heads of 1024 77.9 / 73.6, 64 of 1536 82 / 77, 64 of 2048 129.7 / 131.5, 24 of 4096
-// 186 / 188, 128 of 8192 3446 / 3563; causal, half of whose queries see a key, but the last ones of every sequence see all: 512
-// heads of 512 94 / 76, 256 of 2048 339 / 311, 60 of 3000 163 / 156 but 20 of 3000 71 / 74; window 1300, 20 heads of 8000, 129 / 122.
-// D = 64 converts half as much per block: 64 of 2048 101 / 98, 42 of 3072 143 / 142, 32 of 4096 185 / 186; causal 40 of 4000 147 /
-// 140; window 512 of 3000, 64 heads, 71.2 / 65.0.  Where no more than half of the SMs have a tile, nothing hides the conversion
-// behind another CTA and its cost adds up along the longest tile: 8 heads of 1024 15.4 / 14.0, 4 of 1280 16.8 / 17.4, 1 of 8192 75 / 92.
-// All in a loop of the call; behind the kernel that has just written V the pre-pass costs more, so where both differ little the line
-// is drawn for that: D = 128, not causal, 32 heads of 1536 42.5 / 45.2, but both kernels behind one another 74.5 / 68.8.
+// in the kernel (us), one call behind another: D = 128, not causal, 128 heads of 1024 67 / 60, 64 of 1536 76 / 73, 64 of 2048 114 / 110, 24 of 4096
+// 178 / 181; causal, half of whose queries see a key, but the last ones of every sequence see all: 512 heads of 512 74 / 63, 256 of
+// 2048 277 / 265, 60 of 2500 98 / 96, 60 of 3000 132 / 131; window 1300, 20 heads of 8000, 112 / 109, 300, 128 of 2500, 113 / 107.
+// D = 64 converts half as much per block: 64 of 2048 99 / 95, 42 of 3072 142 / 139, 32 of 4096 187 / 184; causal 40 of 4000 127 / 126, 64 of 5000
+// 299 / 303; window 512 of 3000, 64 heads, 61 / 54.  Behind the kernel that has just written V the pre-pass costs more (both kernels, 32 of
+// 1536 of 128, not causal, 75.0 / 64.0, 64 of 2048 173 / 164, 24 of 4096 223 / 223).  Past the lines the two forms differ by 3 % up to
+// twice the keys, to either side.  Where no more than half of the SMs have a tile, nothing hides the conversion behind another
+// CTA and its cost adds up along the longest tile: 8 heads of 1024 15.4 / 13.6, 4 of 1280 17.5 / 16.8, behind that kernel 24.5 / 26.5 and 24.3 /
+// 23.5; 1 of 8192, with the producer converting, 75 / 92.
 bool converts_v(const LaunchArgs& a, int num_sms) {
     const int limit = a.hd == 128 ? 1536 : 2560;
     const int span = a.causal && a.window > 0 && a.window < a.sl - BM ? a.window + BM : a.sl;   // keys of the longest tile
@@ -1051,19 +1053,20 @@ int heads_together(const LaunchArgs& a, long long tiles, int num_sms) {
 // front, then pair up while other SMs have a short one.  One to an SM, the short ones start where middle ones have finished.  Up to
 // one and a half tiles per SM that was the faster form or level for up to 16 heads; with more heads a sequence has so few tiles that
 // their start and finish count, which two to an SM hide (32 heads of 700 keys of 64, 192 tiles: 11 / 13 us).
-// Behind the kernel that writes Q, K and V, us for both kernels, before V was converted in here / since / one to an SM: D = 64, 5
-// heads of 4000 54.9 / 61.2 / 48.7, 6 of 3500 51.0 / 56.7 / 44.6, 8 of 3000 47.7 / 50.0 / 40.2.  One call behind another: the same
-// 45.9 / 39.6 / 39.3, 42.1 / 35.5 / 35.2, 38.2 / 31.3 / 30.7; D = 128, 6 of 3500 50.7 / 49.8 / 37.8, 8 of 2000 30.4 / 25.7 / 25.7.
+// Behind the kernel that writes Q, K and V, us for both kernels, two to an SM / one: D = 64, 5 heads of 4000 60.4 / 49.7, 6 of 3500 57.2 / 45.0, 8 of
+// 3000 50.9 / 40.5, 16 of 1500 32.4 / 27.3; D = 128, 4 of 4700 70.4 / 66.5, 8 of 2000 43.9 / 37.2, 16 of 1200 34.5 / 30.9.  One call behind
+// another: the same 39.7 / 39.6, 35.6 / 35.3, 31.4 / 30.7, 17.9 / 17.6; 50.2 / 50.0, 24.5 / 24.5, 17.8 / 16.5; D = 128, 6 of 3500 50.7 / 39.2.
 bool one_to_an_sm(const LaunchArgs& a, long long tiles, int num_sms) {
     return a.causal && (a.window <= 0 || a.window >= a.sl) && a.bh <= HEAD_GROUP && 2 * tiles <= 3ll * num_sms;
 }
 
 // Whether a CTA goes on to further tiles: as soon as there are more than fit at once.  That saves a tile its CTA's start (barriers,
-// tensor memory, the first loads' latency: 3000 clk) and part of its end, which the other CTA of the SM hides in part.  Start of a CTA per
-// tile, as it was / a walk, us, both in a loop: D = 128, causal, 1024 heads of 512 136 / 117, 256 of 2048 293 / 274, 64 of 8192 784 / 771; not
-// causal 256 of 1000 140 / 131, 64 of 8192 1550 / 1499; D = 64, 448 of 179, causal, 19.9 / 14.8, 512 of 512 61.6 / 51.8, 64 of 3000, window
-// 512, 63.8 / 54.3, 32 of 8192, causal, 360 / 349.  Just past that line a few causal calls lose (32 of 1300 of 128 22.7 / 23.2, a CTA per
-// tile 22.7) and most gain (28 of 1700 30.4 / 24.1, a CTA per tile 26.5; 300 of 100 11.0 / 8.5 and 10.4).
+// tensor memory, the first loads' latency: 3000 clk) and part of its end, which the other CTA of the SM hides in part.  A CTA per tile / a
+// walk, us, one call behind another, below the power cap: D = 128, causal, 1500 heads of 128 41.0 / 33.8, 500 of 384 49.9 / 42.8, 88 of 2100 112 / 98.6;
+// not causal 1500 of 128 32.8 / 24.5, 500 of 384 49.4 / 40.0, 136 of 1300 125 / 112, 58 of 3300 258 / 246; D = 64, causal, 500 of 384 36.6 / 28.6, 88 of
+// 2100 88.2 / 81.8; not causal 500 of 384 39.0 / 31.5, 58 of 3300 237 / 225; window 512, 64 of 3000, 60.0 / 52.4.  Just past that line a few
+// calls lose (D = 128, 340 to 400 of 128, causal, 12.0 to 12.6 / 12.9 to 13.1, 133 of 384, not causal, 15.5 / 16.4; D = 64, 12 to 27 of 3300 to 1300,
+// causal, 3 %) and most gain (36 of 1300 of 128 25.8 / 23.1, 24 of 2100 33.7 / 30.7; 300 of 128 of 64 9.2 / 7.8).
 bool walks(long long tiles, int num_sms) { return tiles > 2ll * num_sms; }
 
 template <int HD, bool VRAW>

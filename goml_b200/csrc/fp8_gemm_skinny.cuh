@@ -33,8 +33,9 @@ constexpr int smem_of(int per_sm) { return per_sm == 1 ? SMEM_ONE : per_sm == 2 
 
 // Where the codes of the tokens come from: a matrix of them, or (a step of a few sequences) the values that they are made of, which
 // every CTA quantises for itself.  Values of at most MAX_ROWS tokens, of all of K, have one scale, max|value| / 448.  A row costs the
-// four products of a block 4 to 5 us, the quantisers ahead of them 15 to 18 however few rows there are: a step of one sequence 81.2 ->
-// 73.0 us, two 81.7 / 78.5, three 81.9 / 82.8, four 86 / 92.
+// four products of a block 4 to 5 us, the quantisers ahead of them 15 to 18 however few rows there are: a step of a block 4096 wide, of one
+// sequence 73.5 -> 65.3 us, of two 75.6 / 73.2 (a form that took more lost with three, 81.9 / 82.8, and four, 86 / 92).  How long the rows may be
+// is for the caller to say: the block's chain has the line.
 constexpr int MAX_ROWS = 2;
 enum Source : int { CODES = 0, RMS_F32 = 1, F16 = 2, BF16_KNOWN = 3 };   // RMSNorm of fp32 rows; fp16 values; bf16 values whose maximum is known
 struct Rows {
