@@ -96,7 +96,7 @@ struct Cfg {
     // Registers are those of eight warps, two CTAs to an SM: of fourteen warps one of its four schedulers has four, which leaves a thread
     // 128.  Of the masked forms 72 to 80 bytes spill.  With 32 registers of every other thread moved to the softmax threads (setmaxnreg) none
     // did, and 256 heads of 2048, causal, took 247 us (now 264), 1024 of 512 104 (119), 64 of 8192, window 1024, 262 (281), 256 of 1000, not
-    // causal, 119 (131), 40 of 2048 45.4 (46.7).  But beside that split a small change of code, the rescale of O as a loop, raised
+    // causal, 119 (131), 40 of 2048 45.4 (46.7), 900 of 128, causal, 16.6 (21.4).  But beside that split a small change of code, the rescale of O as a loop, raised
     // illegal accesses whose cause was not found, so registers stay where a launch puts them.
     static constexpr int BOUND_THREADS = CONVERTER ? 256 : NUM_THREADS;
     static constexpr int OFF_Q = 0;
