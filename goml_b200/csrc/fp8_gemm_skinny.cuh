@@ -13,9 +13,9 @@
 //    57 bytes a nanosecond, so weights have to be spread over nearly all of them to reach the 6.5 TB/s of HBM);
 //  * the kernel starts before its predecessor on the stream has drained and asks for its first weight tiles to be
 //    brought into L2 while the small kernel ahead (a quantiser, usually) still runs.
-// What is left is 3 us of start, fill and finish beside the stream: M = 16, 8192 x 8192 16.7 -> 13.7 us (floor 10.3),
-// 12288 x 4096 13.3 -> 11.1 (7.7), 22016 x 4096 with SwiGLU
-// 21.9 -> 18.4 (13.8), 11008 x 4096 12.8 -> 10.3 (6.9), 4096 x 11008 12.9 -> 10.8 (6.9), 4096 x 4096 7.8 -> 6.1 (2.6).
+// What is left is 3 us of start, fill and finish beside the stream: M = 16, 8192 x 8192 14.2 us (floor 10.3),
+// 12288 x 4096 11.2 (7.7), 22016 x 4096 with SwiGLU
+// 18.4 (13.8), 4096 x 11008 10.7 (6.9), 4096 x 4096 6.5 (2.6).
 #pragma once
 
 namespace skinny {
@@ -24,12 +24,17 @@ constexpr int W_ROWS = 128;                 // weight rows per tile = TMEM lanes
 constexpr int W_BYTES = W_ROWS * BK;        // of one k-block
 constexpr int MAX_TOKENS = 192;
 constexpr int MAX_STAGES = 16;
+// Most tokens whose partial sums go straight to their owners, with one meeting of the cluster behind the last MMA in the place of two and of reads from
+// other CTAs (us, before / so): 16 tokens, 2048 x 2048 4.76 / 4.00, 1504 x 6000 6.47 / 5.87, 4096 x 11008 added 11.1 / 10.7, 8192 x 8192 14.4 / 14.2; 5 tokens,
+// 3001 x 3008 5.70 / 5.19.  With more, 4 bytes at a time to another CTA take longer than 16 at a time from it: 64 tokens, 4096 x 4096 added 7.77 / 8.28
+// (fetched, with scales asked for ahead of the meeting: 7.59), 173 tokens 10.0 / 11.8 (9.80).
+constexpr int APART_TOKENS = 16;
 constexpr int MAX_SPLIT = 8;                // portable cluster size
 constexpr int THREADS = 192;                // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2-5: read the accumulators back
 constexpr int TAIL_BYTES = 1024 /*align*/ + 512 /*barriers*/;
 constexpr int SMEM_ONE = 227 * 1024;        // of one CTA when it has the SM to itself
 // shared memory of one of up to three CTAs on an SM (228 KB, 1 KB of it the system's for each CTA)
-constexpr int smem_of(int per_sm) { return per_sm == 1 ? SMEM_ONE : per_sm == 2 ? 112 * 1024 : 74 * 1024; }
+constexpr int smem_of(int per_sm) { return per_sm == 1 ? SMEM_ONE : per_sm == 2 ? 112 * 1024 : 75 * 1024; }
 
 // Where the codes of the tokens come from: a matrix of them, or (a step of a few sequences) the values that they are made of, which
 // every CTA quantises for itself.  Values of at most MAX_ROWS tokens, of all of K, have one scale, max|value| / 448.  A row costs the
@@ -63,29 +68,33 @@ struct Params {
     int vec;           // four neighbouring outputs of a token may be stored at once
 };
 
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float4 ld_dsmem(uint32_t addr, uint32_t rank) {
-    float4 v;
-    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\t"
-                 "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(rank) : "memory");
-    return v;
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    return a;
 }
 __device__ __forceinline__ void prefetch_l2_2d(const CUtensorMap* m, int x, int y) {
     asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];"
                  ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y) : "memory");
 }
-// the cluster's partial results for weight rows [row, row + 4) and token j: loads, and their sum in rank order
+// Who finishes what.  APART: a tile's 128 weight rows are 16 pairs of 4 rows and the 4 rows 32 further on (with SwiGLU: gate rows and their up
+// rows), dealt to the CTAs of the cluster in runs of up to PAIRS; the partial sums lie with the owner as [source][token][half][PAIRS][4].
+// Else they lie with their source, as [token][128].
+__host__ __device__ constexpr int pairs_of(int split) { return (16 + split - 1) / split; }
+__host__ __device__ constexpr int apart_bytes(int split, int tokens) { return split * tokens * 2 * pairs_of(split) * 16; }
 template <int SPLIT>
-__device__ __forceinline__ void gather(float4* v, uint32_t part, int j, int row) {
-    const uint32_t a = part + j * (W_ROWS * 4) + row * 4;
-    if (SPLIT == 1) {
-        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[0].z), "=f"(v[0].w) : "r"(a) : "memory");
-    } else {
+__device__ __forceinline__ int first_pair(int rank) { return (16 * rank + SPLIT - 1) / SPLIT; }   // owner of pair u: u * SPLIT / 16
+// the sums of all sources for four rows and a token; a: where they lie in this CTA
+template <int SPLIT, int APART>
+__device__ __forceinline__ void gather(float4* v, uint32_t a, uint32_t source_bytes) {
 #pragma unroll
-        for (int s = 0; s < SPLIT; s++) v[s] = ld_dsmem(a, s);
+    for (int s = 0; s < SPLIT; s++) {
+        if (SPLIT == 1 || APART)
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[s].x), "=f"(v[s].y), "=f"(v[s].z), "=f"(v[s].w) : "r"(a + s * source_bytes) : "memory");
+        else
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[s].x), "=f"(v[s].y), "=f"(v[s].z), "=f"(v[s].w) : "r"(map_rank(a, s)) : "memory");
     }
 }
 template <int SPLIT>
@@ -230,9 +239,11 @@ __device__ __forceinline__ void quantise_rows(const Params& p, uint32_t tok, flo
     }
 }
 
-// VALUES: the tokens come as values (Rows), else as codes
-template <int SPLIT, bool VALUES>
-__global__ void __launch_bounds__(THREADS, 2)
+// VALUES: the tokens come as values (Rows), else as codes.  APART: the partial sums have shared memory of their own, else the ring's place.
+template <int SPLIT, bool VALUES, int APART>
+// Three CTAs on an SM put up to five of their warps on one of its four schedulers, whose registers hold five of 96 registers a thread: the
+// bound says 224 threads so that the compiler stays there (with 104 the third CTA waits for the first to end).
+__global__ void __launch_bounds__(224, 3)
 fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_t, const Params p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;   // swizzle atoms are 1024 bytes
@@ -242,10 +253,12 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     // finds in the block behind, so that there is one block more
     const uint32_t tok = ring + p.stages * stage_bytes;
     const uint32_t tok_bytes = VALUES ? (p.slice + 1) * TOKEN_BYTES : 0;
-    const uint32_t bar_full = tok + tok_bytes;
+    const uint32_t part = APART ? tok + tok_bytes : ring;
+    const uint32_t part_bytes = APART ? apart_bytes(SPLIT, p.g.M) : 0;
+    const uint32_t bar_full = tok + tok_bytes + part_bytes;
     const uint32_t bar_empty = bar_full + 8 * MAX_STAGES;
     const uint32_t bar_done = bar_empty + 8 * MAX_STAGES;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ring_gen + p.stages * stage_bytes + tok_bytes + 16 * MAX_STAGES + 8);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ring_gen + p.stages * stage_bytes + tok_bytes + part_bytes + 16 * MAX_STAGES + 8);
     volatile uint32_t* abort_flag = tmem_slot + 1;
     const uint32_t bar_tok = bar_done + 16;
     float* scale_slot = reinterpret_cast<float*>(tmem_slot + 4);
@@ -257,6 +270,7 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     const int n0 = ((int)blockIdx.x / SPLIT) * W_ROWS;
     const int kb0 = (int)((long long)rank * p.g.k_blocks / SPLIT), kb1 = (int)((long long)(rank + 1) * p.g.k_blocks / SPLIT);
 
+    if (APART) cluster_arrive();   // its phase says that every CTA runs, so that its shared memory may be written
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; s++) {
             mbar_init(bar_full + 8 * s, 1);
@@ -293,6 +307,7 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     }
     pdl_wait();
     pdl_trigger();
+    bool acc_ready = false;   // this warp may read the accumulators
     if (VALUES && blockIdx.x == 0 && (int)threadIdx.x < p.r.zeros) p.r.zero[threadIdx.x] = 0.f;
 
     if (warp == 0) {
@@ -330,64 +345,79 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         if (ok && leader) mma_commit(bar_done);
         __syncwarp();
     } else {
-        // accumulators -> shared memory, token-major ([token][128 weight rows] fp32): lanes write neighbouring words.  The
-        // ring is free by then: every load that was issued has been consumed by an MMA that has retired.
-        const int quad = warp & 3;
         if (VALUES) {
             quantise_rows(p, tok, red, scale_slot, kb0, kb1, (int)threadIdx.x - 64);
             fence_proxy_async_smem();
             mbar_arrive(bar_tok);
             __syncwarp();
         }
-        if (mbar_wait_warp(bar_done, 0, abort_flag, ST_TIMEOUT_EPILOGUE)) {
-            tc_fence_after();
-            for (int j0 = 0; j0 < p.tn; j0 += 16) {
-                uint32_t acc[16];
-                tmem_ld_32x32b_x16(tmem + j0 + (uint32_t(quad * 32) << 16), acc);
-                tmem_ld_wait();
-                const uint32_t dst = ring + j0 * (W_ROWS * 4) + (quad * 32 + lane) * 4;
+        acc_ready = mbar_wait_warp(bar_done, 0, abort_flag, ST_TIMEOUT_EPILOGUE);
+        tc_fence_after();
+    }
+    __syncwarp();
+
+    // ---- finish: the CTAs of the cluster share the tile's outputs.  With little to hand over, a CTA's partial sums go to their owners, into memory
+    // that the ring never uses, and one meeting does; else they take the ring's place (free by then: every load that was issued has been consumed by
+    // an MMA that has retired), the owners fetch them behind a meeting, and nobody leaves before another.
+    const GemmParams& g = p.g;
+    constexpr int PAIRS = pairs_of(SPLIT);
+    const int u0 = first_pair<SPLIT>(rank), pairs = first_pair<SPLIT>(rank + 1) - u0;   // APART: what this CTA owns
+    const uint32_t source_bytes = g.M * 2 * PAIRS * 16;
+    // asked for ahead of the meeting
+    float alpha = g.alpha;
+    if (!VALUES && g.scale_a) alpha *= ld_f32(g.scale_a);
+    const float scale_b = g.scale_b ? ld_f32(g.scale_b) : 1.0f;
+    const float scale_d = (g.D8 && g.scale_d) ? ld_f32(g.scale_d) : 1.0f;
+    if (APART) cluster_wait();
+    if (acc_ready) {   // neighbouring lanes write neighbouring words
+        const int quad = warp & 3, row = quad * 32 + lane;
+        const int u = (row >> 6) * 8 + ((row >> 2) & 7), owner = u * SPLIT / 16;
+        const uint32_t dst = !APART ? part + row * 4
+                                    : map_rank(part + rank * source_bytes + ((quad & 1) * PAIRS + u - first_pair<SPLIT>(owner)) * 16 + (row & 3) * 4, owner);
+        constexpr int TOKEN = APART ? 2 * PAIRS * 16 : W_ROWS * 4;
+        for (int j0 = 0; j0 < (APART ? g.M : p.tn); j0 += 16) {
+            uint32_t acc[16];
+            tmem_ld_32x32b_x16(tmem + j0 + (uint32_t(quad * 32) << 16), acc);
+            tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 16; i++)
-                    asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + i * (W_ROWS * 4)), "r"(acc[i]) : "memory");
+            for (int i = 0; i < 16; i++) {
+                if (!APART) asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + (j0 + i) * TOKEN), "r"(acc[i]) : "memory");
+                else if (j0 + i < g.M) asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(dst + (j0 + i) * TOKEN), "r"(acc[i]) : "memory");
             }
         }
         tc_fence_before();
     }
     __syncwarp();
-    cluster_sync_all();
-
+    cluster_arrive();
     {
-        // The CTAs of the cluster finish the tile's outputs together, blocks of THREADS groups of four outputs in turn.  A
-        // thread takes several groups at a time, all their loads (partial sums, and the residual stream in the accumulate
-        // mode) issued before the first use: one group at a time was bound by their latency (0.35 us a round, 16 rounds for 64
-        // tokens).
-        const GemmParams& g = p.g;
-        constexpr int STEP = SPLIT * THREADS;
-        float alpha = g.alpha;
-        if (VALUES) alpha *= *scale_slot;
-        else if (g.scale_a) alpha *= ld_f32(g.scale_a);
-        if (g.scale_b) alpha *= ld_f32(g.scale_b);
-        const float scale_d = (g.D8 && g.scale_d) ? ld_f32(g.scale_d) : 1.0f;
+        // The CTAs of the cluster finish the tile's outputs together, groups of four outputs of a token.  A thread takes several groups at a time,
+        // all their loads (partial sums, and the residual stream in the accumulate mode) issued before the first use: one group at a time was bound
+        // by their latency (0.35 us a round, 16 rounds for 64 tokens).
+        constexpr int STEP = APART ? THREADS : SPLIT * THREADS;
+        const int first = APART ? (int)threadIdx.x : rank * THREADS + (int)threadIdx.x;
         float tmax = 0.f;
         if (g.H) {
             // gate rows [64c, 64c + 32), up rows [64c + 32, 64c + 64) of the tile
-            constexpr int QUADS = W_ROWS / 8;   // groups of four activation columns
+            constexpr int QUADS = APART ? PAIRS : 16;   // groups of four activation columns
             constexpr int U = SPLIT == 1 ? 4 : SPLIT == 2 ? 2 : 1;
             const int items = g.M * QUADS;
-            for (int it0 = rank * THREADS + threadIdx.x; it0 < items; it0 += U * STEP) {
+            cluster_wait();
+            if (VALUES) alpha *= *scale_slot;
+            alpha *= scale_b;
+            for (int it0 = first; it0 < items; it0 += U * STEP) {
                 float4 gt[U][SPLIT], up[U][SPLIT];
 #pragma unroll
                 for (int u = 0; u < U; u++) {
                     const int it = min(it0 + u * STEP, items - 1), j = it / QUADS, q = it % QUADS;
-                    const int row = (q >> 3) * 64 + (q & 7) * 4;
-                    gather<SPLIT>(gt[u], ring, j, row);
-                    gather<SPLIT>(up[u], ring, j, row + 32);
+                    const uint32_t at = part + (APART ? (j * 2 * PAIRS + q) * 16 : j * (W_ROWS * 4) + ((q >> 3) * 64 + (q & 7) * 4) * 4);
+                    gather<SPLIT, APART>(gt[u], at, source_bytes);
+                    gather<SPLIT, APART>(up[u], at + (APART ? PAIRS * 16 : 32 * 4), source_bytes);
                 }
 #pragma unroll
                 for (int u = 0; u < U; u++) {
                     const int it = it0 + u * STEP, j = it / QUADS, q = it % QUADS;
                     if (it >= items) break;
-                    const int col = (n0 >> 1) + q * 4;
+                    const int col = (n0 >> 1) + (APART ? u0 + q : q) * 4;
                     float gv[4], uv[4], h[4];
                     add_up<SPLIT>(gt[u], gv);
                     add_up<SPLIT>(up[u], uv);
@@ -399,7 +429,7 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
                         h[i] = a * r * (uv[i] * alpha);
                     }
                     const uint32_t w[2] = {pack_out(h[0], h[1], 1), pack_out(h[2], h[3], 1)};
-                    if (col >= g.F) continue;
+                    if (col >= g.F || (APART && q >= pairs)) continue;
 #pragma unroll
                     for (int i = 0; i < 2; i++)   // max of the rounded values; columns past F are zero
                         tmax = fmaxf(tmax, fmaxf(fabsf(__uint_as_float(w[i] << 16)), fabsf(__uint_as_float(w[i] & 0xffff0000u))));
@@ -414,34 +444,49 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
                 }
             }
         } else {
-            constexpr int QUADS = W_ROWS / 4;
+            constexpr int QUADS = APART ? 2 * PAIRS : W_ROWS / 4;
             constexpr int U = SPLIT <= 2 ? 4 : SPLIT <= 4 ? 2 : 1;
             const int items = g.M * QUADS;
-            for (int it0 = rank * THREADS + threadIdx.x; it0 < items; it0 += U * STEP) {
-                float4 part[U][SPLIT];
-                float x[U][4];
+            auto column = [&](int r) {   // of a token's group r; none of it there: N
+                if (!APART) return n0 + r * 4;
+                const int half = r >= PAIRS, q = r - half * PAIRS, u = u0 + q;
+                return q < pairs ? n0 + (u >> 3) * 64 + half * 32 + (u & 7) * 4 : g.N;
+            };
+            float x[U][4];
+            auto residual = [&](int it0) {
 #pragma unroll
                 for (int u = 0; u < U; u++) {
-                    const int it = min(it0 + u * STEP, items - 1), j = it / QUADS, row = (it % QUADS) * 4, col = n0 + row;
-                    if (g.X) {
-                        const float* src = (VALUES ? p.r.x_in : g.X) + (size_t)j * g.N + col;
-                        if (p.vec && col + 4 <= g.N) {
-                            const float4 t = *reinterpret_cast<const float4*>(src);
-                            x[u][0] = t.x; x[u][1] = t.y; x[u][2] = t.z; x[u][3] = t.w;
-                        } else {
+                    const int it = min(it0 + u * STEP, items - 1), j = it / QUADS, col = column(it % QUADS);
+                    const float* src = (VALUES ? p.r.x_in : g.X) + (size_t)j * g.N + col;
+                    if (p.vec && col + 4 <= g.N) {
+                        const float4 t = *reinterpret_cast<const float4*>(src);
+                        x[u][0] = t.x; x[u][1] = t.y; x[u][2] = t.z; x[u][3] = t.w;
+                    } else {
 #pragma unroll
-                            for (int i = 0; i < 4; i++) x[u][i] = col + i < g.N ? src[i] : 0.f;
-                        }
+                        for (int i = 0; i < 4; i++) x[u][i] = col + i < g.N ? src[i] : 0.f;
                     }
-                    gather<SPLIT>(part[u], ring, j, row);
+                }
+            };
+            if (APART && g.X) residual(first);   // only this thread writes there: it need not wait for the meeting
+            __syncwarp();
+            cluster_wait();
+            if (VALUES) alpha *= *scale_slot;
+            alpha *= scale_b;
+            for (int it0 = first; it0 < items; it0 += U * STEP) {
+                float4 sums[U][SPLIT];
+                if (g.X && !(APART && it0 == first)) residual(it0);
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int it = min(it0 + u * STEP, items - 1), j = it / QUADS, r = it % QUADS;
+                    gather<SPLIT, APART>(sums[u], part + (j * QUADS + r) * 16, source_bytes);
                 }
 #pragma unroll
                 for (int u = 0; u < U; u++) {
-                    const int it = it0 + u * STEP, j = it / QUADS, row = (it % QUADS) * 4, col = n0 + row;
+                    const int it = it0 + u * STEP, j = it / QUADS, col = column(it % QUADS);
                     if (it >= items) break;
                     if (col >= g.N) continue;
                     float v[4];
-                    add_up<SPLIT>(part[u], v);
+                    add_up<SPLIT>(sums[u], v);
                     const size_t off = (size_t)j * g.N + col;
                     const bool whole = p.vec && col + 4 <= g.N;
                     if (g.X) {
@@ -495,7 +540,10 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     }
     // ------------------------------------------------------------- teardown
     __syncwarp();
-    cluster_sync_all();   // peers have read this CTA's partial sums
+    if (SPLIT > 1 && !APART) {   // peers have read this CTA's sums
+        cluster_arrive();
+        cluster_wait();
+    }
     const uint32_t code = *abort_flag;
     if (code != 0) {
         if (threadIdx.x == 0) atomicCAS(&g_gemm_status, 0u, code);
@@ -509,13 +557,12 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
 }
 
 using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const Params);
-inline Kernel kernel_for(int split, bool values) {
-    static const Kernel table[2][MAX_SPLIT] = {
-        {fp8_gemm_skinny_kernel<1, false>, fp8_gemm_skinny_kernel<2, false>, fp8_gemm_skinny_kernel<3, false>, fp8_gemm_skinny_kernel<4, false>,
-         fp8_gemm_skinny_kernel<5, false>, fp8_gemm_skinny_kernel<6, false>, fp8_gemm_skinny_kernel<7, false>, fp8_gemm_skinny_kernel<8, false>},
-        {fp8_gemm_skinny_kernel<1, true>, fp8_gemm_skinny_kernel<2, true>, fp8_gemm_skinny_kernel<3, true>, fp8_gemm_skinny_kernel<4, true>,
-         fp8_gemm_skinny_kernel<5, true>, fp8_gemm_skinny_kernel<6, true>, fp8_gemm_skinny_kernel<7, true>, fp8_gemm_skinny_kernel<8, true>}};
-    return table[values][split - 1];
+// kinds: codes with the sums in the ring's place or apart, values
+inline Kernel kernel_for(int split, int kind) {
+#define GOML_KINDS(S) {fp8_gemm_skinny_kernel<S, false, 0>, fp8_gemm_skinny_kernel<S, false, 1>, fp8_gemm_skinny_kernel<S, true, 1>}
+    static const Kernel table[MAX_SPLIT][3] = {GOML_KINDS(1), GOML_KINDS(2), GOML_KINDS(3), GOML_KINDS(4), GOML_KINDS(5), GOML_KINDS(6), GOML_KINDS(7), GOML_KINDS(8)};
+#undef GOML_KINDS
+    return table[split - 1][kind];
 }
 
 // clusters of each size that are resident at once with one CTA to an SM (a cluster stays inside one group of SMs, so this
@@ -542,15 +589,15 @@ inline void configure(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int ti
 inline cudaError_t init(Fit* fit) {
     for (int split = 1; split <= MAX_SPLIT; split++) {
         cudaError_t e = cudaSuccess;
-        for (bool values : {false, true}) {
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel_for(split, values), cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_ONE);
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel_for(split, values), cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        for (int kind = 0; kind < 3; kind++) {
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel_for(split, kind), cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_ONE);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel_for(split, kind), cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         }
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[2];
         configure(cfg, attr, 1, split, SMEM_ONE, nullptr);
         cfg.numAttrs = 1;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fit->one[split], kernel_for(split, false), &cfg);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fit->one[split], kernel_for(split, 0), &cfg);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -628,15 +675,23 @@ inline int launch(GemmParams g, const Plan& plan, const void* A, const void* B, 
     p.idesc = make_idesc_e4m3_f32(W_ROWS, p.tn, 0, 0);
     const int tiles = (g.N + W_ROWS - 1) / W_ROWS;
     const int slice = (g.k_blocks + plan.split - 1) / plan.split;
-    const int stage_bytes = rows ? W_BYTES : W_BYTES + p.tn * BK, part_bytes = p.tn * W_ROWS * 4;
+    const int stage_bytes = rows ? W_BYTES : W_BYTES + p.tn * BK;
     const int tok_bytes = rows ? (slice + 1) * TOKEN_BYTES : 0;
     p.slice = slice;
-    p.stages = (smem_of(plan.per_sm) - TAIL_BYTES - tok_bytes) / stage_bytes;
-    if (rows && p.stages < 2) return (int)cudaErrorNotSupported;
-    if (p.stages > slice) p.stages = slice;
-    if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
+    const int room = smem_of(plan.per_sm) - TAIL_BYTES - tok_bytes;
+    auto stages_in = [&](int bytes) {
+        int n = bytes / stage_bytes;
+        if (rows && plan.per_sm == 3 && n > 3) n = 3;   // the rows' values wait behind what the rings have asked for: a step of one sequence 67.0, with four 67.7
+        return n > slice ? slice : n > MAX_STAGES ? MAX_STAGES : n;
+    };
+    // Partial sums of up to 16 tokens have memory of their own where that costs no stage; a row as values has 512 bytes
+    const int own_bytes = apart_bytes(plan.split, g.M);
+    const bool apart = rows || (g.M <= APART_TOKENS && stages_in(room - own_bytes) == stages_in(room));
+    p.stages = stages_in(apart ? room - own_bytes : room);
+    if (rows && room - own_bytes < 2 * stage_bytes) return (int)cudaErrorNotSupported;
     int ring_bytes = p.stages * stage_bytes;
-    while (ring_bytes < part_bytes) { p.stages++; ring_bytes += stage_bytes; }   // the partial sums take the ring's place
+    const int part_bytes = apart ? own_bytes : 0;
+    while (!apart && ring_bytes < p.tn * W_ROWS * 4) { p.stages++; ring_bytes += stage_bytes; }   // the partial sums take the ring's place
     // How much of the weight is asked for ahead of the wait.  It helps as far as memory is idle until then; past that a CTA's first
     // loads stand behind hints for its last ones.  Half of a CTA's blocks up to 16 (all of up to 8), with several CTAs to an SM no more than 20 MB in
     // all, and four blocks past 80 tokens, whose first loads bring as much again in tokens, which no hint has fetched.  All / as
@@ -659,8 +714,8 @@ inline int launch(GemmParams g, const Plan& plan, const void* A, const void* B, 
     if (rows) tt = tw;   // not looked at
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
-    configure(cfg, attr, tiles, plan.split, (size_t)ring_bytes + tok_bytes + TAIL_BYTES, stream);
-    return (int)cudaLaunchKernelEx(&cfg, kernel_for(plan.split, rows != nullptr), tw, tt, p);
+    configure(cfg, attr, tiles, plan.split, (size_t)ring_bytes + tok_bytes + part_bytes + TAIL_BYTES, stream);
+    return (int)cudaLaunchKernelEx(&cfg, kernel_for(plan.split, rows ? 2 : apart), tw, tt, p);
 }
 
 }  // namespace skinny

@@ -68,6 +68,44 @@ def test_added_to_fp32_by_the_kernel_that_cuts_a_long_k_best(cuda, built_libs, M
     assert (room[:16 + offset] == 7).all() and (room[16 + offset + M * N:] == 7).all()
 
 
+@pytest.mark.parametrize("split,K", [(1, 384), (2, 512), (3, 880), (4, 1024), (5, 6400), (6, 7696), (7, 8960), (8, 10240)])
+@pytest.mark.parametrize("N", [200, 131])
+def test_sums_handed_to_their_owners_and_fetched_are_the_same(cuda, built_libs, split, K, N):
+    # up to 16 rows a CTA's sums go to their owner, past that the owners fetch them: added in the same order, so every row has the same bits
+    from goml_b200 import fp8_gemm as G
+    g = torch.Generator(device="cuda").manual_seed(split + N)
+    a, b = (torch.randint(0, 0x70, (rows, K), generator=g, dtype=torch.uint8, device="cuda") for rows in (17, 2 * ((N + 31) // 32) * 32))
+    a ^= torch.randint(0, 2, a.shape, generator=g, dtype=torch.uint8, device="cuda") << 7
+    s = torch.tensor([3e-3, 2e-3], device="cuda")
+    sa, sb = s.data_ptr(), s.data_ptr() + 4
+    x0 = torch.randn(17, N, generator=g, device="cuda")
+
+    def outputs(M):
+        st = torch.cuda.current_stream().cuda_stream
+        c, x, h = torch.empty(M, N, dtype=torch.bfloat16, device="cuda"), x0[:M].clone(), torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+        d, top = torch.empty(M, N, dtype=torch.uint8, device="cuda"), torch.zeros(2, device="cuda")
+        calls = [lambda: G.FP8GEMMScaled(M, N, K, a.data_ptr(), b.data_ptr(), c.data_ptr(), 1.0, sa, sb, G.OutBF16, torch.cuda.current_stream().cuda_stream),
+                 lambda: G.FP8GEMMAccumulateF32(M, N, K, a.data_ptr(), b.data_ptr(), x.data_ptr(), 1.0, sa, sb, st),
+                 lambda: G.FP8GEMMSwiGLURaise(M, N, K, a.data_ptr(), b.data_ptr(), h.data_ptr(), 1.0, sa, sb, top.data_ptr(), st),
+                 lambda: G.FP8GEMMFP8Out(M, N, K, a.data_ptr(), b.data_ptr(), d.data_ptr(), 1.0, sa, sb, 0, top.data_ptr() + 4, st)]
+        name, = kernels(calls[0])
+        assert f"ILi{split}ELb0ELi{int(M <= 16)}E" in name
+        for call in calls:
+            call()
+        torch.cuda.synchronize()
+        assert G.device_status() == 0 and top[0].item() == h.float().abs().max().item() and top[1].item() > 0
+        return c, x, h, d
+
+    whole = outputs(17)
+    for M in (1, 2, 15, 16):
+        for got, want in zip(outputs(M), whole):
+            assert torch.equal(got.view(torch.uint8), want[:M].contiguous().view(torch.uint8))
+    ref = lambda t: t.view(torch.float8_e4m3fn).double()
+    want = 6e-6 * ref(a) @ ref(b[:N]).t()
+    # a product of 17 bits a term, summed in fp32: 2^-24 a sum, and bf16's 2^-9
+    assert ((whole[0].double() - want).norm() / want.norm()).item() < 4e-3
+
+
 @pytest.mark.parametrize("M,K,few", [(80, 3008, True), (100, 3008, False), (128, 3488, False), (128, 3504, True), (150, 4784, False), (150, 4800, True)])
 def test_codes_on_both_sides_of_the_line(cuda, built_libs, M, K, few):
     from goml_b200 import fp8_gemm as G
