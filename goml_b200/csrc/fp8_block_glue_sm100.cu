@@ -613,10 +613,10 @@ struct QkvOp {
     QkvArgs a;
     using State = NoState;
     __device__ void ahead() const {}
-    __device__ void pass1(float (&m)[3], State&) const { qkv_amax_items(a, oc_tid(), OC_STEP, m); }
+    __device__ void pass1(float (&m)[3], State&) const { qkv_amax_items(a, oc_tid(), oc_step(), m); }
     __device__ void pass2(const float (&m)[3], State&) const {
         if (oc_tid() < 3) a.amaxes[oc_tid()] = oc_tid() == 0 ? m[0] : oc_tid() == 1 ? m[1] : m[2];
-        qkv_quant_items(a, oc_tid(), OC_STEP, m);
+        qkv_quant_items(a, oc_tid(), oc_step(), m);
     }
 };
 
@@ -823,7 +823,7 @@ struct DecOp {
         }
         if (s.q) dec_store_q(a, s.b, s.slot, s.c, s.pos, s.y, __fdiv_rn(1.0f, scale));
         if (a.seq_lens_out == a.positions)
-            for (uint32_t b = oc_tid(); b < (uint32_t)a.batch; b += OC_STEP) a.seq_lens_out[b] = dec_length(a, (int)b);
+            for (uint32_t b = oc_tid(); b < (uint32_t)a.batch; b += oc_step()) a.seq_lens_out[b] = dec_length(a, (int)b);
     }
 };
 __global__ void __launch_bounds__(THREADS) dec_lengths_kernel(const DecAppend a) {
@@ -894,10 +894,10 @@ struct OOp {
     OArgs a;
     using State = NoState;
     __device__ void ahead() const {}
-    __device__ void pass1(float (&m)[1], State&) const { m[0] = o_amax_items(a, oc_tid(), OC_STEP); }
+    __device__ void pass1(float (&m)[1], State&) const { m[0] = o_amax_items(a, oc_tid(), oc_step()); }
     __device__ void pass2(const float (&m)[1], State&) const {
         if (oc_tid() == 0) *a.amax_out = m[0];
-        o_quant_items(a, oc_tid(), OC_STEP, m[0]);
+        o_quant_items(a, oc_tid(), oc_step(), m[0]);
     }
 };
 
@@ -1081,7 +1081,7 @@ int rope_qkv(const Rope& r, bool cleared, cudaStream_t s) {
     a.dv.heads = FastDiv(a.heads);
     a.dv.three = FastDiv(3);
     a.dv.seq = FastDiv(a.seq_len);
-    if (items * 64 <= OC_BYTES_QKV && oc_fits<QkvOp>()) return (int)oc_launch(QkvOp{a}, s);
+    if (items * 64 <= OC_BYTES_QKV && oc_fits<QkvOp>()) return (int)oc_launch(QkvOp{a}, s, oc_threads(items));
     cudaError_t e = cleared ? cudaSuccess : clear_words(a.amaxes, 3, s);
     if (e == cudaSuccess && items > 0) e = launch_pdl_stream(items * 64, qkv_amax_kernel, dim3(grid_for(items)), dim3(THREADS), s, a);
     if (e == cudaSuccess) e = launch_pdl_stream(items * 64, qkv_quant_kernel, dim3(grid_for(items)), dim3(THREADS), s, a);
@@ -1118,7 +1118,7 @@ int append(const fp8_decode_append_args_t* g, bool cleared) {
     a.tab_vec = !misaligned(g->cos_tab) && !misaligned(g->sin_tab);
     a.cph = FastDiv(g->head_dim / 32);
     a.slots = FastDiv(slots);
-    if (items * 64 <= OC_BYTES_DEC && oc_fits<DecOp>()) return (int)oc_launch(DecOp{a}, s);
+    if (items * 64 <= OC_BYTES_DEC && oc_fits<DecOp>()) return (int)oc_launch(DecOp{a}, s, oc_threads(items));
     cudaError_t e = cleared ? cudaSuccess : clear_words(a.q_amax, 1, s);
     if (e == cudaSuccess && items > 0) e = launch_pdl(dec_q_amax_kernel, dim3(grid_for(items)), dim3(THREADS), 0, s, a);
     if (e == cudaSuccess) e = launch_pdl(dec_append_kernel, dim3(grid_for(items)), dim3(THREADS), 0, s, a);
@@ -1141,7 +1141,7 @@ int permute_heads(const void* o_fp16, uint8_t* q, float* scale_out, float* amax_
     a.dv.cph = FastDiv(head_dim / 16);
     a.dv.heads = FastDiv(heads);
     a.dv.seq = FastDiv(seq_len);
-    if (state != Max::KNOWN && n16 * 32 <= OC_BYTES_O && oc_fits<OOp>()) return (int)oc_launch(OOp{a}, s);
+    if (state != Max::KNOWN && n16 * 32 <= OC_BYTES_O && oc_fits<OOp>()) return (int)oc_launch(OOp{a}, s, oc_threads(n16));
     cudaError_t e = state == Max::ANY ? clear_words(amax_out, 1, s) : cudaSuccess;
     // Asking for L1 here as the other streams do cost a sixth (B * S * H * hd = 67 M values 50.4 / 58.1 us, behind their attention 320 / 327).
     if (e == cudaSuccess && n16 > 0 && state != Max::KNOWN) e = launch_pdl(o_amax_kernel, dim3(grid_for(n16)), dim3(THREADS), 0, s, a);

@@ -134,10 +134,10 @@ struct QuantOp {
     float divisor;
     using State = NoState;
     __device__ void ahead() const {}
-    __device__ void pass1(float (&m)[1], State&) const { m[0] = amax_items<WIDE, BATCH>(x, n, oc_tid(), OC_STEP); }
+    __device__ void pass1(float (&m)[1], State&) const { m[0] = amax_items<WIDE, BATCH>(x, n, oc_tid(), oc_step()); }
     __device__ void pass2(const float (&m)[1], State&) const {
         if (oc_tid() == 0) *amax_out = m[0];
-        quant_items<WIDE, BATCH>(x, q, n, oc_tid(), OC_STEP, m[0], scale_out, divisor);
+        quant_items<WIDE, BATCH>(x, q, n, oc_tid(), oc_step(), m[0], scale_out, divisor);
     }
 };
 
@@ -296,7 +296,7 @@ template <bool WIDE>
 int quantize_f32(const float* x, uint8_t* q, float* scale_out, float* amax_out, size_t n, float divisor, cudaStream_t s) {
     const size_t n8 = n / 8;
     if (n * 4 <= OC_BYTES) {
-        if (n8 <= OC_STEP && oc_fits<QuantOp<WIDE, 1>>()) return (int)oc_launch(QuantOp<WIDE, 1>{x, q, n, scale_out, amax_out, divisor}, s);
+        if (n8 <= OC_STEP && oc_fits<QuantOp<WIDE, 1>>()) return (int)oc_launch(QuantOp<WIDE, 1>{x, q, n, scale_out, amax_out, divisor}, s, oc_threads(n8));
         if ((!WIDE || n8 <= 2 * OC_STEP) && oc_fits<QuantOp<WIDE, 2>>()) return (int)oc_launch(QuantOp<WIDE, 2>{x, q, n, scale_out, amax_out, divisor}, s);
         if (oc_fits<QuantOp<WIDE, 4>>()) return (int)oc_launch(QuantOp<WIDE, 4>{x, q, n, scale_out, amax_out, divisor}, s);
     }

@@ -17,7 +17,7 @@
 namespace sm100 {
 
 constexpr int OC_CTAS = 16;        // more than the portable 8: a cluster of 16 fits a group of SMs of the B200
-constexpr int OC_THREADS = 512;
+constexpr int OC_THREADS = 512;    // at most
 
 __device__ __forceinline__ int oc_rank() {
     uint32_t r;
@@ -49,7 +49,8 @@ __device__ __forceinline__ void oc_max(float (&m)[N]) {
         for (int n = 0; n < N; n++) {
             float v = warp_max[n][0];
 #pragma unroll
-            for (int w = 1; w < OC_THREADS / 32; w++) v = fmaxf(v, warp_max[n][w]);
+            for (int w = 1; w < OC_THREADS / 32; w++)
+                if (32 * w < (int)blockDim.x) v = fmaxf(v, warp_max[n][w]);
             const uint32_t mine = (uint32_t)__cvta_generic_to_shared(&slots[n][oc_rank()]);
             asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.f32 [a], %2;\n\t}"
                          ::"r"(mine), "r"(threadIdx.x), "f"(v) : "memory");
@@ -83,14 +84,23 @@ __global__ void __launch_bounds__(OC_THREADS) one_cluster_kernel(const Op op) {
     oc_max(m);
     op.pass2(m, state);
 }
-__device__ __forceinline__ uint32_t oc_tid() { return (uint32_t)oc_rank() * OC_THREADS + threadIdx.x; }
-constexpr uint32_t OC_STEP = OC_CTAS * OC_THREADS;
+__device__ __forceinline__ uint32_t oc_tid() { return (uint32_t)oc_rank() * blockDim.x + threadIdx.x; }
+__device__ __forceinline__ uint32_t oc_step() { return OC_CTAS * blockDim.x; }
+constexpr uint32_t OC_STEP = OC_CTAS * OC_THREADS;   // of a full cluster
+
+// Threads for an op of `items`, one to a thread as far as that goes.  Where there is less to do than 512 threads a CTA, a smaller CTA finds its registers on
+// an SM beside the CTAs of the GEMM ahead and waits there, instead of being launched when those have gone (a step of two sequences, us, 512 threads always /
+// so: 73.7 / 72.2, of three 76.1 / 74.9, of eight 85.9 / 85.2).
+inline int oc_threads(size_t items) {
+    const size_t t = (items + OC_CTAS * 32 - 1) / (OC_CTAS * 32) * 32;
+    return (int)(t < 32 ? 32 : t > OC_THREADS ? OC_THREADS : t);
+}
 
 template <class Op>
-inline cudaLaunchConfig_t oc_config(cudaLaunchAttribute* attr, cudaStream_t stream) {
+inline cudaLaunchConfig_t oc_config(cudaLaunchAttribute* attr, cudaStream_t stream, int threads = OC_THREADS) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(OC_CTAS);
-    cfg.blockDim = dim3(OC_THREADS);
+    cfg.blockDim = dim3((unsigned)threads);
     cfg.stream = stream;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = OC_CTAS;
@@ -124,9 +134,9 @@ inline bool oc_fits() {
 }
 
 template <class Op>
-inline cudaError_t oc_launch(const Op& op, cudaStream_t stream) {
+inline cudaError_t oc_launch(const Op& op, cudaStream_t stream, int threads = OC_THREADS) {
     cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t cfg = oc_config<Op>(attr, stream);
+    const cudaLaunchConfig_t cfg = oc_config<Op>(attr, stream, threads);
     return cudaLaunchKernelEx(&cfg, one_cluster_kernel<Op>, op);
 }
 

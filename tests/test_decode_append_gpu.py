@@ -164,3 +164,9 @@ def test_lengths_advance_in_place(cuda, built_libs, B, Hq, Hkv):
     assert all(torch.equal(a, b) for a, b in zip(*res))
     p = positions.tolist()
     assert res[0][3].tolist() == [0 if x < 0 else min(x + 1, Smax) for x in p]
+
+
+@pytest.mark.parametrize("B,Hq,Hkv", [(1, 2, 1), (2, 32, 32), (3, 32, 32), (11, 32, 8), (37, 32, 8)])
+def test_small_steps_in_clusters_of_every_size(cuda, built_libs, B, Hq, Hkv):
+    # 16 items (one warp to a CTA), 768, 1152, 2112, 7104
+    test_codes_and_cache_rows_bit_exact(cuda, built_libs, B, Hq, Hkv, 96, 128)

@@ -22,3 +22,10 @@ def test_any_alignment_and_size(cuda, built_libs, n, offset):
     codes, scale, amax = O.quantize_f32(x.cpu().numpy())
     assert words.tolist() == [scale, amax]
     assert (q[:n].cpu().numpy() == codes).all() and (q[n:] == 0xAA).all()
+
+
+@pytest.mark.parametrize("n", [4088, 4095, 4096, 4104, 8192, 8200, 61440, 65528])
+def test_clusters_of_every_size(cuda, built_libs, n):
+    # 512 groups of 8 values are one warp to a CTA of the cluster
+    for offset in (0, 4):
+        test_any_alignment_and_size(cuda, built_libs, n, offset)
