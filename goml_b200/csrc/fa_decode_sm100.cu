@@ -21,9 +21,9 @@
 //  * A warp's next K block is on its way while it works on this block's softmax and V, and the next V block during the
 //    next block's scores (Little's law asks for about 45 KB in flight per SM).
 //
-// How the keys are divided (Plan below): a pair (sequence, kv head) may be cut between chunks; the pieces leave partial
-// states in a workspace and the CTA that finishes last merges them in a fixed order, so there is no second kernel and results
-// do not depend on timing: the same call gives the same bits, eager or in a graph, on whatever stream.
+// How the keys are divided (Plan below): a pair (sequence, kv head) may be cut between chunks; the pieces are the CTAs of a cluster and
+// hand their partial states to its first one, or leave them in a workspace where the CTA that finishes last takes them up.  Either merges them in
+// a fixed order, so there is no second kernel and results do not depend on timing: the same call gives the same bits, eager or in a graph, on whatever stream.
 //
 // STREAMS: the rounding of P to fp16 depends on the running maximum it is taken against, so which keys share a warp and
 // where a pair is cut show in the last bits of O.  A block that re-quantises its activations turns last bits into e4m3
@@ -35,6 +35,8 @@
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
+
+#include <mutex>
 
 #include "fa_fwd_sm100.h"
 #include "pdl.cuh"
@@ -49,6 +51,7 @@ constexpr int CHUNK = 64;        // keys per unit of work (page sizes are multip
 constexpr int THREADS = 128;
 constexpr int WARPS = THREADS / 32;
 constexpr float LAG = 6.0f;      // log2 units
+constexpr int MAX_CLUSTER = 16, PORTABLE_CLUSTER = 8;   // splits of a pair that are a cluster
 constexpr int HINTS = 2;         // chunks a CTA asks for ahead of the wait
 // A wide warp step takes twice the keys of a narrow one (8 against 4 KB in flight per warp) and leaves registers for 12
 // warps per SM instead of 16 (two column tiles: 8 instead of 12, or of 16 for D = 64).  It streams faster (0.8 GB of cache: 137 us against 146); the
@@ -95,7 +98,7 @@ __device__ __forceinline__ void ldg64(uint32_t* r, const uint8_t* p) {
 
 // Plans.
 //  SPLITS: CTA i is split i % splits of pair i / splits; a split is chunks_per_split chunks.  Few pairs: one resident CTA
-//          per split.  Many: one CTA per pair.
+//          per split, or a cluster per pair whose CTAs take equal runs of the splits.  Many: one CTA per pair.
 //  LINE:   the chunks of all pairs form one line that is cut into equal pieces, one per resident CTA, so sequences of very
 //          different lengths load all SMs alike.
 enum Plan : int { SPLITS, LINE };
@@ -113,6 +116,7 @@ struct DecodeParams {
     const float* sk;
     const float* sv;
     int plan, splits, chunks_per_split;
+    int cluster;   // CTAs of a pair, each with a run of its splits (CLUSTER)
     bool hints;   // on the line: ask for the first chunks ahead of the wait
     // paged cache: k, v are [num_pages, Hkv, page_size, D]; the chunk at key k0 of sequence b lives in page
     // block_table[b * max_pages + k0 / page_size]
@@ -174,19 +178,40 @@ __device__ __forceinline__ void prefetch_l2(const uint8_t* p, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
+// To the same place in the first CTA of the cluster
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t in_first(const float* p) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+    return a;
+}
+__device__ __forceinline__ void st_first(const float* p, const float4& v) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(in_first(p)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+__device__ __forceinline__ void st_first(const float* p, const float2& v) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(in_first(p)), "f"(v.x), "f"(v.y) : "memory");
+}
+
 struct Segment {
     int b, kvh, len;                // sequence, kv head, keys of the sequence
     int n_chunks, c_begin, c_end;   // chunks of the pair, and those of them this CTA takes
     int pair_u0;                    // unit of the line where the pair starts
 };
 
-template <int D, int NQ, bool WIDE, bool STREAMS, bool PAGED>
+// CLUSTER: the splits of a pair are the CTAs of a cluster (one query head per kv head)
+template <int D, int NQ, bool WIDE, bool STREAMS, bool PAGED, bool CLUSTER = false>
 __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_kernel(const DecodeParams p) {
     using C = Cfg<D, NQ, WIDE>;
-    __shared__ float s_o[WARPS][C::ROWS][C::PITCH];
+    static_assert(!CLUSTER || (STREAMS && NQ == 1), "clusters are for one query head per kv head");
+    __shared__ __align__(16) float s_o[WARPS][CLUSTER ? 1 : C::ROWS][C::PITCH];
     __shared__ float s_m[WARPS][C::ROWS], s_l[WARPS][C::ROWS];
     __shared__ Segment s_next[WARPS];
     __shared__ uint32_t s_last;
+    // CLUSTER: what the splits of the pair hand to its first CTA
+    __shared__ __align__(16) float s_part_o[CLUSTER ? MAX_CLUSTER : 1][CLUSTER ? D : 4];
+    __shared__ __align__(8) float s_part_ml[CLUSTER ? MAX_CLUSTER : 1][2];
+    if (CLUSTER) cluster_arrive();   // its phase says that every CTA runs, so that its shared memory may be written
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;              // MMA fragment coordinates
@@ -269,13 +294,19 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
     auto find_piece = [&](const bool early) {
         seg.b = seg.kvh = seg.len = seg.n_chunks = seg.c_begin = seg.c_end = seg.pair_u0 = 0;
         if (!line) {
-            const int pair = blockIdx.x / p.splits, split = blockIdx.x - pair * p.splits;
+            const int per_pair = CLUSTER ? p.cluster : p.splits;
+            const int pair = blockIdx.x / per_pair, split = blockIdx.x - pair * per_pair;
             seg.b = pair / p.hkv;
             seg.kvh = pair - seg.b * p.hkv;
             seg.len = seq_len_of(p, seg.b);
             seg.n_chunks = chunks_of(seg.len);
-            seg.c_begin = split * p.chunks_per_split;
-            seg.c_end = min(seg.n_chunks, seg.c_begin + p.chunks_per_split);
+            int each = p.chunks_per_split;
+            if (CLUSTER) {   // the splits that the sequence has, in equal runs
+                const int used = (seg.n_chunks + each - 1) / each;
+                each *= (used + p.cluster - 1) / p.cluster;
+            }
+            seg.c_begin = split * each;
+            seg.c_end = min(seg.n_chunks, seg.c_begin + each);
             if (seg.n_chunks == 0 && seg.kvh == 0 && split == 0 && threadIdx.x == 0) empty_sequence(seg.b);
         } else {
 #pragma unroll
@@ -433,7 +464,30 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
             for (int i = 0; i < C::MT; i++) acc[n][i][0] = acc[n][i][1] = acc[n][i][2] = acc[n][i][3] = 0.f;
         }
 
+        // CLUSTER: the same of the splits before this one, of the only query
+        float m_all = -INFINITY, l_all = 0.f, acc_all[CLUSTER ? C::MT : 1][2] = {};
+        auto end_of_split = [&] {
+            const float top = fmaxf(m_all, m[0][0]);
+            if (top == -INFINITY) return;
+            const float f0 = ex2f(m_all - top), f1 = ex2f(m[0][0] - top);
+            m_all = top;
+            l_all = l_all * f0 + l[0][0] * f1;
+#pragma unroll
+            for (int j = 0; j < (CLUSTER ? C::MT : 0); j++) {
+                acc_all[j][0] = acc_all[j][0] * f0 + acc[0][j][0] * f1;
+                acc_all[j][1] = acc_all[j][1] * f0 + acc[0][j][2] * f1;
+                acc[0][j][0] = acc[0][j][2] = 0.f;
+            }
+            m[0][0] = -INFINITY;
+            l[0][0] = 0.f;
+        };
+        int split_end = CLUSTER ? seg.c_begin + p.chunks_per_split : 0;
+
         for (int c = seg.c_begin; c < seg.c_end; c += C::TILES) {
+            if (CLUSTER && c == split_end) {   // P is rounded against the maximum of its own split
+                end_of_split();
+                split_end += p.chunks_per_split;
+            }
             // ---- S^T = K Q^T, one accumulator per k-step: independent MMAs instead of a chain
             float s[NQ][C::TILES][4];
 #pragma unroll
@@ -554,6 +608,16 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
         }
 
         // ---- merge the four warps' states
+        if (CLUSTER) {
+            end_of_split();
+            m[0][0] = m_all;
+            l[0][0] = l_all;
+#pragma unroll
+            for (int j = 0; j < (CLUSTER ? C::MT : 0); j++) {
+                acc[0][j][0] = acc_all[j][0];
+                acc[0][j][2] = acc_all[j][1];
+            }
+        }
         const bool whole = seg.c_begin == 0 && seg.c_end == seg.n_chunks;
 #pragma unroll
         for (int n = 0; n < NQ; n++)
@@ -569,10 +633,11 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
                 if (row < p.group) {
 #pragma unroll
                     for (int j = 0; j < C::MT; j++)
-                        *reinterpret_cast<float2*>(&s_o[warp][row][(D / 8) * g + 2 * j]) = make_float2(acc[n][j][e], acc[n][j][e + 2]);
+                        *reinterpret_cast<float2*>(&s_o[warp][CLUSTER ? 0 : row][(D / 8) * g + 2 * j]) = make_float2(acc[n][j][e], acc[n][j][e + 2]);
                 }
             }
         __syncthreads();
+        if (CLUSTER && !whole) cluster_wait();
         // slots of a cut pair: its splits in order, or on the line the odd slot of the CTA that has its first piece and the
         // even slots of the CTAs after that
         const int slot = !line ? blockIdx.x : 2 * blockIdx.x + (seg.c_begin == 0 ? 1 : 0);
@@ -587,15 +652,40 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
 #pragma unroll
             for (int w = 0; w < WARPS; w++) {
                 const float mw = s_m[w][row];
-                fold(L, O, s_l[w][row], *reinterpret_cast<const float4*>(&s_o[w][row][col]), mw == -INFINITY ? 0.f : ex2f(mw - M));
+                fold(L, O, s_l[w][row], *reinterpret_cast<const float4*>(&s_o[w][CLUSTER ? 0 : row][col]), mw == -INFINITY ? 0.f : ex2f(mw - M));
             }
             if (whole) {
                 store_out<D>(p, ((size_t)b * p.hq + (size_t)kvh * p.group + row), col, M, L, O, vds);
+            } else if (CLUSTER) {
+                const int split = blockIdx.x - (blockIdx.x / p.cluster) * p.cluster;
+                st_first(&s_part_o[split][col], O);
+                if (col == 0) st_first(s_part_ml[split], make_float2(M, L));
             } else {
                 const size_t at = (size_t)slot * C::ROWS + row;
                 __stcg(reinterpret_cast<float4*>(p.ws_o + at * D + col), O);
                 if (col == 0) __stcg(reinterpret_cast<float2*>(p.ws_ml + at * 2), make_float2(M, L));
             }
+        }
+        if (CLUSTER) {
+            if (whole) return;
+            __syncwarp();
+            cluster_arrive();
+            if (seg.c_begin != 0) return;   // what it has handed over is the first one's
+            cluster_wait();
+            // A column to a thread, the pieces in order
+            const int parts = (seg.n_chunks + seg.c_end - 1) / seg.c_end;
+            float M = -INFINITY;
+            for (int i = 0; i < parts; i++) M = fmaxf(M, s_part_ml[i][0]);
+            if (threadIdx.x < D / 4) {
+                float L = 0.f;
+                float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+                const int col = threadIdx.x * 4;
+#pragma unroll 4
+                for (int i = 0; i < parts; i++)
+                    fold(L, O, s_part_ml[i][1], *reinterpret_cast<const float4*>(&s_part_o[i][col]), M == -INFINITY ? 0.f : ex2f(s_part_ml[i][0] - M));
+                store_out<D>(p, (size_t)b * p.hq + kvh, col, M, L, O, vds);
+            }
+            return;
         }
         if (!whole) {
             int parts, slot0, slot_step;   // the pair's pieces: slot0, then slot0 + 1 + i * slot_step
@@ -617,7 +707,56 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
                 if (s_last) p.arrivals[bh] = 0;   // for the next launch
             }
             __syncthreads();
-            if (s_last) {
+            if (s_last && STREAMS) {
+                // one row: a group of D / 4 threads takes every GROUPS-th piece, eight loads in flight, and the groups' states meet in shared memory
+                __threadfence();
+                constexpr int LANES = D / 4, GROUPS = THREADS / LANES;
+                const int group = threadIdx.x / LANES, col = threadIdx.x % LANES * 4;
+                float M = -INFINITY, L = 0.f;
+                float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int i0 = group; i0 < parts; i0 += 8 * GROUPS) {
+                    float2 ml[8];
+                    float4 oi[8];
+#pragma unroll
+                    for (int k = 0; k < 8; k++) {
+                        const int i = i0 + k * GROUPS;
+                        ml[k] = make_float2(-INFINITY, 0.f);
+                        oi[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (i >= parts) continue;
+                        const size_t at = (size_t)(slot0 + i) * C::ROWS;
+                        ml[k] = __ldcg(reinterpret_cast<const float2*>(p.ws_ml + at * 2));
+                        oi[k] = __ldcg(reinterpret_cast<const float4*>(p.ws_o + at * D + col));
+                    }
+                    float M2 = M;
+#pragma unroll
+                    for (int k = 0; k < 8; k++) M2 = fmaxf(M2, ml[k].x);
+                    if (M2 == -INFINITY) continue;
+                    const float f = ex2f(M - M2);
+                    L *= f;
+                    O.x *= f; O.y *= f; O.z *= f; O.w *= f;
+#pragma unroll
+                    for (int k = 0; k < 8; k++) fold(L, O, ml[k].y, oi[k], ex2f(ml[k].x - M2));
+                    M = M2;
+                }
+                float(*const rows)[C::PITCH] = &s_o[0][0];   // GROUPS of them
+                *reinterpret_cast<float4*>(&rows[group][col]) = O;
+                if (col == 0) {
+                    s_m[0][group] = M;
+                    s_l[0][group] = L;
+                }
+                __syncthreads();
+                if (group == 0) {
+                    float top = -INFINITY;
+#pragma unroll
+                    for (int i = 0; i < GROUPS; i++) top = fmaxf(top, s_m[0][i]);
+                    L = 0.f;
+                    O = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int i = 0; i < GROUPS; i++)
+                        fold(L, O, s_l[0][i], *reinterpret_cast<const float4*>(&rows[i][col]), s_m[0][i] == -INFINITY ? 0.f : ex2f(s_m[0][i] - top));
+                    store_out<D>(p, (size_t)b * p.hq + kvh, col, top, L, O, vds);
+                }
+            } else if (s_last) {
                 __threadfence();
                 for (int idx = threadIdx.x; idx < p.group * (D / 4); idx += THREADS) {
                     const int row = idx / (D / 4), col = idx % (D / 4) * 4;
@@ -677,10 +816,64 @@ __global__ void clear_words_kernel(uint32_t* w, uint32_t n) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) w[i] = 0;
 }
 
+// Kernels whose splits are a cluster: [paged][head dim 128]
+using DecodeKernel = void (*)(const DecodeParams);
+DecodeKernel cluster_kernel(int hd, bool paged) {
+    if (hd == 64) return paged ? fa_decode_kernel<64, 1, false, true, true, true> : fa_decode_kernel<64, 1, false, true, false, true>;
+    return paged ? fa_decode_kernel<128, 1, false, true, true, true> : fa_decode_kernel<128, 1, false, true, false, true>;
+}
+cudaLaunchConfig_t cluster_config(cudaLaunchAttribute* attr, int grid, int size, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(THREADS);
+    cfg.stream = stream;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)size;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cfg;
+}
+// Clusters of each size that are resident at once on the current device (the least of the kernels'; asked once per device)
+struct ClusterFit {
+    int n[MAX_CLUSTER + 1] = {};
+};
+const ClusterFit& cluster_fit() {
+    static ClusterFit known[64], none;
+    static std::once_flag asked[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return none;
+    std::call_once(asked[dev], [&] {
+        ClusterFit f;
+        for (int size = 2; size <= MAX_CLUSTER; size++) {
+            int least = 1 << 30;
+            for (int k = 0; k < 4; k++) {
+                const DecodeKernel kernel = cluster_kernel(k & 1 ? 128 : 64, k & 2);
+                cudaLaunchAttribute attr[2];
+                cudaLaunchConfig_t cfg = cluster_config(attr, size, size, nullptr);
+                cfg.numAttrs = 1;
+                int n = 0;
+                if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+                    cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+                    (void)cudaGetLastError();
+                    n = 0;
+                }
+                least = n < least ? n : least;
+            }
+            f.n[size] = least;
+        }
+        known[dev] = f;
+    });
+    return known[dev];
+}
+
 struct Layout {
     int plan, splits, grid, rows;
     bool streams, wide;
-    bool cuts() const { return plan != SPLITS || splits > 1; }   // whether a pair may be cut
+    int cluster;   // 0: none
+    bool cuts() const { return plan != SPLITS || (splits > 1 && !cluster); }   // whether the pieces of a pair meet in a workspace
 };
 // One query head per kv head keeps the streams: fixed splits while the pairs leave room for them, else a CTA per pair, which
 // the hardware hands out as CTAs end, so uneven lengths balance by themselves.  (The freely cut line, with a CTA taking up the
@@ -710,14 +903,32 @@ Layout layout_of(int batch, int q_heads, int kv_heads, int head_dim, int span) {
     const long long pairs = (long long)batch * kv_heads, chunks = ((long long)span + CHUNK - 1) / CHUNK;
     const long long narrow = (long long)ctas_per_sm(head_dim, 1, false) * sms, wide = (long long)ctas_per_sm(head_dim, x.rows / 8, true) * sms;
     x.splits = 1;
+    x.cluster = 0;
     x.wide = !x.streams;
     if (x.streams && pairs <= narrow) {
         long long splits = narrow / pairs;
         if (splits > chunks) splits = chunks;
         if (splits > 64) splits = 64;
         x.splits = splits < 1 ? 1 : (int)splits;
+        // Splits in clusters, of up to eight CTAs or of sizes that only some GPUs place: the largest that has room (112 pairs of 900 keys in as many
+        // clusters of 5 as fit 12.3 us, workspace 10.8), and 8 rather than more.  A CTA takes several splits in turn, which must not cost more
+        // chunks in turn than the workspace's merge costs time.
+        // Us, workspace / cluster: 32 pairs of 1000 keys 6.6 / 5.7 (of 64 6.1 / 4.5), of 100 5.0 / 4.1; 16 of 2000 7.4 / 6.6; 96 of 500 7.9 / 6.8; 112 of 900 10.7 /
+        // 9.8; but where a split has several chunks and a CTA would take two, 32 of 2000 9.0 / 9.4, 192 of 500 9.7 / 12.4.
+        // Fewer than 16 pairs keep the workspace although a cluster is faster there too (8 pairs of 1000 keys 5.6 / 4.4): what such a call leaves
+        // in a graph is held to be allocations and a clearing kernel (tests/test_fa_scratch_gpu.py).
+        const ClusterFit& fit = cluster_fit();
+        const long long each = (chunks + x.splits - 1) / x.splits, used = each ? (chunks + each - 1) / each : 0;
+        auto placed = [&](long long n) { return n > PORTABLE_CLUSTER ? 8 * pairs <= 7 * fit.n[n] : n > 3 ? 16 * pairs <= 15 * fit.n[n] : pairs <= fit.n[n]; };
+        auto steps_of = [&](long long n) { return (used + n - 1) / n * each; };
+        long long size = used < MAX_CLUSTER ? used : MAX_CLUSTER;
+        while (size > 1 && !placed(size)) size--;
+        if (size > PORTABLE_CLUSTER && placed(PORTABLE_CLUSTER) && steps_of(PORTABLE_CLUSTER) <= steps_of(size) + 1) size = PORTABLE_CLUSTER;
+        while (size > PORTABLE_CLUSTER && steps_of(size - 1) == steps_of(size)) size--;
+        // (a cache is rarely full to its last split: 64 pairs of 1000 keys in a cache of 1064 have 8 of 9, 8.4 / 7.6)
+        if (pairs >= 16 && size > 1 && (steps_of(size) <= (each == 1 ? 3 : each + 1) || used <= size + size / 8)) x.cluster = (int)size;
         x.plan = SPLITS;
-        x.grid = (int)(pairs * x.splits);
+        x.grid = (int)(pairs * (x.cluster ? x.cluster : x.splits));
     } else if (x.streams || 2 * pairs >= (x.rows == 8 ? 6 : 3) * wide || (chunks <= 32 && 5 * pairs >= 4 * wide) || pairs * chunks > 0x7fffffffLL) {
         x.plan = SPLITS;
         x.grid = (int)pairs;
@@ -758,7 +969,7 @@ cudaError_t launch_decode(const DecodeArgs& a) {
     p.scale_log2 = a.scale * 1.4426950408889634f;
     p.v_descale = a.v_descale;
     p.sq = a.scale_q_dev; p.sk = a.scale_k_dev; p.sv = a.scale_v_dev;
-    p.plan = x.plan; p.splits = x.splits; p.hints = !a.behind_clear;
+    p.plan = x.plan; p.splits = x.splits; p.cluster = x.cluster; p.hints = !a.behind_clear;
     p.chunks_per_split = (int)((((long long)span + CHUNK - 1) / CHUNK + x.splits - 1) / x.splits);
     p.block_table = a.block_table;
     p.page_mul = p.page_shr = 0;
@@ -772,6 +983,11 @@ cudaError_t launch_decode(const DecodeArgs& a) {
     p.ws_o = static_cast<float*>(a.workspace);
     p.ws_ml = p.ws_o + (size_t)x.grid * 2 * x.rows * a.hd;
     p.arrivals = a.arrivals;
+    if (x.cluster) {
+        cudaLaunchAttribute attr[2];
+        const cudaLaunchConfig_t cfg = cluster_config(attr, x.grid, x.cluster, a.stream);
+        return cudaLaunchKernelEx(&cfg, cluster_kernel(a.hd, a.block_table != nullptr), p);
+    }
     auto run = [&](auto contiguous, auto paged) { return launch_pdl(a.block_table ? paged : contiguous, x.grid, THREADS, 0, a.stream, p); };
 #define KERNEL(D, NQ, WIDE, STREAMS) run(fa_decode_kernel<D, NQ, WIDE, STREAMS, false>, fa_decode_kernel<D, NQ, WIDE, STREAMS, true>)
     if (x.streams) return a.hd == 64 ? KERNEL(64, 1, false, true) : x.wide ? KERNEL(128, 1, true, true) : KERNEL(128, 1, false, true);

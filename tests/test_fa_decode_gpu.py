@@ -243,3 +243,43 @@ def test_capacity_far_above_what_is_held(cuda, built_libs, fa_ctx, B, Hq, Hkv, D
     maxabs, meanrel = O.error_stats(got[some], ref[some])
     assert maxabs <= 2e-2 and meanrel <= 1e-2, (maxabs, meanrel)
     assert np.abs(glse[some] - rl[some]).max() <= 5e-3
+
+
+@pytest.mark.parametrize("B,H,Smax,D,cluster", [(1, 16, 100, 64, True), (9, 32, 200, 64, True), (5, 16, 900, 64, True), (3, 16, 500, 128, True), (1, 32, 1064, 128, True),
+                                                (1, 16, 2000, 64, True), (1, 32, 3000, 128, False), (1, 16, 2500, 64, False), (1, 9, 4100, 128, False)])
+def test_splits_in_clusters_and_in_the_workspace(cuda, built_libs, fa_ctx, B, H, Smax, D, cluster):
+    # clusters of 2 to 16 CTAs with runs of one to three splits, and up to 64 splits that meet in the workspace: whole and part chunks, fewer than CTAs, none; the
+    # paged cache has the same bits
+    from tests.gpu_util import kernels
+    q, k, v, sq, sk, sv = make_case(f"cluster{B}_{H}_{Smax}_{D}", B, H, H, Smax, D)
+    rng = np.random.default_rng(Smax)
+    scale = sq * sk / math.sqrt(D)
+    sets = [rng.integers(1, Smax + 1, size=B) for _ in range(2)] + [np.full(B, n) for n in (Smax, 1, 64, 65, 0)]
+    per_seq = -(-Smax // 64)
+    pad = np.zeros((B, H, per_seq * 64, D), np.uint8)
+    table = rng.permutation(B * per_seq).reshape(B, per_seq).astype(np.int32)
+    pools = []
+    for cache in (k, v):
+        pad[:, :, :Smax] = cache
+        pool = np.empty((B * per_seq, H, 64, D), np.uint8)
+        pool[table.ravel()] = pad.reshape(B, H, per_seq, 64, D).transpose(0, 2, 1, 3, 4).reshape(-1, H, 64, D)
+        pools.append(torch.from_numpy(pool).cuda())
+    qd, td = torch.from_numpy(q).cuda(), torch.from_numpy(table).cuda()
+    for n, lens in enumerate(sets):
+        got, lse = run_decode(fa_ctx, q, k, v, lens, scale, sv)
+        o = torch.full((B, H, D), float("nan"), dtype=torch.float16, device="cuda")
+        ld = torch.from_numpy(np.asarray(lens, np.int32)).cuda()
+        call = lambda: fa_ctx.Decode(qd.data_ptr(), pools[0].data_ptr(), pools[1].data_ptr(), o.data_ptr(), 0, ld.data_ptr(), B, H, H, D, 0, 0, scale, sv,
+                                     stream=torch.cuda.current_stream().cuda_stream, block_table=td.data_ptr(), page_size=64, max_pages_per_seq=per_seq, num_pages=B * per_seq)
+        call()
+        torch.cuda.synchronize()
+        assert np.array_equal(o.double().cpu().numpy(), got)
+        if n == 0:
+            assert len(kernels(call)) == (1 if cluster else 2)   # the workspace's words are cleared by another
+        if not lens.any():
+            assert (got == 0).all() and np.isneginf(lse).all()
+            continue
+        ref, rl = glue.decode_attention_f64(q, k, v, lens, scale, sv)
+        maxabs, meanrel = O.error_stats(got, ref)
+        assert maxabs <= 2e-2 and meanrel <= 1e-2, (lens, maxabs, meanrel)
+        assert np.abs(lse - rl).max() <= 5e-3
