@@ -132,6 +132,7 @@ struct Params {
     uint32_t v_epoch;
     int v_chunks;              // chunks per head
     int group;                 // heads whose tiles are interleaved
+    int few;                   // the launch leaves SMs free: the next kernel may come at once
 };
 
 __device__ __forceinline__ float ex2(float x) {
@@ -434,7 +435,13 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     const uint32_t tmem_s = tmem_base;
     const uint32_t tmem_o = tmem_base + C::O_COL;
     const bool bad_start = (*abort_flag != 0);
-    if (VRAW) pdl_wait();   // no pre-pass has waited for what is ahead
+    if (VRAW) {
+        pdl_wait();   // no pre-pass has waited for what is ahead
+        // The next kernel's start (its launch, barriers, tensor memory) beside this one, where a launch leaves SMs free: 4 heads of 256 keys, not causal, 5.31 / 4.98
+        // us a call, of 128, causal, 5.04 / 4.67, 12 of 1000 12.9 / 12.6; with more CTAs than SMs 9.7 / 9.9.  D = 128 loses by it (4 of 256 5.8 / 6.1, 24
+        // of 700 11.7 / 12.5), and with the trigger ahead of the rows out (32 of 512 9.7 / 9.9).
+        if (HD == 64 && !WALK && p.few) pdl_trigger();
+    }
     if (bad_start) {
         // fall through to teardown
     } else if (warp >= NUM_SOFTMAX_WARPS) {
@@ -992,7 +999,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     tc_fence_before();
     __syncthreads();
     // Triggered at the end of a CTA, not at its start: the next call's pre-pass is spread over the SMs that have room when
-    // it is launched, and during this kernel's last wave those are few (S = 2048 causal: 525 us a call against 343).
+    // it is launched, and during this kernel's last wave those are few (S = 2048 causal: 525 us a call against 343).  (Few tiles of D = 64: above.)
     pdl_trigger();
     const uint32_t code = *abort_flag;
     if (code != 0) {
@@ -1084,6 +1091,7 @@ cudaError_t launch_hd(const LaunchArgs& a, int num_sms) {
         return cudaErrorInvalidValue;
     Params p;
     p.group = heads_together(a, grid, num_sms);
+    p.few = grid <= num_sms;
     p.bh = a.bh; p.sl = a.sl; p.n_qtiles = (a.sl + BM - 1) / BM;
     p.causal = a.causal; p.window = a.window;
     p.scale_log2 = a.scale * 1.4426950408889634f;
