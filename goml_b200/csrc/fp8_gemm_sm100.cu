@@ -46,7 +46,7 @@ constexpr int STAGING_BYTES = 4 * 2 * STAGING_BOX;
 // tensor-efficient shape (the MMA reads (128+BN)*32 operand bytes per BN/2 clocks, within the
 // 128 B/clk shared-memory read rate only for BN >= 128); 128 and 64 exist so that small and
 // skinny problems (few 128x256 tiles) still spread over all SMs — those are HBM/latency-bound,
-// and a narrower tile leaves room for a deeper TMA ring.
+// and a narrower tile leaves room for a deeper TMA ring.  192 fills waves that 256 leaves half empty.
 // MT = 2: a CTA works on a pair of vertically adjacent tiles (256 rows) that share every B tile it loads.
 template <int BN, int MT = 1>
 struct Tile {
@@ -56,8 +56,8 @@ struct Tile {
     static constexpr int KSUB = (BN == 64) ? 2 : 1;
     static constexpr int SUB_BYTES = MT * A_BYTES + B_BYTES;
     static constexpr int STAGE_BYTES = KSUB * SUB_BYTES;
-    static constexpr int STAGES = (MT == 2) ? 3 : (BN == 256) ? 4 : (BN == 128) ? 6 : 4;
-    static constexpr int TMEM_COLS = 2 * BN;  // two accumulator buffers (a power of two >= 32)
+    static constexpr int STAGES = (MT == 2) ? 3 : (BN == 128) ? 6 : 4;
+    static constexpr int TMEM_COLS = BN == 192 ? 512 : 2 * BN;  // two accumulator buffers, in a power of two >= 32
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STAGING_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 };
 
@@ -657,7 +657,21 @@ __global__ void __launch_bounds__(32) gemm_wait_expiry_selftest_kernel() {
 
 // ---------------------------------------------------------------- host side
 
-constexpr int Tile_KSUB(int bn) { return bn == 256 ? Tile<256>::KSUB : bn == 128 ? Tile<128>::KSUB : Tile<64>::KSUB; }
+// What a wave of work units of each shape takes, for problems of at least two rows of tiles: start + waves x (k-blocks x block + end), us, fitted to 110
+// problems of 193 to 6000 rows with 1024 to 22016 columns and K of 1024 to 11008, each shape of unit timed on each (15 % off in the mean, alike for
+// all shapes).  Where it promises a margin it overrides the rule of widths and pairs alone; on 500 other problems of these ranges that is 2.8 % in the
+// mean, up to a quarter where it takes another shape: 3304 x 4096 x 8528 125.7 -> 102.3 us (192-wide pairs), 2538 x 5936 x 3184 62.0 -> 50.5 (256-wide pairs),
+// 4212 x 1472 x 5616 48.6 -> 37.0, 1024 x 5000 x 6000 50.1 -> 38.7, 700 x 8192 x 8192 47.4 -> 41.2, 512 x 5000 x 6000 32.4 -> 27.5 (192-wide tiles).
+struct UnitCost {
+    int bn, mt;
+    float start, block, end;
+};
+constexpr UnitCost UNIT_COSTS[] = {{256, 1, 4.0f, 0.464f, 0.79f}, {256, 2, 0.6f, 0.706f, 5.9f}, {192, 1, 3.8f, 0.408f, 0.44f},
+                                   {192, 2, 1.6f, 0.611f, 3.7f},  {128, 1, 4.1f, 0.318f, 0.27f}, {64, 1, 4.0f, 0.229f, 0.18f}};
+// a last wave of half-width units; of fewer than 16 k-blocks; and of whole ones on a share of the SMs, which get more of the memory each
+constexpr float HALF_WAVE = 0.6f, HALF_WAVE_SHORT = 0.45f, PART_WAVE = 0.7f;
+
+constexpr int Tile_KSUB(int bn) { return bn == 192 ? Tile<192>::KSUB : bn == 256 ? Tile<256>::KSUB : bn == 128 ? Tile<128>::KSUB : Tile<64>::KSUB; }
 
 struct DeviceState {
     std::once_flag once;      // first call on this device, from whichever host thread gets there first
@@ -691,6 +705,10 @@ void init_device(DeviceState* st, int dev) {
                                   Tile<256>::SMEM_BYTES)) != cudaSuccess) { st->init_error = e; return; }
     if ((e = cudaFuncSetAttribute(fp8_gemm_tcgen05_kernel<256, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   Tile<256, 2>::SMEM_BYTES)) != cudaSuccess) { st->init_error = e; return; }
+    if ((e = cudaFuncSetAttribute(fp8_gemm_tcgen05_kernel<192>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  Tile<192>::SMEM_BYTES)) != cudaSuccess) { st->init_error = e; return; }
+    if ((e = cudaFuncSetAttribute(fp8_gemm_tcgen05_kernel<192, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  Tile<192, 2>::SMEM_BYTES)) != cudaSuccess) { st->init_error = e; return; }
     if ((e = cudaFuncSetAttribute(fp8_gemm_tcgen05_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   Tile<128>::SMEM_BYTES)) != cudaSuccess) { st->init_error = e; return; }
     if ((e = cudaFuncSetAttribute(fp8_gemm_tcgen05_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -772,6 +790,35 @@ int launch(int M, int N, int K, const void* A, const void* B, void* C, float alp
         const long long pair_cost = ((pairs + st.num_sms - 1) / st.num_sms) * 2 * 92;
         if (pair_cost > single_cost) pair = false;
     }
+    // K is cut (below) where that leaves few units; else the shape may be chosen by what its waves cost.  Tiles of 192 columns hold no whole
+    // number of the boxes that activations and e4m3 results leave in.  A promise of 4 % is kept (16 % with SwiGLU, whose longer end the fit does not
+    // know: 410 x 16320 x 4096 in pairs promises 14 % and takes 31.5 us for 30.8).  Results that leave through no tensor map have an end several times as long, which pairs pay in full (6820 x 2331 x 4640 85 us, in 192-wide
+    // pairs 99; 820 x 7262 x 10736 added 220 / 291): they keep the old shape.
+    const long long units_now = (pair ? (m_tiles + 1) / 2 : m_tiles) * ((N + bn - 1) / bn);
+    const bool cuts_k = p.x_tma && 2 * units_now <= st.num_sms;
+    const bool mapped = X ? p.x_tma : H ? F % 8 == 0 : D8 ? N % 16 == 0 : N % 8 == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+    if (m_tiles >= 2 && !cuts_k && mapped) {
+        auto cost = [&](const UnitCost& c) {
+            const long long units = (m_tiles + c.mt - 1) / c.mt * ((N + c.bn - 1) / c.bn), full = units / st.num_sms, rem = units % st.num_sms;
+            const bool halves = c.bn == 256 && c.mt == 1 && full > 0 && 2 * rem <= st.num_sms;
+            const float last = halves ? (K < 16 * BK ? HALF_WAVE_SHORT : HALF_WAVE) : full == 0 ? 1.f : PART_WAVE + (1.f - PART_WAVE) * (float)rem / (float)st.num_sms;
+            const float waves = (float)full + (rem == 0 ? 0.f : last);
+            const float end = X && c.mt == 2 ? 1.5f * c.end : c.end;   // fp32 rows of both tiles (4334 x 7584 x 6272 added 162 us, in 256-wide pairs 171)
+            return c.start + waves * ((float)((K + BK - 1) / BK) * c.block + end);
+        };
+        const UnitCost* take = nullptr;
+        float now = 0.f, least = 0.f;
+        for (const UnitCost& c : UNIT_COSTS) {
+            if ((c.mt == 2 && pair_policy() == 0) || (c.bn == 192 && (H || D8))) continue;
+            const float t = cost(c);
+            if (c.bn == bn && c.mt == (pair ? 2 : 1)) now = t;
+            if (!take || t < least) { take = &c; least = t; }
+        }
+        if (take && least < (H ? 0.84f : 0.96f) * now) {
+            bn = take->bn;
+            pair = take->mt == 2;
+        }
+    }
     p.c_tma = (C && !X && !H && !D8 && (N % 8) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) ? 1 : 0;
     p.h_tma = (H && bn >= 128 && (F % 8) == 0 && (reinterpret_cast<uintptr_t>(H) & 15) == 0) ? 1 : 0;
     p.d_tma = (D8 && !H && !X && bn >= 128 && (N % 16) == 0 && (reinterpret_cast<uintptr_t>(D8) & 15) == 0) ? 1 : 0;
@@ -793,7 +840,7 @@ int launch(int M, int N, int K, const void* A, const void* B, void* C, float alp
     // partial sum (the order of those fp32 additions is then not fixed from run to run).
     const int k_stages = (p.k_blocks + Tile_KSUB(bn) - 1) / Tile_KSUB(bn);
     p.ksplit = 1;
-    if (p.x_tma && !split_tail && 2 * tiles <= st.num_sms) {
+    if (cuts_k && !split_tail) {
         long long ks = st.num_sms / tiles;
         if (ks > k_stages / 4) ks = k_stages / 4;   // at least four pipeline stages of work per slice
         if (ks > 8) ks = 8;
@@ -819,8 +866,10 @@ int launch(int M, int N, int K, const void* A, const void* B, void* C, float alp
 
     const int grid = (int)(p.num_units < st.num_sms ? p.num_units : st.num_sms);
     auto start = [&](auto kernel, size_t smem) { return (int)launch_pdl(kernel, dim3(grid), dim3(NUM_THREADS), smem, stream, ta, tb, tbh, tx, p); };
+    if (pair && bn == 192) return start(fp8_gemm_tcgen05_kernel<192, 2>, Tile<192, 2>::SMEM_BYTES);
     if (pair) return start(fp8_gemm_tcgen05_kernel<256, 2>, Tile<256, 2>::SMEM_BYTES);
     if (bn == 256) return start(fp8_gemm_tcgen05_kernel<256>, Tile<256>::SMEM_BYTES);
+    if (bn == 192) return start(fp8_gemm_tcgen05_kernel<192>, Tile<192>::SMEM_BYTES);
     if (bn == 128) return start(fp8_gemm_tcgen05_kernel<128>, Tile<128>::SMEM_BYTES);
     return start(fp8_gemm_tcgen05_kernel<64>, Tile<64>::SMEM_BYTES);
 }

@@ -68,6 +68,45 @@ def test_added_to_fp32_by_the_kernel_that_cuts_a_long_k_best(cuda, built_libs, M
     assert (room[:16 + offset] == 7).all() and (room[16 + offset + M * N:] == 7).all()
 
 
+@pytest.mark.parametrize("M,N,K,variant", [(512, 5000, 2048, "Li192ELi1"), (390, 5000, 2064, "Li192ELi1"), (1024, 5000, 6000, "Li192ELi2"), (900, 5184, 6000, "Li192ELi2"),
+                                           (700, 8192, 4096, "Li192ELi2"), (1500, 5000, 4096, "Li256ELi2")])
+def test_units_that_fill_their_waves(cuda, built_libs, M, N, K, variant):
+    # tiles and pairs of 192 columns: last pairs half empty, last columns of less than a tile; 16-bit results of both types, added to fp32, and the bits
+    # that single tiles of 256 columns give
+    from goml_b200 import fp8_gemm as G
+    stream = lambda: torch.cuda.current_stream().cuda_stream
+    exact(M, N, K)
+    exact(M, N, K, 0, "bf16")
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a, b = (torch.randint(0, 0x78, (rows, K), generator=g, dtype=torch.uint8, device="cuda") for rows in (M, N))
+    s = torch.tensor([3e-3, 2e-3], device="cuda")
+    x0 = torch.randn(M, N, generator=g, device="cuda")
+
+    def outputs():
+        c, x = torch.empty(M, N, dtype=torch.bfloat16, device="cuda"), x0.clone()
+        calls = [lambda: G.FP8GEMMScaled(M, N, K, a.data_ptr(), b.data_ptr(), c.data_ptr(), 1.0, s.data_ptr(), s.data_ptr() + 4, G.OutBF16, stream()),
+                 lambda: G.FP8GEMMAccumulateF32(M, N, K, a.data_ptr(), b.data_ptr(), x.data_ptr(), 1.0, s.data_ptr(), s.data_ptr() + 4, stream())]
+        names = [n for call in calls for n in kernels(call)]
+        for call in calls:
+            call()
+        torch.cuda.synchronize()
+        assert G.device_status() == 0
+        return names, c, x
+
+    names, c, x = outputs()
+    assert len(names) == 2 and all(f"tcgen05_kernelI{variant}E" in n for n in names)
+    G.SetTilePairs(0)
+    try:
+        others, c1, x1 = outputs()
+    finally:
+        G.SetTilePairs(-1)
+    assert all("ELi1E" in n for n in others)
+    assert torch.equal(c, c1) and torch.equal(x, x1)
+    # rows that leave through no tensor map keep the shape that they had
+    name, = kernels(lambda: G.FP8GEMMScaled(M, N - 1, K, a.data_ptr(), b.data_ptr(), c.data_ptr(), 1.0, 0, 0, G.OutBF16, stream()))
+    assert "Li192" not in name
+
+
 @pytest.mark.parametrize("split,K", [(1, 384), (2, 512), (3, 880), (4, 1024), (5, 6400), (6, 7696), (7, 8960), (8, 10240)])
 @pytest.mark.parametrize("N", [200, 131])
 def test_sums_handed_to_their_owners_and_fetched_are_the_same(cuda, built_libs, split, K, N):
