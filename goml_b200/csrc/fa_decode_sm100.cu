@@ -484,7 +484,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
         int split_end = CLUSTER ? seg.c_begin + p.chunks_per_split : 0;
 
         for (int c = seg.c_begin; c < seg.c_end; c += C::TILES) {
-            if (CLUSTER && c == split_end) {   // P is rounded against the maximum of its own split
+            if (CLUSTER && C::TILES == 1 && c == split_end) {   // P is rounded against the maximum of its own split; with two tiles a step, below
                 end_of_split();
                 split_end += p.chunks_per_split;
             }
@@ -540,6 +540,10 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
 #pragma unroll
             for (int i = 0; i < C::TILES; i++) {
                 const int ci = c + tile_chunk(i);
+                if (CLUSTER && C::TILES > 1 && ci == split_end) {
+                    end_of_split();
+                    split_end += p.chunks_per_split;
+                }
                 const int key0 = ci * CHUNK + tile_key(i), key_end = ci < seg.c_end ? seg.len : 0;
                 if (key0 + 16 > key_end) {   // only the last chunk of a sequence has keys past its end
 #pragma unroll
