@@ -13,7 +13,7 @@
 //    57 bytes a nanosecond, so weights have to be spread over nearly all of them to reach the 6.5 TB/s of HBM);
 //  * the kernel starts before its predecessor on the stream has drained and asks for its first weight tiles to be
 //    brought into L2 while the small kernel ahead (a quantiser, usually) still runs.
-// What is left is 3 us of start, fill and finish beside the stream: M = 16, 8192 x 8192 14.2 us (floor 10.3),
+// What is left is 3 us of start, fill and finish beside the stream: M = 16, 8192 x 8192 14.1 us (floor 10.3),
 // 12288 x 4096 11.2 (7.7), 22016 x 4096 with SwiGLU
 // 18.4 (13.8), 4096 x 11008 10.7 (6.9), 4096 x 4096 6.5 (2.6).
 #pragma once
@@ -33,6 +33,7 @@ constexpr int MAX_SPLIT = 8;                // portable cluster size
 constexpr int THREADS = 192;                // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2-5: read the accumulators back
 constexpr int TAIL_BYTES = 1024 /*align*/ + 512 /*barriers*/;
 constexpr int SMEM_ONE = 227 * 1024;        // of one CTA when it has the SM to itself
+constexpr int SMEM_LONG = 160 * 1024;       // what it takes of that for a long stream
 // shared memory of one of up to three CTAs on an SM (228 KB, 1 KB of it the system's for each CTA)
 constexpr int smem_of(int per_sm) { return per_sm == 1 ? SMEM_ONE : per_sm == 2 ? 112 * 1024 : 75 * 1024; }
 
@@ -678,7 +679,11 @@ inline int launch(GemmParams g, const Plan& plan, const void* A, const void* B, 
     const int stage_bytes = rows ? W_BYTES : W_BYTES + p.tn * BK;
     const int tok_bytes = rows ? (slice + 1) * TOKEN_BYTES : 0;
     p.slice = slice;
-    const int room = smem_of(plan.per_sm) - TAIL_BYTES - tok_bytes;
+    // A long stream of up to 32 tokens with an SM to itself has 160 KB in flight and not all 227: what is asked for beyond some 20 MB only waits in front
+    // of memory.  Us, 227 KB / 160 (112 KB: a fifth slower): 16 tokens, 8192 x 8192 14.25 / 14.1, 16384 x 16384 45.2 / 44.7, 5000 x 8000 10.6 / 10.4, 4 tokens,
+    // 7000 x 7008 12.8 / 12.4, 1 token 8192 x 8192 13.8 / 13.6; level or slower from 40 on, and where a CTA's 16 blocks nearly fit 9.03 / 9.17.
+    const int smem = plan.per_sm == 1 && !rows && g.M <= 32 && slice > 16 ? SMEM_LONG : smem_of(plan.per_sm);
+    const int room = smem - TAIL_BYTES - tok_bytes;
     auto stages_in = [&](int bytes) {
         int n = bytes / stage_bytes;
         if (rows && plan.per_sm == 3 && n > 3) n = 3;   // the rows' values wait behind what the rings have asked for: a step of one sequence 67.0, with four 67.7
