@@ -51,6 +51,7 @@ constexpr int CHUNK = 64;        // keys per unit of work (page sizes are multip
 constexpr int THREADS = 128;
 constexpr int WARPS = THREADS / 32;
 constexpr float LAG = 6.0f;      // log2 units
+constexpr int LONGEST_SPLIT = 8;   // chunks of a split up to which a cluster is worth it: past that it is level with the workspace
 constexpr int MAX_CLUSTER = 16, PORTABLE_CLUSTER = 8;   // splits of a pair that are a cluster
 constexpr int HINTS = 2;         // chunks a CTA asks for ahead of the wait
 // A wide warp step takes twice the keys of a narrow one (8 against 4 KB in flight per warp) and leaves registers for 12
@@ -930,7 +931,7 @@ Layout layout_of(int batch, int q_heads, int kv_heads, int head_dim, int span) {
         if (size > PORTABLE_CLUSTER && placed(PORTABLE_CLUSTER) && steps_of(PORTABLE_CLUSTER) <= steps_of(size) + 1) size = PORTABLE_CLUSTER;
         while (size > PORTABLE_CLUSTER && steps_of(size - 1) == steps_of(size)) size--;
         // (a cache is rarely full to its last split: 64 pairs of 1000 keys in a cache of 1064 have 8 of 9, 8.4 / 7.6)
-        if (pairs >= 16 && size > 1 && (steps_of(size) <= (each == 1 ? 3 : each + 1) || used <= size + size / 8)) x.cluster = (int)size;
+        if (pairs >= 16 && size > 1 && each <= LONGEST_SPLIT && (steps_of(size) <= (each == 1 ? 3 : each + 1) || (each <= 2 && used <= size + size / 8))) x.cluster = (int)size;
         x.plan = SPLITS;
         x.grid = (int)(pairs * (x.cluster ? x.cluster : x.splits));
     } else if (x.streams || 2 * pairs >= (x.rows == 8 ? 6 : 3) * wide || (chunks <= 32 && 5 * pairs >= 4 * wide) || pairs * chunks > 0x7fffffffLL) {
