@@ -138,6 +138,7 @@ constexpr size_t OC_BYTES_RMS = 320 << 10;
 constexpr size_t OC_BYTES_QKV = 448 << 10;
 constexpr size_t OC_BYTES_DEC = 448 << 10;
 constexpr size_t OC_BYTES_O = 512 << 10;
+constexpr size_t OC_CACHED = (size_t)64 << 20;
 
 // sets the maxima of an op to zero ahead of its pass 1 (a kernel and not a memset: it takes part in the overlapped launches)
 __global__ void clear_words_kernel(float* w, int n) {
@@ -1118,7 +1119,13 @@ int append(const fp8_decode_append_args_t* g, bool cleared) {
     a.tab_vec = !misaligned(g->cos_tab) && !misaligned(g->sin_tab);
     a.cph = FastDiv(g->head_dim / 32);
     a.slots = FastDiv(slots);
-    if (items * 64 <= OC_BYTES_DEC && oc_fits<DecOp>()) return (int)oc_launch(DecOp{a}, s, oc_threads(items));
+    // The attention behind puts its first CTAs beside these.  CTAs that have waited on their SMs since the projection ran there keep those SMs' storage as
+    // it was, nearly all shared memory, and a long attention's CTAs stream by a third slower in what L1 is left.  So where it has much to read (by
+    // the capacity) this kernel asks for L1 and comes when its SMs are free; CTAs of 512 threads, which did that by their size, left room for one of its CTAs
+    // beside them.  A step, us, 512 threads / small CTAs / small with L1: three sequences of 7400 keys 110.4 / 103 / 97.7, two of 6000 91.0 / 86.6 / 84.3, four
+    // of 7400 111.4 / 117.5 / 110.2, of 3000 89.2 / 91.0 / 88.8; four of 1000 80.3 / 79.0 / 79.9.
+    const size_t cached = 2 * (size_t)a.batch * a.hkv * a.hd * (a.block_table ? (size_t)a.page_size * a.max_pages : (size_t)a.s_max);
+    if (items * 64 <= OC_BYTES_DEC && oc_fits<DecOp>()) return (int)oc_launch(DecOp{a}, s, oc_threads(items), cached <= OC_CACHED ? -1 : cudaSharedmemCarveoutMaxL1);
     cudaError_t e = cleared ? cudaSuccess : clear_words(a.q_amax, 1, s);
     if (e == cudaSuccess && items > 0) e = launch_pdl(dec_q_amax_kernel, dim3(grid_for(items)), dim3(THREADS), 0, s, a);
     if (e == cudaSuccess) e = launch_pdl(dec_append_kernel, dim3(grid_for(items)), dim3(THREADS), 0, s, a);

@@ -97,7 +97,7 @@ inline int oc_threads(size_t items) {
 }
 
 template <class Op>
-inline cudaLaunchConfig_t oc_config(cudaLaunchAttribute* attr, cudaStream_t stream, int threads = OC_THREADS) {
+inline cudaLaunchConfig_t oc_config(cudaLaunchAttribute* attr, cudaStream_t stream, int threads = OC_THREADS, int carveout = -1) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(OC_CTAS);
     cfg.blockDim = dim3((unsigned)threads);
@@ -107,8 +107,10 @@ inline cudaLaunchConfig_t oc_config(cudaLaunchAttribute* attr, cudaStream_t stre
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
+    attr[2].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[2].val.sharedMemCarveout = carveout;
     cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = carveout < 0 ? 2 : 3;
     return cfg;
 }
 
@@ -121,7 +123,7 @@ inline bool oc_fits() {
     int k = known[dev].load(std::memory_order_acquire);
     if (k == 0) {
         int clusters = 0;
-        cudaLaunchAttribute attr[2];
+        cudaLaunchAttribute attr[3];
         cudaLaunchConfig_t cfg = oc_config<Op>(attr, nullptr);
         cfg.numAttrs = 1;
         const bool ok = cudaFuncSetAttribute(one_cluster_kernel<Op>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
@@ -133,10 +135,12 @@ inline bool oc_fits() {
     return k == 1;
 }
 
+// carveout: the per cent of an SM's storage that the kernel wants for shared memory.  With it a CTA is not put on an SM while CTAs there have
+// another share.
 template <class Op>
-inline cudaError_t oc_launch(const Op& op, cudaStream_t stream, int threads = OC_THREADS) {
-    cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t cfg = oc_config<Op>(attr, stream, threads);
+inline cudaError_t oc_launch(const Op& op, cudaStream_t stream, int threads = OC_THREADS, int carveout = -1) {
+    cudaLaunchAttribute attr[3];
+    const cudaLaunchConfig_t cfg = oc_config<Op>(attr, stream, threads, carveout);
     return cudaLaunchKernelEx(&cfg, one_cluster_kernel<Op>, op);
 }
 
