@@ -341,7 +341,17 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
     pdl_wait();
     pdl_trigger();
     find_piece(false);
-    if (seg.c_begin >= seg.c_end) return;
+    // CLUSTER: each CTA reads the length for itself.  Under a caller that rewrites the lengths while the kernel runs a peer may hand over what the first CTA
+    // does not wait for, so the first one ends behind the second phase, when every peer has handed over or gone, whatever it has read itself.  Who has nothing to
+    // hand over (no keys, or all of them) arrives at that phase here.
+    const bool nothing = seg.c_begin >= seg.c_end;
+    if (CLUSTER && (nothing || (seg.c_begin == 0 && seg.c_end == seg.n_chunks))) {
+        __syncwarp();
+        cluster_wait();
+        cluster_arrive();
+        if (nothing && blockIdx.x % p.cluster == 0) cluster_wait();
+    }
+    if (nothing) return;
     float scale_log2 = p.scale_log2;
     if (p.sq) scale_log2 *= ld_f32(p.sq);
     if (p.sk) scale_log2 *= ld_f32(p.sk);
@@ -672,11 +682,11 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
             }
         }
         if (CLUSTER) {
-            if (whole) return;
             __syncwarp();
-            cluster_arrive();
+            if (!whole) cluster_arrive();
             if (seg.c_begin != 0) return;   // what it has handed over is the first one's
             cluster_wait();
+            if (whole) return;
             // A column to a thread, the pieces in order
             const int parts = (seg.n_chunks + seg.c_end - 1) / seg.c_end;
             float M = -INFINITY;

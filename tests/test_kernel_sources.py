@@ -106,6 +106,70 @@ def test_a_part_of_the_decode_line_comes_from_one_reading_of_the_lengths():
     assert body.count("lane_len(") == 1 and "seq_len_of" not in body and "len_of(" not in body.replace("lane_len(", "")
 
 
+def test_the_first_block_of_a_decode_cluster_outlives_what_its_peers_store():
+    # every way out of the cluster form that the first block may take, by whatever it has read of the length, is behind both phases
+    text = re.sub(r"//[^\n]*", "", sources()["fa_decode_sm100.cu"])
+    kernel = text[text.index("find_piece(false);"):]
+    kernel = kernel[:kernel.index("if (!whole) {\n            int parts")]   # behind it: the workspace's merge, not the cluster's
+    # no keys, or all of them; a part, behind which a peer may go
+    assert re.search(r"if \(CLUSTER && \(nothing \|\| \(seg\.c_begin == 0 && seg\.c_end == seg\.n_chunks\)\)\) \{\s*__syncwarp\(\);\s*cluster_wait\(\);\s*cluster_arrive\(\);\s*"
+                     r"if \(nothing && blockIdx\.x % p\.cluster == 0\) cluster_wait\(\);\s*\}\s*if \(nothing\) return;", kernel)
+    assert "if (CLUSTER && !whole) cluster_wait();" in kernel
+    tail = kernel[kernel.rindex("if (CLUSTER) {"):]
+    assert re.match(r"if \(CLUSTER\) \{\s*__syncwarp\(\);\s*if \(!whole\) cluster_arrive\(\);\s*if \(seg\.c_begin != 0\) return;\s*cluster_wait\(\);\s*if \(whole\) return;",
+                    tail)
+    # no other way out than these, a lambda's and the end
+    assert len(re.findall(r"\breturn;", kernel)) == 5
+    assert len(re.findall(r"cluster_(?:wait|arrive)\(\)", kernel)) == 6
+
+
+def decode_cluster(readings, chunks_per_split, stays):
+    """The cluster's blocks by what each has read (in chunks): every order in which they may run.  True where a store can meet a block that has gone."""
+    size = len(readings)
+
+    def steps(rank, chunks):
+        used = -(-chunks // chunks_per_split)
+        each = chunks_per_split * -(-used // size)
+        begin, end = rank * each, min(chunks, (rank + 1) * each)
+        if begin >= end or (begin == 0 and end == chunks):
+            return ["arrive", "wait", "arrive", *["wait"] * (rank == 0), "gone"] if stays else ["arrive", "gone"]
+        return ["arrive", "wait", "store", "arrive", "gone"] if rank else ["arrive", "wait", "store", "arrive", "wait", "gone"]
+
+    plans = [steps(r, n) for r, n in enumerate(readings)]
+    seen, todo, bad = set(), [(0,) * size], False
+    arrivals = [[sum(s == "arrive" for s in plan[:i]) for i in range(len(plan) + 1)] for plan in plans]
+    while todo:
+        at = todo.pop()
+        if at in seen:
+            continue
+        seen.add(at)
+        gone = [i == len(p) for i, p in zip(at, plans)]
+        moved = False
+        for r, plan in enumerate(plans):
+            if gone[r]:
+                continue
+            step = plan[at[r]]
+            # a phase ends when every block has arrived at it or gone
+            if step == "wait" and not all(g or arrivals[q][at[q]] >= arrivals[r][at[r]] for q, g in enumerate(gone)):
+                continue
+            bad |= step == "store" and gone[0]
+            moved = True
+            todo.append(at[:r] + (at[r] + 1,) + at[r + 1:])
+        assert moved or all(gone), (readings, at)   # no order stands still
+    return bad
+
+
+@pytest.mark.parametrize("size,chunks_per_split", [(2, 1), (3, 1), (3, 2), (4, 1)])
+def test_readings_that_disagree_store_to_no_block_that_has_gone(size, chunks_per_split):
+    import itertools
+    most = size * chunks_per_split
+    readings = list(itertools.product(range(most + 1), repeat=size))
+    assert not any(decode_cluster(r, chunks_per_split, True) for r in readings)
+    # the model sees the fault of a first block that leaves by its own reading, and only where readings disagree
+    assert decode_cluster((1,) + (most,) * (size - 1), chunks_per_split, False)
+    assert not any(decode_cluster((n,) * size, chunks_per_split, False) for n in range(most + 1))
+
+
 @pytest.mark.parametrize("name", sources())
 def test_registers_stay_where_a_launch_puts_them(name):
     # an attention form that moved registers between its warps raised illegal accesses after a harmless change of its code, and the
