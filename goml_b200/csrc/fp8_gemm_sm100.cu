@@ -791,12 +791,13 @@ int launch(int M, int N, int K, const void* A, const void* B, void* C, float alp
         if (pair_cost > single_cost) pair = false;
     }
     // K is cut (below) where that leaves few units; else the shape may be chosen by what its waves cost.  Tiles of 192 columns hold no whole
-    // number of the boxes that activations and e4m3 results leave in.  A promise of 4 % is kept (16 % with SwiGLU, whose longer end the fit does not
+    // number of the boxes that activations and e4m3 results leave in, tiles of 64 store these without a map.  A promise of 4 % is kept (16 % with SwiGLU, whose longer end the fit does not
     // know: 410 x 16320 x 4096 in pairs promises 14 % and takes 31.5 us for 30.8).  Results that leave through no tensor map have an end several times as long, which pairs pay in full (6820 x 2331 x 4640 85 us, in 192-wide
     // pairs 99; 820 x 7262 x 10736 added 220 / 291): they keep the old shape.
     const long long units_now = (pair ? (m_tiles + 1) / 2 : m_tiles) * ((N + bn - 1) / bn);
     const bool cuts_k = p.x_tma && 2 * units_now <= st.num_sms;
-    const bool mapped = X ? p.x_tma : H ? F % 8 == 0 : D8 ? N % 16 == 0 : N % 8 == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+    auto on16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+    const bool mapped = X ? p.x_tma : H ? F % 8 == 0 && on16(H) : D8 ? N % 16 == 0 && on16(D8) : N % 8 == 0 && on16(C);
     if (m_tiles >= 2 && !cuts_k && mapped) {
         auto cost = [&](const UnitCost& c) {
             const long long units = (m_tiles + c.mt - 1) / c.mt * ((N + c.bn - 1) / c.bn), full = units / st.num_sms, rem = units % st.num_sms;
@@ -812,6 +813,7 @@ int launch(int M, int N, int K, const void* A, const void* B, void* C, float alp
             if ((c.mt == 2 && pair_policy() == 0) || (c.bn == 192 && (H || D8))) continue;
             const float t = cost(c);
             if (c.bn == bn && c.mt == (pair ? 2 : 1)) now = t;
+            else if (c.bn == 64 && (H || D8)) continue;
             if (!take || t < least) { take = &c; least = t; }
         }
         if (take && least < (H ? 0.84f : 0.96f) * now) {

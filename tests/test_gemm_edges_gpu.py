@@ -1,5 +1,7 @@
 """FP8 GEMM where the output's rows are not whole 16-byte pieces, and on both sides of the few-row kernel's lines: products of
 -1, 0 and 1, whose sums are whole numbers that fp16 holds, so every element is compared exactly."""
+import re
+
 import pytest
 import torch
 
@@ -105,6 +107,48 @@ def test_units_that_fill_their_waves(cuda, built_libs, M, N, K, variant):
     # rows that leave through no tensor map keep the shape that they had
     name, = kernels(lambda: G.FP8GEMMScaled(M, N - 1, K, a.data_ptr(), b.data_ptr(), c.data_ptr(), 1.0, 0, 0, G.OutBF16, stream()))
     assert "Li192" not in name
+
+
+def unit_of(call):
+    """(columns, tiles) of the work units that a product's kernel has."""
+    name, = kernels(call)
+    return tuple(int(n) for n in re.search(r"tcgen05_kernelILi(\d+)ELi(\d)E", name).groups())
+
+
+@pytest.mark.parametrize("M,N,K,swiglu,offset,unit", [(1500, 4992, 4096, False, 0, (256, 2)), (1500, 4992, 4096, False, 1, (256, 1)), (1500, 4992, 4096, False, 8, (256, 1)),
+                                                      (2431, 960, 2256, False, 0, (256, 1)), (1725, 5184, 6096, True, 0, (256, 2)), (1725, 5184, 6096, True, 1, (256, 1)),
+                                                      (1725, 5181, 6096, True, 0, (256, 1))])
+def test_results_that_no_map_describes_keep_their_units(cuda, built_libs, M, N, K, swiglu, offset, unit):
+    # e4m3 results and activations, offset by values past a 16-byte boundary: pairs pay the longer end in full, and tiles of 64 columns have no map
+    from goml_b200 import fp8_gemm as G
+    g = torch.Generator(device="cuda").manual_seed(M + offset)
+    rows = 2 * ((N + 31) // 32) * 32 if swiglu else N
+    a, b = (torch.randint(0, 0x78, (n, K), generator=g, dtype=torch.uint8, device="cuda") for n in (M, rows))
+    s = torch.tensor([3e-3, 2e-3, 1e-2], device="cuda")
+    p, stream = s.data_ptr(), lambda: torch.cuda.current_stream().cuda_stream
+
+    def result(offset):
+        room = torch.full((M * N + 64,), 3, dtype=torch.bfloat16 if swiglu else torch.uint8, device="cuda")
+        out, top = room[16 + offset:16 + offset + M * N], torch.zeros(1, device="cuda")
+        if swiglu:
+            call = lambda: G.FP8GEMMSwiGLURaise(M, N, K, a.data_ptr(), b.data_ptr(), out.data_ptr(), 1.0, p, p + 4, top.data_ptr(), stream())
+        else:
+            call = lambda: G.FP8GEMMFP8Out(M, N, K, a.data_ptr(), b.data_ptr(), out.data_ptr(), 1.0, p, p + 4, p + 8, top.data_ptr(), stream())
+        took = unit_of(call)
+        call()
+        torch.cuda.synchronize()
+        assert G.device_status() == 0
+        assert (room[:16 + offset] == 3).all() and (room[16 + offset + M * N:] == 3).all()
+        return took, out.view(torch.uint8), top
+
+    took, out, top = result(offset)
+    assert took == unit
+    G.SetTilePairs(0)
+    try:
+        single, want, want_top = result(0)
+    finally:
+        G.SetTilePairs(-1)
+    assert single[1] == 1 and torch.equal(out, want) and torch.equal(top, want_top)
 
 
 @pytest.mark.parametrize("split,K", [(1, 384), (2, 512), (3, 880), (4, 1024), (5, 6400), (6, 7696), (7, 8960), (8, 10240)])
