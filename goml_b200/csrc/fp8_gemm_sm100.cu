@@ -658,10 +658,9 @@ __global__ void __launch_bounds__(32) gemm_wait_expiry_selftest_kernel() {
 // ---------------------------------------------------------------- host side
 
 // What a wave of work units of each shape takes, for problems of at least two rows of tiles: start + waves x (k-blocks x block + end), us, fitted to 110
-// problems of 193 to 6000 rows with 1024 to 22016 columns and K of 1024 to 11008, each shape of unit timed on each (15 % off in the mean, alike for
-// all shapes).  Where it promises a margin it overrides the rule of widths and pairs alone; on 500 other problems of these ranges that is 2.8 % in the
-// mean, up to a quarter where it takes another shape: 3304 x 4096 x 8528 125.7 -> 102.3 us (192-wide pairs), 2538 x 5936 x 3184 62.0 -> 50.5 (256-wide pairs),
-// 4212 x 1472 x 5616 48.6 -> 37.0, 1024 x 5000 x 6000 50.1 -> 38.7, 700 x 8192 x 8192 47.4 -> 41.2, 512 x 5000 x 6000 32.4 -> 27.5 (192-wide tiles).
+// problems of 193 to 6000 rows with 1024 to 22016 columns and K of 1024 to 11008, each shape of unit timed on each (15 % off in the mean).  Half of
+// those K were odd multiples of 16: rows that begin off a 32-byte boundary cost the loads of single tiles more than those of pairs, so what a shape gains
+// depends on K's multiple as much as on its waves, and launch() asks for more where rows are aligned.
 struct UnitCost {
     int bn, mt;
     float start, block, end;
@@ -773,7 +772,8 @@ int launch(int M, int N, int K, const void* A, const void* B, void* C, float alp
     // Tile pairs: with at least two waves of 256 x 256 pairs and a K long enough to amortise the three-stage ring, a
     // CTA holds two vertically adjacent 128 x 256 accumulators (both TMEM buffers) and feeds both from each B tile it
     // loads: 32 KB instead of 48 KB of operands per 128 x 256 x 128 block of MMA work (8192^3: 2739 -> 2965 TFLOP/s).
-    // (One wave of pairs is enough when K is long: 4096 x 4096 x 8192 98 us against 106 us; with K = 4096 it is not.)
+    // (One wave of pairs is enough when K is long: 4096 x 4096 x 8192 98 us against 106 us; with K = 4096 it is not, 50.2 against 50.2 and as e4m3 52.5
+    // against 49.8.)
     // A pair-wave costs two tile-waves at about 0.92 of their time, and pair mode has no half-width last wave, so
     // pairs are taken only when that estimate does not lose to single tiles: a pair count just above a multiple of
     // the SM count (150 pairs on 148 SMs) would pay a whole extra double-cost wave.
@@ -791,14 +791,24 @@ int launch(int M, int N, int K, const void* A, const void* B, void* C, float alp
         if (pair_cost > single_cost) pair = false;
     }
     // K is cut (below) where that leaves few units; else the shape may be chosen by what its waves cost.  Tiles of 192 columns hold no whole
-    // number of the boxes that activations and e4m3 results leave in, tiles of 64 store these without a map.  A promise of 4 % is kept (16 % with SwiGLU, whose longer end the fit does not
-    // know: 410 x 16320 x 4096 in pairs promises 14 % and takes 31.5 us for 30.8).  Results that leave through no tensor map have an end several times as long, which pairs pay in full (6820 x 2331 x 4640 85 us, in 192-wide
-    // pairs 99; 820 x 7262 x 10736 added 220 / 291): they keep the old shape.
+    // number of the boxes that activations and e4m3 results leave in.  Results that leave through no tensor map have an end several times as long, which pairs
+    // pay in full (6820 x 2331 x 4640 85 us, in 192-wide pairs 99; 820 x 7262 x 10736 added 220 / 291): they keep the rule's shape.
+    // A promise of 4 % is kept, except (problems of 129 to 60000 rows, 32 to 130000 columns and K up to 32000; us: the rule's shape / the promised one, in turn):
+    //  * below K = 256 (added: 128), where nothing was fitted, the rule stays: 104 of 244 problems are more than 2 % slower, 4096 x 4096 x 128 9.98 / 10.5, 8192 x
+    //    8192 x 128 29.3 / 31.5; from there to 1024 192-wide tiles gain 9 % in 34 problems and lose in none;
+    //  * pairs for single tiles where rows begin on 64 bytes: 12 %, but for added results.  17 of 48 smaller promises lost, as e4m3 4096 x 4096 x 4096 49.8 /
+    //    52.5, as 16 bits 4096 x 4096 x 3072 38.8 / 40.3.  With odd multiples of 16 they are 1.06 to 1.56 times as fast in 255 problems, whatever is promised;
+    //  * pairs for tiles of 128 columns only with odd multiples of 16 (63 problems, 1.09 to 1.20 times; else 35 of 42 lose, 4192 x 2080 x 5888 46.7 / 53.1), 192-wide
+    //    tiles for them where K is no multiple of 64 (93 problems, 1.05; else level);
+    //  * single tiles for pairs only where K is a multiple of 128 (added: of 64; 92 problems, 1.07; else 61 of 96 lose, 7688 x 14880 x 2192 234 / 291);
+    //  * no narrower tiles: 47 of 63 lose with 64 columns, 28 of 37 with 128;
+    //  * SwiGLU, whose longer end the fit does not know: 16 % (410 x 16320 x 4096 in pairs promises 14 % and takes 31.5 us for 30.8), 20 % on 64 bytes.
+    // So 1660 other problems of these ranges whose shape changes are 10 % faster in the mean (8 % with rows on 64 bytes); 48 are more than 2 % slower, at worst 8 %.
     const long long units_now = (pair ? (m_tiles + 1) / 2 : m_tiles) * ((N + bn - 1) / bn);
     const bool cuts_k = p.x_tma && 2 * units_now <= st.num_sms;
     auto on16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
     const bool mapped = X ? p.x_tma : H ? F % 8 == 0 && on16(H) : D8 ? N % 16 == 0 && on16(D8) : N % 8 == 0 && on16(C);
-    if (m_tiles >= 2 && !cuts_k && mapped) {
+    if (m_tiles >= 2 && !cuts_k && mapped && K >= (X ? BK : 2 * BK)) {
         auto cost = [&](const UnitCost& c) {
             const long long units = (m_tiles + c.mt - 1) / c.mt * ((N + c.bn - 1) / c.bn), full = units / st.num_sms, rem = units % st.num_sms;
             const bool halves = c.bn == 256 && c.mt == 1 && full > 0 && 2 * rem <= st.num_sms;
@@ -809,14 +819,17 @@ int launch(int M, int N, int K, const void* A, const void* B, void* C, float alp
         };
         const UnitCost* take = nullptr;
         float now = 0.f, least = 0.f;
+        for (const UnitCost& c : UNIT_COSTS)
+            if (c.bn == bn && c.mt == (pair ? 2 : 1)) now = cost(c);
         for (const UnitCost& c : UNIT_COSTS) {
-            if ((c.mt == 2 && pair_policy() == 0) || (c.bn == 192 && (H || D8))) continue;
+            const bool wider = c.mt == 2 && !pair, aligned = wider && K % 64 == 0;   // wider: pairs in the place of single tiles
+            if (c.bn < 192 || (c.bn == bn && c.mt == (pair ? 2 : 1)) || (c.bn == 192 && (H || D8)) || (c.mt == 2 && pair_policy() == 0)) continue;
+            if (bn < 256 ? (!wider && c.bn == 256) || K % (wider ? 32 : 64) == 0 : pair && c.mt == 1 && K % (X ? 64 : 128) != 0) continue;
+            const float margin = H ? (aligned ? 0.80f : 0.84f) : aligned && !X ? 0.88f : 0.96f;
             const float t = cost(c);
-            if (c.bn == bn && c.mt == (pair ? 2 : 1)) now = t;
-            else if (c.bn == 64 && (H || D8)) continue;
-            if (!take || t < least) { take = &c; least = t; }
+            if (t < margin * now && (!take || t < least)) { take = &c; least = t; }
         }
-        if (take && least < (H ? 0.84f : 0.96f) * now) {
+        if (take) {
             bn = take->bn;
             pair = take->mt == 2;
         }

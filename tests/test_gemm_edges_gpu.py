@@ -151,6 +151,26 @@ def test_results_that_no_map_describes_keep_their_units(cuda, built_libs, M, N, 
     assert single[1] == 1 and torch.equal(out, want) and torch.equal(top, want_top)
 
 
+# what a unit of another shape promises is not kept: a short K; pairs for single tiles or tiles of 128 columns, single tiles for pairs, as rows begin; narrow tiles
+@pytest.mark.parametrize("kind,M,N,K,unit", [("c", 1213, 2560, 240, (256, 1)), ("c", 1213, 2560, 256, (192, 1)), ("x", 1213, 2560, 112, (256, 1)), ("x", 1213, 2560, 128, (192, 1)),
+                                             ("c", 4096, 4096, 128, (256, 1)), ("c", 4096, 4096, 4096, (256, 1)), ("d", 4096, 4096, 4096, (256, 1)), ("c", 4096, 4096, 3072, (256, 1)),
+                                             ("c", 4096, 4096, 3088, (256, 2)), ("c", 4192, 2080, 5888, (128, 1)), ("c", 4192, 2080, 5904, (192, 2)), ("c", 1411, 6192, 1984, (128, 1)),
+                                             ("c", 3524, 19360, 2160, (256, 2)), ("c", 3524, 19360, 2176, (256, 1)), ("d", 10176, 160, 4208, (256, 1))])
+def test_units_that_lose_are_not_taken(cuda, built_libs, kind, M, N, K, unit):
+    from goml_b200 import fp8_gemm as G
+    a, b = (torch.full((rows, K), 0x38, dtype=torch.uint8, device="cuda") for rows in (M, N))
+    out = torch.zeros(M, N, dtype={"c": torch.bfloat16, "x": torch.float32, "d": torch.uint8}[kind], device="cuda")
+    ptrs, stream = (a.data_ptr(), b.data_ptr(), out.data_ptr()), lambda: torch.cuda.current_stream().cuda_stream
+    call = {"c": lambda: G.FP8GEMMScaled(M, N, K, *ptrs, 1.0, 0, 0, G.OutBF16, stream()), "x": lambda: G.FP8GEMMAccumulateF32(M, N, K, *ptrs, 1.0, 0, 0, stream()),
+            "d": lambda: G.FP8GEMMFP8Out(M, N, K, *ptrs, 1.0 / K, 0, 0, 0, 0, stream())}[kind]
+    assert unit_of(call) == unit
+    call()
+    torch.cuda.synchronize()
+    assert G.device_status() == 0
+    want = torch.tensor(K, dtype=torch.float32).to(out.dtype) if kind != "d" else 0x38   # ones: sums of K, or 1 as a code
+    assert (out == want).all()
+
+
 @pytest.mark.parametrize("split,K", [(1, 384), (2, 512), (3, 880), (4, 1024), (5, 6400), (6, 7696), (7, 8960), (8, 10240)])
 @pytest.mark.parametrize("N", [200, 131])
 def test_sums_handed_to_their_owners_and_fetched_are_the_same(cuda, built_libs, split, K, N):
