@@ -179,9 +179,10 @@ __device__ __forceinline__ void prefetch_l2(const uint8_t* p, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
-// To the same place in the first CTA of the cluster
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_here() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }   // nothing is handed over
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// To the same place in the first CTA of the cluster
 __device__ __forceinline__ uint32_t in_first(const float* p) {
     uint32_t a;
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)));
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
     // CLUSTER: what the splits of the pair hand to its first CTA
     __shared__ __align__(16) float s_part_o[CLUSTER ? MAX_CLUSTER : 1][CLUSTER ? D : 4];
     __shared__ __align__(8) float s_part_ml[CLUSTER ? MAX_CLUSTER : 1][2];
-    if (CLUSTER) cluster_arrive();   // its phase says that every CTA runs, so that its shared memory may be written
+    if (CLUSTER) cluster_here();   // its phase says that every CTA runs, so that its shared memory may be written
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;              // MMA fragment coordinates
@@ -342,14 +343,15 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
     pdl_trigger();
     find_piece(false);
     // CLUSTER: each CTA reads the length for itself.  Under a caller that rewrites the lengths while the kernel runs a peer may hand over what the first CTA
-    // does not wait for, so the first one ends behind the second phase, when every peer has handed over or gone, whatever it has read itself.  Who has nothing to
-    // hand over (no keys, or all of them) arrives at that phase here.
+    // does not wait for, so the first one ends behind the second phase, when every peer has handed over or gone, whatever it has read itself.  Where it has no keys
+    // or all of them it arrives at that phase here, without the order of memory that a hand-over needs (five sequences of 130 keys, 32 heads, a cache of 500: 7.9 us
+    // with arrivals that release, 6.8 so; 7.2 without a second phase but with a first arrival that releases).
     const bool nothing = seg.c_begin >= seg.c_end;
-    if (CLUSTER && (nothing || (seg.c_begin == 0 && seg.c_end == seg.n_chunks))) {
+    if (CLUSTER && blockIdx.x % p.cluster == 0 && (nothing || seg.c_end == seg.n_chunks)) {
         __syncwarp();
         cluster_wait();
-        cluster_arrive();
-        if (nothing && blockIdx.x % p.cluster == 0) cluster_wait();
+        cluster_here();
+        if (nothing) cluster_wait();
     }
     if (nothing) return;
     float scale_log2 = p.scale_log2;
@@ -930,8 +932,8 @@ Layout layout_of(int batch, int q_heads, int kv_heads, int head_dim, int span) {
         // chunks in turn than the workspace's merge costs time.
         // Us, workspace / cluster: 32 pairs of 1000 keys 6.6 / 5.7 (of 64 6.1 / 4.5), of 100 5.0 / 4.1; 16 of 2000 7.4 / 6.6; 96 of 500 7.9 / 6.8; 112 of 900 10.7 /
         // 9.8; but where a split has several chunks and a CTA would take two, 32 of 2000 9.0 / 9.4, 192 of 500 9.7 / 12.4.
-        // Fewer than 16 pairs keep the workspace although a cluster is faster there too (8 pairs of 1000 keys 5.6 / 4.4): what such a call leaves
-        // in a graph is held to be allocations and a clearing kernel (tests/test_fa_scratch_gpu.py).
+        // Fewer than 16 pairs keep the workspace, which is not the faster one there (8 pairs of 1000 keys 5.6 / 4.4): the line is not where clusters stop paying, but
+        // calls of eight pairs are what the tests of scratch and of captured calls take for a cut pair in the workspace (tests/test_fa_scratch_gpu.py).
         const ClusterFit& fit = cluster_fit();
         const long long each = (chunks + x.splits - 1) / x.splits, used = each ? (chunks + each - 1) / each : 0;
         auto placed = [&](long long n) { return n > PORTABLE_CLUSTER ? 8 * pairs <= 7 * fit.n[n] : n > 3 ? 16 * pairs <= 15 * fit.n[n] : pairs <= fit.n[n]; };

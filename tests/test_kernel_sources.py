@@ -112,15 +112,15 @@ def test_the_first_block_of_a_decode_cluster_outlives_what_its_peers_store():
     kernel = text[text.index("find_piece(false);"):]
     kernel = kernel[:kernel.index("if (!whole) {\n            int parts")]   # behind it: the workspace's merge, not the cluster's
     # no keys, or all of them; a part, behind which a peer may go
-    assert re.search(r"if \(CLUSTER && \(nothing \|\| \(seg\.c_begin == 0 && seg\.c_end == seg\.n_chunks\)\)\) \{\s*__syncwarp\(\);\s*cluster_wait\(\);\s*cluster_arrive\(\);\s*"
-                     r"if \(nothing && blockIdx\.x % p\.cluster == 0\) cluster_wait\(\);\s*\}\s*if \(nothing\) return;", kernel)
+    assert re.search(r"if \(CLUSTER && blockIdx\.x % p\.cluster == 0 && \(nothing \|\| seg\.c_end == seg\.n_chunks\)\) \{\s*__syncwarp\(\);\s*cluster_wait\(\);\s*cluster_here\(\);\s*"
+                     r"if \(nothing\) cluster_wait\(\);\s*\}\s*if \(nothing\) return;", kernel)
     assert "if (CLUSTER && !whole) cluster_wait();" in kernel
     tail = kernel[kernel.rindex("if (CLUSTER) {"):]
     assert re.match(r"if \(CLUSTER\) \{\s*__syncwarp\(\);\s*if \(!whole\) cluster_arrive\(\);\s*if \(seg\.c_begin != 0\) return;\s*cluster_wait\(\);\s*if \(whole\) return;",
                     tail)
     # no other way out than these, a lambda's and the end
     assert len(re.findall(r"\breturn;", kernel)) == 5
-    assert len(re.findall(r"cluster_(?:wait|arrive)\(\)", kernel)) == 6
+    assert len(re.findall(r"cluster_(?:wait|arrive|here)\(\)", kernel)) == 6
 
 
 def decode_cluster(readings, chunks_per_split, stays):
@@ -132,7 +132,7 @@ def decode_cluster(readings, chunks_per_split, stays):
         each = chunks_per_split * -(-used // size)
         begin, end = rank * each, min(chunks, (rank + 1) * each)
         if begin >= end or (begin == 0 and end == chunks):
-            return ["arrive", "wait", "arrive", *["wait"] * (rank == 0), "gone"] if stays else ["arrive", "gone"]
+            return ["arrive", "wait", "arrive", "wait", "gone"] if stays and rank == 0 else ["arrive", "gone"]
         return ["arrive", "wait", "store", "arrive", "gone"] if rank else ["arrive", "wait", "store", "arrive", "wait", "gone"]
 
     plans = [steps(r, n) for r, n in enumerate(readings)]
