@@ -1123,7 +1123,10 @@ int append(const fp8_decode_append_args_t* g, bool cleared) {
     // it was, nearly all shared memory, and a long attention's CTAs stream by a third slower in what L1 is left.  So where it has much to read (by
     // the capacity) this kernel asks for L1 and comes when its SMs are free; CTAs of 512 threads, which did that by their size, left room for one of its CTAs
     // beside them.  A step, us, 512 threads / small CTAs / small with L1: three sequences of 7400 keys 110.4 / 103 / 97.7, two of 6000 91.0 / 86.6 / 84.3, four
-    // of 7400 111.4 / 117.5 / 110.2, of 3000 89.2 / 91.0 / 88.8; four of 1000 80.3 / 79.0 / 79.9.
+    // of 7400 111.4 / 117.5 / 110.2, of 3000 89.2 / 91.0 / 88.8; four of 1000 80.3 / 79.0 / 79.9.  The lengths are on the device, so the line goes by the capacity, and
+    // one to three sequences pay where a large cache is little filled (small / small with L1: one of 1000 keys in 32768 75.1 / 78.0, of 4000 88.6 / 92.4, two of 2000 in 8192
+    // 83.4 / 84.4, three of 1500 in 8192 91.7 / 93.0) as much as they gain where it is full (one of 9000 77.7 / 76.1, of 30000 109.4 / 101.3); four and more are level or
+    // ahead (four of 2000 in 8192 105.3 / 102.2).
     const size_t cached = 2 * (size_t)a.batch * a.hkv * a.hd * (a.block_table ? (size_t)a.page_size * a.max_pages : (size_t)a.s_max);
     if (items * 64 <= OC_BYTES_DEC && oc_fits<DecOp>()) return (int)oc_launch(DecOp{a}, s, oc_threads(items), cached <= OC_CACHED ? -1 : cudaSharedmemCarveoutMaxL1);
     cudaError_t e = cleared ? cudaSuccess : clear_words(a.q_amax, 1, s);

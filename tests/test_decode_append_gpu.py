@@ -170,3 +170,45 @@ def test_lengths_advance_in_place(cuda, built_libs, B, Hq, Hkv):
 def test_small_steps_in_clusters_of_every_size(cuda, built_libs, B, Hq, Hkv):
     # 16 items (one warp to a CTA), 768, 1152, 2112, 7104
     test_codes_and_cache_rows_bit_exact(cuda, built_libs, B, Hq, Hkv, 96, 128)
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,hd", [(1, 32, 32, 128), (3, 32, 8, 128), (2, 32, 32, 64)])
+@pytest.mark.parametrize("paged", [False, True])
+def test_on_both_sides_of_a_large_cache(cuda, built_libs, B, Hq, Hkv, hd, paged):
+    # past 64 MB of capacity the append asks for L1: the same codes, scale, rows and lengths, and nothing else written
+    from goml_b200 import block_glue as BG
+    page = 64
+    rows = (64 << 20) // (2 * B * Hkv * hd) // page * page   # positions that the line leaves room for
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    qkv = torch.randn(B, (Hq + 2 * Hkv) * hd, generator=g, device="cuda").bfloat16()
+    positions = torch.tensor([rows - 1, 0, 77][:B], dtype=torch.int32, device="cuda")
+    cos, sin = rope_tables(rows, hd)
+    got = []
+    for cap in (rows, rows + page):
+        per = cap // page
+        table = torch.arange(B * per, dtype=torch.int32, device="cuda")
+        k, v = (torch.full((B * cap * Hkv * hd,), 0x55, dtype=torch.uint8, device="cuda") for _ in range(2))
+        q = torch.zeros(B, Hq, hd, dtype=torch.uint8, device="cuda")
+        sc, lens = torch.tensor([0.0, 0.0, 0.01, 0.02], device="cuda"), torch.zeros(B, dtype=torch.int32, device="cuda")
+        more = dict(block_table=table.data_ptr(), page_size=page, max_pages_per_seq=per, num_pages=B * per) if paged else {}
+        BG.DecodeRopeAppend(qkv.data_ptr(), cos.data_ptr(), sin.data_ptr(), positions.data_ptr(), q.data_ptr(), sc.data_ptr(), sc.data_ptr() + 4, k.data_ptr(), v.data_ptr(),
+                            sc.data_ptr() + 8, sc.data_ptr() + 12, B, Hq, Hkv, hd, 0 if paged else cap, rows, seq_lens_out=lens.data_ptr(),
+                            stream=torch.cuda.current_stream().cuda_stream, **more)
+        torch.cuda.synchronize()
+        # [sequence][position][head][...]
+        view = lambda t: t.view(B, per, Hkv, page, hd).transpose(2, 3).reshape(B, cap, Hkv, hd) if paged else t.view(B, Hkv, cap, hd).transpose(1, 2)
+        rest = torch.ones(B, cap, dtype=torch.bool, device="cuda")
+        for b in range(B):
+            rest[b, positions[b]] = False
+        new = [torch.stack([view(t)[b, positions[b]] for b in range(B)]) for t in (k, v)]
+        assert all((view(t)[rest] == 0x55).all() for t in (k, v))
+        got.append((q, sc, lens, *new))
+    assert got[0][2].tolist() == [n + 1 for n in positions.tolist()]
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+    # q against its restatement, and the new rows against the values that they quantise
+    host = qkv.float().cpu().numpy()
+    want = glue.decode_rope_append(host, cos.cpu().numpy(), sin.cpu().numpy(), positions.cpu().numpy(), np.zeros((B, Hkv, rows, hd), np.uint8),
+                                   np.zeros((B, Hkv, rows, hd), np.uint8), 0.01, 0.02, Hq, Hkv, hd)
+    assert np.array_equal(got[0][0].cpu().numpy(), want[0])
+    for b, n in enumerate(positions.tolist()):
+        assert np.array_equal(got[0][3][b].cpu().numpy(), want[3][b, :, n]) and np.array_equal(got[0][4][b].cpu().numpy(), want[4][b, :, n])

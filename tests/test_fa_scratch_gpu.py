@@ -81,6 +81,10 @@ CALLS = {"splits": lambda: Decode(1, 8, 8, 1000, 128), "one split": lambda: Deco
          "forward": lambda: Forward(8, 700, 128), "forward, hd 64": lambda: Forward(3, 300, 64, 0),
          # V converted ahead, with scratch and flags
          "ahead, few tiles": lambda: Forward(4, 1300, 128, 0), "ahead, hd 64": lambda: Forward(6, 2700, 64, 0), "ahead, causal": lambda: Forward(9, 2700, 128)}
+# splits that meet in a cluster: runs of one and of two or three splits, several sequences
+CLUSTERS = {"cluster": lambda: Decode(1, 32, 32, 1064, 128), "cluster, runs": lambda: Decode(1, 16, 16, 2368, 128), "cluster, hd 64": lambda: Decode(5, 16, 16, 900, 64),
+            "cluster, runs, hd 64": lambda: Decode(1, 16, 16, 2368, 64)}
+CALLS.update(CLUSTERS)
 
 
 @pytest.mark.parametrize("name", [n for n in CALLS if "forward" in n or "ahead" in n])
@@ -147,6 +151,50 @@ def test_nodes_of_a_captured_decode(cuda, built_libs, fa_ctx, name, kernels, oth
     kernel, memset, alloc, free = 0, 2, 10, 11
     assert types.count(kernel) == kernels and types.count(memset) == 0
     assert sorted(t for t in types if t != kernel) == sorted([alloc, free] * (others // 2))
+
+
+@pytest.mark.parametrize("name", CLUSTERS)
+def test_a_captured_cluster_leaves_its_kernel_alone(cuda, built_libs, fa_ctx, name):
+    call = CLUSTERS[name]()
+    call.result(fa_ctx)
+    (kind, kernel, _), = captured_nodes(lambda: call(fa_ctx))
+    assert kind == 0 and "fa_decode_kernel" in kernel and kernel.split("EvN")[0].endswith("Lb1EE")
+
+
+@pytest.mark.parametrize("name", CLUSTERS)
+def test_clusters_on_streams_that_come_and_go(cuda, built_libs, fa_ctx, name):
+    test_streams_that_come_and_go(cuda, built_libs, fa_ctx, name)
+
+
+@pytest.mark.parametrize("streams", [1, 4])
+def test_clusters_on_threads(cuda, built_libs, fa_ctx, streams):
+    # four host threads with clusters of different sizes beside a call with scratch
+    import threading
+    calls = [make() for make in [*CLUSTERS.values()][:3]] + [CALLS["splits"]()]
+    want = [c.result(fa_ctx) for c in calls]
+    for c in calls:
+        c.o.fill_(float("nan"))
+    ss = [torch.cuda.Stream() for _ in range(streams)]
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(t):
+        try:
+            torch.cuda.set_device(0)
+            for _ in range(200):
+                calls[t](fa_ctx, ss[t % streams])
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    torch.cuda.synchronize()
+    assert not errors, errors
+    fa_ctx.DeviceStatus()
+    assert all(torch.equal(c.o, w) for c, w in zip(calls, want))
 
 
 def test_buffers_that_grow_and_serve_both_entry_points(cuda, built_libs, fa_ctx):

@@ -93,6 +93,17 @@ def test_append_then_decode(cuda, built_libs, fa_ctx, B, Hq, Hkv, hd, paged):
     assert torch.isfinite(out).all() and lens.tolist() == [n + STEPS for n in lens0.tolist()]
 
 
+@pytest.mark.parametrize("B,H,hd,paged", [(1, 32, 128, False), (4, 32, 128, True), (9, 32, 128, False), (9, 32, 64, True), (1, 16, 64, False)])
+def test_append_then_decode_in_clusters(cuda, built_libs, fa_ctx, B, H, hd, paged):
+    # splits of 256 rows that meet in clusters of two to four: sequences of 1 to 186 keys, which the first of them has all, or some of them
+    x = torch.zeros(B * H * 256 * hd, dtype=torch.uint8, device="cuda")
+    lens = torch.full((B,), 7, dtype=torch.int32, device="cuda")
+    name, = kernels(lambda: fa_ctx.Decode(x.data_ptr(), x.data_ptr(), x.data_ptr(), torch.empty(B, H, hd, dtype=torch.float16, device="cuda").data_ptr(), 0, lens.data_ptr(),
+                                          B, H, H, hd, 256, 0, 1.0, 1.0, stream=torch.cuda.current_stream().cuda_stream))
+    assert "fa_decode_kernel" in name and name.split("EvN")[0].endswith("Lb1EE")
+    test_append_then_decode(cuda, built_libs, fa_ctx, B, H, H, hd, paged)
+
+
 @pytest.mark.parametrize("M,K,F,N,variant", [(300, 512, 704, 520, "Li64ELi1"), (1000, 1024, 1376, 517, "Li256ELi1"), (2048, 2048, 4736, 520, "Li256ELi2")])
 def test_quantise_then_square_gemm(cuda, built_libs, M, K, F, N, variant):
     # norm + quantiser -> gate/up GEMM -> quantiser -> GEMM into 16 bits, rows of whole pieces and odd ones -> and the next step's norm
