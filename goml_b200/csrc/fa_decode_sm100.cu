@@ -182,17 +182,17 @@ __device__ __forceinline__ void prefetch_l2(const uint8_t* p, uint32_t bytes) {
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_here() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }   // nothing is handed over
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// To the same place in the first CTA of the cluster
-__device__ __forceinline__ uint32_t in_first(const float* p) {
+// To the same place in another CTA of the cluster
+__device__ __forceinline__ uint32_t in_rank(const float* p, int rank) {
     uint32_t a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
     return a;
 }
-__device__ __forceinline__ void st_first(const float* p, const float4& v) {
-    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(in_first(p)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+__device__ __forceinline__ void st_rank(const float* p, int rank, const float4& v) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(in_rank(p, rank)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
-__device__ __forceinline__ void st_first(const float* p, const float2& v) {
-    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(in_first(p)), "f"(v.x), "f"(v.y) : "memory");
+__device__ __forceinline__ void st_rank(const float* p, int rank, const float2& v) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(in_rank(p, rank)), "f"(v.x), "f"(v.y) : "memory");
 }
 
 struct Segment {
@@ -201,7 +201,7 @@ struct Segment {
     int pair_u0;                    // unit of the line where the pair starts
 };
 
-// CLUSTER: the splits of a pair are the CTAs of a cluster (one query head per kv head)
+// CLUSTER: the splits of a pair are the CTAs of a cluster (one query head per kv head), its first CTA the one with the first run of them
 template <int D, int NQ, bool WIDE, bool STREAMS, bool PAGED, bool CLUSTER = false>
 __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_kernel(const DecodeParams p) {
     using C = Cfg<D, NQ, WIDE>;
@@ -289,6 +289,10 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
     // that one starts when the append has ended, and the hints cost a call 0.9 us.  (As two trips of one loop the search cost pieces of one to two
     // chunks: one sequence of 4000 18.3, now 16.5, 16.6 without.)  A CTA per pair or split gains nothing (a step of 64 sequences 336 / 341, of one
     // 78.1 / 77.7) and is found once.
+    //
+    // CLUSTER: the run of splits that this CTA has, and whose rank the first run is.  Equal ranks of clusters lie on few SMs, and short sequences give work to the
+    // first runs alone, so that these go round the ranks: 5 sequences of 300 keys, 16 heads of 128, a cache of 1064 7.9 / 7.3 us, 2 of 60, 32 heads, 4.4 / 3.9, full caches level.
+    int run = 0, first_rank = 0;
     Segment seg;
     int cut_q = 0, cut_r = 0;
     int mid = 0, mid_end = 0;    // units of the segments still to come in line order
@@ -297,7 +301,12 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
         seg.b = seg.kvh = seg.len = seg.n_chunks = seg.c_begin = seg.c_end = seg.pair_u0 = 0;
         if (!line) {
             const int per_pair = CLUSTER ? p.cluster : p.splits;
-            const int pair = blockIdx.x / per_pair, split = blockIdx.x - pair * per_pair;
+            const int pair = blockIdx.x / per_pair;
+            int split = blockIdx.x - pair * per_pair;
+            if (CLUSTER) {
+                first_rank = pair % per_pair;
+                split = run = (split < first_rank ? split + per_pair : split) - first_rank;
+            }
             seg.b = pair / p.hkv;
             seg.kvh = pair - seg.b * p.hkv;
             seg.len = seq_len_of(p, seg.b);
@@ -347,7 +356,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
     // or all of them it arrives at that phase here, without the order of memory that a hand-over needs (five sequences of 130 keys, 32 heads, a cache of 500: 7.9 us
     // with arrivals that release, 6.8 so; 7.2 without a second phase but with a first arrival that releases).
     const bool nothing = seg.c_begin >= seg.c_end;
-    if (CLUSTER && blockIdx.x % p.cluster == 0 && (nothing || seg.c_end == seg.n_chunks)) {
+    if (CLUSTER && run == 0 && (nothing || seg.c_end == seg.n_chunks)) {
         __syncwarp();
         cluster_wait();
         cluster_here();
@@ -674,9 +683,8 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
             if (whole) {
                 store_out<D>(p, ((size_t)b * p.hq + (size_t)kvh * p.group + row), col, M, L, O, vds);
             } else if (CLUSTER) {
-                const int split = blockIdx.x - (blockIdx.x / p.cluster) * p.cluster;
-                st_first(&s_part_o[split][col], O);
-                if (col == 0) st_first(s_part_ml[split], make_float2(M, L));
+                st_rank(&s_part_o[run][col], first_rank, O);
+                if (col == 0) st_rank(s_part_ml[run], first_rank, make_float2(M, L));
             } else {
                 const size_t at = (size_t)slot * C::ROWS + row;
                 __stcg(reinterpret_cast<float4*>(p.ws_o + at * D + col), O);

@@ -112,7 +112,7 @@ def test_the_first_block_of_a_decode_cluster_outlives_what_its_peers_store():
     kernel = text[text.index("find_piece(false);"):]
     kernel = kernel[:kernel.index("if (!whole) {\n            int parts")]   # behind it: the workspace's merge, not the cluster's
     # no keys, or all of them; a part, behind which a peer may go
-    assert re.search(r"if \(CLUSTER && blockIdx\.x % p\.cluster == 0 && \(nothing \|\| seg\.c_end == seg\.n_chunks\)\) \{\s*__syncwarp\(\);\s*cluster_wait\(\);\s*cluster_here\(\);\s*"
+    assert re.search(r"if \(CLUSTER && run == 0 && \(nothing \|\| seg\.c_end == seg\.n_chunks\)\) \{\s*__syncwarp\(\);\s*cluster_wait\(\);\s*cluster_here\(\);\s*"
                      r"if \(nothing\) cluster_wait\(\);\s*\}\s*if \(nothing\) return;", kernel)
     assert "if (CLUSTER && !whole) cluster_wait();" in kernel
     tail = kernel[kernel.rindex("if (CLUSTER) {"):]
