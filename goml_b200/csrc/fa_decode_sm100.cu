@@ -939,12 +939,14 @@ Layout layout_of(int batch, int q_heads, int kv_heads, int head_dim, int span) {
         // clusters of 5 as fit 12.3 us, workspace 10.8), and 8 rather than more.  A CTA takes several splits in turn, which must not cost more
         // chunks in turn than the workspace's merge costs time.
         // Us, workspace / cluster: 32 pairs of 1000 keys 6.6 / 5.7 (of 64 6.1 / 4.5), of 100 5.0 / 4.1; 16 of 2000 7.4 / 6.6; 96 of 500 7.9 / 6.8; 112 of 900 10.7 /
-        // 9.8; but where a split has several chunks and a CTA would take two, 32 of 2000 9.0 / 9.4, 192 of 500 9.7 / 12.4.
+        // 9.8; but where a split has several chunks and a CTA would take two, 32 of 2000 9.0 / 9.4, 192 of 500 9.7 / 12.4.  Near what fits clusters wait for room: 40 of 2200
+        // in 13s of 38 that fit 9.8 / 12.0, 172 of 900 in 3s of 187 12.8 / 12.5 (of 64 10.4 / 13.5), 184 13.0 / 17.2 (10.5 / 14.0), 164 12.7 / 11.8 (10.3 / 9.6); pairs of CTAs do not (all 296: of 500
+        // keys 11.9 / 11.1), nor 4s up to 132 of 142 (11.4 / 10.4).
         // Fewer than 16 pairs keep the workspace, which is not the faster one there (8 pairs of 1000 keys 5.6 / 4.4): the line is not where clusters stop paying, but
         // calls of eight pairs are what the tests of scratch and of captured calls take for a cut pair in the workspace (tests/test_fa_scratch_gpu.py).
         const ClusterFit& fit = cluster_fit();
         const long long each = (chunks + x.splits - 1) / x.splits, used = each ? (chunks + each - 1) / each : 0;
-        auto placed = [&](long long n) { return n > PORTABLE_CLUSTER ? 8 * pairs <= 7 * fit.n[n] : n > 3 ? 16 * pairs <= 15 * fit.n[n] : pairs <= fit.n[n]; };
+        auto placed = [&](long long n) { return n > PORTABLE_CLUSTER ? 8 * pairs <= 7 * fit.n[n] : n > 3 ? 16 * pairs <= 15 * fit.n[n] : n == 3 ? 9 * pairs <= 8 * fit.n[n] : pairs <= fit.n[n]; };
         auto steps_of = [&](long long n) { return (used + n - 1) / n * each; };
         long long size = used < MAX_CLUSTER ? used : MAX_CLUSTER;
         while (size > 1 && !placed(size)) size--;

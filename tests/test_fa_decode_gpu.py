@@ -302,3 +302,24 @@ def test_a_run_of_splits_is_rounded_as_splits_of_their_own(cuda, built_libs, fa_
         (runs, lse), (own, own_lse) = (run_decode(fa_ctx, q[:, :h], k[:, :h], v[:, :h], [n], scale, sv) for h in (16, 15))
         assert (runs[:, :15] != own).mean() <= 0.02, (n, (runs[:, :15] != own).mean())
         assert np.abs(lse[:, :15] - own_lse).max() <= 1e-5
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,H,Smax,cluster", [(41, 4, 900, True), (42, 4, 900, False), (11, 16, 900, False), (46, 4, 130, True), (47, 4, 130, True), (74, 4, 500, True)])
+def test_clusters_of_three_keep_clear_of_what_fits(cuda, built_libs, fa_ctx, D, B, H, Smax, cluster):
+    # near the number that is resident at once they wait for one another; pairs of blocks do not (184 sequences and heads of three chunks are pairs), and all that there
+    # is room for are taken
+    from tests.gpu_util import kernels
+    q, k, v, sq, sk, sv = make_case(f"threes{B}_{H}_{Smax}_{D}", B, H, H, Smax, D)
+    scale = sq * sk / math.sqrt(D)
+    qd, kd, vd = (torch.from_numpy(t).cuda() for t in (q, k, v))
+    lens = np.random.default_rng(B).integers(1, Smax + 1, size=B)
+    o, ld = torch.empty(B, H, D, dtype=torch.float16, device="cuda"), torch.from_numpy(lens.astype(np.int32)).cuda()
+    names = kernels(lambda: fa_ctx.Decode(qd.data_ptr(), kd.data_ptr(), vd.data_ptr(), o.data_ptr(), 0, ld.data_ptr(), B, H, H, D, Smax, 0, scale, sv,
+                                          stream=torch.cuda.current_stream().cuda_stream))
+    assert len(names) == (1 if cluster else 2)   # the workspace's words are cleared by another
+    got, lse = run_decode(fa_ctx, q, k, v, lens, scale, sv)
+    ref, rl = glue.decode_attention_f64(q, k, v, lens, scale, sv)
+    maxabs, meanrel = O.error_stats(got, ref)
+    assert maxabs <= 2e-2 and meanrel <= 1e-2, (maxabs, meanrel)
+    assert np.abs(lse - rl).max() <= 5e-3
