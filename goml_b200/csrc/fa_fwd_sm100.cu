@@ -437,8 +437,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     const bool bad_start = (*abort_flag != 0);
     if (VRAW) {
         pdl_wait();   // no pre-pass has waited for what is ahead
-        // The next kernel's start (its launch, barriers, tensor memory) beside this one, where a launch leaves SMs free: 4 heads of 256 keys, not causal, 5.31 / 4.98
-        // us a call, of 128, causal, 5.04 / 4.67, 12 of 1000 12.9 / 12.6; with more CTAs than SMs 9.7 / 9.9.  D = 128 loses by it (4 of 256 5.8 / 6.1, 24
+        // The next kernel's start (its launch, barriers, tensor memory) beside this one, where a launch leaves SMs free: calls behind one another, 4 heads of 256 keys, not
+        // causal, 5.31 / 4.98 us each, of 128, causal, 5.04 / 4.67, 12 of 1000 12.9 / 12.6 (a call with nothing behind it takes what it took); with more CTAs than SMs 9.7 / 9.9.  D = 128 loses by it (4 of 256 5.8 / 6.1, 24
         // of 700 11.7 / 12.5), and with the trigger ahead of the rows out (32 of 512 9.7 / 9.9).
         if (HD == 64 && !WALK && p.few) pdl_trigger();
     }

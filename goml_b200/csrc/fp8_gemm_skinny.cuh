@@ -13,7 +13,7 @@
 //    57 bytes a nanosecond, so weights have to be spread over nearly all of them to reach the 6.5 TB/s of HBM);
 //  * the kernel starts before its predecessor on the stream has drained and asks for its first weight tiles to be
 //    brought into L2 while the small kernel ahead (a quantiser, usually) still runs.
-// What is left is 3 us of start, fill and finish beside the stream: M = 16, 8192 x 8192 14.1 us (floor 10.3),
+// What is left is 3 us of start, fill and finish beside the stream: M = 16, 8192 x 8192 14.0 us (floor 10.3),
 // 12288 x 4096 11.2 (7.7), 22016 x 4096 with SwiGLU
 // 18.4 (13.8), 4096 x 11008 10.7 (6.9), 4096 x 4096 6.5 (2.6).
 #pragma once
@@ -686,10 +686,11 @@ inline int launch(GemmParams g, const Plan& plan, const void* A, const void* B, 
     const int room = smem - TAIL_BYTES - tok_bytes;
     auto stages_in = [&](int bytes) {
         int n = bytes / stage_bytes;
-        if (rows && plan.per_sm == 3 && n > 3) n = 3;   // the rows' values wait behind what the rings have asked for: a step of one sequence 67.0, with four 67.7
+        if (rows && plan.per_sm == 3 && n > 3) n = 3;   // the rows' values wait behind what the rings have asked for: a step of one sequence of a 4096 wide block 64.6 us, with four 65.7;
+                                                        // two sequences, and blocks 1024 to 6144 wide, level
         return n > slice ? slice : n > MAX_STAGES ? MAX_STAGES : n;
     };
-    // Partial sums of up to 16 tokens have memory of their own where that costs no stage; a row as values has 512 bytes
+    // Partial sums of up to 16 tokens have memory of their own where that costs no stage; a row as values has 512 to 672 bytes, by the cut
     const int own_bytes = apart_bytes(plan.split, g.M);
     const bool apart = rows || (g.M <= APART_TOKENS && stages_in(room - own_bytes) == stages_in(room));
     p.stages = stages_in(apart ? room - own_bytes : room);
