@@ -85,6 +85,10 @@ __device__ __forceinline__ void prefetch_l2_2d(const CUtensorMap* m, int x, int 
 // Else they lie with their source, as [token][128].
 __host__ __device__ constexpr int pairs_of(int split) { return (16 + split - 1) / split; }
 __host__ __device__ constexpr int apart_bytes(int split, int tokens) { return split * tokens * 2 * pairs_of(split) * 16; }
+// with rows as values at least the block that the last MMAs read behind the codes
+__host__ __device__ constexpr int part_room(int split, int tokens, bool values) {
+    return values && apart_bytes(split, tokens) < TOKEN_BYTES ? TOKEN_BYTES : apart_bytes(split, tokens);
+}
 template <int SPLIT>
 __device__ __forceinline__ int first_pair(int rank) { return (16 * rank + SPLIT - 1) / SPLIT; }   // owner of pair u: u * SPLIT / 16
 // the sums of all sources for four rows and a token; a: where they lie in this CTA
@@ -250,12 +254,12 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;   // swizzle atoms are 1024 bytes
     uint8_t* ring_gen = smem_raw + (ring - smem_u32(smem_raw));
     const int stage_bytes = VALUES ? W_BYTES : W_BYTES + p.tn * BK;   // a multiple of 2048
-    // VALUES: the codes of this CTA's k-blocks, eight rows each.  The MMA takes sixteen tokens; the other eight, which nobody looks at, it
-    // finds in the block behind, so that there is one block more
+    // VALUES: the codes of this CTA's k-blocks, eight rows each.  The MMA takes sixteen tokens; the other eight, whose sums nobody looks at, it
+    // finds in the block behind, be it codes or partial sums that arrive
     const uint32_t tok = ring + p.stages * stage_bytes;
-    const uint32_t tok_bytes = VALUES ? (p.slice + 1) * TOKEN_BYTES : 0;
+    const uint32_t tok_bytes = VALUES ? p.slice * TOKEN_BYTES : 0;
     const uint32_t part = APART ? tok + tok_bytes : ring;
-    const uint32_t part_bytes = APART ? apart_bytes(SPLIT, p.g.M) : 0;
+    const uint32_t part_bytes = APART ? part_room(SPLIT, p.g.M, VALUES) : 0;
     const uint32_t bar_full = tok + tok_bytes + part_bytes;
     const uint32_t bar_empty = bar_full + 8 * MAX_STAGES;
     const uint32_t bar_done = bar_empty + 8 * MAX_STAGES;
@@ -677,7 +681,7 @@ inline int launch(GemmParams g, const Plan& plan, const void* A, const void* B, 
     const int tiles = (g.N + W_ROWS - 1) / W_ROWS;
     const int slice = (g.k_blocks + plan.split - 1) / plan.split;
     const int stage_bytes = rows ? W_BYTES : W_BYTES + p.tn * BK;
-    const int tok_bytes = rows ? (slice + 1) * TOKEN_BYTES : 0;
+    const int tok_bytes = rows ? slice * TOKEN_BYTES : 0;
     p.slice = slice;
     // A long stream of up to 32 tokens with an SM to itself has 160 KB in flight and not all 227: what is asked for beyond some 20 MB only waits in front
     // of memory.  Us, 227 KB / 160 (112 KB: a fifth slower): 16 tokens, 8192 x 8192 14.25 / 14.1, 16384 x 16384 45.2 / 44.7, 5000 x 8000 10.6 / 10.4, 4 tokens,
@@ -690,11 +694,12 @@ inline int launch(GemmParams g, const Plan& plan, const void* A, const void* B, 
                                                         // two sequences, and blocks 1024 to 6144 wide, level
         return n > slice ? slice : n > MAX_STAGES ? MAX_STAGES : n;
     };
-    // Partial sums of up to 16 tokens have memory of their own where that costs no stage; a row as values has 512 to 672 bytes, by the cut
-    const int own_bytes = apart_bytes(plan.split, g.M);
+    // Partial sums of up to 16 tokens have memory of their own where that costs no stage; a row as values has 512 to 672 bytes, by the cut, and they begin in the block
+    // behind the codes, so that as long a K finds room for two stages as without them (two rows: 192, 77 and 39 k-blocks to one of one, two and three CTAs of an SM)
+    const int own_bytes = part_room(plan.split, g.M, rows != nullptr);
     const bool apart = rows || (g.M <= APART_TOKENS && stages_in(room - own_bytes) == stages_in(room));
     p.stages = stages_in(apart ? room - own_bytes : room);
-    if (rows && room - own_bytes < 2 * stage_bytes) return (int)cudaErrorNotSupported;
+    if (rows && (room - own_bytes < 2 * stage_bytes || (plan.per_sm == 3 && slice > 39))) return (int)cudaErrorNotSupported;
     int ring_bytes = p.stages * stage_bytes;
     const int part_bytes = apart ? own_bytes : 0;
     while (!apart && ring_bytes < p.tn * W_ROWS * 4) { p.stages++; ring_bytes += stage_bytes; }   // the partial sums take the ring's place

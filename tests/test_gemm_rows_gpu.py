@@ -75,6 +75,30 @@ def test_rows_against_quantiser_and_product(cuda, built_libs, m, n, k, source):
     assert G.device_status() == 0
 
 
+# as many k-blocks to a CTA as leave two stages: 192 of a whole K, of two and three slices, 77 where two CTAs share an SM, 39 of two slices where three do; one more is refused
+@pytest.mark.parametrize("m,n,k,taken", [(2, 14336, 24576, True), (1, 14336, 24576, True), (2, 14336, 24592, False), (2, 7680, 49152, True), (1, 5120, 73728, True), (2, 5120, 73728, True),
+                                         (2, 30720, 9856, True), (2, 30720, 9872, False), (2, 20480, 9984, True), (2, 20480, 10000, False)])
+def test_the_longest_rows(cuda, built_libs, m, n, k, taken):
+    # 448 times -1, 0 or 1 has the scale 1, and the sums with weights of -1, 0 and 1 are multiples of 448 that fp32 holds
+    import torch
+    from goml_b200 import fp8_gemm as G
+    lib = G._init()
+    g = torch.Generator(device="cuda").manual_seed(n + k + m)
+    ones = lambda *shape: torch.randint(-1, 2, shape, generator=g, dtype=torch.int8, device="cuda")
+    x, w = ones(m, k), ones(n, k)
+    x[:, 0] = 1
+    rows = (448 * x.float()).half()
+    codes = torch.where(w == 0, 0, torch.where(w > 0, 0x38, 0xb8)).to(torch.uint8)
+    base, one = torch.randint(-50, 50, (m, n), generator=g, device="cuda").float(), torch.ones(1, device="cuda")
+    out = torch.full((m + 1, n), 7.0, device="cuda")
+    rc = call(lib, rows=rows.data_ptr(), b=codes.data_ptr(), scale_b=one.data_ptr(), x=out.data_ptr(), x_in=base.data_ptr(), m=m, n=n, k=k, source=G.RowsF16)
+    torch.cuda.synchronize()
+    assert G.device_status() == 0
+    assert rc == (0 if taken else NOT_SUPPORTED)
+    want = base.double() + 448 * torch.stack([torch.cat([(x[j:j + 1] * part).sum(1, dtype=torch.int32) for part in w.split(1024)]) for j in range(m)])
+    assert torch.equal(out[:m].double(), want if taken else torch.full_like(want, 7.0)) and (out[m] == 7).all()
+
+
 # n a multiple of four or not, whole and cut tiles; sizes that need four slices and one
 @pytest.mark.parametrize("m,n,k", [(1, 4096, 4096), (2, 1000, 2048), (2, 1001, 2000)])
 def test_the_stream_may_lie_on_any_four_bytes(cuda, built_libs, m, n, k):
