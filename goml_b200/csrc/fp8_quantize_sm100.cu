@@ -134,10 +134,13 @@ struct QuantOp {
     float divisor;
     using State = NoState;
     __device__ void ahead() const {}
-    __device__ void pass1(float (&m)[1], State&) const { m[0] = amax_items<WIDE, BATCH>(x, n, oc_tid(), oc_step()); }
+    // The step of a full cluster, known to the compiler: a smaller one has a group per thread at most.  With the step from the launch, us, alone / behind a
+    // GEMM of 16 x 4096 x 4096 (before clusters had sizes; now): 32 values 2.32 / 8.38 (2.12 / 8.93; 2.05 / 8.07), 4096 2.58 / 8.53 (2.53 / 9.27; 2.32 / 8.33), 53866 3.06 / 9.08
+    // (2.92 / 9.76; 2.85 / 8.86).
+    __device__ void pass1(float (&m)[1], State&) const { m[0] = amax_items<WIDE, BATCH>(x, n, oc_tid(), OC_STEP); }
     __device__ void pass2(const float (&m)[1], State&) const {
         if (oc_tid() == 0) *amax_out = m[0];
-        quant_items<WIDE, BATCH>(x, q, n, oc_tid(), oc_step(), m[0], scale_out, divisor);
+        quant_items<WIDE, BATCH>(x, q, n, oc_tid(), OC_STEP, m[0], scale_out, divisor);
     }
 };
 
