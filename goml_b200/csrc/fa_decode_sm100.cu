@@ -52,6 +52,7 @@ constexpr int THREADS = 128;
 constexpr int WARPS = THREADS / 32;
 constexpr float LAG = 6.0f;      // log2 units
 constexpr int LONGEST_SPLIT = 8;   // chunks of a split up to which a cluster is worth it: past that it is level with the workspace
+constexpr int FEW_SPLITS = 8;      // up to so many the last CTA takes up the pieces of a pair in one round of 32 threads (16, D = 64)
 constexpr int MAX_CLUSTER = 16, PORTABLE_CLUSTER = 8;   // splits of a pair that are a cluster
 constexpr int HINTS = 2;         // chunks a CTA asks for ahead of the wait
 // A wide warp step takes twice the keys of a narrow one (8 against 4 KB in flight per warp) and leaves registers for 12
@@ -202,10 +203,12 @@ struct Segment {
 };
 
 // CLUSTER: the splits of a pair are the CTAs of a cluster (one query head per kv head), its first CTA the one with the first run of them
-template <int D, int NQ, bool WIDE, bool STREAMS, bool PAGED, bool CLUSTER = false>
+// MANY: all threads of the last CTA take up the pieces of a pair in the workspace (one query head per kv head).  A kernel of its own, for its code costs every call 0.1 us:
+// 12 heads of 16 keys, us, with it / without 2.73 / 2.64, 2 of 385 (7 splits) 4.98 / 4.79, 14 of 256 (4) 4.84 / 4.65; but 8 of 1000 (16) 5.30 / 5.92, 2 of 4000 5.65 / 8.86.
+template <int D, int NQ, bool WIDE, bool STREAMS, bool PAGED, bool MANY = false, bool CLUSTER = false>
 __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_kernel(const DecodeParams p) {
     using C = Cfg<D, NQ, WIDE>;
-    static_assert(!CLUSTER || (STREAMS && NQ == 1), "clusters are for one query head per kv head");
+    static_assert(!(CLUSTER || MANY) || (STREAMS && NQ == 1), "clusters and many pieces are for one query head per kv head");
     __shared__ __align__(16) float s_o[WARPS][CLUSTER ? 1 : C::ROWS][C::PITCH];
     __shared__ float s_m[WARPS][C::ROWS], s_l[WARPS][C::ROWS];
     __shared__ Segment s_next[WARPS];
@@ -732,7 +735,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(D, NQ, WIDE)) fa_decode_k
                 if (s_last) p.arrivals[bh] = 0;   // for the next launch
             }
             __syncthreads();
-            if (s_last && STREAMS) {
+            if (s_last && MANY) {
                 // one row: a group of D / 4 threads takes every GROUPS-th piece, eight loads in flight, and the groups' states meet in shared memory
                 __threadfence();
                 constexpr int LANES = D / 4, GROUPS = THREADS / LANES;
@@ -844,8 +847,8 @@ __global__ void clear_words_kernel(uint32_t* w, uint32_t n) {
 // Kernels whose splits are a cluster: [paged][head dim 128]
 using DecodeKernel = void (*)(const DecodeParams);
 DecodeKernel cluster_kernel(int hd, bool paged) {
-    if (hd == 64) return paged ? fa_decode_kernel<64, 1, false, true, true, true> : fa_decode_kernel<64, 1, false, true, false, true>;
-    return paged ? fa_decode_kernel<128, 1, false, true, true, true> : fa_decode_kernel<128, 1, false, true, false, true>;
+    if (hd == 64) return paged ? fa_decode_kernel<64, 1, false, true, true, false, true> : fa_decode_kernel<64, 1, false, true, false, false, true>;
+    return paged ? fa_decode_kernel<128, 1, false, true, true, false, true> : fa_decode_kernel<128, 1, false, true, false, false, true>;
 }
 cudaLaunchConfig_t cluster_config(cudaLaunchAttribute* attr, int grid, int size, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
@@ -1016,6 +1019,9 @@ cudaError_t launch_decode(const DecodeArgs& a) {
         return cudaLaunchKernelEx(&cfg, cluster_kernel(a.hd, a.block_table != nullptr), p);
     }
     auto run = [&](auto contiguous, auto paged) { return launch_pdl(a.block_table ? paged : contiguous, x.grid, THREADS, 0, a.stream, p); };
+    if (x.streams && x.splits > FEW_SPLITS)
+        return a.hd == 64 ? run(fa_decode_kernel<64, 1, false, true, false, true>, fa_decode_kernel<64, 1, false, true, true, true>)
+                          : run(fa_decode_kernel<128, 1, false, true, false, true>, fa_decode_kernel<128, 1, false, true, true, true>);
 #define KERNEL(D, NQ, WIDE, STREAMS) run(fa_decode_kernel<D, NQ, WIDE, STREAMS, false>, fa_decode_kernel<D, NQ, WIDE, STREAMS, true>)
     if (x.streams) return a.hd == 64 ? KERNEL(64, 1, false, true) : x.wide ? KERNEL(128, 1, true, true) : KERNEL(128, 1, false, true);
     if (x.rows == 8) return a.hd == 64 ? KERNEL(64, 1, true, false) : KERNEL(128, 1, true, false);

@@ -132,7 +132,7 @@ struct Params {
     uint32_t v_epoch;
     int v_chunks;              // chunks per head
     int group;                 // heads whose tiles are interleaved
-    int few;                   // the launch leaves SMs free: the next kernel may come at once
+    int few;                   // the launch leaves SMs free, and O's quantiser is not what follows: the next kernel may come at once
 };
 
 __device__ __forceinline__ float ex2(float x) {
@@ -437,9 +437,11 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     const bool bad_start = (*abort_flag != 0);
     if (VRAW) {
         pdl_wait();   // no pre-pass has waited for what is ahead
-        // The next kernel's start (its launch, barriers, tensor memory) beside this one, where a launch leaves SMs free: calls behind one another, 4 heads of 256 keys, not
-        // causal, 5.31 / 4.98 us each, of 128, causal, 5.04 / 4.67, 12 of 1000 12.9 / 12.6 (a call with nothing behind it takes what it took); with more CTAs than SMs 9.7 / 9.9.  D = 128 loses by it (4 of 256 5.8 / 6.1, 24
-        // of 700 11.7 / 12.5), and with the trigger ahead of the rows out (32 of 512 9.7 / 9.9).
+        // The next kernel's start (its launch, barriers, tensor memory, hints) beside this one, where a launch leaves SMs free: calls behind one another, 4 heads of 256
+        // keys, not causal, 5.43 / 5.05 us each, 28 of 125, causal, 5.24 / 4.91, 13 of 1251 15.2 / 15.0 (a call with nothing behind it takes what it took), in front of a GEMM of 16 x
+        // 4096 x 4096 11.6 / 10.8, 11.4 / 10.4 and 21.8 / 20.7 for both; with more CTAs than SMs 9.7 / 9.9.  D = 128 loses by it (4 of 256 5.8 / 6.1, 24 of 700 11.7 / 12.5), and with the
+        // trigger ahead of the rows out (32 of 512 9.7 / 9.9).  A quantiser of O behind it has little to set up and then takes longer from the wait on (7.6 / 7.5, 8.4 / 8.7, 19.9 / 20.1), so a
+        // call that leaves it the maximum keeps the trigger at the end: a block of 32 heads over 100 tokens 50.4 / 50.7, 256 62.3 / 62.7, 512 84.3 / 85.0.
         if (HD == 64 && !WALK && p.few) pdl_trigger();
     }
     if (bad_start) {
@@ -1091,7 +1093,7 @@ cudaError_t launch_hd(const LaunchArgs& a, int num_sms) {
         return cudaErrorInvalidValue;
     Params p;
     p.group = heads_together(a, grid, num_sms);
-    p.few = grid <= num_sms;
+    p.few = grid <= num_sms && !a.o_amax;
     p.bh = a.bh; p.sl = a.sl; p.n_qtiles = (a.sl + BM - 1) / BM;
     p.causal = a.causal; p.window = a.window;
     p.scale_log2 = a.scale * 1.4426950408889634f;

@@ -285,6 +285,19 @@ def test_splits_in_clusters_and_in_the_workspace(cuda, built_libs, fa_ctx, B, H,
         assert np.abs(lse - rl).max() <= 5e-3
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,H,Smax,many", [(1, 8, 128, False), (1, 8, 512, False), (1, 8, 513, True), (2, 7, 575, True), (2, 7, 500, False), (3, 2, 2500, True), (1, 1, 4200, True)])
+def test_few_and_many_pieces_in_the_workspace(cuda, built_libs, fa_ctx, B, H, Smax, D, many):
+    # up to eight pieces of a pair are taken up by one group of threads, more by all of the block's, in a kernel of its own
+    from tests.gpu_util import kernels
+    x = torch.zeros(B * H * Smax * D, dtype=torch.uint8, device="cuda")
+    o = torch.empty(B, H, D, dtype=torch.float16, device="cuda")
+    names = kernels(lambda: fa_ctx.Decode(x.data_ptr(), x.data_ptr(), x.data_ptr(), o.data_ptr(), 0, 0, B, H, H, D, Smax, Smax, 1.0, 1.0, stream=torch.cuda.current_stream().cuda_stream))
+    name, = (n for n in names if "fa_decode_kernel" in n)
+    assert name.split("EvN")[0].endswith("Lb1ELb0EE" if many else "Lb0ELb0EE")
+    test_splits_in_clusters_and_in_the_workspace(cuda, built_libs, fa_ctx, B, H, Smax, D, False)
+
+
 @pytest.mark.parametrize("D,Smax", [(64, 2368), (64, 2000), (128, 2368), (128, 1800)])
 def test_a_run_of_splits_is_rounded_as_splits_of_their_own(cuda, built_libs, fa_ctx, D, Smax):
     # A block of a cluster that takes two or three splits in turn starts a maximum for each: 16 heads are clusters, the first 15 of them meet in the workspace, and P
