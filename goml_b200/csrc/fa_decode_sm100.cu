@@ -944,7 +944,8 @@ Layout layout_of(int batch, int q_heads, int kv_heads, int head_dim, int span) {
         // Us, workspace / cluster: 32 pairs of 1000 keys 6.6 / 5.7 (of 64 6.1 / 4.5), of 100 5.0 / 4.1; 16 of 2000 7.4 / 6.6; 96 of 500 7.9 / 6.8; 112 of 900 10.7 /
         // 9.8; but where a split has several chunks and a CTA would take two, 32 of 2000 9.0 / 9.4, 192 of 500 9.7 / 12.4.  Near what fits clusters wait for room: 40 of 2200
         // in 13s of 38 that fit 9.8 / 12.0, 172 of 900 in 3s of 187 12.8 / 12.5 (of 64 10.4 / 13.5), 184 13.0 / 17.2 (10.5 / 14.0), 164 12.7 / 11.8 (10.3 / 9.6); pairs of CTAs do not (all 296: of 500
-        // keys 11.9 / 11.1), nor 4s up to 132 of 142 (11.4 / 10.4).
+        // keys 11.9 / 11.1), nor 4s up to 132 of 142 (11.4 / 10.4).  The lengths are on the device: sequences that fill an eighth of the cache or less pay a cluster's start for nothing, 32 of 28 of 64
+        // in 226 2.9 / 3.3, 64 of 60 in 500 3.5 / 3.75, 288 of up to 90 in 718 4.4 / 5.0.
         // Fewer than 16 pairs keep the workspace, which is not the faster one there (8 pairs of 1000 keys 5.6 / 4.4): the line is not where clusters stop paying, but
         // calls of eight pairs are what the tests of scratch and of captured calls take for a cut pair in the workspace (tests/test_fa_scratch_gpu.py).
         const ClusterFit& fit = cluster_fit();
